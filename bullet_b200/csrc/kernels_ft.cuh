@@ -33,8 +33,9 @@ constexpr int kStatusOutsideBlock = 1;  // a feature fell outside its position's
 
 struct FtArgs {
     const float* table;   // [n_inputs][H] effective weights: l0w, or l0w + tiled l0f already merged
-    const float* factor;  // tiled forward only: [factor_rows][H] l0f to be added to `table` (= l0w) on the fly, or null
+    const float* factor;  // forward only: [factor_rows][H] l0f to be added to `table` (= l0w) on the fly, or null
     int factor_rows;
+    int block_rows;       // gather forward only: > 0 drops features outside the block of their pair's first one, as the tiled kernels do
     const float* bias;    // [H]
     const uint16_t* idx_stm;
     const uint16_t* idx_nstm;  // [n][nnz] each, 0xFFFF = empty slot
@@ -103,6 +104,10 @@ __device__ __forceinline__ void load_slots(const uint16_t* list, int nnz, int la
 
 // ---------------------------------------------------------------- gather forward
 // grid = (ceil(2n / pairs_per_block), chunks); block = 256 threads (8 warps).
+// Takes index sets without block structure, and the small batches of networks that have it: staging the table's tiles
+// costs the tiled kernel the whole table whatever the batch holds, here only the rows of the batch are read.
+// Bound by L2 for large batches and by load latency (one pair per warp, four rows in flight) for small ones.  With a
+// factoriser the two rows of a feature are added as they arrive, so a small batch does not merge the table first.
 template <bool PAIRWISE>
 __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pairs_per_block) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -120,10 +125,20 @@ __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pa
         const uint16_t* list = (p ? a.idx_nstm : a.idx_stm) + (size_t)b * a.nnz;
         uint32_t slot[2];
         load_slots(list, a.nnz, lane, slot[0], slot[1]);
+        unsigned mask[2];
+        mask[0] = __ballot_sync(0xffffffffu, slot[0] < (uint32_t)a.n_inputs);
+        mask[1] = __ballot_sync(0xffffffffu, slot[1] < (uint32_t)a.n_inputs);
+        if (a.block_rows > 0 && (mask[0] | mask[1])) {
+            const uint32_t first = __shfl_sync(0xffffffffu, mask[0] ? slot[0] : slot[1], __ffs(mask[0] ? mask[0] : mask[1]) - 1);
+            const uint32_t base = first / a.block_rows * a.block_rows;
+            mask[0] &= __ballot_sync(0xffffffffu, slot[0] - base < (uint32_t)a.block_rows);
+            mask[1] &= __ballot_sync(0xffffffffu, slot[1] - base < (uint32_t)a.block_rows);
+        }
+        const uint32_t frow[2] = {a.factor ? slot[0] % a.factor_rows : 0u, a.factor ? slot[1] % a.factor_rows : 0u};
         float4 lo = make_float4(0, 0, 0, 0), hi = lo;
 #pragma unroll
         for (int half = 0; half < 2; half++) {
-            unsigned m = __ballot_sync(0xffffffffu, slot[half] < (uint32_t)a.n_inputs);
+            unsigned m = mask[half];
             while (m) {  // up to four independent row loads in flight, added in slot order
                 int s[4];
                 int cnt = 0;
@@ -133,7 +148,7 @@ __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pa
                     if (m) cnt++;
                     m &= m - 1;
                 }
-                float4 vlo[4], vhi[4];
+                float4 vlo[4], vhi[4], flo[4], fhi[4];
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
                     const uint32_t f = __shfl_sync(0xffffffffu, slot[half], s[k]);
@@ -142,6 +157,23 @@ __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pa
                         vlo[k] = __ldg(reinterpret_cast<const float4*>(row + col));
                         if (PAIRWISE) vhi[k] = __ldg(reinterpret_cast<const float4*>(row + unit + col));
                     }
+                }
+                if (a.factor) {
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const uint32_t f = __shfl_sync(0xffffffffu, frow[half], s[k]);
+                        if (k < cnt && active) {
+                            const float* row = a.factor + (size_t)f * a.H;
+                            flo[k] = __ldg(reinterpret_cast<const float4*>(row + col));
+                            if (PAIRWISE) fhi[k] = __ldg(reinterpret_cast<const float4*>(row + unit + col));
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; k++)
+                        if (k < cnt && active) {
+                            vlo[k] = add4(vlo[k], flo[k]);
+                            if (PAIRWISE) vhi[k] = add4(vhi[k], fhi[k]);
+                        }
                 }
 #pragma unroll
                 for (int k = 0; k < 4; k++)

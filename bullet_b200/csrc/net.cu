@@ -52,6 +52,7 @@
 namespace {
 
 constexpr int64_t kAlignFloats = 64;       // 256-byte tensor alignment in the flat buffers
+constexpr int kGatherRowsPerPosition = 34;  // active features of both perspectives of a middling chess position
 constexpr int kMinItemPairs = 128;         // a forward work item serves at least this many pairs per tile load
 
 struct Tensor {
@@ -172,7 +173,9 @@ struct b200_net {
     bool sig_on = false;                 // the running backward announces finished row blocks
     int sig_value = 0;
     bool manual_grad_zero = false;  // the caller zeroes the gradient buffer range by range (b200_grad_zero_range)
-    bool tiled_ok = false, table_dirty = true, have_backward = false;
+    bool tiled_ok = false, have_backward = false;
+    bool w1_dirty = true, merged_dirty = true;  // the weights moved since the regrouped first dense layer / the merged table was built
+    bool trains = false;  // a training pass has run: uploads then also build what only the backward reads
     int nblocks = 1, nslabs = 1;
     int last_n = 0;
     // per-step CUDA events on the compute stream, kept for the last kTimingRing steps
@@ -195,6 +198,18 @@ struct b200_net {
     // AUTO: both passes take the shared-memory kernels whenever the inputs allow it (measured
     // at 16384 positions, H = 2048: backward 0.50 ms against 0.61 ms for global vector reductions)
     bool fwd_tiled() const { return ft_fwd_mode == B200_FT_TILED || (ft_fwd_mode == B200_FT_AUTO && tiled_ok); }
+    // ... for a whole batch of n positions.  The tiled forward stages every table row once whatever the batch holds, in few
+    // CTAs when there are few pairs; the gather forward reads the rows of the batch only (two per feature with a
+    // factoriser).  Measured (king buckets, 2048 wide, forward of n positions in us): n = 1 52 against 458, n = 512 86
+    // against 97, n = 1024 122 against 100: the lines cross where the gather reads about four times the table's rows.
+    bool fwd_tiled(int n) const {
+        if (ft_fwd_mode == B200_FT_AUTO && tiled_ok && (long long)n * kGatherRowsPerPosition * (d.factoriser_rows ? 2 : 1) <= 4LL * d.n_inputs) return false;
+        return fwd_tiled();
+    }
+    // The gather forward of n positions reads the merged table (one row per feature, after a pass over the whole table)
+    // when the batch gathers several times the table's rows; below that it adds the factoriser row by row.
+    bool merged_table(int n) const { return d.factoriser_rows && !fwd_tiled(n) && (long long)n * d.nnz >= 5LL * d.n_inputs; }
+    void weights_moved() { w1_dirty = merged_dirty = true; }
     bool bwd_tiled() const { return ft_bwd_mode == B200_FT_TILED || (ft_bwd_mode == B200_FT_AUTO && tiled_ok); }
     // the register-tiled dense forward (rows per bucket in fours, more layers after the first) also
     // forms the gradients of those later layers
@@ -300,8 +315,11 @@ int launch_ft_forward(b200_net* net, const b200::FtArgs& a, const b200::TileArgs
         b200::ft_forward_tiled_kernel<PW><<<grid, b200::kFwdThreads, b200::ft_fwd_smem(t.block_rows, t.list_len), net->stream>>>(a, t);
     } else {
         const int unit = PW ? a.H / 2 : a.H;
-        dim3 grid((2 * a.n + 63) / 64, (unit + 127) / 128);
-        b200::ft_forward_gather_kernel<PW><<<grid, 256, 0, net->stream>>>(a, 64);
+        // one pair per warp while there are few, up to eight once that leaves two waves of eight CTAs per SM
+        const long long pieces = (long long)2 * a.n * ((unit + 127) / 128);
+        const int pairs = 8 * (int)std::max<long long>(1, std::min<long long>(8, pieces / (8LL * 16 * net->sm_count)));
+        dim3 grid((2 * a.n + pairs - 1) / pairs, (unit + 127) / 128);
+        b200::ft_forward_gather_kernel<PW><<<grid, 256, 0, net->stream>>>(a, pairs);
     }
     LAUNCHED(net);
     return 0;
@@ -385,12 +403,13 @@ int ft_backward_grid(const b200_net* net, const Slot& s, int first, int last, bo
 b200::FtArgs ft_args(b200_net* net, const Slot& s) {
     b200::FtArgs a{};
     const b200_net_desc& d = net->d;
-    // the tiled forward adds the factoriser while it fills its tile; only the gather forward
+    // the tiled forward adds the factoriser while it fills its tile; only the gather forward of a large batch
     // needs the merged table
-    const bool merged = net->d.factoriser_rows && !net->fwd_tiled();
+    const bool merged = net->merged_table(s.n);
     a.table = merged ? net->table : net->P + net->find("l0w")->off;
     a.factor = (net->d.factoriser_rows && !merged) ? net->P + net->find("l0f")->off : nullptr;
     a.factor_rows = net->d.factoriser_rows;
+    a.block_rows = net->ft_fwd_mode == B200_FT_AUTO && net->tiled_ok ? d.ft_block_rows : 0;
     a.bias = net->P + net->find("l0b")->off;
     a.idx_stm = s.dev<uint16_t>(s.off_stm);
     a.idx_nstm = s.dev<uint16_t>(s.off_nstm);
@@ -479,9 +498,8 @@ b200::DenseArgs dense_args(b200_net* net, const Slot& s, bool want_grad) {
     return a;
 }
 
-int refresh_table(b200_net* net) {
-    if (!net->table_dirty) return 0;
-    if (net->d.factoriser_rows && !net->fwd_tiled()) {
+int refresh_table(b200_net* net, int n) {
+    if (net->merged_dirty && net->merged_table(n)) {
         const Tensor* w = net->find("l0w");
         const Tensor* f = net->find("l0f");
         const size_t n4 = (size_t)w->n / 4, block4 = (size_t)f->n / 4;
@@ -489,14 +507,15 @@ int refresh_table(b200_net* net) {
             reinterpret_cast<const float4*>(net->P + w->off), reinterpret_cast<const float4*>(net->P + f->off),
             reinterpret_cast<float4*>(net->table), n4, block4);
         LAUNCHED(net);
+        net->merged_dirty = false;
     }
-    {
+    if (net->w1_dirty) {
         const Tensor* w1 = net->find("l1w");
         b200::dense_regroup_kernel<<<std::min<int>(net->sm_count * 4, (int)((w1->n + 255) / 256)), 256, 0, net->stream>>>(
             net->P + w1->off, net->w1g, net->D1(), net->d.n_out_buckets, net->d.dense_out[0]);
         LAUNCHED(net);
+        net->w1_dirty = false;
     }
-    net->table_dirty = false;
     return 0;
 }
 
@@ -513,7 +532,7 @@ int check_slot(b200_net* net, int slot, const char* who) {
 int forward_prepare(b200_net* net, Slot& s, bool want_grad) {
     b200::FtArgs fa = ft_args(net, s);
     b200::TileArgs ta = tile_args(net, s, false);
-    const bool needed = net->fwd_tiled() || (want_grad && net->bwd_tiled());
+    const bool needed = net->fwd_tiled(s.n) || (want_grad && net->bwd_tiled());
     if (needed && !s.prepared) {  // normally built at upload; here only if the kernel choice changed since
         b200::ft_prepare_kernel<<<(2 * s.n + 7) / 8, 256, 0, net->stream>>>(fa, ta);
         LAUNCHED(net);
@@ -525,7 +544,8 @@ int forward_prepare(b200_net* net, Slot& s, bool want_grad) {
 }
 
 int forward_ft_blocks(b200_net* net, Slot& s, int first_block, int last_block) {
-    const bool tiled = net->fwd_tiled();
+    const bool whole = first_block == 0 && last_block == net->nblocks;
+    const bool tiled = whole ? net->fwd_tiled(s.n) : net->fwd_tiled();
     b200::FtArgs fa = ft_args(net, s);
     b200::TileArgs ta = tile_args(net, s, false);
     int grid = 0;
@@ -914,7 +934,6 @@ int b200_net_set_option(b200_net* net, const char* key, int64_t value) {
                               "tiled feature-transformer kernels need ft_block_rows > 0 dividing n_inputs, at most "
                               "about 800 rows per block, and ft_out a multiple of 64");
         if (strcmp(key, "ft_bwd_mode")) net->ft_fwd_mode = (int)value;
-        net->table_dirty = true;  // the gather forward reads the merged table, the tiled one does not keep it fresh
         if (strcmp(key, "ft_fwd_mode")) net->ft_bwd_mode = (int)value;
         return 0;
     }
@@ -1019,7 +1038,7 @@ int b200_net_set_tensor(b200_net* net, const char* name, int kind, const float* 
     if (int rc = set_device(net)) return rc;
     CK(cudaStreamSynchronize(net->stream));
     CK(cudaMemcpy(kind_base(net, kind) + t->off, host, n * sizeof(float), cudaMemcpyHostToDevice));
-    if (kind == B200_KIND_WEIGHT) net->table_dirty = true;
+    if (kind == B200_KIND_WEIGHT) net->weights_moved();
     return 0;
 }
 
@@ -1234,13 +1253,14 @@ static int upload_launch_lists(b200_net* net, Slot& s, int32_t n) {
     const b200_net_desc& d = net->d;
     s.prepared = s.csr_built = false;
     s.n = n;
-    if (net->tiled_ok && (net->fwd_tiled() || net->bwd_tiled())) {
+    const bool backward = net->bwd_tiled() && net->trains;
+    if (net->tiled_ok && (net->fwd_tiled(n) || backward)) {
         b200::FtArgs fa = ft_args(net, s);
         b200::TileArgs ta = tile_args(net, s, true);
         b200::ft_prepare_kernel<<<(2 * n + 7) / 8, 256, 0, net->copy_stream>>>(fa, ta);
         LAUNCHED(net);
         s.prepared = true;
-        if (net->bwd_tiled() && s.n_chunks > 0) {
+        if (backward && s.n_chunks > 0) {
             b200::ft_csr_kernel<<<s.n_chunks, b200::kCsrThreads, b200::ft_csr_smem(d.ft_block_rows, d.nnz, s.chunk_len), net->copy_stream>>>(fa, ta);
             LAUNCHED(net);
             s.csr_built = true;
@@ -1429,7 +1449,8 @@ int b200_forward_begin(b200_net* net, int slot) {
     if (int rc = set_device(net)) return rc;
     Slot& s = net->slots[slot];
     CK(cudaStreamWaitEvent(net->stream, s.ready, 0));
-    if (int rc = refresh_table(net)) return rc;
+    net->trains = true;
+    if (int rc = refresh_table(net, s.n)) return rc;
     if (!net->manual_grad_zero) {
         // every gradient is accumulated with reductions, so the buffer starts at zero; nothing before
         // the dense layers writes to it, so the clearing runs on a side stream beside the FT forward
@@ -1615,7 +1636,7 @@ int b200_update_range(b200_net* net, float lr, float grad_factor, int64_t first_
     const long long blocks = std::min<long long>((a.total4 + 255) / 256, net->sm_count * 16);
     b200::adamw_flat_kernel<<<(unsigned)blocks, 256, 0, net->stream>>>(a);
     LAUNCHED(net);
-    net->table_dirty = true;
+    net->weights_moved();
     return 0;
 }
 
@@ -1745,7 +1766,7 @@ int b200_update_exchange_range(b200_net* net, float lr, float grad_factor, int64
         }
 #undef BULK
         LAUNCHED(net);
-        net->table_dirty = true;
+        net->weights_moved();
         if (first_float == 0) net->loss_in_param = true;
         return 0;
     }
@@ -1756,7 +1777,7 @@ int b200_update_exchange_range(b200_net* net, float lr, float grad_factor, int64
         default: b200::adamw_exchange_kernel<0><<<(unsigned)blocks, 128, 0, on>>>(x); break;
     }
     LAUNCHED(net);
-    net->table_dirty = true;
+    net->weights_moved();
     if (first_float == 0) net->loss_in_param = true;  // the range holds the loss: it now sits in P[0]
     return 0;
 }
@@ -1877,7 +1898,7 @@ int b200_step_exchange(b200_net* net, int slot, float lr, float grad_factor) {
     CK(cudaStreamWaitEvent(net->stream, net->xch_join, 0));
     net->loss_in_param = true;  // every rank reduced the loss into float 0 of its parameter buffer
     net->xch_fenced_used = true;
-    net->table_dirty = true;
+    net->weights_moved();
     return b200_update_end(net);
 }
 
@@ -1929,10 +1950,10 @@ int b200_update_end(b200_net* net) {
         if (any && net->S) {
             b200::lookahead_kernel<<<net->sm_count * 8, 256, 0, net->stream>>>(la);
             LAUNCHED(net);
-            net->table_dirty = true;
+            net->weights_moved();
         }
     }
-    if (int rc = refresh_table(net)) return rc;
+    if (int rc = refresh_table(net, net->last_n)) return rc;
     if (net->step_open) {  // close the timed step begun by the matching backward
         CK(cudaEventRecord(net->tev[net->steps_begun % b200_net::kTimingRing][7], net->stream));
         net->steps_begun++;
@@ -2009,7 +2030,7 @@ int b200_forward(b200_net* net, int slot, float* out_host) {
     if (int rc = set_device(net)) return rc;
     Slot& s = net->slots[slot];
     CK(cudaStreamWaitEvent(net->stream, s.ready, 0));
-    if (int rc = refresh_table(net)) return rc;
+    if (int rc = refresh_table(net, s.n)) return rc;
     if (int rc = forward_part(net, s, false)) return rc;
     CK(cudaEventRecord(s.consumed, net->stream));
     s.has_consumed = true;
