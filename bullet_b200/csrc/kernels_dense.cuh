@@ -13,20 +13,19 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include "kernels_ft.cuh"
+#include "kernels_group.cuh"
 
 namespace b200 {
 
-constexpr int kDenseTile = 32;    // positions of one output bucket handled by one CTA (8 warps)
-constexpr int kDenseWarpPos = 4;  // of which each warp takes four
+constexpr int kDenseWarpPos = 4;  // positions of a tile (kDenseTile of them, 8 warps) that each warp takes
 constexpr int kDenseChunk = 128;  // first-layer columns staged in shared memory per round
 
 struct DenseArgs {
     const float* x;        // [n][K1] dense-stack input
     const int* buckets;    // [n] output bucket per position
     const float* targets;  // [n]
-    const int* order;      // [n] position ids grouped by output bucket
-    const int2* tiles;     // [ntiles] (begin, count <= kDenseTile) ranges of `order`, one bucket each
+    const int* order;      // [n] position ids grouped by output bucket, or null (one bucket): as they come
+    const int2* tiles;     // [ntiles] (begin, count <= kDenseTile) ranges of `order`, one bucket each, or null as well
     int n, ntiles, K1, O, n_dense;
     int M[3], act[3];
     const float* W[3];
@@ -36,6 +35,7 @@ struct DenseArgs {
     float* a2;         // [n][M2]
     float* dz[3];      // gradient at each layer's selected pre-activation: [n][M_i]
     float* out;        // [n] network output
+    float* out_host;   // the same in pinned host memory, or null
     float* loss;       // scalar, accumulated
     int want_grad;
     // the register-tiled forward also forms the weight and bias gradients of the layers after the
@@ -44,6 +44,12 @@ struct DenseArgs {
     float* gW[3];
     float* gB[3];
 };
+
+// tile `i` of a batch of n positions, and the position at place `at` of the order
+__device__ __forceinline__ int2 dense_tile_at(const int2* tiles, int i, int n) {
+    return tiles ? tiles[i] : make_int2(i * kDenseTile, min(kDenseTile, n - i * kDenseTile));
+}
+__device__ __forceinline__ int dense_order_at(const int* order, int at) { return order ? order[at] : at; }
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -138,8 +144,9 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_forward_kernel(D
     __shared__ float loss_part[8];
     __shared__ int s_pos[kDenseTile];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int2 t = a.tiles[blockIdx.x];
-    if (threadIdx.x < kDenseTile) s_pos[threadIdx.x] = a.order[t.x + min((int)threadIdx.x, t.y - 1)];
+    const int2 t = dense_tile_at(a.tiles, blockIdx.x, a.n);
+    if (t.y <= 0) return;  // (the launch is sized from the batch size alone)
+    if (threadIdx.x < kDenseTile) s_pos[threadIdx.x] = dense_order_at(a.order, t.x + min((int)threadIdx.x, t.y - 1));
     __syncthreads();
     const int k = a.buckets[s_pos[0]];
     const int npos = max(0, min(P, t.y - warp * P));
@@ -222,7 +229,10 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_forward_kernel(D
                 o = warp_sum(term) + a.B[2][k];
             }
         }
-        if (lane == 0) a.out[b] = o;
+        if (lane == 0) {
+            a.out[b] = o;
+            if (a.out_host) a.out_host[b] = o;
+        }
         if (!a.want_grad) continue;
 
         const float s = 1.f / (1.f + expf(-o));
@@ -300,8 +310,9 @@ __global__ void __launch_bounds__(256, 2) dense_forward_tile_kernel(DenseArgs a)
     __shared__ int s_pos[kDenseTile];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int rg = lane % RG, pg = lane / RG;
-    const int2 t = a.tiles[blockIdx.x];
-    if (threadIdx.x < kDenseTile) s_pos[threadIdx.x] = a.order[t.x + min((int)threadIdx.x, t.y - 1)];
+    const int2 t = dense_tile_at(a.tiles, blockIdx.x, a.n);
+    if (t.y <= 0) return;  // (the launch is sized from the batch size alone)
+    if (threadIdx.x < kDenseTile) s_pos[threadIdx.x] = dense_order_at(a.order, t.x + min((int)threadIdx.x, t.y - 1));
     __syncthreads();
     const int k = a.buckets[s_pos[0]];
     const int M2 = a.M[1], OM2 = a.O * M2;
@@ -407,7 +418,10 @@ __global__ void __launch_bounds__(256, 2) dense_forward_tile_kernel(DenseArgs a)
             a2v = lane < M2 ? act_fwd(a.act[1], z2) : 0.f;
             o = warp_sum(s_w3[lane] * a2v) + a.B[2][k];
         }
-        if (lane == 0) a.out[b] = o;
+        if (lane == 0) {
+            a.out[b] = o;
+            if (a.out_host) a.out_host[b] = o;
+        }
         if (!a.want_grad) continue;
 
         const float s = 1.f / (1.f + expf(-o));
@@ -477,12 +491,13 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_dx_kernel(DenseA
     constexpr int P = kDenseWarpPos, MP = dense_col_stride<M1>();
     __shared__ __align__(16) float wbuf[2][kDenseChunk * MP];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int2 t = a.tiles[blockIdx.x];
-    const int k = a.buckets[a.order[t.x]];
+    const int2 t = dense_tile_at(a.tiles, blockIdx.x, a.n);
+    if (t.y <= 0) return;
+    const int k = a.buckets[dense_order_at(a.order, t.x)];
     const int npos = max(0, min(P, t.y - warp * P));
     int pos[P];
 #pragma unroll
-    for (int j = 0; j < P; j++) pos[j] = a.order[npos ? t.x + warp * P + min(j, npos - 1) : t.x];
+    for (int j = 0; j < P; j++) pos[j] = dense_order_at(a.order, npos ? t.x + warp * P + min(j, npos - 1) : t.x);
     float g[P][M1];
 #pragma unroll
     for (int j = 0; j < P; j++)
@@ -626,7 +641,7 @@ struct SmallGradArgs {
     const int* order;
     const int2* tiles;
     const int* buckets;
-    int O, n_layers;     // layers handled here: dense layers 1 .. n_dense-1
+    int n, O, n_layers;  // layers handled here: dense layers 1 .. n_dense-1
     int K[2], M[2];
     const float* X[2];   // [n][K]
     const float* dY[2];  // [n][M]
@@ -637,8 +652,9 @@ struct SmallGradArgs {
 static __global__ void __launch_bounds__(256) dense_small_grads_kernel(SmallGradArgs a) {
     __shared__ float s_x[32][33], s_dy[32][33];
     __shared__ int s_pos[32];
-    const int2 t = a.tiles[blockIdx.x];
-    if (threadIdx.x < t.y) s_pos[threadIdx.x] = a.order[t.x + threadIdx.x];
+    const int2 t = dense_tile_at(a.tiles, blockIdx.x, a.n);
+    if (t.y <= 0) return;
+    if (threadIdx.x < t.y) s_pos[threadIdx.x] = dense_order_at(a.order, t.x + threadIdx.x);
     __syncthreads();
     const int k = a.buckets[s_pos[0]];
     for (int l = 0; l < a.n_layers; l++) {

@@ -31,6 +31,16 @@ namespace b200 {
 constexpr uint32_t kNoFeature = 0xFFFFu;
 constexpr int kStatusOutsideBlock = 1;  // a feature fell outside its position's declared row block
 
+// A kernel's largest dynamic shared memory holds for the process, whatever network asks: always all there is.
+template <class K>
+cudaError_t allow_smem(K* kernel) {
+    cudaFuncAttributes attr;
+    const cudaError_t e = cudaFuncGetAttributes(&attr, reinterpret_cast<const void*>(kernel));
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(reinterpret_cast<const void*>(kernel), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)(227 * 1024 - attr.sharedSizeBytes));
+}
+
 struct FtArgs {
     const float* table;   // [n_inputs][H] effective weights: l0w, or l0w + tiled l0f already merged
     const float* factor;  // forward only: [factor_rows][H] l0f to be added to `table` (= l0w) on the fly, or null
@@ -56,19 +66,18 @@ struct TileArgs {
     // contiguous pieces of that line: every SM gets the same amount of work whatever the blocks hold, and
     // a tile is loaded about once per (block, slab) and SM that touches it.
     int first_block, last_block;
-    const int* pair_order;   // [2n] pair ids (position*2 + perspective) grouped by block, or null = identity
-    const int* block_begin;  // [nblocks+1] offsets into pair_order
+    const int2* pairs;       // [2n] (pair id = position*2 + perspective, number of active rows) grouped by block
+    const int* block_begin;  // [nblocks+1] offsets into pairs
     const int* chunk_begin;  // backward: [nblocks+1] first chunk of every block
     int* status;
-    // written by ft_prepare_kernel, read by the tiled kernels: for the i-th pair in visiting
+    // written by the grouping (kernels_group.cuh): for the i-th pair in visiting
     // order its active rows (local to the pair's block) in slot order; the tail of the last
     // 16-byte group is filled with the index of the all-zero row (= block_rows) and never walked
-    uint16_t* lists;  // [2n][list_len]
-    int* list_count;  // [2n] number of active rows
+    const uint16_t* lists;  // [2n][list_len]
     int list_len;     // nnz rounded up to a multiple of 8 (16-byte groups)
     // backward only: the visiting order cut into chunks of at most ft_bwd_chunk pairs that never
     // straddle a block, and per chunk the row-major lists built by ft_csr_kernel
-    const int4* chunks;            // [nchunks] (block, first index into pair_order, pairs, 0)
+    const int4* chunks;            // [nchunks] (block, first index into `pairs`, pairs, 0)
     uint16_t* csr_ent;             // [nchunks][ent_cap] pairs of the chunk grouped by row, every list starting on 16 bytes
     int* csr_start;                // [nchunks][start_cap] per row (start / 8) << 16 | length; [R] = entries in all
     int ent_cap, start_cap;
@@ -323,42 +332,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-__device__ __forceinline__ const uint16_t* pair_list(const FtArgs& a, int pair) {
-    return ((pair & 1) ? a.idx_nstm : a.idx_stm) + (size_t)(pair >> 1) * a.nnz;
-}
-
-// Per batch, once: turns every (position, perspective) pair's slots into the list the tiled
-// kernels walk — rows local to the pair's block, compacted in slot order, the last 16-byte
-// group filled up with the index of the all-zero row.  A valid feature outside the block raises
-// the status bit and is dropped.  One warp per pair, in visiting order.  grid = ceil(2n / 8), block = 256.
-static __global__ void __launch_bounds__(256) ft_prepare_kernel(FtArgs a, TileArgs t) {
-    const int lane = threadIdx.x & 31;
-    const int i = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (i >= 2 * a.n) return;
-    const int pair = t.pair_order ? t.pair_order[i] : i;
-    uint32_t slot0, slot1;
-    load_slots(pair_list(a, pair), a.nnz, lane, slot0, slot1);
-    const bool v0 = slot0 < (uint32_t)a.n_inputs, v1 = slot1 < (uint32_t)a.n_inputs;
-    // the block of a pair is the block of its first valid feature (as the grouping defines it)
-    const unsigned mv0 = __ballot_sync(0xffffffffu, v0), mv1 = __ballot_sync(0xffffffffu, v1);
-    int block = 0;
-    if (mv0)
-        block = (int)__shfl_sync(0xffffffffu, slot0, __ffs(mv0) - 1) / t.block_rows;
-    else if (mv1)
-        block = (int)__shfl_sync(0xffffffffu, slot1, __ffs(mv1) - 1) / t.block_rows;
-    const int row0 = (int)slot0 - block * t.block_rows, row1 = (int)slot1 - block * t.block_rows;
-    const bool in0 = v0 && (unsigned)row0 < (unsigned)t.block_rows, in1 = v1 && (unsigned)row1 < (unsigned)t.block_rows;
-    if ((v0 && !in0) || (v1 && !in1)) atomicOr(t.status, kStatusOutsideBlock);
-    const unsigned m0 = __ballot_sync(0xffffffffu, in0), m1 = __ballot_sync(0xffffffffu, in1);
-    const unsigned lt = (1u << lane) - 1u;
-    const int cnt0 = __popc(m0), cnt = cnt0 + __popc(m1), cnt8 = (cnt + 7) & ~7;
-    uint16_t* list = t.lists + (size_t)i * t.list_len;
-    if (in0) list[__popc(m0 & lt)] = (uint16_t)row0;
-    if (in1) list[cnt0 + __popc(m1 & lt)] = (uint16_t)row1;
-    if (lane < cnt8 - cnt) list[cnt + lane] = (uint16_t)t.block_rows;
-    if (lane == 0) t.list_count[i] = cnt;
-}
-
 // One 256-byte line of shared memory (a tile row, or a staged gradient line), this lane's 8 bytes of it.
 __device__ __forceinline__ f32x2 line_at(const unsigned char* mine, uint32_t index) {
     return *reinterpret_cast<const f32x2*>(mine + index * kTileRowBytes);
@@ -459,20 +432,18 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
         uint32_t* ring = reinterpret_cast<uint32_t*>(smem_raw + (size_t)(R + 1) * kTileRowBytes) + warp * list_words;
         const uint32_t* lists_w = reinterpret_cast<const uint32_t*>(t.lists);
         int i = t.block_begin[block] + first + warp;
-        int pair = 0, cnt = 0;
+        int2 pc = make_int2(0, 0);
         uint32_t word = 0;
         if (i < seg_end) {
-            pair = t.pair_order ? t.pair_order[i] : i;
-            cnt = t.list_count[i];
+            pc = __ldg(t.pairs + i);
             if (lane < list_words) word = __ldg(lists_w + (size_t)i * list_words + lane);
         }
         for (; i < seg_end; i += NW) {
-            int pair_next = 0, cnt_next = 0;
+            const int pair = pc.x, cnt = pc.y;
             __syncwarp();  // every lane has finished with the list of the pair before
             if (lane < list_words) ring[lane] = word;
             if (i + NW < seg_end) {
-                pair_next = t.pair_order ? t.pair_order[i + NW] : i + NW;
-                cnt_next = t.list_count[i + NW];
+                pc = __ldg(t.pairs + i + NW);
                 if (lane < list_words) word = __ldg(lists_w + (size_t)(i + NW) * list_words + lane);
             }
             __syncwarp();
@@ -497,8 +468,6 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
                 *reinterpret_cast<float2*>(x_out + (size_t)pair * x_row) =
                     make_float2(ft_act_fwd(a.act, lo2(acc)), ft_act_fwd(a.act, hi2(acc)));
             }
-            pair = pair_next;
-            cnt = cnt_next;
         }
     }
 }
@@ -535,12 +504,13 @@ __host__ __device__ inline size_t ft_csr_smem(int R, int nnz, int cp) {
     return (size_t)ft_bwd_ent_cap(R, nnz, cp) * 2 + (size_t)(2 * (R + 2) + 32 + cp) * 4;
 }
 
-// grid = number of chunks, block = kCsrThreads.
+// grid = most chunks there can be, block = kCsrThreads.
 static __global__ void __launch_bounds__(kCsrThreads) ft_csr_kernel(FtArgs a, TileArgs t) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int NW = kCsrThreads / 32;
     const int4 chunk = t.chunks[blockIdx.x];
+    if (chunk.z == 0) return;  // (the launch is sized from the batch size alone)
     const int R = t.block_rows, CP = t.chunk_len, L = t.list_len, c0 = chunk.y, cn = chunk.z;
     uint16_t* ent = reinterpret_cast<uint16_t*>(smem_raw);
     int* start = reinterpret_cast<int*>(ent + t.ent_cap);  // [R + 1]
@@ -549,7 +519,7 @@ static __global__ void __launch_bounds__(kCsrThreads) ft_csr_kernel(FtArgs a, Ti
     int* count_s = warp_tot + 32;                                        // [CP] prepared list lengths
     const int zero_row = R;
     for (int r = threadIdx.x; r < R; r += kCsrThreads) cursor[r] = 0;
-    for (int k = threadIdx.x; k < cn; k += kCsrThreads) count_s[k] = t.list_count[c0 + k];
+    for (int k = threadIdx.x; k < cn; k += kCsrThreads) count_s[k] = t.pairs[c0 + k].y;
     __syncthreads();
     // count how often each row occurs in the chunk: a warp per pair, a lane per list entry,
     // four pairs in flight
@@ -717,7 +687,7 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
             const int total = __ldg(start_in + R);
             const uint16_t* ent_in = t.csr_ent + (size_t)ch * t.ent_cap;
             for (int i = threadIdx.x; i < (total + 7) / 8; i += kBwdThreads) cp_async16(ent + 8 * i, ent_in + 8 * i);
-            for (int k = threadIdx.x; k < cn; k += kBwdThreads) pairs_s[k] = t.pair_order ? t.pair_order[c0 + k] : c0 + k;
+            for (int k = threadIdx.x; k < cn; k += kBwdThreads) pairs_s[k] = __ldg(t.pairs + c0 + k).x;
             ch_loaded = ch;
             __syncthreads();  // the pair ids (and, on the first unit, the zeroed lines) are in place
         }

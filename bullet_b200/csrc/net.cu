@@ -33,6 +33,7 @@
 #include "kernels_opt.cuh"
 #include "kernels_prep.cuh"
 #include "host_map.h"
+#include "op_pool.h"
 
 #define CK(call)                                                                                          \
     do {                                                                                                  \
@@ -53,6 +54,7 @@ namespace {
 
 constexpr int64_t kAlignFloats = 64;       // 256-byte tensor alignment in the flat buffers
 constexpr int kGatherRowsPerPosition = 34;  // active features of both perspectives of a middling chess position
+constexpr int kDirectOutputs = 256;        // up to as many outputs of an evaluation the kernel stores to pinned memory itself
 constexpr int kMinItemPairs = 128;         // a forward work item serves at least this many pairs per tile load
 
 struct Tensor {
@@ -71,27 +73,19 @@ struct Slot {
     char* h_blob = nullptr;
     size_t capacity = 0;
     int n = 0;
-    int n_dtiles = 0;  // CTA tiles of the dense kernels held in off_dtiles
-    int n_chunks = 0, chunk_len = 0;  // chunks of the tiled FT backward held in off_chunks, and their size
-    std::vector<int> block_begin;     // [nblocks + 1] host copy: first pair (in visiting order) of every block
-    std::vector<int> chunk_begin;     // [nblocks + 1] host copy: first chunk of every block
+    int n_dtiles = 0;  // CTA tiles of the dense kernels: as many as there can be, the rest are empty
+    int n_chunks = 0, chunk_len = 0;  // the same for the chunks of the tiled FT backward held in off_chunks, and their size
     int expect_grid = 0;              // grid size the per-block CTA counts in off_bexpect were made for
-    // device-side batch preparation (b200_batch_upload_records_gpu): raw records, scratch, totals read-back
-    uint4* d_records = nullptr;
-    uint16_t* d_pair_block = nullptr;
-    int* d_cta_hist = nullptr;
-    int* d_totals = nullptr;
-    int* h_totals = nullptr;          // pinned: bin totals, bin bases, then the status word
-    cudaEvent_t totals_ready = nullptr;
     // derived from the indices alone, so built once per upload on the copy stream (or on first use):
     uint16_t* lists = nullptr;        // prepared per-pair row lists of the tiled kernels
-    int* list_count = nullptr;
     uint16_t* csr_ent = nullptr;      // per-chunk row-major lists of the tiled backward
     int* csr_start = nullptr;
     bool prepared = false, csr_built = false;
-    size_t off_status = 0;            // one int in the blob, zero on upload: bits raised by ft_prepare_kernel
-    size_t off_stm = 0, off_nstm = 0, off_buckets = 0, off_targets = 0, off_order = 0, off_pairs = 0, off_blocks = 0,
-           off_dtiles = 0, off_chunks = 0, off_cbegin = 0, off_bexpect = 0, bytes = 0;
+    // what crosses PCIe comes first: either the packed lists, buckets, targets and (if the host made them) the dense
+    // kernels' order and tiles, or the raw records; everything behind is written on the device
+    size_t off_stm = 0, off_nstm = 0, off_buckets = 0, off_targets = 0, off_order = 0, off_dtiles = 0, off_records = 0, off_pairs = 0,
+           off_blocks = 0, off_chunks = 0, off_cbegin = 0, off_bexpect = 0, off_status = 0, off_info = 0, off_hist = 0, bytes = 0;
+    size_t off_many[3] = {0, 0, 0};   // counters of the grouping by more row blocks than its windows hold
     cudaEvent_t ready = nullptr, consumed = nullptr;
     bool has_ready = false, has_consumed = false;
     template <class T>
@@ -126,6 +120,7 @@ struct b200_net {
     int* h_status = nullptr;
     int* d_status = nullptr;       // [kLossRing] the slot's status word, saved before the slot is released to the uploader
     float* h_loss = nullptr;
+    float* h_out = nullptr;        // pinned [max_batch]: network outputs of an evaluation
     cudaEvent_t loss_ev[kLossRing] = {};
     int64_t updates = 0;
     Slot slots[B200_NUM_SLOTS];
@@ -253,7 +248,11 @@ int set_device(const b200_net* net) {
 template <class T>
 int dev_alloc(b200_net* net, T** p, size_t count) {
     void* raw = nullptr;
-    CK(cudaMalloc(&raw, std::max<size_t>(count, 1) * sizeof(T)));
+    if (cudaMalloc(&raw, std::max<size_t>(count, 1) * sizeof(T)) != cudaSuccess) {  // once more without what the operator's pool keeps
+        cudaGetLastError();
+        b200::op_pool_trim(net->device);
+        CK(cudaMalloc(&raw, std::max<size_t>(count, 1) * sizeof(T)));
+    }
     net->allocations.push_back(raw);
     *p = static_cast<T*>(raw);
     return 0;
@@ -294,18 +293,26 @@ void slot_layout(const b200_net* net, Slot& s, int n) {
         off = align_up(off + bytes, 256);
         return at;
     };
+    const size_t nb = net->nblocks, O = d.n_out_buckets, bins = nb + O;
+    const bool many = net->nblocks > b200::kGroupMaxBlocks;
     s.off_stm = take((size_t)n * d.nnz * 2);
     s.off_nstm = take((size_t)n * d.nnz * 2);
     s.off_buckets = take((size_t)n * 4);
     s.off_targets = take((size_t)n * 4);
     s.off_order = take((size_t)n * 4);
-    s.off_pairs = take((size_t)n * 8);
-    s.off_blocks = take((size_t)(net->nblocks + 1) * 4);
-    s.off_dtiles = take(((size_t)n / b200::kDenseTile + d.n_out_buckets + 1) * 8);
-    s.off_chunks = take(((size_t)2 * n / b200::ft_bwd_chunk(d.nnz, false) + net->nblocks + 1) * 16);
-    s.off_cbegin = take((size_t)(net->nblocks + 1) * 4);
-    s.off_bexpect = take((size_t)net->nblocks * 4);
+    s.off_dtiles = take(((size_t)n / b200::kDenseTile + O + 1) * 8);
+    s.off_records = take((size_t)n * 32);
+    s.off_pairs = take((size_t)n * 16);
+    s.off_blocks = take((nb + 1) * 4);
+    s.off_chunks = take(((size_t)2 * n / b200::ft_bwd_chunk(d.nnz, false) + nb + 1) * 16);
+    s.off_cbegin = take((nb + 1) * 4);
+    s.off_bexpect = take(nb * 4);
     s.off_status = take(4);
+    s.off_info = take((size_t)n * 8);
+    s.off_hist = take(many ? 4 : (size_t)b200::group_ctas(n) * bins * 4);
+    s.off_many[0] = take(many ? bins * 4 : 4);
+    s.off_many[1] = take(many ? (bins + 2) * 4 : 4);
+    s.off_many[2] = take(many ? (bins + 1) * 4 : 4);
     s.bytes = off;
 }
 
@@ -387,14 +394,17 @@ cudaError_t set_dense_forward_smem() {
                                 (int)b200::dense_fwd_smem<MM>());
 }
 
-// Grid of the tiled kernels for the row blocks [first, last): one CTA per SM (two for the 512-thread
-// backward), fewer when there is too little work to give every CTA a worthwhile piece.
-int ft_forward_grid(const b200_net* net, const Slot& s, int first, int last) {
-    const long long line = (long long)net->nslabs * (s.block_begin[last] - s.block_begin[first]);
+// Most chunks that a batch of n positions can be cut into: every block may end in a partly filled one.
+int most_chunks(const b200_net* net, int n, int chunk_len) { return std::min(2 * n, 2 * n / chunk_len + net->nblocks); }
+
+// Grid of the tiled kernels: one CTA per SM (two for the 512-thread backward), fewer when there is too little work to give
+// every CTA a worthwhile piece.  What a run of row blocks holds is known on the device only: a CTA without work returns.
+int ft_forward_grid(const b200_net* net, const Slot& s) {
+    const long long line = (long long)net->nslabs * 2 * s.n;
     return (int)std::max<long long>(1, std::min<long long>(net->sm_count, line / kMinItemPairs));
 }
-int ft_backward_grid(const b200_net* net, const Slot& s, int first, int last, bool beside_exchange) {
-    const long long units = (long long)net->nslabs * (s.chunk_begin[last] - s.chunk_begin[first]);
+int ft_backward_grid(const b200_net* net, const Slot& s, bool beside_exchange) {
+    const long long units = (long long)net->nslabs * s.n_chunks;
     const int per_sm = s.chunk_len > b200::ft_bwd_chunk(net->d.nnz, false) ? 1 : 2;
     const int sms = net->sm_count - (beside_exchange ? std::min(net->overlap_ctas, net->sm_count - 1) : 0);
     return (int)std::max<long long>(1, std::min<long long>((long long)sms * per_sm, units));
@@ -433,11 +443,10 @@ b200::TileArgs tile_args(b200_net* net, const Slot& s, bool backward) {
     t.first_block = 0;
     t.last_block = net->nblocks;
     t.chunk_begin = s.dev<int>(s.off_cbegin);
-    t.pair_order = net->nblocks > 1 ? s.dev<int>(s.off_pairs) : nullptr;
+    t.pairs = s.dev<int2>(s.off_pairs);
     t.block_begin = s.dev<int>(s.off_blocks);
     t.status = s.dev<int>(s.off_status);
     t.lists = s.lists;
-    t.list_count = s.list_count;
     t.list_len = (net->d.nnz + 7) & ~7;
     t.chunks = s.dev<int4>(s.off_chunks);
     t.csr_ent = s.csr_ent;
@@ -478,13 +487,14 @@ b200::DenseArgs dense_args(b200_net* net, const Slot& s, bool want_grad) {
         a.B[l] = net->P + net->find(name)->off;
         a.dz[l] = net->dz[l];
     }
-    a.order = s.dev<int>(s.off_order);
-    a.tiles = s.dev<int2>(s.off_dtiles);
+    a.order = d.n_out_buckets > 1 ? s.dev<int>(s.off_order) : nullptr;
+    a.tiles = d.n_out_buckets > 1 ? s.dev<int2>(s.off_dtiles) : nullptr;
     a.ntiles = s.n_dtiles;
     a.W1g = net->w1g;
     a.a1 = net->a1;
     a.a2 = net->a2;
     a.out = net->out;
+    a.out_host = !want_grad && s.n <= kDirectOutputs ? net->h_out : nullptr;
     a.loss = net->G;
     a.want_grad = want_grad ? 1 : 0;
     a.fuse_small = want_grad && net->fused_small_grads() ? 1 : 0;
@@ -527,16 +537,97 @@ int check_slot(b200_net* net, int slot, const char* who) {
     return 0;
 }
 
+b200::GroupArgs group_args(b200_net* net, Slot& s, bool want_lists, bool want_order) {
+    const b200_net_desc& d = net->d;
+    b200::GroupArgs g{};
+    g.stm = s.dev<uint16_t>(s.off_stm);
+    g.nstm = s.dev<uint16_t>(s.off_nstm);
+    g.buckets = s.dev<int>(s.off_buckets);
+    g.n = s.n;
+    g.nnz = d.nnz;
+    g.n_inputs = d.n_inputs;
+    g.block_rows = net->tiled_ok ? d.ft_block_rows : d.n_inputs;
+    g.nblocks = net->nblocks;
+    g.n_out_buckets = d.n_out_buckets;
+    g.info = s.dev<int>(s.off_info);
+    g.hist = s.dev<int>(s.off_hist);
+    g.status = s.dev<int>(s.off_status);
+    g.clear_status = 1;
+    g.want_lists = want_lists;
+    g.nslabs = net->nslabs;
+    if (want_lists) {
+        g.pairs = s.dev<int2>(s.off_pairs);
+        g.lists = s.lists;
+        g.list_len = (d.nnz + 7) & ~7;
+        g.block_begin = s.dev<int>(s.off_blocks);
+        g.chunks = s.dev<int4>(s.off_chunks);
+        g.chunk_begin = s.dev<int>(s.off_cbegin);
+        g.max_chunks = s.n_chunks;
+        g.chunk_len = s.chunk_len;
+        g.expect = s.dev<int>(s.off_bexpect);
+        g.expect_grid = s.expect_grid;
+    }
+    if (want_order) {
+        g.order = s.dev<int>(s.off_order);
+        g.tiles = s.dev<int2>(s.off_dtiles);
+        g.max_tiles = s.n_dtiles;
+    }
+    return g;
+}
+
+// How the slot's batch is cut; the device fills the tables in.  The dense kernels' tiles at upload, what the tiled kernels
+// take whenever their lists are built.
+void cut_dense(b200_net* net, Slot& s) {
+    const int O = net->d.n_out_buckets;
+    s.n_dtiles = O > 1 ? s.n / b200::kDenseTile + std::min(O, s.n) : (s.n + b200::kDenseTile - 1) / b200::kDenseTile;
+}
+void cut_ft(b200_net* net, Slot& s) {
+    if (!net->tiled_ok) return;
+    s.chunk_len = net->bwd_chunk(s.n);
+    s.n_chunks = most_chunks(net, s.n, s.chunk_len);
+    s.expect_grid = ft_backward_grid(net, s, net->overlap_mode);
+}
+
+// Groups the slot's batch on `stream` (kernels_group.cuh); `counted`: the first pass has run with the featuriser.
+int group_slot(b200_net* net, Slot& s, const b200::GroupArgs& g, bool counted, cudaStream_t stream) {
+    if (g.nblocks > b200::kGroupMaxBlocks) {
+        int *count = s.dev<int>(s.off_many[0]), *at = s.dev<int>(s.off_many[1]), *scratch = s.dev<int>(s.off_many[2]);
+        const int pairs = (2 * g.n + 7) / 8;
+        CK(cudaMemsetAsync(count, 0, (size_t)(g.nblocks + g.n_out_buckets) * sizeof(int), stream));
+        b200::group_many_count_kernel<<<pairs, 256, 0, stream>>>(g, count);
+        LAUNCHED(net);
+        b200::group_many_scan_kernel<<<1, 1024, 0, stream>>>(g, count, at, scratch);
+        LAUNCHED(net);
+        b200::group_many_place_kernel<<<pairs, 256, 0, stream>>>(g, count);
+        LAUNCHED(net);
+    } else {
+        const bool vec = b200::group_vec(g);
+        if (!counted) {
+            b200::group_lists_kernel<<<b200::group_ctas(g.n), b200::kGroupThreads, 0, stream>>>(g, vec);
+            LAUNCHED(net);
+        }
+        b200::group_place_kernel<<<b200::group_windows(g.n), b200::kPlaceThreads, 0, stream>>>(g, vec);
+        LAUNCHED(net);
+    }
+    if (g.want_lists) s.prepared = true;
+    return 0;
+}
+
+int build_csr(b200_net* net, Slot& s, cudaStream_t stream) {
+    b200::ft_csr_kernel<<<s.n_chunks, b200::kCsrThreads, b200::ft_csr_smem(net->d.ft_block_rows, net->d.nnz, s.chunk_len), stream>>>(
+        ft_args(net, s), tile_args(net, s, true));
+    LAUNCHED(net);
+    s.csr_built = true;
+    return 0;
+}
+
 // The forward pass in three pieces: the per-pair row lists, the feature-transformer items of a
 // run of work items, and the dense layers.
 int forward_prepare(b200_net* net, Slot& s, bool want_grad) {
-    b200::FtArgs fa = ft_args(net, s);
-    b200::TileArgs ta = tile_args(net, s, false);
     const bool needed = net->fwd_tiled(s.n) || (want_grad && net->bwd_tiled());
-    if (needed && !s.prepared) {  // normally built at upload; here only if the kernel choice changed since
-        b200::ft_prepare_kernel<<<(2 * s.n + 7) / 8, 256, 0, net->stream>>>(fa, ta);
-        LAUNCHED(net);
-        s.prepared = true;
+    if (needed && !s.prepared) {  // normally built at upload; here on the first training pass or after a change of kernels
+        cut_ft(net, s);
+        if (int rc = group_slot(net, s, group_args(net, s, true, false), false, net->stream)) return rc;
     }
     if (want_grad) net->status_slot = needed ? (int)(&s - net->slots) : -1;
     if (want_grad) CK(cudaEventRecord(net->tev[net->steps_begun % b200_net::kTimingRing][0], net->stream));
@@ -550,10 +641,9 @@ int forward_ft_blocks(b200_net* net, Slot& s, int first_block, int last_block) {
     b200::TileArgs ta = tile_args(net, s, false);
     int grid = 0;
     if (tiled) {
-        if (s.block_begin[last_block] == s.block_begin[first_block]) return 0;  // no position in these blocks
         ta.first_block = first_block;
         ta.last_block = last_block;
-        grid = ft_forward_grid(net, s, first_block, last_block);
+        grid = ft_forward_grid(net, s);
     }
     return net->d.pairwise ? launch_ft_forward<true>(net, fa, ta, tiled, grid) : launch_ft_forward<false>(net, fa, ta, tiled, grid);
 }
@@ -619,9 +709,10 @@ int launch_dense_grads(b200_net* net, Slot& s) {
     const b200_net_desc& d = net->d;
     if (net->d.n_dense > 1 && !net->fused_small_grads()) {  // the narrow layers' weight and bias gradients, one launch
         b200::SmallGradArgs g{};
-        g.order = s.dev<int>(s.off_order);
-        g.tiles = s.dev<int2>(s.off_dtiles);
+        g.order = d.n_out_buckets > 1 ? s.dev<int>(s.off_order) : nullptr;
+        g.tiles = d.n_out_buckets > 1 ? s.dev<int2>(s.off_dtiles) : nullptr;
         g.buckets = s.dev<int>(s.off_buckets);
+        g.n = s.n;
         g.O = d.n_out_buckets;
         g.n_layers = d.n_dense - 1;
         for (int l = 1; l < d.n_dense; l++) {
@@ -670,7 +761,7 @@ int preload_kernels(b200_net* net) {
     ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 512, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, true>);
     ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, false>);
     ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 512, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, false>);
-    ok = ok && load_kernel(b200::ft_prepare_kernel) && load_kernel(b200::ft_csr_kernel);
+    ok = ok && load_kernel(b200::ft_csr_kernel);
     ok = ok && load_kernel(b200::factoriser_merge_kernel) && load_kernel(b200::factoriser_grad_kernel);
     ok = ok && load_kernel(b200::adamw_flat_kernel) && load_kernel(b200::lookahead_kernel);
     ok = ok && load_kernel(b200::adamw_exchange_kernel<0>) && load_kernel(b200::adamw_exchange_kernel<2>);
@@ -681,7 +772,8 @@ int preload_kernels(b200_net* net) {
     ok = ok && load_kernel(b200::adamw_exchange_bulk_kernel<0, 128, 6>);
     ok = ok && load_kernel(b200::adamw_exchange_overlap_kernel<0>) && load_kernel(b200::adamw_exchange_overlap_kernel<2>);
     ok = ok && load_kernel(b200::adamw_exchange_overlap_kernel<4>) && load_kernel(b200::adamw_exchange_overlap_kernel<8>);
-    ok = ok && load_kernel(b200::prep_featurise_kernel) && load_kernel(b200::prep_scan_kernel) && load_kernel(b200::prep_scatter_kernel);
+    ok = ok && load_kernel(b200::prep_featurise_kernel) && load_kernel(b200::group_lists_kernel) && load_kernel(b200::group_place_kernel);
+    ok = ok && load_kernel(b200::group_many_count_kernel) && load_kernel(b200::group_many_scan_kernel) && load_kernel(b200::group_many_place_kernel);
     ok = ok && load_kernel(b200::peer_signal_kernel) && load_kernel(b200::peer_wait_kernel) && load_kernel(b200::bucket_presignal_kernel);
     if (!ok) return b200::fail(B200_ERR_CUDA, "net_create: loading the kernels failed: %s", cudaGetErrorString(cudaGetLastError()));
     return 0;
@@ -791,6 +883,8 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     // the fence counters get an allocation of their own size class (2 MiB), so that its IPC handle maps exactly it
     rc = rc ? rc : dev_alloc(net, &net->xch_flags, (size_t)(2 << 20) / sizeof(int));
     if (!rc) cudaMemsetAsync(net->xch_flags, 0, (size_t)2 << 20, net->stream);
+    rc = rc ? rc : dev_alloc(net, &net->d_win_rate, 65536);
+    rc = rc ? rc : dev_alloc(net, &net->d_expanded, 64);
     rc = rc ? rc : dev_alloc(net, &net->d_peers, 1);
     rc = rc ? rc : dev_alloc(net, &net->done_count, (size_t)net->nblocks);
     if (!rc) cudaMemsetAsync(net->done_count, 0, (size_t)net->nblocks * sizeof(int), net->stream);
@@ -798,18 +892,17 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
         rc = rc ? rc : dev_alloc(net, &net->facc, (size_t)d.ft_block_rows * d.ft_out / 2);
     if (net->tiled_ok) {
         // sized for whichever backward shape needs more: every block may end in a partly filled chunk
-        size_t ent_total = 0, max_chunks = 0;
+        size_t ent_total = 0, chunks_total = 0;
         for (int shape = 0; shape < 3; shape++) {
             const int cp = shape == 2 ? net->wide_chunk : b200::ft_bwd_chunk(d.nnz, shape != 0);
-            const size_t chunks = 2 * B / cp + net->nblocks + 1;
-            max_chunks = std::max(max_chunks, chunks);
+            const size_t chunks = most_chunks(net, (int)B, cp);
+            chunks_total = std::max(chunks_total, chunks);
             ent_total = std::max(ent_total, chunks * b200::ft_bwd_ent_cap(d.ft_block_rows, d.nnz, cp));
         }
         for (auto& s : net->slots) {
             rc = rc ? rc : dev_alloc(net, &s.lists, 2 * B * ((d.nnz + 7) & ~7));
-            rc = rc ? rc : dev_alloc(net, &s.list_count, 2 * B);
             rc = rc ? rc : dev_alloc(net, &s.csr_ent, ent_total);
-            rc = rc ? rc : dev_alloc(net, &s.csr_start, max_chunks * b200::ft_bwd_start_cap(d.ft_block_rows));
+            rc = rc ? rc : dev_alloc(net, &s.csr_start, chunks_total * b200::ft_bwd_start_cap(d.ft_block_rows));
         }
     }
     if (rc) return bail(rc);
@@ -825,7 +918,7 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
         void* raw = nullptr;
         if (cudaMalloc(&raw, s.capacity) != cudaSuccess) return bail(b200::fail(B200_ERR_CUDA, "net_create: slot allocation failed"));
         s.d_blob = static_cast<char*>(raw);
-        if (cudaHostAlloc(&raw, s.capacity, cudaHostAllocDefault) != cudaSuccess)
+        if (cudaHostAlloc(&raw, std::max(s.off_records, (size_t)d.max_batch * 32), cudaHostAllocDefault) != cudaSuccess)
             return bail(b200::fail(B200_ERR_CUDA, "net_create: pinned slot allocation failed"));
         s.h_blob = static_cast<char*>(raw);
         cudaEventCreateWithFlags(&s.ready, cudaEventDisableTiming);
@@ -835,6 +928,8 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     void* raw = nullptr;
     if (cudaHostAlloc(&raw, 128, cudaHostAllocDefault) != cudaSuccess) return bail(b200::fail(B200_ERR_CUDA, "net_create: pinned alloc failed"));
     net->h_loss = static_cast<float*>(raw);
+    if (cudaHostAlloc(&raw, B * sizeof(float), cudaHostAllocDefault) != cudaSuccess) return bail(b200::fail(B200_ERR_CUDA, "net_create: pinned alloc failed"));
+    net->h_out = static_cast<float*>(raw);
     net->h_status = reinterpret_cast<int*>(net->h_loss + 8);
     net->h_xstatus = net->h_status + b200_net::kLossRing;
     memset(net->h_loss, 0, 128);  // 8 floats, 4 status words, 4 x 4 fence words
@@ -854,21 +949,18 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
         if (int rc2 = set_dense(d.dense_out[0])) return bail(rc2);
     }
     if (net->tiled_ok) {
-        const int fs = (int)b200::ft_fwd_smem(d.ft_block_rows, (d.nnz + 7) & ~7);
-        const int wide = net->wide_chunk, narrow = b200::ft_bwd_chunk(d.nnz, false);
-        const int bs = (int)b200::ft_bwd_smem(d.ft_block_rows, d.nnz, wide, net->nslabs), bn = (int)b200::ft_bwd_smem(d.ft_block_rows, d.nnz, narrow, net->nslabs);
-        cudaFuncSetAttribute(b200::ft_forward_tiled_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, fs);
-        cudaFuncSetAttribute(b200::ft_forward_tiled_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, fs);
-        cudaFuncSetAttribute(b200::ft_backward_tiled_kernel<true, 1024, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bs);
-        cudaFuncSetAttribute(b200::ft_backward_tiled_kernel<false, 1024, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bs);
-        cudaFuncSetAttribute(b200::ft_backward_tiled_kernel<true, 512, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bn);
-        cudaFuncSetAttribute(b200::ft_backward_tiled_kernel<false, 512, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, bn);
-        cudaFuncSetAttribute(b200::ft_backward_tiled_kernel<true, 1024, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bs);
-        cudaFuncSetAttribute(b200::ft_backward_tiled_kernel<false, 1024, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bs);
-        cudaFuncSetAttribute(b200::ft_backward_tiled_kernel<true, 512, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bn);
-        cudaFuncSetAttribute(b200::ft_backward_tiled_kernel<false, 512, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, bn);
-        cudaFuncSetAttribute(b200::ft_csr_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)b200::ft_csr_smem(d.ft_block_rows, d.nnz, wide));
+        cudaError_t e = b200::allow_smem(b200::ft_forward_tiled_kernel<true>);
+        e = e ? e : b200::allow_smem(b200::ft_forward_tiled_kernel<false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 1024, true>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 1024, true>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 512, true>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, true>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 1024, false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 1024, false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 512, false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, false>);
+        e = e ? e : b200::allow_smem(b200::ft_csr_kernel);
+        if (e != cudaSuccess) return bail(b200::fail(B200_ERR_CUDA, "net_create: shared memory of the tiled kernels: %s", cudaGetErrorString(e)));
     }
     cudaFuncSetAttribute(b200::adamw_exchange_overlap_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b200::kOverlapSmem);
     cudaFuncSetAttribute(b200::adamw_exchange_overlap_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, b200::kOverlapSmem);
@@ -898,16 +990,11 @@ int b200_net_destroy(b200_net* net) {
     for (auto& s : net->slots) {
         if (s.d_blob) cudaFree(s.d_blob);
         if (s.h_blob) cudaFreeHost(s.h_blob);
-        if (s.d_records) cudaFree(s.d_records);
-        if (s.d_pair_block) cudaFree(s.d_pair_block);
-        if (s.d_cta_hist) cudaFree(s.d_cta_hist);
-        if (s.d_totals) cudaFree(s.d_totals);
-        if (s.h_totals) cudaFreeHost(s.h_totals);
-        if (s.totals_ready) cudaEventDestroy(s.totals_ready);
         if (s.ready) cudaEventDestroy(s.ready);
         if (s.consumed) cudaEventDestroy(s.consumed);
     }
     if (net->h_loss) cudaFreeHost(net->h_loss);
+    if (net->h_out) cudaFreeHost(net->h_out);
     for (auto& e : net->loss_ev)
         if (e) cudaEventDestroy(e);
     for (auto& ring : net->tev)
@@ -1108,7 +1195,24 @@ static int upload_begin(b200_net* net, int slot, int32_t n, const char* who) {
     return 0;
 }
 
-static int upload_finish(b200_net* net, Slot& s, int32_t n);
+// The row lists of the tiled kernels depend on the indices only: they are built right behind the copy, on the copy stream,
+// where they run beside the step that is still computing.  What only the backward reads waits for a network that trains.
+static bool upload_wants_lists(const b200_net* net, int32_t n) {
+    return net->tiled_ok && (net->fwd_tiled(n) || (net->bwd_tiled() && net->trains));
+}
+
+// Common end: the slot's batch is on its way to the device; group it and mark the slot ready.
+static int upload_finish(b200_net* net, Slot& s, bool want_order, bool counted) {
+    const bool want_lists = upload_wants_lists(net, s.n);
+    if (want_lists || want_order)
+        if (int rc = group_slot(net, s, group_args(net, s, want_lists, want_order), counted, net->copy_stream)) return rc;
+    if (want_lists && net->bwd_tiled() && net->trains)
+        if (int rc = build_csr(net, s, net->copy_stream)) return rc;
+    CK(cudaEventRecord(s.ready, net->copy_stream));
+    s.has_ready = true;
+    s.has_consumed = false;
+    return 0;
+}
 
 int b200_batch_upload(b200_net* net, int slot, const int32_t* stm, const int32_t* nstm, const int32_t* buckets,
                       const float* targets, int32_t n) {
@@ -1139,219 +1243,48 @@ int b200_batch_upload(b200_net* net, int slot, const int32_t* stm, const int32_t
         memset(h_buckets, 0, (size_t)n * 4);
     }
     memcpy(s.host<float>(s.off_targets), targets, (size_t)n * 4);
-    return upload_finish(net, s, n);
+    s.n = n;
+    s.prepared = s.csr_built = false;
+    cut_dense(net, s);
+    cut_ft(net, s);
+    // positions by output bucket: with the row lists on the device; for a batch that needs no lists here, which is a small
+    // one or one of a network without them, before the copy: two launches fewer
+    const bool order_here = O > 1 && !upload_wants_lists(net, n) && n <= 4096;
+    size_t bytes = s.off_order;
+    if (order_here) {
+        int begin[b200::kGroupMaxBuckets + 1] = {0};
+        for (int i = 0; i < n; i++) begin[h_buckets[i] + 1]++;
+        int2* h_tiles = s.host<int2>(s.off_dtiles);
+        s.n_dtiles = 0;
+        for (int k = 0; k < O; k++) {
+            begin[k + 1] += begin[k];
+            for (int at = begin[k]; at < begin[k + 1]; at += b200::kDenseTile)
+                h_tiles[s.n_dtiles++] = make_int2(at, std::min(b200::kDenseTile, begin[k + 1] - at));
+        }
+        int* h_order = s.host<int>(s.off_order);
+        for (int i = 0; i < n; i++) h_order[begin[h_buckets[i]]++] = i;
+        bytes = s.off_records;
+    }
+    CK(cudaMemcpyAsync(s.d_blob, s.h_blob, bytes, cudaMemcpyHostToDevice, net->copy_stream));
+    net->h2d_bytes += (int64_t)bytes;
+    return upload_finish(net, s, O > 1 && !order_here, false);
 }
 
-// Records in, batch on the device: the featuriser, the output bucket and the target blend of
-// ValueTrainerState::make_mapper (crates/bullet_lib/src/value.rs:77-117) write straight into the
-// pinned staging block as packed u16 lists; no int32 arrays in between.
-int b200_batch_upload_records(b200_net* net, int slot, const void* records, int32_t n, int32_t game, const int32_t* layout32,
-                              float scale, float blend) {
-    if (!net || !records) return b200::fail(B200_ERR_ARG, "batch_upload_records: null argument");
-    if (game < B200_GAME_CHESS768 || game > B200_GAME_ATAXX147) return b200::fail(B200_ERR_ARG, "batch_upload_records: unknown game %d", game);
-    if (game == B200_GAME_CHESS_BUCKETS_MIRRORED && !layout32) return b200::fail(B200_ERR_ARG, "batch_upload_records: the king-bucket layout is missing");
-    if (!(blend >= 0.f && blend <= 1.f) || !(scale > 0.f)) return b200::fail(B200_ERR_ARG, "batch_upload_records: bad scale or blend");
+// Records in, batch prepared on the device: the raw 32 bytes per position are checked while they are copied into the
+// pinned block and cross PCIe as they are; the featuriser, the output bucket and the target blend of
+// ValueTrainerState::make_mapper (crates/bullet_lib/src/value.rs:77-117) and the grouping run as kernels on the copy
+// stream.  Nothing is read back, so the call returns when everything is enqueued.
+static int upload_records(b200_net* net, int slot, const void* records, int32_t n, int32_t game, const int32_t* layout32, float scale, float blend,
+                          const char* who) {
+    if (!net || !records) return b200::fail(B200_ERR_ARG, "%s: null argument", who);
+    if (game < B200_GAME_CHESS768 || game > B200_GAME_ATAXX147) return b200::fail(B200_ERR_ARG, "%s: unknown game %d", who, game);
+    if (game == B200_GAME_CHESS_BUCKETS_MIRRORED && !layout32) return b200::fail(B200_ERR_ARG, "%s: the king-bucket layout is missing", who);
+    if (!(blend >= 0.f && blend <= 1.f) || !(scale > 0.f)) return b200::fail(B200_ERR_ARG, "%s: bad scale or blend", who);
     const b200_net_desc& d = net->d;
     const int O = d.n_out_buckets;
-    if (O > 1 && game == B200_GAME_ATAXX147) return b200::fail(B200_ERR_UNSUPPORTED, "batch_upload_records: no output buckets for ataxx records");
-    if (int rc = upload_begin(net, slot, n, "batch_upload_records")) return rc;
+    if (O > 1 && game == B200_GAME_ATAXX147) return b200::fail(B200_ERR_UNSUPPORTED, "%s: no output buckets for ataxx records", who);
+    if (int rc = upload_begin(net, slot, n, who)) return rc;
     Slot& s = net->slots[slot];
-    uint16_t* h_stm = s.host<uint16_t>(s.off_stm);
-    uint16_t* h_nstm = s.host<uint16_t>(s.off_nstm);
-    int* h_buckets = s.host<int>(s.off_buckets);
-    float* h_targets = s.host<float>(s.off_targets);
-    int32_t expanded[64] = {0};
-    if (game == B200_GAME_CHESS_BUCKETS_MIRRORED) b200::expand_king_buckets(layout32, expanded);
-    const b200::ChessRecord* chess = static_cast<const b200::ChessRecord*>(records);
-    const b200::AtaxxRecord* ataxx = static_cast<const b200::AtaxxRecord*>(records);
-    const int nnz = d.nnz;
-    const uint32_t limit = (uint32_t)d.n_inputs;
-    const float rscale = 1.0f / scale;
-    int bad = n, bad_bucket = n;
-#pragma omp parallel for schedule(static) reduction(min : bad) reduction(min : bad_bucket) if (n >= 4096)
-    for (int32_t i = 0; i < n; i++) {
-        uint16_t* a = h_stm + (size_t)i * nnz;
-        uint16_t* b = h_nstm + (size_t)i * nnz;
-        int count;
-        if (game == B200_GAME_CHESS768)
-            count = b200::map_chess_record<false, uint16_t>(chess[i], expanded, a, b, nnz, (uint16_t)0xFFFFu);
-        else if (game == B200_GAME_CHESS_BUCKETS_MIRRORED)
-            count = b200::map_chess_record<true, uint16_t>(chess[i], expanded, a, b, nnz, (uint16_t)0xFFFFu);
-        else
-            count = b200::map_ataxx_record<uint16_t>(ataxx[i], a, b, nnz, (uint16_t)0xFFFFu);
-        if (count < 0) {
-            bad = i < bad ? i : bad;
-            continue;
-        }
-        for (int k = 0; k < count; k++) {  // as b200_batch_upload: an index the table does not have is an empty slot
-            if (a[k] >= limit) a[k] = 0xFFFFu;
-            if (b[k] >= limit) b[k] = 0xFFFFu;
-        }
-        int bucket = 0;
-        if (O > 1) {
-            bucket = b200::material_bucket(chess[i].occ, O);
-            if ((unsigned)bucket >= (unsigned)O) bad_bucket = i < bad_bucket ? i : bad_bucket;
-        }
-        h_buckets[i] = bucket;
-        h_targets[i] = b200::blended_target(chess[i].score, chess[i].result, rscale, blend);  // same offsets in both record types
-    }
-    if (bad < n) return b200::fail(B200_ERR_DATA, "batch_upload_records: record %d holds more than nnz=%d pieces", bad, nnz);
-    if (bad_bucket < n) return b200::fail(B200_ERR_DATA, "batch_upload_records: record %d has no valid output bucket", bad_bucket);
-    return upload_finish(net, s, n);
-}
-
-// Everything the kernels need beyond the batch itself, from two histograms: how many positions take each
-// output bucket and how many (position, perspective) pairs fall into each table row block.  Fills, in the
-// slot's pinned block: the dense kernels' tiles, the blocks' first pairs, the backward's chunks, their
-// first chunk per block and the per-block CTA counts of a whole-batch backward launch.
-static void derive_tables(b200_net* net, Slot& s, const int* bucket_count, const int* block_count) {
-    const b200_net_desc& d = net->d;
-    const int O = d.n_out_buckets, nb = net->nblocks;
-    {   // CTA tiles of the dense kernels: runs of up to kDenseTile positions of one bucket
-        int2* h_tiles = s.host<int2>(s.off_dtiles);
-        int nt = 0, at = 0;
-        for (int k = 0; k < O; k++) {
-            const int end = at + bucket_count[k];
-            for (; at < end; at += b200::kDenseTile) h_tiles[nt++] = make_int2(at, std::min(b200::kDenseTile, end - at));
-            at = end;
-        }
-        s.n_dtiles = nt;
-    }
-    int* h_blocks = s.host<int>(s.off_blocks);
-    h_blocks[0] = 0;
-    for (int b = 0; b < nb; b++) h_blocks[b + 1] = h_blocks[b] + block_count[b];
-    s.block_begin.assign(h_blocks, h_blocks + nb + 1);
-    if (net->tiled_ok) {
-        // chunks of the tiled backward: every block cut into the fewest equal runs of at most ft_bwd_chunk pairs
-        int4* h_chunks = s.host<int4>(s.off_chunks);
-        int* h_cbegin = s.host<int>(s.off_cbegin);
-        const int cp = net->bwd_chunk(h_blocks[nb] / 2);  // (all pairs of the batch = two per position)
-        s.chunk_len = cp;
-        int nc = 0;
-        for (int b = 0; b < nb; b++) {
-            h_cbegin[b] = nc;
-            const int pairs = h_blocks[b + 1] - h_blocks[b], pieces = (pairs + cp - 1) / cp;
-            const int size = pieces ? (pairs + pieces - 1) / pieces : 0;
-            for (int at = h_blocks[b]; at < h_blocks[b + 1]; at += size) h_chunks[nc++] = make_int4(b, at, std::min(size, h_blocks[b + 1] - at), 0);
-        }
-        h_cbegin[nb] = nc;
-        s.n_chunks = nc;
-        s.chunk_begin.assign(h_cbegin, h_cbegin + nb + 1);
-        // How many CTAs of a whole-batch backward launch work on each block, for the data-parallel runs that
-        // announce finished blocks: there CTA k takes the units k, k + grid, ... of the block-ordered numbering.
-        int* h_expect = s.host<int>(s.off_bexpect);
-        const int grid = ft_backward_grid(net, s, 0, nb, net->overlap_mode);
-        s.expect_grid = grid;
-        for (int blk = 0; blk < nb; blk++) h_expect[blk] = std::min(grid, net->nslabs * (h_cbegin[blk + 1] - h_cbegin[blk]));
-    }
-    *s.host<int>(s.off_status) = 0;
-}
-
-// The row lists of the tiled kernels depend on the indices only: build them right behind the copy, on
-// the copy stream, where they run beside the step that is still computing; then mark the slot ready.
-static int upload_launch_lists(b200_net* net, Slot& s, int32_t n) {
-    const b200_net_desc& d = net->d;
-    s.prepared = s.csr_built = false;
-    s.n = n;
-    const bool backward = net->bwd_tiled() && net->trains;
-    if (net->tiled_ok && (net->fwd_tiled(n) || backward)) {
-        b200::FtArgs fa = ft_args(net, s);
-        b200::TileArgs ta = tile_args(net, s, true);
-        b200::ft_prepare_kernel<<<(2 * n + 7) / 8, 256, 0, net->copy_stream>>>(fa, ta);
-        LAUNCHED(net);
-        s.prepared = true;
-        if (backward && s.n_chunks > 0) {
-            b200::ft_csr_kernel<<<s.n_chunks, b200::kCsrThreads, b200::ft_csr_smem(d.ft_block_rows, d.nnz, s.chunk_len), net->copy_stream>>>(fa, ta);
-            LAUNCHED(net);
-            s.csr_built = true;
-        }
-    }
-    CK(cudaEventRecord(s.ready, net->copy_stream));
-    s.has_ready = true;
-    s.has_consumed = false;
-    s.n = n;
-    return 0;
-}
-
-static int upload_finish(b200_net* net, Slot& s, int32_t n) {
-    const b200_net_desc& d = net->d;
-    const int O = d.n_out_buckets, nb = net->nblocks;
-    int* h_buckets = s.host<int>(s.off_buckets);
-    const uint16_t* h_stm = s.host<uint16_t>(s.off_stm);
-    const uint16_t* h_nstm = s.host<uint16_t>(s.off_nstm);
-    // visiting order of the dense weight-gradient kernel: positions grouped by output bucket (stable)
-    std::vector<int> bucket_count(O, 0), block_count(nb, 0);
-    {
-        int* h_order = s.host<int>(s.off_order);
-        std::vector<int> begin(O + 1, 0);
-        for (int i = 0; i < n; i++) begin[h_buckets[i] + 1]++;
-        for (int k = 0; k < O; k++) bucket_count[k] = begin[k + 1];
-        for (int k = 0; k < O; k++) begin[k + 1] += begin[k];
-        for (int i = 0; i < n; i++) h_order[begin[h_buckets[i]]++] = i;
-    }
-    // visiting order of the tiled feature-transformer kernels: (position, perspective)
-    // pairs grouped by the table row block their features live in (stable)
-    if (nb > 1) {
-        int* h_pairs = s.host<int>(s.off_pairs);
-        const int R = d.ft_block_rows, nnz = d.nnz;
-        std::vector<int> begin(nb + 1, 0);
-        std::vector<uint16_t> blk((size_t)2 * n);
-#pragma omp parallel for schedule(static) if (n > 8192)
-        for (int i = 0; i < n; i++) {
-            for (int p = 0; p < 2; p++) {
-                const uint16_t* list = (p ? h_nstm : h_stm) + (size_t)i * nnz;
-                int b = 0;
-                for (int k = 0; k < nnz; k++)
-                    if (list[k] != 0xFFFFu) {
-                        b = list[k] / R;
-                        break;
-                    }
-                blk[(size_t)2 * i + p] = (uint16_t)b;
-            }
-        }
-        for (size_t i = 0; i < blk.size(); i++) begin[blk[i] + 1]++;
-        for (int k = 0; k < nb; k++) block_count[k] = begin[k + 1];
-        for (int k = 0; k < nb; k++) begin[k + 1] += begin[k];
-        for (size_t i = 0; i < blk.size(); i++) h_pairs[begin[blk[i]]++] = (int)i;
-    } else {
-        block_count[0] = 2 * n;
-    }
-    derive_tables(net, s, bucket_count.data(), block_count.data());
-    CK(cudaMemcpyAsync(s.d_blob, s.h_blob, s.bytes, cudaMemcpyHostToDevice, net->copy_stream));
-    net->h2d_bytes += (int64_t)s.bytes;
-    return upload_launch_lists(net, s, n);
-}
-
-// Records in, batch prepared ON the device: 32 bytes per position cross PCIe instead of the packed lists,
-// and the host only sizes the launches from two small histograms it reads back.
-int b200_batch_upload_records_gpu(b200_net* net, int slot, const void* records, int32_t n, int32_t game, const int32_t* layout32,
-                                  float scale, float blend) {
-    if (!net || !records) return b200::fail(B200_ERR_ARG, "batch_upload_records_gpu: null argument");
-    if (game < B200_GAME_CHESS768 || game > B200_GAME_ATAXX147) return b200::fail(B200_ERR_ARG, "batch_upload_records_gpu: unknown game %d", game);
-    if (game == B200_GAME_CHESS_BUCKETS_MIRRORED && !layout32) return b200::fail(B200_ERR_ARG, "batch_upload_records_gpu: the king-bucket layout is missing");
-    if (!(blend >= 0.f && blend <= 1.f) || !(scale > 0.f)) return b200::fail(B200_ERR_ARG, "batch_upload_records_gpu: bad scale or blend");
-    const b200_net_desc& d = net->d;
-    const int O = d.n_out_buckets, nb = net->nblocks, nbins = nb + O;
-    if (O > 1 && game == B200_GAME_ATAXX147) return b200::fail(B200_ERR_UNSUPPORTED, "batch_upload_records_gpu: no output buckets for ataxx records");
-    if (nb > b200::kPrepMaxBins || O > b200::kPrepMaxBins)
-        return b200::fail(B200_ERR_UNSUPPORTED, "batch_upload_records_gpu: at most %d row blocks and output buckets; use b200_batch_upload_records",
-                          b200::kPrepMaxBins);
-    if (int rc = upload_begin(net, slot, n, "batch_upload_records_gpu")) return rc;
-    Slot& s = net->slots[slot];
-    const size_t B = d.max_batch;
-    const int max_ctas = (int)((B + b200::kPrepPositions - 1) / b200::kPrepPositions);
-    if (!s.d_records) {  // first use of this slot by the device path: its scratch, sized for the largest batch
-        CK(cudaMalloc(&s.d_records, B * 32));
-        CK(cudaMalloc(&s.d_pair_block, 2 * B * sizeof(uint16_t)));
-        CK(cudaMalloc(&s.d_cta_hist, (size_t)max_ctas * nbins * sizeof(int)));
-        CK(cudaMalloc(&s.d_totals, (size_t)2 * nbins * sizeof(int)));
-        CK(cudaHostAlloc(&s.h_totals, ((size_t)2 * nbins + 1) * sizeof(int), cudaHostAllocDefault));
-        CK(cudaEventCreateWithFlags(&s.totals_ready, cudaEventDisableTiming));
-    }
-    if (!net->d_win_rate) {
-        CK(cudaMalloc(&net->d_win_rate, 65536 * sizeof(float)));
-        CK(cudaMalloc(&net->d_expanded, 64 * sizeof(int)));
-    }
     if (net->win_rate_scale != scale) {  // the same function the host mapper evaluates, for every possible score
         std::vector<float> table(65536);
         const float rscale = 1.0f / scale;
@@ -1368,20 +1301,35 @@ int b200_batch_upload_records_gpu(b200_net* net, int slot, const void* records, 
         memcpy(net->expanded_layout, layout32, sizeof net->expanded_layout);
         net->expanded_valid = true;
     }
-    // the records go through the slot's pinned block (its list sections are not used on the host here)
-    memcpy(s.h_blob, records, (size_t)n * 32);
-    CK(cudaMemcpyAsync(s.d_records, s.h_blob, (size_t)n * 32, cudaMemcpyHostToDevice, net->copy_stream));
-    CK(cudaMemsetAsync(s.dev<int>(s.off_status), 0, sizeof(int), net->copy_stream));
+    int bad = n, bad_bucket = n;
+    {
+        const b200::AtaxxRecord* in = static_cast<const b200::AtaxxRecord*>(records);  // (both kinds start with 64-bit boards)
+        b200::AtaxxRecord* out = reinterpret_cast<b200::AtaxxRecord*>(s.h_blob);
+        const int nnz = d.nnz;
+        const bool ataxx = game == B200_GAME_ATAXX147;
+#pragma omp parallel for schedule(static) reduction(min : bad) reduction(min : bad_bucket) if (n >= 8192)
+        for (int32_t i = 0; i < n; i++) {
+            const b200::AtaxxRecord r = in[i];
+            out[i] = r;
+            int pieces = __builtin_popcountll(r.bbs[0]);
+            if (ataxx) pieces += __builtin_popcountll(r.bbs[1]) + __builtin_popcountll(r.bbs[2]);
+            if (pieces > nnz) bad = i < bad ? i : bad;
+            if (O > 1 && (unsigned)b200::material_bucket(r.bbs[0], O) >= (unsigned)O) bad_bucket = i < bad_bucket ? i : bad_bucket;
+        }
+    }
+    if (bad < n) return b200::fail(B200_ERR_DATA, "%s: record %d holds more than nnz=%d pieces", who, bad, d.nnz);
+    if (bad_bucket < n) return b200::fail(B200_ERR_DATA, "%s: record %d has no valid output bucket", who, bad_bucket);
     net->h2d_bytes += (int64_t)n * 32;
+    s.n = n;
+    s.prepared = s.csr_built = false;
+    cut_dense(net, s);
+    cut_ft(net, s);
     b200::PrepArgs p{};
-    p.records = s.d_records;
-    p.n = n;
-    p.nnz = d.nnz;
-    p.n_inputs = d.n_inputs;
+    // an evaluation waits for its batch: the featuriser then reads the pinned block itself.  (Beside a training step its CTAs
+    // would wait for PCIe on SMs that the step could use.)
+    const bool direct = !net->trains && n <= 16384;
+    p.records = direct ? reinterpret_cast<const uint4*>(s.h_blob) : s.dev<uint4>(s.off_records);
     p.game = game;
-    p.n_out_buckets = O;
-    p.block_rows = net->tiled_ok ? d.ft_block_rows : d.n_inputs;
-    p.nblocks = nb;
     p.expanded = net->d_expanded;
     p.win_rate = net->d_win_rate;
     p.blend = blend;
@@ -1389,33 +1337,20 @@ int b200_batch_upload_records_gpu(b200_net* net, int slot, const void* records, 
     p.nstm = s.dev<uint16_t>(s.off_nstm);
     p.buckets = s.dev<int>(s.off_buckets);
     p.targets = s.dev<float>(s.off_targets);
-    p.pair_block = s.d_pair_block;
-    p.cta_hist = s.d_cta_hist;
-    p.totals = s.d_totals;
-    p.order = s.dev<int>(s.off_order);
-    p.pair_order = s.dev<int>(s.off_pairs);
-    p.status = s.dev<int>(s.off_status);
-    const int ctas = (n + b200::kPrepPositions - 1) / b200::kPrepPositions;
-    b200::prep_featurise_kernel<<<ctas, b200::kPrepPositions, 0, net->copy_stream>>>(p);
+    if (!direct) CK(cudaMemcpyAsync(s.d_blob + s.off_records, s.h_blob, (size_t)n * 32, cudaMemcpyHostToDevice, net->copy_stream));
+    const b200::GroupArgs g = group_args(net, s, upload_wants_lists(net, n), O > 1);
+    b200::prep_featurise_kernel<<<b200::group_ctas(n), b200::kPrepThreads, 0, net->copy_stream>>>(p, g);
     LAUNCHED(net);
-    b200::prep_scan_kernel<<<1, 512, 0, net->copy_stream>>>(p, ctas);
-    LAUNCHED(net);
-    CK(cudaMemcpyAsync(s.h_totals, s.d_totals, (size_t)2 * nbins * sizeof(int), cudaMemcpyDeviceToHost, net->copy_stream));
-    CK(cudaMemcpyAsync(s.h_totals + 2 * nbins, s.dev<int>(s.off_status), sizeof(int), cudaMemcpyDeviceToHost, net->copy_stream));
-    CK(cudaEventRecord(s.totals_ready, net->copy_stream));
-    b200::prep_scatter_kernel<<<ctas, 2 * b200::kPrepPositions, 0, net->copy_stream>>>(p);
-    LAUNCHED(net);
-    // the host needs the bin totals to lay out chunks and tiles and to size the step's launches
-    CK(cudaEventSynchronize(s.totals_ready));
-    const int status = s.h_totals[2 * nbins];
-    if (status & b200::kStatusTooManyPieces) return b200::fail(B200_ERR_DATA, "batch_upload_records_gpu: a record holds more than nnz=%d pieces", d.nnz);
-    if (status & b200::kStatusBadBucket) return b200::fail(B200_ERR_DATA, "batch_upload_records_gpu: a record has no valid output bucket");
-    derive_tables(net, s, s.h_totals + nb, s.h_totals);
-    // only the derived tables travel: they sit behind the lists and the two orders in the slot's block
-    const size_t tail = s.off_blocks;
-    CK(cudaMemcpyAsync(s.d_blob + tail, s.h_blob + tail, s.bytes - tail, cudaMemcpyHostToDevice, net->copy_stream));
-    net->h2d_bytes += (int64_t)(s.bytes - tail);
-    return upload_launch_lists(net, s, n);
+    return upload_finish(net, s, O > 1, true);
+}
+
+int b200_batch_upload_records(b200_net* net, int slot, const void* records, int32_t n, int32_t game, const int32_t* layout32,
+                              float scale, float blend) {
+    return upload_records(net, slot, records, n, game, layout32, scale, blend, "batch_upload_records");
+}
+int b200_batch_upload_records_gpu(b200_net* net, int slot, const void* records, int32_t n, int32_t game, const int32_t* layout32,
+                                  float scale, float blend) {
+    return upload_records(net, slot, records, n, game, layout32, scale, blend, "batch_upload_records_gpu");
 }
 
 int b200_slot_read(b200_net* net, int slot, uint16_t* stm, uint16_t* nstm, int32_t* buckets, float* targets, int32_t* order,
@@ -1429,13 +1364,31 @@ int b200_slot_read(b200_net* net, int slot, uint16_t* stm, uint16_t* nstm, int32
     if (nstm) CK(cudaMemcpy(nstm, s.d_blob + s.off_nstm, list, cudaMemcpyDeviceToHost));
     if (buckets) CK(cudaMemcpy(buckets, s.d_blob + s.off_buckets, count * 4, cudaMemcpyDeviceToHost));
     if (targets) CK(cudaMemcpy(targets, s.d_blob + s.off_targets, count * 4, cudaMemcpyDeviceToHost));
-    if (order) CK(cudaMemcpy(order, s.d_blob + s.off_order, count * 4, cudaMemcpyDeviceToHost));
+    // both groupings as they are defined: ascending inside a group.  (The kernels visit the pairs of a block in another
+    // order, which the lists' lengths decide.)
+    if (order) {
+        std::vector<int> bucket(count);
+        CK(cudaMemcpy(bucket.data(), s.d_blob + s.off_buckets, count * 4, cudaMemcpyDeviceToHost));
+        std::vector<int> begin(net->d.n_out_buckets + 1, 0);
+        for (size_t i = 0; i < count; i++) begin[bucket[i] + 1]++;
+        for (int k = 0; k < net->d.n_out_buckets; k++) begin[k + 1] += begin[k];
+        for (size_t i = 0; i < count; i++) order[begin[bucket[i]]++] = (int32_t)i;
+    }
     if (pair_order) {
-        if (net->nblocks > 1) {
-            CK(cudaMemcpy(pair_order, s.d_blob + s.off_pairs, count * 8, cudaMemcpyDeviceToHost));
-        } else {  // a single row block is visited in pair order and keeps no list
-            for (size_t i = 0; i < 2 * count; i++) pair_order[i] = (int32_t)i;
+        const int nnz = net->d.nnz, R = net->nblocks > 1 ? net->d.ft_block_rows : net->d.n_inputs;
+        std::vector<uint16_t> lists[2] = {std::vector<uint16_t>(count * nnz), std::vector<uint16_t>(count * nnz)};
+        CK(cudaMemcpy(lists[0].data(), s.d_blob + s.off_stm, list, cudaMemcpyDeviceToHost));
+        CK(cudaMemcpy(lists[1].data(), s.d_blob + s.off_nstm, list, cudaMemcpyDeviceToHost));
+        std::vector<int> block(2 * count), begin(net->nblocks + 1, 0);
+        for (size_t i = 0; i < 2 * count; i++) {
+            const uint16_t* own = lists[i & 1].data() + (i >> 1) * nnz;
+            int k = 0;
+            while (k < nnz && own[k] >= net->d.n_inputs) k++;
+            block[i] = k < nnz ? own[k] / R : 0;
+            begin[block[i] + 1]++;
         }
+        for (int k = 0; k < net->nblocks; k++) begin[k + 1] += begin[k];
+        for (size_t i = 0; i < 2 * count; i++) pair_order[begin[block[i]]++] = (int32_t)i;
     }
     if (n) *n = s.n;
     return 0;
@@ -1503,13 +1456,8 @@ int b200_backward_begin(b200_net* net, int slot) {
     if (int rc = forward_dense(net, s, true)) return rc;
     cudaEvent_t* ev = net->tev[net->steps_begun % b200_net::kTimingRing];
     CK(cudaEventRecord(ev[2], net->stream));
-    if (net->bwd_tiled() && s.n_chunks > 0 && !s.csr_built) {  // normally built at upload
-        b200::FtArgs fa = ft_args(net, s);
-        b200::TileArgs ta = tile_args(net, s, true);
-        b200::ft_csr_kernel<<<s.n_chunks, b200::kCsrThreads, b200::ft_csr_smem(d.ft_block_rows, d.nnz, s.chunk_len), net->stream>>>(fa, ta);
-        LAUNCHED(net);
-        s.csr_built = true;
-    }
+    if (net->bwd_tiled() && !s.csr_built)  // normally built at upload
+        if (int rc = build_csr(net, s, net->stream)) return rc;
     {
         b200::DenseArgs da = dense_args(net, s, true);
         DISPATCH_M(d.dense_out[0], b200::dense_dx_kernel<MM><<<s.n_dtiles, 256, 0, net->stream>>>(da, net->dx));
@@ -1542,19 +1490,15 @@ int b200_backward_ft(b200_net* net, int slot, int part, int n_parts) {
         b200::FtArgs fa = ft_args(net, s);
         b200::TileArgs ta = tile_args(net, s, true);
         int grid = 0;
-        bool any = true;
         if (tiled) {  // this part's run of blocks
             ta.first_block = part * per;
             ta.last_block = n_parts > 1 ? (part + 1) * per : net->nblocks;
-            any = s.chunk_begin[ta.last_block] > s.chunk_begin[ta.first_block];
-            grid = ft_backward_grid(net, s, ta.first_block, ta.last_block, net->sig_on);
+            grid = ft_backward_grid(net, s, net->sig_on);
             if (net->sig_on && grid != s.expect_grid)
                 return b200::fail(B200_ERR_STATE, "backward_ft: the batch was uploaded before the exchange under the backward was switched on");
         }
-        if (any) {
-            int rc = d.pairwise ? launch_ft_backward<true>(net, fa, ta, tiled, grid) : launch_ft_backward<false>(net, fa, ta, tiled, grid);
-            if (rc) return rc;
-        }
+        int rc = d.pairwise ? launch_ft_backward<true>(net, fa, ta, tiled, grid) : launch_ft_backward<false>(net, fa, ta, tiled, grid);
+        if (rc) return rc;
     }
     if (part == n_parts - 1) CK(cudaEventRecord(ev[4], net->stream));
     if (d.factoriser_rows && !(net->sig_on && net->facc)) {  // (the overlapped exchange sums the reduced blocks itself)
@@ -2035,8 +1979,9 @@ int b200_forward(b200_net* net, int slot, float* out_host) {
     CK(cudaEventRecord(s.consumed, net->stream));
     s.has_consumed = true;
     net->last_n = s.n;
-    CK(cudaMemcpyAsync(out_host, net->out, (size_t)s.n * sizeof(float), cudaMemcpyDeviceToHost, net->stream));
+    if (s.n > kDirectOutputs) CK(cudaMemcpyAsync(net->h_out, net->out, (size_t)s.n * sizeof(float), cudaMemcpyDeviceToHost, net->stream));
     CK(cudaStreamSynchronize(net->stream));
+    memcpy(out_host, net->h_out, (size_t)s.n * sizeof(float));
     return 0;
 }
 

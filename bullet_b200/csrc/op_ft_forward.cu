@@ -9,19 +9,20 @@
 // device pointers of the caller.
 //
 // The tiled kernel visits (position, perspective) pairs grouped by the table row block their
-// features live in.  A b200_net gets that grouping from the host packer; here it is built on
-// the device into scratch memory: a block id per pair, a histogram, its scan and the grouped
-// pair order.  b200_op_ft_forward takes that scratch from cudaMalloc for the duration of the
-// call; b200_op_ft_forward_noalloc keeps it in a fixed array that is part of the library image.
+// features live in; the grouping (kernels_group.cuh) is built on the device into scratch memory.
+// b200_op_ft_forward takes that scratch from a memory pool of its own; b200_op_ft_forward_noalloc keeps
+// it in a fixed array that is part of the library image.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 
 #include "../../include/bullet_b200.h"
 #include "common.h"
-#include "kernels_ft.cuh"
+#include "kernels_group.cuh"
+#include "op_pool.h"
 
 #define CK(call)                                                                                          \
     do {                                                                                                  \
@@ -35,69 +36,55 @@ namespace {
 
 constexpr int kMaxBlocks = 1024;  // table row blocks the grouping supports
 
-// Scratch layout, in ints: [0] status word, [1 .. 1+kMaxBlocks] histogram then running
-// cursors, [.. +kMaxBlocks+1] block_begin, one work item (int4) per block, then per pair:
-// block id [2n], pair order [2n], prepared list length [2n], and the prepared row lists
-// [2n][nnz rounded up to 4] as u16.
-// Every section starts on a 256-byte boundary: the row lists are read with 16-byte loads.
+// Scratch layout, in ints, every section on a 256-byte boundary: the blocks' first pairs, per pair its
+// block and list length [2n], (pair id, rows) [2n] and the prepared row lists [2n][nnz rounded up to 8] as u16, then the
+// histograms of the grouping's first pass, or its counters where there are more blocks than its windows hold.
 constexpr size_t kSectionAlign = 64;  // ints
 constexpr size_t align_ints(size_t v) { return (v + kSectionAlign - 1) / kSectionAlign * kSectionAlign; }
-constexpr size_t kItemsAt = align_ints(1 + (kMaxBlocks + 1) + (kMaxBlocks + 1));
-constexpr size_t kScratchHeader = kItemsAt + 4 * kMaxBlocks;
-int list_len(int nnz) { return (nnz + 7) & ~7; }  // 16-byte groups of u16 row indices
-size_t scratch_ints(int n, int nnz) { return kScratchHeader + 3 * align_ints((size_t)2 * n) + (size_t)2 * n * list_len(nnz); }
+constexpr size_t kScratchHeader = align_ints(kMaxBlocks + 1);
+constexpr int list_len(int nnz) { return (nnz + 7) & ~7; }  // 16-byte groups of u16 row indices
+constexpr size_t hist_ints(int n, int nblocks) {
+    return nblocks > b200::kGroupMaxBlocks ? align_ints(3 * (size_t)(nblocks + 3))
+                                           : align_ints((size_t)((n + b200::kGroupPositions - 1) / b200::kGroupPositions) * (nblocks + 1));
+}
+constexpr size_t scratch_ints(int n, int nnz, int nblocks) {
+    return kScratchHeader + align_ints((size_t)2 * n) + align_ints((size_t)4 * n) + (size_t)n * list_len(nnz) + hist_ints(n, nblocks);
+}
 
 // Scratch of b200_op_ft_forward_noalloc: room for B200_OP_NOALLOC_MAX_POSITIONS positions of
-// up to 32 index slots (about 4.6 MB).  It is a file-scope device array, so every GPU on
+// up to 32 index slots (about 2.7 MB).  It is a file-scope device array, so every GPU on
 // which the library is loaded carries it from load until the process exits, and every call
 // on that GPU uses the same bytes.
-constexpr size_t kStaticInts =
-    kScratchHeader + 3 * align_ints((size_t)2 * B200_OP_NOALLOC_MAX_POSITIONS) + (size_t)2 * B200_OP_NOALLOC_MAX_POSITIONS * 32;
+constexpr size_t kStaticInts = scratch_ints(B200_OP_NOALLOC_MAX_POSITIONS, 32, b200::kGroupMaxBlocks);
 static __device__ __align__(256) int g_op_scratch[kStaticInts];
 
-__global__ void group_count_kernel(const uint16_t* stm, const uint16_t* nstm, int n, int nnz, int n_inputs,
-                                   int block_rows, int* counts, int* blk) {
-    const int pair = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pair >= 2 * n) return;
-    const uint16_t* list = ((pair & 1) ? nstm : stm) + (size_t)(pair >> 1) * nnz;
-    int b = 0;  // a perspective without any valid feature may go anywhere
-    for (int k = 0; k < nnz; k++) {
-        const unsigned v = list[k];
-        if (v < (unsigned)n_inputs) {
-            b = (int)v / block_rows;
-            break;
-        }
+// A call's status word: pinned host memory that the kernels touch only if there is something to report, so that nothing has
+// to be copied back.  A process keeps one block of them (4 KB for as long as it lives); a call holds one for its duration.
+constexpr int kStatusWords = 64;
+struct StatusWord {
+    int* status = nullptr;
+    StatusWord() {
+        static int* words = [] {
+            void* raw = nullptr;
+            return cudaHostAlloc(&raw, kStatusWords * 64, cudaHostAllocPortable) == cudaSuccess ? static_cast<int*>(raw) : nullptr;
+        }();
+        if (!words) return;
+        while (!status)  // as many calls as there are words are under way at once at most
+            for (int k = 0; k < kStatusWords && !status; k++) {
+                bool free = false;
+                if (taken()[k].compare_exchange_strong(free, true)) at = k, status = words + 16 * k;
+            }
+        *status = 0;
     }
-    blk[pair] = b;
-    atomicAdd(&counts[b], 1);
-}
-
-// one CTA: exclusive scan of the histogram -> block_begin, cursors = block_begin
-__global__ void group_scan_kernel(int* counts, int* begin, int nblocks) {
-    __shared__ int s[kMaxBlocks + 1];
-    for (int i = threadIdx.x; i < nblocks; i += blockDim.x) s[i] = counts[i];
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int run = 0;
-        for (int i = 0; i < nblocks; i++) {
-            const int c = s[i];
-            s[i] = run;
-            run += c;
-        }
-        s[nblocks] = run;
+    ~StatusWord() {
+        if (status) taken()[at] = false;
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i <= nblocks; i += blockDim.x) {
-        begin[i] = s[i];
-        if (i < nblocks) counts[i] = s[i];
+    static std::atomic<bool>* taken() {
+        static std::atomic<bool> flags[kStatusWords];
+        return flags;
     }
-}
-
-__global__ void group_fill_kernel(const int* blk, int n, int* cursors, int* order) {
-    const int pair = blockIdx.x * blockDim.x + threadIdx.x;
-    if (pair >= 2 * n) return;
-    order[atomicAdd(&cursors[blk[pair]], 1)] = pair;
-}
+    int at = 0;
+};
 
 int check_op(const b200_ft_op* op, const char* who) {
     if (!op) return b200::fail(B200_ERR_ARG, "%s: null operator description", who);
@@ -124,19 +111,41 @@ int check_op(const b200_ft_op* op, const char* who) {
 // reports a feature outside its block.  Allocates nothing.
 int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) {
     const int n = op->n, R = op->ft_block_rows, nblocks = op->n_inputs / R;
-    int* status = scratch;
-    int* counts = scratch + 1;
-    int* begin = counts + kMaxBlocks + 1;
-    int* blk = scratch + kScratchHeader;
-    int* order = blk + align_ints((size_t)2 * n);
-    int* counts_per_pair = order + align_ints((size_t)2 * n);
-    int* lists = counts_per_pair + align_ints((size_t)2 * n);
-    // the scratch keeps whatever the previous call left: clear what must start at zero
-    CK(cudaMemsetAsync(scratch, 0, (1 + kMaxBlocks + 1) * sizeof(int), stream));
-    const int threads = 256, grid = (2 * n + threads - 1) / threads;
-    group_count_kernel<<<grid, threads, 0, stream>>>(op->idx_stm, op->idx_nstm, n, op->nnz, op->n_inputs, R, counts, blk);
-    group_scan_kernel<<<1, 256, 0, stream>>>(counts, begin, nblocks);
-    group_fill_kernel<<<grid, threads, 0, stream>>>(blk, n, counts, order);
+    StatusWord word;
+    if (!word.status) return b200::fail(B200_ERR_CUDA, "op_ft_forward: no pinned memory for a status word");
+    int* begin = scratch;
+    int* info = scratch + kScratchHeader;
+    int* pairs = info + align_ints((size_t)2 * n);
+    int* lists = pairs + align_ints((size_t)4 * n);
+    int* hist = lists + (size_t)n * list_len(op->nnz);
+    b200::GroupArgs g{};
+    g.stm = op->idx_stm;
+    g.nstm = op->idx_nstm;
+    g.n = n;
+    g.nnz = op->nnz;
+    g.n_inputs = op->n_inputs;
+    g.block_rows = R;
+    g.nblocks = nblocks;
+    g.n_out_buckets = 1;
+    g.info = info;
+    g.hist = hist;
+    g.status = word.status;
+    g.want_lists = 1;
+    g.pairs = reinterpret_cast<int2*>(pairs);
+    g.lists = reinterpret_cast<uint16_t*>(lists);
+    g.list_len = list_len(op->nnz);
+    g.block_begin = begin;
+    if (nblocks > b200::kGroupMaxBlocks) {
+        int *at = hist + nblocks + 1, *spare = at + nblocks + 3;
+        CK(cudaMemsetAsync(hist, 0, (size_t)(nblocks + 1) * sizeof(int), stream));
+        b200::group_many_count_kernel<<<(2 * n + 7) / 8, 256, 0, stream>>>(g, hist);
+        b200::group_many_scan_kernel<<<1, 1024, 0, stream>>>(g, hist, at, spare);
+        b200::group_many_place_kernel<<<(2 * n + 7) / 8, 256, 0, stream>>>(g, hist);
+    } else {
+        const bool vec = b200::group_vec(g);
+        b200::group_lists_kernel<<<b200::group_ctas(n), b200::kGroupThreads, 0, stream>>>(g, vec);
+        b200::group_place_kernel<<<b200::group_windows(n), b200::kPlaceThreads, 0, stream>>>(g, vec);
+    }
     CK(cudaGetLastError());
 
     b200::FtArgs a{};
@@ -156,47 +165,85 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
     t.nslabs = op->ft_out / b200::kTileCols;
     t.first_block = 0;
     t.last_block = nblocks;
-    t.pair_order = order;
+    t.pairs = g.pairs;
     t.block_begin = begin;
-    t.status = status;
-    t.lists = reinterpret_cast<uint16_t*>(lists);
-    t.list_count = counts_per_pair;
-    t.list_len = list_len(op->nnz);
+    t.status = word.status;
+    t.lists = g.lists;
+    t.list_len = g.list_len;
     t.once = 1;
-    b200::ft_prepare_kernel<<<(2 * n + 7) / 8, 256, 0, stream>>>(a, t);
-    CK(cudaGetLastError());
     const size_t smem = b200::ft_fwd_smem(R, t.list_len);
     // one CTA per SM, each taking an equal piece of the (block, slab, pair) work line
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const int ctas = (int)std::max<long long>(1, std::min<long long>(sms, (long long)2 * n * t.nslabs / 128));
     if (op->pairwise) {
-        CK(cudaFuncSetAttribute(b200::ft_forward_tiled_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(b200::allow_smem(b200::ft_forward_tiled_kernel<true>));
         b200::ft_forward_tiled_kernel<true><<<ctas, b200::kFwdThreads, smem, stream>>>(a, t);
     } else {
-        CK(cudaFuncSetAttribute(b200::ft_forward_tiled_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        CK(b200::allow_smem(b200::ft_forward_tiled_kernel<false>));
         b200::ft_forward_tiled_kernel<false><<<ctas, b200::kFwdThreads, smem, stream>>>(a, t);
     }
     CK(cudaGetLastError());
-    int host_status = 0;
-    CK(cudaMemcpyAsync(&host_status, status, sizeof(int), cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
-    if (host_status & b200::kStatusOutsideBlock)
+    if (*reinterpret_cast<volatile int*>(word.status) & b200::kStatusOutsideBlock)
         return b200::fail(B200_ERR_DATA, "a feature index fell outside the row block of its position (ft_block_rows=%d)", R);
     return 0;
 }
 
 }  // namespace
 
+// One pool per device for the scratch of b200_op_ft_forward.  It keeps at most kPoolKeep bytes between calls; a network that
+// finds no room for its own buffers has it give those back (op_pool_trim).  Stream-ordered, so calls on several streams and
+// threads never share memory that is in use.
+namespace b200 {
+namespace {
+constexpr uint64_t kPoolKeep = 32u << 20;
+constexpr int kPoolDevices = 64;
+std::mutex pool_lock;
+cudaMemPool_t pools[kPoolDevices] = {};
+}  // namespace
+
+int op_pool_alloc(int device, cudaStream_t stream, size_t bytes, int** out) {
+    if (device < 0 || device >= kPoolDevices) return fail(B200_ERR_ARG, "op_ft_forward: device %d out of range", device);
+    cudaMemPool_t pool = nullptr;
+    {
+        std::lock_guard<std::mutex> guard(pool_lock);
+        if (!pools[device]) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = device;
+            cudaMemPool_t made = nullptr;
+            CK(cudaMemPoolCreate(&made, &props));
+            uint64_t keep = kPoolKeep;
+            CK(cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep));
+            pools[device] = made;
+        }
+        pool = pools[device];
+    }
+    void* raw = nullptr;
+    CK(cudaMallocFromPoolAsync(&raw, bytes, pool, stream));
+    *out = static_cast<int*>(raw);
+    return 0;
+}
+
+void op_pool_trim(int device) {
+    std::lock_guard<std::mutex> guard(pool_lock);
+    if (device >= 0 && device < kPoolDevices && pools[device]) cudaMemPoolTrimTo(pools[device], 0);
+}
+}  // namespace b200
+
 extern "C" {
 
 int b200_op_ft_forward(int device, void* stream, const b200_ft_op* op) {
     if (int rc = check_op(op, "op_ft_forward")) return rc;
     CK(cudaSetDevice(device));
+    // cudaMalloc and cudaFree synchronise the device and cost 0.6 ms and more a call; the pool's stream-ordered ones do not
     int* scratch = nullptr;
-    CK(cudaMalloc(&scratch, scratch_ints(op->n, op->nnz) * sizeof(int)));
-    const int rc = run_op(device, static_cast<cudaStream_t>(stream), op, scratch);
-    cudaFree(scratch);
+    cudaStream_t on = static_cast<cudaStream_t>(stream);
+    if (int rc = b200::op_pool_alloc(device, on, scratch_ints(op->n, op->nnz, op->n_inputs / op->ft_block_rows) * sizeof(int), &scratch)) return rc;
+    const int rc = run_op(device, on, op, scratch);
+    cudaFreeAsync(scratch, on);
     return rc;
 }
 
@@ -217,7 +264,7 @@ int b200_op_ft_forward(int device, void* stream, const b200_ft_op* op) {
 int b200_op_ft_forward_noalloc(int device, void* stream, const b200_ft_op* op) {
     if (int rc = check_op(op, "op_ft_forward_noalloc")) return rc;
     const int most = op->nnz <= 32 ? B200_OP_NOALLOC_MAX_POSITIONS : B200_OP_NOALLOC_MAX_POSITIONS / 2;
-    if (op->n > most || scratch_ints(op->n, op->nnz) > kStaticInts)
+    if (op->n > most || scratch_ints(op->n, op->nnz, op->n_inputs / op->ft_block_rows) > kStaticInts)
         return b200::fail(B200_ERR_ARG,
                           "op_ft_forward_noalloc: %d positions do not fit the fixed scratch, which holds at most %d with "
                           "nnz=%d; split the batch or call b200_op_ft_forward",
