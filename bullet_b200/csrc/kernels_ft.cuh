@@ -299,13 +299,6 @@ __device__ __forceinline__ f32x2 pack2(float a, float b) {
 __device__ __forceinline__ float lo2(f32x2 v) { return __uint_as_float((unsigned)v); }
 __device__ __forceinline__ float hi2(f32x2 v) { return __uint_as_float((unsigned)(v >> 32)); }
 
-template <bool PAIRWISE>
-__device__ __forceinline__ int tile_col_a(int slab, int lane, int H) { return PAIRWISE ? slab * 32 + lane : slab * 64 + 2 * lane; }
-template <bool PAIRWISE>
-__device__ __forceinline__ int tile_col_b(int slab, int lane, int H) {
-    return PAIRWISE ? H / 2 + slab * 32 + lane : slab * 64 + 2 * lane + 1;
-}
-
 // Loads of data that is read once per kernel and must not claim L1 lines: with 196-228 KB of the SM's 256 KB
 // configured as shared memory only 28-60 KB of L1 are left, less than these kernels keep in flight.
 __device__ __forceinline__ float4 ld_once4(const float4* p) {
@@ -313,17 +306,6 @@ __device__ __forceinline__ float4 ld_once4(const float4* p) {
     asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
     return v;
 }
-__device__ __forceinline__ float2 ld_once2(const float2* p) {
-    float2 v;
-    asm("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
-    return v;
-}
-__device__ __forceinline__ float ld_once(const float* p) {
-    float v;
-    asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -332,24 +314,55 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
-// One 256-byte line of shared memory (a tile row, or a staged gradient line), this lane's 8 bytes of it.
-__device__ __forceinline__ f32x2 line_at(const unsigned char* mine, uint32_t index) {
-    return *reinterpret_cast<const f32x2*>(mine + index * kTileRowBytes);
+// The row walks take a line with 16 lanes and 16 bytes each, so that a warp serves two lists at a time: lane l owns floats
+// 4 (l mod 16) .. + 3 of the line.  A list entry is a 16-bit line index; one byte permutation turns it into the byte offset
+// of this lane's piece, because a line is 256 bytes and `lane16` = 16 (l mod 16) fills exactly the lowest byte.
+__device__ __forceinline__ uint32_t entry_lo(uint32_t word, uint32_t lane16) { return __byte_perm(word, lane16, 0x5104); }
+__device__ __forceinline__ uint32_t entry_hi(uint32_t word, uint32_t lane16) { return __byte_perm(word, lane16, 0x5324); }
+struct f32x4 {  // four floats as two packed pairs
+    f32x2 a, b;
+};
+__device__ __forceinline__ f32x4 quad_at(const unsigned char* lines, uint32_t offset) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(lines + offset);
+    return {v.x, v.y};
+}
+__device__ __forceinline__ f32x4 add2(f32x4 x, f32x4 y) { return {add2(x.a, y.a), add2(x.b, y.b)}; }
+// Sum of the lines that `len` entries at `list` (shared memory, 8-byte aligned) name, added in list order from +0.  Four
+// entries per 8-byte load, fetched one group ahead (up to 16 bytes past the list's last group are read and not used);
+// the lanes of a half warp agree on list and length, the two halves need not.
+__device__ __forceinline__ f32x4 sum_lines(const unsigned char* lines, const uint2* list, int len, uint32_t lane16) {
+    f32x4 acc = {0, 0};
+    uint2 g = list[0];
+    int k = 4;
+    for (; k <= len; k += 4) {
+        const uint2 ahead = list[k >> 2];
+        const f32x4 v0 = quad_at(lines, entry_lo(g.x, lane16)), v1 = quad_at(lines, entry_hi(g.x, lane16));
+        const f32x4 v2 = quad_at(lines, entry_lo(g.y, lane16)), v3 = quad_at(lines, entry_hi(g.y, lane16));
+        acc = add2(add2(add2(add2(acc, v0), v1), v2), v3);
+        g = ahead;
+    }
+    const int rest = len - (k - 4);  // none to three more
+    if (rest > 0) {
+        acc = add2(acc, quad_at(lines, entry_lo(g.x, lane16)));
+        if (rest > 1) acc = add2(acc, quad_at(lines, entry_hi(g.x, lane16)));
+        if (rest > 2) acc = add2(acc, quad_at(lines, entry_lo(g.y, lane16)));
+    }
+    return acc;
 }
 
-// Forward.  One CTA of 1024 threads per SM; dynamic shared memory = (R+1) tile rows, the extra row all
-// zero, then per warp one prepared list (and 16 bytes that a read-ahead may touch).  A CTA walks its piece of
-// the work line segment by segment; a segment is a run of pairs of one (block, slab), whose tile the CTA loads
-// first.  Each warp serves one (position, perspective) at a time.  The pair's prepared list reaches the warp
-// one pair ahead: every lane loads one 32-bit word of it (two row indices) into a register while the pair
-// before is still being walked, and stores it into the warp's list buffer afterwards, so the walk itself
-// reads no global memory and the buffer costs one shared-memory wavefront per pair (a cp.async of the same 64
-// bytes by four lanes cost seven).  The walk takes four row indices per (warp-uniform) 8-byte shared-memory
-// load, and every lane adds its column pair with one 64-bit shared-memory load and one packed add per row, in
-// slot order — the same order and arithmetic as the interpreter (adding the zero row changes nothing).
+// Forward.  One CTA of 1024 threads per SM; dynamic shared memory = R tile rows, then per warp two prepared lists (and 16
+// bytes that a read-ahead may touch).  A CTA walks its piece of the work line segment by segment; a segment is a run of
+// pairs of one (block, slab), whose tile the CTA loads first.  Each warp serves two neighbouring pairs at a time, one per
+// half warp; the grouping has put lists of nearly the same length side by side.  The lists reach the warp one round ahead:
+// the lanes load them as 32-bit words into registers while the pairs before are still being walked, and store them into the
+// warp's buffer afterwards, so the walk itself reads no global memory.  Every lane adds its four columns with one 16-byte
+// shared-memory load and two packed adds per row, in slot order — the same order and arithmetic as the interpreter.
+// Bound by the shared-memory pipe: 256 bytes per (row, pair, slab) at 128 bytes a clock.  (One pair per warp, 8 bytes per
+// lane, spent twice the instructions per row and was bound by their issue: 1.65 against FWD_LARGE ms at 131072 positions and
+// width 2048, 0.255 against FWD_MID ms at 16384.)
 constexpr int kFwdThreads = 1024;
 __host__ __device__ inline size_t ft_fwd_smem(int R, int list_len) {
-    return (size_t)(R + 1) * kTileRowBytes + (size_t)(kFwdThreads / 32) * list_len * 2 + 16;
+    return (size_t)R * kTileRowBytes + (size_t)(kFwdThreads / 32) * list_len * 4 + 16;
 }
 
 template <bool PAIRWISE>
@@ -357,7 +370,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int NW = kFwdThreads / 32;
-    const int R = t.block_rows;
+    const int R = t.block_rows, half = lane >> 4, l16 = lane & 15;
+    const uint32_t lane16 = 16 * l16;
     float* tile = reinterpret_cast<float*>(smem_raw);
     // this CTA's piece [v, v_end) of the line of nslabs x (pairs of the launch's blocks) positions
     const int pair0 = t.block_begin[t.first_block];
@@ -365,10 +379,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
     long long v = line * blockIdx.x / gridDim.x;
     const long long v_end = line * (blockIdx.x + 1) / gridDim.x;
     int block = t.first_block;
-    if (threadIdx.x < kTileCols) tile[R * kTileCols + threadIdx.x] = 0.f;  // the zero row
-    const unsigned char* mine = smem_raw + lane * 8;
     // outputs of pair p start at p * (row length): x is [n][2 persp][H or H/2], u is [n][2][H]
     const int x_row = PAIRWISE ? a.H / 2 : a.H;
+    const int words = t.list_len;  // 32-bit words of two lists
+    uint32_t* ring = reinterpret_cast<uint32_t*>(smem_raw + (size_t)R * kTileRowBytes) + warp * words;
+    const uint2* list = reinterpret_cast<const uint2*>(ring + half * (words / 2));
+    const uint32_t* lists_w = reinterpret_cast<const uint32_t*>(t.lists);
     while (v < v_end) {
         // the segment v lies in: block, slab, first pair
         long long base = (long long)t.nslabs * (t.block_begin[block] - pair0);
@@ -386,87 +402,73 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
             // with a factoriser the table row is l0w[row] + l0f[row mod factor_rows], one fp32 add per
             // element exactly as the reference forms `l0w + l0f.repeat(n)` (model/builder.rs:421-424)
             const float* src = a.table + (size_t)block * R * a.H;
+#pragma unroll 3
             for (int i = threadIdx.x; i < R * 8; i += kFwdThreads) {
                 const int row = i >> 3, q = i & 7;
                 float4* dst = reinterpret_cast<float4*>(tile + row * kTileCols + q * 8);
                 const float* frow = a.factor ? a.factor + (size_t)((block * R + row) % a.factor_rows) * a.H : nullptr;
-                if (PAIRWISE) {
-                    const int c_lo = slab * 32 + q * 4, c_hi = a.H / 2 + c_lo;
-                    const float4* plo = reinterpret_cast<const float4*>(src + (size_t)row * a.H + c_lo);
-                    const float4* phi = reinterpret_cast<const float4*>(src + (size_t)row * a.H + c_hi);
-                    float4 lo = t.once ? ld_once4(plo) : __ldg(plo);
-                    float4 hi = t.once ? ld_once4(phi) : __ldg(phi);
-                    if (frow) {
-                        lo = add4(lo, __ldg(reinterpret_cast<const float4*>(frow + c_lo)));  // (these gain from L1)
-                        hi = add4(hi, __ldg(reinterpret_cast<const float4*>(frow + c_hi)));
-                    }
-                    // (the work items of a row lie 32 bytes apart: the upper four of a row store their second half
-                    // first, so that the eight 16-byte stores of a quarter warp fall into eight different bank groups)
-                    const int h = q >> 2;
-                    const float4 first = make_float4(lo.x, hi.x, lo.y, hi.y), second = make_float4(lo.z, hi.z, lo.w, hi.w);
-                    dst[h] = h ? second : first;
-                    dst[h ^ 1] = h ? first : second;
-                } else {
-                    const int c0 = slab * 64 + q * 8;
-                    const float4* g = reinterpret_cast<const float4*>(src + (size_t)row * a.H + c0);
-                    float4 v0 = t.once ? ld_once4(g) : __ldg(g), v1 = t.once ? ld_once4(g + 1) : __ldg(g + 1);
-                    if (frow) {
-                        v0 = add4(v0, __ldg(reinterpret_cast<const float4*>(frow + c0)));
-                        v1 = add4(v1, __ldg(reinterpret_cast<const float4*>(frow + c0 + 4)));
-                    }
-                    const int h = q >> 2;
-                    dst[h] = h ? v1 : v0;
-                    dst[h ^ 1] = h ? v0 : v1;
+                // with pairwise the tile row holds (low-half column, its high-half partner) side by side, both factors of
+                // one product.  (The work items of a row lie 32 bytes apart: the upper four of a row store their second half
+                // first, so that the eight 16-byte stores of a quarter warp fall into eight different bank groups)
+                const int c0 = PAIRWISE ? slab * 32 + q * 4 : slab * 64 + q * 8, c1 = PAIRWISE ? a.H / 2 + c0 : c0 + 4;
+                const float4* p0 = reinterpret_cast<const float4*>(src + (size_t)row * a.H + c0);
+                const float4* p1 = reinterpret_cast<const float4*>(src + (size_t)row * a.H + c1);
+                float4 v0 = t.once ? ld_once4(p0) : __ldg(p0), v1 = t.once ? ld_once4(p1) : __ldg(p1);
+                if (frow) {
+                    v0 = add4(v0, __ldg(reinterpret_cast<const float4*>(frow + c0)));  // (these gain from L1)
+                    v1 = add4(v1, __ldg(reinterpret_cast<const float4*>(frow + c1)));
                 }
+                const int h = q >> 2;
+                const float4 first4 = PAIRWISE ? make_float4(v0.x, v1.x, v0.y, v1.y) : v0;
+                const float4 second4 = PAIRWISE ? make_float4(v0.z, v1.z, v0.w, v1.w) : v1;
+                dst[h] = h ? second4 : first4;
+                dst[h ^ 1] = h ? first4 : second4;
             }
         }
-        const int col_a = tile_col_a<PAIRWISE>(slab, lane, a.H), col_b = tile_col_b<PAIRWISE>(slab, lane, a.H);
-        const f32x2 bias = pack2(a.bias[col_a], a.bias[col_b]);
-        float* x_out = a.x + col_a;  // with pairwise col_a is also the product's column within the perspective
+        // this lane's columns: two products, or four neighbours
+        const int col = PAIRWISE ? slab * 32 + 2 * l16 : slab * 64 + 4 * l16;
+        f32x4 bias;
+        if (PAIRWISE) {
+            const float2 lo = *reinterpret_cast<const float2*>(a.bias + col), hi = *reinterpret_cast<const float2*>(a.bias + a.H / 2 + col);
+            bias = {pack2(lo.x, hi.x), pack2(lo.y, hi.y)};
+        } else {
+            const float4 b = *reinterpret_cast<const float4*>(a.bias + col);
+            bias = {pack2(b.x, b.y), pack2(b.z, b.w)};
+        }
+        float* x_out = a.x + col;
         __syncthreads();
-        // pair id, list length and the list itself are fetched one pair ahead into registers: every lane holds one
-        // 32-bit word (two row indices) of the next pair's list and puts it into the warp's list buffer when the walk
-        // of the current pair is over, so the walk reads its indices from shared memory and never waits for global memory
         const int seg_end = t.block_begin[block] + last;
-        const int list_words = t.list_len / 2;
-        uint32_t* ring = reinterpret_cast<uint32_t*>(smem_raw + (size_t)(R + 1) * kTileRowBytes) + warp * list_words;
-        const uint32_t* lists_w = reinterpret_cast<const uint32_t*>(t.lists);
-        int i = t.block_begin[block] + first + warp;
-        int2 pc = make_int2(0, 0);
-        uint32_t word = 0;
-        if (i < seg_end) {
-            pc = __ldg(t.pairs + i);
-            if (lane < list_words) word = __ldg(lists_w + (size_t)i * list_words + lane);
-        }
-        for (; i < seg_end; i += NW) {
-            const int pair = pc.x, cnt = pc.y;
-            __syncwarp();  // every lane has finished with the list of the pair before
-            if (lane < list_words) ring[lane] = word;
-            if (i + NW < seg_end) {
-                pc = __ldg(t.pairs + i + NW);
-                if (lane < list_words) word = __ldg(lists_w + (size_t)(i + NW) * list_words + lane);
-            }
+        int i = t.block_begin[block] + first + 2 * warp;
+        int2 next = make_int2(0, 0);  // this half's next pair and its length
+        uint32_t w0 = 0, w1 = 0;      // this lane's words of the next two lists
+        auto fetch = [&](int at) {
+            if (at + half < seg_end) next = __ldg(t.pairs + at + half);
+            // (a single last pair: the second list of the two may lie past the end of the lists)
+            const int have = at + 1 < seg_end ? words : words / 2;
+            const uint32_t* src = lists_w + (size_t)at * (words / 2);
+            if (at < seg_end && lane < have) w0 = __ldg(src + lane);
+            if (at < seg_end && lane + 32 < have) w1 = __ldg(src + lane + 32);
+        };
+        fetch(i);
+        for (; i < seg_end; i += 2 * NW) {
+            const int pair = next.x, cnt = i + half < seg_end ? next.y : 0;
+            __syncwarp();  // every lane has finished with the lists of the pairs before
+            if (lane < words) ring[lane] = w0;
+            if (lane + 32 < words) ring[lane + 32] = w1;
+            fetch(i + 2 * NW);
             __syncwarp();
-            f32x2 acc = 0;  // (+0.0f, +0.0f)
-            const uint2* list = reinterpret_cast<const uint2*>(ring);
-            uint2 g = list[0];
-            for (int k = 0; k < cnt; k += 4) {
-                const uint2 g_ahead = list[(k >> 2) + 1];  // (past the last group: the next warp's buffer or the spare 16 bytes, unused)
-                const f32x2 v0 = line_at(mine, g.x & 0xffffu), v1 = line_at(mine, g.x >> 16);
-                const f32x2 v2 = line_at(mine, g.y & 0xffffu), v3 = line_at(mine, g.y >> 16);
-                acc = add2(add2(add2(add2(acc, v0), v1), v2), v3);
-                g = g_ahead;
-            }
-            acc = add2(acc, bias);
-            if (PAIRWISE) {
-                const float ua = crelu_f(lo2(acc)), ub = crelu_f(hi2(acc));
-                float* up = a.u + (size_t)pair * a.H;
-                up[col_a] = ua;
-                up[col_b] = ub;
-                x_out[(size_t)pair * x_row] = ua * ub;
-            } else {
-                *reinterpret_cast<float2*>(x_out + (size_t)pair * x_row) =
-                    make_float2(ft_act_fwd(a.act, lo2(acc)), ft_act_fwd(a.act, hi2(acc)));
+            const f32x4 acc = add2(sum_lines(smem_raw, list, cnt, lane16), bias);
+            if (i + half < seg_end) {
+                if (PAIRWISE) {
+                    const float2 ulo = make_float2(crelu_f(lo2(acc.a)), crelu_f(lo2(acc.b))), uhi = make_float2(crelu_f(hi2(acc.a)), crelu_f(hi2(acc.b)));
+                    float* up = a.u + (size_t)pair * a.H + col;
+                    *reinterpret_cast<float2*>(up) = ulo;
+                    *reinterpret_cast<float2*>(up + a.H / 2) = uhi;
+                    *reinterpret_cast<float2*>(x_out + (size_t)pair * x_row) = make_float2(ulo.x * uhi.x, ulo.y * uhi.y);
+                } else {
+                    *reinterpret_cast<float4*>(x_out + (size_t)pair * x_row) =
+                        make_float4(ft_act_fwd(a.act, lo2(acc.a)), ft_act_fwd(a.act, hi2(acc.a)), ft_act_fwd(a.act, lo2(acc.b)), ft_act_fwd(a.act, hi2(acc.b)));
+                }
             }
         }
     }
@@ -475,14 +477,15 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
 // Backward.  Positions are visited in chunks of at most CP pairs of one row block.
 //   ft_csr_kernel (one CTA per chunk, once per batch) turns the chunk's prepared lists around:
 //     for every table row of the block, the list of the chunk's pairs that hold it (a count
-//     pass, a scan and a fill pass in shared memory), every list starting on a 16-byte
-//     boundary and stored with its exact length.  All column slabs share the result.
+//     pass, a scan and a fill pass in shared memory), every list starting on an 8-byte
+//     boundary.  Lists are cut into pieces of at most kPiece entries and the pieces put in
+//     order of their lengths, longest first.  All column slabs share the result.
 //   ft_backward_tiled_kernel (same grid as the forward) then, per chunk, copies that list
 //     structure into shared memory, stages the chunk's pre-activation gradients (from dx and
-//     the kept activations) as one 64-float line per pair, and every warp walks the lists of
-//     the rows it owns (row = warp, warp + 32, ...), sums the staged lines in registers and
-//     adds the row's total to the table gradient with one global reduction per lane.
-// Accumulation needs no atomics, and the table gradient sees one reduction per (row, chunk)
+//     the kept activations) as one 64-float line per pair, and every half warp walks pieces,
+//     sums the staged lines in registers and adds the total to the row of the table gradient
+//     with one 16-byte global reduction per lane.
+// Accumulation needs no atomics, and the table gradient sees one reduction per (row piece, chunk)
 // instead of one per (row, position).  The table gradient must be zero on entry.
 constexpr int kCsrThreads = 512;
 
@@ -493,15 +496,20 @@ __host__ __device__ inline int ft_bwd_chunk(int nnz, bool wide) { return (wide ?
 // The wide shape takes 640-pair chunks where they fit (768-row blocks with 32 slots: 223 KB): a fifth fewer
 // list copies, barriers and per-row reductions for the same walk; measured 2 % faster at 131072 positions.
 __host__ __device__ inline int ft_bwd_chunk_large(int nnz) { return 640 / (nnz <= 32 ? 1 : 2); }
-// entries per chunk: every slot of every pair plus up to seven padding entries per row (lists start on 16 bytes)
-__host__ __device__ inline int ft_bwd_ent_cap(int R, int nnz, int cp) { return (cp * nnz + 8 * R + 7) & ~7; }
-__host__ __device__ inline int ft_bwd_start_cap(int R) { return (R + 1 + 3) & ~3; }
-__host__ __device__ inline size_t ft_bwd_smem(int R, int nnz, int cp, int nslabs) {
-    return (size_t)(cp + 1) * kTileRowBytes + (size_t)ft_bwd_ent_cap(R, nnz, cp) * 2 + (size_t)ft_bwd_start_cap(R) * 4 + (size_t)cp * 4 +
-           (size_t)nslabs * kTileRowBytes;  // staged lines, row lists, their starts, pair ids, bias-gradient sums per slab
+// Most entries of a piece: the pieces of a chunk differ in length by little from one warp's next to another's, and a king's
+// row, which half the pairs of a chunk may hold, is shared out.
+constexpr int kPiece = 64;
+// entries per chunk: every slot of every pair plus up to three unused ones per row (lists start on 8 bytes), and 16 bytes
+// that a read-ahead may touch
+__host__ __device__ inline int ft_bwd_ent_cap(int R, int nnz, int cp) { return (cp * nnz + 4 * R + 8 + 7) & ~7; }
+// per chunk: entries, pieces, two unused words, then the pieces: first entry / 4 << 17 | length << 10 | row
+__host__ __device__ inline int ft_bwd_start_cap(int R, int nnz, int cp) { return (4 + R + cp * nnz / kPiece + 3) & ~3; }
+__host__ __device__ inline size_t ft_bwd_smem(int R, int nnz, int cp) {
+    return (size_t)cp * kTileRowBytes + (size_t)ft_bwd_ent_cap(R, nnz, cp) * 2 + (size_t)ft_bwd_start_cap(R, nnz, cp) * 4 + (size_t)cp * 4 +
+           32 * kTileRowBytes;  // staged lines, row lists, their pieces, pair ids, bias-gradient sums per warp
 }
 __host__ __device__ inline size_t ft_csr_smem(int R, int nnz, int cp) {
-    return (size_t)ft_bwd_ent_cap(R, nnz, cp) * 2 + (size_t)(2 * (R + 2) + 32 + cp) * 4;
+    return (size_t)ft_bwd_ent_cap(R, nnz, cp) * 2 + (size_t)(2 * (R + 2) + 32 + 2 * (kPiece + 2) + cp) * 4;
 }
 
 // grid = most chunks there can be, block = kCsrThreads.
@@ -511,14 +519,16 @@ static __global__ void __launch_bounds__(kCsrThreads) ft_csr_kernel(FtArgs a, Ti
     constexpr int NW = kCsrThreads / 32;
     const int4 chunk = t.chunks[blockIdx.x];
     if (chunk.z == 0) return;  // (the launch is sized from the batch size alone)
-    const int R = t.block_rows, CP = t.chunk_len, L = t.list_len, c0 = chunk.y, cn = chunk.z;
+    const int R = t.block_rows, L = t.list_len, c0 = chunk.y, cn = chunk.z;
     uint16_t* ent = reinterpret_cast<uint16_t*>(smem_raw);
     int* start = reinterpret_cast<int*>(ent + t.ent_cap);  // [R + 1]
     int* cursor = start + R + 2;                                         // [R]
     int* warp_tot = cursor + R + 2;                                      // [32]
-    int* count_s = warp_tot + 32;                                        // [CP] prepared list lengths
-    const int zero_row = R;
+    int* bin = warp_tot + 32;                                            // [kPiece + 2] pieces by length, then their first places
+    int* count_s = bin + 2 * (kPiece + 2);                               // [CP] prepared list lengths
+    const int zero_row = R;  // (no row: a lane without an entry)
     for (int r = threadIdx.x; r < R; r += kCsrThreads) cursor[r] = 0;
+    if (threadIdx.x < kPiece + 2) bin[threadIdx.x] = 0;
     for (int k = threadIdx.x; k < cn; k += kCsrThreads) count_s[k] = t.pairs[c0 + k].y;
     __syncthreads();
     // count how often each row occurs in the chunk: a warp per pair, a lane per list entry,
@@ -538,12 +548,14 @@ static __global__ void __launch_bounds__(kCsrThreads) ft_csr_kernel(FtArgs a, Ti
                 if (o[k] != zero_row) atomicAdd(&cursor[o[k]], 1);
         }
     __syncthreads();
-    // exclusive scan of the row counts, each rounded up to a multiple of eight entries (16 bytes)
+    // exclusive scan of the row counts, each rounded up to a multiple of four entries (8 bytes)
     {
         int carry = 0;
         for (int base = 0; base < R; base += kCsrThreads) {
             const int r = base + threadIdx.x;
-            const int v = r < R ? (cursor[r] + 7) & ~7 : 0;
+            const int cnt = r < R ? cursor[r] : 0, v = (cnt + 3) & ~3;
+            if (cnt >= kPiece) atomicAdd(&bin[kPiece], cnt / kPiece);
+            if (cnt % kPiece) atomicAdd(&bin[cnt % kPiece], 1);
             int incl = v;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
@@ -582,17 +594,37 @@ static __global__ void __launch_bounds__(kCsrThreads) ft_csr_kernel(FtArgs a, Ti
                 if (o[k] != zero_row) ent[atomicAdd(&cursor[o[k]], 1)] = (uint16_t)(pl0 + k * NW);
         }
     __syncthreads();
-    // the unused tail of every list's last 16-byte group points at the all-zero line (index CP)
-    for (int r = threadIdx.x; r < R; r += kCsrThreads)
-        for (int e = cursor[r]; e < start[r + 1]; e++) ent[e] = (uint16_t)CP;
+    // places of the pieces, longest first
+    if (warp == 0) {
+        int run = 0;
+        for (int base = kPiece; base > 0; base -= 32) {
+            const int own = bin[base - lane];
+            int incl = own;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int n = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += n;
+            }
+            bin[base - lane] = run + incl - own;
+            run += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) bin[0] = run;  // (no piece is empty: the place of length 0 holds their number)
+    }
     __syncthreads();
-    // publish: the entries in 16-byte pieces, and per row its start (in 16-byte units) and exact length
-    const int total = start[R];
+    // publish: the entries in 16-byte pieces, and the list pieces
+    const int total = start[R], pieces = bin[0];
+    __syncthreads();
     uint4* ent_out = reinterpret_cast<uint4*>(t.csr_ent + (size_t)blockIdx.x * t.ent_cap);
-    for (int i = threadIdx.x; i < total / 8; i += kCsrThreads) ent_out[i] = reinterpret_cast<const uint4*>(ent)[i];
-    int* start_out = t.csr_start + (size_t)blockIdx.x * t.start_cap;
-    for (int r = threadIdx.x; r < R; r += kCsrThreads) start_out[r] = ((start[r] >> 3) << 16) | (cursor[r] - start[r]);
-    if (threadIdx.x == 0) start_out[R] = total;
+    for (int i = threadIdx.x; i < (total + 7) / 8; i += kCsrThreads) ent_out[i] = reinterpret_cast<const uint4*>(ent)[i];
+    int* out = t.csr_start + (size_t)blockIdx.x * t.start_cap;
+    if (threadIdx.x == 0) *reinterpret_cast<int4*>(out) = make_int4(total, pieces, 0, 0);
+    for (int r = threadIdx.x; r < R; r += kCsrThreads) {
+        const int first = start[r], cnt = cursor[r] - first;
+        for (int k = 0; k < cnt; k += kPiece) {
+            const int len = min(kPiece, cnt - k);
+            out[4 + atomicAdd(&bin[len], 1)] = ((first + k) >> 2) << 17 | len << 10 | r;
+        }
+    }
 }
 
 // The backward's work line: block b contributes, per column slab, its pairs plus a fixed amount per chunk
@@ -633,6 +665,12 @@ __host__ __device__ inline int ft_bwd_unit_at(long long at, const int* block_beg
 // numbering, so that all CTAs move through the blocks together, and announces a block it has left after
 // the staging phase of its next unit, when that block's reductions have had time to land (the fence
 // that must precede the announcement then finds little to wait for).
+//
+// Staging: a pair's line takes 8 lanes (pairwise: 32 columns of each half of the accumulator) or 16 lanes, 16 bytes per
+// load.  Walk: a half warp per list piece (see sum_lines).  Pieces are handed out `grab` at a time by a shared-memory
+// counter, longest first.  Bound by the shared-memory pipe in the walk (256 bytes per (row, pair, slab)) and by load
+// latency in the staging.  (One row per warp with 8 bytes per lane, rows in table order: 2.29 against BWD_LARGE ms at 131072
+// positions and width 2048, 0.332 against BWD_MID ms at 16384.)
 template <bool PAIRWISE, int THREADS, bool SIGNAL>
 __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_tiled_kernel(FtArgs a, TileArgs t) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -640,22 +678,27 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
     constexpr int kBwdThreads = THREADS;
     constexpr int NW = kBwdThreads / 32;
     const int R = t.block_rows, CP = t.chunk_len;
-    f32x2* g_s = reinterpret_cast<f32x2*>(smem_raw);                                          // [CP + 1][32] (A, B) pairs
-    uint16_t* ent = reinterpret_cast<uint16_t*>(smem_raw + (size_t)(CP + 1) * kTileRowBytes);  // lists of the chunk
-    int* start = reinterpret_cast<int*>(ent + t.ent_cap);                                     // [R + 1]
-    int* pairs_s = start + t.start_cap;                                                       // [CP] pair ids of the chunk
-    float* bias_s = reinterpret_cast<float*>(pairs_s + CP);                                   // [nslabs][64] bias-gradient sums
-    __shared__ int next_rows;  // the walk's row counter
-    if (threadIdx.x < 32) g_s[CP * 32 + threadIdx.x] = 0;  // the all-zero line that list padding points at
-    for (int i = threadIdx.x; i < t.nslabs * kTileCols; i += kBwdThreads) bias_s[i] = 0.f;
-
+    float* g_s = reinterpret_cast<float*>(smem_raw);                                       // [CP][64] staged lines
+    uint16_t* ent = reinterpret_cast<uint16_t*>(smem_raw + (size_t)CP * kTileRowBytes);    // lists of the chunk
+    int* start = reinterpret_cast<int*>(ent + t.ent_cap);                                  // entries, pieces, -, -, then the pieces
+    int* pairs_s = start + t.start_cap;                                                    // [CP] pair ids of the chunk
+    float* bias_s = reinterpret_cast<float*>(pairs_s + CP);                                // [warps][64] bias-gradient sums of a unit
+    __shared__ int next_piece;  // the walk's counter
     const long long line = ft_bwd_line(t.block_begin, t.chunk_begin, t.first_block, t.last_block, t.nslabs);
     const int u_begin = ft_bwd_unit_at(line * blockIdx.x / gridDim.x, t.block_begin, t.chunk_begin, t.first_block, t.last_block, t.nslabs);
     const int u_end = ft_bwd_unit_at(line * (blockIdx.x + 1) / gridDim.x, t.block_begin, t.chunk_begin, t.first_block, t.last_block, t.nslabs);
 
-    // Bias gradient: a warp adds the sums of the pairs it staged to the slab's line of bias_s (shared-memory
-    // atomics); the CTA adds the lines to global memory once, at the end.
-    int col_a = 0, col_b = 0, slab = -1, block = -1, ch_loaded = -1;
+    // lanes of a warp per staged pair, and the four floats of the line that a lane holds: with pairwise the line is the 32
+    // low-half columns, then the 32 high-half ones, so that a lane of the walk owns four neighbouring columns of the table
+    constexpr int kLanes = PAIRWISE ? 8 : 16, kPairsPerWarp = 32 / kLanes;
+    const int q = lane % kLanes, sub = lane / kLanes;
+    const int l16 = lane & 15, half = lane >> 4;
+    const uint32_t lane16 = 16 * l16;
+
+    // Bias gradient: a warp leaves the sums of the pairs it staged in its line of bias_s; during the walk two warps add the
+    // lines up, a thread per column, and reduce the result to global memory.  (Shared-memory float atomics in their place
+    // took an eighth of all passes through the shared-memory pipe.)
+    int slab = -1, block = -1, ch_loaded = -1;
     int scan_block = t.first_block, scan_base = 0;  // units before scan_block
     int all_units = 0, left_block = -1;             // SIGNAL: a block this CTA has left and not yet announced
     if (SIGNAL) all_units = t.nslabs * (t.chunk_begin[t.last_block] - t.chunk_begin[t.first_block]);
@@ -666,16 +709,14 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
             scan_block++;
             nch = t.chunk_begin[scan_block + 1] - t.chunk_begin[scan_block];
         }
-        const int local = u - scan_base, new_slab = local % t.nslabs, ch = t.chunk_begin[scan_block] + local / t.nslabs;
-        if (new_slab != slab || scan_block != block) {
-            if (SIGNAL && block >= 0 && scan_block != block) {
+        const int local = u - scan_base, ch = t.chunk_begin[scan_block] + local / t.nslabs;
+        slab = local % t.nslabs;
+        if (scan_block != block) {
+            if (SIGNAL && block >= 0) {
                 if (left_block >= 0) bucket_signal(t.sig, left_block);  // (only if a whole block went by within one unit)
                 left_block = block;
             }
-            slab = new_slab;
             block = scan_block;
-            col_a = tile_col_a<PAIRWISE>(slab, lane, a.H);
-            col_b = tile_col_b<PAIRWISE>(slab, lane, a.H);
         }
         const int4 chunk = t.chunks[ch];
         const int c0 = chunk.y, cn = chunk.z;
@@ -683,67 +724,70 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
         // overlapped with the staging below
         if (ch != ch_loaded) {
             const int* start_in = t.csr_start + (size_t)ch * t.start_cap;
-            for (int i = threadIdx.x; i < t.start_cap / 4; i += kBwdThreads) cp_async16(start + 4 * i, start_in + 4 * i);
-            const int total = __ldg(start_in + R);
+            const int4 head = __ldg(reinterpret_cast<const int4*>(start_in));
+            for (int i = threadIdx.x; i < (head.y + 7) / 4; i += kBwdThreads) cp_async16(start + 4 * i, start_in + 4 * i);
             const uint16_t* ent_in = t.csr_ent + (size_t)ch * t.ent_cap;
-            for (int i = threadIdx.x; i < (total + 7) / 8; i += kBwdThreads) cp_async16(ent + 8 * i, ent_in + 8 * i);
+            for (int i = threadIdx.x; i < (head.x + 7) / 8; i += kBwdThreads) cp_async16(ent + 8 * i, ent_in + 8 * i);
             for (int k = threadIdx.x; k < cn; k += kBwdThreads) pairs_s[k] = __ldg(t.pairs + c0 + k).x;
             ch_loaded = ch;
-            __syncthreads();  // the pair ids (and, on the first unit, the zeroed lines) are in place
+            __syncthreads();  // the pair ids are in place
         }
-        float bsum_a = 0.f, bsum_b = 0.f;
         // stage this chunk's gradients at the feature-transformer pre-activation
-        for (int pl0 = warp; pl0 < cn; pl0 += 4 * NW) {
-            float q0[4], q1[4], q2[4];
+        float4 sum_a = make_float4(0, 0, 0, 0), sum_b = sum_a;
+        const int col = PAIRWISE ? slab * 32 + 4 * q : slab * 64 + 4 * q;
+        constexpr int U = 2;  // pairs in flight per lane
+        for (int pl0 = warp * kPairsPerWarp + sub; pl0 < cn; pl0 += U * NW * kPairsPerWarp) {
+            float4 y0[U], y1[U], d[U];
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int pl = pl0 + k * NW;
-                q0[k] = q1[k] = q2[k] = 0.f;
-                if (pl < cn) {
-                    const int pair = pairs_s[pl];
-                    if (PAIRWISE) {
-                        const float* pa = a.u + (size_t)pair * a.H + col_a;
-                        const float* pb = a.u + (size_t)pair * a.H + col_b;
-                        const float* pd = a.dx + (size_t)pair * (a.H / 2) + col_a;
-                        q0[k] = t.once ? ld_once(pa) : *pa;
-                        q1[k] = t.once ? ld_once(pb) : *pb;
-                        q2[k] = t.once ? ld_once(pd) : *pd;
-                    } else {
-                        const size_t at = (size_t)pair * a.H + col_a;
-                        const float2* pd = reinterpret_cast<const float2*>(a.dx + at);
-                        const float2* py = reinterpret_cast<const float2*>(a.x + at);
-                        const float2 d = t.once ? ld_once2(pd) : *pd;
-                        const float2 y = t.once ? ld_once2(py) : *py;
-                        q0[k] = d.x * ft_act_bwd(a.act, y.x);
-                        q1[k] = d.y * ft_act_bwd(a.act, y.y);
-                    }
+            for (int k = 0; k < U; k++) {
+                const int pl = pl0 + k * NW * kPairsPerWarp;
+                if (pl >= cn) break;
+                const int pair = pairs_s[pl];
+                const float4* p0 = reinterpret_cast<const float4*>((PAIRWISE ? a.u : a.x) + (size_t)pair * a.H + col);
+                const float4* pd = reinterpret_cast<const float4*>(a.dx + (size_t)pair * (PAIRWISE ? a.H / 2 : a.H) + col);
+                y0[k] = t.once ? ld_once4(p0) : *p0;
+                if (PAIRWISE) {
+                    const float4* p1 = p0 + a.H / 8;  // (H / 2 floats on)
+                    y1[k] = t.once ? ld_once4(p1) : *p1;
                 }
+                d[k] = t.once ? ld_once4(pd) : *pd;
             }
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int pl = pl0 + k * NW;
-                if (pl < cn) {
-                    float ga = q0[k], gb = q1[k];
-                    if (PAIRWISE) {
-                        ga = (q2[k] * q1[k]) * ft_act_bwd(1, q0[k]);
-                        gb = (q2[k] * q0[k]) * ft_act_bwd(1, q1[k]);
-                    }
-                    if (PAIRWISE) {  // the line holds the 32 low-half columns, then the 32 high-half ones: a lane of the
-                                     // walk then owns two neighbouring columns of the table and reduces them at once
-                        float* gf = reinterpret_cast<float*>(g_s) + pl * kTileCols;
-                        gf[lane] = ga;
-                        gf[32 + lane] = gb;
-                    } else {
-                        g_s[pl * 32 + lane] = pack2(ga, gb);
-                    }
-                    bsum_a += ga;
-                    bsum_b += gb;
+            for (int k = 0; k < U; k++) {
+                const int pl = pl0 + k * NW * kPairsPerWarp;
+                if (pl >= cn) break;
+                float* out = g_s + pl * kTileCols + 4 * q;
+                if (PAIRWISE) {
+                    const float4 ga = make_float4((d[k].x * y1[k].x) * ft_act_bwd(1, y0[k].x), (d[k].y * y1[k].y) * ft_act_bwd(1, y0[k].y),
+                                                  (d[k].z * y1[k].z) * ft_act_bwd(1, y0[k].z), (d[k].w * y1[k].w) * ft_act_bwd(1, y0[k].w));
+                    const float4 gb = make_float4((d[k].x * y0[k].x) * ft_act_bwd(1, y1[k].x), (d[k].y * y0[k].y) * ft_act_bwd(1, y1[k].y),
+                                                  (d[k].z * y0[k].z) * ft_act_bwd(1, y1[k].z), (d[k].w * y0[k].w) * ft_act_bwd(1, y1[k].w));
+                    *reinterpret_cast<float4*>(out) = ga;
+                    *reinterpret_cast<float4*>(out + 32) = gb;
+                    sum_a = add4(sum_a, ga);
+                    sum_b = add4(sum_b, gb);
+                } else {
+                    const float4 ga = make_float4(d[k].x * ft_act_bwd(a.act, y0[k].x), d[k].y * ft_act_bwd(a.act, y0[k].y),
+                                                  d[k].z * ft_act_bwd(a.act, y0[k].z), d[k].w * ft_act_bwd(a.act, y0[k].w));
+                    *reinterpret_cast<float4*>(out) = ga;
+                    sum_a = add4(sum_a, ga);
                 }
             }
         }
-        if (threadIdx.x == 0) next_rows = 0;
-        if (bsum_a != 0.f) atomicAdd(bias_s + slab * kTileCols + lane, bsum_a);
-        if (bsum_b != 0.f) atomicAdd(bias_s + slab * kTileCols + 32 + lane, bsum_b);
+        if (threadIdx.x == 0) next_piece = 0;
+#pragma unroll
+        for (int o = kLanes; o < 32; o <<= 1) {
+            sum_a = add4(sum_a, make_float4(__shfl_xor_sync(0xffffffffu, sum_a.x, o), __shfl_xor_sync(0xffffffffu, sum_a.y, o),
+                                            __shfl_xor_sync(0xffffffffu, sum_a.z, o), __shfl_xor_sync(0xffffffffu, sum_a.w, o)));
+            if (PAIRWISE)
+                sum_b = add4(sum_b, make_float4(__shfl_xor_sync(0xffffffffu, sum_b.x, o), __shfl_xor_sync(0xffffffffu, sum_b.y, o),
+                                                __shfl_xor_sync(0xffffffffu, sum_b.z, o), __shfl_xor_sync(0xffffffffu, sum_b.w, o)));
+        }
+        if (sub == 0) {
+            float* b = bias_s + warp * kTileCols + 4 * q;
+            *reinterpret_cast<float4*>(b) = sum_a;
+            if (PAIRWISE) *reinterpret_cast<float4*>(b + 32) = sum_b;
+        }
         cp_async_wait_all();
         __syncthreads();
         if (SIGNAL && left_block >= 0) {
@@ -752,7 +796,7 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
         }
         // The next unit of a CTA that walks consecutive units is the same chunk's next slab: ask L2 for the lines
         // its staging will read (the neighbours of the ones just staged) now, so that they arrive during the walk.
-        if (!SIGNAL && t.once && new_slab + 1 < t.nslabs && u + 1 < u_end && (int)threadIdx.x < cn) {
+        if (!SIGNAL && t.once && slab + 1 < t.nslabs && u + 1 < u_end && (int)threadIdx.x < cn) {
             const int pair = pairs_s[threadIdx.x];
             if (PAIRWISE) {
                 const float* pu = a.u + (size_t)pair * a.H + (slab + 1) * 32;
@@ -767,41 +811,31 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
                 prefetch_l2(a.x + at + 32);
             }
         }
-        // accumulate: each warp walks the lists of the rows it owns, four entries per 8-byte load
-        const unsigned char* gl = smem_raw + lane * 8;
-        // the two table columns this lane sums (see the staging above for the pairwise layout of a line)
-        const int col_w = !PAIRWISE ? col_a : lane < 16 ? slab * 32 + 2 * lane : a.H / 2 + slab * 32 + 2 * (lane - 16);
-        // rows are handed out a few at a time to whichever warp is free: list lengths differ a lot from row to row
+        // the four table columns this lane sums
+        const int col_w = !PAIRWISE ? slab * 64 + 4 * l16 : l16 < 8 ? slab * 32 + 4 * l16 : a.H / 2 + slab * 32 + 4 * (l16 - 8);
+        float* g_block = a.g_table + (size_t)block * R * a.H + col_w;
+        if (threadIdx.x >= kBwdThreads - kTileCols) {
+            const int j = (int)threadIdx.x - (kBwdThreads - kTileCols);
+            float sum = 0.f;
+#pragma unroll 8
+            for (int w = 0; w < NW; w++) sum += bias_s[w * kTileCols + j];
+            if (sum != 0.f) atomicAdd(a.g_bias + (!PAIRWISE ? slab * 64 + j : j < 32 ? slab * 32 + j : a.H / 2 + slab * 32 + j - 32), sum);
+        }
+        const int pieces = start[1];
         for (;;) {
-            int row2 = 0;
-            if (lane == 0) row2 = atomicAdd(&next_rows, t.grab);
-            row2 = __shfl_sync(0xffffffffu, row2, 0);
-            if (row2 >= R) break;
-            for (int row = row2; row < min(R, row2 + t.grab); row++) {
-            const unsigned sl = (unsigned)start[row];
-            const int len = (int)(sl & 0xffffu);
-            const uint2* lp = reinterpret_cast<const uint2*>(ent + (sl >> 16) * 8);
-            f32x2 acc = 0;
-            uint2 g = lp[0];  // (reads beyond a list's end stay inside the entry array, which has room to spare, and are never used)
-            for (int k = 0; k < len; k += 4) {
-                const uint2 g_ahead = lp[(k >> 2) + 1];  // the next four entries, before the current four lines are added
-                const f32x2 v0 = line_at(gl, g.x & 0xffffu), v1 = line_at(gl, g.x >> 16);
-                const f32x2 v2 = line_at(gl, g.y & 0xffffu), v3 = line_at(gl, g.y >> 16);
-                acc = add2(add2(add2(add2(acc, v0), v1), v2), v3);
-                g = g_ahead;
-            }
-            float* dst = a.g_table + (size_t)(block * R + row) * a.H + col_w;
-            const float ga = lo2(acc), gb = hi2(acc);
-            if (ga != 0.f || gb != 0.f) atomicAdd(reinterpret_cast<float2*>(dst), make_float2(ga, gb));
+            int first = 0;
+            if (lane == 0) first = atomicAdd(&next_piece, t.grab);
+            first = __shfl_sync(0xffffffffu, first, 0);
+            if (first >= pieces) break;
+            for (int p = first + half; p < min(pieces, first + t.grab); p += 2) {
+                const unsigned piece = (unsigned)start[4 + p];
+                const f32x4 acc = sum_lines(smem_raw, reinterpret_cast<const uint2*>(ent) + (piece >> 17), (int)(piece >> 10) & 0x7f, lane16);
+                const float4 g = make_float4(lo2(acc.a), hi2(acc.a), lo2(acc.b), hi2(acc.b));
+                if (g.x != 0.f || g.y != 0.f || g.z != 0.f || g.w != 0.f)
+                    atomicAdd(reinterpret_cast<float4*>(g_block + (size_t)(piece & 0x3ffu) * a.H), g);
             }
         }
         __syncthreads();
-    }
-    // entry [slab][j] holds, for j < 32, lane j's first column of that slab, for j >= 32 lane (j - 32)'s second
-    for (int i = threadIdx.x; i < t.nslabs * kTileCols; i += kBwdThreads) {
-        const float v = bias_s[i];
-        const int sl = i / kTileCols, j = i % kTileCols;
-        if (v != 0.f) atomicAdd(a.g_bias + (j < 32 ? tile_col_a<PAIRWISE>(sl, j, a.H) : tile_col_b<PAIRWISE>(sl, j - 32, a.H)), v);
     }
     if (SIGNAL && left_block >= 0) bucket_signal(t.sig, left_block);
     if (SIGNAL && block >= 0) bucket_signal(t.sig, block);

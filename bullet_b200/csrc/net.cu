@@ -335,7 +335,7 @@ int launch_ft_forward(b200_net* net, const b200::FtArgs& a, const b200::TileArgs
 template <bool PW>
 int launch_ft_backward(b200_net* net, const b200::FtArgs& a, const b200::TileArgs& t, bool tiled, int grid) {
     if (tiled) {
-        const size_t smem = b200::ft_bwd_smem(t.block_rows, a.nnz, t.chunk_len, t.nslabs);
+        const size_t smem = b200::ft_bwd_smem(t.block_rows, a.nnz, t.chunk_len);
         const bool wide = t.chunk_len > b200::ft_bwd_chunk(a.nnz, false);
 // data-parallel runs that announce finished row blocks take an instantiation of their own: the
         // fence it ends with makes every CTA wait for its reductions to land (measured: +18 %)
@@ -457,7 +457,7 @@ b200::TileArgs tile_args(b200_net* net, const Slot& s, bool backward) {
     // grabs per warp and unit to even out the list lengths), two to four for the 147-row ataxx table
     t.grab = net->bwd_grab > 0 ? net->bwd_grab : std::max(2, std::min(8, net->d.ft_block_rows / 96));
     t.ent_cap = b200::ft_bwd_ent_cap(net->d.ft_block_rows, net->d.nnz, s.chunk_len);
-    t.start_cap = b200::ft_bwd_start_cap(net->d.ft_block_rows);
+    t.start_cap = b200::ft_bwd_start_cap(net->d.ft_block_rows, net->d.nnz, s.chunk_len);
     if (backward && net->sig_on) {
         t.sig.done_count = net->done_count;
         t.sig.done_expect = s.dev<int>(s.off_bexpect);
@@ -853,13 +853,13 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     }
     net->n_flat = (off + 1023) / 1024 * 1024;  // a multiple of 4 floats x 256: splits evenly over up to 256 ranks
 
-    constexpr size_t kMaxSmem = 227 * 1024;
+    constexpr size_t kMaxSmem = 227 * 1024 - 64;  // (the tiled kernels declare a few static bytes)
     net->tiled_ok = d.ft_block_rows > 0 && d.n_inputs % d.ft_block_rows == 0 && d.ft_out % b200::kTileCols == 0 &&
                     b200::ft_fwd_smem(d.ft_block_rows, (d.nnz + 7) & ~7) <= kMaxSmem &&
-                    b200::ft_bwd_smem(d.ft_block_rows, d.nnz, b200::ft_bwd_chunk(d.nnz, true), d.ft_out / b200::kTileCols) <= kMaxSmem;
+                    b200::ft_bwd_smem(d.ft_block_rows, d.nnz, b200::ft_bwd_chunk(d.nnz, true)) <= kMaxSmem && d.ft_block_rows < 1024;
     if (net->tiled_ok) {
         const int larger = b200::ft_bwd_chunk_large(d.nnz);
-        net->wide_chunk = b200::ft_bwd_smem(d.ft_block_rows, d.nnz, larger, d.ft_out / b200::kTileCols) <= kMaxSmem ? larger : b200::ft_bwd_chunk(d.nnz, true);
+        net->wide_chunk = b200::ft_bwd_smem(d.ft_block_rows, d.nnz, larger) <= kMaxSmem ? larger : b200::ft_bwd_chunk(d.nnz, true);
     }
     net->nblocks = net->tiled_ok ? d.n_inputs / d.ft_block_rows : 1;
     net->nslabs = d.ft_out / b200::kTileCols;
@@ -892,17 +892,17 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
         rc = rc ? rc : dev_alloc(net, &net->facc, (size_t)d.ft_block_rows * d.ft_out / 2);
     if (net->tiled_ok) {
         // sized for whichever backward shape needs more: every block may end in a partly filled chunk
-        size_t ent_total = 0, chunks_total = 0;
+        size_t ent_total = 0, start_total = 0;
         for (int shape = 0; shape < 3; shape++) {
             const int cp = shape == 2 ? net->wide_chunk : b200::ft_bwd_chunk(d.nnz, shape != 0);
             const size_t chunks = most_chunks(net, (int)B, cp);
-            chunks_total = std::max(chunks_total, chunks);
+            start_total = std::max(start_total, chunks * b200::ft_bwd_start_cap(d.ft_block_rows, d.nnz, cp));
             ent_total = std::max(ent_total, chunks * b200::ft_bwd_ent_cap(d.ft_block_rows, d.nnz, cp));
         }
         for (auto& s : net->slots) {
             rc = rc ? rc : dev_alloc(net, &s.lists, 2 * B * ((d.nnz + 7) & ~7));
             rc = rc ? rc : dev_alloc(net, &s.csr_ent, ent_total);
-            rc = rc ? rc : dev_alloc(net, &s.csr_start, chunks_total * b200::ft_bwd_start_cap(d.ft_block_rows));
+            rc = rc ? rc : dev_alloc(net, &s.csr_start, start_total);
         }
     }
     if (rc) return bail(rc);
