@@ -81,7 +81,6 @@ struct TileArgs {
     uint16_t* csr_ent;             // [nchunks][ent_cap] pairs of the chunk grouped by row, every list starting on 16 bytes
     int* csr_start;                // [nchunks][start_cap] per row (start / 8) << 16 | length; [R] = entries in all
     int ent_cap, start_cap;
-    int once;                      // table rows and activations through loads that claim no L1 line
     int grab;                      // rows a warp of the backward takes from the row counter at a time
     int chunk_len;  // CP: most pairs per chunk
     // backward only, data-parallel runs: the last CTA of every row block tells all ranks that the block's
@@ -398,31 +397,34 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
         const int last = (int)min((long long)in_block, first + (v_end - v));
         v += last - first;
         __syncthreads();  // every warp has left the previous tile
-        {   // fill the tile: 8 work items per row, each 8 floats of the row
+        {   // fill the tile: eight threads per row, each two 16-byte pieces that its neighbours continue
             // with a factoriser the table row is l0w[row] + l0f[row mod factor_rows], one fp32 add per
             // element exactly as the reference forms `l0w + l0f.repeat(n)` (model/builder.rs:421-424)
             const float* src = a.table + (size_t)block * R * a.H;
+            const int q = threadIdx.x & 7, c0 = PAIRWISE ? slab * 32 + q * 4 : slab * 64 + q * 4, c1 = PAIRWISE ? a.H / 2 + c0 : c0 + 32;
 #pragma unroll 3
-            for (int i = threadIdx.x; i < R * 8; i += kFwdThreads) {
-                const int row = i >> 3, q = i & 7;
-                float4* dst = reinterpret_cast<float4*>(tile + row * kTileCols + q * 8);
-                const float* frow = a.factor ? a.factor + (size_t)((block * R + row) % a.factor_rows) * a.H : nullptr;
-                // with pairwise the tile row holds (low-half column, its high-half partner) side by side, both factors of
-                // one product.  (The work items of a row lie 32 bytes apart: the upper four of a row store their second half
-                // first, so that the eight 16-byte stores of a quarter warp fall into eight different bank groups)
-                const int c0 = PAIRWISE ? slab * 32 + q * 4 : slab * 64 + q * 8, c1 = PAIRWISE ? a.H / 2 + c0 : c0 + 4;
-                const float4* p0 = reinterpret_cast<const float4*>(src + (size_t)row * a.H + c0);
-                const float4* p1 = reinterpret_cast<const float4*>(src + (size_t)row * a.H + c1);
-                float4 v0 = t.once ? ld_once4(p0) : __ldg(p0), v1 = t.once ? ld_once4(p1) : __ldg(p1);
-                if (frow) {
-                    v0 = add4(v0, __ldg(reinterpret_cast<const float4*>(frow + c0)));  // (these gain from L1)
+            for (int row = threadIdx.x >> 3; row < R; row += kFwdThreads / 8) {
+                float4* dst = reinterpret_cast<float4*>(tile + row * kTileCols);
+                float4 v0 = ld_once4(reinterpret_cast<const float4*>(src + (size_t)row * a.H + c0));
+                float4 v1 = ld_once4(reinterpret_cast<const float4*>(src + (size_t)row * a.H + c1));
+                if (a.factor) {
+                    const float* frow = a.factor + (size_t)((block * R + row) % a.factor_rows) * a.H;
+                    v0 = add4(v0, __ldg(reinterpret_cast<const float4*>(frow + c0)));
                     v1 = add4(v1, __ldg(reinterpret_cast<const float4*>(frow + c1)));
                 }
-                const int h = q >> 2;
-                const float4 first4 = PAIRWISE ? make_float4(v0.x, v1.x, v0.y, v1.y) : v0;
-                const float4 second4 = PAIRWISE ? make_float4(v0.z, v1.z, v0.w, v1.w) : v1;
-                dst[h] = h ? second4 : first4;
-                dst[h ^ 1] = h ? first4 : second4;
+                if (PAIRWISE) {
+                    // the tile row holds (low-half column, its high-half partner) side by side, both factors of one product.
+                    // (A thread's pieces lie next to each other, 32 bytes from its neighbour's: the upper four threads of a
+                    // row store their second piece first, so that the eight stores of a quarter warp fall into eight
+                    // different bank groups)
+                    const int h = q >> 2;
+                    const float4 first4 = make_float4(v0.x, v1.x, v0.y, v1.y), second4 = make_float4(v0.z, v1.z, v0.w, v1.w);
+                    dst[2 * q + h] = h ? second4 : first4;
+                    dst[2 * q + (h ^ 1)] = h ? first4 : second4;
+                } else {
+                    dst[q] = v0;
+                    dst[q + 8] = v1;
+                }
             }
         }
         // this lane's columns: two products, or four neighbours
@@ -735,7 +737,7 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
         // stage this chunk's gradients at the feature-transformer pre-activation
         float4 sum_a = make_float4(0, 0, 0, 0), sum_b = sum_a;
         const int col = PAIRWISE ? slab * 32 + 4 * q : slab * 64 + 4 * q;
-        constexpr int U = 2;  // pairs in flight per lane
+        constexpr int U = PAIRWISE ? 2 : 4;  // pairs in flight per lane
         for (int pl0 = warp * kPairsPerWarp + sub; pl0 < cn; pl0 += U * NW * kPairsPerWarp) {
             float4 y0[U], y1[U], d[U];
 #pragma unroll
@@ -745,12 +747,12 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
                 const int pair = pairs_s[pl];
                 const float4* p0 = reinterpret_cast<const float4*>((PAIRWISE ? a.u : a.x) + (size_t)pair * a.H + col);
                 const float4* pd = reinterpret_cast<const float4*>(a.dx + (size_t)pair * (PAIRWISE ? a.H / 2 : a.H) + col);
-                y0[k] = t.once ? ld_once4(p0) : *p0;
+                y0[k] = ld_once4(p0);
                 if (PAIRWISE) {
                     const float4* p1 = p0 + a.H / 8;  // (H / 2 floats on)
-                    y1[k] = t.once ? ld_once4(p1) : *p1;
+                    y1[k] = ld_once4(p1);
                 }
-                d[k] = t.once ? ld_once4(pd) : *pd;
+                d[k] = ld_once4(pd);
             }
 #pragma unroll
             for (int k = 0; k < U; k++) {
@@ -796,7 +798,7 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
         }
         // The next unit of a CTA that walks consecutive units is the same chunk's next slab: ask L2 for the lines
         // its staging will read (the neighbours of the ones just staged) now, so that they arrive during the walk.
-        if (!SIGNAL && t.once && slab + 1 < t.nslabs && u + 1 < u_end && (int)threadIdx.x < cn) {
+        if (!SIGNAL && slab + 1 < t.nslabs && u + 1 < u_end && (int)threadIdx.x < cn) {
             const int pair = pairs_s[threadIdx.x];
             if (PAIRWISE) {
                 const float* pu = a.u + (size_t)pair * a.H + (slab + 1) * 32;

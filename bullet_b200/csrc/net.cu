@@ -128,7 +128,6 @@ struct b200_net {
     bool bwd_wide = true;  // shape of the tiled backward (see ft_bwd_chunk)
     int exchange_bulk = 0;  // the peer exchange moves gradients and weights with bulk asynchronous copies (measured no faster)
     int bwd_grab = 0;  // rows a warp of the tiled backward takes from the row counter at a time (0: chosen by block size)
-    int ft_once = 1;       // bit 0: the tiled kernels read table rows and activations with loads that claim no L1 line
     int wide_chunk = 0;    // the larger chunk of the 1024-thread backward where it fits into shared memory, else the standard one
     // Pairs per chunk for a batch of n positions.  The larger chunk saves list copies, barriers and reductions,
     // but needs enough units to keep every SM's share even: measured faster from about eight units per SM.
@@ -452,7 +451,6 @@ b200::TileArgs tile_args(b200_net* net, const Slot& s, bool backward) {
     t.csr_ent = s.csr_ent;
     t.csr_start = s.csr_start;
     t.chunk_len = s.chunk_len;
-    t.once = net->ft_once;
     // rows per grab: measured best at eight for 768-row blocks (runs of neighbouring rows per warp, and still four
     // grabs per warp and unit to even out the list lengths), two to four for the 147-row ataxx table
     t.grab = net->bwd_grab > 0 ? net->bwd_grab : std::max(2, std::min(8, net->d.ft_block_rows / 96));
@@ -1068,8 +1066,7 @@ int b200_net_set_option(b200_net* net, const char* key, int64_t value) {
         return 0;
     }
     if (!strcmp(key, "ft_once")) {
-        net->ft_once = (int)value;
-        return 0;
+        return 0;  // (no load of the tiled kernels gains from an L1 line any more: one form)
     }
     if (!strcmp(key, "ft_bwd_wide")) {  // takes effect for batches uploaded afterwards
         net->bwd_wide = value != 0;

@@ -170,7 +170,6 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
     t.status = word.status;
     t.lists = g.lists;
     t.list_len = g.list_len;
-    t.once = 1;
     const size_t smem = b200::ft_fwd_smem(R, t.list_len);
     // one CTA per SM, each taking an equal piece of the (block, slab, pair) work line
     int sms = 0;

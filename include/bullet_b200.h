@@ -98,7 +98,7 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
 int b200_net_destroy(b200_net* net);
 /* Tuning switches (no counterpart in the reference; every one has a measured default):
  *   "ft_mode" / "ft_fwd_mode" / "ft_bwd_mode"  B200_FT_*; "ft_bwd_wide" 0 = two 512-thread backward CTAs per SM;
- *   "ft_once" 0 = table rows and activations through ordinary (L1-allocating) loads;
+ *   "ft_once" accepted, without effect (one form of loads is left);
  *   "ft_bwd_grab" rows a warp of the tiled backward takes from the row counter at a time (0 = by block size);
  *   "exchange_bulk" 1 = the peer exchange moves gradients and weights with bulk asynchronous copies;
  *   "overlap_ctas", "overlap_mode", "exchange_ctas", "exchange_wait_ms", "exchange_step", "manual_grad_zero": see the
