@@ -28,7 +28,7 @@
 
 #include "../../include/bullet_b200.h"
 #include "common.h"
-#include "kernels_dense.cuh"
+#include "kernels_dense_mma.cuh"
 #include "kernels_ft.cuh"
 #include "kernels_opt.cuh"
 #include "kernels_prep.cuh"
@@ -112,6 +112,7 @@ struct b200_net {
     int64_t n_flat = 0;
     float *P = nullptr, *G = nullptr, *M = nullptr, *V = nullptr, *table = nullptr;
     float *x = nullptr, *u = nullptr, *dx = nullptr, *a1 = nullptr, *a2 = nullptr, *out = nullptr, *w1g = nullptr;
+    float4 *w1f = nullptr, *w1d = nullptr;  // the first dense layer's fragment tables (dense_mma)
     float* dz[3] = {nullptr, nullptr, nullptr};
     int wgrad_per_sm = 0;          // resident CTAs per SM of the first layer's weight-gradient kernel (looked up once)
     int status_slot = -1;          // slot whose status word the running step reports (-1: the step used no tiled kernel)
@@ -207,7 +208,9 @@ struct b200_net {
     bool bwd_tiled() const { return ft_bwd_mode == B200_FT_TILED || (ft_bwd_mode == B200_FT_AUTO && tiled_ok); }
     // the register-tiled dense forward (rows per bucket in fours, more layers after the first) also
     // forms the gradients of those later layers
-    bool fused_small_grads() const { return d.dense_out[0] % 4 == 0 && d.n_dense >= 2; }
+    bool fused_small_grads() const { return dense_mma(); }
+    // first dense layers of four and more rows per bucket run on the tensor pipe
+    bool dense_mma() const { return d.dense_out[0] >= 4; }
 };
 
 namespace {
@@ -355,6 +358,13 @@ int launch_ft_backward(b200_net* net, const b200::FtArgs& a, const b200::TileArg
     return 0;
 }
 
+// the layers of fewer than four rows, which the fp32 kernels take
+#define DISPATCH_M12(m, ...)                                                  \
+    switch (m) {                                                              \
+        case 1: { constexpr int MM = 1; __VA_ARGS__; } break;                 \
+        case 2: { constexpr int MM = 2; __VA_ARGS__; } break;                 \
+        default: return b200::fail(B200_ERR_UNSUPPORTED, "rows per bucket %d", m); \
+    }
 #define DISPATCH_M(m, ...)                                                    \
     switch (m) {                                                              \
         case 1: { constexpr int MM = 1; __VA_ARGS__; } break;                 \
@@ -366,31 +376,31 @@ int launch_ft_backward(b200_net* net, const b200::FtArgs& a, const b200::TileArg
         default: return b200::fail(B200_ERR_UNSUPPORTED, "rows per bucket %d", m); \
     }
 
-// The first dense layer's forward: register-tiled when its rows per bucket come in fours and
-// more layers follow, else the dot-product kernel (single-output networks).
-template <int MM>
-constexpr bool dense_tiled() { return MM % 4 == 0; }
-
 template <int MM>
 void launch_dense_forward(b200_net* net, const b200::DenseArgs& da, int ntiles) {
-    if constexpr (dense_tiled<MM>()) {
-        if (da.n_dense >= 2) {
-            b200::dense_forward_tile_kernel<MM><<<ntiles, 256, b200::dense_fwd_tile_smem<MM>(), net->stream>>>(da);
-            return;
-        }
-    }
-    b200::dense_forward_kernel<MM><<<ntiles, 256, b200::dense_fwd_smem<MM>(), net->stream>>>(da);
+    if constexpr (MM >= 4)
+        b200::dense_forward_mma_kernel<MM><<<ntiles, 256, b200::dense_mma_smem<MM>(), net->stream>>>(da);
+    else
+        b200::dense_forward_kernel<MM><<<ntiles, 256, b200::dense_fwd_smem<MM>(), net->stream>>>(da);
+}
+template <int MM>
+void launch_wgrad_mma(b200_net* net, const b200::DenseArgs& a, float* gW, float* gB, dim3 grid, int threads, int per_run) {
+    if constexpr (MM >= 4) b200::dense_wgrad_mma_kernel<MM><<<grid, threads, 0, net->stream>>>(a, gW, gB, per_run);
+}
+template <int MM>
+void launch_dense_dx(b200_net* net, const b200::DenseArgs& da, int ntiles) {
+    if constexpr (MM >= 4)
+        b200::dense_dx_mma_kernel<MM><<<ntiles, 256, 0, net->stream>>>(da, net->dx);
+    else
+        b200::dense_dx_kernel<MM><<<ntiles, 256, 0, net->stream>>>(da, net->dx);
 }
 
 template <int MM>
 cudaError_t set_dense_forward_smem() {
-    if constexpr (dense_tiled<MM>()) {
-        cudaError_t e = cudaFuncSetAttribute(b200::dense_forward_tile_kernel<MM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)b200::dense_fwd_tile_smem<MM>());
-        if (e != cudaSuccess) return e;
-    }
-    return cudaFuncSetAttribute(b200::dense_forward_kernel<MM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)b200::dense_fwd_smem<MM>());
+    if constexpr (MM >= 4)
+        return b200::allow_smem(b200::dense_forward_mma_kernel<MM>);
+    else
+        return b200::allow_smem(b200::dense_forward_kernel<MM>);
 }
 
 // Most chunks that a batch of n positions can be cut into: every block may end in a partly filled one.
@@ -489,6 +499,8 @@ b200::DenseArgs dense_args(b200_net* net, const Slot& s, bool want_grad) {
     a.tiles = d.n_out_buckets > 1 ? s.dev<int2>(s.off_dtiles) : nullptr;
     a.ntiles = s.n_dtiles;
     a.W1g = net->w1g;
+    a.W1f = net->w1f;
+    a.W1d = net->w1d;
     a.a1 = net->a1;
     a.a2 = net->a2;
     a.out = net->out;
@@ -519,8 +531,15 @@ int refresh_table(b200_net* net, int n) {
     }
     if (net->w1_dirty) {
         const Tensor* w1 = net->find("l1w");
-        b200::dense_regroup_kernel<<<std::min<int>(net->sm_count * 4, (int)((w1->n + 255) / 256)), 256, 0, net->stream>>>(
-            net->P + w1->off, net->w1g, net->D1(), net->d.n_out_buckets, net->d.dense_out[0]);
+        const int O = net->d.n_out_buckets, M1 = net->d.dense_out[0];
+        if (net->dense_mma()) {
+            const int lanes = (int)(b200::mma_table_floats(net->D1(), O, M1) / 8);
+            b200::dense_fragments_kernel<<<std::min(net->sm_count * 4, (lanes + 255) / 256), 256, 0, net->stream>>>(
+                net->P + w1->off, net->w1f, net->w1d, net->D1(), O, M1, M1 >= 8 ? M1 / 8 : 1);
+        } else {
+            b200::dense_regroup_kernel<<<std::min<int>(net->sm_count * 4, (int)((w1->n + 255) / 256)), 256, 0, net->stream>>>(
+                net->P + w1->off, net->w1g, net->D1(), O, M1);
+        }
         LAUNCHED(net);
         net->w1_dirty = false;
     }
@@ -664,21 +683,28 @@ int forward_part(b200_net* net, Slot& s, bool want_grad) {
     return forward_dense(net, s, want_grad);
 }
 
-int launch_wgrad(b200_net* net, const Slot& s, int layer) {
+int launch_wgrad(b200_net* net, const Slot& s) {
     const b200_net_desc& d = net->d;
+    float *gW = net->G + net->find("l1w")->off, *gB = net->G + net->find("l1b")->off;
+    if (net->dense_mma()) {
+        const b200::DenseArgs a = dense_args(net, s, true);
+        const int warps = std::min(8, (a.K1 + b200::kWgradCols - 1) / b200::kWgradCols), gx = (a.K1 + warps * b200::kWgradCols - 1) / (warps * b200::kWgradCols);
+        const int runs = std::max(1, std::min(s.n_dtiles, 2 * net->sm_count * 8 / warps / gx)), per_run = (s.n_dtiles + runs - 1) / runs;
+        const dim3 grid(gx, (s.n_dtiles + per_run - 1) / per_run);
+        DISPATCH_M(d.dense_out[0], launch_wgrad_mma<MM>(net, a, gW, gB, grid, 32 * warps, per_run));
+        LAUNCHED(net);
+        return 0;
+    }
     b200::WgradArgs w{};
-    w.X = layer == 0 ? net->x : (layer == 1 ? net->a1 : net->a2);
-    w.dY = net->dz[layer];
+    w.X = net->x;
+    w.dY = net->dz[0];
     w.order = d.n_out_buckets > 1 ? s.dev<int>(s.off_order) : nullptr;
     w.buckets = s.dev<int>(s.off_buckets);
     w.n = s.n;
-    w.K = net->dense_in(layer);
+    w.K = net->dense_in(0);
     w.O = d.n_out_buckets;
-    char name[16];
-    snprintf(name, sizeof name, "l%dw", layer + 1);
-    w.gW = net->G + net->find(name)->off;
-    snprintf(name, sizeof name, "l%db", layer + 1);
-    w.gB = net->G + net->find(name)->off;
+    w.gW = gW;
+    w.gB = gB;
     const int groups = w.K / 4 + 1;  // four columns per thread, plus the bias
     const int threads = groups >= 128 ? 128 : ((groups + 31) / 32) * 32;
     const int gx = (groups + threads - 1) / threads;
@@ -686,7 +712,7 @@ int launch_wgrad(b200_net* net, const Slot& s, int layer) {
     // left over for another wave would double the kernel's time.
     if (!net->wgrad_per_sm) {
         int per_sm = 0;
-        DISPATCH_M(d.dense_out[layer], cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, b200::dense_wgrad_kernel<MM>, threads, 0));
+        DISPATCH_M12(d.dense_out[0], cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, b200::dense_wgrad_kernel<MM>, threads, 0));
         net->wgrad_per_sm = std::max(1, per_sm);
     }
     const int slots = net->wgrad_per_sm * net->sm_count;
@@ -695,7 +721,7 @@ int launch_wgrad(b200_net* net, const Slot& s, int layer) {
     w.chunk_len = (s.n + chunks - 1) / chunks;
     chunks = (s.n + w.chunk_len - 1) / w.chunk_len;
     dim3 grid(gx, chunks);
-    DISPATCH_M(d.dense_out[layer], b200::dense_wgrad_kernel<MM><<<grid, threads, 0, net->stream>>>(w));
+    DISPATCH_M12(d.dense_out[0], b200::dense_wgrad_kernel<MM><<<grid, threads, 0, net->stream>>>(w));
     LAUNCHED(net);
     return 0;
 }
@@ -727,7 +753,7 @@ int launch_dense_grads(b200_net* net, Slot& s) {
         b200::dense_small_grads_kernel<<<s.n_dtiles, 256, 0, net->stream>>>(g);
         LAUNCHED(net);
     }
-    return launch_wgrad(net, s, 0);
+    return launch_wgrad(net, s);
 }
 
 // With lazy module loading (the CUDA default) a kernel's code reaches the GPU at its first launch, and
@@ -742,16 +768,16 @@ bool load_kernel(K* kernel) {
 
 template <int MM>
 bool load_dense_kernels() {
-    bool ok = load_kernel(b200::dense_forward_kernel<MM>) && load_kernel(b200::dense_dx_kernel<MM>) && load_kernel(b200::dense_wgrad_kernel<MM>);
-    if constexpr (dense_tiled<MM>()) ok = ok && load_kernel(b200::dense_forward_tile_kernel<MM>);
-    return ok;
+    if constexpr (MM >= 4)
+        return load_kernel(b200::dense_forward_mma_kernel<MM>) && load_kernel(b200::dense_dx_mma_kernel<MM>) && load_kernel(b200::dense_wgrad_mma_kernel<MM>);
+    else
+        return load_kernel(b200::dense_forward_kernel<MM>) && load_kernel(b200::dense_dx_kernel<MM>) && load_kernel(b200::dense_wgrad_kernel<MM>);
 }
 
 int preload_kernels(b200_net* net) {
     bool ok = true;
     DISPATCH_M(net->d.dense_out[0], ok = load_dense_kernels<MM>());
-    for (int l = 1; l < net->d.n_dense; l++) DISPATCH_M(net->d.dense_out[l], ok = ok && load_kernel(b200::dense_wgrad_kernel<MM>));
-    ok = ok && load_kernel(b200::dense_regroup_kernel) && load_kernel(b200::dense_small_grads_kernel);
+    ok = ok && load_kernel(b200::dense_regroup_kernel) && load_kernel(b200::dense_fragments_kernel) && load_kernel(b200::dense_small_grads_kernel);
     ok = ok && load_kernel(b200::ft_forward_gather_kernel<true>) && load_kernel(b200::ft_forward_gather_kernel<false>);
     ok = ok && load_kernel(b200::ft_backward_gather_kernel<true>) && load_kernel(b200::ft_backward_gather_kernel<false>);
     ok = ok && load_kernel(b200::ft_forward_tiled_kernel<true>) && load_kernel(b200::ft_forward_tiled_kernel<false>);
@@ -877,7 +903,13 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     for (int l = 0; l < 3; l++) rc = rc ? rc : dev_alloc(net, &net->dz[l], B * 32);
     rc = rc ? rc : dev_alloc(net, &net->out, B);
     rc = rc ? rc : dev_alloc(net, &net->d_status, b200_net::kLossRing);
-    rc = rc ? rc : dev_alloc(net, &net->w1g, (size_t)d.n_out_buckets * d.dense_out[0] * net->D1());
+    if (net->dense_mma()) {
+        const size_t table = b200::mma_table_floats(net->D1(), d.n_out_buckets, d.dense_out[0]) / 4;
+        rc = rc ? rc : dev_alloc(net, &net->w1f, table);
+        rc = rc ? rc : dev_alloc(net, &net->w1d, table);
+    } else {
+        rc = rc ? rc : dev_alloc(net, &net->w1g, (size_t)d.n_out_buckets * d.dense_out[0] * net->D1());
+    }
     // the fence counters get an allocation of their own size class (2 MiB), so that its IPC handle maps exactly it
     rc = rc ? rc : dev_alloc(net, &net->xch_flags, (size_t)(2 << 20) / sizeof(int));
     if (!rc) cudaMemsetAsync(net->xch_flags, 0, (size_t)2 << 20, net->stream);
@@ -1457,7 +1489,7 @@ int b200_backward_begin(b200_net* net, int slot) {
         if (int rc = build_csr(net, s, net->stream)) return rc;
     {
         b200::DenseArgs da = dense_args(net, s, true);
-        DISPATCH_M(d.dense_out[0], b200::dense_dx_kernel<MM><<<s.n_dtiles, 256, 0, net->stream>>>(da, net->dx));
+        DISPATCH_M(d.dense_out[0], launch_dense_dx<MM>(net, da, s.n_dtiles));
         LAUNCHED(net);
     }
     if (int rc = launch_dense_grads(net, s)) return rc;
