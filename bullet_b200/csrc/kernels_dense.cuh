@@ -40,6 +40,7 @@ struct DenseArgs {
     float* out_host;   // the same in pinned host memory, or null
     float* loss;       // scalar, accumulated
     int want_grad;
+    unsigned long long* stamp;  // as in FtArgs
     // the register-tiled forward also forms the weight and bias gradients of the layers after the
     // first (it holds everything they need in shared memory): gradient tensors of layers 2 and 3
     int fuse_small;
@@ -140,6 +141,7 @@ __host__ __device__ constexpr size_t dense_fwd_smem() {
 
 template <int M1>
 __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_forward_kernel(DenseArgs a) {
+    step_begin(a.stamp);
     constexpr int P = kDenseWarpPos, MP = dense_col_stride<M1>();
     constexpr int kStageFloats = kDenseChunk * MP + kDenseTile * kDenseChunk;
     extern __shared__ __align__(16) float dense_smem[];
@@ -285,6 +287,7 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_forward_kernel(D
 // selected rows).  Same tiling and weight staging as the forward; grid = ntiles, block = 256.
 template <int M1>
 __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_dx_kernel(DenseArgs a, float* dx) {
+    step_begin(a.stamp);
     constexpr int P = kDenseWarpPos, MP = dense_col_stride<M1>();
     __shared__ __align__(16) float wbuf[2][kDenseChunk * MP];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -349,6 +352,7 @@ struct WgradArgs {
 
 template <int M>
 __global__ void __launch_bounds__(128) dense_wgrad_kernel(WgradArgs a) {
+    step_begin(nullptr);
     constexpr int S = 64;  // positions staged per round
     __shared__ int s_pos[S], s_bucket[S];
     __shared__ __align__(16) float s_dy[S][M];
@@ -447,6 +451,7 @@ struct SmallGradArgs {
 };
 
 static __global__ void __launch_bounds__(256) dense_small_grads_kernel(SmallGradArgs a) {
+    step_begin(nullptr);
     __shared__ float s_x[32][33], s_dy[32][33];
     __shared__ int s_pos[32];
     const int2 t = dense_tile_at(a.tiles, blockIdx.x, a.n);

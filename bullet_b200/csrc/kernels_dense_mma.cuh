@@ -82,6 +82,7 @@ __host__ __device__ constexpr size_t dense_mma_smem() { return (size_t)8 * kDens
 
 template <int M1>
 __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_forward_mma_kernel(DenseArgs a) {
+    step_begin(a.stamp);
     constexpr int NT = mma_tiles<M1>();
     extern __shared__ __align__(16) float dense_smem[];
     __shared__ float s_w2[M1][33], s_b2[32], s_w3[32], s_a1[kDenseTile][M1], loss_part[8];
@@ -280,6 +281,7 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_forward_mma_kern
 // grid = ntiles, block = 256.
 template <int M1>
 __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_dx_mma_kernel(DenseArgs a, float* dx) {
+    step_begin(a.stamp);
     constexpr int NT = mma_tiles<M1>();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
     const int2 t = dense_tile_at(a.tiles, blockIdx.x, a.n);
@@ -351,6 +353,7 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_dx_mma_kernel(De
 constexpr int kWgradCols = 64;
 template <int M1>
 __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_wgrad_mma_kernel(DenseArgs a, float* gW, float* gB, int tiles_per_run) {
+    step_begin(nullptr);
     constexpr int MT = M1 > 16 ? M1 / 16 : 1;
     __shared__ int s_pos[kDenseTile];
     __shared__ uint32_t s_hi[kDenseTile][M1 + 1], s_lo[kDenseTile][M1 + 1];

@@ -24,6 +24,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch.cuh"
 #include "peer_flags.cuh"
 
 namespace b200 {
@@ -52,10 +53,26 @@ struct FtArgs {
     int n, nnz, H, n_inputs, act;
     float* x;         // dense-stack input: [n][2H], or [n][H] with pairwise
     float* u;         // pairwise only: crelu outputs [n][2][H]
-    const float* dx;  // backward: gradient at x
+    const float* dx;  // backward: gradient at x, or (null) what it is the product of, for networks whose only dense layer is
+    const float* w1;          // one row per output bucket: the layer's weights [bucket][K1],
+    const float* dout;        // [n] the loss gradient at the output
+    const int* out_bucket;    // [n] and the bucket
     float* g_table;   // backward: [n_inputs][H] gradient of the table
     float* g_bias;    // backward: [H]
+    unsigned long long* stamp;  // of a step that keeps its own time: where the kernel's start goes
+    unsigned long long* stamp_end;  // forward: the step's last stamp, cleared
+    float4* zero;     // forward: the gradient buffer, where this kernel clears it (zero4 float4s), or null
+    long long zero4;
 };
+
+__device__ __forceinline__ void ft_step_begin(const FtArgs& a) {
+    step_begin(a.stamp);
+    if (a.stamp_end && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) *a.stamp_end = 0;
+    if (a.zero) {  // nothing adds to it before the kernels that follow
+        const long long per = (long long)gridDim.x * gridDim.y * blockDim.x;
+        for (long long i = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < a.zero4; i += per) a.zero[i] = make_float4(0, 0, 0, 0);
+    }
+}
 
 struct TileArgs {
     int block_rows;          // R
@@ -105,6 +122,8 @@ __device__ __forceinline__ float ft_act_bwd(int act, float y) {
 
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
+__device__ __forceinline__ float4 scale4(float4 v, float f) { return make_float4(v.x * f, v.y * f, v.z * f, v.w * f); }
+
 __device__ __forceinline__ void load_slots(const uint16_t* list, int nnz, int lane, uint32_t& s0, uint32_t& s1) {
     s0 = lane < nnz ? list[lane] : kNoFeature;
     s1 = lane + 32 < nnz ? list[lane + 32] : kNoFeature;
@@ -118,6 +137,7 @@ __device__ __forceinline__ void load_slots(const uint16_t* list, int nnz, int la
 // factoriser the two rows of a feature are added as they arrive, so a small batch does not merge the table first.
 template <bool PAIRWISE>
 __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pairs_per_block) {
+    ft_step_begin(a);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int unit = PAIRWISE ? a.H / 2 : a.H;
     const int col = blockIdx.y * 128 + lane * 4;
@@ -212,8 +232,9 @@ __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pa
 // --------------------------------------------------------------- gather backward
 // Same decomposition.  The table gradient must be zero on entry; gradients are
 // added with 128-bit global reductions, the bias gradient once per lane per block.
-template <bool PAIRWISE>
+template <bool PAIRWISE, bool ONE>
 __global__ void __launch_bounds__(256) ft_backward_gather_kernel(FtArgs a, int pairs_per_block) {
+    step_begin(a.stamp);
     __shared__ float4 red[2][8][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int unit = PAIRWISE ? a.H / 2 : a.H;
@@ -224,12 +245,14 @@ __global__ void __launch_bounds__(256) ft_backward_gather_kernel(FtArgs a, int p
     for (int pair = blockIdx.x * pairs_per_block + warp; pair < pair_end; pair += 8) {
         const int b = pair >> 1, p = pair & 1;
         float4 glo = make_float4(0, 0, 0, 0), ghi = glo;
+        const float dout = ONE ? a.dout[b] : 0.f;
+        const float* w1 = ONE ? a.w1 + (size_t)a.out_bucket[b] * 2 * unit + p * unit + col : nullptr;
         if (active) {
             if (PAIRWISE) {
                 const float* up = a.u + (size_t)pair * a.H;
                 const float4 ul = *reinterpret_cast<const float4*>(up + col);
                 const float4 uh = *reinterpret_cast<const float4*>(up + unit + col);
-                const float4 d = *reinterpret_cast<const float4*>(a.dx + (size_t)b * a.H + (size_t)p * unit + col);
+                const float4 d = ONE ? scale4(__ldg(reinterpret_cast<const float4*>(w1)), dout) : *reinterpret_cast<const float4*>(a.dx + (size_t)b * a.H + (size_t)p * unit + col);
                 glo = make_float4((d.x * uh.x) * ft_act_bwd(1, ul.x), (d.y * uh.y) * ft_act_bwd(1, ul.y),
                                   (d.z * uh.z) * ft_act_bwd(1, ul.z), (d.w * uh.w) * ft_act_bwd(1, ul.w));
                 ghi = make_float4((d.x * ul.x) * ft_act_bwd(1, uh.x), (d.y * ul.y) * ft_act_bwd(1, uh.y),
@@ -237,7 +260,7 @@ __global__ void __launch_bounds__(256) ft_backward_gather_kernel(FtArgs a, int p
             } else {
                 const size_t at = (size_t)b * 2 * a.H + (size_t)p * a.H + col;
                 const float4 y = *reinterpret_cast<const float4*>(a.x + at);
-                const float4 d = *reinterpret_cast<const float4*>(a.dx + at);
+                const float4 d = ONE ? scale4(__ldg(reinterpret_cast<const float4*>(w1)), dout) : *reinterpret_cast<const float4*>(a.dx + at);
                 glo = make_float4(d.x * ft_act_bwd(a.act, y.x), d.y * ft_act_bwd(a.act, y.y),
                                   d.z * ft_act_bwd(a.act, y.z), d.w * ft_act_bwd(a.act, y.w));
             }
@@ -366,6 +389,7 @@ __host__ __device__ inline size_t ft_fwd_smem(int R, int list_len) {
 
 template <bool PAIRWISE>
 __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs a, TileArgs t) {
+    ft_step_begin(a);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int NW = kFwdThreads / 32;
@@ -507,8 +531,8 @@ __host__ __device__ inline int ft_bwd_ent_cap(int R, int nnz, int cp) { return (
 // per chunk: entries, pieces, two unused words, then the pieces: first entry / 4 << 17 | length << 10 | row
 __host__ __device__ inline int ft_bwd_start_cap(int R, int nnz, int cp) { return (4 + R + cp * nnz / kPiece + 3) & ~3; }
 __host__ __device__ inline size_t ft_bwd_smem(int R, int nnz, int cp) {
-    return (size_t)cp * kTileRowBytes + (size_t)ft_bwd_ent_cap(R, nnz, cp) * 2 + (size_t)ft_bwd_start_cap(R, nnz, cp) * 4 + (size_t)cp * 4 +
-           32 * kTileRowBytes;  // staged lines, row lists, their pieces, pair ids, bias-gradient sums per warp
+    return (size_t)cp * kTileRowBytes + (size_t)ft_bwd_ent_cap(R, nnz, cp) * 2 + (size_t)ft_bwd_start_cap(R, nnz, cp) * 4 + (size_t)cp * 12 +
+           32 * kTileRowBytes;  // staged lines, row lists, their pieces, what a pair needs, bias-gradient sums per warp
 }
 __host__ __device__ inline size_t ft_csr_smem(int R, int nnz, int cp) {
     return (size_t)ft_bwd_ent_cap(R, nnz, cp) * 2 + (size_t)(2 * (R + 2) + 32 + 2 * (kPiece + 2) + cp) * 4;
@@ -673,8 +697,9 @@ __host__ __device__ inline int ft_bwd_unit_at(long long at, const int* block_beg
 // counter, longest first.  Bound by the shared-memory pipe in the walk (256 bytes per (row, pair, slab)) and by load
 // latency in the staging.  (One row per warp with 8 bytes per lane, rows in table order: 2.29 against BWD_LARGE ms at 131072
 // positions and width 2048, 0.332 against BWD_MID ms at 16384.)
-template <bool PAIRWISE, int THREADS, bool SIGNAL>
+template <bool PAIRWISE, int THREADS, bool SIGNAL, bool ONE>
 __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_tiled_kernel(FtArgs a, TileArgs t) {
+    step_begin(a.stamp);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     constexpr int kBwdThreads = THREADS;
@@ -685,6 +710,7 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
     int* start = reinterpret_cast<int*>(ent + t.ent_cap);                                  // entries, pieces, -, -, then the pieces
     int* pairs_s = start + t.start_cap;                                                    // [CP] pair ids of the chunk
     float* bias_s = reinterpret_cast<float*>(pairs_s + CP);                                // [warps][64] bias-gradient sums of a unit
+    int2* one_s = reinterpret_cast<int2*>(bias_s + NW * kTileCols);                        // ONE: [CP] (loss gradient, first weight) of the pair
     __shared__ int next_piece;  // the walk's counter
     const long long line = ft_bwd_line(t.block_begin, t.chunk_begin, t.first_block, t.last_block, t.nslabs);
     const int u_begin = ft_bwd_unit_at(line * blockIdx.x / gridDim.x, t.block_begin, t.chunk_begin, t.first_block, t.last_block, t.nslabs);
@@ -730,7 +756,14 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
             for (int i = threadIdx.x; i < (head.y + 7) / 4; i += kBwdThreads) cp_async16(start + 4 * i, start_in + 4 * i);
             const uint16_t* ent_in = t.csr_ent + (size_t)ch * t.ent_cap;
             for (int i = threadIdx.x; i < (head.x + 7) / 8; i += kBwdThreads) cp_async16(ent + 8 * i, ent_in + 8 * i);
-            for (int k = threadIdx.x; k < cn; k += kBwdThreads) pairs_s[k] = __ldg(t.pairs + c0 + k).x;
+            for (int k = threadIdx.x; k < cn; k += kBwdThreads) {
+                const int pair = __ldg(t.pairs + c0 + k).x;
+                pairs_s[k] = pair;
+                if (ONE) {
+                    const int row = PAIRWISE ? a.H / 2 : a.H;  // columns of x per perspective
+                    one_s[k] = make_int2(__float_as_int(a.dout[pair >> 1]), (2 * a.out_bucket[pair >> 1] + (pair & 1)) * row);
+                }
+            }
             ch_loaded = ch;
             __syncthreads();  // the pair ids are in place
         }
@@ -746,18 +779,20 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
                 if (pl >= cn) break;
                 const int pair = pairs_s[pl];
                 const float4* p0 = reinterpret_cast<const float4*>((PAIRWISE ? a.u : a.x) + (size_t)pair * a.H + col);
-                const float4* pd = reinterpret_cast<const float4*>(a.dx + (size_t)pair * (PAIRWISE ? a.H / 2 : a.H) + col);
+                const float4* pd = ONE ? reinterpret_cast<const float4*>(a.w1 + one_s[pl].y + col)
+                                       : reinterpret_cast<const float4*>(a.dx + (size_t)pair * (PAIRWISE ? a.H / 2 : a.H) + col);
                 y0[k] = ld_once4(p0);
                 if (PAIRWISE) {
                     const float4* p1 = p0 + a.H / 8;  // (H / 2 floats on)
                     y1[k] = ld_once4(p1);
                 }
-                d[k] = ld_once4(pd);
+                d[k] = ONE ? __ldg(pd) : ld_once4(pd);
             }
 #pragma unroll
             for (int k = 0; k < U; k++) {
                 const int pl = pl0 + k * NW * kPairsPerWarp;
                 if (pl >= cn) break;
+                if (ONE) d[k] = scale4(d[k], __int_as_float(one_s[pl].x));
                 float* out = g_s + pl * kTileCols + 4 * q;
                 if (PAIRWISE) {
                     const float4 ga = make_float4((d[k].x * y1[k].x) * ft_act_bwd(1, y0[k].x), (d[k].y * y1[k].y) * ft_act_bwd(1, y0[k].y),
@@ -804,11 +839,11 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
                 const float* pu = a.u + (size_t)pair * a.H + (slab + 1) * 32;
                 prefetch_l2(pu);
                 prefetch_l2(pu + a.H / 2);
-                prefetch_l2(a.dx + (size_t)pair * (a.H / 2) + (slab + 1) * 32);
+                if (!ONE) prefetch_l2(a.dx + (size_t)pair * (a.H / 2) + (slab + 1) * 32);
             } else {
                 const size_t at = (size_t)pair * a.H + (slab + 1) * 64;
-                prefetch_l2(a.dx + at);
-                prefetch_l2(a.dx + at + 32);
+                if (!ONE) prefetch_l2(a.dx + at);
+                if (!ONE) prefetch_l2(a.dx + at + 32);
                 prefetch_l2(a.x + at);
                 prefetch_l2(a.x + at + 32);
             }

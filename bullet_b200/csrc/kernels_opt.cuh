@@ -15,6 +15,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "bulk_copy.cuh"
+#include "launch.cuh"
 #include "peer_flags.cuh"
 
 namespace b200 {
@@ -99,6 +101,105 @@ __global__ void __launch_bounds__(256) adamw_flat_kernel(const __grid_constant__
         a.m[i] = m;
         a.v[i] = v;
     }
+}
+
+// The whole update of a single-GPU step in one launch: the factoriser's gradient (g_l0f = sum of the gradients of its copies
+// in l0w, first copy first, reduce.rs:96-120), the update of every tensor, the tables that the next forward reads instead of
+// l1w, and the step's loss and status word straight into pinned memory.  A thread that owns four columns of a factoriser row
+// owns them in all its copies: it sums their gradients while it updates them, so the table gradient is read once (the sum
+// used to be a kernel of its own that read it again).  HBM: 28 bytes per parameter.
+struct StepUpdateArgs {
+    AdamArgs adam;             // first4, total4 unused
+    float4* g;                 // gradients, writable (l0f's is formed here)
+    long long rest4;           // float4s of the buffer that are updated one by one: all, or (factoriser) those before l0w
+    int l0f_seg, l0w_seg;      // -1 without a factoriser
+    long long l0f4, l0w4, block4;
+    int copies;
+    // first dense layer: l1w's range and what is written from it
+    long long l1w4_begin, l1w4_end;
+    int K1, O, M1, tiles;      // tiles > 0: fragment tables of that many 8-row tiles, else w1g
+    float* w1g;                // [bucket][column][row]
+    float* w1f;                // kernels_dense_mma.cuh
+    float* w1d;
+    // read-back
+    const float* loss;
+    const int* status;         // null: the step used no row lists
+    float* h_loss;
+    int* h_status;
+    unsigned long long* stamps;  // [8] of this step
+};
+
+// where l1w's element `e` (column-major, rows k * M1 + r of all buckets) goes
+__device__ __forceinline__ void store_w1(const StepUpdateArgs& u, long long e, float w) {
+    const int OM = u.O * u.M1, col = (int)(e / OM), row = (int)(e - (long long)col * OM), k = row / u.M1, r = row - k * u.M1;
+    if (u.tiles == 0) {
+        u.w1g[((size_t)k * u.K1 + col) * u.M1 + r] = w;
+        return;
+    }
+    const uint32_t hi = __float_as_uint(w) + 0x1000u;  // as tf32_split
+    const float part[2] = {__uint_as_float(hi), __uint_as_float(__float_as_uint(w - __uint_as_float(hi & 0xffffe000u)) + 0x1000u)};
+    const int groups = (u.K1 + 15) / 16, c = col & 15, tile = r >> 3, r8 = r & 7;
+    const size_t base = (((size_t)k * groups + (col >> 4)) * u.tiles + tile) * 2 * 32 * 4;
+    const int f = (4 * r8 + (c >> 2)) * 4 + (c & 3);
+    const int d = (4 * (2 * (c >> 2) + (c & 1)) + (r8 & 3)) * 4 + 2 * ((c & 3) >> 1) + (r8 >> 2);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+        u.w1f[base + h * 128 + f] = part[h];
+        u.w1d[base + h * 128 + d] = part[h];
+    }
+}
+
+__global__ void __launch_bounds__(256) step_update_kernel(const __grid_constant__ StepUpdateArgs u) {
+    step_begin(u.stamps ? u.stamps + 4 : nullptr);
+    const AdamArgs& a = u.adam;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *(volatile float*)u.h_loss = *u.loss;
+        *(volatile int*)u.h_status = u.status ? *u.status : 0;
+    }
+    const long long stride = (long long)gridDim.x * blockDim.x, me = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    auto update = [&](const AdamSegment& s, long long i, float4 g) {
+        float4 p = a.p[i], m = a.m[i], v = a.v[i];
+        adam_op(s, a.rate, a.adj * g.x, p.x, m.x, v.x);
+        adam_op(s, a.rate, a.adj * g.y, p.y, m.y, v.y);
+        adam_op(s, a.rate, a.adj * g.z, p.z, m.z, v.z);
+        adam_op(s, a.rate, a.adj * g.w, p.w, m.w, v.w);
+        a.p[i] = p;
+        a.m[i] = m;
+        a.v[i] = v;
+        return p;
+    };
+    if (u.l0f_seg >= 0) {
+        const AdamSegment &sw = a.seg[u.l0w_seg], &sf = a.seg[u.l0f_seg];
+        for (long long j = me; j < u.block4; j += stride) {
+            float4 sum = make_float4(0, 0, 0, 0);
+#pragma unroll 4
+            for (int c = 0; c < u.copies; c++) {
+                const long long i = u.l0w4 + c * u.block4 + j;
+                const float4 g = u.g[i];
+                if (c == 0) sum = g;
+                else sum.x += g.x, sum.y += g.y, sum.z += g.z, sum.w += g.w;
+                update(sw, i, g);
+            }
+            u.g[u.l0f4 + j] = sum;
+            update(sf, u.l0f4 + j, sum);
+        }
+    }
+    for (long long i = me; i < u.rest4; i += stride) {
+        int si = -1;
+#pragma unroll 1
+        for (int k = 0; k < a.nseg; k++)
+            if (i >= a.seg[k].begin4 && i < a.seg[k].end4) si = k;
+        if (si < 0 || si == u.l0f_seg) continue;  // alignment padding between tensors
+        const float4 p = update(a.seg[si], i, u.g[i]);
+        if (i >= u.l1w4_begin && i < u.l1w4_end) {
+            const long long e = 4 * (i - u.l1w4_begin), n = (long long)u.K1 * u.O * u.M1;
+            store_w1(u, e, p.x);
+            if (e + 1 < n) store_w1(u, e + 1, p.y);
+            if (e + 2 < n) store_w1(u, e + 2, p.z);
+            if (e + 3 < n) store_w1(u, e + 3, p.w);
+        }
+    }
+    if (u.stamps && threadIdx.x == 0) atomicMax(u.stamps + 7, clock_ns());
 }
 
 // Data-parallel update over peer memory: reduce-scatter, AdamW and all-gather in one launch.
@@ -208,37 +309,6 @@ template <int WORLD, int kBulkTile, int kBulkStages>
 __host__ __device__ constexpr size_t exchange_bulk_smem() {
     return (size_t)kBulkStages * ((WORLD > 0 ? WORLD : kMaxRanks) + 6) * kBulkTile * sizeof(float4) + kBulkStages * 8;
 }
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-__device__ __forceinline__ void mbar_init(uint64_t* bar, int count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(smem_u32(bar)), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
-__device__ __forceinline__ void bulk_load(void* smem_dst, const void* gmem_src, uint32_t bytes, uint64_t* bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(smem_dst)),
-                 "l"(gmem_src), "r"(bytes), "r"(smem_u32(bar))
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_store(void* gmem_dst, const void* smem_src, uint32_t bytes) {
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gmem_dst), "r"(smem_u32(smem_src)), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
-__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
-__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 template <int WORLD, int kBulkTile, int kBulkStages>
 __global__ void __launch_bounds__(kBulkTile, 1) adamw_exchange_bulk_kernel(const __grid_constant__ ExchangeArgs x) {

@@ -29,6 +29,7 @@
 #include "../../include/bullet_b200.h"
 #include "common.h"
 #include "kernels_dense_mma.cuh"
+#include "kernels_dense_one.cuh"
 #include "kernels_ft.cuh"
 #include "kernels_opt.cuh"
 #include "kernels_prep.cuh"
@@ -54,6 +55,7 @@ namespace {
 
 constexpr int64_t kAlignFloats = 64;       // 256-byte tensor alignment in the flat buffers
 constexpr int kGatherRowsPerPosition = 34;  // active features of both perspectives of a middling chess position
+constexpr int64_t kClearInForward = 2 << 20;  // floats of a gradient buffer that the forward kernel clears itself
 constexpr int kDirectOutputs = 256;        // up to as many outputs of an evaluation the kernel stores to pinned memory itself
 constexpr int kMinItemPairs = 128;         // a forward work item serves at least this many pairs per tile load
 
@@ -177,12 +179,21 @@ struct b200_net {
     static constexpr int kTimingRing = 256, kTimingEvents = 8;
     cudaEvent_t tev[kTimingRing][kTimingEvents] = {};
     int64_t steps_begun = 0, steps_done = 0, timing_origin = 0;
+    bool events_made = false;
+    // ... or, for whole steps (b200_step), time stamps that the kernels write themselves (launch.cuh)
+    unsigned long long* d_stamps = nullptr;  // [kTimingRing][kTimingEvents]
+    bool stamped[kTimingRing] = {};          // how the ring's entry was taken
+    bool chained = false;                    // the launches being enqueued are one whole step's
+    unsigned long long* stamp(int k) const { return chained ? d_stamps + (steps_begun % kTimingRing) * kTimingEvents + k : nullptr; }
     bool step_open = false;
     int64_t opt_step = 0;   // completed optimiser steps (RAdam's step count; reset when the rule changes)
     float* S = nullptr;     // Ranger's slow weights, same layout as P (allocated when a tensor first uses Ranger)
     int64_t launches = 0, h2d_bytes = 0;
     std::vector<void*> allocations;
 
+    int* kept_bucket = nullptr;  // dense_one: the output bucket of every position of the last pass
+    int w1_now = 0;              // which of two copies of the regrouped weights is current; the last pass may have used the other
+    const float* w1_used = nullptr;
     int D1() const { return d.pairwise ? d.ft_out : 2 * d.ft_out; }
     int dense_in(int l) const { return l == 0 ? D1() : d.dense_out[l - 1]; }
     Tensor* find(const char* name) {
@@ -204,11 +215,14 @@ struct b200_net {
     // The gather forward of n positions reads the merged table (one row per feature, after a pass over the whole table)
     // when the batch gathers several times the table's rows; below that it adds the factoriser row by row.
     bool merged_table(int n) const { return d.factoriser_rows && !fwd_tiled(n) && (long long)n * d.nnz >= 5LL * d.n_inputs; }
+    float* w1g_now() const { return w1g ? w1g + (size_t)w1_now * d.n_out_buckets * d.dense_out[0] * D1() : nullptr; }
     void weights_moved() { w1_dirty = merged_dirty = true; }
     bool bwd_tiled() const { return ft_bwd_mode == B200_FT_TILED || (ft_bwd_mode == B200_FT_AUTO && tiled_ok); }
     // the register-tiled dense forward (rows per bucket in fours, more layers after the first) also
     // forms the gradients of those later layers
     bool fused_small_grads() const { return dense_mma(); }
+    // one row per bucket and nothing behind it (and rows that fit the kernel's stages): dense_one_kernel
+    bool dense_one() const { return d.n_dense == 1 && D1() <= b200::kOneMaxK; }
     // first dense layers of four and more rows per bucket run on the tensor pipe
     bool dense_mma() const { return d.dense_out[0] >= 4; }
 };
@@ -321,7 +335,7 @@ void slot_layout(const b200_net* net, Slot& s, int n) {
 template <bool PW>
 int launch_ft_forward(b200_net* net, const b200::FtArgs& a, const b200::TileArgs& t, bool tiled, int grid) {
     if (tiled) {
-        b200::ft_forward_tiled_kernel<PW><<<grid, b200::kFwdThreads, b200::ft_fwd_smem(t.block_rows, t.list_len), net->stream>>>(a, t);
+        CK(b200::launch_step(false, b200::ft_forward_tiled_kernel<PW>, grid, b200::kFwdThreads, b200::ft_fwd_smem(t.block_rows, t.list_len), net->stream, a, t));
     } else {
         const int unit = PW ? a.H / 2 : a.H;
         // one pair per warp while there are few, up to eight once that leaves two waves of eight CTAs per SM
@@ -334,25 +348,32 @@ int launch_ft_forward(b200_net* net, const b200::FtArgs& a, const b200::TileArgs
     return 0;
 }
 
+template <bool PW, bool ONE>
+void launch_ft_backward_tiled(const b200::FtArgs& a, const b200::TileArgs& t, bool wide, int grid, size_t smem, bool chained, cudaStream_t stream) {
+    // data-parallel runs that announce finished row blocks take an instantiation of their own: the
+    // fence it ends with makes every CTA wait for its reductions to land (measured: +18 %)
+    if (wide && t.sig.done_count)
+        b200::launch_step(chained, b200::ft_backward_tiled_kernel<PW, 1024, true, ONE>, grid, 1024, smem, stream, a, t);
+    else if (wide)
+        b200::launch_step(chained, b200::ft_backward_tiled_kernel<PW, 1024, false, ONE>, grid, 1024, smem, stream, a, t);
+    else if (t.sig.done_count)
+        b200::launch_step(chained, b200::ft_backward_tiled_kernel<PW, 512, true, ONE>, grid, 512, smem, stream, a, t);
+    else
+        b200::launch_step(chained, b200::ft_backward_tiled_kernel<PW, 512, false, ONE>, grid, 512, smem, stream, a, t);
+}
+
 template <bool PW>
 int launch_ft_backward(b200_net* net, const b200::FtArgs& a, const b200::TileArgs& t, bool tiled, int grid) {
     if (tiled) {
         const size_t smem = b200::ft_bwd_smem(t.block_rows, a.nnz, t.chunk_len);
         const bool wide = t.chunk_len > b200::ft_bwd_chunk(a.nnz, false);
-// data-parallel runs that announce finished row blocks take an instantiation of their own: the
-        // fence it ends with makes every CTA wait for its reductions to land (measured: +18 %)
-        if (wide && t.sig.done_count)
-            b200::ft_backward_tiled_kernel<PW, 1024, true><<<grid, 1024, smem, net->stream>>>(a, t);
-        else if (wide)
-            b200::ft_backward_tiled_kernel<PW, 1024, false><<<grid, 1024, smem, net->stream>>>(a, t);
-        else if (t.sig.done_count)
-            b200::ft_backward_tiled_kernel<PW, 512, true><<<grid, 512, smem, net->stream>>>(a, t);
-        else
-            b200::ft_backward_tiled_kernel<PW, 512, false><<<grid, 512, smem, net->stream>>>(a, t);
+        if (net->dense_one()) launch_ft_backward_tiled<PW, true>(a, t, wide, grid, smem, net->chained, net->stream);
+        else launch_ft_backward_tiled<PW, false>(a, t, wide, grid, smem, net->chained, net->stream);
     } else {
         const int unit = PW ? a.H / 2 : a.H;
         dim3 grid((2 * a.n + 63) / 64, (unit + 127) / 128);
-        b200::ft_backward_gather_kernel<PW><<<grid, 256, 0, net->stream>>>(a, 64);
+        if (net->dense_one()) b200::launch_step(net->chained, b200::ft_backward_gather_kernel<PW, true>, grid, 256, 0, net->stream, a, 64);
+        else b200::launch_step(net->chained, b200::ft_backward_gather_kernel<PW, false>, grid, 256, 0, net->stream, a, 64);
     }
     LAUNCHED(net);
     return 0;
@@ -379,20 +400,20 @@ int launch_ft_backward(b200_net* net, const b200::FtArgs& a, const b200::TileArg
 template <int MM>
 void launch_dense_forward(b200_net* net, const b200::DenseArgs& da, int ntiles) {
     if constexpr (MM >= 4)
-        b200::dense_forward_mma_kernel<MM><<<ntiles, 256, b200::dense_mma_smem<MM>(), net->stream>>>(da);
+        b200::launch_step(net->chained, b200::dense_forward_mma_kernel<MM>, ntiles, 256, b200::dense_mma_smem<MM>(), net->stream, da);
     else
-        b200::dense_forward_kernel<MM><<<ntiles, 256, b200::dense_fwd_smem<MM>(), net->stream>>>(da);
+        b200::launch_step(net->chained, b200::dense_forward_kernel<MM>, ntiles, 256, b200::dense_fwd_smem<MM>(), net->stream, da);
 }
 template <int MM>
 void launch_wgrad_mma(b200_net* net, const b200::DenseArgs& a, float* gW, float* gB, dim3 grid, int threads, int per_run) {
-    if constexpr (MM >= 4) b200::dense_wgrad_mma_kernel<MM><<<grid, threads, 0, net->stream>>>(a, gW, gB, per_run);
+    if constexpr (MM >= 4) b200::launch_step(net->chained, b200::dense_wgrad_mma_kernel<MM>, grid, threads, 0, net->stream, a, gW, gB, per_run);
 }
 template <int MM>
 void launch_dense_dx(b200_net* net, const b200::DenseArgs& da, int ntiles) {
     if constexpr (MM >= 4)
-        b200::dense_dx_mma_kernel<MM><<<ntiles, 256, 0, net->stream>>>(da, net->dx);
+        b200::launch_step(net->chained, b200::dense_dx_mma_kernel<MM>, ntiles, 256, 0, net->stream, da, net->dx);
     else
-        b200::dense_dx_kernel<MM><<<ntiles, 256, 0, net->stream>>>(da, net->dx);
+        b200::launch_step(net->chained, b200::dense_dx_kernel<MM>, ntiles, 256, 0, net->stream, da, net->dx);
 }
 
 template <int MM>
@@ -440,6 +461,10 @@ b200::FtArgs ft_args(b200_net* net, const Slot& s) {
     a.x = net->x;
     a.u = net->u;
     a.dx = net->dx;
+    a.w1 = net->w1_used;
+    a.dout = net->dz[0];
+    a.out_bucket = net->kept_bucket;
+    a.stamp = nullptr;
     a.g_table = net->G + net->find("l0w")->off;
     a.g_bias = net->G + net->find("l0b")->off;
     return a;
@@ -498,7 +523,7 @@ b200::DenseArgs dense_args(b200_net* net, const Slot& s, bool want_grad) {
     a.order = d.n_out_buckets > 1 ? s.dev<int>(s.off_order) : nullptr;
     a.tiles = d.n_out_buckets > 1 ? s.dev<int2>(s.off_dtiles) : nullptr;
     a.ntiles = s.n_dtiles;
-    a.W1g = net->w1g;
+    a.W1g = net->w1g_now();
     a.W1f = net->w1f;
     a.W1d = net->w1d;
     a.a1 = net->a1;
@@ -537,8 +562,9 @@ int refresh_table(b200_net* net, int n) {
             b200::dense_fragments_kernel<<<std::min(net->sm_count * 4, (lanes + 255) / 256), 256, 0, net->stream>>>(
                 net->P + w1->off, net->w1f, net->w1d, net->D1(), O, M1, M1 >= 8 ? M1 / 8 : 1);
         } else {
+            net->w1_now ^= 1;
             b200::dense_regroup_kernel<<<std::min<int>(net->sm_count * 4, (int)((w1->n + 255) / 256)), 256, 0, net->stream>>>(
-                net->P + w1->off, net->w1g, net->D1(), O, M1);
+                net->P + w1->off, net->w1g_now(), net->D1(), O, M1);
         }
         LAUNCHED(net);
         net->w1_dirty = false;
@@ -647,7 +673,7 @@ int forward_prepare(b200_net* net, Slot& s, bool want_grad) {
         if (int rc = group_slot(net, s, group_args(net, s, true, false), false, net->stream)) return rc;
     }
     if (want_grad) net->status_slot = needed ? (int)(&s - net->slots) : -1;
-    if (want_grad) CK(cudaEventRecord(net->tev[net->steps_begun % b200_net::kTimingRing][0], net->stream));
+    if (want_grad && !net->chained) CK(cudaEventRecord(net->tev[net->steps_begun % b200_net::kTimingRing][0], net->stream));
     return 0;
 }
 
@@ -666,12 +692,30 @@ int forward_ft_blocks(b200_net* net, Slot& s, int first_block, int last_block) {
 }
 
 int forward_dense(b200_net* net, Slot& s, bool want_grad) {
-    if (want_grad) CK(cudaEventRecord(net->tev[net->steps_begun % b200_net::kTimingRing][1], net->stream));
+    if (want_grad && !net->chained) CK(cudaEventRecord(net->tev[net->steps_begun % b200_net::kTimingRing][1], net->stream));
     if (net->zero_pending) {  // the loss and every gradient from here on land in the cleared buffer
         CK(cudaStreamWaitEvent(net->stream, net->zero_done, 0));
         net->zero_pending = false;
     }
     b200::DenseArgs da = dense_args(net, s, want_grad);
+    da.stamp = net->stamp(1);
+    if (net->dense_one()) {
+        b200::OneArgs a{};
+        a.x = da.x, a.buckets = da.buckets, a.targets = da.targets, a.order = da.order, a.tiles = da.tiles;
+        a.n = da.n, a.ntiles = da.ntiles, a.K1 = da.K1, a.O = da.O;
+        a.W = da.W1g, a.B = da.B[0];
+        a.dout = net->dz[0], a.kept_bucket = net->kept_bucket, a.out = da.out, a.out_host = da.out_host, a.loss = da.loss;
+        a.gW = net->G + net->find("l1w")->off, a.gB = net->G + net->find("l1b")->off;
+        a.want_grad = da.want_grad;
+        a.stamp = da.stamp;
+        net->w1_used = da.W1g;
+        const size_t smem = b200::one_smem(a.K1);
+        const int units = a.ntiles * (b200::kDenseTile / b200::one_rows(a.K1)), slots = net->sm_count * std::max(1, std::min(4, (int)(220 * 1024 / smem)));
+        a.units_per_run = (units + slots - 1) / slots;
+        b200::launch_step(net->chained, b200::dense_one_kernel, (units + a.units_per_run - 1) / a.units_per_run, b200::kOneThreads, smem, net->stream, a);
+        LAUNCHED(net);
+        return 0;
+    }
     DISPATCH_M(net->d.dense_out[0], launch_dense_forward<MM>(net, da, s.n_dtiles));
     LAUNCHED(net);
     return 0;
@@ -721,7 +765,7 @@ int launch_wgrad(b200_net* net, const Slot& s) {
     w.chunk_len = (s.n + chunks - 1) / chunks;
     chunks = (s.n + w.chunk_len - 1) / w.chunk_len;
     dim3 grid(gx, chunks);
-    DISPATCH_M12(d.dense_out[0], b200::dense_wgrad_kernel<MM><<<grid, threads, 0, net->stream>>>(w));
+    DISPATCH_M12(d.dense_out[0], b200::launch_step(net->chained, b200::dense_wgrad_kernel<MM>, grid, threads, 0, net->stream, w));
     LAUNCHED(net);
     return 0;
 }
@@ -750,7 +794,7 @@ int launch_dense_grads(b200_net* net, Slot& s) {
             snprintf(name, sizeof name, "l%db", l + 1);
             g.gB[l - 1] = net->G + net->find(name)->off;
         }
-        b200::dense_small_grads_kernel<<<s.n_dtiles, 256, 0, net->stream>>>(g);
+        b200::launch_step(net->chained, b200::dense_small_grads_kernel, s.n_dtiles, 256, 0, net->stream, g);
         LAUNCHED(net);
     }
     return launch_wgrad(net, s);
@@ -777,17 +821,17 @@ bool load_dense_kernels() {
 int preload_kernels(b200_net* net) {
     bool ok = true;
     DISPATCH_M(net->d.dense_out[0], ok = load_dense_kernels<MM>());
-    ok = ok && load_kernel(b200::dense_regroup_kernel) && load_kernel(b200::dense_fragments_kernel) && load_kernel(b200::dense_small_grads_kernel);
+    ok = ok && load_kernel(b200::dense_regroup_kernel) && load_kernel(b200::dense_one_kernel) && load_kernel(b200::dense_one_dx_kernel) && load_kernel(b200::dense_fragments_kernel) && load_kernel(b200::dense_small_grads_kernel);
     ok = ok && load_kernel(b200::ft_forward_gather_kernel<true>) && load_kernel(b200::ft_forward_gather_kernel<false>);
-    ok = ok && load_kernel(b200::ft_backward_gather_kernel<true>) && load_kernel(b200::ft_backward_gather_kernel<false>);
+    ok = ok && load_kernel(b200::ft_backward_gather_kernel<true, true>) && load_kernel(b200::ft_backward_gather_kernel<true, false>) && load_kernel(b200::ft_backward_gather_kernel<false, true>) && load_kernel(b200::ft_backward_gather_kernel<false, false>);
     ok = ok && load_kernel(b200::ft_forward_tiled_kernel<true>) && load_kernel(b200::ft_forward_tiled_kernel<false>);
-    ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, true>);
-    ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 512, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, true>);
-    ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, false>);
-    ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 512, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, false>);
+    ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, true, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, true, false>);
+    ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 512, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 512, true, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, true, false>);
+    ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, false, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, false, false>);
+    ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 512, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 512, false, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, false, false>);
     ok = ok && load_kernel(b200::ft_csr_kernel);
     ok = ok && load_kernel(b200::factoriser_merge_kernel) && load_kernel(b200::factoriser_grad_kernel);
-    ok = ok && load_kernel(b200::adamw_flat_kernel) && load_kernel(b200::lookahead_kernel);
+    ok = ok && load_kernel(b200::adamw_flat_kernel) && load_kernel(b200::step_update_kernel) && load_kernel(b200::lookahead_kernel);
     ok = ok && load_kernel(b200::adamw_exchange_kernel<0>) && load_kernel(b200::adamw_exchange_kernel<2>);
     ok = ok && load_kernel(b200::adamw_exchange_kernel<4>) && load_kernel(b200::adamw_exchange_kernel<8>);
     ok = ok && load_kernel(b200::adamw_exchange_bulk_kernel<2, 256, 6>) && load_kernel(b200::adamw_exchange_bulk_kernel<2, 512, 3>);
@@ -902,13 +946,15 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     rc = rc ? rc : dev_alloc(net, &net->a2, B * 32);
     for (int l = 0; l < 3; l++) rc = rc ? rc : dev_alloc(net, &net->dz[l], B * 32);
     rc = rc ? rc : dev_alloc(net, &net->out, B);
+    rc = rc ? rc : dev_alloc(net, &net->d_stamps, b200_net::kTimingRing * b200_net::kTimingEvents);
     rc = rc ? rc : dev_alloc(net, &net->d_status, b200_net::kLossRing);
     if (net->dense_mma()) {
         const size_t table = b200::mma_table_floats(net->D1(), d.n_out_buckets, d.dense_out[0]) / 4;
         rc = rc ? rc : dev_alloc(net, &net->w1f, table);
         rc = rc ? rc : dev_alloc(net, &net->w1d, table);
     } else {
-        rc = rc ? rc : dev_alloc(net, &net->w1g, (size_t)d.n_out_buckets * d.dense_out[0] * net->D1());
+        rc = rc ? rc : dev_alloc(net, &net->w1g, (size_t)2 * d.n_out_buckets * d.dense_out[0] * net->D1());
+        if (net->dense_one()) rc = rc ? rc : dev_alloc(net, &net->kept_bucket, B);
     }
     // the fence counters get an allocation of their own size class (2 MiB), so that its IPC handle maps exactly it
     rc = rc ? rc : dev_alloc(net, &net->xch_flags, (size_t)(2 << 20) / sizeof(int));
@@ -964,9 +1010,6 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     net->h_xstatus = net->h_status + b200_net::kLossRing;
     memset(net->h_loss, 0, 128);  // 8 floats, 4 status words, 4 x 4 fence words
     for (auto& e : net->loss_ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
-    for (auto& ring : net->tev)
-        for (auto& e : ring) cudaEventCreate(&e);
-
     {
         constexpr int MM_unused = 0;
         (void)MM_unused;
@@ -977,18 +1020,27 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
             return 0;
         };
         if (int rc2 = set_dense(d.dense_out[0])) return bail(rc2);
+        if (b200::allow_smem(b200::dense_one_kernel) != cudaSuccess) return bail(b200::fail(B200_ERR_CUDA, "net_create: shared memory of the dense kernel"));
     }
     if (net->tiled_ok) {
         cudaError_t e = b200::allow_smem(b200::ft_forward_tiled_kernel<true>);
         e = e ? e : b200::allow_smem(b200::ft_forward_tiled_kernel<false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 1024, true>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 1024, true>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 512, true>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, true>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 1024, false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 1024, false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 512, false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 1024, true, true>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 1024, true, false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 1024, true, true>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 1024, true, false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 512, true, true>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 512, true, false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, true, true>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, true, false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 1024, false, true>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 1024, false, false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 1024, false, true>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 1024, false, false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 512, false, true>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 512, false, false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, false, true>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, false, false>);
         e = e ? e : b200::allow_smem(b200::ft_csr_kernel);
         if (e != cudaSuccess) return bail(b200::fail(B200_ERR_CUDA, "net_create: shared memory of the tiled kernels: %s", cudaGetErrorString(e)));
     }
@@ -1425,6 +1477,16 @@ int b200_slot_read(b200_net* net, int slot, uint16_t* stm, uint16_t* nstm, int32
 
 // ---- the training forward pass in pieces (b200_backward_begin runs them itself when the caller has not)
 
+// Clears the gradient buffer on a side stream, beside the FT forward, which does not touch it; the dense layers wait for it.
+static int clear_gradients_aside(b200_net* net) {
+    CK(cudaEventRecord(net->zero_fork, net->stream));
+    CK(cudaStreamWaitEvent(net->zero_stream, net->zero_fork, 0));
+    CK(cudaMemsetAsync(net->G, 0, (size_t)net->n_flat * 4, net->zero_stream));
+    CK(cudaEventRecord(net->zero_done, net->zero_stream));
+    net->zero_pending = true;
+    return 0;
+}
+
 int b200_forward_begin(b200_net* net, int slot) {
     if (int rc = check_slot(net, slot, "forward_begin")) return rc;
     if (net->bwd_slot >= 0) return b200::fail(B200_ERR_STATE, "forward_begin: the backward pass of slot %d is not finished", net->bwd_slot);
@@ -1435,13 +1497,15 @@ int b200_forward_begin(b200_net* net, int slot) {
     if (int rc = refresh_table(net, s.n)) return rc;
     if (!net->manual_grad_zero) {
         // every gradient is accumulated with reductions, so the buffer starts at zero; nothing before
-        // the dense layers writes to it, so the clearing runs on a side stream beside the FT forward
-        CK(cudaEventRecord(net->zero_fork, net->stream));
-        CK(cudaStreamWaitEvent(net->zero_stream, net->zero_fork, 0));
-        CK(cudaMemsetAsync(net->G, 0, (size_t)net->n_flat * 4, net->zero_stream));
-        CK(cudaEventRecord(net->zero_done, net->zero_stream));
-        net->zero_pending = true;
+        // the dense layers writes to it
+        if (int rc = clear_gradients_aside(net)) return rc;
     }
+    if (!net->events_made) {  // the steps that run in pieces are timed with events
+        for (auto& ring : net->tev)
+            for (auto& e : ring) CK(cudaEventCreate(&e));
+        net->events_made = true;
+    }
+    net->stamped[net->steps_begun % b200_net::kTimingRing] = false;
     if (int rc = forward_prepare(net, s, true)) return rc;
     net->fwd_slot = slot;
     net->fwd_parts_done = 0;
@@ -1487,12 +1551,12 @@ int b200_backward_begin(b200_net* net, int slot) {
     CK(cudaEventRecord(ev[2], net->stream));
     if (net->bwd_tiled() && !s.csr_built)  // normally built at upload
         if (int rc = build_csr(net, s, net->stream)) return rc;
-    {
+    if (!net->dense_one()) {
         b200::DenseArgs da = dense_args(net, s, true);
         DISPATCH_M(d.dense_out[0], launch_dense_dx<MM>(net, da, s.n_dtiles));
         LAUNCHED(net);
+        if (int rc = launch_dense_grads(net, s)) return rc;
     }
-    if (int rc = launch_dense_grads(net, s)) return rc;
     CK(cudaEventRecord(ev[3], net->stream));
     net->bwd_slot = slot;
     net->bwd_parts_done = 0;
@@ -1884,6 +1948,33 @@ int b200_grad_zero_range(b200_net* net, int64_t first_float, int64_t n_floats) {
     return 0;
 }
 
+// Ranger: every k-th step the fast weights are pulled towards the slow ones, which then follow.  Due after the update that is
+// about to be counted?
+static bool lookahead_due(const b200_net* net) {
+    for (const Tensor& t : net->tensors)
+        if (net->S && t.opt_kind == B200_OPT_RANGER && (net->opt_step + 1) % t.lookahead_k == 0) return true;
+    return false;
+}
+static int launch_lookahead(b200_net* net) {  // (after the count)
+    b200::LookaheadArgs la{};
+    la.p = reinterpret_cast<float4*>(net->P);
+    la.slow = reinterpret_cast<float4*>(net->S);
+    la.total4 = net->n_flat / 4;
+    la.nseg = (int)net->tensors.size();
+    for (int i = 0; i < la.nseg; i++) {
+        const Tensor& t = net->tensors[i];
+        la.begin4[i] = t.off / 4;
+        la.end4[i] = (t.off + t.n + 3) / 4;
+        const bool due = t.opt_kind == B200_OPT_RANGER && net->opt_step % t.lookahead_k == 0;
+        la.alpha[i] = due ? t.alpha : -1.f;
+        la.one_minus[i] = 1.0f - t.alpha;
+    }
+    b200::lookahead_kernel<<<net->sm_count * 8, 256, 0, net->stream>>>(la);
+    LAUNCHED(net);
+    net->weights_moved();
+    return 0;
+}
+
 int b200_update_end(b200_net* net) {
     if (!net) return b200::fail(B200_ERR_ARG, "update_end: null net");
     if (!net->have_backward) return b200::fail(B200_ERR_STATE, "update_end: no gradients yet");
@@ -1903,29 +1994,10 @@ int b200_update_end(b200_net* net) {
     }
     CK(cudaEventRecord(net->loss_ev[ring], net->stream));
     net->updates++;
+    const bool lookahead = lookahead_due(net);
     net->opt_step++;
-    {   // Ranger: every k-th step the fast weights are pulled towards the slow ones, which then follow
-        b200::LookaheadArgs la{};
-        la.p = reinterpret_cast<float4*>(net->P);
-        la.slow = reinterpret_cast<float4*>(net->S);
-        la.total4 = net->n_flat / 4;
-        la.nseg = (int)net->tensors.size();
-        bool any = false;
-        for (int i = 0; i < la.nseg; i++) {
-            const Tensor& t = net->tensors[i];
-            la.begin4[i] = t.off / 4;
-            la.end4[i] = (t.off + t.n + 3) / 4;
-            const bool due = t.opt_kind == B200_OPT_RANGER && net->opt_step % t.lookahead_k == 0;
-            la.alpha[i] = due ? t.alpha : -1.f;
-            la.one_minus[i] = 1.0f - t.alpha;
-            any = any || due;
-        }
-        if (any && net->S) {
-            b200::lookahead_kernel<<<net->sm_count * 8, 256, 0, net->stream>>>(la);
-            LAUNCHED(net);
-            net->weights_moved();
-        }
-    }
+    if (lookahead)
+        if (int rc = launch_lookahead(net)) return rc;
     if (int rc = refresh_table(net, net->last_n)) return rc;
     if (net->step_open) {  // close the timed step begun by the matching backward
         CK(cudaEventRecord(net->tev[net->steps_begun % b200_net::kTimingRing][7], net->stream));
@@ -1942,7 +2014,123 @@ int b200_update(b200_net* net, float lr, float grad_factor) {
     return b200_update_end(net);
 }
 
+// A whole step enqueued at once: nothing is observed between its phases, so its kernels are chained (launch.cuh), keep their
+// own time, and the update forms the factoriser's gradient, the first dense layer's tables and the read-back itself.
+static int step_chained(b200_net* net, Slot& s, int slot, float lr, float grad_factor) {
+    const b200_net_desc& d = net->d;
+    CK(cudaStreamWaitEvent(net->stream, s.ready, 0));
+    net->trains = true;
+    if (int rc = refresh_table(net, s.n)) return rc;
+    const int ring = (int)(net->updates % b200_net::kLossRing);
+    // a small gradient buffer is cleared by the forward kernel; a large one would hold it up
+    const bool clear_here = net->n_flat <= kClearInForward;
+    if (!clear_here)
+        if (int rc = clear_gradients_aside(net)) return rc;
+    if (int rc = forward_prepare(net, s, true)) return rc;
+    const bool bwd_tiled = net->bwd_tiled();
+    if (bwd_tiled && !s.csr_built)
+        if (int rc = build_csr(net, s, net->stream)) return rc;
+    {
+        const bool tiled = net->fwd_tiled(s.n);
+        b200::FtArgs fa = ft_args(net, s);
+        b200::TileArgs ta = tile_args(net, s, false);
+        fa.stamp = net->stamp(0);
+        fa.stamp_end = net->stamp(7);
+        if (clear_here) {
+            fa.zero = reinterpret_cast<float4*>(net->G);
+            fa.zero4 = net->n_flat / 4;
+        }
+        const int grid = tiled ? ft_forward_grid(net, s) : 0;
+        int rc = d.pairwise ? launch_ft_forward<true>(net, fa, ta, tiled, grid) : launch_ft_forward<false>(net, fa, ta, tiled, grid);
+        if (rc) return rc;
+    }
+    if (int rc = forward_dense(net, s, true)) return rc;
+    if (!net->dense_one()) {
+        b200::DenseArgs da = dense_args(net, s, true);
+        da.stamp = net->stamp(2);
+        DISPATCH_M(d.dense_out[0], launch_dense_dx<MM>(net, da, s.n_dtiles));
+        LAUNCHED(net);
+        if (int rc = launch_dense_grads(net, s)) return rc;
+    }
+    {
+        b200::FtArgs fa = ft_args(net, s);
+        b200::TileArgs ta = tile_args(net, s, true);
+        fa.stamp = net->stamp(3);
+        const int grid = bwd_tiled ? ft_backward_grid(net, s, false) : 0;
+        int rc = d.pairwise ? launch_ft_backward<true>(net, fa, ta, bwd_tiled, grid) : launch_ft_backward<false>(net, fa, ta, bwd_tiled, grid);
+        if (rc) return rc;
+    }
+    const bool lookahead = lookahead_due(net);
+    {
+        b200::StepUpdateArgs u{};
+        b200::AdamArgs& a = u.adam;
+        a.p = reinterpret_cast<float4*>(net->P);
+        a.m = reinterpret_cast<float4*>(net->M);
+        a.v = reinterpret_cast<float4*>(net->V);
+        a.rate = lr;
+        a.adj = grad_factor;
+        fill_segments(net, a);
+        u.g = reinterpret_cast<float4*>(net->G);
+        const Tensor *l0w = net->find("l0w"), *l0f = d.factoriser_rows ? net->find("l0f") : nullptr, *l1w = net->find("l1w");
+        u.l0f_seg = u.l0w_seg = -1;
+        if (l0f)
+            for (int i = 0; i < a.nseg; i++) {
+                if (&net->tensors[i] == l0w) u.l0w_seg = i;
+                if (&net->tensors[i] == l0f) u.l0f_seg = i;
+            }
+        u.rest4 = l0f ? l0w->off / 4 : net->n_flat / 4;
+        u.l0w4 = l0w->off / 4;
+        u.l0f4 = l0f ? l0f->off / 4 : 0;
+        u.block4 = l0f ? l0f->n / 4 : 0;
+        u.copies = l0f ? (int)(l0w->n / l0f->n) : 0;
+        u.l1w4_begin = l1w->off / 4;
+        u.l1w4_end = lookahead ? u.l1w4_begin : (l1w->off + l1w->n + 3) / 4;  // (the lookahead moves the weights once more)
+        u.K1 = net->D1();
+        u.O = d.n_out_buckets;
+        u.M1 = d.dense_out[0];
+        u.tiles = net->dense_mma() ? (u.M1 >= 8 ? u.M1 / 8 : 1) : 0;
+        if (!lookahead && !net->dense_mma()) net->w1_now ^= 1;
+        u.w1g = net->w1g_now();
+        u.w1f = reinterpret_cast<float*>(net->w1f);
+        u.w1d = reinterpret_cast<float*>(net->w1d);
+        u.loss = net->G;
+        u.status = net->status_slot >= 0 ? s.dev<int>(s.off_status) : nullptr;
+        u.h_loss = net->h_loss + ring;
+        u.h_status = net->h_status + ring;
+        u.stamps = net->stamp(0);
+        const long long items = std::max(u.rest4, u.block4), blocks = std::min<long long>((items + 255) / 256, net->sm_count * 8);
+        CK(b200::launch_step(true, b200::step_update_kernel, (unsigned)blocks, 256, 0, net->stream, u));
+        LAUNCHED(net);
+        net->weights_moved();
+        net->w1_dirty = lookahead;
+    }
+    CK(cudaEventRecord(s.consumed, net->stream));
+    s.has_consumed = true;
+    CK(cudaEventRecord(net->loss_ev[ring], net->stream));
+    net->last_n = s.n;
+    net->have_backward = true;
+    net->loss_in_param = false;
+    net->updates++;
+    net->opt_step++;
+    net->stamped[net->steps_begun % b200_net::kTimingRing] = true;
+    net->steps_begun++;
+    net->steps_done = net->steps_begun;
+    if (lookahead) {
+        if (int rc = launch_lookahead(net)) return rc;
+        if (int rc = refresh_table(net, net->last_n)) return rc;
+    }
+    return 0;
+}
+
 int b200_step(b200_net* net, int slot, float lr, float grad_factor) {
+    if (int rc = check_slot(net, slot, "step")) return rc;
+    if (net->fwd_slot < 0 && net->bwd_slot < 0 && !net->manual_grad_zero && !net->sig_on && !net->xch_fenced_used) {
+        if (int rc = set_device(net)) return rc;
+        net->chained = true;
+        const int rc = step_chained(net, net->slots[slot], slot, lr, grad_factor);
+        net->chained = false;
+        return rc;
+    }
     if (int rc = b200_backward(net, slot)) return rc;
     return b200_update(net, lr, grad_factor);
 }
@@ -2034,7 +2222,18 @@ int b200_get_timings(b200_net* net, b200_timings* out) {
     // events: 0 start, 1 FT forward, 2 dense forward, 3 dx, 4 FT backward, 5 factoriser sums,
     // 6 dense weight gradients, 7 update
     double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    std::vector<unsigned long long> stamps((size_t)b200_net::kTimingRing * b200_net::kTimingEvents);
+    CK(cudaMemcpy(stamps.data(), net->d_stamps, stamps.size() * sizeof(stamps[0]), cudaMemcpyDeviceToHost));
     for (int64_t i = first; i < net->steps_done; i++) {
+        if (net->stamped[i % b200_net::kTimingRing]) {
+            // whole steps: starts of FT forward, dense forward, dx, FT backward and update, end of the update
+            unsigned long long* t = stamps.data() + (i % b200_net::kTimingRing) * b200_net::kTimingEvents;
+            if (net->dense_one()) t[2] = t[3];
+            const int from[7] = {0, 1, 2, 3, 4, 4, 4}, to[7] = {1, 2, 3, 4, 4, 4, 7};
+            for (int k = 0; k < 7; k++) acc[k] += (double)(int64_t)(t[to[k]] - t[from[k]]) * 1e-6;
+            acc[7] += (double)(int64_t)(t[7] - t[0]) * 1e-6;
+            continue;
+        }
         cudaEvent_t* ev = net->tev[i % b200_net::kTimingRing];
         float ms = 0.f;
         for (int k = 0; k < 7; k++) {
@@ -2083,6 +2282,10 @@ int b200_net_get_activation(b200_net* net, int which, float* host, int64_t n) {
     if (!src || want == 0) return b200::fail(B200_ERR_STATE, "get_activation: buffer %d is not used by this network", which);
     if (n != want) return b200::fail(B200_ERR_ARG, "get_activation: buffer %d holds %lld values, %lld asked", which, (long long)want, (long long)n);
     if (int rc = set_device(net)) return rc;
+    if (which == 2 && net->dense_one() && net->w1_used) {  // formed on the fly by the backward: form it once more
+        b200::dense_one_dx_kernel<<<net->sm_count * 8, 256, 0, net->stream>>>(net->w1_used, net->dz[0], net->kept_bucket, net->dx, (int)B, net->D1());
+        LAUNCHED(net);
+    }
     CK(cudaStreamSynchronize(net->stream));
     CK(cudaMemcpy(host, src, n * sizeof(float), cudaMemcpyDeviceToHost));
     return 0;
