@@ -33,6 +33,8 @@ struct DenseArgs {
     const float* W1g;  // first-layer weights regrouped as [bucket][column][row] (fewer than four rows)
     const float4* W1f; // ... or as the fragment tables of kernels_dense_mma.cuh
     const float4* W1d;
+    float* partial;    // with few tiles: [tile][slice][32][M1] sums of the slices, and how many have arrived per tile (zero between launches)
+    int* arrived;
     float* a1;         // [n][M1] activated layer-1 output (kept for the weight gradients)
     float* a2;         // [n][M2]
     float* dz[3];      // gradient at each layer's selected pre-activation: [n][M_i]

@@ -76,7 +76,7 @@ static __global__ void __launch_bounds__(256) dense_fragments_kernel(const float
 // ahead of the products.  The warps' sums meet in shared memory; the small layers, the loss, the way back to the first
 // layer's pre-activation gradient and the weight gradients of the small layers follow there, one warp per position.
 // At 131072 positions (K1 = 2048, M1 = 16) DFWD_BEFORE -> DFWD_AFTER ms against 0.165 for reading x at the copy rate.
-// grid = ntiles, block = 256, dynamic shared memory = dense_mma_smem<M1>().
+// grid = (ntiles, slices of the columns), block = 256, dynamic shared memory = dense_mma_smem<M1>().
 template <int M1>
 __host__ __device__ constexpr size_t dense_mma_smem() { return (size_t)8 * kDenseTile * M1 * sizeof(float); }
 
@@ -95,6 +95,7 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_forward_mma_kern
     __syncthreads();
     const int k = a.buckets[s_pos[0]];
     const int M2 = a.M[1], OM2 = a.O * M2;
+    const int slice = blockIdx.y, slices = gridDim.y;
     // the bucket's small-layer weights: needed only after the long loop
     for (int i = threadIdx.x; i < M1 * M2; i += blockDim.x) s_w2[i / M2][i % M2] = a.W[1][(i / M2) * OM2 + k * M2 + i % M2];
     if (threadIdx.x < 32) {
@@ -126,8 +127,8 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_forward_mma_kern
 #pragma unroll
                     for (int part = 0; part < 2; part++) wv[nt][part] = __ldg(table + (size_t)(grp * NT + nt) * 64 + 32 * part);
         };
-        fetch(warp);
-        for (int grp = warp; grp < groups; grp += 8) {
+        fetch(8 * slice + warp);
+        for (int grp = 8 * slice + warp; grp < groups; grp += 8 * slices) {
             float xs[4][4];
             uint32_t b[NT][2][4];
 #pragma unroll
@@ -139,7 +140,7 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_forward_mma_kern
                     b[nt][part][0] = __float_as_uint(wv[nt][part].x), b[nt][part][1] = __float_as_uint(wv[nt][part].y);
                     b[nt][part][2] = __float_as_uint(wv[nt][part].z), b[nt][part][3] = __float_as_uint(wv[nt][part].w);
                 }
-            fetch(grp + 8);
+            fetch(grp + 8 * slices);
             float part_sum[2][NT][4];
 #pragma unroll
             for (int m = 0; m < 2; m++)
@@ -180,11 +181,32 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_forward_mma_kern
                 }
     }
     const float* red = dense_smem;
+    int parts = 8;
     __syncthreads();
+    if (slices > 1) {
+        // few tiles: the columns are split over CTAs; the one that arrives last adds the slices up, in their order
+        __shared__ int last;
+        float* mine = a.partial + ((size_t)blockIdx.x * slices + slice) * kDenseTile * M1;
+        for (int o = threadIdx.x; o < kDenseTile * M1; o += blockDim.x) {
+            float z = 0.f;
+#pragma unroll
+            for (int w = 0; w < 8; w++) z += red[w * kDenseTile * M1 + o];
+            mine[o] = z;
+        }
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) last = atomicAdd(a.arrived + blockIdx.x, 1) == slices - 1;
+        __syncthreads();
+        if (!last) return;
+        if (threadIdx.x == 0) a.arrived[blockIdx.x] = 0;
+        __threadfence();
+        red = a.partial + (size_t)blockIdx.x * slices * kDenseTile * M1;
+        parts = slices;
+    }
     for (int o = threadIdx.x; o < kDenseTile * M1; o += blockDim.x) {
         float z = 0.f;
-#pragma unroll
-        for (int w = 0; w < 8; w++) z += red[w * kDenseTile * M1 + o];
+#pragma unroll 8
+        for (int w = 0; w < parts; w++) z += red[w * kDenseTile * M1 + o];
         const int p = o / M1, r = o % M1;
         const float v = act_fwd(a.act[0], z + a.B[0][k * M1 + r]);
         s_a1[p][r] = v;

@@ -28,6 +28,8 @@ __host__ __device__ inline int one_rows(int K1) {
 }
 __host__ __device__ inline size_t one_smem(int K1) { return ((size_t)kOneStages * one_rows(K1) + 1) * K1 * sizeof(float); }
 
+__device__ __forceinline__ float4 square4(float4 v) { return make_float4(v.x * v.x, v.y * v.y, v.z * v.z, v.w * v.w); }
+
 struct OneArgs {
     const float* x;        // [n][K1]
     const int* buckets;    // [n]
@@ -45,16 +47,19 @@ struct OneArgs {
     float* gW;             // l1w [column][bucket]
     float* gB;
     int want_grad, units_per_run;
+    int* gave_up;          // pinned word, raised if a wait runs out
     unsigned long long* stamp;
 };
 
-static __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __grid_constant__ OneArgs a) {
+// SQUARE: x holds the roots of its values (activation 3 of kernels_ft.cuh).
+template <bool SQUARE>
+__global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __grid_constant__ OneArgs a) {
     step_begin(a.stamp);
     extern __shared__ __align__(128) float one_smem_raw[];
     __shared__ uint64_t full[kOneStages];
     __shared__ int s_pos[kOneStages][32], s_rows[kOneStages], s_bucket[kOneStages];
     __shared__ float4 s_sum[kOneThreads];
-    __shared__ float s_target[kOneStages][32], s_part[8], s_dout[32], s_loss[32], s_bias;
+    __shared__ float s_part[8], s_dout[32], s_loss[32], s_bias;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int P = one_rows(a.K1), per_tile = kDenseTile / P, cols4 = a.K1 / 4;
     float* s_w = one_smem_raw + (size_t)kOneStages * P * a.K1;
@@ -66,7 +71,6 @@ static __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __g
     __syncthreads();
     // Warp 0 fetches: what unit u holds (one unit ahead of its copies, so that the look-ups are not waited for) ...
     int f_pos = 0, f_rows = 0, f_bucket = 0;
-    float f_target = 0.f;
     auto look_up = [&](int u) {
         f_rows = 0;
         if (u < u_end) {
@@ -76,13 +80,12 @@ static __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __g
             if (lane < f_rows) {
                 f_pos = dense_order_at(a.order, t.x + at + lane);
                 if (a.O > 1 && lane == 0) f_bucket = a.buckets[f_pos];
-                if (a.want_grad) f_target = a.targets[f_pos];
             }
         }
     };
     // ... and its rows, one copy per lane
     auto issue = [&](int stage) {
-        if (lane < f_rows) s_pos[stage][lane] = f_pos, s_target[stage][lane] = f_target;
+        if (lane < f_rows) s_pos[stage][lane] = f_pos;
         if (lane == 0) {
             s_rows[stage] = f_rows;
             s_bucket[stage] = f_bucket;
@@ -145,7 +148,11 @@ static __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __g
                 for (int c = tid; c < cols4; c += kOneThreads) reinterpret_cast<float4*>(s_w)[c] = __ldg(reinterpret_cast<const float4*>(a.W + (size_t)k * a.K1) + c);
                 __syncthreads();
             }
-            if (!mbar_wait(&full[stage], (step / kOneStages) & 1)) return;
+            const float target = a.want_grad && in_row == 0 && row < rows ? __ldg(a.targets + s_pos[stage][row]) : 0.f;  // (arrives under the sums)
+            if (!mbar_wait(&full[stage], (step / kOneStages) & 1)) {
+                *a.gave_up = 1;
+                return;
+            }
             const float4* x = reinterpret_cast<const float4*>(one_smem_raw + (size_t)stage * P * a.K1);
             float dot = 0.f;
             if (row < rows) {
@@ -153,7 +160,9 @@ static __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __g
                 float4 d4 = make_float4(0, 0, 0, 0);
 #pragma unroll 4
                 for (int c = in_row; c < cols4; c += per_row) {
-                    const float4 v = xr[c], w = reinterpret_cast<const float4*>(s_w)[c];
+                    float4 v = xr[c];
+                    const float4 w = reinterpret_cast<const float4*>(s_w)[c];
+                    if (SQUARE) v = square4(v);
                     d4.x += v.x * w.x, d4.y += v.y * w.y, d4.z += v.z * w.z, d4.w += v.w * w.w;
                 }
                 dot = (d4.x + d4.y) + (d4.z + d4.w);
@@ -173,7 +182,7 @@ static __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __g
                     if (a.out_host) a.out_host[b] = o;
                     if (a.want_grad) {
                         const float s = 1.f / (1.f + expf(-o));
-                        const float diff = s - s_target[stage][row];
+                        const float diff = s - target;
                         s_loss[row] = diff * diff;
                         dout = (diff + diff) * (s * (1.f - s));
                         a.dout[b] = dout;
@@ -192,12 +201,14 @@ static __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __g
                         for (int i = 0; i < 4; i++) {
                             const int c4 = col + i * kOneThreads;
                             if (c4 >= cols4) break;
-                            const float4 v = x[(size_t)r * cols4 + c4];
+                            float4 v = x[(size_t)r * cols4 + c4];
+                            if (SQUARE) v = square4(v);
                             acc[i].x += d * v.x, acc[i].y += d * v.y, acc[i].z += d * v.z, acc[i].w += d * v.w;
                         }
                     }
             }
         } else if (!mbar_wait(&full[stage], (step / kOneStages) & 1)) {
+            *a.gave_up = 1;
             return;
         }
         __syncthreads();  // the stage is free again (and its new description is read several barriers later)

@@ -76,7 +76,7 @@ __device__ __forceinline__ void ft_step_begin(const FtArgs& a) {
 
 struct TileArgs {
     int block_rows;          // R
-    int nslabs;              // H/64 column slabs
+    int nslabs;              // column slabs of 64 (the last may be partly filled)
     // A launch covers the row blocks [first_block, last_block) with gridDim.x CTAs.  The work of those
     // blocks is laid out in one line (block by block; inside a block column slab by column slab; inside a
     // slab pair by pair, for the backward chunk by chunk) and CTA k takes the k-th of gridDim.x near-equal
@@ -98,8 +98,9 @@ struct TileArgs {
     uint16_t* csr_ent;             // [nchunks][ent_cap] pairs of the chunk grouped by row, every list starting on 16 bytes
     int* csr_start;                // [nchunks][start_cap] per row (start / 8) << 16 | length; [R] = entries in all
     int ent_cap, start_cap;
-    int grab;                      // rows a warp of the backward takes from the row counter at a time
+    int grab;                      // eighths of the list pieces that the backward deals out in advance
     int chunk_len;  // CP: most pairs per chunk
+    int wide;       // 1024 threads per CTA, one per SM; else 512 and two
     // backward only, data-parallel runs: the last CTA of every row block tells all ranks that the block's
     // gradient is complete (done_count null: nobody is told)
     BucketSignal sig;
@@ -107,13 +108,19 @@ struct TileArgs {
 
 __device__ __forceinline__ float crelu_f(float v) { return fminf(fmaxf(v, 0.f), 1.f); }
 
-// activation of the FT output: 1 = crelu, 2 = screlu
+// activation of the FT output: 1 = crelu, 2 = screlu, 3 = screlu kept as its root: the buffer holds the clamped value, and
+// whoever reads it squares it.  The root of fl(c * c) is c to the last bit, so the derivative needs no square root (which made
+// the backward's staging twice as long as with crelu) and nothing else changes.
 __device__ __forceinline__ float ft_act_fwd(int act, float v) {
     const float c = crelu_f(v);
     return act == 2 ? c * c : c;
 }
 // d(activation)/d(input) as a function of the activation OUTPUT y (dfo.rs:70-88)
 __device__ __forceinline__ float ft_act_bwd(int act, float y) {
+    if (act == 3) {
+        const float sq = __fmul_rn(y, y);
+        return sq > 0.f && (1.f - sq) > 0.f ? y + y : 0.f;
+    }
     const float c = (y > 0.f && (1.f - y) > 0.f) ? 1.f : 0.f;
     if (act != 2) return c;
     const float half = c * sqrtf(y);
@@ -426,15 +433,17 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
             // element exactly as the reference forms `l0w + l0f.repeat(n)` (model/builder.rs:421-424)
             const float* src = a.table + (size_t)block * R * a.H;
             const int q = threadIdx.x & 7, c0 = PAIRWISE ? slab * 32 + q * 4 : slab * 64 + q * 4, c1 = PAIRWISE ? a.H / 2 + c0 : c0 + 32;
+            const bool in0 = c0 < x_row, in1 = PAIRWISE ? in0 : c1 < x_row;  // the last slab of a width that 64 does not divide
 #pragma unroll 3
             for (int row = threadIdx.x >> 3; row < R; row += kFwdThreads / 8) {
                 float4* dst = reinterpret_cast<float4*>(tile + row * kTileCols);
-                float4 v0 = ld_once4(reinterpret_cast<const float4*>(src + (size_t)row * a.H + c0));
-                float4 v1 = ld_once4(reinterpret_cast<const float4*>(src + (size_t)row * a.H + c1));
+                float4 v0 = make_float4(0, 0, 0, 0), v1 = v0;
+                if (in0) v0 = ld_once4(reinterpret_cast<const float4*>(src + (size_t)row * a.H + c0));
+                if (in1) v1 = ld_once4(reinterpret_cast<const float4*>(src + (size_t)row * a.H + c1));
                 if (a.factor) {
                     const float* frow = a.factor + (size_t)((block * R + row) % a.factor_rows) * a.H;
-                    v0 = add4(v0, __ldg(reinterpret_cast<const float4*>(frow + c0)));
-                    v1 = add4(v1, __ldg(reinterpret_cast<const float4*>(frow + c1)));
+                    if (in0) v0 = add4(v0, __ldg(reinterpret_cast<const float4*>(frow + c0)));
+                    if (in1) v1 = add4(v1, __ldg(reinterpret_cast<const float4*>(frow + c1)));
                 }
                 if (PAIRWISE) {
                     // the tile row holds (low-half column, its high-half partner) side by side, both factors of one product.
@@ -453,8 +462,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
         }
         // this lane's columns: two products, or four neighbours
         const int col = PAIRWISE ? slab * 32 + 2 * l16 : slab * 64 + 4 * l16;
-        f32x4 bias;
-        if (PAIRWISE) {
+        f32x4 bias = {0, 0};
+        const bool col_on = col < x_row;
+        if (!col_on) {
+        } else if (PAIRWISE) {
             const float2 lo = *reinterpret_cast<const float2*>(a.bias + col), hi = *reinterpret_cast<const float2*>(a.bias + a.H / 2 + col);
             bias = {pack2(lo.x, hi.x), pack2(lo.y, hi.y)};
         } else {
@@ -484,7 +495,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
             fetch(i + 2 * NW);
             __syncwarp();
             const f32x4 acc = add2(sum_lines(smem_raw, list, cnt, lane16), bias);
-            if (i + half < seg_end) {
+            if (i + half < seg_end && col_on) {
                 if (PAIRWISE) {
                     const float2 ulo = make_float2(crelu_f(lo2(acc.a)), crelu_f(lo2(acc.b))), uhi = make_float2(crelu_f(hi2(acc.a)), crelu_f(hi2(acc.b)));
                     float* up = a.u + (size_t)pair * a.H + col;
@@ -515,13 +526,10 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
 // instead of one per (row, position).  The table gradient must be zero on entry.
 constexpr int kCsrThreads = 512;
 
-// Two shapes of the backward: "wide" = one CTA of 1024 threads per SM working on chunks of 512
-// pairs, otherwise two CTAs of 512 threads on chunks of 256, so that one CTA's global loads
-// overlap the other's shared-memory work.  Chunks halve when nnz > 32.
-__host__ __device__ inline int ft_bwd_chunk(int nnz, bool wide) { return (wide ? 512 : 256) / (nnz <= 32 ? 1 : 2); }
-// The wide shape takes 640-pair chunks where they fit (768-row blocks with 32 slots: 223 KB): a fifth fewer
-// list copies, barriers and per-row reductions for the same walk; measured 2 % faster at 131072 positions.
-__host__ __device__ inline int ft_bwd_chunk_large(int nnz) { return 640 / (nnz <= 32 ? 1 : 2); }
+// Two shapes of the backward: "wide" = one CTA of 1024 threads per SM, otherwise two CTAs of 512 threads on chunks of 256
+// pairs (half of it when nnz > 32), so that one CTA's global loads overlap the other's shared-memory work.
+constexpr int kChunkLeast = 128, kChunkMost = 640;  // pairs per chunk of the wide shape
+__host__ __device__ inline int ft_bwd_chunk_narrow(int nnz) { return nnz <= 32 ? 256 : 128; }
 // Most entries of a piece: the pieces of a chunk differ in length by little from one warp's next to another's, and a king's
 // row, which half the pairs of a chunk may hold, is shared out.
 constexpr int kPiece = 64;
@@ -654,34 +662,55 @@ static __global__ void __launch_bounds__(kCsrThreads) ft_csr_kernel(FtArgs a, Ti
 }
 
 // The backward's work line: block b contributes, per column slab, its pairs plus a fixed amount per chunk
-// (the one reduction per row costs about as much as this many pairs).  A unit is one (block, chunk, slab);
-// units are numbered block by block, chunk by chunk, and slab by slab INSIDE a chunk: a CTA that takes
+// (the one reduction per row costs about as much as this many pairs).  A unit is one (chunk, slab);
+// units are numbered chunk by chunk, and slab by slab INSIDE a chunk: a CTA that takes
 // consecutive units keeps the chunk's row lists (which do not depend on the slab) in shared memory for all
 // slabs, and reads neighbouring 128- or 256-byte pieces of the same activation rows from one unit to the next.
 constexpr int kChunkFixed = 96;
-__host__ __device__ inline long long ft_bwd_block_weight(int pairs, int chunks) { return pairs + (long long)kChunkFixed * chunks; }
-__host__ __device__ inline long long ft_bwd_line(const int* block_begin, const int* chunk_begin, int first_block, int last_block, int nslabs) {
+// The units [x, y) of CTA `k` of `parts`, counted from the launch's first chunk: those between the k-th and the (k+1)-th of
+// `parts` equal cuts of the line.  A whole warp, a lane per block, so that the blocks' tables cost one load latency.
+__device__ __forceinline__ int2 ft_bwd_units(const TileArgs& t, int k, int parts, int lane) {
     long long line = 0;
-    for (int b = first_block; b < last_block; b++)
-        line += nslabs * ft_bwd_block_weight(block_begin[b + 1] - block_begin[b], chunk_begin[b + 1] - chunk_begin[b]);
-    return line;
-}
-// the unit that holds position `at` of the line (the number of units if `at` is the line's end)
-__host__ __device__ inline int ft_bwd_unit_at(long long at, const int* block_begin, const int* chunk_begin, int first_block, int last_block,
-                                              int nslabs) {
+    for (int b0 = t.first_block; b0 < t.last_block; b0 += 32) {
+        const int b = b0 + lane;
+        int w = 0;
+        if (b < t.last_block) w = t.block_begin[b + 1] - t.block_begin[b] + kChunkFixed * (t.chunk_begin[b + 1] - t.chunk_begin[b]);
+        line += __reduce_add_sync(0xffffffffu, w);
+    }
+    line *= t.nslabs;
+    // (rounded up: units that divide evenly over the CTAs must not fall just short of their cut)
+    const long long cut[2] = {(line * k + parts - 1) / parts, (line * (k + 1) + parts - 1) / parts};
+    int unit[2] = {-1, -1};
     long long base = 0;
     int units = 0;
-    for (int b = first_block; b < last_block; b++) {
-        const int nch = chunk_begin[b + 1] - chunk_begin[b];
-        const long long wb = ft_bwd_block_weight(block_begin[b + 1] - block_begin[b], nch);
-        if (nch > 0 && at < base + nslabs * wb) {
-            const long long j = (at - base) * nch / wb;  // a block's chunks are of equal size, so its units weigh the same
-            return units + (int)(j < (long long)nslabs * nch - 1 ? j : (long long)nslabs * nch - 1);
+    for (int b0 = t.first_block; b0 < t.last_block; b0 += 32) {
+        const int b = b0 + lane;
+        int nch = 0, w = 0;
+        if (b < t.last_block) {
+            nch = t.chunk_begin[b + 1] - t.chunk_begin[b];
+            w = t.block_begin[b + 1] - t.block_begin[b] + kChunkFixed * nch;
         }
-        base += nslabs * wb;
-        units += nslabs * nch;
+        int w_incl = w, c_incl = nch;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int wu = __shfl_up_sync(0xffffffffu, w_incl, o), cu = __shfl_up_sync(0xffffffffu, c_incl, o);
+            if (lane >= o) w_incl += wu, c_incl += cu;
+        }
+        const long long first = base + (long long)t.nslabs * (w_incl - w);
+        for (int e = 0; e < 2; e++) {
+            const bool here = nch > 0 && cut[e] >= first && cut[e] < first + (long long)t.nslabs * w;
+            int at = 0;
+            if (here) {  // a block's chunks are of equal size, so its units weigh the same
+                const long long j = (cut[e] - first) * nch / w;
+                at = units + t.nslabs * (c_incl - nch) + (int)(j < (long long)t.nslabs * nch - 1 ? j : (long long)t.nslabs * nch - 1);
+            }
+            const unsigned m = __ballot_sync(0xffffffffu, here);
+            if (m) unit[e] = __shfl_sync(0xffffffffu, at, __ffs(m) - 1);
+        }
+        base += (long long)t.nslabs * __shfl_sync(0xffffffffu, w_incl, 31);
+        units += t.nslabs * __shfl_sync(0xffffffffu, c_incl, 31);
     }
-    return units;
+    return make_int2(unit[0] < 0 ? units : unit[0], unit[1] < 0 ? units : unit[1]);
 }
 
 // grid = one CTA of 1024 threads per SM (or two of 512); CTA k takes the units between the k-th and
@@ -712,9 +741,8 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
     float* bias_s = reinterpret_cast<float*>(pairs_s + CP);                                // [warps][64] bias-gradient sums of a unit
     int2* one_s = reinterpret_cast<int2*>(bias_s + NW * kTileCols);                        // ONE: [CP] (loss gradient, first weight) of the pair
     __shared__ int next_piece;  // the walk's counter
-    const long long line = ft_bwd_line(t.block_begin, t.chunk_begin, t.first_block, t.last_block, t.nslabs);
-    const int u_begin = ft_bwd_unit_at(line * blockIdx.x / gridDim.x, t.block_begin, t.chunk_begin, t.first_block, t.last_block, t.nslabs);
-    const int u_end = ft_bwd_unit_at(line * (blockIdx.x + 1) / gridDim.x, t.block_begin, t.chunk_begin, t.first_block, t.last_block, t.nslabs);
+    const int first_chunk = t.chunk_begin[t.first_block];
+    const int2 mine = SIGNAL ? make_int2(blockIdx.x, t.nslabs * (t.chunk_begin[t.last_block] - first_chunk)) : ft_bwd_units(t, blockIdx.x, gridDim.x, lane);
 
     // lanes of a warp per staged pair, and the four floats of the line that a lane holds: with pairwise the line is the 32
     // low-half columns, then the 32 high-half ones, so that a lane of the walk owns four neighbouring columns of the table
@@ -726,28 +754,44 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
     // Bias gradient: a warp leaves the sums of the pairs it staged in its line of bias_s; during the walk two warps add the
     // lines up, a thread per column, and reduce the result to global memory.  (Shared-memory float atomics in their place
     // took an eighth of all passes through the shared-memory pipe.)
-    int slab = -1, block = -1, ch_loaded = -1;
-    int scan_block = t.first_block, scan_base = 0;  // units before scan_block
-    int all_units = 0, left_block = -1;             // SIGNAL: a block this CTA has left and not yet announced
-    if (SIGNAL) all_units = t.nslabs * (t.chunk_begin[t.last_block] - t.chunk_begin[t.first_block]);
-    for (int u = SIGNAL ? (int)blockIdx.x : u_begin; u < (SIGNAL ? all_units : u_end); u += SIGNAL ? (int)gridDim.x : 1) {
-        int nch = t.chunk_begin[scan_block + 1] - t.chunk_begin[scan_block];
-        while (u >= scan_base + t.nslabs * nch) {
-            scan_base += t.nslabs * nch;
-            scan_block++;
-            nch = t.chunk_begin[scan_block + 1] - t.chunk_begin[scan_block];
+    // staging: this lane's operands of the next U pairs on their way
+    constexpr int U = PAIRWISE ? 2 : 4;
+    float4 y0[U], y1[U], d[U];
+    const int x_row = PAIRWISE ? a.H / 2 : a.H;  // columns of x per perspective
+    auto fetch = [&](int pl0, int cn, int sl) {
+        const int col = PAIRWISE ? sl * 32 + 4 * q : sl * 64 + 4 * q;
+#pragma unroll
+        for (int k = 0; k < U; k++) {
+            const int pl = pl0 + k * NW * kPairsPerWarp;
+            if (pl >= cn) break;
+            if (col >= x_row) {  // the last slab of a width that 64 does not divide
+                y0[k] = y1[k] = d[k] = make_float4(0, 0, 0, 0);
+                continue;
+            }
+            const int pair = pairs_s[pl];
+            const float* y = (PAIRWISE ? a.u : a.x) + (size_t)pair * a.H + col;
+            y0[k] = ld_once4(reinterpret_cast<const float4*>(y));
+            if (PAIRWISE) y1[k] = ld_once4(reinterpret_cast<const float4*>(y + a.H / 2));
+            d[k] = ONE ? __ldg(reinterpret_cast<const float4*>(a.w1 + one_s[pl].y + col))
+                       : ld_once4(reinterpret_cast<const float4*>(a.dx + (size_t)pair * x_row + col));
         }
-        const int local = u - scan_base, ch = t.chunk_begin[scan_block] + local / t.nslabs;
-        slab = local % t.nslabs;
-        if (scan_block != block) {
-            if (SIGNAL && block >= 0) {
+    };
+    bool fetched = false;  // the unit before has fetched this one's first pairs
+    int block = -1, ch_loaded = -1, cn = 0;
+    int left_block = -1;  // SIGNAL: a block this CTA has left and not yet announced
+    int ch = first_chunk + mine.x / t.nslabs, slab = mine.x % t.nslabs;
+    for (int u = mine.x; u < mine.y; u += SIGNAL ? (int)gridDim.x : 1) {
+        int c0 = 0;
+        if (ch != ch_loaded) {
+            const int4 chunk = t.chunks[ch];
+            c0 = chunk.y;
+            cn = chunk.z;
+            if (SIGNAL && block >= 0 && chunk.x != block) {
                 if (left_block >= 0) bucket_signal(t.sig, left_block);  // (only if a whole block went by within one unit)
                 left_block = block;
             }
-            block = scan_block;
+            block = chunk.x;
         }
-        const int4 chunk = t.chunks[ch];
-        const int c0 = chunk.y, cn = chunk.z;
         // the chunk's row lists, unless the unit before left them here: asynchronous copy into shared memory,
         // overlapped with the staging below
         if (ch != ch_loaded) {
@@ -759,35 +803,15 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
             for (int k = threadIdx.x; k < cn; k += kBwdThreads) {
                 const int pair = __ldg(t.pairs + c0 + k).x;
                 pairs_s[k] = pair;
-                if (ONE) {
-                    const int row = PAIRWISE ? a.H / 2 : a.H;  // columns of x per perspective
-                    one_s[k] = make_int2(__float_as_int(a.dout[pair >> 1]), (2 * a.out_bucket[pair >> 1] + (pair & 1)) * row);
-                }
+                if (ONE) one_s[k] = make_int2(__float_as_int(a.dout[pair >> 1]), (2 * a.out_bucket[pair >> 1] + (pair & 1)) * x_row);
             }
             ch_loaded = ch;
             __syncthreads();  // the pair ids are in place
         }
         // stage this chunk's gradients at the feature-transformer pre-activation
         float4 sum_a = make_float4(0, 0, 0, 0), sum_b = sum_a;
-        const int col = PAIRWISE ? slab * 32 + 4 * q : slab * 64 + 4 * q;
-        constexpr int U = PAIRWISE ? 2 : 4;  // pairs in flight per lane
+        if (!fetched) fetch(warp * kPairsPerWarp + sub, cn, slab);
         for (int pl0 = warp * kPairsPerWarp + sub; pl0 < cn; pl0 += U * NW * kPairsPerWarp) {
-            float4 y0[U], y1[U], d[U];
-#pragma unroll
-            for (int k = 0; k < U; k++) {
-                const int pl = pl0 + k * NW * kPairsPerWarp;
-                if (pl >= cn) break;
-                const int pair = pairs_s[pl];
-                const float4* p0 = reinterpret_cast<const float4*>((PAIRWISE ? a.u : a.x) + (size_t)pair * a.H + col);
-                const float4* pd = ONE ? reinterpret_cast<const float4*>(a.w1 + one_s[pl].y + col)
-                                       : reinterpret_cast<const float4*>(a.dx + (size_t)pair * (PAIRWISE ? a.H / 2 : a.H) + col);
-                y0[k] = ld_once4(p0);
-                if (PAIRWISE) {
-                    const float4* p1 = p0 + a.H / 8;  // (H / 2 floats on)
-                    y1[k] = ld_once4(p1);
-                }
-                d[k] = ONE ? __ldg(pd) : ld_once4(pd);
-            }
 #pragma unroll
             for (int k = 0; k < U; k++) {
                 const int pl = pl0 + k * NW * kPairsPerWarp;
@@ -810,6 +834,7 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
                     sum_a = add4(sum_a, ga);
                 }
             }
+            fetch(pl0 + U * NW * kPairsPerWarp, cn, slab);
         }
         if (threadIdx.x == 0) next_piece = 0;
 #pragma unroll
@@ -833,19 +858,22 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
         }
         // The next unit of a CTA that walks consecutive units is the same chunk's next slab: ask L2 for the lines
         // its staging will read (the neighbours of the ones just staged) now, so that they arrive during the walk.
-        if (!SIGNAL && slab + 1 < t.nslabs && u + 1 < u_end && (int)threadIdx.x < cn) {
-            const int pair = pairs_s[threadIdx.x];
+        const bool next_slab = !SIGNAL && slab + 1 < t.nslabs && u + 1 < mine.y;
+        if (next_slab && (int)threadIdx.x < cn) {
+            const int pair = pairs_s[threadIdx.x], col = (slab + 1) * (PAIRWISE ? 32 : 64);
             if (PAIRWISE) {
-                const float* pu = a.u + (size_t)pair * a.H + (slab + 1) * 32;
+                const float* pu = a.u + (size_t)pair * a.H + col;
                 prefetch_l2(pu);
                 prefetch_l2(pu + a.H / 2);
-                if (!ONE) prefetch_l2(a.dx + (size_t)pair * (a.H / 2) + (slab + 1) * 32);
+                if (!ONE) prefetch_l2(a.dx + (size_t)pair * x_row + col);
             } else {
-                const size_t at = (size_t)pair * a.H + (slab + 1) * 64;
+                const size_t at = (size_t)pair * a.H + col;
                 if (!ONE) prefetch_l2(a.dx + at);
-                if (!ONE) prefetch_l2(a.dx + at + 32);
                 prefetch_l2(a.x + at);
-                prefetch_l2(a.x + at + 32);
+                if (col + 32 < x_row) {
+                    if (!ONE) prefetch_l2(a.dx + at + 32);
+                    prefetch_l2(a.x + at + 32);
+                }
             }
         }
         // the four table columns this lane sums
@@ -859,18 +887,38 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
             if (sum != 0.f) atomicAdd(a.g_bias + (!PAIRWISE ? slab * 64 + j : j < 32 ? slab * 32 + j : a.H / 2 + slab * 32 + j - 32), sum);
         }
         const int pieces = start[1];
+        auto walk = [&](unsigned piece) {
+            const f32x4 acc = sum_lines(smem_raw, reinterpret_cast<const uint2*>(ent) + (piece >> 17), (int)(piece >> 10) & 0x7f, lane16);
+            const float4 g = make_float4(lo2(acc.a), hi2(acc.a), lo2(acc.b), hi2(acc.b));
+            if (g.x != 0.f || g.y != 0.f || g.z != 0.f || g.w != 0.f)
+                atomicAdd(reinterpret_cast<float4*>(g_block + (size_t)(piece & 0x3ffu) * a.H), g);
+        };
+        // most pieces are dealt to the half warps, to and fro, so that each gets the same mixture of lengths; the shortest are
+        // handed out by a counter to whoever is done first
+        constexpr int HW = 2 * NW;
+        const int h = 2 * warp + half, dealt = pieces / HW * t.grab / 8;
+        unsigned piece = dealt > 0 ? (unsigned)start[4 + h] : 0u;
+        for (int r = 0; r < dealt; r++) {
+            const unsigned now = piece;
+            if (r + 1 < dealt) piece = (unsigned)start[4 + (r + 1) * HW + (r & 1 ? h : HW - 1 - h)];
+            walk(now);
+        }
+        __syncwarp();
         for (;;) {
             int first = 0;
-            if (lane == 0) first = atomicAdd(&next_piece, t.grab);
-            first = __shfl_sync(0xffffffffu, first, 0);
-            if (first >= pieces) break;
-            for (int p = first + half; p < min(pieces, first + t.grab); p += 2) {
-                const unsigned piece = (unsigned)start[4 + p];
-                const f32x4 acc = sum_lines(smem_raw, reinterpret_cast<const uint2*>(ent) + (piece >> 17), (int)(piece >> 10) & 0x7f, lane16);
-                const float4 g = make_float4(lo2(acc.a), hi2(acc.a), lo2(acc.b), hi2(acc.b));
-                if (g.x != 0.f || g.y != 0.f || g.z != 0.f || g.w != 0.f)
-                    atomicAdd(reinterpret_cast<float4*>(g_block + (size_t)(piece & 0x3ffu) * a.H), g);
-            }
+            if (lane == 0) first = atomicAdd(&next_piece, 2);
+            first = __shfl_sync(0xffffffffu, first, 0) + dealt * HW + half;
+            if (first < pieces) walk((unsigned)start[4 + first]);
+            if (first - half + 2 >= pieces) break;
+        }
+        fetched = next_slab;
+        if (next_slab) fetch(warp * kPairsPerWarp + sub, cn, slab + 1);  // (arrives while the slowest warps finish)
+        if (SIGNAL) {
+            ch = first_chunk + (u + (int)gridDim.x) / t.nslabs;
+            slab = (u + (int)gridDim.x) % t.nslabs;
+        } else if (++slab == t.nslabs) {
+            slab = 0;
+            ch++;
         }
         __syncthreads();
     }

@@ -158,14 +158,15 @@ __global__ void __launch_bounds__(256) step_update_kernel(const __grid_constant_
     }
     const long long stride = (long long)gridDim.x * blockDim.x, me = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     auto update = [&](const AdamSegment& s, long long i, float4 g) {
-        float4 p = a.p[i], m = a.m[i], v = a.v[i];
+        // (the moments are not needed before the next update: they leave L2 to the weights)
+        float4 p = a.p[i], m = __ldcs(a.m + i), v = __ldcs(a.v + i);
         adam_op(s, a.rate, a.adj * g.x, p.x, m.x, v.x);
         adam_op(s, a.rate, a.adj * g.y, p.y, m.y, v.y);
         adam_op(s, a.rate, a.adj * g.z, p.z, m.z, v.z);
         adam_op(s, a.rate, a.adj * g.w, p.w, m.w, v.w);
         a.p[i] = p;
-        a.m[i] = m;
-        a.v[i] = v;
+        __stcs(a.m + i, m);
+        __stcs(a.v + i, v);
         return p;
     };
     if (u.l0f_seg >= 0) {

@@ -73,9 +73,9 @@ struct Tensor {
 struct Slot {
     char* d_blob = nullptr;
     char* h_blob = nullptr;
-    size_t capacity = 0;
     int n = 0;
     int n_dtiles = 0;  // CTA tiles of the dense kernels: as many as there can be, the rest are empty
+    bool wide = true;                 // shape of the tiled backward that its chunks were cut for
     int n_chunks = 0, chunk_len = 0;  // the same for the chunks of the tiled FT backward held in off_chunks, and their size
     int expect_grid = 0;              // grid size the per-block CTA counts in off_bexpect were made for
     // derived from the indices alone, so built once per upload on the copy stream (or on first use):
@@ -114,6 +114,8 @@ struct b200_net {
     int64_t n_flat = 0;
     float *P = nullptr, *G = nullptr, *M = nullptr, *V = nullptr, *table = nullptr;
     float *x = nullptr, *u = nullptr, *dx = nullptr, *a1 = nullptr, *a2 = nullptr, *out = nullptr, *w1g = nullptr;
+    float* dense_partial = nullptr;  // the dense forward's sums of split tiles
+    int* dense_arrived = nullptr;
     float4 *w1f = nullptr, *w1d = nullptr;  // the first dense layer's fragment tables (dense_mma)
     float* dz[3] = {nullptr, nullptr, nullptr};
     int wgrad_per_sm = 0;          // resident CTAs per SM of the first layer's weight-gradient kernel (looked up once)
@@ -123,6 +125,7 @@ struct b200_net {
     int* h_status = nullptr;
     int* d_status = nullptr;       // [kLossRing] the slot's status word, saved before the slot is released to the uploader
     float* h_loss = nullptr;
+    char* h_pinned = nullptr;      // the one pinned allocation that the slots' blocks, h_out and the ring lie in
     float* h_out = nullptr;        // pinned [max_batch]: network outputs of an evaluation
     cudaEvent_t loss_ev[kLossRing] = {};
     int64_t updates = 0;
@@ -131,13 +134,23 @@ struct b200_net {
     bool bwd_wide = true;  // shape of the tiled backward (see ft_bwd_chunk)
     int exchange_bulk = 0;  // the peer exchange moves gradients and weights with bulk asynchronous copies (measured no faster)
     int bwd_grab = 0;  // rows a warp of the tiled backward takes from the row counter at a time (0: chosen by block size)
-    int wide_chunk = 0;    // the larger chunk of the 1024-thread backward where it fits into shared memory, else the standard one
-    // Pairs per chunk for a batch of n positions.  The larger chunk saves list copies, barriers and reductions,
-    // but needs enough units to keep every SM's share even: measured faster from about eight units per SM.
+    int wide_chunk = 0;    // the largest chunk of the 1024-thread backward that fits into shared memory
+    // Pairs per chunk for a batch of n positions: large chunks save reductions and list copies per pair, small ones fill the
+    // SMs evenly when there are few units.  Measured, a unit takes a part that grows with the table's rows and the chunk's
+    // pairs (clocks, 768 rows and 17 of 32 slots active: 13.4 k + 48 per pair; 147 rows, 27 of 49: 6.6 k + 78 per pair), and a
+    // CTA takes whole units.
     int bwd_chunk(int n) const {
-        if (!bwd_wide) return b200::ft_bwd_chunk(d.nnz, false);
-        const long long units = (long long)nslabs * ((2LL * n + wide_chunk - 1) / wide_chunk);
-        return units >= 8LL * sm_count ? wide_chunk : b200::ft_bwd_chunk(d.nnz, true);
+        if (!bwd_wide) return b200::ft_bwd_chunk_narrow(d.nnz);
+        int best = wide_chunk;
+        double least = 1e30;
+        for (int len = wide_chunk; len >= b200::kChunkLeast; len -= 8) {
+            const double chunks = nblocks > 1 ? 2.0 * n / len + 0.5 * nblocks : (double)((2LL * n + len - 1) / len);
+            const double pairs = std::min<double>(len, 2.0 * n / chunks);
+            const double units = chunks * nslabs, rounds = std::ceil(units / sm_count);
+            const double time = rounds * (5000 + 11.0 * block_rows + 1.5 * d.nnz * pairs);
+            if (time < least * 0.995) least = time, best = len;
+        }
+        return best;
     }
     int bwd_slot = -1, bwd_parts_done = 0, bwd_parts = 0;  // progress of a phased backward
     int fwd_slot = -1, fwd_parts_done = 0, fwd_parts = 0;  // progress of a forward pass run in pieces
@@ -151,6 +164,7 @@ struct b200_net {
     long long xch_spin_limit = b200::kPeerWaitSpins;
     int xch_wait_ready = 0;    // value the next exchange launch waits for at kFlagReady (0: the caller fences)
     bool xch_fenced_used = false;
+    int* h_gave_up = nullptr;  // pinned: raised by a kernel whose wait for its own copies ran out
     int* h_xstatus = nullptr;  // pinned ring beside h_status: per update the fence time-out word and what was missing
     bool loss_in_param = false;  // the last update left the summed loss in P[0] instead of G[0]
     int exchange_ctas = 0;          // CTAs of a side-stream exchange launch (0: one per SM)
@@ -170,10 +184,12 @@ struct b200_net {
     bool sig_on = false;                 // the running backward announces finished row blocks
     int sig_value = 0;
     bool manual_grad_zero = false;  // the caller zeroes the gradient buffer range by range (b200_grad_zero_range)
-    bool tiled_ok = false, have_backward = false;
+    bool tiled_ok = false, tiled_promised = false;  // promised: what the caller may ask for by name (FT_TILED)
+    bool have_backward = false;
     bool w1_dirty = true, merged_dirty = true;  // the weights moved since the regrouped first dense layer / the merged table was built
     bool trains = false;  // a training pass has run: uploads then also build what only the backward reads
     int nblocks = 1, nslabs = 1;
+    int block_rows = 0;  // table rows per block: as promised, or a small table as a single block
     int last_n = 0;
     // per-step CUDA events on the compute stream, kept for the last kTimingRing steps
     static constexpr int kTimingRing = 256, kTimingEvents = 8;
@@ -223,6 +239,8 @@ struct b200_net {
     bool fused_small_grads() const { return dense_mma(); }
     // one row per bucket and nothing behind it (and rows that fit the kernel's stages): dense_one_kernel
     bool dense_one() const { return d.n_dense == 1 && D1() <= b200::kOneMaxK; }
+    // such a network's x holds the roots of squared activations (activation 3 of kernels_ft.cuh)
+    bool keep_root() const { return dense_one() && d.ft_act == B200_ACT_SCRELU; }
     // first dense layers of four and more rows per bucket run on the tensor pipe
     bool dense_mma() const { return d.dense_out[0] >= 4; }
 };
@@ -274,6 +292,30 @@ int dev_alloc(b200_net* net, T** p, size_t count) {
     return 0;
 }
 
+// Device buffers to be taken from one allocation.
+struct Plan {
+    struct Item {
+        void** p;
+        size_t bytes;
+    };
+    std::vector<Item> items;
+    template <class T>
+    void add(T** p, size_t count) {
+        items.push_back({reinterpret_cast<void**>(p), align_up(std::max<size_t>(count, 1) * sizeof(T), 256)});
+    }
+    int allocate(b200_net* net) {
+        size_t total = 0;
+        for (const Item& i : items) total += i.bytes;
+        char* base = nullptr;
+        if (int rc = dev_alloc(net, &base, total)) return rc;
+        for (const Item& i : items) {
+            *i.p = base;
+            base += i.bytes;
+        }
+        return 0;
+    }
+};
+
 bool supported_m(int m) { return m == 1 || m == 2 || m == 4 || m == 8 || m == 16 || m == 32; }
 
 int validate(const b200_net_desc& d) {
@@ -320,7 +362,7 @@ void slot_layout(const b200_net* net, Slot& s, int n) {
     s.off_records = take((size_t)n * 32);
     s.off_pairs = take((size_t)n * 16);
     s.off_blocks = take((nb + 1) * 4);
-    s.off_chunks = take(((size_t)2 * n / b200::ft_bwd_chunk(d.nnz, false) + nb + 1) * 16);
+    s.off_chunks = take(((size_t)2 * n / b200::kChunkLeast + nb + 1) * 16);
     s.off_cbegin = take((nb + 1) * 4);
     s.off_bexpect = take(nb * 4);
     s.off_status = take(4);
@@ -366,7 +408,7 @@ template <bool PW>
 int launch_ft_backward(b200_net* net, const b200::FtArgs& a, const b200::TileArgs& t, bool tiled, int grid) {
     if (tiled) {
         const size_t smem = b200::ft_bwd_smem(t.block_rows, a.nnz, t.chunk_len);
-        const bool wide = t.chunk_len > b200::ft_bwd_chunk(a.nnz, false);
+        const bool wide = t.wide;
         if (net->dense_one()) launch_ft_backward_tiled<PW, true>(a, t, wide, grid, smem, net->chained, net->stream);
         else launch_ft_backward_tiled<PW, false>(a, t, wide, grid, smem, net->chained, net->stream);
     } else {
@@ -397,10 +439,18 @@ int launch_ft_backward(b200_net* net, const b200::FtArgs& a, const b200::TileArg
         default: return b200::fail(B200_ERR_UNSUPPORTED, "rows per bucket %d", m); \
     }
 
+// A tile is a chain of loads for its CTA (20 us at 2048 columns): while there are tiles for a quarter of the SMs at most, up to
+// eight CTAs share one.
+constexpr int kMostSlices = 8;
+int dense_slices(const b200_net* net, int ntiles) {
+    const int groups = (net->D1() + b200::kMmaCols - 1) / b200::kMmaCols;
+    return std::max(1, std::min({kMostSlices, net->sm_count / (2 * ntiles), groups / 8}));
+}
+
 template <int MM>
 void launch_dense_forward(b200_net* net, const b200::DenseArgs& da, int ntiles) {
     if constexpr (MM >= 4)
-        b200::launch_step(net->chained, b200::dense_forward_mma_kernel<MM>, ntiles, 256, b200::dense_mma_smem<MM>(), net->stream, da);
+        b200::launch_step(net->chained, b200::dense_forward_mma_kernel<MM>, dim3(ntiles, dense_slices(net, ntiles)), 256, b200::dense_mma_smem<MM>(), net->stream, da);
     else
         b200::launch_step(net->chained, b200::dense_forward_kernel<MM>, ntiles, 256, b200::dense_fwd_smem<MM>(), net->stream, da);
 }
@@ -435,7 +485,7 @@ int ft_forward_grid(const b200_net* net, const Slot& s) {
 }
 int ft_backward_grid(const b200_net* net, const Slot& s, bool beside_exchange) {
     const long long units = (long long)net->nslabs * s.n_chunks;
-    const int per_sm = s.chunk_len > b200::ft_bwd_chunk(net->d.nnz, false) ? 1 : 2;
+    const int per_sm = s.wide ? 1 : 2;
     const int sms = net->sm_count - (beside_exchange ? std::min(net->overlap_ctas, net->sm_count - 1) : 0);
     return (int)std::max<long long>(1, std::min<long long>((long long)sms * per_sm, units));
 }
@@ -449,7 +499,7 @@ b200::FtArgs ft_args(b200_net* net, const Slot& s) {
     a.table = merged ? net->table : net->P + net->find("l0w")->off;
     a.factor = (net->d.factoriser_rows && !merged) ? net->P + net->find("l0f")->off : nullptr;
     a.factor_rows = net->d.factoriser_rows;
-    a.block_rows = net->ft_fwd_mode == B200_FT_AUTO && net->tiled_ok ? d.ft_block_rows : 0;
+    a.block_rows = net->ft_fwd_mode == B200_FT_AUTO && net->tiled_ok ? net->block_rows : 0;
     a.bias = net->P + net->find("l0b")->off;
     a.idx_stm = s.dev<uint16_t>(s.off_stm);
     a.idx_nstm = s.dev<uint16_t>(s.off_nstm);
@@ -457,7 +507,7 @@ b200::FtArgs ft_args(b200_net* net, const Slot& s) {
     a.nnz = d.nnz;
     a.H = d.ft_out;
     a.n_inputs = d.n_inputs;
-    a.act = d.ft_act;
+    a.act = net->keep_root() ? 3 : d.ft_act;
     a.x = net->x;
     a.u = net->u;
     a.dx = net->dx;
@@ -472,7 +522,7 @@ b200::FtArgs ft_args(b200_net* net, const Slot& s) {
 
 b200::TileArgs tile_args(b200_net* net, const Slot& s, bool backward) {
     b200::TileArgs t{};
-    t.block_rows = net->d.ft_block_rows;
+    t.block_rows = net->block_rows;
     t.nslabs = net->nslabs;
     t.first_block = 0;
     t.last_block = net->nblocks;
@@ -486,11 +536,10 @@ b200::TileArgs tile_args(b200_net* net, const Slot& s, bool backward) {
     t.csr_ent = s.csr_ent;
     t.csr_start = s.csr_start;
     t.chunk_len = s.chunk_len;
-    // rows per grab: measured best at eight for 768-row blocks (runs of neighbouring rows per warp, and still four
-    // grabs per warp and unit to even out the list lengths), two to four for the 147-row ataxx table
-    t.grab = net->bwd_grab > 0 ? net->bwd_grab : std::max(2, std::min(8, net->d.ft_block_rows / 96));
-    t.ent_cap = b200::ft_bwd_ent_cap(net->d.ft_block_rows, net->d.nnz, s.chunk_len);
-    t.start_cap = b200::ft_bwd_start_cap(net->d.ft_block_rows, net->d.nnz, s.chunk_len);
+    t.wide = s.wide;
+    t.grab = net->bwd_grab > 0 ? std::min(8, net->bwd_grab) : 6;
+    t.ent_cap = b200::ft_bwd_ent_cap(net->block_rows, net->d.nnz, s.chunk_len);
+    t.start_cap = b200::ft_bwd_start_cap(net->block_rows, net->d.nnz, s.chunk_len);
     if (backward && net->sig_on) {
         t.sig.done_count = net->done_count;
         t.sig.done_expect = s.dev<int>(s.off_bexpect);
@@ -526,6 +575,8 @@ b200::DenseArgs dense_args(b200_net* net, const Slot& s, bool want_grad) {
     a.W1g = net->w1g_now();
     a.W1f = net->w1f;
     a.W1d = net->w1d;
+    a.partial = net->dense_partial;
+    a.arrived = net->dense_arrived;
     a.a1 = net->a1;
     a.a2 = net->a2;
     a.out = net->out;
@@ -589,7 +640,7 @@ b200::GroupArgs group_args(b200_net* net, Slot& s, bool want_lists, bool want_or
     g.n = s.n;
     g.nnz = d.nnz;
     g.n_inputs = d.n_inputs;
-    g.block_rows = net->tiled_ok ? d.ft_block_rows : d.n_inputs;
+    g.block_rows = net->tiled_ok ? net->block_rows : d.n_inputs;
     g.nblocks = net->nblocks;
     g.n_out_buckets = d.n_out_buckets;
     g.info = s.dev<int>(s.off_info);
@@ -626,6 +677,7 @@ void cut_dense(b200_net* net, Slot& s) {
 }
 void cut_ft(b200_net* net, Slot& s) {
     if (!net->tiled_ok) return;
+    s.wide = net->bwd_wide;
     s.chunk_len = net->bwd_chunk(s.n);
     s.n_chunks = most_chunks(net, s.n, s.chunk_len);
     s.expect_grid = ft_backward_grid(net, s, net->overlap_mode);
@@ -657,7 +709,7 @@ int group_slot(b200_net* net, Slot& s, const b200::GroupArgs& g, bool counted, c
 }
 
 int build_csr(b200_net* net, Slot& s, cudaStream_t stream) {
-    b200::ft_csr_kernel<<<s.n_chunks, b200::kCsrThreads, b200::ft_csr_smem(net->d.ft_block_rows, net->d.nnz, s.chunk_len), stream>>>(
+    b200::ft_csr_kernel<<<s.n_chunks, b200::kCsrThreads, b200::ft_csr_smem(net->block_rows, net->d.nnz, s.chunk_len), stream>>>(
         ft_args(net, s), tile_args(net, s, true));
     LAUNCHED(net);
     s.csr_built = true;
@@ -708,11 +760,12 @@ int forward_dense(b200_net* net, Slot& s, bool want_grad) {
         a.gW = net->G + net->find("l1w")->off, a.gB = net->G + net->find("l1b")->off;
         a.want_grad = da.want_grad;
         a.stamp = da.stamp;
+        a.gave_up = net->h_gave_up;
         net->w1_used = da.W1g;
         const size_t smem = b200::one_smem(a.K1);
         const int units = a.ntiles * (b200::kDenseTile / b200::one_rows(a.K1)), slots = net->sm_count * std::max(1, std::min(4, (int)(220 * 1024 / smem)));
         a.units_per_run = (units + slots - 1) / slots;
-        b200::launch_step(net->chained, b200::dense_one_kernel, (units + a.units_per_run - 1) / a.units_per_run, b200::kOneThreads, smem, net->stream, a);
+        b200::launch_step(net->chained, net->keep_root() ? b200::dense_one_kernel<true> : b200::dense_one_kernel<false>, (units + a.units_per_run - 1) / a.units_per_run, b200::kOneThreads, smem, net->stream, a);
         LAUNCHED(net);
         return 0;
     }
@@ -821,7 +874,7 @@ bool load_dense_kernels() {
 int preload_kernels(b200_net* net) {
     bool ok = true;
     DISPATCH_M(net->d.dense_out[0], ok = load_dense_kernels<MM>());
-    ok = ok && load_kernel(b200::dense_regroup_kernel) && load_kernel(b200::dense_one_kernel) && load_kernel(b200::dense_one_dx_kernel) && load_kernel(b200::dense_fragments_kernel) && load_kernel(b200::dense_small_grads_kernel);
+    ok = ok && load_kernel(b200::dense_regroup_kernel) && load_kernel(b200::dense_one_kernel<true>) && load_kernel(b200::dense_one_kernel<false>) && load_kernel(b200::dense_one_dx_kernel) && load_kernel(b200::dense_fragments_kernel) && load_kernel(b200::dense_small_grads_kernel);
     ok = ok && load_kernel(b200::ft_forward_gather_kernel<true>) && load_kernel(b200::ft_forward_gather_kernel<false>);
     ok = ok && load_kernel(b200::ft_backward_gather_kernel<true, true>) && load_kernel(b200::ft_backward_gather_kernel<true, false>) && load_kernel(b200::ft_backward_gather_kernel<false, true>) && load_kernel(b200::ft_backward_gather_kernel<false, false>);
     ok = ok && load_kernel(b200::ft_forward_tiled_kernel<true>) && load_kernel(b200::ft_forward_tiled_kernel<false>);
@@ -922,65 +975,79 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     net->n_flat = (off + 1023) / 1024 * 1024;  // a multiple of 4 floats x 256: splits evenly over up to 256 ranks
 
     constexpr size_t kMaxSmem = 227 * 1024 - 64;  // (the tiled kernels declare a few static bytes)
-    net->tiled_ok = d.ft_block_rows > 0 && d.n_inputs % d.ft_block_rows == 0 && d.ft_out % b200::kTileCols == 0 &&
-                    b200::ft_fwd_smem(d.ft_block_rows, (d.nnz + 7) & ~7) <= kMaxSmem &&
-                    b200::ft_bwd_smem(d.ft_block_rows, d.nnz, b200::ft_bwd_chunk(d.nnz, true)) <= kMaxSmem && d.ft_block_rows < 1024;
-    if (net->tiled_ok) {
-        const int larger = b200::ft_bwd_chunk_large(d.nnz);
-        net->wide_chunk = b200::ft_bwd_smem(d.ft_block_rows, d.nnz, larger) <= kMaxSmem ? larger : b200::ft_bwd_chunk(d.nnz, true);
-    }
-    net->nblocks = net->tiled_ok ? d.n_inputs / d.ft_block_rows : 1;
-    net->nslabs = d.ft_out / b200::kTileCols;
+    // The tiled kernels need features of one perspective that fall into one block.  A table that is small enough is one block
+    // whatever was promised, and then any width will do (a width that 64 does not divide costs as much as the next that does).
+    const bool promised = d.ft_block_rows > 0 && d.n_inputs % d.ft_block_rows == 0 && d.ft_out % b200::kTileCols == 0;
+    const int R = promised ? d.ft_block_rows : d.n_inputs;
+    net->tiled_ok = (promised || (d.pairwise ? d.ft_out / 2 : d.ft_out) >= 32) && R < 1024 &&
+                    b200::ft_fwd_smem(R, (d.nnz + 7) & ~7) <= kMaxSmem &&
+                    b200::ft_bwd_smem(R, d.nnz, 256) <= kMaxSmem;
+    net->tiled_promised = net->tiled_ok && promised;
+    net->block_rows = R;
+    if (net->tiled_ok)
+        for (net->wide_chunk = b200::kChunkMost; b200::ft_bwd_smem(R, d.nnz, net->wide_chunk) > kMaxSmem;) net->wide_chunk -= 8;
+    net->nblocks = net->tiled_ok ? d.n_inputs / R : 1;
+    net->nslabs = (d.ft_out + b200::kTileCols - 1) / b200::kTileCols;
 
     const size_t B = d.max_batch;
+    for (auto& s : net->slots) {
+        slot_layout(net, s, d.max_batch);
+        s.n = 0;
+    }
+    // One allocation for everything but the buffers that peers map: allocations cost a few hundred us each
+    Plan plan;
     int rc = 0;
     rc = rc ? rc : dev_alloc(net, &net->P, net->n_flat);
     rc = rc ? rc : dev_alloc(net, &net->G, net->n_flat);
-    rc = rc ? rc : dev_alloc(net, &net->M, net->n_flat);
-    rc = rc ? rc : dev_alloc(net, &net->V, net->n_flat);
-    if (d.factoriser_rows) rc = rc ? rc : dev_alloc(net, &net->table, (size_t)d.n_inputs * d.ft_out);
-    rc = rc ? rc : dev_alloc(net, &net->x, B * net->D1());
-    if (d.pairwise) rc = rc ? rc : dev_alloc(net, &net->u, B * 2 * d.ft_out);
-    rc = rc ? rc : dev_alloc(net, &net->dx, B * net->D1());
-    rc = rc ? rc : dev_alloc(net, &net->a1, B * d.dense_out[0]);
-    rc = rc ? rc : dev_alloc(net, &net->a2, B * 32);
-    for (int l = 0; l < 3; l++) rc = rc ? rc : dev_alloc(net, &net->dz[l], B * 32);
-    rc = rc ? rc : dev_alloc(net, &net->out, B);
-    rc = rc ? rc : dev_alloc(net, &net->d_stamps, b200_net::kTimingRing * b200_net::kTimingEvents);
-    rc = rc ? rc : dev_alloc(net, &net->d_status, b200_net::kLossRing);
+    plan.add(&net->M, net->n_flat);
+    plan.add(&net->V, net->n_flat);
+    if (d.factoriser_rows) plan.add(&net->table, (size_t)d.n_inputs * d.ft_out);
+    plan.add(&net->x, B * net->D1());
+    if (d.pairwise) plan.add(&net->u, B * 2 * d.ft_out);
+    plan.add(&net->dx, B * net->D1());
+    plan.add(&net->a1, B * d.dense_out[0]);
+    plan.add(&net->a2, B * 32);
+    for (int l = 0; l < 3; l++) plan.add(&net->dz[l], B * 32);
+    plan.add(&net->out, B);
+    plan.add(&net->d_stamps, b200_net::kTimingRing * b200_net::kTimingEvents);
+    plan.add(&net->d_status, b200_net::kLossRing);
     if (net->dense_mma()) {
         const size_t table = b200::mma_table_floats(net->D1(), d.n_out_buckets, d.dense_out[0]) / 4;
-        rc = rc ? rc : dev_alloc(net, &net->w1f, table);
-        rc = rc ? rc : dev_alloc(net, &net->w1d, table);
+        plan.add(&net->w1f, table);
+        plan.add(&net->w1d, table);
+        plan.add(&net->dense_partial, (size_t)net->sm_count * kMostSlices * b200::kDenseTile * d.dense_out[0]);
+        plan.add(&net->dense_arrived, (size_t)net->sm_count);
     } else {
-        rc = rc ? rc : dev_alloc(net, &net->w1g, (size_t)2 * d.n_out_buckets * d.dense_out[0] * net->D1());
-        if (net->dense_one()) rc = rc ? rc : dev_alloc(net, &net->kept_bucket, B);
+        plan.add(&net->w1g, (size_t)2 * d.n_out_buckets * d.dense_out[0] * net->D1());
+        if (net->dense_one()) plan.add(&net->kept_bucket, B);
     }
     // the fence counters get an allocation of their own size class (2 MiB), so that its IPC handle maps exactly it
     rc = rc ? rc : dev_alloc(net, &net->xch_flags, (size_t)(2 << 20) / sizeof(int));
     if (!rc) cudaMemsetAsync(net->xch_flags, 0, (size_t)2 << 20, net->stream);
-    rc = rc ? rc : dev_alloc(net, &net->d_win_rate, 65536);
-    rc = rc ? rc : dev_alloc(net, &net->d_expanded, 64);
-    rc = rc ? rc : dev_alloc(net, &net->d_peers, 1);
-    rc = rc ? rc : dev_alloc(net, &net->done_count, (size_t)net->nblocks);
-    if (!rc) cudaMemsetAsync(net->done_count, 0, (size_t)net->nblocks * sizeof(int), net->stream);
-    if (net->tiled_ok && d.factoriser_rows == d.ft_block_rows)
-        rc = rc ? rc : dev_alloc(net, &net->facc, (size_t)d.ft_block_rows * d.ft_out / 2);
+    plan.add(&net->d_win_rate, 65536);
+    plan.add(&net->d_expanded, 64);
+    plan.add(&net->d_peers, 1);
+    plan.add(&net->done_count, (size_t)net->nblocks);
+    if (net->tiled_promised && d.factoriser_rows == d.ft_block_rows)
+        plan.add(&net->facc, (size_t)d.ft_block_rows * d.ft_out / 2);
     if (net->tiled_ok) {
-        // sized for whichever backward shape needs more: every block may end in a partly filled chunk
+        // sized for whichever chunk length needs more: every block may end in a partly filled chunk
         size_t ent_total = 0, start_total = 0;
-        for (int shape = 0; shape < 3; shape++) {
-            const int cp = shape == 2 ? net->wide_chunk : b200::ft_bwd_chunk(d.nnz, shape != 0);
+        for (int cp : {b200::kChunkLeast, b200::ft_bwd_chunk_narrow(d.nnz), net->wide_chunk}) {
             const size_t chunks = most_chunks(net, (int)B, cp);
-            start_total = std::max(start_total, chunks * b200::ft_bwd_start_cap(d.ft_block_rows, d.nnz, cp));
-            ent_total = std::max(ent_total, chunks * b200::ft_bwd_ent_cap(d.ft_block_rows, d.nnz, cp));
+            start_total = std::max(start_total, chunks * b200::ft_bwd_start_cap(R, d.nnz, cp));
+            ent_total = std::max(ent_total, chunks * b200::ft_bwd_ent_cap(R, d.nnz, cp));
         }
         for (auto& s : net->slots) {
-            rc = rc ? rc : dev_alloc(net, &s.lists, 2 * B * ((d.nnz + 7) & ~7));
-            rc = rc ? rc : dev_alloc(net, &s.csr_ent, ent_total);
-            rc = rc ? rc : dev_alloc(net, &s.csr_start, start_total);
+            plan.add(&s.lists, 2 * B * ((d.nnz + 7) & ~7));
+            plan.add(&s.csr_ent, ent_total);
+            plan.add(&s.csr_start, start_total);
         }
     }
+    for (auto& s : net->slots) plan.add(&s.d_blob, s.bytes);
+    rc = rc ? rc : plan.allocate(net);
+    if (!rc && net->dense_arrived) cudaMemsetAsync(net->dense_arrived, 0, (size_t)net->sm_count * sizeof(int), net->stream);
+    if (!rc) cudaMemsetAsync(net->done_count, 0, (size_t)net->nblocks * sizeof(int), net->stream);
     if (rc) return bail(rc);
     if (!d.factoriser_rows) net->table = net->P + net->find("l0w")->off;
     cudaMemsetAsync(net->P, 0, net->n_flat * 4, net->stream);
@@ -988,27 +1055,26 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     cudaMemsetAsync(net->M, 0, net->n_flat * 4, net->stream);
     cudaMemsetAsync(net->V, 0, net->n_flat * 4, net->stream);
 
-    for (auto& s : net->slots) {
-        slot_layout(net, s, d.max_batch);
-        s.capacity = s.bytes;
+    const size_t pinned_slot = align_up(std::max(net->slots[0].off_records, (size_t)d.max_batch * 32), 4096);
+    {   // pinned memory: the slots' staging blocks, the outputs of an evaluation, the read-back ring
         void* raw = nullptr;
-        if (cudaMalloc(&raw, s.capacity) != cudaSuccess) return bail(b200::fail(B200_ERR_CUDA, "net_create: slot allocation failed"));
-        s.d_blob = static_cast<char*>(raw);
-        if (cudaHostAlloc(&raw, std::max(s.off_records, (size_t)d.max_batch * 32), cudaHostAllocDefault) != cudaSuccess)
-            return bail(b200::fail(B200_ERR_CUDA, "net_create: pinned slot allocation failed"));
-        s.h_blob = static_cast<char*>(raw);
+        const size_t out_bytes = align_up(B * sizeof(float), 4096);
+        if (cudaHostAlloc(&raw, B200_NUM_SLOTS * pinned_slot + out_bytes + 128, cudaHostAllocDefault) != cudaSuccess)
+            return bail(b200::fail(B200_ERR_CUDA, "net_create: pinned allocation failed"));
+        net->h_pinned = static_cast<char*>(raw);
+        net->h_out = reinterpret_cast<float*>(net->h_pinned + B200_NUM_SLOTS * pinned_slot);
+        net->h_loss = reinterpret_cast<float*>(net->h_pinned + B200_NUM_SLOTS * pinned_slot + out_bytes);
+    }
+    for (auto& s : net->slots) {
+        s.h_blob = net->h_pinned + (&s - net->slots) * pinned_slot;
         cudaEventCreateWithFlags(&s.ready, cudaEventDisableTiming);
         cudaEventCreateWithFlags(&s.consumed, cudaEventDisableTiming);
         s.n = 0;
     }
-    void* raw = nullptr;
-    if (cudaHostAlloc(&raw, 128, cudaHostAllocDefault) != cudaSuccess) return bail(b200::fail(B200_ERR_CUDA, "net_create: pinned alloc failed"));
-    net->h_loss = static_cast<float*>(raw);
-    if (cudaHostAlloc(&raw, B * sizeof(float), cudaHostAllocDefault) != cudaSuccess) return bail(b200::fail(B200_ERR_CUDA, "net_create: pinned alloc failed"));
-    net->h_out = static_cast<float*>(raw);
     net->h_status = reinterpret_cast<int*>(net->h_loss + 8);
     net->h_xstatus = net->h_status + b200_net::kLossRing;
-    memset(net->h_loss, 0, 128);  // 8 floats, 4 status words, 4 x 4 fence words
+    net->h_gave_up = net->h_xstatus + 4 * b200_net::kLossRing;
+    memset(net->h_loss, 0, 128);  // 8 floats, 4 status words, 4 x 4 fence words, the wait word
     for (auto& e : net->loss_ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
     {
         constexpr int MM_unused = 0;
@@ -1020,7 +1086,7 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
             return 0;
         };
         if (int rc2 = set_dense(d.dense_out[0])) return bail(rc2);
-        if (b200::allow_smem(b200::dense_one_kernel) != cudaSuccess) return bail(b200::fail(B200_ERR_CUDA, "net_create: shared memory of the dense kernel"));
+        if (b200::allow_smem(b200::dense_one_kernel<true>) != cudaSuccess || b200::allow_smem(b200::dense_one_kernel<false>) != cudaSuccess) return bail(b200::fail(B200_ERR_CUDA, "net_create: shared memory of the dense kernel"));
     }
     if (net->tiled_ok) {
         cudaError_t e = b200::allow_smem(b200::ft_forward_tiled_kernel<true>);
@@ -1070,13 +1136,10 @@ int b200_net_destroy(b200_net* net) {
         }
     for (void* p : net->allocations) cudaFree(p);
     for (auto& s : net->slots) {
-        if (s.d_blob) cudaFree(s.d_blob);
-        if (s.h_blob) cudaFreeHost(s.h_blob);
         if (s.ready) cudaEventDestroy(s.ready);
         if (s.consumed) cudaEventDestroy(s.consumed);
     }
-    if (net->h_loss) cudaFreeHost(net->h_loss);
-    if (net->h_out) cudaFreeHost(net->h_out);
+    if (net->h_pinned) cudaFreeHost(net->h_pinned);
     for (auto& e : net->loss_ev)
         if (e) cudaEventDestroy(e);
     for (auto& ring : net->tev)
@@ -1098,7 +1161,7 @@ int b200_net_set_option(b200_net* net, const char* key, int64_t value) {
     if (!net || !key) return b200::fail(B200_ERR_ARG, "set_option: null argument");
     if (!strcmp(key, "ft_mode") || !strcmp(key, "ft_fwd_mode") || !strcmp(key, "ft_bwd_mode")) {
         if (value < B200_FT_AUTO || value > B200_FT_TILED) return b200::fail(B200_ERR_ARG, "ft_mode %lld unknown", (long long)value);
-        if (value == B200_FT_TILED && !net->tiled_ok)
+        if (value == B200_FT_TILED && !net->tiled_promised)
             return b200::fail(B200_ERR_UNSUPPORTED,
                               "tiled feature-transformer kernels need ft_block_rows > 0 dividing n_inputs, at most "
                               "about 800 rows per block, and ft_out a multiple of 64");
@@ -1456,7 +1519,7 @@ int b200_slot_read(b200_net* net, int slot, uint16_t* stm, uint16_t* nstm, int32
         for (size_t i = 0; i < count; i++) order[begin[bucket[i]]++] = (int32_t)i;
     }
     if (pair_order) {
-        const int nnz = net->d.nnz, R = net->nblocks > 1 ? net->d.ft_block_rows : net->d.n_inputs;
+        const int nnz = net->d.nnz, R = net->nblocks > 1 ? net->block_rows : net->d.n_inputs;
         std::vector<uint16_t> lists[2] = {std::vector<uint16_t>(count * nnz), std::vector<uint16_t>(count * nnz)};
         CK(cudaMemcpy(lists[0].data(), s.d_blob + s.off_stm, list, cudaMemcpyDeviceToHost));
         CK(cudaMemcpy(lists[1].data(), s.d_blob + s.off_nstm, list, cudaMemcpyDeviceToHost));
@@ -1857,7 +1920,7 @@ int b200_step_exchange(b200_net* net, int slot, float lr, float grad_factor) {
     const Tensor* l0w = net->find("l0w");
     const Tensor* l0f = d.factoriser_rows ? net->find("l0f") : nullptr;
     const int64_t block_floats = (int64_t)d.ft_block_rows * d.ft_out;
-    if (!net->bwd_tiled() || net->nblocks > b200::kMaxSignalBlocks)
+    if (!net->bwd_tiled() || !net->tiled_promised || net->nblocks > b200::kMaxSignalBlocks)
         return b200::fail(B200_ERR_UNSUPPORTED, "step_exchange: needs the tiled backward (ft_block_rows > 0) and at most %d row blocks",
                           b200::kMaxSignalBlocks);
     if (block_floats % (4 * net->xch_world)) return b200::fail(B200_ERR_UNSUPPORTED, "step_exchange: a row block does not split over %d ranks", net->xch_world);
@@ -2098,7 +2161,7 @@ static int step_chained(b200_net* net, Slot& s, int slot, float lr, float grad_f
         u.h_loss = net->h_loss + ring;
         u.h_status = net->h_status + ring;
         u.stamps = net->stamp(0);
-        const long long items = std::max(u.rest4, u.block4), blocks = std::min<long long>((items + 255) / 256, net->sm_count * 8);
+        const long long items = std::max(u.rest4, u.block4), blocks = std::min<long long>((items + 255) / 256, net->sm_count * 32);
         CK(b200::launch_step(true, b200::step_update_kernel, (unsigned)blocks, 256, 0, net->stream, u));
         LAUNCHED(net);
         net->weights_moved();
@@ -2151,6 +2214,12 @@ int b200_flat_buffer(b200_net* net, int kind, void** device_ptr, int64_t* n_floa
     return 0;
 }
 
+static int check_waits(b200_net* net) {
+    if (!*(volatile int*)net->h_gave_up) return 0;
+    *net->h_gave_up = 0;
+    return b200::fail(B200_ERR_CUDA, "a kernel gave up waiting for its own copies; the results of that pass are not valid");
+}
+
 int b200_loss_of(b200_net* net, int steps_back, float* loss_sum) {
     if (!net || !loss_sum) return b200::fail(B200_ERR_ARG, "loss: null argument");
     if (steps_back < 0 || steps_back >= b200_net::kLossRing - 1)
@@ -2160,6 +2229,7 @@ int b200_loss_of(b200_net* net, int steps_back, float* loss_sum) {
     const int ring = (int)((net->updates - 1 - steps_back) % b200_net::kLossRing);
     CK(cudaEventSynchronize(net->loss_ev[ring]));
     *loss_sum = net->h_loss[ring];
+    if (int rc = check_waits(net)) return rc;
     if (net->h_xstatus[4 * ring]) {
         const int* x = net->h_xstatus + 4 * ring;
         const int base = x[1], value = x[2], who = x[3];
@@ -2199,6 +2269,7 @@ int b200_forward(b200_net* net, int slot, float* out_host) {
     if (s.n > kDirectOutputs) CK(cudaMemcpyAsync(net->h_out, net->out, (size_t)s.n * sizeof(float), cudaMemcpyDeviceToHost, net->stream));
     CK(cudaStreamSynchronize(net->stream));
     memcpy(out_host, net->h_out, (size_t)s.n * sizeof(float));
+    if (int rc = check_waits(net)) return rc;
     return 0;
 }
 
@@ -2288,6 +2359,8 @@ int b200_net_get_activation(b200_net* net, int which, float* host, int64_t n) {
     }
     CK(cudaStreamSynchronize(net->stream));
     CK(cudaMemcpy(host, src, n * sizeof(float), cudaMemcpyDeviceToHost));
+    if (which == 0 && net->keep_root())
+        for (int64_t i = 0; i < n; i++) host[i] *= host[i];
     return 0;
 }
 
