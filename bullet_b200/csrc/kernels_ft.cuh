@@ -513,8 +513,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
 
 // Backward.  Positions are visited in chunks of at most CP pairs of one row block.
 //   ft_csr_kernel (one CTA per chunk, once per batch) turns the chunk's prepared lists around:
-//     for every table row of the block, the list of the chunk's pairs that hold it (a count
-//     pass, a scan and a fill pass in shared memory), every list starting on an 8-byte
+//     for every table row of the block, the list of the chunk's pairs that hold it (a count,
+//     a scan and a fill in shared memory), every list starting on an 8-byte
 //     boundary.  Lists are cut into pieces of at most kPiece entries and the pieces put in
 //     order of their lengths, longest first.  All column slabs share the result.
 //   ft_backward_tiled_kernel (same grid as the forward) then, per chunk, copies that list
@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
 //     with one 16-byte global reduction per lane.
 // Accumulation needs no atomics, and the table gradient sees one reduction per (row piece, chunk)
 // instead of one per (row, position).  The table gradient must be zero on entry.
-constexpr int kCsrThreads = 512;
+constexpr int kCsrThreads = 1024;
 
 // Two shapes of the backward: "wide" = one CTA of 1024 threads per SM, otherwise two CTAs of 512 threads on chunks of 256
 // pairs (half of it when nnz > 32), so that one CTA's global loads overlap the other's shared-memory work.
@@ -543,122 +543,103 @@ __host__ __device__ inline size_t ft_bwd_smem(int R, int nnz, int cp) {
            32 * kTileRowBytes;  // staged lines, row lists, their pieces, what a pair needs, bias-gradient sums per warp
 }
 __host__ __device__ inline size_t ft_csr_smem(int R, int nnz, int cp) {
-    return (size_t)ft_bwd_ent_cap(R, nnz, cp) * 2 + (size_t)(2 * (R + 2) + 32 + 2 * (kPiece + 2) + cp) * 4;
+    return (size_t)ft_bwd_ent_cap(R, nnz, cp) * 2 + (size_t)(2 * (R + 2)) * 4;
 }
 
-// grid = most chunks there can be, block = kCsrThreads.
+// grid = most chunks there can be, block = kCsrThreads.  Bound by latency: one load of the lists, whose entries and ranks stay
+// in registers from the count to the fill (a second pass over them, with a second atomic each, made it 15 us instead of
+// CSR_NOW for chunks of 443 pairs; while a step runs, a CTA of this kernel holds up whatever kernel of the step wants its SM).
 static __global__ void __launch_bounds__(kCsrThreads) ft_csr_kernel(FtArgs a, TileArgs t) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ int warp_tot[32], bin[kPiece + 1];  // bin: pieces by length, then their first places
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int NW = kCsrThreads / 32;
     const int4 chunk = t.chunks[blockIdx.x];
     if (chunk.z == 0) return;  // (the launch is sized from the batch size alone)
-    const int R = t.block_rows, L = t.list_len, c0 = chunk.y, cn = chunk.z;
+    const int R = t.block_rows, c0 = chunk.y, cn = chunk.z, Q = t.list_len / 8;  // 16-byte pieces per list
     uint16_t* ent = reinterpret_cast<uint16_t*>(smem_raw);
     int* start = reinterpret_cast<int*>(ent + t.ent_cap);  // [R + 1]
-    int* cursor = start + R + 2;                                         // [R]
-    int* warp_tot = cursor + R + 2;                                      // [32]
-    int* bin = warp_tot + 32;                                            // [kPiece + 2] pieces by length, then their first places
-    int* count_s = bin + 2 * (kPiece + 2);                               // [CP] prepared list lengths
-    const int zero_row = R;  // (no row: a lane without an entry)
-    for (int r = threadIdx.x; r < R; r += kCsrThreads) cursor[r] = 0;
-    if (threadIdx.x < kPiece + 2) bin[threadIdx.x] = 0;
-    for (int k = threadIdx.x; k < cn; k += kCsrThreads) count_s[k] = t.pairs[c0 + k].y;
-    __syncthreads();
-    // count how often each row occurs in the chunk: a warp per pair, a lane per list entry,
-    // four pairs in flight
-    const uint16_t* lists = t.lists + (size_t)c0 * L;
-    for (int pl0 = warp; pl0 < cn; pl0 += 4 * NW)
-        for (int k0 = 0; k0 < L; k0 += 32) {
-            int o[4];
+    int* count = start + R + 2;                             // [R]
+    constexpr int V = (kChunkMost * 8 + kCsrThreads - 1) / kCsrThreads;
+    uint4 list[V];
+    int pair[V], len[V];  // of each piece: its pair and how many of its eight entries count
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int pl = pl0 + k * NW;
-                o[k] = zero_row;
-                if (pl < cn && k0 + lane < count_s[pl]) o[k] = __ldg(lists + (size_t)pl * L + k0 + lane);
-            }
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-                if (o[k] != zero_row) atomicAdd(&cursor[o[k]], 1);
+    for (int v = 0; v < V; v++) {
+        const int e = threadIdx.x + v * kCsrThreads;
+        len[v] = 0;
+        if (e < cn * Q) {
+            pair[v] = e / Q;
+            const int q = e - pair[v] * Q;
+            list[v] = __ldg(reinterpret_cast<const uint4*>(t.lists + (size_t)(c0 + pair[v]) * t.list_len) + q);
+            len[v] = __ldg(&t.pairs[c0 + pair[v]].y) - 8 * q;
         }
+    }
+    for (int r = threadIdx.x; r < R; r += kCsrThreads) count[r] = 0;
+    if (threadIdx.x <= kPiece) bin[threadIdx.x] = 0;
     __syncthreads();
-    // exclusive scan of the row counts, each rounded up to a multiple of four entries (8 bytes)
-    {
-        int carry = 0;
-        for (int base = 0; base < R; base += kCsrThreads) {
-            const int r = base + threadIdx.x;
-            const int cnt = r < R ? cursor[r] : 0, v = (cnt + 3) & ~3;
-            if (cnt >= kPiece) atomicAdd(&bin[kPiece], cnt / kPiece);
-            if (cnt % kPiece) atomicAdd(&bin[cnt % kPiece], 1);
-            int incl = v;
+    // count how often each row occurs in the chunk; an entry's rank among its row's is what the counter held
+    uint32_t rank[V][4];
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int n = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += n;
-            }
-            if (lane == 31) warp_tot[warp] = incl;
-            __syncthreads();
-            int before = carry, all = 0;
-            for (int k = 0; k < NW; k++) {
-                if (k < warp) before += warp_tot[k];
-                all += warp_tot[k];
-            }
-            if (r < R) {
-                start[r] = before + incl - v;
-                cursor[r] = before + incl - v;
-            }
-            carry += all;
-            __syncthreads();
+    for (int v = 0; v < V; v++) {
+        const uint32_t w[4] = {list[v].x, list[v].y, list[v].z, list[v].w};
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+            rank[v][h] = 0;
+            if (2 * h < len[v]) rank[v][h] = (uint32_t)atomicAdd(&count[w[h] & 0xffffu], 1);
+            if (2 * h + 1 < len[v]) rank[v][h] |= (uint32_t)atomicAdd(&count[w[h] >> 16], 1) << 16;
         }
-        if (threadIdx.x == 0) start[R] = carry;
     }
     __syncthreads();
-    // fill: entry = index of the pair within the chunk, grouped by row
-    for (int pl0 = warp; pl0 < cn; pl0 += 4 * NW)
-        for (int k0 = 0; k0 < L; k0 += 32) {
-            int o[4];
+    // exclusive scan of the row counts, each rounded up to a multiple of four entries (8 bytes); R is less than the threads
+    static_assert(kCsrThreads >= 1023, "a thread per row");
+    const int r = threadIdx.x, mine = r < R ? count[r] : 0, room = (mine + 3) & ~3;
+    int incl = room;
 #pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const int pl = pl0 + k * NW;
-                o[k] = zero_row;
-                if (pl < cn && k0 + lane < count_s[pl]) o[k] = __ldg(lists + (size_t)pl * L + k0 + lane);
-            }
-#pragma unroll
-            for (int k = 0; k < 4; k++)
-                if (o[k] != zero_row) ent[atomicAdd(&cursor[o[k]], 1)] = (uint16_t)(pl0 + k * NW);
-        }
+    for (int o = 1; o < 32; o <<= 1) {
+        const int n = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += n;
+    }
+    if (lane == 31) warp_tot[warp] = incl;
+    if (mine >= kPiece) atomicAdd(&bin[kPiece], mine / kPiece);
+    if (mine % kPiece) atomicAdd(&bin[mine % kPiece], 1);
     __syncthreads();
-    // places of the pieces, longest first
-    if (warp == 0) {
+    const int before = __reduce_add_sync(0xffffffffu, lane < warp ? warp_tot[lane] : 0), total = __reduce_add_sync(0xffffffffu, warp_tot[lane]);
+    const int first = before + incl - room;
+    if (r < R) start[r] = first;
+    if (warp == 0) {  // places of the pieces, longest first
         int run = 0;
         for (int base = kPiece; base > 0; base -= 32) {
             const int own = bin[base - lane];
-            int incl = own;
+            int sum = own;
 #pragma unroll
             for (int o = 1; o < 32; o <<= 1) {
-                const int n = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += n;
+                const int n = __shfl_up_sync(0xffffffffu, sum, o);
+                if (lane >= o) sum += n;
             }
-            bin[base - lane] = run + incl - own;
-            run += __shfl_sync(0xffffffffu, incl, 31);
+            bin[base - lane] = run + sum - own;
+            run += __shfl_sync(0xffffffffu, sum, 31);
         }
         if (lane == 0) bin[0] = run;  // (no piece is empty: the place of length 0 holds their number)
     }
     __syncthreads();
-    // publish: the entries in 16-byte pieces, and the list pieces
-    const int total = start[R], pieces = bin[0];
+    // fill: entry = index of the pair within the chunk, grouped by row; and the list pieces
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+        const uint32_t w[4] = {list[v].x, list[v].y, list[v].z, list[v].w};
+#pragma unroll
+        for (int h = 0; h < 4; h++) {
+            if (2 * h < len[v]) ent[start[w[h] & 0xffffu] + (rank[v][h] & 0xffffu)] = (uint16_t)pair[v];
+            if (2 * h + 1 < len[v]) ent[start[w[h] >> 16] + (rank[v][h] >> 16)] = (uint16_t)pair[v];
+        }
+    }
+    int* out = t.csr_start + (size_t)blockIdx.x * t.start_cap;
+    if (threadIdx.x == 0) *reinterpret_cast<int4*>(out) = make_int4(total, bin[0], 0, 0);
+    for (int k = 0; k < mine; k += kPiece) {
+        const int n = min(kPiece, mine - k);
+        out[4 + atomicAdd(&bin[n], 1)] = ((first + k) >> 2) << 17 | n << 10 | r;
+    }
     __syncthreads();
     uint4* ent_out = reinterpret_cast<uint4*>(t.csr_ent + (size_t)blockIdx.x * t.ent_cap);
     for (int i = threadIdx.x; i < (total + 7) / 8; i += kCsrThreads) ent_out[i] = reinterpret_cast<const uint4*>(ent)[i];
-    int* out = t.csr_start + (size_t)blockIdx.x * t.start_cap;
-    if (threadIdx.x == 0) *reinterpret_cast<int4*>(out) = make_int4(total, pieces, 0, 0);
-    for (int r = threadIdx.x; r < R; r += kCsrThreads) {
-        const int first = start[r], cnt = cursor[r] - first;
-        for (int k = 0; k < cnt; k += kPiece) {
-            const int len = min(kPiece, cnt - k);
-            out[4 + atomicAdd(&bin[len], 1)] = ((first + k) >> 2) << 17 | len << 10 | r;
-        }
-    }
 }
 
 // The backward's work line: block b contributes, per column slab, its pairs plus a fixed amount per chunk

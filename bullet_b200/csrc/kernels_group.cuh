@@ -218,14 +218,16 @@ __device__ __forceinline__ int prepare_list_warp(const GroupArgs& g, uint32_t s0
 }
 
 constexpr int kPlaceThreads = 2 * kWindowPositions;
+constexpr int kCountedBlocks = 32;  // up to as many row blocks a window orders its pairs by counting, beyond by sorting
 
 // Pass 2.  grid = group_windows(n) CTAs of one thread per pair of the window.  `vec`: see group_vec.
-// Latency bound (one CTA per SM at most for ordinary batches): one sweep over the histograms, a bitonic sort in registers
-// and shared memory, one gather of the lists.
+// Latency bound (one CTA per SM at most for ordinary batches): one sweep over the histograms, a counting sort (a bitonic one
+// for many blocks: its 45 barriers took a third of the kernel's 13 us), one gather of the lists.
 static __global__ void __launch_bounds__(kPlaceThreads) group_place_kernel(GroupArgs g, int vec) {
     __shared__ int before[kGroupMaxBlocks + kGroupMaxBuckets], block_at[kGroupMaxBlocks + 1], bucket_at[kGroupMaxBuckets + 1];
     __shared__ int scan_s[kGroupMaxBlocks + 1], run_start[kGroupMaxBlocks];
     __shared__ unsigned key_s[kPlaceThreads];
+    __shared__ int counter_s[kCountedBlocks * 65];
     __shared__ int place_s[kPlaceThreads], warp_count[kWindowPositions / 32][kGroupMaxBuckets];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, tid = threadIdx.x;
     const int nb = g.nblocks, nbins = nb + g.n_out_buckets;
@@ -259,25 +261,62 @@ static __global__ void __launch_bounds__(kPlaceThreads) group_place_kernel(Group
             const unsigned info = (unsigned)g.info[base + tid];
             key = (info >> 8) << 17 | (info & 0x7fu) << 10 | (unsigned)tid;
         }
-        for (int k = 2; k <= kPlaceThreads; k <<= 1)
-            for (int j = k >> 1; j > 0; j >>= 1) {
-                unsigned other;
-                if (j >= 32) {
-                    __syncthreads();
-                    key_s[tid] = key;
-                    __syncthreads();
-                    other = key_s[tid ^ j];
-                } else {
-                    other = __shfl_xor_sync(0xffffffffu, key, j);
-                }
-                const bool keep_min = ((tid & j) == 0) == ((tid & k) == 0);
-                key = keep_min ? min(key, other) : max(key, other);
+        if (nb <= kCountedBlocks) {
+            // one counter per block and length; pairs of the same block and length come in any order
+            constexpr int kLengths = 65, B = (kCountedBlocks * kLengths + kPlaceThreads - 1) / kPlaceThreads;
+            const int bins = nb * kLengths;
+            for (int k = tid; k < bins; k += kPlaceThreads) counter_s[k] = 0;
+            __syncthreads();
+            const int bin = (int)(key >> 17) * kLengths + (int)(key >> 10 & 0x7fu);
+            int rank = 0;
+            if (tid < live) rank = atomicAdd(&counter_s[bin], 1);
+            __syncthreads();
+            int own[B], sum = 0;
+#pragma unroll
+            for (int k = 0; k < B; k++) {
+                own[k] = tid * B + k < bins ? counter_s[tid * B + k] : 0;
+                sum += own[k];
             }
-        __syncthreads();
-        key_s[tid] = key;
-        __syncthreads();
-        if (tid < live && (tid == 0 || (key_s[tid - 1] >> 17) != (key >> 17))) run_start[key >> 17] = tid;
-        __syncthreads();
+            int incl = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += up;
+            }
+            if (lane == 31) place_s[warp] = incl;
+            __syncthreads();
+            int at = incl - sum + __reduce_add_sync(0xffffffffu, lane < warp ? place_s[lane] : 0);
+#pragma unroll
+            for (int k = 0; k < B; k++) {
+                if (tid * B + k < bins) counter_s[tid * B + k] = at;
+                at += own[k];
+            }
+            __syncthreads();
+            if (tid < nb) run_start[tid] = counter_s[tid * kLengths];
+            if (tid < live) key_s[counter_s[bin] + rank] = key;
+            __syncthreads();
+            key = key_s[tid];
+        } else {
+            for (int k = 2; k <= kPlaceThreads; k <<= 1)
+                for (int j = k >> 1; j > 0; j >>= 1) {
+                    unsigned other;
+                    if (j >= 32) {
+                        __syncthreads();
+                        key_s[tid] = key;
+                        __syncthreads();
+                        other = key_s[tid ^ j];
+                    } else {
+                        other = __shfl_xor_sync(0xffffffffu, key, j);
+                    }
+                    const bool keep_min = ((tid & j) == 0) == ((tid & k) == 0);
+                    key = keep_min ? min(key, other) : max(key, other);
+                }
+            __syncthreads();
+            key_s[tid] = key;
+            __syncthreads();
+            if (tid < live && (tid == 0 || (key_s[tid - 1] >> 17) != (key >> 17))) run_start[key >> 17] = tid;
+            __syncthreads();
+        }
         if (tid < live) place_s[tid] = block_at[key >> 17] + before[key >> 17] + tid - run_start[key >> 17];
         __syncthreads();
         if (vec) {

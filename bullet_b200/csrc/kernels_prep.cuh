@@ -35,8 +35,8 @@ struct PrepArgs {
 // One thread per position for what a position has one of (bucket, target), then one warp per position for the lists: a lane
 // owns two squares, and the place of a piece in the list is the number of occupied squares below it, so nothing loops over
 // pieces.  (A thread per position that walked its bitboards took 14 us for 16384 positions and stored two bytes at a time.)
-// The records may lie in pinned host memory: they are read once, coalesced.  grid = group_ctas(n), block = 256.
-constexpr int kPrepThreads = 256;
+// The records may lie in pinned host memory: they are read once, coalesced.  grid = group_ctas(n), block = kPrepThreads.
+constexpr int kPrepThreads = 512;
 static __global__ void __launch_bounds__(kPrepThreads) prep_featurise_kernel(PrepArgs p, GroupArgs g) {
     __shared__ uint4 record_s[kGroupPositions][2];
     __shared__ int hist[kGroupMaxBlocks + kGroupMaxBuckets];
@@ -47,7 +47,7 @@ static __global__ void __launch_bounds__(kPrepThreads) prep_featurise_kernel(Pre
     const int first = (int)blockIdx.x * kGroupPositions, live = min(kGroupPositions, g.n - first);
     for (int k = threadIdx.x; k < nbins; k += kPrepThreads) hist[k] = 0;
     if (blockIdx.x == 0 && threadIdx.x == 0 && g.clear_status) *g.status = 0;
-    static_assert(kPrepThreads == 2 * kGroupPositions, "one 16-byte half of a record per thread");
+    static_assert(kPrepThreads >= 2 * kGroupPositions, "one 16-byte half of a record per thread");
     if ((int)threadIdx.x < 2 * live) record_s[threadIdx.x >> 1][threadIdx.x & 1] = p.records[2 * first + threadIdx.x];
     __syncthreads();
     if ((int)threadIdx.x < live) {
