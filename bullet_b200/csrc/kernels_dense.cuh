@@ -33,8 +33,7 @@ struct DenseArgs {
     const float* W1g;  // first-layer weights regrouped as [bucket][column][row] (fewer than four rows)
     const float4* W1f; // ... or as the fragment tables of kernels_dense_mma.cuh
     const float4* W1d;
-    float* partial;    // with few tiles: [tile][slice][32][M1] sums of the slices, and how many have arrived per tile (zero between launches)
-    int* arrived;
+    float* partial;    // [part][tile][32][M1] sums of slices of the first layer's columns
     float* a1;         // [n][M1] activated layer-1 output (kept for the weight gradients)
     float* a2;         // [n][M2]
     float* dz[3];      // gradient at each layer's selected pre-activation: [n][M_i]
@@ -43,6 +42,7 @@ struct DenseArgs {
     float* loss;       // scalar, accumulated
     int want_grad;
     unsigned long long* stamp;  // as in FtArgs
+    int* gave_up;               // pinned word, raised if a wait for copies runs out
     // the register-tiled forward also forms the weight and bias gradients of the layers after the
     // first (it holds everything they need in shared memory): gradient tensors of layers 2 and 3
     int fuse_small;

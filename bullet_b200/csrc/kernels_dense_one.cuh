@@ -132,7 +132,10 @@ __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __grid_con
             }
 #pragma unroll
         for (int i = 0; i < 4; i++) acc[i] = make_float4(0, 0, 0, 0);
-        if (tid < P && g_bias != 0.f) atomicAdd(a.gB + cur, g_bias);
+        if (warp == 0) {  // (one addition per CTA: the sum of many rounds once for each)
+            const float sum = warp_sum(g_bias);
+            if (lane == 0 && sum != 0.f) atomicAdd(a.gB + cur, sum);
+        }
         g_bias = 0.f;
     };
     __syncthreads();

@@ -114,8 +114,7 @@ struct b200_net {
     int64_t n_flat = 0;
     float *P = nullptr, *G = nullptr, *M = nullptr, *V = nullptr, *table = nullptr;
     float *x = nullptr, *u = nullptr, *dx = nullptr, *a1 = nullptr, *a2 = nullptr, *out = nullptr, *w1g = nullptr;
-    float* dense_partial = nullptr;  // the dense forward's sums of split tiles
-    int* dense_arrived = nullptr;
+    float* dense_partial = nullptr;  // the first dense layer's sums of slices of its columns
     float4 *w1f = nullptr, *w1d = nullptr;  // the first dense layer's fragment tables (dense_mma)
     float* dz[3] = {nullptr, nullptr, nullptr};
     int wgrad_per_sm = 0;          // resident CTAs per SM of the first layer's weight-gradient kernel (looked up once)
@@ -439,24 +438,36 @@ int launch_ft_backward(b200_net* net, const b200::FtArgs& a, const b200::TileArg
         default: return b200::fail(B200_ERR_UNSUPPORTED, "rows per bucket %d", m); \
     }
 
-// A tile is a chain of loads for its CTA (20 us at 2048 columns): while there are tiles for a quarter of the SMs at most, up to
-// eight CTAs share one.
-constexpr int kMostSlices = 8;
-int dense_slices(const b200_net* net, int ntiles) {
-    const int groups = (net->D1() + b200::kMmaCols - 1) / b200::kMmaCols;
-    return std::max(1, std::min({kMostSlices, net->sm_count / (2 * ntiles), groups / 8}));
+// A slice of a tile is a chain of sixteen rounds of loads for its warp: while there are fewer of them than warps, up to eight
+// warps share one (but none is left without a group of columns).
+int dense_slices(const b200_net* net) { return (net->D1() + b200::kSliceCols - 1) / b200::kSliceCols; }
+int dense_split(const b200_net* net, int ntiles) {
+    const int slices = dense_slices(net), all = b200::kSliceCols / b200::kMmaCols;
+    const int in_last = (net->D1() + b200::kMmaCols - 1) / b200::kMmaCols - (slices - 1) * all;
+    int split = 8;
+    while (split > 1 && ((long long)slices * split * ntiles > 8LL * net->sm_count || (split - 1) * (all / split) >= in_last)) split /= 2;
+    return split;
 }
 
 template <int MM>
 void launch_dense_forward(b200_net* net, const b200::DenseArgs& da, int ntiles) {
-    if constexpr (MM >= 4)
-        b200::launch_step(net->chained, b200::dense_forward_mma_kernel<MM>, dim3(ntiles, dense_slices(net, ntiles)), 256, b200::dense_mma_smem<MM>(), net->stream, da);
-    else
+    if constexpr (MM >= 4) {
+        const int slices = dense_slices(net), split = dense_split(net, ntiles);
+        const dim3 grid(slices, std::max(1, std::min((ntiles * split + 7) / 8, b200::dense_mma_ctas(MM) * net->sm_count / slices)));
+        b200::launch_step(net->chained, b200::dense_first_mma_kernel<MM>, grid, 256, b200::dense_mma_smem<MM>(), net->stream, da, split);
+        net->launches++;
+        b200::launch_step(net->chained, b200::dense_small_mma_kernel<MM>, std::min(ntiles, b200::kSmallCtas * net->sm_count), b200::kSmallThreads, 0, net->stream, da,
+                          slices * split);
+    } else
         b200::launch_step(net->chained, b200::dense_forward_kernel<MM>, ntiles, 256, b200::dense_fwd_smem<MM>(), net->stream, da);
 }
 template <int MM>
-void launch_wgrad_mma(b200_net* net, const b200::DenseArgs& a, float* gW, float* gB, dim3 grid, int threads, int per_run) {
-    if constexpr (MM >= 4) b200::launch_step(net->chained, b200::dense_wgrad_mma_kernel<MM>, grid, threads, 0, net->stream, a, gW, gB, per_run);
+void launch_wgrad_mma(b200_net* net, const b200::DenseArgs& a, float* gW, float* gB) {
+    if constexpr (MM >= 4) {
+        const int cols = 8 * b200::kWgradCols, gx = (a.K1 + cols - 1) / cols;
+        const dim3 grid(gx, std::max(1, std::min(a.ntiles, b200::dense_mma_ctas(MM) * net->sm_count / gx)));
+        b200::launch_step(net->chained, b200::dense_wgrad_mma_kernel<MM>, grid, b200::kRingThreads, b200::wgrad_smem<MM>(), net->stream, a, gW, gB);
+    }
 }
 template <int MM>
 void launch_dense_dx(b200_net* net, const b200::DenseArgs& da, int ntiles) {
@@ -469,8 +480,10 @@ void launch_dense_dx(b200_net* net, const b200::DenseArgs& da, int ntiles) {
 template <int MM>
 cudaError_t set_dense_forward_smem() {
     if constexpr (MM >= 4)
-        return b200::allow_smem(b200::dense_forward_mma_kernel<MM>);
-    else
+    {
+        const cudaError_t e = b200::allow_smem(b200::dense_first_mma_kernel<MM>);
+        return e ? e : b200::allow_smem(b200::dense_wgrad_mma_kernel<MM>);
+    } else
         return b200::allow_smem(b200::dense_forward_kernel<MM>);
 }
 
@@ -576,7 +589,7 @@ b200::DenseArgs dense_args(b200_net* net, const Slot& s, bool want_grad) {
     a.W1f = net->w1f;
     a.W1d = net->w1d;
     a.partial = net->dense_partial;
-    a.arrived = net->dense_arrived;
+    a.gave_up = net->h_gave_up;
     a.a1 = net->a1;
     a.a2 = net->a2;
     a.out = net->out;
@@ -785,10 +798,7 @@ int launch_wgrad(b200_net* net, const Slot& s) {
     float *gW = net->G + net->find("l1w")->off, *gB = net->G + net->find("l1b")->off;
     if (net->dense_mma()) {
         const b200::DenseArgs a = dense_args(net, s, true);
-        const int warps = std::min(8, (a.K1 + b200::kWgradCols - 1) / b200::kWgradCols), gx = (a.K1 + warps * b200::kWgradCols - 1) / (warps * b200::kWgradCols);
-        const int runs = std::max(1, std::min(s.n_dtiles, 2 * net->sm_count * 8 / warps / gx)), per_run = (s.n_dtiles + runs - 1) / runs;
-        const dim3 grid(gx, (s.n_dtiles + per_run - 1) / per_run);
-        DISPATCH_M(d.dense_out[0], launch_wgrad_mma<MM>(net, a, gW, gB, grid, 32 * warps, per_run));
+        DISPATCH_M(d.dense_out[0], launch_wgrad_mma<MM>(net, a, gW, gB));
         LAUNCHED(net);
         return 0;
     }
@@ -866,7 +876,7 @@ bool load_kernel(K* kernel) {
 template <int MM>
 bool load_dense_kernels() {
     if constexpr (MM >= 4)
-        return load_kernel(b200::dense_forward_mma_kernel<MM>) && load_kernel(b200::dense_dx_mma_kernel<MM>) && load_kernel(b200::dense_wgrad_mma_kernel<MM>);
+        return load_kernel(b200::dense_first_mma_kernel<MM>) && load_kernel(b200::dense_small_mma_kernel<MM>) && load_kernel(b200::dense_dx_mma_kernel<MM>) && load_kernel(b200::dense_wgrad_mma_kernel<MM>);
     else
         return load_kernel(b200::dense_forward_kernel<MM>) && load_kernel(b200::dense_dx_kernel<MM>) && load_kernel(b200::dense_wgrad_kernel<MM>);
 }
@@ -1015,8 +1025,9 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
         const size_t table = b200::mma_table_floats(net->D1(), d.n_out_buckets, d.dense_out[0]) / 4;
         plan.add(&net->w1f, table);
         plan.add(&net->w1d, table);
-        plan.add(&net->dense_partial, (size_t)net->sm_count * kMostSlices * b200::kDenseTile * d.dense_out[0]);
-        plan.add(&net->dense_arrived, (size_t)net->sm_count);
+        // one part per slice, or more of them for few tiles (dense_split)
+        const size_t tiles = (size_t)d.max_batch / b200::kDenseTile + std::min(d.n_out_buckets, d.max_batch) + 1;
+        plan.add(&net->dense_partial, std::max(dense_slices(net) * tiles, (size_t)8 * net->sm_count) * b200::kDenseTile * d.dense_out[0]);
     } else {
         plan.add(&net->w1g, (size_t)2 * d.n_out_buckets * d.dense_out[0] * net->D1());
         if (net->dense_one()) plan.add(&net->kept_bucket, B);
@@ -1046,7 +1057,6 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     }
     for (auto& s : net->slots) plan.add(&s.d_blob, s.bytes);
     rc = rc ? rc : plan.allocate(net);
-    if (!rc && net->dense_arrived) cudaMemsetAsync(net->dense_arrived, 0, (size_t)net->sm_count * sizeof(int), net->stream);
     if (!rc) cudaMemsetAsync(net->done_count, 0, (size_t)net->nblocks * sizeof(int), net->stream);
     if (rc) return bail(rc);
     if (!d.factoriser_rows) net->table = net->P + net->find("l0w")->off;
