@@ -34,6 +34,7 @@ struct DenseArgs {
     const float4* W1f; // ... or as the fragment tables of kernels_dense_mma.cuh
     const float4* W1d;
     float* partial;    // [part][tile][32][M1] sums of slices of the first layer's columns
+    float* dz_frag;    // dz[0] as the tensor pipe's operand of the weight gradient (dense_small_mma_kernel)
     float* a1;         // [n][M1] activated layer-1 output (kept for the weight gradients)
     float* a2;         // [n][M2]
     float* dz[3];      // gradient at each layer's selected pre-activation: [n][M_i]

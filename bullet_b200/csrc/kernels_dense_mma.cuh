@@ -292,8 +292,13 @@ __global__ void __launch_bounds__(256, dense_mma_ctas(M1)) dense_first_mma_kerne
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
+// floats before step `i` (eight places of a tile) of the weight gradient's operand: [step][16-row tile][hi, lo][lane] float4
+template <int M1>
+__host__ __device__ constexpr size_t wgrad_table_floats(size_t i) { return i * (M1 > 16 ? M1 / 16 : 1) * 256; }
+
 // The rest of the forward: sum of the first layer's parts, small layers, loss, the way back to the first layer's
-// pre-activation gradient, weight gradients of the small layers (kept in registers until the bucket changes).  A CTA takes a
+// pre-activation gradient (also as the operand of its weight gradient), weight gradients of the small layers and the first
+// layer's bias gradient (kept in registers until the bucket changes).  A CTA takes a
 // run of tiles, a warp eight of a tile's 32 positions: four lanes per position, each with a quarter of the second layer's 32
 // rows (zero past the last); for the weight gradients a lane is a row.  Bound by latency: SMALL_LARGE us at 131072 positions
 // (64 MB of parts), SMALL_MID at 16384.
@@ -305,13 +310,15 @@ __global__ void __launch_bounds__(kSmallThreads, M1 > 16 ? 2 : 4) dense_small_mm
     __shared__ __align__(16) float s_w2[32 * M1 + 16];     // [row][column], four floats further every eight rows: a quarter each, no two in one bank
     __shared__ float s_b1[M1], s_b2[32], s_w3[32], s_bias3;
     __shared__ __align__(16) float s_a1[4][8][kRow];
-    __shared__ float s_dz2[4][8][33], s_a2[4][8][33], s_dout[4][8], s_own[4][M1 + 2][32], s_own_bias[4];
+    __shared__ float s_dz2[4][8][33], s_a2[4][8][33], s_dout[4][8], s_own[4][M1 + 2][32], s_own1[4][M1], s_own_bias[4];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, p = lane >> 2, quarter = lane & 3;
     const int M2 = a.M[1], OM2 = a.O * M2;
     const int first = (int)((long long)a.ntiles * blockIdx.x / gridDim.x), last = (int)((long long)a.ntiles * (blockIdx.x + 1) / gridDim.x);
-    float own[M1 + 1], own3 = 0.f, own3_bias = 0.f, my_loss = 0.f;  // this lane's row of the second layer: its columns, its bias; the third layer
+    float own1[kPer], own[M1 + 1], own3 = 0.f, own3_bias = 0.f, my_loss = 0.f;  // this lane's row of the second layer: its columns, its bias; the third layer
 #pragma unroll
     for (int c = 0; c <= M1; c++) own[c] = 0.f;
+#pragma unroll
+    for (int i = 0; i < kPer; i++) own1[i] = 0.f;
     int cur = -1;
     auto flush = [&]() {
         if (cur < 0 || !a.want_grad) return;  // (uniform) the four warps' sums, then one addition per CTA
@@ -320,7 +327,15 @@ __global__ void __launch_bounds__(kSmallThreads, M1 > 16 ? 2 : 4) dense_small_mm
         s_own[warp][M1 + 1][lane] = own3;
         own3_bias = warp_sum(own3_bias);
         if (lane == 0) s_own_bias[warp] = own3_bias;
+#pragma unroll
+        for (int i = 0; i < kPer; i++) {
+#pragma unroll
+            for (int d = 4; d < 32; d <<= 1) own1[i] += __shfl_xor_sync(0xffffffffu, own1[i], d);
+            if (p == 0) s_own1[warp][kPer * quarter + i] = own1[i];
+            own1[i] = 0.f;
+        }
         __syncthreads();
+        if ((int)threadIdx.x < M1) atomicAdd(a.gB[0] + cur * M1 + threadIdx.x, (s_own1[0][threadIdx.x] + s_own1[1][threadIdx.x]) + (s_own1[2][threadIdx.x] + s_own1[3][threadIdx.x]));
         for (int c = warp; c < M1 + 2; c += 4) {
             const float sum = (s_own[0][c][lane] + s_own[1][c][lane]) + (s_own[2][c][lane] + s_own[3][c][lane]);
             if (lane < M2 && (c <= M1 || a.n_dense == 3) && sum != 0.f)
@@ -461,12 +476,18 @@ __global__ void __launch_bounds__(kSmallThreads, M1 > 16 ? 2 : 4) dense_small_mm
             }
             mine[0] = quarter == 0 ? dz1[0] : quarter == 1 ? dz1[1] : quarter == 2 ? dz1[2] : dz1[3];
         }
-        if (on)
 #pragma unroll
-            for (int i = 0; i < kPer; i++) {
-                const float y = s_a1[warp][p][kPer * quarter + i];
-                a.dz[0][(size_t)pos * M1 + kPer * quarter + i] = mine[i] * act_bwd(a.act[0], y);
-            }
+        for (int i = 0; i < kPer; i++) {
+            const int r = kPer * quarter + i;
+            const float d = on ? mine[i] * act_bwd(a.act[0], s_a1[warp][p][r]) : 0.f;
+            if (on) a.dz[0][(size_t)pos * M1 + r] = d;
+            own1[i] += d;
+            // A of the weight gradient, step `warp` of the tile: lane 4 (r % 8) + p % 4, element (r / 8 % 2) + 2 (p / 4)
+            uint32_t hi, lo;
+            tf32_split(d, hi, lo);
+            float* at = a.dz_frag + wgrad_table_floats<M1>((size_t)tile * 4 + warp) + (r >> 4) * 256 + (4 * (r & 7) + (p & 3)) * 4 + (r >> 3 & 1) + 2 * (p >> 2);
+            at[0] = __uint_as_float(hi), at[128] = __uint_as_float(lo);
+        }
         __syncwarp();
 #pragma unroll 4
         for (int q = 0; q < 8; q++) {  // layer 2: X = a1, dY = dz2; layer 3: X = a2, dY = dout (one row)
@@ -562,62 +583,62 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_dx_mma_kernel(De
     }
 }
 
-// Weight and bias gradient of the first layer: gW[c][k][r] += sum_b [k_b == k] dz1[b][r] * x[b][c].  Positions contract, eight
+// Weight gradient of the first layer: gW[c][k][r] += sum_b [k_b == k] dz1[b][r] * x[b][c].  Positions contract, eight
 // a step; r is the M of the product and columns its N: a lane takes four neighbouring columns of two positions, and value j
 // of each belongs to column tile j.  A warp owns 64 columns (two groups of 32), the eight of a CTA 512; the CTA walks a
-// run of dense tiles, of which a ninth warp copies eight rows of x and of dz1 at a time into a ring of stages, and adds its
-// sums to the gradient when the output bucket changes.  The first CTA of a run sums the bias gradient.
-// (With x loaded into registers and dz1 split through shared memory a tile at a time, loads waited at two barriers a tile.)
-// 0.365 -> DWG_NOW ms at 131072 positions (0.165 for reading x at the copy rate).
+// run of dense tiles, of which a ninth warp copies eight rows of x and their dz1 (fragments that the small layers' kernel has
+// written in the order of the tiles) at a time into a ring of stages, and adds its sums to the gradient when the output bucket
+// changes.  (x loaded into registers and dz1 split through shared memory a tile at a time, with two barriers: 0.365 ms at
+// 131072 positions, K1 = 2048, M1 = 16; lanes copying their own pieces by cp.async, as the forward does: 0.370; this: DWG_NOW,
+// against 0.165 for reading x at the copy rate.  A bulk copy costs the warp that issues it 70 to 100 clocks, so it should be long.)
 // grid = (ceil(K1 / 512), runs), block = 288, dynamic shared memory = wgrad_smem<M1>().
 constexpr int kRingThreads = 288;
 constexpr int kWgradCols = 64, kWgradStages = 5, kWgradPitch = 8 * kWgradCols + 8;
-__host__ __device__ constexpr int wgrad_dz_pitch(int M1) { return M1 >= 16 ? M1 + 8 : M1; }
 template <int M1>
-__host__ __device__ constexpr int wgrad_stage_floats() { return 8 * (kWgradPitch + wgrad_dz_pitch(M1)); }
+__host__ __device__ constexpr int wgrad_stage_floats() { return 8 * kWgradPitch + (int)wgrad_table_floats<M1>(1); }
 template <int M1>
 __host__ __device__ constexpr size_t wgrad_smem() { return (size_t)kWgradStages * wgrad_stage_floats<M1>() * sizeof(float); }
 
 template <int M1>
-__global__ void __launch_bounds__(kRingThreads, dense_mma_ctas(M1)) dense_wgrad_mma_kernel(const __grid_constant__ DenseArgs a, float* gW, float* gB) {
-    constexpr int MT = M1 > 16 ? M1 / 16 : 1, kDzPitch = wgrad_dz_pitch(M1);
+__global__ void __launch_bounds__(kRingThreads, dense_mma_ctas(M1)) dense_wgrad_mma_kernel(const __grid_constant__ DenseArgs a, float* gW) {
+    constexpr int MT = M1 > 16 ? M1 / 16 : 1, kTable = (int)wgrad_table_floats<M1>(1);
     extern __shared__ __align__(16) float wgrad_smem_raw[];
     __shared__ Ring<kWgradStages> ring;
     __shared__ int s_rows[kWgradStages], s_bucket[kWgradStages];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
     if (threadIdx.x == 0) ring.init(8);
     __syncthreads();
-    step_begin(nullptr);
     const int first = (int)((long long)a.ntiles * blockIdx.y / gridDim.y), last = (int)((long long)a.ntiles * (blockIdx.y + 1) / gridDim.y);
     const int cta_col = blockIdx.x * 8 * kWgradCols;
     RingPlace<kWgradStages> at;
     if (warp == 8) {
         TileLookup lookup(a, lane, first, last);
+        step_begin(nullptr);  // everything so far was there before the kernel before this one began
         const uint32_t bytes = (uint32_t)min(8 * kWgradCols, a.K1 - cta_col) * 4;
         for (int tile = first;; tile++) {
             const TileAhead now = lookup.next(tile);
             for (int p = 0; p < max(1, now.t.y); p += 8) {
                 const int rows = max(0, min(8, now.t.y - p)), pos = __shfl_sync(0xffffffffu, now.pos, (p + lane) & 31);
-                const int dz_pos = __shfl_sync(0xffffffffu, pos, lane & 7);
                 if (!mbar_wait(&ring.empty[at.slot], at.phase ^ 1)) return;
                 __syncwarp();
                 float* stage = wgrad_smem_raw + (size_t)at.slot * wgrad_stage_floats<M1>();
                 if (lane == 0) {
                     s_rows[at.slot] = rows;
                     s_bucket[at.slot] = now.bucket;
-                    mbar_expect_tx(&ring.full[at.slot], rows * (bytes + M1 * 4));
+                    mbar_expect_tx(&ring.full[at.slot], rows ? rows * bytes + kTable * 4 : 0);
                 }
                 __syncwarp();
                 if (lane < rows) bulk_load(stage + lane * kWgradPitch, a.x + (size_t)pos * a.K1 + cta_col, bytes, &ring.full[at.slot]);
-                if (lane >= 8 && lane < 8 + rows)
-                    bulk_load(stage + 8 * kWgradPitch + (lane - 8) * kDzPitch, a.dz[0] + (size_t)dz_pos * M1, M1 * 4, &ring.full[at.slot]);
+                if (lane == 8 && rows)
+                    bulk_load(stage + 8 * kWgradPitch, a.dz_frag + wgrad_table_floats<M1>((size_t)tile * 4 + (p >> 3)), kTable * 4, &ring.full[at.slot]);
                 at.advance();
             }
             if (now.t.y <= 0) return;  // (the readers stop at a stage without rows)
         }
     }
+    step_begin(nullptr);
     const int c0 = cta_col + warp * kWgradCols, OM = a.O * M1;
-    float acc[MT][8][4], bias_sum = 0.f;
+    float acc[MT][8][4];
     auto clear = [&]() {
 #pragma unroll
         for (int m = 0; m < MT; m++)
@@ -625,7 +646,6 @@ __global__ void __launch_bounds__(kRingThreads, dense_mma_ctas(M1)) dense_wgrad_
             for (int j = 0; j < 8; j++)
 #pragma unroll
                 for (int e = 0; e < 4; e++) acc[m][j][e] = 0.f;
-        bias_sum = 0.f;
     };
     clear();
     int cur = -1;
@@ -641,7 +661,6 @@ __global__ void __launch_bounds__(kRingThreads, dense_mma_ctas(M1)) dense_wgrad_
                     const int c = c0 + 32 * (j >> 2) + 4 * (2 * t4 + (e & 1)) + (j & 3), r = 16 * m + g + 8 * (e >> 1);
                     if (c < a.K1 && r < M1 && acc[m][j][e] != 0.f) atomicAdd(gW + (size_t)c * OM + cur * M1 + r, acc[m][j][e]);
                 }
-        if (bias_sum != 0.f) atomicAdd(gB + cur * M1 + lane, bias_sum);
         clear();
     };
     for (;; at.advance()) {
@@ -656,19 +675,20 @@ __global__ void __launch_bounds__(kRingThreads, dense_mma_ctas(M1)) dense_wgrad_
             cur = k;
         }
         const float* stage = wgrad_smem_raw + (size_t)at.slot * wgrad_stage_floats<M1>();
-        const float* dz = stage + 8 * kWgradPitch;
-        // rows past the last hold what the stage held before, or nothing: both factors are taken as zero there
+        const float4* table = reinterpret_cast<const float4*>(stage + 8 * kWgradPitch) + lane;
+        // rows past the last hold what the stage held before, or nothing (their factor in the operand is zero)
         const bool on0 = t4 < rows, on1 = t4 + 4 < rows;
         uint32_t ahi[MT][4], alo[MT][4];
 #pragma unroll
-        for (int m = 0; m < MT; m++)
+        for (int m = 0; m < MT; m++) {
+            const float4 hi = table[64 * m], lo = table[64 * m + 32];
+            const float vh[4] = {hi.x, hi.y, hi.z, hi.w}, vl[4] = {lo.x, lo.y, lo.z, lo.w};
 #pragma unroll
             for (int e = 0; e < 4; e++) {
-                const int r = 16 * m + g + 8 * (e & 1);
-                tf32_split(r < M1 && (e >> 1 ? on1 : on0) ? dz[(t4 + 4 * (e >> 1)) * kDzPitch + r] : 0.f, ahi[m][e], alo[m][e]);
+                const bool on = 16 * m + 8 * (e & 1) + g < M1;  // (the table has no rows past M1)
+                ahi[m][e] = on ? __float_as_uint(vh[e]) : 0u, alo[m][e] = on ? __float_as_uint(vl[e]) : 0u;
             }
-        if (blockIdx.x == 0 && warp == 0 && lane < M1)
-            for (int p = 0; p < rows; p++) bias_sum += dz[p * kDzPitch + lane];
+        }
 #pragma unroll
         for (int h = 0; h < 2; h++) {  // the warp's two groups of 32 columns
             const int c = warp * kWgradCols + 32 * h + 4 * g;

@@ -114,6 +114,7 @@ struct b200_net {
     int64_t n_flat = 0;
     float *P = nullptr, *G = nullptr, *M = nullptr, *V = nullptr, *table = nullptr;
     float *x = nullptr, *u = nullptr, *dx = nullptr, *a1 = nullptr, *a2 = nullptr, *out = nullptr, *w1g = nullptr;
+    float* dz_frag = nullptr;        // the gradient at the first dense layer's pre-activation as an operand of its weight gradient
     float* dense_partial = nullptr;  // the first dense layer's sums of slices of its columns
     float4 *w1f = nullptr, *w1d = nullptr;  // the first dense layer's fragment tables (dense_mma)
     float* dz[3] = {nullptr, nullptr, nullptr};
@@ -462,11 +463,11 @@ void launch_dense_forward(b200_net* net, const b200::DenseArgs& da, int ntiles) 
         b200::launch_step(net->chained, b200::dense_forward_kernel<MM>, ntiles, 256, b200::dense_fwd_smem<MM>(), net->stream, da);
 }
 template <int MM>
-void launch_wgrad_mma(b200_net* net, const b200::DenseArgs& a, float* gW, float* gB) {
+void launch_wgrad_mma(b200_net* net, const b200::DenseArgs& a, float* gW) {
     if constexpr (MM >= 4) {
         const int cols = 8 * b200::kWgradCols, gx = (a.K1 + cols - 1) / cols;
         const dim3 grid(gx, std::max(1, std::min(a.ntiles, b200::dense_mma_ctas(MM) * net->sm_count / gx)));
-        b200::launch_step(net->chained, b200::dense_wgrad_mma_kernel<MM>, grid, b200::kRingThreads, b200::wgrad_smem<MM>(), net->stream, a, gW, gB);
+        b200::launch_step(net->chained, b200::dense_wgrad_mma_kernel<MM>, grid, b200::kRingThreads, b200::wgrad_smem<MM>(), net->stream, a, gW);
     }
 }
 template <int MM>
@@ -589,6 +590,7 @@ b200::DenseArgs dense_args(b200_net* net, const Slot& s, bool want_grad) {
     a.W1f = net->w1f;
     a.W1d = net->w1d;
     a.partial = net->dense_partial;
+    a.dz_frag = net->dz_frag;
     a.gave_up = net->h_gave_up;
     a.a1 = net->a1;
     a.a2 = net->a2;
@@ -597,7 +599,7 @@ b200::DenseArgs dense_args(b200_net* net, const Slot& s, bool want_grad) {
     a.loss = net->G;
     a.want_grad = want_grad ? 1 : 0;
     a.fuse_small = want_grad && net->fused_small_grads() ? 1 : 0;
-    for (int l = 1; l < d.n_dense; l++) {
+    for (int l = 0; l < d.n_dense; l++) {
         char name[16];
         snprintf(name, sizeof name, "l%dw", l + 1);
         a.gW[l] = net->G + net->find(name)->off;
@@ -798,7 +800,7 @@ int launch_wgrad(b200_net* net, const Slot& s) {
     float *gW = net->G + net->find("l1w")->off, *gB = net->G + net->find("l1b")->off;
     if (net->dense_mma()) {
         const b200::DenseArgs a = dense_args(net, s, true);
-        DISPATCH_M(d.dense_out[0], launch_wgrad_mma<MM>(net, a, gW, gB));
+        DISPATCH_M(d.dense_out[0], launch_wgrad_mma<MM>(net, a, gW));
         LAUNCHED(net);
         return 0;
     }
@@ -1027,6 +1029,7 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
         plan.add(&net->w1d, table);
         // one part per slice, or more of them for few tiles (dense_split)
         const size_t tiles = (size_t)d.max_batch / b200::kDenseTile + std::min(d.n_out_buckets, d.max_batch) + 1;
+        plan.add(&net->dz_frag, tiles * 4 * (d.dense_out[0] > 16 ? d.dense_out[0] / 16 : 1) * 256);
         plan.add(&net->dense_partial, std::max(dense_slices(net) * tiles, (size_t)8 * net->sm_count) * b200::kDenseTile * d.dense_out[0]);
     } else {
         plan.add(&net->w1g, (size_t)2 * d.n_out_buckets * d.dense_out[0] * net->D1());
