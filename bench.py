@@ -453,8 +453,7 @@ def run_ours(args, rank, world, local_rank):
                          f"{n_local * (desc.dense_in0 * 2 + 2 * desc.ft_out) * 4 / 1e6:.0f} MB",
                    "active_features_per_position": rows / n_local},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": int(h2d_per_step) * world,
-                "d2h_bytes_per_step": (8 + (4 * (2 * (desc.n_inputs // desc.ft_block_rows + desc.n_out_buckets) + 1)
-                                            if args.e2e_source == "records" else 0)) * world,
+                "d2h_bytes_per_step": 8 * world,  # loss and status word
                 "ms_per_step": e2e_s * 1e3 / args.steps,
                 "source": {"records": "raw 32-byte records; featuriser, packing and grouping as kernels on the copy stream",
                            "records-host": "raw 32-byte records; featuriser and packing on the host cores",

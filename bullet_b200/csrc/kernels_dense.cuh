@@ -44,9 +44,7 @@ struct DenseArgs {
     int want_grad;
     unsigned long long* stamp;  // as in FtArgs
     int* gave_up;               // pinned word, raised if a wait for copies runs out
-    // the register-tiled forward also forms the weight and bias gradients of the layers after the
-    // first (it holds everything they need in shared memory): gradient tensors of layers 2 and 3
-    int fuse_small;
+    // gradient tensors (of the kernels that form them on the way)
     float* gW[3];
     float* gB[3];
 };
@@ -83,11 +81,6 @@ __global__ void dense_regroup_kernel(const float* __restrict__ W1, float* __rest
     }
 }
 
-// Shared-memory stride of one column's M1 weights: padded so that the 128-bit reads of
-// eight neighbouring lanes (neighbouring columns) fall into different banks.
-template <int M1>
-__host__ __device__ constexpr int dense_col_stride() { return M1 % 8 == 0 ? M1 + 4 : M1; }
-
 __device__ __forceinline__ void dense_cp_async16(void* smem, const void* gmem) {
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem) : "memory");
@@ -99,40 +92,16 @@ __device__ __forceinline__ void dense_cp_wait() { asm volatile("cp.async.wait_gr
 // Stages columns [chunk*128, chunk*128+128) of bucket k's first-layer weights; columns past
 // K1 are zero-filled.  All 256 threads take part.
 template <int M1>
-__device__ __forceinline__ void dense_stage_chunk(const DenseArgs& a, int k, int chunk, float* buf, bool commit = true) {
-    constexpr int MP = dense_col_stride<M1>();
+__device__ __forceinline__ void dense_stage_chunk(const DenseArgs& a, int k, int chunk, float* buf) {
     const int c_begin = chunk * kDenseChunk;
     const float* src = a.W1g + ((size_t)k * a.K1 + c_begin) * M1;
-    if (M1 % 4 == 0) {
-        constexpr int Q = M1 >= 4 ? M1 / 4 : 1;  // 16-byte pieces per column
-        for (int i = threadIdx.x; i < kDenseChunk * Q; i += blockDim.x) {
-            const int c = i / Q, q = i % Q;
-            float* dst = buf + c * MP + q * 4;
-            if (c_begin + c < a.K1)
-                dense_cp_async16(dst, src + (size_t)c * M1 + q * 4);
-            else
-                *reinterpret_cast<float4*>(dst) = make_float4(0, 0, 0, 0);
-        }
-    } else {
-        for (int i = threadIdx.x; i < kDenseChunk * M1; i += blockDim.x)
-            buf[i] = c_begin + i / M1 < a.K1 ? __ldg(src + i) : 0.f;
-    }
-    if (commit) dense_cp_commit();
+    for (int i = threadIdx.x; i < kDenseChunk * M1; i += blockDim.x) buf[i] = c_begin + i / M1 < a.K1 ? __ldg(src + i) : 0.f;
 }
 
 template <int M1>
 __device__ __forceinline__ void dense_read_weights(const float* buf, int c, float (&w)[M1]) {
-    constexpr int MP = dense_col_stride<M1>();
-    if (M1 % 4 == 0) {
 #pragma unroll
-        for (int r = 0; r < M1; r += 4) {
-            const float4 wv = *reinterpret_cast<const float4*>(buf + c * MP + r);
-            w[r] = wv.x, w[r + 1] = wv.y, w[r + 2] = wv.z, w[r + 3] = wv.w;
-        }
-    } else {
-#pragma unroll
-        for (int r = 0; r < M1; r++) w[r] = buf[c * MP + r];
-    }
+    for (int r = 0; r < M1; r++) w[r] = buf[c * M1 + r];
 }
 
 // One CTA per tile of up to 32 positions of the same output bucket, four per warp.  The
@@ -145,14 +114,14 @@ __device__ __forceinline__ void dense_read_weights(const float* buf, int c, floa
 constexpr int kDenseStages = 3;
 template <int M1>
 __host__ __device__ constexpr size_t dense_fwd_smem() {
-    return (size_t)kDenseStages * (kDenseChunk * dense_col_stride<M1>() + kDenseTile * kDenseChunk) * sizeof(float);
+    return (size_t)kDenseStages * (kDenseChunk * M1 + kDenseTile * kDenseChunk) * sizeof(float);
 }
 
 template <int M1>
-__global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_forward_kernel(DenseArgs a) {
+__global__ void __launch_bounds__(256, 2) dense_forward_kernel(DenseArgs a) {
     step_begin(a.stamp);
-    constexpr int P = kDenseWarpPos, MP = dense_col_stride<M1>();
-    constexpr int kStageFloats = kDenseChunk * MP + kDenseTile * kDenseChunk;
+    constexpr int P = kDenseWarpPos;
+    constexpr int kStageFloats = kDenseChunk * M1 + kDenseTile * kDenseChunk;
     extern __shared__ __align__(16) float dense_smem[];
     __shared__ float loss_part[8];
     __shared__ int s_pos[kDenseTile];
@@ -176,8 +145,8 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_forward_kernel(D
     auto stage = [&](int ch) {
         if (ch < nchunks) {
             float* wb = dense_smem + (ch % kDenseStages) * kStageFloats;
-            float* xb = wb + kDenseChunk * MP;
-            dense_stage_chunk<M1>(a, k, ch, wb, false);
+            float* xb = wb + kDenseChunk * M1;
+            dense_stage_chunk<M1>(a, k, ch, wb);
             for (int i = threadIdx.x; i < kDenseTile * (kDenseChunk / 4); i += blockDim.x) {
                 const int p = i / (kDenseChunk / 4), q = i % (kDenseChunk / 4);
                 const int c = ch * kDenseChunk + q * 4;  // K1 is a multiple of four: a quad is inside or outside
@@ -198,7 +167,7 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_forward_kernel(D
         __syncthreads();
         if (npos) {
             const float* wb = dense_smem + (ch % kDenseStages) * kStageFloats;
-            const float* xb = wb + kDenseChunk * MP + (warp * P) * kDenseChunk;
+            const float* xb = wb + kDenseChunk * M1 + (warp * P) * kDenseChunk;
 #pragma unroll
             for (int jj = 0; jj < 4; jj++) {
                 float w[M1];
@@ -295,10 +264,10 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_forward_kernel(D
 // dx[b][c] = sum_r W1[c][k_b][r] * dz1[b][r]   (Matmul::backward, matmul.rs:99-126, on the
 // selected rows).  Same tiling and weight staging as the forward; grid = ntiles, block = 256.
 template <int M1>
-__global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_dx_kernel(DenseArgs a, float* dx) {
+__global__ void __launch_bounds__(256, 2) dense_dx_kernel(DenseArgs a, float* dx) {
     step_begin(a.stamp);
-    constexpr int P = kDenseWarpPos, MP = dense_col_stride<M1>();
-    __shared__ __align__(16) float wbuf[2][kDenseChunk * MP];
+    constexpr int P = kDenseWarpPos;
+    __shared__ __align__(16) float wbuf[2][kDenseChunk * M1];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int2 t = dense_tile_at(a.tiles, blockIdx.x, a.n);
     if (t.y <= 0) return;
@@ -315,12 +284,7 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_dx_kernel(DenseA
     const int nchunks = (a.K1 + kDenseChunk - 1) / kDenseChunk;
     dense_stage_chunk<M1>(a, k, 0, wbuf[0]);
     for (int ch = 0; ch < nchunks; ch++) {
-        if (ch + 1 < nchunks) {
-            dense_stage_chunk<M1>(a, k, ch + 1, wbuf[(ch + 1) & 1]);
-            dense_cp_wait<1>();
-        } else {
-            dense_cp_wait<0>();
-        }
+        if (ch + 1 < nchunks) dense_stage_chunk<M1>(a, k, ch + 1, wbuf[(ch + 1) & 1]);
         __syncthreads();
         if (npos) {
             const float* buf = wbuf[ch & 1];

@@ -129,7 +129,7 @@ __device__ __forceinline__ void copy16_async(void* smem_dst, const void* src) {
 // With few tiles `split` warps share a slice of one.  The layers behind, and the sum of the parts, have a kernel of their own:
 // they keep a CTA's loads from flowing, and the weights read from L2 for every tile (as much as x) cost 75 us at 131072.
 // At 131072 positions (K1 = 2048, M1 = 16) 0.400 ms for both kernels' work in one, a CTA per tile with x loaded into registers
-// -> DFWD_NOW against 0.165 for reading x at the copy rate.
+// -> 0.245 + 0.037 against 0.165 for reading x at the copy rate; 0.060 -> 0.053 at 16384.
 // grid = (slices, runs), block = 256, dynamic shared memory = dense_mma_smem<M1>().
 constexpr int kSliceCols = 256, kFwdDepth = 5, kFwdAhead = 8;
 template <int M1>
@@ -300,8 +300,8 @@ __host__ __device__ constexpr size_t wgrad_table_floats(size_t i) { return i * (
 // pre-activation gradient (also as the operand of its weight gradient), weight gradients of the small layers and the first
 // layer's bias gradient (kept in registers until the bucket changes).  A CTA takes a
 // run of tiles, a warp eight of a tile's 32 positions: four lanes per position, each with a quarter of the second layer's 32
-// rows (zero past the last); for the weight gradients a lane is a row.  Bound by latency: SMALL_LARGE us at 131072 positions
-// (64 MB of parts), SMALL_MID at 16384.
+// rows (zero past the last); for the weight gradients a lane is a row.  Bound by latency: 37 us at 131072 positions
+// (64 MB of parts), 12 at 16384.
 // grid = up to kSmallCtas per SM, block = 128.
 constexpr int kSmallThreads = 128, kSmallCtas = 4;
 template <int M1>
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(kSmallThreads, M1 > 16 ? 2 : 4) dense_small_mm
         for (int i = 0; i < kPer; i++) z1[i] = 0.f;
         {
             const float* src = a.partial + ((size_t)tile * kDenseTile + min(at, t.y - 1)) * M1 + kPer * quarter;
-#pragma unroll 4
+#pragma unroll 8
             for (int w = 0; w < parts; w++, src += (size_t)a.ntiles * kDenseTile * M1)
                 if constexpr (kPer >= 4) {
 #pragma unroll
@@ -516,7 +516,8 @@ __global__ void __launch_bounds__(kSmallThreads, M1 > 16 ? 2 : 4) dense_small_mm
 
 // dx[b][c] = sum_r W1[c][k_b][r] * dz1[b][r]   (Matmul::backward, matmul.rs:99-126, on the selected rows).  Same tiles; a
 // warp keeps the split gradients of all 32 positions in registers and walks the 16-column groups, storing four neighbouring
-// columns per lane and row.  DDX_BEFORE -> DDX_AFTER ms at 131072 positions (0.165 for writing dx at the copy rate).
+// columns per lane and row.  With fp32 multiply-adds this and the weight
+// gradient took 0.681 ms at 131072 positions, K1 = 2048, M1 = 16; now 0.239 here (0.165 for writing dx at the copy rate).
 // grid = ntiles, block = 256.
 template <int M1>
 __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_dx_mma_kernel(DenseArgs a, float* dx) {
@@ -589,7 +590,7 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_dx_mma_kernel(De
 // run of dense tiles, of which a ninth warp copies eight rows of x and their dz1 (fragments that the small layers' kernel has
 // written in the order of the tiles) at a time into a ring of stages, and adds its sums to the gradient when the output bucket
 // changes.  (x loaded into registers and dz1 split through shared memory a tile at a time, with two barriers: 0.365 ms at
-// 131072 positions, K1 = 2048, M1 = 16; lanes copying their own pieces by cp.async, as the forward does: 0.370; this: DWG_NOW,
+// 131072 positions, K1 = 2048, M1 = 16; lanes copying their own pieces by cp.async, as the forward does: 0.370; this: 0.235,
 // against 0.165 for reading x at the copy rate.  A bulk copy costs the warp that issues it 70 to 100 clocks, so it should be long.)
 // grid = (ceil(K1 / 512), runs), block = 288, dynamic shared memory = wgrad_smem<M1>().
 constexpr int kRingThreads = 288;

@@ -92,7 +92,7 @@ struct TileArgs {
     // 16-byte group is filled with the index of the all-zero row (= block_rows) and never walked
     const uint16_t* lists;  // [2n][list_len]
     int list_len;     // nnz rounded up to a multiple of 8 (16-byte groups)
-    // backward only: the visiting order cut into chunks of at most ft_bwd_chunk pairs that never
+    // backward only: the visiting order cut into chunks of at most kChunkMost pairs that never
     // straddle a block, and per chunk the row-major lists built by ft_csr_kernel
     const int4* chunks;            // [nchunks] (block, first index into `pairs`, pairs, 0)
     uint16_t* csr_ent;             // [nchunks][ent_cap] pairs of the chunk grouped by row, every list starting on 16 bytes
@@ -387,8 +387,8 @@ __device__ __forceinline__ f32x4 sum_lines(const unsigned char* lines, const uin
 // warp's buffer afterwards, so the walk itself reads no global memory.  Every lane adds its four columns with one 16-byte
 // shared-memory load and two packed adds per row, in slot order — the same order and arithmetic as the interpreter.
 // Bound by the shared-memory pipe: 256 bytes per (row, pair, slab) at 128 bytes a clock.  (One pair per warp, 8 bytes per
-// lane, spent twice the instructions per row and was bound by their issue: 1.65 against FWD_LARGE ms at 131072 positions and
-// width 2048, 0.255 against FWD_MID ms at 16384.)
+// lane, spent twice the instructions per row and was bound by their issue: 1.69 against 1.55 ms at 131072 positions and
+// width 2048, 0.273 against 0.260 ms at 16384.)
 constexpr int kFwdThreads = 1024;
 __host__ __device__ inline size_t ft_fwd_smem(int R, int list_len) {
     return (size_t)R * kTileRowBytes + (size_t)(kFwdThreads / 32) * list_len * 4 + 16;
@@ -548,7 +548,7 @@ __host__ __device__ inline size_t ft_csr_smem(int R, int nnz, int cp) {
 
 // grid = most chunks there can be, block = kCsrThreads.  Bound by latency: one load of the lists, whose entries and ranks stay
 // in registers from the count to the fill (a second pass over them, with a second atomic each, made it 15 us instead of
-// CSR_NOW for chunks of 443 pairs; while a step runs, a CTA of this kernel holds up whatever kernel of the step wants its SM).
+// 8.7 for chunks of 443 pairs; while a step runs, a CTA of this kernel holds up whatever kernel of the step wants its SM).
 static __global__ void __launch_bounds__(kCsrThreads) ft_csr_kernel(FtArgs a, TileArgs t) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ int warp_tot[32], bin[kPiece + 1];  // bin: pieces by length, then their first places
@@ -703,10 +703,10 @@ __device__ __forceinline__ int2 ft_bwd_units(const TileArgs& t, int k, int parts
 // that must precede the announcement then finds little to wait for).
 //
 // Staging: a pair's line takes 8 lanes (pairwise: 32 columns of each half of the accumulator) or 16 lanes, 16 bytes per
-// load.  Walk: a half warp per list piece (see sum_lines).  Pieces are handed out `grab` at a time by a shared-memory
-// counter, longest first.  Bound by the shared-memory pipe in the walk (256 bytes per (row, pair, slab)) and by load
-// latency in the staging.  (One row per warp with 8 bytes per lane, rows in table order: 2.29 against BWD_LARGE ms at 131072
-// positions and width 2048, 0.332 against BWD_MID ms at 16384.)
+// load.  Walk: a half warp per list piece (see sum_lines).  Most of the pieces are dealt to the half warps in advance,
+// longest first, the rest handed out by a shared-memory counter.  Bound by the shared-memory pipe in the walk (256 bytes
+// per (row, pair, slab)) and by load latency in the staging.  (One row per warp with 8 bytes per lane, rows in table order: 2.29 against 1.97 ms at 131072
+// positions and width 2048, 0.332 against 0.281 ms at 16384.)
 template <bool PAIRWISE, int THREADS, bool SIGNAL, bool ONE>
 __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_tiled_kernel(FtArgs a, TileArgs t) {
     step_begin(a.stamp);

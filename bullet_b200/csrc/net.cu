@@ -131,9 +131,9 @@ struct b200_net {
     int64_t updates = 0;
     Slot slots[B200_NUM_SLOTS];
     int ft_fwd_mode = B200_FT_AUTO, ft_bwd_mode = B200_FT_AUTO;
-    bool bwd_wide = true;  // shape of the tiled backward (see ft_bwd_chunk)
+    bool bwd_wide = true;  // shape of the tiled backward (see kChunkMost)
     int exchange_bulk = 0;  // the peer exchange moves gradients and weights with bulk asynchronous copies (measured no faster)
-    int bwd_grab = 0;  // rows a warp of the tiled backward takes from the row counter at a time (0: chosen by block size)
+    int bwd_grab = 0;  // eighths of a unit's pieces that the tiled backward deals out in advance (0: the default)
     int wide_chunk = 0;    // the largest chunk of the 1024-thread backward that fits into shared memory
     // Pairs per chunk for a batch of n positions: large chunks save reductions and list copies per pair, small ones fill the
     // SMs evenly when there are few units.  Measured, a unit takes a part that grows with the table's rows and the chunk's
@@ -598,7 +598,6 @@ b200::DenseArgs dense_args(b200_net* net, const Slot& s, bool want_grad) {
     a.out_host = !want_grad && s.n <= kDirectOutputs ? net->h_out : nullptr;
     a.loss = net->G;
     a.want_grad = want_grad ? 1 : 0;
-    a.fuse_small = want_grad && net->fused_small_grads() ? 1 : 0;
     for (int l = 0; l < d.n_dense; l++) {
         char name[16];
         snprintf(name, sizeof name, "l%dw", l + 1);
@@ -1045,13 +1044,17 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     if (net->tiled_promised && d.factoriser_rows == d.ft_block_rows)
         plan.add(&net->facc, (size_t)d.ft_block_rows * d.ft_out / 2);
     if (net->tiled_ok) {
-        // sized for whichever chunk length needs more: every block may end in a partly filled chunk
+        // sized for whichever chunk length needs most, of all that bwd_chunk may choose for a batch: how many chunks there can be
+        // falls in steps, so a length in between may need more than the shortest and the longest
         size_t ent_total = 0, start_total = 0;
-        for (int cp : {b200::kChunkLeast, b200::ft_bwd_chunk_narrow(d.nnz), net->wide_chunk}) {
+        auto room_for = [&](int cp) {
             const size_t chunks = most_chunks(net, (int)B, cp);
             start_total = std::max(start_total, chunks * b200::ft_bwd_start_cap(R, d.nnz, cp));
             ent_total = std::max(ent_total, chunks * b200::ft_bwd_ent_cap(R, d.nnz, cp));
-        }
+        };
+        room_for(b200::ft_bwd_chunk_narrow(d.nnz));
+        for (int cp = net->wide_chunk; cp >= b200::kChunkLeast; cp -= 8) room_for(cp);
+        room_for(net->wide_chunk);
         for (auto& s : net->slots) {
             plan.add(&s.lists, 2 * B * ((d.nnz + 7) & ~7));
             plan.add(&s.csr_ent, ent_total);

@@ -99,7 +99,7 @@ int b200_net_destroy(b200_net* net);
 /* Tuning switches (no counterpart in the reference; every one has a measured default):
  *   "ft_mode" / "ft_fwd_mode" / "ft_bwd_mode"  B200_FT_*; "ft_bwd_wide" 0 = two 512-thread backward CTAs per SM;
  *   "ft_once" accepted, without effect (one form of loads is left);
- *   "ft_bwd_grab" rows a warp of the tiled backward takes from the row counter at a time (0 = by block size);
+ *   "ft_bwd_grab" eighths of a unit's row pieces that the tiled backward deals to its warps in advance (0 = default);
  *   "exchange_bulk" 1 = the peer exchange moves gradients and weights with bulk asynchronous copies;
  *   "overlap_ctas", "overlap_mode", "exchange_ctas", "exchange_wait_ms", "exchange_step", "manual_grad_zero": see the
  *   data-parallel entry points below. */
@@ -158,11 +158,11 @@ int b200_batch_upload_records(b200_net* net, int slot, const void* records, int3
  * the featuriser, the output bucket and the target blend; two more group the positions by output bucket and the
  * (position, perspective) pairs by table row block, in the same stable order the host path produces.  The slot
  * ends up bit-identical to b200_batch_upload_records' (lists, buckets, targets, both orders), so training results
- * are identical too.  The call waits once for two small histograms (it needs them to size the step's launches);
- * everything runs on the library's copy stream, beside a step that is still computing.  What it replaces in the
+ * are identical too.  Nothing is read back: the call returns when everything is enqueued, and it
+ * runs on the library's copy stream, beside a step that is still computing.  What it replaces in the
  * reference: the per-position mapper closure of ValueTrainerState::make_mapper (crates/bullet_lib/src/value.rs:77-117)
  * run by the loader threads (crates/trainer/src/model/inputs.rs:86-109) plus the copy of its five arrays.
- * At most 256 row blocks and 256 output buckets. */
+ * At most 256 output buckets. */
 int b200_batch_upload_records_gpu(b200_net* net, int slot, const void* records, int32_t n, int32_t game, const int32_t* layout32,
                                   float scale, float blend);
 
@@ -275,8 +275,8 @@ int b200_loss_of(b200_net* net, int steps_back, float* loss_sum);
 int b200_forward(b200_net* net, int slot, float* out_host);
 int b200_sync(b200_net* net);
 /* Average device time per phase over the complete steps (backward + update) enqueued since
- * the previous call, at most the last 256; waits for them.  ft_forward and ft_backward each
- * span exactly one kernel launch. */
+ * the previous call, at most the last 256; waits for them.  A phase of b200_step runs from the start of its first
+ * kernel to the start of the next phase's (dense_backward is 0 where the dense forward makes the dense gradients). */
 int b200_get_timings(b200_net* net, b200_timings* out);
 /* Counters: "launches" (kernels launched so far), "h2d_bytes" (batch bytes copied so far),
  * "flat_floats" (length of the flat parameter buffer), "ft_tiled" (bit 0: the forward runs the
@@ -357,7 +357,7 @@ int b200_op_ft_forward(int device, void* stream, const b200_ft_op* op);
  * runtime allocates every buffer through its own Buffer type.)  Use it from code that runs
  * beside a training loop on the same GPU, or after all device memory has been handed out:
  * cudaMalloc/cudaFree stall every stream of the device, and a fixed memory budget leaves
- * nothing to allocate.  The grouping scratch is a fixed array inside the library (about 4.6 MB
+ * nothing to allocate.  The grouping scratch is a fixed array inside the library (about 2.7 MB
  * on every GPU that loads it), so n is limited to B200_OP_NOALLOC_MAX_POSITIONS (half of it
  * when nnz > 32); larger n is refused with B200_ERR_ARG.  No cudaMalloc, cudaFree or other allocating call is made.
  * The first call on a device looks up the array's address: make it before any stream capture.

@@ -1,0 +1,91 @@
+"""The kernels' forms at the edges of their ranges, against the CPU oracle: row-block counts on either side of every way of
+grouping, list lengths and holes, widths that leave a slab or a column group unfilled, dense layers of every row count with
+one tile, one tile more, and batches on either side of the small-batch kernels.
+
+Tolerances: the feature-transformer output is bit-exact (rows are added in slot order); outputs and gradients are sums in
+another order than the oracle's, of fp32 products (the tensor pipe's operands are split so that a product keeps 2^-22): at most
+K = 4096 terms whose rounding errors add like a random walk, sqrt(K) 2^-24 = 4e-6 of the largest term, taken as 2e-5 of the
+largest entry, the bound of the other gradient tests."""
+import numpy as np
+import pytest
+
+from bullet_b200.configs import ACT_CRELU, ACT_NONE, ACT_SCRELU, NetDesc
+
+pytestmark = pytest.mark.gpu
+
+
+def draw_batch(desc, n, seed):
+    """Lists whose features lie in one row block per (position, perspective), with empty slots anywhere."""
+    rng = np.random.default_rng(seed)
+    rows = desc.ft_block_rows or desc.n_inputs
+    lists = []
+    for _ in range(2):
+        block = rng.integers(0, (desc.n_inputs + rows - 1) // rows, n)
+        local = np.argsort(rng.random((n, rows)), axis=1)[:, : desc.nnz]
+        index = block[:, None] * rows + local
+        index[(rng.random(index.shape) < 0.2) | (index >= desc.n_inputs)] = -1
+        lists.append(index.astype(np.int32))
+    return lists[0], lists[1], rng.integers(0, desc.n_out_buckets, n).astype(np.int32), rng.random(n).astype(np.float32)
+
+
+def net_of(blocks, rows, ft_out, nnz, buckets, dense, act=ACT_CRELU, pairwise=False):
+    return NetDesc(n_inputs=blocks * rows, nnz=nnz, ft_out=ft_out, ft_act=act, pairwise=pairwise, n_out_buckets=buckets,
+                   dense_out=dense, dense_act=(ACT_SCRELU,) * (len(dense) - 1) + (ACT_NONE,), ft_block_rows=rows)
+
+
+CASES = {
+    # row blocks: counted up to 32 of them, sorted up to 256, by a kernel of its own beyond; lists of any length
+    "blocks-32": (net_of(32, 64, 64, 20, 1, (1,)), 700),
+    "blocks-33": (net_of(33, 64, 64, 20, 1, (1,)), 700),
+    "blocks-256": (net_of(256, 40, 64, 9, 3, (1,)), 700),
+    "blocks-257": (net_of(257, 40, 64, 9, 3, (1,)), 1300),
+    "list-of-one": (net_of(4, 96, 64, 1, 2, (1,)), 500),
+    "list-of-64": (net_of(2, 200, 64, 64, 2, (1,)), 500),
+    # chunks of a length between the shortest and the longest, few enough that the last one's lists end close to the room
+    "chunks-in-between": (net_of(1, 768, 128, 32, 4, (8, 1)), 313),
+    "chunks-in-between-wide": (net_of(1, 147, 1920, 49, 1, (1,)), 1467),
+    # widths: a part of one slab, a slab and a part, a pairwise half that is no slab
+    "width-8": (net_of(1, 300, 8, 31, 1, (1,), ACT_SCRELU), 1500),
+    "width-72": (net_of(3, 300, 72, 31, 1, (1,), ACT_SCRELU), 1500),
+    "width-200-pairwise": (net_of(3, 300, 200, 32, 8, (16, 32, 1), pairwise=True), 1500),
+    # dense layers: row counts, columns short of a group of 16, of a slice of 256 and of 512; one tile, one more, many
+    "rows-4-columns-16": (net_of(1, 100, 8, 16, 1, (4, 1)), 1),
+    "rows-4-columns-272": (net_of(1, 100, 136, 16, 2, (4, 8, 1)), 33),
+    "rows-8-columns-528": (net_of(1, 100, 264, 16, 5, (8, 16, 1)), 31),
+    "rows-16-columns-2048": (net_of(2, 100, 2048, 16, 8, (16, 32, 1), pairwise=True), 32),
+    "rows-16-columns-1040": (net_of(2, 100, 520, 16, 3, (16, 32, 1)), 2100),
+    "rows-32-columns-784": (net_of(2, 100, 392, 16, 3, (32, 32, 1)), 1100),
+    "rows-32-last-layer": (net_of(1, 100, 64, 16, 64, (32, 1)), 900),
+    "one-row-columns-4096": (net_of(1, 100, 2048, 16, 7, (1,), ACT_SCRELU), 37),
+    "one-row-columns-16": (net_of(1, 100, 8, 16, 64, (1,)), 1000),
+}
+
+
+@pytest.mark.parametrize("case", CASES)
+def test_kernel_forms_at_the_edges_of_their_ranges(oracle32, case):
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, oracle_ft_output, rich_weights
+
+    desc, n = CASES[case]
+    desc = dataclasses.replace(desc, max_batch=n)
+    batch = draw_batch(desc, n, seed=len(case) + n)
+    w = rich_weights(desc)
+    x_ref = oracle_ft_output(oracle32, desc, w, *batch[:2])
+    loss_ref, g_ref, out_ref = oracle32.net_grad(desc, w, *batch)
+    net = make_net(desc, 0, w)
+    net.upload(0, *batch)
+    out = net.forward(0, n)
+    assert np.array_equal(net.activation(0, n * desc.dense_in0).reshape(n, -1), x_ref)
+    assert np.abs(out - out_ref).max() <= 2e-5 * np.abs(out_ref).max()
+    net.step(0, 0.0, 1.0 / n)  # a whole step that leaves the weights where they are
+    assert np.array_equal(net.activation(0, n * desc.dense_in0).reshape(n, -1), x_ref)
+    assert abs(net.loss() - loss_ref) <= 2e-5 * loss_ref
+    g = net.tensors(kind=3)
+    for k in g_ref:
+        assert np.abs(g[k] - g_ref[k]).max() <= 2e-5 * np.abs(g_ref[k]).max(), k
+    net.backward(0)  # the same in phases
+    g = net.tensors(kind=3)
+    for k in g_ref:
+        assert np.abs(g[k] - g_ref[k]).max() <= 2e-5 * np.abs(g_ref[k]).max(), k
+    net.close()
