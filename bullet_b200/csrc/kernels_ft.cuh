@@ -857,21 +857,25 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
                 }
             }
         }
-        // the four table columns this lane sums
-        const int col_w = !PAIRWISE ? slab * 64 + 4 * l16 : l16 < 8 ? slab * 32 + 4 * l16 : a.H / 2 + slab * 32 + 4 * (l16 - 8);
+        // the four table columns this lane sums; those past the width (the last slab of one that 64 does not divide) are not
+        // the table's to write, whatever was staged for them: a loss gradient that is not finite makes NaN of their zeros
+        const int in_half = PAIRWISE ? slab * 32 + 4 * (l16 & 7) : slab * 64 + 4 * l16;
+        const int col_w = PAIRWISE && l16 >= 8 ? a.H / 2 + in_half : in_half;
+        const bool col_on = in_half < x_row;
         float* g_block = a.g_table + (size_t)block * R * a.H + col_w;
         if (threadIdx.x >= kBwdThreads - kTileCols) {
             const int j = (int)threadIdx.x - (kBwdThreads - kTileCols);
             float sum = 0.f;
 #pragma unroll 8
             for (int w = 0; w < NW; w++) sum += bias_s[w * kTileCols + j];
-            if (sum != 0.f) atomicAdd(a.g_bias + (!PAIRWISE ? slab * 64 + j : j < 32 ? slab * 32 + j : a.H / 2 + slab * 32 + j - 32), sum);
+            const int c = PAIRWISE ? slab * 32 + (j & 31) : slab * 64 + j;
+            if (c < x_row && sum != 0.f) atomicAdd(a.g_bias + (PAIRWISE && j >= 32 ? a.H / 2 + c : c), sum);
         }
         const int pieces = start[1];
         auto walk = [&](unsigned piece) {
             const f32x4 acc = sum_lines(smem_raw, reinterpret_cast<const uint2*>(ent) + (piece >> 17), (int)(piece >> 10) & 0x7f, lane16);
             const float4 g = make_float4(lo2(acc.a), hi2(acc.a), lo2(acc.b), hi2(acc.b));
-            if (g.x != 0.f || g.y != 0.f || g.z != 0.f || g.w != 0.f)
+            if (col_on && (g.x != 0.f || g.y != 0.f || g.z != 0.f || g.w != 0.f))
                 atomicAdd(reinterpret_cast<float4*>(g_block + (size_t)(piece & 0x3ffu) * a.H), g);
         };
         // most pieces are dealt to the half warps, to and fro, so that each gets the same mixture of lengths; the shortest are

@@ -89,3 +89,49 @@ def test_kernel_forms_at_the_edges_of_their_ranges(oracle32, case):
     for k in g_ref:
         assert np.abs(g[k] - g_ref[k]).max() <= 2e-5 * np.abs(g_ref[k]).max(), k
     net.close()
+
+
+@pytest.mark.parametrize("ft_out,pairwise,act,buckets", [(72, False, ACT_SCRELU, 1), (96, False, ACT_CRELU, 3), (136, True, ACT_CRELU, 2)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_a_loss_gradient_that_is_not_finite_stays_in_its_rows(oracle32, ft_out, pairwise, act, buckets, mode):
+    """One target is NaN: the rows that its position holds are lost, every other row's gradient is what the other positions
+    give.  The widths leave a part of the last slab of 64 columns empty; nothing may be written past them.  Bounds as above."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    n, bad = 40, 17
+    desc = dataclasses.replace(net_of(1, 300, ft_out, 31, buckets, (1,), act, pairwise), max_batch=n)
+    stm, nstm, bucket, target = draw_batch(desc, n, seed=ft_out)
+    w = rich_weights(desc)
+    rest = np.arange(n) != bad
+    _, g_ref, _ = oracle32.net_grad(desc, w, stm[rest], nstm[rest], bucket[rest], target[rest])
+    target[bad] = np.nan
+    net = make_net(desc, mode, w)
+    net.upload(0, stm, nstm, bucket, target)
+    lost = np.zeros(desc.n_inputs, dtype=bool)
+    for row in np.concatenate([stm[bad], nstm[bad]]):
+        lost[max(row, 0)] |= row >= 0
+    ref = g_ref["l0w"].reshape(desc.n_inputs, ft_out)
+    for step in (lambda: net.backward(0), lambda: net.step(0, 0.0, 1.0 / n)):
+        step()
+        g = net.tensors(kind=3)
+        got = g["l0w"].reshape(desc.n_inputs, ft_out)
+        assert np.isnan(got[lost]).all()
+        assert np.isnan(g["l0b"]).all()
+        assert np.abs(got[~lost] - ref[~lost]).max() <= 2e-5 * np.abs(ref).max()
+        first = net.tensor_range("l0w")[0]  # what lies behind the last row
+        assert not np.isnan(net_flat(net, 3)[first + got.size:]).any()
+    net.close()
+
+
+def net_flat(net, kind):
+    import torch
+
+    class Buffer:
+        pass
+
+    ptr, count = net.flat_buffer(kind)
+    Buffer.__cuda_array_interface__ = {"shape": (count,), "typestr": "<f4", "data": (ptr, False), "version": 3, "strides": None}
+    net.sync()
+    return torch.as_tensor(Buffer(), device="cuda").cpu().numpy()
