@@ -207,9 +207,12 @@ struct b200_net {
     int64_t launches = 0, h2d_bytes = 0;
     std::vector<void*> allocations;
 
-    int* kept_bucket = nullptr;  // dense_one: the output bucket of every position of the last pass
-    int w1_now = 0;              // which of two copies of the regrouped weights is current; the last pass may have used the other
-    const float* w1_used = nullptr;
+    int* kept_bucket = nullptr;  // dense_one: the output bucket of every position of the last training pass
+    int w1_now = 0;              // which of two copies of the regrouped weights is current; the last training pass may have used the other
+    const float* w1_used = nullptr;  // the copy that the last training pass used
+    int grad_n = 0;              // its positions (0: none has run)
+    bool dx_formed = false;      // dx holds its gradient at x, which such a network forms only where somebody asks
+    float* w1g_copy(int k) const { return w1g + (size_t)k * d.n_out_buckets * d.dense_out[0] * D1(); }
     int D1() const { return d.pairwise ? d.ft_out : 2 * d.ft_out; }
     int dense_in(int l) const { return l == 0 ? D1() : d.dense_out[l - 1]; }
     Tensor* find(const char* name) {
@@ -231,7 +234,7 @@ struct b200_net {
     // The gather forward of n positions reads the merged table (one row per feature, after a pass over the whole table)
     // when the batch gathers several times the table's rows; below that it adds the factoriser row by row.
     bool merged_table(int n) const { return d.factoriser_rows && !fwd_tiled(n) && (long long)n * d.nnz >= 5LL * d.n_inputs; }
-    float* w1g_now() const { return w1g ? w1g + (size_t)w1_now * d.n_out_buckets * d.dense_out[0] * D1() : nullptr; }
+    float* w1g_now() const { return w1g ? w1g_copy(w1_now) : nullptr; }
     void weights_moved() { w1_dirty = merged_dirty = true; }
     bool bwd_tiled() const { return ft_bwd_mode == B200_FT_TILED || (ft_bwd_mode == B200_FT_AUTO && tiled_ok); }
     // the register-tiled dense forward (rows per bucket in fours, more layers after the first) also
@@ -608,6 +611,15 @@ b200::DenseArgs dense_args(b200_net* net, const Slot& s, bool want_grad) {
     return a;
 }
 
+// dense_one: the gradient at x of the last training pass, for inspection (the backward forms it where it uses it)
+int form_dx(b200_net* net) {
+    if (net->grad_n < 1 || net->dx_formed) return 0;
+    b200::dense_one_dx_kernel<<<net->sm_count * 8, 256, 0, net->stream>>>(net->w1_used, net->dz[0], net->kept_bucket, net->dx, net->grad_n, net->D1());
+    LAUNCHED(net);
+    net->dx_formed = true;
+    return 0;
+}
+
 int refresh_table(b200_net* net, int n) {
     if (net->merged_dirty && net->merged_table(n)) {
         const Tensor* w = net->find("l0w");
@@ -628,6 +640,8 @@ int refresh_table(b200_net* net, int n) {
                 net->P + w1->off, net->w1f, net->w1d, net->D1(), O, M1, M1 >= 8 ? M1 / 8 : 1);
         } else {
             net->w1_now ^= 1;
+            if (net->w1g_now() == net->w1_used)  // (only if the weights moved twice since the last training pass)
+                if (int rc = form_dx(net)) return rc;
             b200::dense_regroup_kernel<<<std::min<int>(net->sm_count * 4, (int)((w1->n + 255) / 256)), 256, 0, net->stream>>>(
                 net->P + w1->off, net->w1g_now(), net->D1(), O, M1);
         }
@@ -775,7 +789,7 @@ int forward_dense(b200_net* net, Slot& s, bool want_grad) {
         a.want_grad = da.want_grad;
         a.stamp = da.stamp;
         a.gave_up = net->h_gave_up;
-        net->w1_used = da.W1g;
+        if (want_grad) net->w1_used = da.W1g, net->grad_n = s.n, net->dx_formed = false;
         const size_t smem = b200::one_smem(a.K1);
         const int units = a.ntiles * (b200::kDenseTile / b200::one_rows(a.K1)), slots = net->sm_count * std::max(1, std::min(4, (int)(220 * 1024 / smem)));
         a.units_per_run = (units + slots - 1) / slots;
@@ -2379,9 +2393,10 @@ int b200_net_get_activation(b200_net* net, int which, float* host, int64_t n) {
     if (!src || want == 0) return b200::fail(B200_ERR_STATE, "get_activation: buffer %d is not used by this network", which);
     if (n != want) return b200::fail(B200_ERR_ARG, "get_activation: buffer %d holds %lld values, %lld asked", which, (long long)want, (long long)n);
     if (int rc = set_device(net)) return rc;
-    if (which == 2 && net->dense_one() && net->w1_used) {  // formed on the fly by the backward: form it once more
-        b200::dense_one_dx_kernel<<<net->sm_count * 8, 256, 0, net->stream>>>(net->w1_used, net->dz[0], net->kept_bucket, net->dx, (int)B, net->D1());
-        LAUNCHED(net);
+    if (which == 2 && net->dense_one()) {
+        if (int rc = form_dx(net)) return rc;
+        // the last pass may have been an evaluation of more positions: those have no gradient
+        if (B > net->grad_n) CK(cudaMemsetAsync(net->dx + net->grad_n * (int64_t)net->D1(), 0, (size_t)(B - net->grad_n) * net->D1() * sizeof(float), net->stream));
     }
     CK(cudaStreamSynchronize(net->stream));
     CK(cudaMemcpy(host, src, n * sizeof(float), cudaMemcpyDeviceToHost));

@@ -135,3 +135,57 @@ def net_flat(net, kind):
     Buffer.__cuda_array_interface__ = {"shape": (count,), "typestr": "<f4", "data": (ptr, False), "version": 3, "strides": None}
     net.sync()
     return torch.as_tensor(Buffer(), device="cuda").cpu().numpy()
+
+
+@pytest.mark.parametrize("act,buckets", [(ACT_CRELU, 1), (ACT_SCRELU, 4)])
+def test_gradient_at_x_is_that_of_the_last_training_pass(act, buckets):
+    """Networks with one dense row per bucket keep no gradient at x, but tell it: that of the last training pass, also after
+    evaluations of more positions, an update, and weights that were set anew.  Positions without one are zero."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    few, many = 8, 100
+    desc = dataclasses.replace(net_of(1, 300, 64, 31, buckets, (1,), act), max_batch=many)
+    K = desc.dense_in0
+    w = rich_weights(desc)
+    net = make_net(desc, 0, w)
+    stm, nstm, bucket, target = draw_batch(desc, many, seed=3)
+    net.upload(0, stm[:few], nstm[:few], bucket[:few], target[:few])
+    net.upload(1, stm, nstm, bucket, target)
+    net.forward(1, many)
+    assert not net.activation(2, many * K).any()  # no training pass yet
+    net.backward(0)
+    # the weight of the position's bucket times its loss gradient
+    out = net.activation(3, few).astype(np.float64)
+    s = 1 / (1 + np.exp(-out))
+    dout = 2 * (s - target[:few]) * s * (1 - s)
+    ref = w["l1w"].reshape(K, buckets).T[bucket[:few]] * dout[:, None]
+    got = net.activation(2, few * K).reshape(few, K)
+    assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()  # of 32 bits, and of the sigmoid's exponential
+
+    def check():
+        dx = net.activation(2, many * K).reshape(many, K)
+        assert np.array_equal(dx[:few], got) and not dx[few:].any()
+
+    net.forward(1, many)
+    check()
+    net.update(1e-2, 1.0 / few)
+    net.forward(1, many)
+    check()
+    for seed in (11, 12):
+        net.load_weights(rich_weights(desc, seed=seed))
+        net.forward(1, many)
+        check()
+    net.step(0, 1e-2, 1.0 / few)  # the next training pass, in one call, with the weights set last
+    out = net.activation(3, few).astype(np.float64)
+    s = 1 / (1 + np.exp(-out))
+    dout = 2 * (s - target[:few]) * s * (1 - s)
+    ref = rich_weights(desc, seed=12)["l1w"].reshape(K, buckets).T[bucket[:few]] * dout[:, None]
+    got = net.activation(2, few * K).reshape(few, K)
+    assert np.abs(got - ref).max() <= 1e-5 * np.abs(ref).max()
+    for seed in (13, 14, 15):  # formed only now, after the copy that the pass used would have been overwritten
+        net.load_weights(rich_weights(desc, seed=seed))
+        net.forward(1, many)
+    check()
+    net.close()
