@@ -747,7 +747,9 @@ int build_csr(b200_net* net, Slot& s, cudaStream_t stream) {
 // The forward pass in three pieces: the per-pair row lists, the feature-transformer items of a
 // run of work items, and the dense layers.
 int forward_prepare(b200_net* net, Slot& s, bool want_grad) {
-    const bool needed = net->fwd_tiled(s.n) || (want_grad && net->bwd_tiled());
+    // (a training pass wants the lists whenever its kernels may be the tiled ones, also where a small batch then takes the
+    // gather forward: they report features outside their block, and the forward may be run in parts, which are tiled)
+    const bool needed = want_grad ? net->fwd_tiled() || net->bwd_tiled() : net->fwd_tiled(s.n);
     if (needed && !s.prepared) {  // normally built at upload; here on the first training pass or after a change of kernels
         cut_ft(net, s);
         if (int rc = group_slot(net, s, group_args(net, s, true, false), false, net->stream)) return rc;
@@ -1372,7 +1374,7 @@ static int upload_begin(b200_net* net, int slot, int32_t n, const char* who) {
 // The row lists of the tiled kernels depend on the indices only: they are built right behind the copy, on the copy stream,
 // where they run beside the step that is still computing.  What only the backward reads waits for a network that trains.
 static bool upload_wants_lists(const b200_net* net, int32_t n) {
-    return net->tiled_ok && (net->fwd_tiled(n) || (net->bwd_tiled() && net->trains));
+    return net->tiled_ok && (net->trains ? net->fwd_tiled() || net->bwd_tiled() : net->fwd_tiled(n));
 }
 
 // Common end: the slot's batch is on its way to the device; group it and mark the slot ready.

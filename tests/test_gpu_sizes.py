@@ -189,3 +189,50 @@ def test_gradient_at_x_is_that_of_the_last_training_pass(act, buckets):
         net.forward(1, many)
     check()
     net.close()
+
+
+@pytest.mark.parametrize("bwd_mode", [0, 1])
+def test_forward_in_parts_and_reports_of_a_small_batch(oracle32, bwd_mode):
+    """A batch small enough for the gather forward, with the backward's kernels left to choose and the gather ones asked for:
+    the forward may still be run in parts, by the tiled kernel, also in a slot that held another batch before, and a feature
+    outside its row block is still reported.  Bounds as above."""
+    import dataclasses
+
+    from bullet_b200._lib import B200Error
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    most, n = 900, 6
+    desc = dataclasses.replace(net_of(8, 96, 64, 20, 2, (8, 1)), max_batch=most)
+    w = rich_weights(desc)
+    net = make_net(desc, 0, w)
+    net.set_option("ft_bwd_mode", bwd_mode)
+    for count, seed in ((n, 5), (most, 6), (n, 7)):
+        stm, nstm, bucket, target = draw_batch(desc, count, seed)
+        net.upload(0, stm, nstm, bucket, target)
+        x_ref = oracle_x(oracle32, desc, w, stm, nstm)
+        _, g_ref, _ = oracle32.net_grad(desc, w, stm, nstm, bucket, target)
+        for parts in (4, 1):
+            net.forward_begin(0)
+            for part in range(parts):
+                net.forward_ft(0, part, parts)
+            net.backward_begin(0)
+            assert np.array_equal(net.activation(0, count * desc.dense_in0).reshape(count, -1), x_ref)
+            net.backward_ft(0, 0, 1)
+            net.backward_end(0)
+            g = net.tensors(kind=3)
+            for k in g_ref:
+                assert np.abs(g[k] - g_ref[k]).max() <= 2e-5 * np.abs(g_ref[k]).max(), k
+    stm[0, :2] = [3, 200]  # rows of two blocks
+    net.upload(1, stm, nstm, bucket, target)
+    for step in (lambda: net.step(1, 0.0, 1.0 / n), lambda: (net.backward(1), net.update(0.0, 1.0 / n))):
+        step()
+        with pytest.raises(B200Error) as e:
+            net.loss()
+        assert e.value.code == -4
+    net.close()
+
+
+def oracle_x(oracle32, desc, w, stm, nstm):
+    from tests.test_gpu_parity import oracle_ft_output
+
+    return oracle_ft_output(oracle32, desc, w, stm, nstm)
