@@ -36,12 +36,13 @@ namespace {
 
 constexpr int kMaxBlocks = 1024;  // table row blocks the grouping supports
 
-// Scratch layout, in ints, every section on a 256-byte boundary: the blocks' first pairs, per pair its
+// Scratch layout, in ints, every section on a 256-byte boundary: the blocks' first pairs and a status word, per pair its
 // block and list length [2n], (pair id, rows) [2n] and the prepared row lists [2n][nnz rounded up to 8] as u16, then the
 // histograms of the grouping's first pass, or its counters where there are more blocks than its windows hold.
 constexpr size_t kSectionAlign = 64;  // ints
 constexpr size_t align_ints(size_t v) { return (v + kSectionAlign - 1) / kSectionAlign * kSectionAlign; }
-constexpr size_t kScratchHeader = align_ints(kMaxBlocks + 1);
+constexpr size_t kStatusAt = kMaxBlocks + 1;
+constexpr size_t kScratchHeader = align_ints(kMaxBlocks + 2);
 constexpr int list_len(int nnz) { return (nnz + 7) & ~7; }  // 16-byte groups of u16 row indices
 constexpr size_t hist_ints(int n, int nblocks) {
     return nblocks > b200::kGroupMaxBlocks ? align_ints(3 * (size_t)(nblocks + 3))
@@ -58,32 +59,55 @@ constexpr size_t scratch_ints(int n, int nnz, int nblocks) {
 constexpr size_t kStaticInts = scratch_ints(B200_OP_NOALLOC_MAX_POSITIONS, 32, b200::kGroupMaxBlocks);
 static __device__ __align__(256) int g_op_scratch[kStaticInts];
 
-// A call's status word: pinned host memory that the kernels touch only if there is something to report, so that nothing has
-// to be copied back.  A process keeps one block of them (4 KB for as long as it lives); a call holds one for its duration.
-constexpr int kStatusWords = 64;
+// A call's status word: memory of the library image that both sides may touch at any time, and that the kernels touch only if
+// there is something to report, so that nothing has to be allocated and nothing copied back.  (A 4-byte copy behind the forward
+// takes 10 us: b200_op_ft_forward_noalloc on 2048 positions, king buckets, width 1024: 72 us with it, 62 without.)  A call holds a
+// word from its first kernel until its stream has finished.  A call that finds none free, or a device that cannot share such
+// memory while it is running, has the word in its scratch and copies it back.
+constexpr int kStatusWords = 64, kStatusStride = 16;  // (a cache line each)
+static __managed__ int g_op_status[kStatusWords * kStatusStride];
+
+// Whether `device` can share g_op_status; asks the runtime once per device, and has the words stay in host memory.
+bool shares_status(int device) {
+    constexpr int kDevices = 64;
+    static std::atomic<signed char> known[kDevices];  // 0 not asked yet, 1 yes, -1 no
+    if (device < 0 || device >= kDevices) return false;
+    if (const signed char k = known[device]) return k > 0;
+    int concurrent = 0;
+    if (cudaDeviceGetAttribute(&concurrent, cudaDevAttrConcurrentManagedAccess, device) != cudaSuccess) concurrent = 0;
+    if (concurrent) {  // (hints: without them a report would move the page to the device and back)
+        cudaMemAdvise(g_op_status, sizeof g_op_status, cudaMemAdviseSetPreferredLocation, cudaCpuDeviceId);
+        cudaMemAdvise(g_op_status, sizeof g_op_status, cudaMemAdviseSetAccessedBy, device);
+    }
+    cudaGetLastError();
+    known[device] = concurrent ? 1 : -1;
+    return concurrent != 0;
+}
+
 struct StatusWord {
-    int* status = nullptr;
-    StatusWord() {
-        static int* words = [] {
-            void* raw = nullptr;
-            return cudaHostAlloc(&raw, kStatusWords * 64, cudaHostAllocPortable) == cudaSuccess ? static_cast<int*>(raw) : nullptr;
-        }();
-        if (!words) return;
-        while (!status)  // as many calls as there are words are under way at once at most
-            for (int k = 0; k < kStatusWords && !status; k++) {
-                bool free = false;
-                if (taken()[k].compare_exchange_strong(free, true)) at = k, status = words + 16 * k;
-            }
-        *status = 0;
+    StatusWord(int device, cudaStream_t on) : stream(on) {
+        if (!shares_status(device)) return;
+        for (int k = 0; k < kStatusWords && !status; k++) {
+            bool free = false;
+            if (taken()[k].compare_exchange_strong(free, true)) at = k, status = g_op_status + kStatusStride * k;
+        }
+        if (status) *status = 0;
     }
     ~StatusWord() {
-        if (status) taken()[at] = false;
+        if (!status) return;
+        if (!finished) cudaStreamSynchronize(stream);  // a call that failed half way: kernels may still be about to write
+        taken()[at] = false;
     }
+    StatusWord(const StatusWord&) = delete;
+    StatusWord& operator=(const StatusWord&) = delete;
     static std::atomic<bool>* taken() {
         static std::atomic<bool> flags[kStatusWords];
         return flags;
     }
+    cudaStream_t stream;
+    int* status = nullptr;
     int at = 0;
+    bool finished = false;
 };
 
 int check_op(const b200_ft_op* op, const char* who) {
@@ -111,8 +135,8 @@ int check_op(const b200_ft_op* op, const char* who) {
 // reports a feature outside its block.  Allocates nothing.
 int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) {
     const int n = op->n, R = op->ft_block_rows, nblocks = op->n_inputs / R;
-    StatusWord word;
-    if (!word.status) return b200::fail(B200_ERR_CUDA, "op_ft_forward: no pinned memory for a status word");
+    StatusWord word(device, stream);
+    int* status = word.status ? word.status : scratch + kStatusAt;
     int* begin = scratch;
     int* info = scratch + kScratchHeader;
     int* pairs = info + align_ints((size_t)2 * n);
@@ -129,7 +153,8 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
     g.n_out_buckets = 1;
     g.info = info;
     g.hist = hist;
-    g.status = word.status;
+    g.status = status;
+    g.clear_status = !word.status;
     g.want_lists = 1;
     g.pairs = reinterpret_cast<int2*>(pairs);
     g.lists = reinterpret_cast<uint16_t*>(lists);
@@ -167,7 +192,7 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
     t.last_block = nblocks;
     t.pairs = g.pairs;
     t.block_begin = begin;
-    t.status = word.status;
+    t.status = status;
     t.lists = g.lists;
     t.list_len = g.list_len;
     const size_t smem = b200::ft_fwd_smem(R, t.list_len);
@@ -183,8 +208,12 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
         b200::ft_forward_tiled_kernel<false><<<ctas, b200::kFwdThreads, smem, stream>>>(a, t);
     }
     CK(cudaGetLastError());
+    int reported = 0;
+    if (!word.status) CK(cudaMemcpyAsync(&reported, status, sizeof reported, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
-    if (*reinterpret_cast<volatile int*>(word.status) & b200::kStatusOutsideBlock)
+    word.finished = true;
+    if (word.status) reported = *reinterpret_cast<volatile int*>(status);
+    if (reported & b200::kStatusOutsideBlock)
         return b200::fail(B200_ERR_DATA, "a feature index fell outside the row block of its position (ft_block_rows=%d)", R);
     return 0;
 }

@@ -359,7 +359,8 @@ int b200_op_ft_forward(int device, void* stream, const b200_ft_op* op);
  * cudaMalloc/cudaFree stall every stream of the device, and a fixed memory budget leaves
  * nothing to allocate.  The grouping scratch is a fixed array inside the library (about 2.7 MB
  * on every GPU that loads it), so n is limited to B200_OP_NOALLOC_MAX_POSITIONS (half of it
- * when nnz > 32); larger n is refused with B200_ERR_ARG.  No cudaMalloc, cudaFree or other allocating call is made.
+ * when nnz > 32); larger n is refused with B200_ERR_ARG.  No cudaMalloc, cudaFree or other allocating call is made, of device
+ * or of host memory, not by a process's first call either.
  * The first call on a device looks up the array's address: make it before any stream capture.
  * Calls on one device share the array, so calls whose GPU work overlaps race: serialise them. */
 #define B200_OP_NOALLOC_MAX_POSITIONS 16384

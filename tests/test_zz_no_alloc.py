@@ -61,3 +61,59 @@ def test_noalloc_wide_index_lists_and_their_smaller_limit(oracle32):
     assert rc == -1 and b"8192" in _lib.load().b200_last_error()
     rc, x, _ = run_op("b200_op_ft_forward", desc, table, w["l0b"], stm, nstm, n + 1)   # the allocating entry takes it
     assert rc == 0 and np.array_equal(x, x_ref)
+
+
+FIRST_CALL = """
+import ctypes, sys
+import numpy as np, torch
+from bullet_b200 import _lib
+n, rows, H = 300, 96, 64
+table, bias = torch.randn((4 * rows, H), device="cuda"), torch.randn(H, device="cuda")
+index = torch.randint(0, rows, (2, n, 20), device="cuda").to(torch.int16)
+x = torch.zeros((n, 2 * H), device="cuda")
+op = _lib.CFtOp(4 * rows, 20, H, 1, 0, rows, n, table.data_ptr(), bias.data_ptr(), index[0].data_ptr(), index[1].data_ptr(), x.data_ptr(), None)
+lib = _lib.load()
+torch.cuda.synchronize()
+with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU, torch.profiler.ProfilerActivity.CUDA]) as trace:
+    rc = lib.b200_op_ft_forward_noalloc(0, None, ctypes.byref(op))
+    torch.cuda.synchronize()
+assert rc == 0
+print(" ".join(sorted({e.name for e in trace.events() if e.name.startswith("cu")})))
+"""
+
+
+def test_the_first_call_of_a_process_makes_no_allocating_call():
+    """A trace of the runtime calls of a process's first operator call holds its launches, and nothing that allocates."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", FIRST_CALL], cwd=root, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr
+    calls = done.stdout.split()
+    if not any("Launch" in c for c in calls):
+        pytest.skip("this machine lets no process trace its runtime calls")
+    assert not [c for c in calls if any(word in c for word in ("Alloc", "Malloc", "Free", "Register"))], calls
+
+
+@pytest.mark.parametrize("entry", ["b200_op_ft_forward", "b200_op_ft_forward_noalloc"])
+def test_reports_of_calls_that_follow_each_other_or_run_together(oracle32, entry):
+    """A feature outside its row block is reported by the call that met it and by no other, whichever came before; from more
+    threads at once than there are status words as well (the allocation-free calls one after the other, as they must be)."""
+    from concurrent.futures import ThreadPoolExecutor
+
+    name, desc, game = CASES[0]
+    n = 200
+    stm, nstm, w, table, x_ref = op_inputs(oracle32, desc, game, n, 76)
+    bad = stm.copy()
+    bad[n - 1, :2] = [5, 800]
+
+    def call(wrong):
+        rc, x, _ = run_op(entry, desc, table, w["l0b"], bad if wrong else stm, nstm, n)
+        return rc == (-4 if wrong else 0) and (wrong or np.array_equal(x, x_ref))
+
+    assert all(call(wrong) for wrong in (True, False, True, True, False, False))
+    if entry == "b200_op_ft_forward":
+        with ThreadPoolExecutor(80) as pool:
+            assert all(pool.map(call, [k % 3 == 0 for k in range(240)]))
