@@ -379,6 +379,17 @@ __device__ __forceinline__ f32x4 sum_lines(const unsigned char* lines, const uin
     return acc;
 }
 
+template <bool ANY>
+__device__ __forceinline__ void store_piece(float* p, float2 v) {
+    if (ANY) p[0] = v.x, p[1] = v.y;
+    else *reinterpret_cast<float2*>(p) = v;
+}
+template <bool ANY>
+__device__ __forceinline__ void store_piece(float* p, float4 v) {
+    if (ANY) p[0] = v.x, p[1] = v.y, p[2] = v.z, p[3] = v.w;
+    else *reinterpret_cast<float4*>(p) = v;
+}
+
 // Forward.  One CTA of 1024 threads per SM; dynamic shared memory = R tile rows, then per warp two prepared lists (and 16
 // bytes that a read-ahead may touch).  A CTA walks its piece of the work line segment by segment; a segment is a run of
 // pairs of one (block, slab), whose tile the CTA loads first.  Each warp serves two neighbouring pairs at a time, one per
@@ -394,7 +405,9 @@ __host__ __device__ inline size_t ft_fwd_smem(int R, int list_len) {
     return (size_t)R * kTileRowBytes + (size_t)(kFwdThreads / 32) * list_len * 4 + 16;
 }
 
-template <bool PAIRWISE>
+// ANY: bias, x and u start on any float (the operator's caller owns them); else on 8 bytes with the pairwise product, on 16
+// without, and move in pieces of that size.
+template <bool PAIRWISE, bool ANY = false>
 __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs a, TileArgs t) {
     ft_step_begin(a);
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -465,6 +478,9 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
         f32x4 bias = {0, 0};
         const bool col_on = col < x_row;
         if (!col_on) {
+        } else if (ANY) {
+            const float* b = a.bias + col;
+            bias = PAIRWISE ? f32x4{pack2(b[0], b[a.H / 2]), pack2(b[1], b[a.H / 2 + 1])} : f32x4{pack2(b[0], b[1]), pack2(b[2], b[3])};
         } else if (PAIRWISE) {
             const float2 lo = *reinterpret_cast<const float2*>(a.bias + col), hi = *reinterpret_cast<const float2*>(a.bias + a.H / 2 + col);
             bias = {pack2(lo.x, hi.x), pack2(lo.y, hi.y)};
@@ -499,12 +515,13 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
                 if (PAIRWISE) {
                     const float2 ulo = make_float2(crelu_f(lo2(acc.a)), crelu_f(lo2(acc.b))), uhi = make_float2(crelu_f(hi2(acc.a)), crelu_f(hi2(acc.b)));
                     float* up = a.u + (size_t)pair * a.H + col;
-                    *reinterpret_cast<float2*>(up) = ulo;
-                    *reinterpret_cast<float2*>(up + a.H / 2) = uhi;
-                    *reinterpret_cast<float2*>(x_out + (size_t)pair * x_row) = make_float2(ulo.x * uhi.x, ulo.y * uhi.y);
+                    store_piece<ANY>(up, ulo);
+                    store_piece<ANY>(up + a.H / 2, uhi);
+                    store_piece<ANY>(x_out + (size_t)pair * x_row, make_float2(ulo.x * uhi.x, ulo.y * uhi.y));
                 } else {
-                    *reinterpret_cast<float4*>(x_out + (size_t)pair * x_row) =
-                        make_float4(ft_act_fwd(a.act, lo2(acc.a)), ft_act_fwd(a.act, hi2(acc.a)), ft_act_fwd(a.act, lo2(acc.b)), ft_act_fwd(a.act, hi2(acc.b)));
+                    store_piece<ANY>(
+                        x_out + (size_t)pair * x_row,
+                        make_float4(ft_act_fwd(a.act, lo2(acc.a)), ft_act_fwd(a.act, hi2(acc.a)), ft_act_fwd(a.act, lo2(acc.b)), ft_act_fwd(a.act, hi2(acc.b))));
                 }
             }
         }

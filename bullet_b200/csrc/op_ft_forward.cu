@@ -200,13 +200,13 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const int ctas = (int)std::max<long long>(1, std::min<long long>(sms, (long long)2 * n * t.nslabs / 128));
-    if (op->pairwise) {
-        CK(b200::allow_smem(b200::ft_forward_tiled_kernel<true>));
-        b200::ft_forward_tiled_kernel<true><<<ctas, b200::kFwdThreads, smem, stream>>>(a, t);
-    } else {
-        CK(b200::allow_smem(b200::ft_forward_tiled_kernel<false>));
-        b200::ft_forward_tiled_kernel<false><<<ctas, b200::kFwdThreads, smem, stream>>>(a, t);
-    }
+    // the caller's arrays may start on any float: pieces of 8 and 16 bytes where they do so, else single floats
+    const bool any = (((uintptr_t)op->bias | (uintptr_t)op->x | (op->pairwise ? (uintptr_t)op->u : 0)) & (op->pairwise ? 7 : 15)) != 0;
+    void (*const kernel)(b200::FtArgs, b200::TileArgs) =
+        op->pairwise ? (any ? b200::ft_forward_tiled_kernel<true, true> : b200::ft_forward_tiled_kernel<true>)
+                     : (any ? b200::ft_forward_tiled_kernel<false, true> : b200::ft_forward_tiled_kernel<false>);
+    CK(b200::allow_smem(kernel));
+    kernel<<<ctas, b200::kFwdThreads, smem, stream>>>(a, t);
     CK(cudaGetLastError());
     int reported = 0;
     if (!word.status) CK(cudaMemcpyAsync(&reported, status, sizeof reported, cudaMemcpyDeviceToHost, stream));

@@ -85,3 +85,42 @@ def test_op_ft_forward_errors(oracle32):
     assert rc == -5
     lib = _lib.load()
     assert lib.b200_op_ft_forward(0, None, None) == -1
+
+
+@pytest.mark.parametrize("entry", ["b200_op_ft_forward", "b200_op_ft_forward_noalloc"])
+@pytest.mark.parametrize("name,desc,game", CASES, ids=[c[0] for c in CASES])
+@pytest.mark.parametrize("bias_at,x_at,u_at", [(1, 0, 0), (0, 2, 2), (3, 1, 1), (2, 0, 0)])
+def test_op_ft_forward_on_arrays_that_start_on_any_float(oracle32, entry, name, desc, game, bias_at, x_at, u_at):
+    """Bias and outputs of the caller may be slices of larger arrays: bit-exact, and nothing written around them."""
+    import torch
+
+    from bullet_b200 import _lib
+    from bullet_b200.net import pack_indices
+
+    n, dev = 321, torch.device("cuda", 0)
+    stm, nstm, w, table, x_ref = op_inputs(oracle32, desc, game, n, seed=64)
+    t_table = torch.from_numpy(np.ascontiguousarray(table, dtype=np.float32)).to(dev)
+    lists = [torch.from_numpy(pack_indices(a).view(np.int16)).to(dev) for a in (stm, nstm)]
+
+    def holder(count, at):
+        return torch.full((count + 8,), 7.0, device=dev), at, count
+
+    def inside(h):
+        return h[0][h[1]:h[1] + h[2]]
+
+    bias = holder(desc.ft_out, bias_at)
+    inside(bias).copy_(torch.from_numpy(w["l0b"].astype(np.float32)))
+    x = holder(x_ref.size, x_at)
+    u = holder(n * 2 * desc.ft_out, u_at) if desc.pairwise else None
+    op = _lib.CFtOp(desc.n_inputs, desc.nnz, desc.ft_out, desc.ft_act, int(desc.pairwise), desc.ft_block_rows, n, t_table.data_ptr(),
+                    inside(bias).data_ptr(), lists[0].data_ptr(), lists[1].data_ptr(), inside(x).data_ptr(),
+                    inside(u).data_ptr() if u else None)
+    torch.cuda.synchronize()
+    assert getattr(_lib.load(), entry)(0, None, ctypes.byref(op)) == 0
+    torch.cuda.synchronize()
+    assert np.array_equal(inside(x).cpu().numpy().reshape(x_ref.shape), x_ref)
+    if u:
+        half = inside(u).cpu().numpy().reshape(n, 2, 2, desc.ft_out // 2)
+        assert np.array_equal((half[:, :, 0] * half[:, :, 1]).reshape(n, -1), x_ref)
+    for h in (x, u) if u else (x,):
+        assert (h[0][:h[1]] == 7.0).all() and (h[0][h[1] + h[2]:] == 7.0).all()
