@@ -92,6 +92,7 @@ struct TileArgs {
     // 16-byte group is filled with the index of the all-zero row (= block_rows) and never walked
     const uint16_t* lists;  // [2n][list_len]
     int list_len;     // nnz rounded up to a multiple of 8 (16-byte groups)
+    int walk_warps;   // forward: see ft_fwd_warps
     // backward only: the visiting order cut into chunks of at most kChunkMost pairs that never
     // straddle a block, and per chunk the row-major lists built by ft_csr_kernel
     const int4* chunks;            // [nchunks] (block, first index into `pairs`, pairs, 0)
@@ -401,8 +402,17 @@ __device__ __forceinline__ void store_piece(float* p, float4 v) {
 // lane, spent twice the instructions per row and was bound by their issue: 1.69 against 1.55 ms at 131072 positions and
 // width 2048, 0.273 against 0.260 ms at 16384.)
 constexpr int kFwdThreads = 1024;
+// Tables of up to about 900 rows: the tile and two lists for each of 16 warps at least must fit.
+__host__ __device__ inline bool ft_fwd_fits(int R, int list_len) {
+    return (size_t)(R + 1) * kTileRowBytes + (size_t)(kFwdThreads / 32) * list_len * 2 + 16 <= 227 * 1024;
+}
+// Warps that walk lists: all of them, or (the last few rows of that range) as many as have room for two lists beside the tile.
+__host__ __device__ inline int ft_fwd_warps(int R, int list_len) {
+    const int room = (227 * 1024 - 16 - R * kTileRowBytes) / (list_len * 4);
+    return room < kFwdThreads / 32 ? room : kFwdThreads / 32;
+}
 __host__ __device__ inline size_t ft_fwd_smem(int R, int list_len) {
-    return (size_t)R * kTileRowBytes + (size_t)(kFwdThreads / 32) * list_len * 4 + 16;
+    return (size_t)R * kTileRowBytes + (size_t)ft_fwd_warps(R, list_len) * list_len * 4 + 16;
 }
 
 // ANY: bias, x and u start on any float (the operator's caller owns them); else on 8 bytes with the pairwise product, on 16
@@ -412,7 +422,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
     ft_step_begin(a);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    constexpr int NW = kFwdThreads / 32;
+    const int NW = t.walk_warps;
     const int R = t.block_rows, half = lane >> 4, l16 = lane & 15;
     const uint32_t lane16 = 16 * l16;
     float* tile = reinterpret_cast<float*>(smem_raw);
@@ -491,7 +501,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
         float* x_out = a.x + col;
         __syncthreads();
         const int seg_end = t.block_begin[block] + last;
-        int i = t.block_begin[block] + first + 2 * warp;
+        int i = warp < NW ? t.block_begin[block] + first + 2 * warp : seg_end;
         int2 next = make_int2(0, 0);  // this half's next pair and its length
         uint32_t w0 = 0, w1 = 0;      // this lane's words of the next two lists
         auto fetch = [&](int at) {

@@ -549,6 +549,7 @@ b200::TileArgs tile_args(b200_net* net, const Slot& s, bool backward) {
     t.status = s.dev<int>(s.off_status);
     t.lists = s.lists;
     t.list_len = (net->d.nnz + 7) & ~7;
+    t.walk_warps = b200::ft_fwd_warps(net->block_rows, t.list_len);
     t.chunks = s.dev<int4>(s.off_chunks);
     t.csr_ent = s.csr_ent;
     t.csr_start = s.csr_start;
@@ -1007,7 +1008,7 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     const bool promised = d.ft_block_rows > 0 && d.n_inputs % d.ft_block_rows == 0 && d.ft_out % b200::kTileCols == 0;
     const int R = promised ? d.ft_block_rows : d.n_inputs;
     net->tiled_ok = (promised || (d.pairwise ? d.ft_out / 2 : d.ft_out) >= 32) && R < 1024 &&
-                    b200::ft_fwd_smem(R, (d.nnz + 7) & ~7) <= kMaxSmem &&
+                    b200::ft_fwd_fits(R, (d.nnz + 7) & ~7) &&
                     b200::ft_bwd_smem(R, d.nnz, 256) <= kMaxSmem;
     net->tiled_promised = net->tiled_ok && promised;
     net->block_rows = R;

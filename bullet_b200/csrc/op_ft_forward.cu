@@ -123,7 +123,7 @@ int check_op(const b200_ft_op* op, const char* who) {
     if (op->pairwise && op->ft_act != B200_ACT_CRELU) return b200::fail(B200_ERR_UNSUPPORTED, "%s: pairwise needs CReLU", who);
     const int R = op->ft_block_rows;
     if (R < 1 || op->n_inputs % R || op->ft_out < 64 || op->ft_out % b200::kTileCols || op->n_inputs / R > kMaxBlocks ||
-        b200::ft_fwd_smem(R, list_len(op->nnz)) > 227 * 1024)
+        !b200::ft_fwd_fits(R, list_len(op->nnz)))
         return b200::fail(B200_ERR_UNSUPPORTED,
                           "%s: needs ft_block_rows > 0 dividing n_inputs (at most about 800 rows, at most %d blocks) "
                           "and ft_out a multiple of 64",
@@ -195,6 +195,7 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
     t.status = status;
     t.lists = g.lists;
     t.list_len = g.list_len;
+    t.walk_warps = b200::ft_fwd_warps(R, t.list_len);
     const size_t smem = b200::ft_fwd_smem(R, t.list_len);
     // one CTA per SM, each taking an equal piece of the (block, slab, pair) work line
     int sms = 0;

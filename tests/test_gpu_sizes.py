@@ -125,6 +125,35 @@ def test_a_loss_gradient_that_is_not_finite_stays_in_its_rows(oracle32, ft_out, 
     net.close()
 
 
+@pytest.mark.parametrize("nnz", [8, 32, 64])
+@pytest.mark.parametrize("rows_less", [0, 3, 16])
+def test_the_largest_tables_of_the_tiled_kernels(oracle32, nnz, rows_less):
+    """Row blocks up to the largest whose tile fits into shared memory beside two bytes per list slot and warp: the last of them
+    leave room for the lists of some of the warps only.  Network (kernels asked for by name) and operator.  Bounds as above."""
+    import dataclasses
+
+    from tests.test_gpu_ops import run_op
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    rows, n = (227 * 1024 - 16 - 64 * ((nnz + 7) // 8 * 8)) // 256 - 1 - rows_less, 500
+    desc = dataclasses.replace(net_of(2, rows, 128, nnz, 1, (1,)), max_batch=n)
+    stm, nstm, bucket, target = draw_batch(desc, n, seed=nnz)
+    w = rich_weights(desc)
+    x_ref = oracle_x(oracle32, desc, w, stm, nstm)
+    net = make_net(desc, 2, w)
+    net.upload(0, stm, nstm, bucket, target)
+    net.backward(0)
+    assert np.array_equal(net.activation(0, n * desc.dense_in0).reshape(n, -1), x_ref)
+    _, g_ref, _ = oracle32.net_grad(desc, w, stm, nstm, bucket, target)
+    g = net.tensors(kind=3)
+    for k in g_ref:
+        assert np.abs(g[k] - g_ref[k]).max() <= 2e-5 * np.abs(g_ref[k]).max(), k
+    net.close()
+    for entry in ("b200_op_ft_forward", "b200_op_ft_forward_noalloc"):
+        rc, x, _ = run_op(entry, desc, w["l0w"], w["l0b"], stm, nstm, n)
+        assert rc == 0 and np.array_equal(x, x_ref)
+
+
 def net_flat(net, kind):
     import torch
 
