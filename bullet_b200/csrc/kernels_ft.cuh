@@ -884,19 +884,19 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
                 }
             }
         }
-        // the four table columns this lane sums; those past the width (the last slab of one that 64 does not divide) are not
-        // the table's to write, whatever was staged for them: a loss gradient that is not finite makes NaN of their zeros
-        const int in_half = PAIRWISE ? slab * 32 + 4 * (l16 & 7) : slab * 64 + 4 * l16;
-        const int col_w = PAIRWISE && l16 >= 8 ? a.H / 2 + in_half : in_half;
-        const bool col_on = in_half < x_row;
+        // The four table columns this lane sums.  Those past the width (the last slab of one that 64 does not divide) are not
+        // the table's to write: their operands are zero, and zero sums are not written, but with ONE a loss gradient that is
+        // not finite makes NaN of the zeros.  (Asked in the staging instead, or of every network: 2 to 4 % of the kernel.)
+        const int col_w = !PAIRWISE ? slab * 64 + 4 * l16 : l16 < 8 ? slab * 32 + 4 * l16 : a.H / 2 + slab * 32 + 4 * (l16 - 8);
+        const bool col_on = !ONE || (PAIRWISE ? slab * 32 + 4 * (l16 & 7) : col_w) < x_row;
         float* g_block = a.g_table + (size_t)block * R * a.H + col_w;
         if (threadIdx.x >= kBwdThreads - kTileCols) {
             const int j = (int)threadIdx.x - (kBwdThreads - kTileCols);
             float sum = 0.f;
 #pragma unroll 8
             for (int w = 0; w < NW; w++) sum += bias_s[w * kTileCols + j];
-            const int c = PAIRWISE ? slab * 32 + (j & 31) : slab * 64 + j;
-            if (c < x_row && sum != 0.f) atomicAdd(a.g_bias + (PAIRWISE && j >= 32 ? a.H / 2 + c : c), sum);
+            const bool on = !ONE || (PAIRWISE ? slab * 32 + (j & 31) : slab * 64 + j) < x_row;
+            if (on && sum != 0.f) atomicAdd(a.g_bias + (!PAIRWISE ? slab * 64 + j : j < 32 ? slab * 32 + j : a.H / 2 + slab * 32 + j - 32), sum);
         }
         const int pieces = start[1];
         auto walk = [&](unsigned piece) {
