@@ -31,10 +31,10 @@ struct DenseArgs {
     const float* W[3];
     const float* B[3];
     const float* W1g;  // first-layer weights regrouped as [bucket][column][row] (fewer than four rows)
-    const float4* W1f; // ... or as the fragment tables of kernels_dense_mma.cuh
-    const float4* W1d;
+    const uint32_t* W1f; // ... or as the fragment tables of kernels_dense_mma.cuh
+    const uint32_t* W1d;
     float* partial;    // [part][tile][32][M1] sums of slices of the first layer's columns
-    float* dz_frag;    // dz[0] as the tensor pipe's operand of the weight gradient (dense_small_mma_kernel)
+    uint32_t* dz_frag; // dz[0] as the tensor pipe's operand of the weight gradient (dense_small_mma_kernel)
     float* a1;         // [n][M1] activated layer-1 output (kept for the weight gradients)
     float* a2;         // [n][M2]
     float* dz[3];      // gradient at each layer's selected pre-activation: [n][M_i]

@@ -6,13 +6,20 @@
 // (they held the kernels at a third of the copy rate); mma.sync does at a few per cent of its own rate, straight from
 // registers, without the staging through shared memory and tensor memory that tcgen05 would add for a 16-wide product.
 //
-// fp32 operands are split into two TF32 parts, each rounded to nearest: hi keeps 11 bits and lo the next 11, so that hi + lo
-// is within 2^-24 of the value; of the four products lo * lo (2^-24 and less of the result) is left out.  A few steps
-// accumulate in the tensor pipe, then their sum is added to the running total with an ordinary fp32 add.
+// An fp32 operand is split into three bf16 parts, each rounded to nearest: v = h + m + l exactly (8 bits each, short of
+// numbers whose last bits lie below 2^-133).  Of the nine products three are left out, m l, l m and l l, which together are
+// within 2^-25 of the product: less than one rounding of an fp32 product.  The products of the high parts have an accumulator
+// of their own, the five small ones share another, both start from zero for every 16 columns (rows, positions), and ordinary
+// fp32 adds take them to the running total: what the tensor pipe cuts off a sum it accumulates stays small.  2-norm error
+// against 64 bits, 16384 positions of 2048 -> (16, 32, 1), gradient at x / of the weights: 2.76e-7 / 2.63e-7 with two TF32 parts
+// and three products in one accumulator, 2.11e-7 / 2.29e-7 with fp32 multiply-adds, 1.63e-7 / 1.86e-7 here.
+// A NaN stays a NaN in the high part; an infinity becomes one (its remainder is infinity - infinity).
 //
-// Fragments of mma.m16n8k8 (lane = 4 g + t): A (16 x 8) a0 (g, t) a1 (g + 8, t) a2 (g, t + 4) a3 (g + 8, t + 4); B (8 x 8)
-// b0 (t, g) b1 (t + 4, g); C (16 x 8) c0 (g, 2 t) c1 (g, 2 t + 1) c2 (g + 8, 2 t) c3 (g + 8, 2 t + 1).  Which column of x an
-// index of a fragment stands for is free, and chosen so that a lane always moves four neighbouring columns.
+// Fragments of mma.m16n8k16 (lane = 4 g + t), two bf16 per register, the first in the low half: A (16 x 16) a0 (g, 2 t + {0, 1})
+// a1 (g + 8, 2 t + {0, 1}) a2 (g, 2 t + 8 + {0, 1}) a3 (g + 8, 2 t + 8 + {0, 1}); B (16 x 8) b0 (2 t + {0, 1}, g)
+// b1 (2 t + 8 + {0, 1}, g); C (16 x 8) c0 (g, 2 t) c1 (g, 2 t + 1) c2 (g + 8, 2 t) c3 (g + 8, 2 t + 1).  m16n8k8 has a0, a1
+// and b0 only.  Which column of x an index of a fragment stands for is free, and chosen so that a lane always moves four
+// neighbouring columns.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -22,53 +29,104 @@
 
 namespace b200 {
 
-// The tensor pipe reads the upper 19 bits of a TF32 operand, so adding half of the last of them rounds to nearest, ties away
-// (cvt.rna.tf32 is several instructions more; it also keeps infinities, which become NaN here: a pass that met one is lost
-// either way).
-__device__ __forceinline__ void tf32_split(float v, uint32_t& hi, uint32_t& lo) {
-    hi = __float_as_uint(v) + 0x1000u;
-    lo = __float_as_uint(v - __uint_as_float(hi & 0xffffe000u)) + 0x1000u;
+// Two values into their parts: each register holds the part of `a` in its low half, of `b` in its high half.
+__device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(b), "f"(a));
+    return r;
 }
-__device__ __forceinline__ void mma_tf32(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+__device__ __forceinline__ float bf16_lo(uint32_t pair) { return __uint_as_float(pair << 16); }
+__device__ __forceinline__ float bf16_hi(uint32_t pair) { return __uint_as_float(pair & 0xffff0000u); }
+struct Split {
+    uint32_t h, m, l;
+};
+__device__ __forceinline__ Split bf16_split(float a, float b) {
+    Split s;
+    s.h = bf16_pair(a, b);
+    a -= bf16_lo(s.h), b -= bf16_hi(s.h);
+    s.m = bf16_pair(a, b);
+    s.l = bf16_pair(a - bf16_lo(s.m), b - bf16_hi(s.m));
+    return s;
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
         : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[2], const uint32_t (&b)[1]) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, {%0, %1, %2, %3};"
+        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+        : "r"(a[0]), "r"(a[1]), "r"(b[0]));
+}
+// total += A B, both in parts [high, middle, low]
+template <int NA, int NB>
+__device__ __forceinline__ void mma_split(float (&total)[4], const uint32_t (&a)[3][NA], const uint32_t (&b)[3][NB]) {
+    float high[4] = {0.f, 0.f, 0.f, 0.f}, rest[4] = {0.f, 0.f, 0.f, 0.f};
+    mma_bf16(high, a[0], b[0]);
+    mma_bf16(rest, a[1], b[1]);
+    mma_bf16(rest, a[0], b[2]);
+    mma_bf16(rest, a[2], b[0]);
+    mma_bf16(rest, a[0], b[1]);
+    mma_bf16(rest, a[1], b[0]);
+#pragma unroll
+    for (int e = 0; e < 4; e++) total[e] += high[e] + rest[e];
 }
 
 constexpr int kMmaCols = 16;  // columns of x in one group of the forward and of dx
 template <int M1>
 __host__ __device__ constexpr int mma_tiles() { return M1 >= 8 ? M1 / 8 : 1; }  // 8-row tiles (a layer of four rows fills half of one)
-// floats of one fragment table: [bucket][16-column group][8-row tile][hi, lo][lane] float4
-__host__ __device__ inline size_t mma_table_floats(int K1, int O, int M1) {
-    return (size_t)O * ((K1 + kMmaCols - 1) / kMmaCols) * (M1 >= 8 ? M1 / 8 : 1) * 2 * 32 * 4;
+constexpr int kTileWords = 32 * 6;  // 32-bit words of 16 columns of an 8-row tile, three parts
+// rows that the gradient at x contracts in one step
+__host__ __device__ constexpr int dx_rows(int M1) { return M1 >= 16 ? 16 : 8; }
+// Words of one fragment table.  Forward, B with (k = column, n = row): [bucket][16-column group][8-row tile], of each lane
+// (h0, h1, m0, m1), then of each (l0, l1); its columns are 16 group + 4 t + 0..3 in the order of the pairs, its row is
+// 8 tile + g.  Gradient at x, B with (k = row, n = column): [bucket][group][step of dx_rows][part], of each lane the registers
+// of columns j = 0, 1: column 16 group + 4 (g / 2) + 2 j + g % 2, rows of the step 4 t + 0..3 in the order of the pairs (16 a
+// step) or 2 t + 0, 1 (8 a step).
+__host__ __device__ inline size_t mma_table_words(int K1, int O, int M1) {
+    return (size_t)O * ((K1 + kMmaCols - 1) / kMmaCols) * (M1 >= 8 ? M1 / 8 : 1) * kTileWords;
+}
+__device__ __forceinline__ uint32_t split_part(const Split& s, int part) { return part == 0 ? s.h : part == 1 ? s.m : s.l; }
+
+// Weights of one column and four neighbouring rows (k, row .. row + 3) into both tables.
+__device__ __forceinline__ void store_fragments(uint32_t* fwd, uint32_t* dxt, int K1, int M1, int k, int col, int row, float4 w) {
+    const int groups = (K1 + kMmaCols - 1) / kMmaCols, tiles = M1 >= 8 ? M1 / 8 : 1, c = col & 15;
+    const size_t at = ((size_t)k * groups + (col >> 4)) * tiles * kTileWords;
+    const Split a = bf16_split(w.x, w.y), b = bf16_split(w.z, w.w);
+    uint16_t* f = reinterpret_cast<uint16_t*>(fwd + at + (row >> 3) * kTileWords);
+    const int t = c >> 2, pair = (c & 3) >> 1, half = c & 1;
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const int lane = 4 * ((row + i) & 7) + t;
+        const Split& s = i < 2 ? a : b;
+        f[(lane * 4 + pair) * 2 + half] = (uint16_t)(i & 1 ? s.h >> 16 : s.h);
+        f[(lane * 4 + 2 + pair) * 2 + half] = (uint16_t)(i & 1 ? s.m >> 16 : s.m);
+        f[(128 + lane * 2 + pair) * 2 + half] = (uint16_t)(i & 1 ? s.l >> 16 : s.l);
+    }
+    const int g = 2 * (c >> 2) + (c & 1), j = (c & 3) >> 1;
+#pragma unroll
+    for (int part = 0; part < 3; part++) {
+        const uint32_t lo = split_part(a, part), hi = split_part(b, part);
+        if (M1 >= 16) {
+            uint32_t* d = dxt + at + (row >> 4) * 2 * kTileWords + part * 128 + (4 * g + ((row & 15) >> 2)) * 4 + 2 * j;
+            *reinterpret_cast<uint2*>(d) = make_uint2(lo, hi);
+        } else {
+            uint32_t* d = dxt + at + part * 64 + (4 * g + (row >> 1)) * 2 + j;
+            d[0] = lo, d[2] = hi;
+        }
+    }
 }
 
-// Rebuilds both fragment tables from l1w [column][bucket][row] after every update.  `fwd`: B of the forward, (k = column,
-// n = row): element (s, i) of a lane's float4 is column 16 grp + 4 t + 2 s + i, row 8 tile + g.  `dxt`: B of dx, (k = row,
-// n = column): element (j, i) is column 16 grp + 4 (g / 2) + 2 j + g % 2, row 8 tile + t + 4 i.
-static __global__ void __launch_bounds__(256) dense_fragments_kernel(const float* __restrict__ W1, float4* __restrict__ fwd, float4* __restrict__ dxt,
-                                                                    int K1, int O, int M1, int tiles) {
-    const int groups = (K1 + kMmaCols - 1) / kMmaCols, total = O * groups * tiles * 32;
+// Rebuilds both fragment tables from l1w [column][bucket][row]: a thread per column and four rows, those past the last
+// (a layer of four rows fills half a tile, the last group of columns may be short) as zeros.
+static __global__ void __launch_bounds__(256) dense_fragments_kernel(const float* __restrict__ W1, uint32_t* __restrict__ fwd, uint32_t* __restrict__ dxt,
+                                                                    int K1, int O, int M1) {
+    const int cols = (K1 + kMmaCols - 1) / kMmaCols * kMmaCols, quads = M1 >= 8 ? M1 / 4 : 2, total = O * cols * quads;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
-        const int lane = i & 31, tile = (i >> 5) % tiles, grp = (i >> 5) / tiles % groups, k = (i >> 5) / (tiles * groups);
-        const int g = lane >> 2, t = lane & 3;
-        auto at = [&](int col, int row) { return col < K1 && row < M1 ? W1[(size_t)col * (O * M1) + k * M1 + row] : 0.f; };
-        float f[4], d[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            f[e] = at(16 * grp + 4 * t + e, 8 * tile + g);
-            d[e] = at(16 * grp + 4 * (g >> 1) + 2 * (e >> 1) + (g & 1), 8 * tile + t + 4 * (e & 1));
-        }
-        uint32_t hi[4], lo[4];
-        const size_t out = (size_t)((i >> 5) * 2) * 32 + lane;
-#pragma unroll
-        for (int e = 0; e < 4; e++) tf32_split(f[e], hi[e], lo[e]);
-        fwd[out] = make_float4(__uint_as_float(hi[0]), __uint_as_float(hi[1]), __uint_as_float(hi[2]), __uint_as_float(hi[3]));
-        fwd[out + 32] = make_float4(__uint_as_float(lo[0]), __uint_as_float(lo[1]), __uint_as_float(lo[2]), __uint_as_float(lo[3]));
-#pragma unroll
-        for (int e = 0; e < 4; e++) tf32_split(d[e], hi[e], lo[e]);
-        dxt[out] = make_float4(__uint_as_float(hi[0]), __uint_as_float(hi[1]), __uint_as_float(hi[2]), __uint_as_float(hi[3]));
-        dxt[out + 32] = make_float4(__uint_as_float(lo[0]), __uint_as_float(lo[1]), __uint_as_float(lo[2]), __uint_as_float(lo[3]));
+        const int row = i % quads * 4, col = i / quads % cols, k = i / (quads * cols);
+        const bool in = row < M1 && col < K1;
+        const float4 w = in ? *reinterpret_cast<const float4*>(W1 + (size_t)col * (O * M1) + k * M1 + row) : make_float4(0, 0, 0, 0);
+        store_fragments(fwd, dxt, K1, M1, k, col, row, w);
     }
 }
 
@@ -128,13 +186,14 @@ __device__ __forceinline__ void copy16_async(void* smem_dst, const void* src) {
 // ends, so that no warp waits for another; the look-ups (range, positions, bucket) run a tile ahead of the copies.
 // With few tiles `split` warps share a slice of one.  The layers behind, and the sum of the parts, have a kernel of their own:
 // they keep a CTA's loads from flowing, and the weights read from L2 for every tile (as much as x) cost 75 us at 131072.
-// At 131072 positions (K1 = 2048, M1 = 16) 0.400 ms for both kernels' work in one, a CTA per tile with x loaded into registers
-// -> 0.245 + 0.037 against 0.165 for reading x at the copy rate; 0.060 -> 0.053 at 16384.
+// At 131072 positions (K1 = 2048, M1 = 16) 0.400 ms for both kernels' work in one, a CTA per tile with x loaded into registers;
+// now 0.249 + 0.060 from a cold cache, 0.337 for both in a step (this kernel with two TF32 parts: 0.228), against 0.165 for
+// reading x at the copy rate; at 16384 0.060.
 // grid = (slices, runs), block = 256, dynamic shared memory = dense_mma_smem<M1>().
 constexpr int kSliceCols = 256, kFwdDepth = 5, kFwdAhead = 8;
 template <int M1>
 __host__ __device__ constexpr size_t dense_mma_smem() {
-    return ((size_t)kFwdDepth * 4 * 256 + (size_t)kSliceCols / kMmaCols * mma_tiles<M1>() * 64) * sizeof(float4);
+    return ((size_t)kFwdDepth * 4 * 256 * sizeof(float4) + (size_t)kSliceCols / kMmaCols * mma_tiles<M1>() * kTileWords * 4);
 }
 
 template <int M1>
@@ -149,7 +208,7 @@ __global__ void __launch_bounds__(256, dense_mma_ctas(M1)) dense_first_mma_kerne
     // units = tiles x split; a CTA's run of them is dealt to its warps in turn
     const int run0 = (int)((long long)a.ntiles * split * blockIdx.y / gridDim.y), run1 = (int)((long long)a.ntiles * split * (blockIdx.y + 1) / gridDim.y);
     float4* ring = reinterpret_cast<float4*>(dense_smem) + threadIdx.x;
-    float4* s_w = reinterpret_cast<float4*>(dense_smem) + kFwdDepth * 4 * 256;
+    uint32_t* s_w = reinterpret_cast<uint32_t*>(dense_smem) + kFwdDepth * 4 * 256 * 4;
 
     // The copies' side: rows and range of the unit being copied, positions of the next one, range of the one after that.
     auto range = [&](int unit) { return unit < run1 ? dense_tile_at(a.tiles, unit / split, a.n) : make_int2(0, 0); };
@@ -197,8 +256,8 @@ __global__ void __launch_bounds__(256, dense_mma_ctas(M1)) dense_first_mma_kerne
     int2 range2 = range(run0 + 16);
     int held = -1, stage = 0;  // the bucket whose fragments are in shared memory
     auto hold = [&](int bucket) {
-        const float4* table = a.W1f + ((size_t)bucket * groups + slice * kGroups) * NT * 64;
-        for (int i = threadIdx.x; i < slice_groups * NT * 64; i += 256) s_w[i] = __ldg(table + i);
+        const uint4* table = reinterpret_cast<const uint4*>(a.W1f + ((size_t)bucket * groups + slice * kGroups) * NT * kTileWords);
+        for (int i = threadIdx.x; i < slice_groups * NT * (kTileWords / 4); i += 256) reinterpret_cast<uint4*>(s_w)[i] = __ldg(table + i);
         held = bucket;
     };
     if (bucket0 >= 0) hold(bucket0);
@@ -222,7 +281,7 @@ __global__ void __launch_bounds__(256, dense_mma_ctas(M1)) dense_first_mma_kerne
         if (at.y <= 0) continue;
         const int first = unit % split * per_unit, last = min(first + per_unit, slice_groups);
         // (a tile of the next bucket that shares a round with tiles of this one reads the fragments where they are)
-        const float4* table = (at.z == held ? s_w : a.W1f + ((size_t)at.z * groups + slice * kGroups) * NT * 64) + lane;
+        const uint32_t* table = at.z == held ? s_w : a.W1f + ((size_t)at.z * groups + slice * kGroups) * NT * kTileWords;
         float acc[2][NT][4];
 #pragma unroll
         for (int m = 0; m < 2; m++)
@@ -234,49 +293,31 @@ __global__ void __launch_bounds__(256, dense_mma_ctas(M1)) dense_first_mma_kerne
         for (int group = first; group < last; group++) {
             asm volatile("cp.async.wait_group %0;" ::"n"(kFwdDepth - 2) : "memory");
             const bool in = slice * kSliceCols + group * kMmaCols + 4 * t4 < a.K1;
-            float xs[4][4];
-            float4 wv[NT][2];
+            float4 xs[4];
+            uint32_t w[NT][3][2];
 #pragma unroll
-            for (int r = 0; r < 4; r++) {
-                const float4 v = in ? ring[(stage * 4 + r) * 256] : make_float4(0, 0, 0, 0);
-                xs[r][0] = v.x, xs[r][1] = v.y, xs[r][2] = v.z, xs[r][3] = v.w;
+            for (int r = 0; r < 4; r++) xs[r] = in ? ring[(stage * 4 + r) * 256] : make_float4(0, 0, 0, 0);
+#pragma unroll
+            for (int nt = 0; nt < NT; nt++) {
+                const uint32_t* tile = table + (group * NT + nt) * kTileWords;
+                const uint4 hm = *reinterpret_cast<const uint4*>(tile + 4 * lane);
+                const uint2 l = *reinterpret_cast<const uint2*>(tile + 128 + 2 * lane);
+                w[nt][0][0] = hm.x, w[nt][0][1] = hm.y, w[nt][1][0] = hm.z, w[nt][1][1] = hm.w, w[nt][2][0] = l.x, w[nt][2][1] = l.y;
             }
-#pragma unroll
-            for (int nt = 0; nt < NT; nt++)
-#pragma unroll
-                for (int part = 0; part < 2; part++) wv[nt][part] = table[(group * NT + nt) * 64 + 32 * part];
             stage = stage + 1 < kFwdDepth ? stage + 1 : 0;
             copy();
-            float part_sum[2][NT][4];
 #pragma unroll
-            for (int m = 0; m < 2; m++)
+            for (int m = 0; m < 2; m++) {
+                uint32_t xp[3][4];
 #pragma unroll
-                for (int nt = 0; nt < NT; nt++)
-#pragma unroll
-                    for (int e = 0; e < 4; e++) part_sum[m][nt][e] = 0.f;
-#pragma unroll
-            for (int s = 0; s < 2; s++)
-#pragma unroll
-                for (int m = 0; m < 2; m++) {
-                    uint32_t hi[4], lo[4];
-#pragma unroll
-                    for (int e = 0; e < 4; e++) tf32_split(xs[2 * m + (e & 1)][2 * s + (e >> 1)], hi[e], lo[e]);
-#pragma unroll
-                    for (int nt = 0; nt < NT; nt++) {
-                        const float4 wh = wv[nt][0], wl = wv[nt][1];
-                        const uint32_t h0 = __float_as_uint(s ? wh.z : wh.x), h1 = __float_as_uint(s ? wh.w : wh.y);
-                        const uint32_t l0 = __float_as_uint(s ? wl.z : wl.x), l1 = __float_as_uint(s ? wl.w : wl.y);
-                        mma_tf32(part_sum[m][nt], lo, h0, h1);
-                        mma_tf32(part_sum[m][nt], hi, l0, l1);
-                        mma_tf32(part_sum[m][nt], hi, h0, h1);
-                    }
+                for (int e = 0; e < 4; e++) {  // rows g and g + 8 of the half, first and second pair of columns
+                    const float4 v = xs[2 * m + (e & 1)];
+                    const Split s = e < 2 ? bf16_split(v.x, v.y) : bf16_split(v.z, v.w);
+                    xp[0][e] = s.h, xp[1][e] = s.m, xp[2][e] = s.l;
                 }
 #pragma unroll
-            for (int m = 0; m < 2; m++)
-#pragma unroll
-                for (int nt = 0; nt < NT; nt++)
-#pragma unroll
-                    for (int e = 0; e < 4; e++) acc[m][nt][e] += part_sum[m][nt][e];
+                for (int nt = 0; nt < NT; nt++) mma_split(acc[m][nt], xp, w[nt]);
+            }
         }
         float* partial = a.partial + ((size_t)(slice * split + unit % split) * a.ntiles + unit / split) * kDenseTile * M1;
 #pragma unroll
@@ -292,9 +333,11 @@ __global__ void __launch_bounds__(256, dense_mma_ctas(M1)) dense_first_mma_kerne
     asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-// floats before step `i` (eight places of a tile) of the weight gradient's operand: [step][16-row tile][hi, lo][lane] float4
+// words before step `i` (16 places of a tile) of the weight gradient's operand: [step][16-row tile][part][lane] uint4, rows r = 16
+// tile + g (+ 8), places of the step 2 t + {0, 1} (+ 8)
+constexpr int kWgradStep = 16;
 template <int M1>
-__host__ __device__ constexpr size_t wgrad_table_floats(size_t i) { return i * (M1 > 16 ? M1 / 16 : 1) * 256; }
+__host__ __device__ constexpr size_t wgrad_table_words(size_t i) { return i * (M1 > 16 ? M1 / 16 : 1) * 384; }
 
 // The rest of the forward: sum of the first layer's parts, small layers, loss, the way back to the first layer's
 // pre-activation gradient (also as the operand of its weight gradient), weight gradients of the small layers and the first
@@ -482,11 +525,14 @@ __global__ void __launch_bounds__(kSmallThreads, M1 > 16 ? 2 : 4) dense_small_mm
             const float d = on ? mine[i] * act_bwd(a.act[0], s_a1[warp][p][r]) : 0.f;
             if (on) a.dz[0][(size_t)pos * M1 + r] = d;
             own1[i] += d;
-            // A of the weight gradient, step `warp` of the tile: lane 4 (r % 8) + p % 4, element (r / 8 % 2) + 2 (p / 4)
-            uint32_t hi, lo;
-            tf32_split(d, hi, lo);
-            float* at = a.dz_frag + wgrad_table_floats<M1>((size_t)tile * 4 + warp) + (r >> 4) * 256 + (4 * (r & 7) + (p & 3)) * 4 + (r >> 3 & 1) + 2 * (p >> 2);
-            at[0] = __uint_as_float(hi), at[128] = __uint_as_float(lo);
+            // A of the weight gradient: the lane of an even place stores its own and its neighbour's
+            const float next = __shfl_xor_sync(0xffffffffu, d, 4);
+            if (!(p & 1)) {
+                const Split pair = bf16_split(d, next);
+                const int q = at & (kWgradStep - 1);
+                uint32_t* out = a.dz_frag + wgrad_table_words<M1>((size_t)tile * 2 + (at >> 4)) + (r >> 4) * 384 + (4 * (r & 7) + ((q & 7) >> 1)) * 4 + (r >> 3 & 1) + 2 * (q >> 3);
+                out[0] = pair.h, out[128] = pair.m, out[256] = pair.l;
+            }
         }
         __syncwarp();
 #pragma unroll 4
@@ -517,65 +563,77 @@ __global__ void __launch_bounds__(kSmallThreads, M1 > 16 ? 2 : 4) dense_small_mm
 // dx[b][c] = sum_r W1[c][k_b][r] * dz1[b][r]   (Matmul::backward, matmul.rs:99-126, on the selected rows).  Same tiles; a
 // warp keeps the split gradients of all 32 positions in registers and walks the 16-column groups, storing four neighbouring
 // columns per lane and row.  With fp32 multiply-adds this and the weight
-// gradient took 0.681 ms at 131072 positions, K1 = 2048, M1 = 16; now 0.239 here (0.165 for writing dx at the copy rate).
+// gradient took 0.681 ms at 131072 positions, K1 = 2048, M1 = 16; now 0.229 here (0.165 for writing dx at the copy rate).
 // grid = ntiles, block = 256.
 template <int M1>
 __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_dx_mma_kernel(DenseArgs a, float* dx) {
     step_begin(a.stamp);
-    constexpr int NT = mma_tiles<M1>();
+    constexpr int S = M1 >= 16 ? M1 / 16 : 1, NA = M1 >= 16 ? 4 : 2, NB = NA / 2;  // steps; registers of a part of A and of one column tile of B
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t4 = lane & 3;
     const int2 t = dense_tile_at(a.tiles, blockIdx.x, a.n);
     if (t.y <= 0) return;
     const int groups = (a.K1 + kMmaCols - 1) / kMmaCols;
     float* row[4];
-    uint32_t hi[2][NT][4], lo[2][NT][4];
+    uint32_t dz[2][S][3][NA];
     int k = 0;
 #pragma unroll
     for (int r = 0; r < 4; r++) {
         const int pos = dense_order_at(a.order, t.x + min(g + 8 * r, t.y - 1));
         if (r == 0) k = a.buckets[pos];
         row[r] = dx + (size_t)pos * a.K1 + 4 * t4;
+        const float* own = a.dz[0] + (size_t)pos * M1;
 #pragma unroll
-        for (int nt = 0; nt < NT; nt++)
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const int rr = 8 * nt + t4 + 4 * i;
-                const float v = rr < M1 ? a.dz[0][(size_t)pos * M1 + rr] : 0.f;
-                tf32_split(v, hi[r >> 1][nt][(r & 1) + 2 * i], lo[r >> 1][nt][(r & 1) + 2 * i]);
+        for (int s = 0; s < S; s++) {
+            auto put = [&](int e, Split v) { dz[r >> 1][s][0][e] = v.h, dz[r >> 1][s][1][e] = v.m, dz[r >> 1][s][2][e] = v.l; };
+            if constexpr (NA == 4) {
+                const float4 v = *reinterpret_cast<const float4*>(own + 16 * s + 4 * t4);
+                put(r & 1, bf16_split(v.x, v.y));
+                put((r & 1) + 2, bf16_split(v.z, v.w));
+            } else {
+                float2 v = make_float2(0.f, 0.f);
+                if (2 * t4 < M1) v = *reinterpret_cast<const float2*>(own + 2 * t4);
+                put(r & 1, bf16_split(v.x, v.y));
             }
+        }
     }
-    const float4* table = a.W1d + (size_t)k * groups * NT * 64 + lane;
-    float4 wv[NT][2];
+    const uint32_t* table = a.W1d + (size_t)k * groups * S * (NB * kTileWords) + lane * 2 * NB;
+    uint32_t ahead[S][3][2 * NB];  // [step][part][column tile, register]
     auto fetch = [&](int grp) {
         if (grp < groups)
 #pragma unroll
-            for (int nt = 0; nt < NT; nt++)
+            for (int s = 0; s < S; s++)
 #pragma unroll
-                for (int part = 0; part < 2; part++) wv[nt][part] = __ldg(table + (size_t)(grp * NT + nt) * 64 + 32 * part);
+                for (int part = 0; part < 3; part++) {
+                    const uint32_t* src = table + (size_t)(grp * S + s) * (NB * kTileWords) + part * 64 * NB;
+                    if constexpr (NB == 2) {
+                        const uint4 v = __ldg(reinterpret_cast<const uint4*>(src));
+                        ahead[s][part][0] = v.x, ahead[s][part][1] = v.y, ahead[s][part][2] = v.z, ahead[s][part][3] = v.w;
+                    } else {
+                        const uint2 v = __ldg(reinterpret_cast<const uint2*>(src));
+                        ahead[s][part][0] = v.x, ahead[s][part][1] = v.y;
+                    }
+                }
     };
     fetch(warp);
     for (int grp = warp; grp < groups; grp += 8) {
-        uint32_t b[NT][2][4];
+        uint32_t b[S][2][3][NB];
 #pragma unroll
-        for (int nt = 0; nt < NT; nt++)
+        for (int s = 0; s < S; s++)
 #pragma unroll
-            for (int part = 0; part < 2; part++) {
-                b[nt][part][0] = __float_as_uint(wv[nt][part].x), b[nt][part][1] = __float_as_uint(wv[nt][part].y);
-                b[nt][part][2] = __float_as_uint(wv[nt][part].z), b[nt][part][3] = __float_as_uint(wv[nt][part].w);
-            }
+            for (int j = 0; j < 2; j++)
+#pragma unroll
+                for (int part = 0; part < 3; part++)
+#pragma unroll
+                    for (int e = 0; e < NB; e++) b[s][j][part][e] = ahead[s][part][NB * j + e];
         fetch(grp + 8);
         const bool in = grp * kMmaCols + 4 * t4 < a.K1;
 #pragma unroll
         for (int m = 0; m < 2; m++) {
             float c[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
-            for (int nt = 0; nt < NT; nt++)
+            for (int s = 0; s < S; s++)
 #pragma unroll
-                for (int j = 0; j < 2; j++) {
-                    mma_tf32(c[j], lo[m][nt], b[nt][0][2 * j], b[nt][0][2 * j + 1]);
-                    mma_tf32(c[j], hi[m][nt], b[nt][1][2 * j], b[nt][1][2 * j + 1]);
-                    mma_tf32(c[j], hi[m][nt], b[nt][0][2 * j], b[nt][0][2 * j + 1]);
-                }
+                for (int j = 0; j < 2; j++) mma_split(c[j], dz[m][s], b[s][j]);
 #pragma unroll
             for (int h = 0; h < 2; h++)
                 if (in && 16 * m + 8 * h + g < t.y)
@@ -584,25 +642,27 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_dx_mma_kernel(De
     }
 }
 
-// Weight gradient of the first layer: gW[c][k][r] += sum_b [k_b == k] dz1[b][r] * x[b][c].  Positions contract, eight
-// a step; r is the M of the product and columns its N: a lane takes four neighbouring columns of two positions, and value j
+// Weight gradient of the first layer: gW[c][k][r] += sum_b [k_b == k] dz1[b][r] * x[b][c].  Positions contract, sixteen
+// a step; r is the M of the product and columns its N: a lane takes four neighbouring columns of four positions, and value j
 // of each belongs to column tile j.  A warp owns 64 columns (two groups of 32), the eight of a CTA 512; the CTA walks a
-// run of dense tiles, of which a ninth warp copies eight rows of x and their dz1 (fragments that the small layers' kernel has
+// run of dense tiles, of which a ninth warp copies sixteen rows of x and their dz1 (fragments that the small layers' kernel has
 // written in the order of the tiles) at a time into a ring of stages, and adds its sums to the gradient when the output bucket
 // changes.  (x loaded into registers and dz1 split through shared memory a tile at a time, with two barriers: 0.365 ms at
-// 131072 positions, K1 = 2048, M1 = 16; lanes copying their own pieces by cp.async, as the forward does: 0.370; this: 0.235,
-// against 0.165 for reading x at the copy rate.  A bulk copy costs the warp that issues it 70 to 100 clocks, so it should be long.)
+// 131072 positions, K1 = 2048, M1 = 16; lanes copying their own pieces by cp.async, as the forward does: 0.370; this: 0.244
+// from a cold cache (0.240 with two TF32 parts and eight positions a step), against 0.165 for reading x at the copy rate.  A
+// bulk copy costs the warp that issues it 70 to 100 clocks, so it should be long.)
 // grid = (ceil(K1 / 512), runs), block = 288, dynamic shared memory = wgrad_smem<M1>().
 constexpr int kRingThreads = 288;
-constexpr int kWgradCols = 64, kWgradStages = 5, kWgradPitch = 8 * kWgradCols + 8;
+constexpr int kWgradCols = 64, kWgradStages = 3;
+constexpr int kWgradPitch = 8 * kWgradCols + 4;  // (rows 2 t of a step, four banks and eight apart: no two lanes of a load in one bank)
 template <int M1>
-__host__ __device__ constexpr int wgrad_stage_floats() { return 8 * kWgradPitch + (int)wgrad_table_floats<M1>(1); }
+__host__ __device__ constexpr int wgrad_stage_floats() { return kWgradStep * kWgradPitch + (int)wgrad_table_words<M1>(1); }
 template <int M1>
 __host__ __device__ constexpr size_t wgrad_smem() { return (size_t)kWgradStages * wgrad_stage_floats<M1>() * sizeof(float); }
 
 template <int M1>
 __global__ void __launch_bounds__(kRingThreads, dense_mma_ctas(M1)) dense_wgrad_mma_kernel(const __grid_constant__ DenseArgs a, float* gW) {
-    constexpr int MT = M1 > 16 ? M1 / 16 : 1, kTable = (int)wgrad_table_floats<M1>(1);
+    constexpr int MT = M1 > 16 ? M1 / 16 : 1, kTable = (int)wgrad_table_words<M1>(1);
     extern __shared__ __align__(16) float wgrad_smem_raw[];
     __shared__ Ring<kWgradStages> ring;
     __shared__ int s_rows[kWgradStages], s_bucket[kWgradStages];
@@ -618,8 +678,8 @@ __global__ void __launch_bounds__(kRingThreads, dense_mma_ctas(M1)) dense_wgrad_
         const uint32_t bytes = (uint32_t)min(8 * kWgradCols, a.K1 - cta_col) * 4;
         for (int tile = first;; tile++) {
             const TileAhead now = lookup.next(tile);
-            for (int p = 0; p < max(1, now.t.y); p += 8) {
-                const int rows = max(0, min(8, now.t.y - p)), pos = __shfl_sync(0xffffffffu, now.pos, (p + lane) & 31);
+            for (int p = 0; p < max(1, now.t.y); p += kWgradStep) {
+                const int rows = max(0, min(kWgradStep, now.t.y - p)), pos = __shfl_sync(0xffffffffu, now.pos, (p + lane) & 31);
                 if (!mbar_wait(&ring.empty[at.slot], at.phase ^ 1)) return;
                 __syncwarp();
                 float* stage = wgrad_smem_raw + (size_t)at.slot * wgrad_stage_floats<M1>();
@@ -630,8 +690,8 @@ __global__ void __launch_bounds__(kRingThreads, dense_mma_ctas(M1)) dense_wgrad_
                 }
                 __syncwarp();
                 if (lane < rows) bulk_load(stage + lane * kWgradPitch, a.x + (size_t)pos * a.K1 + cta_col, bytes, &ring.full[at.slot]);
-                if (lane == 8 && rows)
-                    bulk_load(stage + 8 * kWgradPitch, a.dz_frag + wgrad_table_floats<M1>((size_t)tile * 4 + (p >> 3)), kTable * 4, &ring.full[at.slot]);
+                if (lane == kWgradStep && rows)
+                    bulk_load(stage + kWgradStep * kWgradPitch, a.dz_frag + wgrad_table_words<M1>((size_t)tile * 2 + p / kWgradStep), kTable * 4, &ring.full[at.slot]);
                 at.advance();
             }
             if (now.t.y <= 0) return;  // (the readers stop at a stage without rows)
@@ -676,41 +736,34 @@ __global__ void __launch_bounds__(kRingThreads, dense_mma_ctas(M1)) dense_wgrad_
             cur = k;
         }
         const float* stage = wgrad_smem_raw + (size_t)at.slot * wgrad_stage_floats<M1>();
-        const float4* table = reinterpret_cast<const float4*>(stage + 8 * kWgradPitch) + lane;
-        // rows past the last hold what the stage held before, or nothing (their factor in the operand is zero)
-        const bool on0 = t4 < rows, on1 = t4 + 4 < rows;
-        uint32_t ahi[MT][4], alo[MT][4];
+        const uint4* table = reinterpret_cast<const uint4*>(stage + kWgradStep * kWgradPitch) + lane;
+        uint32_t dz[MT][3][4];
 #pragma unroll
-        for (int m = 0; m < MT; m++) {
-            const float4 hi = table[64 * m], lo = table[64 * m + 32];
-            const float vh[4] = {hi.x, hi.y, hi.z, hi.w}, vl[4] = {lo.x, lo.y, lo.z, lo.w};
+        for (int m = 0; m < MT; m++)
 #pragma unroll
-            for (int e = 0; e < 4; e++) {
-                const bool on = 16 * m + 8 * (e & 1) + g < M1;  // (the table has no rows past M1)
-                ahi[m][e] = on ? __float_as_uint(vh[e]) : 0u, alo[m][e] = on ? __float_as_uint(vl[e]) : 0u;
+            for (int part = 0; part < 3; part++) {
+                const uint4 v = table[(3 * m + part) * 32];
+                const uint32_t e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                for (int i = 0; i < 4; i++) dz[m][part][i] = 16 * m + 8 * (i & 1) + g < M1 ? e[i] : 0u;  // (the table has no rows past M1)
             }
-        }
 #pragma unroll
         for (int h = 0; h < 2; h++) {  // the warp's two groups of 32 columns
             const int c = warp * kWgradCols + 32 * h + 4 * g;
             const bool in = cta_col + c < a.K1;
-            const float4 x0 = in && on0 ? *reinterpret_cast<const float4*>(stage + t4 * kWgradPitch + c) : make_float4(0, 0, 0, 0);
-            const float4 x1 = in && on1 ? *reinterpret_cast<const float4*>(stage + (t4 + 4) * kWgradPitch + c) : make_float4(0, 0, 0, 0);
-            const float v0[4] = {x0.x, x0.y, x0.z, x0.w}, v1[4] = {x1.x, x1.y, x1.z, x1.w};
+            float4 x[4];  // of four places; those past the last hold what the stage held before, or nothing (their factor is zero)
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                const int place = 2 * t4 + (i & 1) + 8 * (i >> 1);
+                x[i] = in && place < rows ? *reinterpret_cast<const float4*>(stage + place * kWgradPitch + c) : make_float4(0, 0, 0, 0);
+            }
 #pragma unroll
             for (int j = 0; j < 4; j++) {
-                uint32_t h0, l0, h1, l1;
-                tf32_split(v0[j], h0, l0);
-                tf32_split(v1[j], h1, l1);
+                auto col = [&](const float4& v) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; };
+                const Split s0 = bf16_split(col(x[0]), col(x[1])), s1 = bf16_split(col(x[2]), col(x[3]));
+                const uint32_t xp[3][2] = {{s0.h, s1.h}, {s0.m, s1.m}, {s0.l, s1.l}};
 #pragma unroll
-                for (int m = 0; m < MT; m++) {
-                    float part_sum[4] = {0.f, 0.f, 0.f, 0.f};
-                    mma_tf32(part_sum, ahi[m], l0, l1);
-                    mma_tf32(part_sum, alo[m], h0, h1);
-                    mma_tf32(part_sum, ahi[m], h0, h1);
-#pragma unroll
-                    for (int e = 0; e < 4; e++) acc[m][4 * h + j][e] += part_sum[e];
-                }
+                for (int m = 0; m < MT; m++) mma_split(acc[m][4 * h + j], dz[m], xp);
             }
         }
         __syncwarp();

@@ -16,6 +16,7 @@
 #include <stdint.h>
 
 #include "bulk_copy.cuh"
+#include "kernels_dense_mma.cuh"
 #include "launch.cuh"
 #include "peer_flags.cuh"
 
@@ -117,10 +118,10 @@ struct StepUpdateArgs {
     int copies;
     // first dense layer: l1w's range and what is written from it
     long long l1w4_begin, l1w4_end;
-    int K1, O, M1, tiles;      // tiles > 0: fragment tables of that many 8-row tiles, else w1g
-    float* w1g;                // [bucket][column][row]
-    float* w1f;                // kernels_dense_mma.cuh
-    float* w1d;
+    int K1, O, M1;
+    float* w1g;                // [bucket][column][row], or (null)
+    uint32_t* w1f;             // the fragment tables of kernels_dense_mma.cuh
+    uint32_t* w1d;
     // read-back
     const float* loss;
     const int* status;         // null: the step used no row lists
@@ -129,27 +130,25 @@ struct StepUpdateArgs {
     unsigned long long* stamps;  // [8] of this step
 };
 
-// where l1w's element `e` (column-major, rows k * M1 + r of all buckets) goes
-__device__ __forceinline__ void store_w1(const StepUpdateArgs& u, long long e, float w) {
-    const int OM = u.O * u.M1, col = (int)(e / OM), row = (int)(e - (long long)col * OM), k = row / u.M1, r = row - k * u.M1;
-    if (u.tiles == 0) {
-        u.w1g[((size_t)k * u.K1 + col) * u.M1 + r] = w;
+// where l1w's elements `e` .. e + 3 (column-major, rows k * M1 + r of all buckets) go
+__device__ __forceinline__ void store_w1(const StepUpdateArgs& u, long long e, float4 w) {
+    const int OM = u.O * u.M1;
+    if (!u.w1g) {  // (rows in fours: the elements are of one column and bucket)
+        const int col = (int)(e / OM), row = (int)(e - (long long)col * OM), k = row / u.M1;
+        store_fragments(u.w1f, u.w1d, u.K1, u.M1, k, col, row - k * u.M1, w);
         return;
     }
-    const uint32_t hi = __float_as_uint(w) + 0x1000u;  // as tf32_split
-    const float part[2] = {__uint_as_float(hi), __uint_as_float(__float_as_uint(w - __uint_as_float(hi & 0xffffe000u)) + 0x1000u)};
-    const int groups = (u.K1 + 15) / 16, c = col & 15, tile = r >> 3, r8 = r & 7;
-    const size_t base = (((size_t)k * groups + (col >> 4)) * u.tiles + tile) * 2 * 32 * 4;
-    const int f = (4 * r8 + (c >> 2)) * 4 + (c & 3);
-    const int d = (4 * (2 * (c >> 2) + (c & 1)) + (r8 & 3)) * 4 + 2 * ((c & 3) >> 1) + (r8 >> 2);
+    const long long n = (long long)u.K1 * OM;
+    const float v[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-    for (int h = 0; h < 2; h++) {
-        u.w1f[base + h * 128 + f] = part[h];
-        u.w1d[base + h * 128 + d] = part[h];
+    for (int i = 0; i < 4; i++) {
+        if (e + i >= n) return;
+        const int col = (int)((e + i) / OM), row = (int)(e + i - (long long)col * OM), k = row / u.M1;
+        u.w1g[((size_t)k * u.K1 + col) * u.M1 + row - k * u.M1] = v[i];
     }
 }
 
-__global__ void __launch_bounds__(256) step_update_kernel(const __grid_constant__ StepUpdateArgs u) {
+__global__ void __launch_bounds__(256, 3) step_update_kernel(const __grid_constant__ StepUpdateArgs u) {
     step_begin(u.stamps ? u.stamps + 4 : nullptr);
     const AdamArgs& a = u.adam;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -192,13 +191,7 @@ __global__ void __launch_bounds__(256) step_update_kernel(const __grid_constant_
             if (i >= a.seg[k].begin4 && i < a.seg[k].end4) si = k;
         if (si < 0 || si == u.l0f_seg) continue;  // alignment padding between tensors
         const float4 p = update(a.seg[si], i, u.g[i]);
-        if (i >= u.l1w4_begin && i < u.l1w4_end) {
-            const long long e = 4 * (i - u.l1w4_begin), n = (long long)u.K1 * u.O * u.M1;
-            store_w1(u, e, p.x);
-            if (e + 1 < n) store_w1(u, e + 1, p.y);
-            if (e + 2 < n) store_w1(u, e + 2, p.z);
-            if (e + 3 < n) store_w1(u, e + 3, p.w);
-        }
+        if (i >= u.l1w4_begin && i < u.l1w4_end) store_w1(u, 4 * (i - u.l1w4_begin), p);
     }
     if (u.stamps && threadIdx.x == 0) atomicMax(u.stamps + 7, clock_ns());
 }

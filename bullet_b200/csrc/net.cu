@@ -114,9 +114,9 @@ struct b200_net {
     int64_t n_flat = 0;
     float *P = nullptr, *G = nullptr, *M = nullptr, *V = nullptr, *table = nullptr;
     float *x = nullptr, *u = nullptr, *dx = nullptr, *a1 = nullptr, *a2 = nullptr, *out = nullptr, *w1g = nullptr;
-    float* dz_frag = nullptr;        // the gradient at the first dense layer's pre-activation as an operand of its weight gradient
+    uint32_t* dz_frag = nullptr;     // the gradient at the first dense layer's pre-activation as an operand of its weight gradient
     float* dense_partial = nullptr;  // the first dense layer's sums of slices of its columns
-    float4 *w1f = nullptr, *w1d = nullptr;  // the first dense layer's fragment tables (dense_mma)
+    uint32_t *w1f = nullptr, *w1d = nullptr;  // the first dense layer's fragment tables (dense_mma)
     float* dz[3] = {nullptr, nullptr, nullptr};
     int wgrad_per_sm = 0;          // resident CTAs per SM of the first layer's weight-gradient kernel (looked up once)
     int status_slot = -1;          // slot whose status word the running step reports (-1: the step used no tiled kernel)
@@ -636,9 +636,9 @@ int refresh_table(b200_net* net, int n) {
         const Tensor* w1 = net->find("l1w");
         const int O = net->d.n_out_buckets, M1 = net->d.dense_out[0];
         if (net->dense_mma()) {
-            const int lanes = (int)(b200::mma_table_floats(net->D1(), O, M1) / 8);
-            b200::dense_fragments_kernel<<<std::min(net->sm_count * 4, (lanes + 255) / 256), 256, 0, net->stream>>>(
-                net->P + w1->off, net->w1f, net->w1d, net->D1(), O, M1, M1 >= 8 ? M1 / 8 : 1);
+            const int quads = (int)(b200::mma_table_words(net->D1(), O, M1) / 6);  // (a thread writes six words of each table)
+            b200::dense_fragments_kernel<<<std::min(net->sm_count * 4, (quads + 255) / 256), 256, 0, net->stream>>>(
+                net->P + w1->off, net->w1f, net->w1d, net->D1(), O, M1);
         } else {
             net->w1_now ^= 1;
             if (net->w1g_now() == net->w1_used)  // (only if the weights moved twice since the last training pass)
@@ -1040,12 +1040,12 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     plan.add(&net->d_stamps, b200_net::kTimingRing * b200_net::kTimingEvents);
     plan.add(&net->d_status, b200_net::kLossRing);
     if (net->dense_mma()) {
-        const size_t table = b200::mma_table_floats(net->D1(), d.n_out_buckets, d.dense_out[0]) / 4;
+        const size_t table = b200::mma_table_words(net->D1(), d.n_out_buckets, d.dense_out[0]);
         plan.add(&net->w1f, table);
         plan.add(&net->w1d, table);
         // one part per slice, or more of them for few tiles (dense_split)
         const size_t tiles = (size_t)d.max_batch / b200::kDenseTile + std::min(d.n_out_buckets, d.max_batch) + 1;
-        plan.add(&net->dz_frag, tiles * 4 * (d.dense_out[0] > 16 ? d.dense_out[0] / 16 : 1) * 256);
+        plan.add(&net->dz_frag, tiles * (b200::kDenseTile / b200::kWgradStep) * b200::wgrad_table_words<16>(1) * (d.dense_out[0] > 16 ? d.dense_out[0] / 16 : 1));
         plan.add(&net->dense_partial, std::max(dense_slices(net) * tiles, (size_t)8 * net->sm_count) * b200::kDenseTile * d.dense_out[0]);
     } else {
         plan.add(&net->w1g, (size_t)2 * d.n_out_buckets * d.dense_out[0] * net->D1());
@@ -2184,11 +2184,10 @@ static int step_chained(b200_net* net, Slot& s, int slot, float lr, float grad_f
         u.K1 = net->D1();
         u.O = d.n_out_buckets;
         u.M1 = d.dense_out[0];
-        u.tiles = net->dense_mma() ? (u.M1 >= 8 ? u.M1 / 8 : 1) : 0;
         if (!lookahead && !net->dense_mma()) net->w1_now ^= 1;
         u.w1g = net->w1g_now();
-        u.w1f = reinterpret_cast<float*>(net->w1f);
-        u.w1d = reinterpret_cast<float*>(net->w1d);
+        u.w1f = net->w1f;
+        u.w1d = net->w1d;
         u.loss = net->G;
         u.status = net->status_slot >= 0 ? s.dev<int>(s.off_status) : nullptr;
         u.h_loss = net->h_loss + ring;

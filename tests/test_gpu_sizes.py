@@ -3,7 +3,7 @@ grouping, list lengths and holes, widths that leave a slab or a column group unf
 one tile, one tile more, and batches on either side of the small-batch kernels.
 
 Tolerances: the feature-transformer output is bit-exact (rows are added in slot order); outputs and gradients are sums in
-another order than the oracle's, of fp32 products (the tensor pipe's operands are split so that a product keeps 2^-22): at most
+another order than the oracle's, of fp32 products (the tensor pipe's operands are split so that a product keeps 2^-24): at most
 K = 4096 terms whose rounding errors add like a random walk, sqrt(K) 2^-24 = 4e-6 of the largest term, taken as 2e-5 of the
 largest entry, the bound of the other gradient tests."""
 import numpy as np
@@ -265,3 +265,73 @@ def oracle_x(oracle32, desc, w, stm, nstm):
     from tests.test_gpu_parity import oracle_ft_output
 
     return oracle_ft_output(oracle32, desc, w, stm, nstm)
+
+
+@pytest.mark.parametrize("dense,buckets", [((4, 1), 1), ((8, 1), 3), ((16, 32, 1), 2), ((32, 32, 1), 2)])
+def test_products_of_the_first_dense_layer_keep_32_bits(dense, buckets):
+    """One position: the weight gradient is x times the gradient at the layer's output, one product an entry, and that gradient is
+    the bias gradient; the gradient at x is a sum of as many products as the layer has rows.  A product whose operands are split
+    into parts is off by at most 2^-24 for the sum of its parts, 2^-25 for the parts left out and 2^-8 2^-22 for what the
+    accumulator of the small parts loses: below 2^-23.  A sum of R products adds at most log2(R) + 2 such roundings."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    desc = dataclasses.replace(net_of(1, 300, 264, 31, buckets, dense), max_batch=1, dense_act=(ACT_NONE,) * len(dense))
+    K, M = desc.dense_in0, dense[0]
+    for seed in range(6):
+        w = rich_weights(desc, seed=seed)
+        rng = np.random.default_rng(seed)
+        w["l1w"] = rng.normal(0, 0.05, w["l1w"].size).astype(np.float32)
+        net = make_net(desc, 0, w)
+        net.upload(0, *draw_batch(desc, 1, seed + 40))
+        net.backward(0)
+        k = int(draw_batch(desc, 1, seed + 40)[2][0])
+        g = net.tensors(kind=3)
+        x = net.activation(0, K).astype(np.float64)
+        dz = g["l1b"].reshape(buckets, M)[k].astype(np.float64)
+        assert (dz != 0).sum() > M // 2 and (x != 0).sum() > K // 8
+        gw = g["l1w"].reshape(K, buckets, M)
+        exact = x[:, None] * dz[None]
+        assert (np.abs(gw[:, k] - exact) <= 2.0**-23 * np.abs(exact)).all()
+        assert not gw[:, [b for b in range(buckets) if b != k]].any()
+        terms = w["l1w"].reshape(K, buckets, M)[:, k].astype(np.float64) * dz
+        bound = (np.log2(M) + 2) * 2.0**-23 * np.abs(terms).sum(1)
+        assert (np.abs(net.activation(2, K) - terms.sum(1)) <= bound).all()
+        net.close()
+
+
+@pytest.mark.parametrize("dense", [(4, 1), (8, 1), (16, 32, 1), (32, 32, 1)])
+def test_nan_passes_through_the_first_dense_layer(dense):
+    """A target that is NaN, or a weight, reaches every gradient that it is part of, and no other."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    n, bad, buckets = 50, 20, 2
+    desc = dataclasses.replace(net_of(1, 300, 136, 31, buckets, dense), max_batch=n)
+    K, M = desc.dense_in0, dense[0]
+    w = rich_weights(desc)
+    w["l1b"] = np.full(w["l1b"].size, 0.4, np.float32)
+    w["l1w"] *= np.float32(0.1)  # no output is clamped
+    batch = draw_batch(desc, n, seed=2)
+    batch[3][bad] = np.nan
+    k = int(batch[2][bad])
+    net = make_net(desc, 0, w)
+    net.upload(0, *batch)
+    for step in (lambda: net.backward(0), lambda: net.step(0, 0.0, 1.0 / n)):
+        step()
+        dx = net.activation(2, n * K).reshape(n, K)
+        assert np.isnan(dx[bad]).all() and not np.isnan(np.delete(dx, bad, 0)).any()
+        gw = net.tensors(kind=3)["l1w"].reshape(K, buckets, M)
+        assert np.isnan(gw[:, k]).all() and not np.isnan(gw[:, 1 - k]).any()
+    net.close()
+    batch[3][bad] = 0.5
+    for nan in (0x7FC00000, 0x7FFFFFFF, 0xFFFFFFFF):
+        w2 = {name: v.copy() for name, v in w.items()}
+        w2["l1w"].reshape(K, buckets, M)[5, k, 1] = np.array([nan], np.uint32).view(np.float32)[0]
+        net = make_net(dataclasses.replace(desc, dense_act=(ACT_NONE,) * len(dense)), 0, w2)
+        net.upload(0, *batch)
+        out = net.forward(0, n)
+        assert np.array_equal(np.isnan(out), batch[2] == k)
+        net.close()
