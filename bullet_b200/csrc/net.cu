@@ -1002,7 +1002,7 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     }
     net->n_flat = (off + 1023) / 1024 * 1024;  // a multiple of 4 floats x 256: splits evenly over up to 256 ranks
 
-    constexpr size_t kMaxSmem = 227 * 1024 - 64;  // (the tiled kernels declare a few static bytes)
+    constexpr size_t kMaxSmem = 227 * 1024 - 128;  // (the tiled backward's own few bytes count as 128)
     // The tiled kernels need features of one perspective that fall into one block.  A table that is small enough is one block
     // whatever was promised, and then any width will do (a width that 64 does not divide costs as much as the next that does).
     const bool promised = d.ft_block_rows > 0 && d.n_inputs % d.ft_block_rows == 0 && d.ft_out % b200::kTileCols == 0;

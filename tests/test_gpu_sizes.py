@@ -154,6 +154,29 @@ def test_the_largest_tables_of_the_tiled_kernels(oracle32, nnz, rows_less):
         assert rc == 0 and np.array_equal(x, x_ref)
 
 
+@pytest.mark.parametrize("rows", [855, 860, 861, 863, 865, 866])
+def test_the_longest_chunks_of_the_backward(oracle32, rows):
+    """Row counts on either side of where chunks of 640 pairs just fit into shared memory, with a batch that is cut into 148 of
+    them (one for every SM), and with one that is not.  Bounds as above."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    most = 148 * 320
+    desc = dataclasses.replace(net_of(1, rows, 64, 32, 1, (1,)), max_batch=most)
+    w = rich_weights(desc)
+    net = make_net(desc, 0, w)
+    for n in (most, 3001):
+        batch = draw_batch(desc, n, seed=rows)
+        net.upload(0, *batch)
+        net.backward(0)
+        _, g_ref, _ = oracle32.net_grad(desc, w, *batch)
+        g = net.tensors(kind=3)
+        for k in g_ref:
+            assert np.abs(g[k] - g_ref[k]).max() <= 2e-5 * np.abs(g_ref[k]).max(), k
+    net.close()
+
+
 def net_flat(net, kind):
     import torch
 
