@@ -5,8 +5,8 @@
 //   pass 1  one kernel per source (group_lists_kernel here, prep_featurise_kernel for raw records): per pair its block and
 //           list length, per CTA of kGroupPositions positions a histogram of blocks and output buckets
 //   pass 2  group_place_kernel: one CTA per window of kWindowPositions positions.  It sums the histograms before it (the
-//           whole table of them is a few tens of KB), orders its pairs by (block, list length) and writes their lists in
-//           place; CTA 0 also derives the tables.
+//           whole table of them is a few tens of KB; a long one has been summed up by group_scan_kernel), orders its pairs by
+//           (block, list length) and writes their lists in place; CTA 0 also derives the tables.
 //
 // Pairs of one block and window lie in the order of their list lengths, so that neighbours, which the row walks serve two
 // at a time, have lists of nearly the same length; a window is small enough that every stretch of a block's pairs holds
@@ -31,7 +31,7 @@ struct GroupArgs {
     const int* buckets;    // [n] output bucket per position (n_out_buckets > 1)
     int n, nnz, n_inputs, block_rows, nblocks, n_out_buckets;
     int* info;             // scratch [2n]: block << 8 | list length
-    int* hist;             // scratch [CTAs of pass 1][nblocks + n_out_buckets]
+    int* hist;             // scratch [CTAs of pass 1 + 1][nblocks + n_out_buckets]
     int* status;           // device or pinned host word
     int clear_status;      // pass 1 clears it first
     // pass 2
@@ -52,6 +52,37 @@ struct GroupArgs {
 
 __host__ __device__ inline int group_ctas(int n) { return (n + kGroupPositions - 1) / kGroupPositions; }
 __host__ __device__ inline int group_windows(int n) { return (n + kWindowPositions - 1) / kWindowPositions; }
+
+// Every window reads all histograms, so that the reads grow with the square of the batch.  Up to 131072 positions that is the
+// cheaper way (18 MB out of L2 with 17 bins, about 4 us, as much as one more launch); beyond, their running sums are formed once.
+// Operator of 64 columns, 32 slots, 16 blocks, without and with the sums: 207 and 170 us at 262144 positions, 11.9 and 2.1 ms at
+// 4 million.
+inline bool group_scans(int n) { return group_ctas(n) > 1024; }
+
+// hist[c][bin] -> sum of the rows before c, and the total in one more row.  grid = bins, block = 1024.
+static __global__ void __launch_bounds__(1024) group_scan_kernel(int* hist, int ctas, int nbins) {
+    __shared__ int warp_tot[32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int* column = hist + blockIdx.x;
+    int run = 0;
+    for (int base = 0; base < ctas; base += 1024) {
+        const int c = base + (int)threadIdx.x;
+        const int own = c < ctas ? column[(size_t)c * nbins] : 0;
+        int incl = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += up;
+        }
+        if (lane == 31) warp_tot[warp] = incl;
+        __syncthreads();
+        const int before = __reduce_add_sync(0xffffffffu, lane < warp ? warp_tot[lane] : 0), all = __reduce_add_sync(0xffffffffu, warp_tot[lane]);
+        if (c < ctas) column[(size_t)c * nbins] = run + before + incl - own;
+        run += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) column[(size_t)ctas * nbins] = run;
+}
 
 // Whether a thread can take eight slots of a list with one load: the lists start on 16 bytes and hold 8, 16, 32 or 64 slots.
 inline bool group_vec(const GroupArgs& g) {
@@ -220,10 +251,11 @@ __device__ __forceinline__ int prepare_list_warp(const GroupArgs& g, uint32_t s0
 constexpr int kPlaceThreads = 2 * kWindowPositions;
 constexpr int kCountedBlocks = 32;  // up to as many row blocks a window orders its pairs by counting, beyond by sorting
 
-// Pass 2.  grid = group_windows(n) CTAs of one thread per pair of the window.  `vec`: see group_vec.
+// Pass 2.  grid = group_windows(n) CTAs of one thread per pair of the window.  `vec`: see group_vec; `scanned`: the histograms are
+// running sums already (group_scan_kernel).
 // Latency bound (one CTA per SM at most for ordinary batches): one sweep over the histograms, a counting sort (a bitonic one
 // for many blocks: its 45 barriers took a third of the kernel's 13 us), one gather of the lists.
-static __global__ void __launch_bounds__(kPlaceThreads) group_place_kernel(GroupArgs g, int vec) {
+static __global__ void __launch_bounds__(kPlaceThreads) group_place_kernel(GroupArgs g, int vec, int scanned) {
     __shared__ int before[kGroupMaxBlocks + kGroupMaxBuckets], block_at[kGroupMaxBlocks + 1], bucket_at[kGroupMaxBuckets + 1];
     __shared__ int scan_s[kGroupMaxBlocks + 1], run_start[kGroupMaxBlocks];
     __shared__ unsigned key_s[kPlaceThreads];
@@ -235,7 +267,13 @@ static __global__ void __launch_bounds__(kPlaceThreads) group_place_kernel(Group
     for (int k = tid; k <= kGroupMaxBlocks; k += kPlaceThreads) block_at[k] = 0;
     if (tid <= kGroupMaxBuckets) bucket_at[tid] = 0;
     __syncthreads();
-    {   // totals, and what lies before this window, of every bin
+    if (scanned) {
+        const int ctas = group_ctas(g.n), mine = (int)blockIdx.x * (kWindowPositions / kGroupPositions);
+        if (tid < nbins) {
+            before[tid] = __ldg(g.hist + (size_t)mine * nbins + tid);
+            *(tid < nb ? &block_at[tid] : &bucket_at[tid - nb]) = __ldg(g.hist + (size_t)ctas * nbins + tid);
+        }
+    } else {  // totals, and what lies before this window, of every bin
         int width = 1;
         while (width < nbins) width <<= 1;
         const int bin = tid & (width - 1), ctas = group_ctas(g.n), mine = (int)blockIdx.x * (kWindowPositions / kGroupPositions);

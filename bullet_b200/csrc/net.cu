@@ -370,7 +370,7 @@ void slot_layout(const b200_net* net, Slot& s, int n) {
     s.off_bexpect = take(nb * 4);
     s.off_status = take(4);
     s.off_info = take((size_t)n * 8);
-    s.off_hist = take(many ? 4 : (size_t)b200::group_ctas(n) * bins * 4);
+    s.off_hist = take(many ? 4 : (size_t)(b200::group_ctas(n) + 1) * bins * 4);
     s.off_many[0] = take(many ? bins * 4 : 4);
     s.off_many[1] = take(many ? (bins + 2) * 4 : 4);
     s.off_many[2] = take(many ? (bins + 1) * 4 : 4);
@@ -730,7 +730,13 @@ int group_slot(b200_net* net, Slot& s, const b200::GroupArgs& g, bool counted, c
             b200::group_lists_kernel<<<b200::group_ctas(g.n), b200::kGroupThreads, 0, stream>>>(g, vec);
             LAUNCHED(net);
         }
-        b200::group_place_kernel<<<b200::group_windows(g.n), b200::kPlaceThreads, 0, stream>>>(g, vec);
+        const bool scans = b200::group_scans(g.n);
+        if (scans) {
+            const int bins = g.nblocks + g.n_out_buckets;
+            b200::group_scan_kernel<<<bins, 1024, 0, stream>>>(g.hist, b200::group_ctas(g.n), bins);
+            LAUNCHED(net);
+        }
+        b200::group_place_kernel<<<b200::group_windows(g.n), b200::kPlaceThreads, 0, stream>>>(g, vec, scans);
         LAUNCHED(net);
     }
     if (g.want_lists) s.prepared = true;
@@ -921,7 +927,7 @@ int preload_kernels(b200_net* net) {
     ok = ok && load_kernel(b200::adamw_exchange_bulk_kernel<0, 128, 6>);
     ok = ok && load_kernel(b200::adamw_exchange_overlap_kernel<0>) && load_kernel(b200::adamw_exchange_overlap_kernel<2>);
     ok = ok && load_kernel(b200::adamw_exchange_overlap_kernel<4>) && load_kernel(b200::adamw_exchange_overlap_kernel<8>);
-    ok = ok && load_kernel(b200::prep_featurise_kernel) && load_kernel(b200::group_lists_kernel) && load_kernel(b200::group_place_kernel);
+    ok = ok && load_kernel(b200::prep_featurise_kernel) && load_kernel(b200::group_lists_kernel) && load_kernel(b200::group_scan_kernel) && load_kernel(b200::group_place_kernel);
     ok = ok && load_kernel(b200::group_many_count_kernel) && load_kernel(b200::group_many_scan_kernel) && load_kernel(b200::group_many_place_kernel);
     ok = ok && load_kernel(b200::peer_signal_kernel) && load_kernel(b200::peer_wait_kernel) && load_kernel(b200::bucket_presignal_kernel);
     if (!ok) return b200::fail(B200_ERR_CUDA, "net_create: loading the kernels failed: %s", cudaGetErrorString(cudaGetLastError()));

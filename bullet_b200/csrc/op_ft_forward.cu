@@ -46,7 +46,7 @@ constexpr size_t kScratchHeader = align_ints(kMaxBlocks + 2);
 constexpr int list_len(int nnz) { return (nnz + 7) & ~7; }  // 16-byte groups of u16 row indices
 constexpr size_t hist_ints(int n, int nblocks) {
     return nblocks > b200::kGroupMaxBlocks ? align_ints(3 * (size_t)(nblocks + 3))
-                                           : align_ints((size_t)((n + b200::kGroupPositions - 1) / b200::kGroupPositions) * (nblocks + 1));
+                                           : align_ints((size_t)((n + b200::kGroupPositions - 1) / b200::kGroupPositions + 1) * (nblocks + 1));
 }
 constexpr size_t scratch_ints(int n, int nnz, int nblocks) {
     return kScratchHeader + align_ints((size_t)2 * n) + align_ints((size_t)4 * n) + (size_t)n * list_len(nnz) + hist_ints(n, nblocks);
@@ -169,7 +169,9 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
     } else {
         const bool vec = b200::group_vec(g);
         b200::group_lists_kernel<<<b200::group_ctas(n), b200::kGroupThreads, 0, stream>>>(g, vec);
-        b200::group_place_kernel<<<b200::group_windows(n), b200::kPlaceThreads, 0, stream>>>(g, vec);
+        const bool scans = b200::group_scans(n);
+        if (scans) b200::group_scan_kernel<<<nblocks + 1, 1024, 0, stream>>>(hist, b200::group_ctas(n), nblocks + 1);
+        b200::group_place_kernel<<<b200::group_windows(n), b200::kPlaceThreads, 0, stream>>>(g, vec, scans);
     }
     CK(cudaGetLastError());
 

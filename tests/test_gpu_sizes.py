@@ -177,6 +177,33 @@ def test_the_longest_chunks_of_the_backward(oracle32, rows):
     net.close()
 
 
+@pytest.mark.parametrize("n", [131072, 131073, 262144 + 77])
+def test_grouping_of_long_batches(oracle32, n):
+    """The last batch whose windows sum the counts themselves, and longer ones whose counts have been summed up before, by one and
+    by more rounds: feature-transformer output bit-exact by network and operator, gradients with the bounds above."""
+    import dataclasses
+
+    from tests.test_gpu_ops import run_op
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    desc = dataclasses.replace(net_of(5, 60, 64, 6, 3, (1,)), max_batch=n)
+    batch = draw_batch(desc, n, seed=n & 15)
+    w = rich_weights(desc)
+    x_ref = oracle_x(oracle32, desc, w, *batch[:2])
+    net = make_net(desc, 0, w)
+    net.upload(0, *batch)
+    net.backward(0)
+    assert np.array_equal(net.activation(0, n * desc.dense_in0).reshape(n, -1), x_ref)
+    _, g_ref, _ = oracle32.net_grad(desc, w, *batch)
+    g = net.tensors(kind=3)
+    for k in g_ref:
+        # (the oracle adds n terms one after the other: sqrt(n) 2^-24 of the sum in a random walk, and as much again for a drift)
+        assert np.abs(g[k] - g_ref[k]).max() <= 6e-5 * np.abs(g_ref[k]).max(), k
+    net.close()
+    rc, x, _ = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], *batch[:2], n)
+    assert rc == 0 and np.array_equal(x, x_ref)
+
+
 def net_flat(net, kind):
     import torch
 
