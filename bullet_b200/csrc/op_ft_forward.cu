@@ -223,8 +223,8 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
 
 }  // namespace
 
-// One pool per device for the scratch of b200_op_ft_forward.  It keeps at most kPoolKeep bytes between calls; a network that
-// finds no room for its own buffers has it give those back (op_pool_trim).  Stream-ordered, so calls on several streams and
+// One pool per device for the scratch of b200_op_ft_forward.  It keeps at most kPoolKeep bytes between calls, for as long as the
+// process lives or until a network that finds no room for its own buffers has it give those back (op_pool_trim).  Stream-ordered, so calls on several streams and
 // threads never share memory that is in use.
 namespace b200 {
 namespace {

@@ -339,8 +339,9 @@ int b200_save_unquantised(b200_net* net, const b200_saved_format* fmt, int32_t n
  * (crates/compiler/src/model/builder.rs:145-147), the activation (autograd/dfo.rs:47-88), the
  * optional pairwise product (model/builder.rs:390-393) and the stm|nstm concat (builder.rs:375-388).
  * Needs the block structure (ft_block_rows > 0 dividing n_inputs) and ft_out a multiple of 64.
- * Groups the positions by row block on the device, in scratch memory taken from cudaMalloc for
- * the duration of the call; runs on `stream` (NULL = default stream) and waits for it. */
+ * Groups the positions by row block on the device, in scratch memory taken from a stream-ordered pool of the
+ * library for the duration of the call (the pool keeps up to 32 MB per device between calls); runs on `stream`
+ * (NULL = default stream) and waits for it. */
 typedef struct b200_ft_op {
     int32_t n_inputs, nnz, ft_out, ft_act, pairwise, ft_block_rows;
     int32_t n;                /* positions */

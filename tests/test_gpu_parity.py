@@ -637,7 +637,9 @@ def test_full_size_properties_without_the_oracle():
     loss_again, g_again = grads_of(full)
     (loss_a, g_a), (loss_b, g_b) = grads_of(halves[0]), grads_of(halves[1])
     assert abs(loss_full - (loss_a + loss_b)) <= 1e-5 * loss_full
-    assert abs(loss_full - loss_again) <= 1e-6 * loss_full
+    # up to 592 CTAs (four per SM) add their part of the loss to one float in any order, each rounding by up to 2^-24 of the sum:
+    # a random walk of sqrt(592) 2^-24 = 1.5e-6 for each of the two, three times their difference
+    assert abs(loss_full - loss_again) <= 6e-6 * loss_full
     for k in g_full:
         assert rel2(g_a[k] + g_b[k], g_full[k]) <= 1e-5, k
         assert rel2(g_again[k], g_full[k]) <= 1e-6, k
