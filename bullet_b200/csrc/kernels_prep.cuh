@@ -24,6 +24,7 @@ struct PrepArgs {
     int game;
     const int* expanded;    // [64] 768 * king bucket of every square (king-bucketed chess inputs)
     const float* win_rate;  // [65536] sigmoid(score / scale) for every 16-bit score, index score + 32768
+    const float* given;     // the targets as the host has formed them, or null
     float blend;
     uint16_t* stm;          // out [n][nnz], 0xFFFF = empty
     uint16_t* nstm;
@@ -64,8 +65,12 @@ static __global__ void __launch_bounds__(kPrepThreads) prep_featurise_kernel(Pre
         p.buckets[i] = bucket;
         // blend * result / 2 + (1 - blend) * sigmoid(score / scale), every operation rounded on its own as the
         // host compiler does it (no fused multiply-add)
-        const float wr = p.win_rate[score + 32768];
-        p.targets[i] = __fadd_rn(__fmul_rn(p.blend, __fdiv_rn((float)result, 2.0f)), __fmul_rn(__fsub_rn(1.0f, p.blend), wr));
+        if (p.given) {
+            p.targets[i] = p.given[i];
+        } else {
+            const float wr = p.win_rate[score + 32768];
+            p.targets[i] = __fadd_rn(__fmul_rn(p.blend, __fdiv_rn((float)result, 2.0f)), __fmul_rn(__fsub_rn(1.0f, p.blend), wr));
+        }
     }
     const unsigned below = (1u << lane) - 1u;
 #pragma unroll 4

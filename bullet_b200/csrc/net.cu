@@ -176,6 +176,8 @@ struct b200_net {
     float* facc = nullptr;               // running block sum of this rank's share of the factoriser gradient
     float* d_win_rate = nullptr;         // device-side preparation: sigmoid(score / scale) for every 16-bit score
     float win_rate_scale = 0.f;          // the scale the table was made for (0: none yet)
+    float host_scale = 0.f;              // the scale of the records that came without a table, one after the other,
+    int64_t host_positions = 0;          // and how many there were
     int* d_expanded = nullptr;           // [64] 768 * king bucket per square, and the layout it was made from
     int32_t expanded_layout[32] = {};
     bool expanded_valid = false;
@@ -362,7 +364,7 @@ void slot_layout(const b200_net* net, Slot& s, int n) {
     s.off_targets = take((size_t)n * 4);
     s.off_order = take((size_t)n * 4);
     s.off_dtiles = take(((size_t)n / b200::kDenseTile + O + 1) * 8);
-    s.off_records = take((size_t)n * 32);
+    s.off_records = take((size_t)n * 36);  // and, of some batches, their targets
     s.off_pairs = take((size_t)n * 16);
     s.off_blocks = take((nb + 1) * 4);
     s.off_chunks = take(((size_t)2 * n / b200::kChunkLeast + nb + 1) * 16);
@@ -1094,7 +1096,7 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     cudaMemsetAsync(net->M, 0, net->n_flat * 4, net->stream);
     cudaMemsetAsync(net->V, 0, net->n_flat * 4, net->stream);
 
-    const size_t pinned_slot = align_up(std::max(net->slots[0].off_records, (size_t)d.max_batch * 32), 4096);
+    const size_t pinned_slot = align_up(std::max(net->slots[0].off_records, (size_t)d.max_batch * 36), 4096);
     {   // pinned memory: the slots' staging blocks, the outputs of an evaluation, the read-back ring
         void* raw = nullptr;
         const size_t out_bytes = align_up(B * sizeof(float), 4096);
@@ -1468,32 +1470,46 @@ static int upload_records(b200_net* net, int slot, const void* records, int32_t 
     if (O > 1 && game == B200_GAME_ATAXX147) return b200::fail(B200_ERR_UNSUPPORTED, "%s: no output buckets for ataxx records", who);
     if (int rc = upload_begin(net, slot, n, who)) return rc;
     Slot& s = net->slots[slot];
-    if (net->win_rate_scale != scale) {  // the same function the host mapper evaluates, for every possible score
+    // The device looks the win rate of a score up in a table, which takes the host as long to make as the targets of 65536
+    // positions do: until a scale has seen that many, the host forms the targets while it goes through the records.
+    // (First upload and evaluation of a network, king buckets, width 2048, with the table made first and now: 1 position 357
+    // and 120 us, 1024 434 and 197, 16384 696 and 464.)
+    bool host_targets = false;
+    if (net->win_rate_scale != scale) {
+        if (net->host_scale != scale) net->host_scale = scale, net->host_positions = 0;
+        net->host_positions += n;
+        host_targets = net->host_positions < 65536;
+    }
+    const float rscale = 1.0f / scale;
+    if (net->win_rate_scale != scale && !host_targets) {  // the same function the host mapper evaluates, for every possible score
         std::vector<float> table(65536);
-        const float rscale = 1.0f / scale;
+#pragma omp parallel for schedule(static)
         for (int v = -32768; v < 32768; v++) table[v + 32768] = b200::blended_target((int16_t)v, 0, rscale, 0.0f);
-        CK(cudaStreamSynchronize(net->copy_stream));
-        CK(cudaMemcpy(net->d_win_rate, table.data(), table.size() * sizeof(float), cudaMemcpyHostToDevice));
+        // (behind the kernels that read the table before; out of pageable memory, so it has been read when the call returns)
+        CK(cudaMemcpyAsync(net->d_win_rate, table.data(), table.size() * sizeof(float), cudaMemcpyHostToDevice, net->copy_stream));
         net->win_rate_scale = scale;
+        net->host_positions = 0;
     }
     if (game == B200_GAME_CHESS_BUCKETS_MIRRORED && (!net->expanded_valid || memcmp(net->expanded_layout, layout32, sizeof net->expanded_layout))) {
         int32_t expanded[64];
         b200::expand_king_buckets(layout32, expanded);
-        CK(cudaStreamSynchronize(net->copy_stream));
-        CK(cudaMemcpy(net->d_expanded, expanded, sizeof expanded, cudaMemcpyHostToDevice));
+        net->expanded_valid = false;
+        CK(cudaMemcpyAsync(net->d_expanded, expanded, sizeof expanded, cudaMemcpyHostToDevice, net->copy_stream));
         memcpy(net->expanded_layout, layout32, sizeof net->expanded_layout);
         net->expanded_valid = true;
     }
+    float* targets = reinterpret_cast<float*>(s.h_blob + (size_t)n * 32);  // behind the records
     int bad = n, bad_bucket = n;
     {
         const b200::AtaxxRecord* in = static_cast<const b200::AtaxxRecord*>(records);  // (both kinds start with 64-bit boards)
         b200::AtaxxRecord* out = reinterpret_cast<b200::AtaxxRecord*>(s.h_blob);
         const int nnz = d.nnz;
         const bool ataxx = game == B200_GAME_ATAXX147;
-#pragma omp parallel for schedule(static) reduction(min : bad) reduction(min : bad_bucket) if (n >= 8192)
+#pragma omp parallel for schedule(static) reduction(min : bad) reduction(min : bad_bucket) if (n >= (host_targets ? 2048 : 8192))
         for (int32_t i = 0; i < n; i++) {
             const b200::AtaxxRecord r = in[i];
             out[i] = r;
+            if (host_targets) targets[i] = b200::blended_target(r.score, r.result, rscale, blend);  // same offsets in both record types
             int pieces = __builtin_popcountll(r.bbs[0]);
             if (ataxx) pieces += __builtin_popcountll(r.bbs[1]) + __builtin_popcountll(r.bbs[2]);
             if (pieces > nnz) bad = i < bad ? i : bad;
@@ -1502,7 +1518,8 @@ static int upload_records(b200_net* net, int slot, const void* records, int32_t 
     }
     if (bad < n) return b200::fail(B200_ERR_DATA, "%s: record %d holds more than nnz=%d pieces", who, bad, d.nnz);
     if (bad_bucket < n) return b200::fail(B200_ERR_DATA, "%s: record %d has no valid output bucket", who, bad_bucket);
-    net->h2d_bytes += (int64_t)n * 32;
+    const size_t bytes = (size_t)n * (host_targets ? 36 : 32);
+    net->h2d_bytes += (int64_t)bytes;
     s.n = n;
     s.prepared = s.csr_built = false;
     cut_dense(net, s);
@@ -1512,6 +1529,7 @@ static int upload_records(b200_net* net, int slot, const void* records, int32_t 
     // would wait for PCIe on SMs that the step could use.)
     const bool direct = !net->trains && n <= 16384;
     p.records = direct ? reinterpret_cast<const uint4*>(s.h_blob) : s.dev<uint4>(s.off_records);
+    if (host_targets) p.given = reinterpret_cast<const float*>(p.records + 2 * (size_t)n);
     p.game = game;
     p.expanded = net->d_expanded;
     p.win_rate = net->d_win_rate;
@@ -1520,7 +1538,7 @@ static int upload_records(b200_net* net, int slot, const void* records, int32_t 
     p.nstm = s.dev<uint16_t>(s.off_nstm);
     p.buckets = s.dev<int>(s.off_buckets);
     p.targets = s.dev<float>(s.off_targets);
-    if (!direct) CK(cudaMemcpyAsync(s.d_blob + s.off_records, s.h_blob, (size_t)n * 32, cudaMemcpyHostToDevice, net->copy_stream));
+    if (!direct) CK(cudaMemcpyAsync(s.d_blob + s.off_records, s.h_blob, bytes, cudaMemcpyHostToDevice, net->copy_stream));
     const b200::GroupArgs g = group_args(net, s, upload_wants_lists(net, n), O > 1);
     b200::prep_featurise_kernel<<<b200::group_ctas(n), b200::kPrepThreads, 0, net->copy_stream>>>(p, g);
     LAUNCHED(net);

@@ -743,3 +743,27 @@ def test_device_preparation_fills_the_slot_exactly_as_the_host_path(ci):
             small.upload_records(0, c.game, synth.records(c.game, 64, seed=5), on_device=True)
         assert e.value.code == -4
         small.close()
+
+
+@pytest.mark.parametrize("ci", [0, 3])
+def test_targets_of_records_whoever_forms_them(ci):
+    """The first records of a scale get their targets from the host, later ones from a table on the device: bit for bit those of
+    the mapper, also where the scale changes in between, and for a network that trains (whose records go another way)."""
+    from bullet_b200.net import featurise
+
+    c = config(ci)
+    most = 40000
+    desc = dataclasses.replace(c.desc, ft_out=128, max_batch=most)
+    net = make_net(desc, 0, synth.init_weights(desc, seed=ci))
+    calls = [(1, 400.0, 0.5), (3000, 400.0, 0.25), (500, 250.0, 0.5), (most, 400.0, 0.5), (30000, 400.0, 0.75), (700, 400.0, 1.0),
+             (800, 250.0, 0.0), (900, 400.0, 0.5)]
+    for trains in (False, True):
+        for k, (n, scale, blend) in enumerate(calls):
+            rec = synth.records(c.game, n, seed=300 + k)
+            net.upload_records(k % 3, c.game, rec, scale=scale, blend=blend)
+            if trains:
+                net.step(k % 3, 1e-3, 1.0 / n)
+            want = featurise(c.game, rec, desc, scale=scale, blend=blend)
+            assert np.array_equal(net.slot_contents(k % 3)["targets"], want[3]), (trains, k)
+        net.step(0, 0.0, 1.0)
+    net.close()
