@@ -1558,38 +1558,42 @@ int b200_slot_read(b200_net* net, int slot, uint16_t* stm, uint16_t* nstm, int32
                    int32_t* pair_order, int32_t* n) {
     if (int rc = check_slot(net, slot, "slot_read")) return rc;
     if (int rc = set_device(net)) return rc;
-    const Slot& s = net->slots[slot];
+    Slot& s = net->slots[slot];
     CK(cudaStreamSynchronize(net->copy_stream));
     const size_t count = (size_t)s.n, list = count * net->d.nnz * sizeof(uint16_t);
     if (stm) CK(cudaMemcpy(stm, s.d_blob + s.off_stm, list, cudaMemcpyDeviceToHost));
     if (nstm) CK(cudaMemcpy(nstm, s.d_blob + s.off_nstm, list, cudaMemcpyDeviceToHost));
     if (buckets) CK(cudaMemcpy(buckets, s.d_blob + s.off_buckets, count * 4, cudaMemcpyDeviceToHost));
     if (targets) CK(cudaMemcpy(targets, s.d_blob + s.off_targets, count * 4, cudaMemcpyDeviceToHost));
-    // both groupings as they are defined: ascending inside a group.  (The kernels visit the pairs of a block in another
-    // order, which the lists' lengths decide.)
-    if (order) {
+    // Both groupings as the kernels have them, every group in ascending order (which the kernels keep for the positions of up to
+    // kGroupMaxBlocks row blocks only: they visit the pairs of a block in the order of their lists' lengths).
+    if (order && net->d.n_out_buckets > 1) {
         std::vector<int> bucket(count);
         CK(cudaMemcpy(bucket.data(), s.d_blob + s.off_buckets, count * 4, cudaMemcpyDeviceToHost));
-        std::vector<int> begin(net->d.n_out_buckets + 1, 0);
-        for (size_t i = 0; i < count; i++) begin[bucket[i] + 1]++;
-        for (int k = 0; k < net->d.n_out_buckets; k++) begin[k + 1] += begin[k];
-        for (size_t i = 0; i < count; i++) order[begin[bucket[i]]++] = (int32_t)i;
+        CK(cudaMemcpy(order, s.d_blob + s.off_order, count * 4, cudaMemcpyDeviceToHost));
+        if (net->nblocks > b200::kGroupMaxBlocks)
+            for (size_t at = 0, end; at < count; at = end) {  // runs of one bucket
+                for (end = at + 1; end < count && bucket[order[end]] == bucket[order[at]];) end++;
+                std::sort(order + at, order + end);
+            }
+    } else if (order) {
+        for (size_t i = 0; i < count; i++) order[i] = (int32_t)i;
     }
-    if (pair_order) {
-        const int nnz = net->d.nnz, R = net->nblocks > 1 ? net->block_rows : net->d.n_inputs;
-        std::vector<uint16_t> lists[2] = {std::vector<uint16_t>(count * nnz), std::vector<uint16_t>(count * nnz)};
-        CK(cudaMemcpy(lists[0].data(), s.d_blob + s.off_stm, list, cudaMemcpyDeviceToHost));
-        CK(cudaMemcpy(lists[1].data(), s.d_blob + s.off_nstm, list, cudaMemcpyDeviceToHost));
-        std::vector<int> block(2 * count), begin(net->nblocks + 1, 0);
-        for (size_t i = 0; i < 2 * count; i++) {
-            const uint16_t* own = lists[i & 1].data() + (i >> 1) * nnz;
-            int k = 0;
-            while (k < nnz && own[k] >= net->d.n_inputs) k++;
-            block[i] = k < nnz ? own[k] / R : 0;
-            begin[block[i] + 1]++;
+    if (pair_order && net->tiled_ok) {
+        if (!s.prepared) {  // (a batch that no tiled kernel has needed yet)
+            cut_ft(net, s);
+            if (int rc = group_slot(net, s, group_args(net, s, true, false), false, net->copy_stream)) return rc;
+            CK(cudaStreamSynchronize(net->copy_stream));
         }
-        for (int k = 0; k < net->nblocks; k++) begin[k + 1] += begin[k];
-        for (size_t i = 0; i < 2 * count; i++) pair_order[begin[block[i]]++] = (int32_t)i;
+        CK(cudaStreamSynchronize(net->stream));  // (the lists may have been made by a training pass)
+        std::vector<int2> pairs(2 * count);
+        std::vector<int> begin(net->nblocks + 1);
+        CK(cudaMemcpy(pairs.data(), s.d_blob + s.off_pairs, pairs.size() * sizeof(int2), cudaMemcpyDeviceToHost));
+        CK(cudaMemcpy(begin.data(), s.d_blob + s.off_blocks, begin.size() * sizeof(int), cudaMemcpyDeviceToHost));
+        for (size_t i = 0; i < 2 * count; i++) pair_order[i] = pairs[i].x;
+        for (int k = 0; k < net->nblocks; k++) std::sort(pair_order + begin[k], pair_order + begin[k + 1]);
+    } else if (pair_order) {  // without row blocks the pairs are visited as they come
+        for (size_t i = 0; i < 2 * count; i++) pair_order[i] = (int32_t)i;
     }
     if (n) *n = s.n;
     return 0;

@@ -710,33 +710,58 @@ def test_upload_from_records_equals_featurise_then_upload(ci):
     b.close()
 
 
+def slot_by_hand(desc, batch):
+    """What a slot holds for the mapper's arrays: packed lists, buckets, targets, and the positions by output bucket and the
+    (position, perspective) pairs by the row block of their first feature, both in ascending order inside a group."""
+    stm, nstm, buckets, targets = batch
+    n = len(targets)
+    lists = [np.where((a >= 0) & (a < desc.n_inputs), a, 0xFFFF).astype(np.uint16) for a in (stm, nstm)]
+    pairs = np.stack(lists, 1).reshape(2 * n, -1)
+    block = np.zeros(2 * n, np.int64)
+    if desc.ft_block_rows:
+        first = (pairs != 0xFFFF).argmax(1)
+        feature = pairs[np.arange(2 * n), first].astype(np.int64)
+        block = np.where(feature == 0xFFFF, 0, feature // desc.ft_block_rows)
+    return {"stm": lists[0], "nstm": lists[1], "buckets": buckets, "targets": targets,
+            "order": np.argsort(buckets, kind="stable"), "pair_order": np.argsort(block, kind="stable")}
+
+
 @pytest.mark.parametrize("ci", [0, 1, 2, 3])
 def test_device_preparation_fills_the_slot_exactly_as_the_host_path(ci):
-    """b200_batch_upload_records_gpu (featuriser, bucket, target and both stable groupings as kernels) leaves the
-    slot bit-identical to b200_batch_upload_records: packed lists, buckets, targets, positions by output bucket,
-    pairs by row block.  Forward outputs are then bit-identical and a training step agrees to rounding."""
+    """Both record uploads (featuriser, bucket, target and both groupings as kernels) and the upload of the mapper's arrays leave
+    the slot bit-identical to what the host mappers and a stable sort on the CPU say: packed lists, buckets, targets, positions by
+    output bucket, pairs by row block.  Forward outputs are then bit-identical and a training step agrees to rounding."""
     from bullet_b200._lib import B200Error
+    from bullet_b200.net import featurise
 
     c = config(ci)
     w = synth.init_weights(c.desc, seed=ci)
     for n in (5000, 257, 1):   # several CTAs of the preparation kernels, a ragged last one, a single position
         desc = dataclasses.replace(c.desc, max_batch=5000)
         rec = synth.records(c.game, n, seed=161 + ci)
-        a, b = make_net(desc, 0, w), make_net(desc, 0, w)
+        batch = featurise(c.game, rec, desc)
+        want = slot_by_hand(desc, batch)
+        nets = [make_net(desc, 0, w) for _ in range(3)]
+        a, b, arrays = nets
         a.upload_records(1, c.game, rec)
         b.upload_records(1, c.game, rec, on_device=True)
-        sa, sb = a.slot_contents(1), b.slot_contents(1)
-        for k in sa:
-            assert np.array_equal(sa[k], sb[k]), (n, k)
-        assert np.array_equal(a.forward(1, n), b.forward(1, n))
+        arrays.upload(1, *batch)
+        for trained in (False, True):
+            for k in want:
+                for net in nets:
+                    assert np.array_equal(net.slot_contents(1)[k], want[k]), (n, k, trained)
+            out = a.forward(1, n)
+            assert np.array_equal(b.forward(1, n), out) and np.array_equal(arrays.forward(1, n), out)
+            for net in nets:
+                net.step(1, 0.0, 1.0 / n)  # (with what a training pass adds to the slot)
         a.step(1, 1e-3, 1.0 / n)
         b.step(1, 1e-3, 1.0 / n)
         assert abs(a.loss() - b.loss()) <= 1e-6 * abs(a.loss())
         wa, wb = a.tensors(0), b.tensors(0)
         for k in wa:  # identical inputs: what is left is the order of the floating-point reductions of two runs
             assert rel2(wb[k], wa[k]) <= 1e-5, (n, k)
-        a.close()
-        b.close()
+        for net in nets:
+            net.close()
     if ci == 0:   # a record with more pieces than slots is refused, as on the host path
         small = make_net(dataclasses.replace(c.desc, nnz=8, max_batch=64), 0, w)
         with pytest.raises(B200Error) as e:

@@ -204,6 +204,32 @@ def test_grouping_of_long_batches(oracle32, n):
     assert rc == 0 and np.array_equal(x, x_ref)
 
 
+@pytest.mark.parametrize("case", ["blocks-32", "blocks-33", "blocks-256", "blocks-257", "rows-32-last-layer", "list-of-64", "width-8"])
+def test_groupings_that_the_kernels_made(case):
+    """The positions by output bucket and the pairs by row block that lie on the device, for every way of grouping, before and
+    after a training pass: the sets and the order that a stable sort on the CPU gives."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights, slot_by_hand
+
+    desc, n = CASES[case]
+    for n in (n, 5000):
+        desc = dataclasses.replace(desc, max_batch=n)
+        batch = draw_batch(desc, n, seed=n)
+        want = slot_by_hand(desc, batch)
+        net = make_net(desc, 0, rich_weights(desc))
+        for _ in range(2):
+            net.upload(2, *batch)
+            got = net.slot_contents(2)
+            for k in want:
+                assert np.array_equal(got[k], want[k]), k
+            net.step(2, 0.0, 1.0 / n)
+            got = net.slot_contents(2)
+            for k in want:
+                assert np.array_equal(got[k], want[k]), k
+        net.close()
+
+
 def net_flat(net, kind):
     import torch
 
