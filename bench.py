@@ -456,7 +456,7 @@ def run_ours(args, rank, world, local_rank):
                 "d2h_bytes_per_step": 8 * world,  # loss and status word
                 "ms_per_step": e2e_s * 1e3 / args.steps,
                 "source": {"records": "raw 32-byte records; featuriser, packing and grouping as kernels on the copy stream",
-                           "records-host": "raw 32-byte records; featuriser and packing on the host cores",
+                           "records-host": "raw 32-byte records through b200_batch_upload_records, which prepares on the device as well",
                            "arrays": "index arrays made by the host mapper before the clock starts"}[args.e2e_source],
                 "loss_per_position": None if last_loss is None else last_loss / GLOBAL_BATCH},
         "gpu_launches": int(launches),

@@ -1,5 +1,5 @@
-// Per-record featurisers shared by the stand-alone mappers (host_pack.cpp) and the upload that
-// maps records straight into a pinned staging slot (net.cu).  No CUDA here.
+// Per-record featurisers of the stand-alone mappers (host_pack.cpp); bucket, target and king-bucket table also serve the
+// upload of raw records (net.cu), whose featuriser is a kernel (kernels_prep.cuh).  No CUDA here.
 //
 // Reference (jw1912/bullet): Chess768::map_features crates/bullet_lib/src/game/inputs/chess768.rs:20-30,
 // ChessBucketsMirrored crates/bullet_lib/src/game/inputs/chess_buckets.rs:57-88,

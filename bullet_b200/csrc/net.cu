@@ -1118,8 +1118,6 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     memset(net->h_loss, 0, 128);  // 8 floats, 4 status words, 4 x 4 fence words, the wait word
     for (auto& e : net->loss_ev) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
     {
-        constexpr int MM_unused = 0;
-        (void)MM_unused;
         auto set_dense = [&](int m) -> int {
             cudaError_t e = cudaSuccess;
             DISPATCH_M(m, e = set_dense_forward_smem<MM>());
@@ -1250,7 +1248,7 @@ int b200_net_set_option(b200_net* net, const char* key, int64_t value) {
     }
     if (!strcmp(key, "ft_bwd_grab")) {
         if (value < 0 || value > 64) return b200::fail(B200_ERR_ARG, "ft_bwd_grab must be in [0, 64]");
-        net->bwd_grab = (int)value;
+        net->bwd_grab = (int)value;  // (more than eight eighths: all of them, see tile_args)
         return 0;
     }
     if (!strcmp(key, "ft_once")) {

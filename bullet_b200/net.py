@@ -102,8 +102,8 @@ class Net:
     # -------------------------------------------------------------------- step
     def upload_records(self, slot: int, game: str, records: np.ndarray, scale: float = 400.0, blend: float = 0.5,
                        on_device: bool = False) -> None:
-        """Raw 32-byte records -> featurised, packed batch in the slot: one pass on all host cores, or
-        (`on_device`) 32 bytes per position copied and everything else done by kernels on the copy stream."""
+        """Raw 32-byte records -> featurised, packed batch in the slot: checked and copied on the host, everything else done by
+        kernels on the copy stream (`on_device` picks one of two entry points that do the same)."""
         records = np.ascontiguousarray(records)
         code = {"chess768": 0, "chess_buckets": 1, "ataxx147": 2}[game]
         layout = np.asarray(KING_BUCKETS_16, dtype=np.int32) if code == 1 else None
@@ -111,7 +111,8 @@ class Net:
         _lib.check(fn(self._h, slot, _p(records), len(records), code, _p(layout) if layout is not None else None, scale, blend))
 
     def slot_contents(self, slot: int) -> dict:
-        """Debug/inspection: what the slot holds on the device (packed lists, buckets, targets, the two orders)."""
+        """Debug/inspection: what the slot holds on the device: packed lists, buckets, targets, positions by output bucket and
+        pairs by row block (ascending inside a group)."""
         count = ctypes.c_int32()
         _lib.check(self.lib.b200_slot_read(self._h, slot, None, None, None, None, None, None, ctypes.byref(count)))
         n, nnz = count.value, self.desc.nnz

@@ -99,7 +99,7 @@ int b200_net_destroy(b200_net* net);
 /* Tuning switches (no counterpart in the reference; every one has a measured default):
  *   "ft_mode" / "ft_fwd_mode" / "ft_bwd_mode"  B200_FT_*; "ft_bwd_wide" 0 = two 512-thread backward CTAs per SM;
  *   "ft_once" accepted, without effect (one form of loads is left);
- *   "ft_bwd_grab" eighths of a unit's row pieces that the tiled backward deals to its warps in advance (0 = default);
+ *   "ft_bwd_grab" eighths of a unit's row pieces that the tiled backward deals to its warps in advance (0 = default, more than 8 counts as 8);
  *   "exchange_bulk" 1 = the peer exchange moves gradients and weights with bulk asynchronous copies;
  *   "overlap_ctas", "overlap_mode", "exchange_ctas", "exchange_wait_ms", "exchange_step", "manual_grad_zero": see the
  *   data-parallel entry points below. */
@@ -145,30 +145,29 @@ int b200_batch_upload(b200_net* net, int slot, const int32_t* stm, const int32_t
                       const float* targets, int32_t n);
 /* The same from raw 32-byte position records: the featuriser (`game`), MaterialCount<n_out_buckets>
  * (crates/bullet_lib/src/game/outputs.rs:24-31; networks with output buckets take chess records) and
- * the target blend of ValueTrainerState::make_mapper (crates/bullet_lib/src/value.rs:77-117) run on
- * all host cores and write the packed lists straight into the pinned staging block.  `layout32` is the
- * king-bucket layout of ChessBucketsMirrored (32 entries), NULL for the other games. */
+ * the target blend of ValueTrainerState::make_mapper (crates/bullet_lib/src/value.rs:77-117).  The host checks the
+ * records while it copies them into the pinned staging block (and, until a scale has seen 65536 of them, forms their
+ * targets); everything else runs as kernels on the library's copy stream, beside a step that is still computing.  Nothing
+ * is read back: the call returns when everything is enqueued.  The slot ends up with the lists, buckets and targets that
+ * the stand-alone mappers (b200_map_*, b200_material_count, b200_make_targets) and b200_batch_upload give.  `layout32` is
+ * the king-bucket layout of ChessBucketsMirrored (32 entries), NULL for the other games.  What it replaces in the
+ * reference: the per-position mapper closure run by the loader threads (crates/trainer/src/model/inputs.rs:86-109) plus
+ * the copy of its five arrays. */
 #define B200_GAME_CHESS768 0
 #define B200_GAME_CHESS_BUCKETS_MIRRORED 1
 #define B200_GAME_ATAXX147 2
 int b200_batch_upload_records(b200_net* net, int slot, const void* records, int32_t n, int32_t game, const int32_t* layout32,
                               float scale, float blend);
 
-/* The same with the preparation on the DEVICE: the raw records (32 bytes per position) are copied and a kernel runs
- * the featuriser, the output bucket and the target blend; two more group the positions by output bucket and the
- * (position, perspective) pairs by table row block, in the same stable order the host path produces.  The slot
- * ends up bit-identical to b200_batch_upload_records' (lists, buckets, targets, both orders), so training results
- * are identical too.  Nothing is read back: the call returns when everything is enqueued, and it
- * runs on the library's copy stream, beside a step that is still computing.  What it replaces in the
- * reference: the per-position mapper closure of ValueTrainerState::make_mapper (crates/bullet_lib/src/value.rs:77-117)
- * run by the loader threads (crates/trainer/src/model/inputs.rs:86-109) plus the copy of its five arrays.
- * At most 256 output buckets. */
+/* The same under an earlier name: it prepared on the device when b200_batch_upload_records still did so on the host. */
 int b200_batch_upload_records_gpu(b200_net* net, int slot, const void* records, int32_t n, int32_t game, const int32_t* layout32,
                                   float scale, float blend);
 
 /* Debug/inspection: copies what a slot holds on the device to the host (any pointer may be NULL): the packed index
  * lists [n][nnz], buckets [n], targets [n], the positions grouped by output bucket [n] and the (position,
- * perspective) pairs (id = 2 * position + perspective) grouped by row block [2n]; *n = positions in the slot. */
+ * perspective) pairs (id = 2 * position + perspective) grouped by row block [2n], both in ascending order inside a group
+ * (the kernels visit the pairs of a block in the order of their lists' lengths); *n = positions in the slot.  Waits for
+ * the streams of the network. */
 int b200_slot_read(b200_net* net, int slot, uint16_t* stm, uint16_t* nstm, int32_t* buckets, float* targets, int32_t* order,
                    int32_t* pair_order, int32_t* n);
 
