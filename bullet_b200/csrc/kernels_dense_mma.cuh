@@ -343,8 +343,8 @@ __host__ __device__ constexpr size_t wgrad_table_words(size_t i) { return i * (M
 // pre-activation gradient (also as the operand of its weight gradient), weight gradients of the small layers and the first
 // layer's bias gradient (kept in registers until the bucket changes).  A CTA takes a
 // run of tiles, a warp eight of a tile's 32 positions: four lanes per position, each with a quarter of the second layer's 32
-// rows (zero past the last); for the weight gradients a lane is a row.  Bound by latency: 37 us at 131072 positions
-// (64 MB of parts), 12 at 16384.
+// rows (zero past the last); for the weight gradients a lane is a row.  Bound by latency: 60 us at 131072 positions
+// (64 MB of parts), 17 at 16384, from a cold cache.
 // grid = up to kSmallCtas per SM, block = 128.
 constexpr int kSmallThreads = 128, kSmallCtas = 4;
 template <int M1>
