@@ -44,6 +44,7 @@ struct DenseArgs {
     int want_grad;
     unsigned long long* stamp;  // as in FtArgs
     int* gave_up;               // pinned word, raised if a wait for copies runs out
+    unsigned* gmax;             // see FtArgs
     // gradient tensors (of the kernels that form them on the way)
     float* gW[3];
     float* gB[3];
@@ -282,6 +283,7 @@ __global__ void __launch_bounds__(256, 2) dense_dx_kernel(DenseArgs a, float* dx
 #pragma unroll
         for (int r = 0; r < M1; r++) g[j][r] = a.dz[0][(size_t)pos[j] * M1 + r];
     const int nchunks = (a.K1 + kDenseChunk - 1) / kDenseChunk;
+    unsigned largest = 0;
     dense_stage_chunk<M1>(a, k, 0, wbuf[0]);
     for (int ch = 0; ch < nchunks; ch++) {
         if (ch + 1 < nchunks) dense_stage_chunk<M1>(a, k, ch + 1, wbuf[(ch + 1) & 1]);
@@ -298,12 +300,16 @@ __global__ void __launch_bounds__(256, 2) dense_dx_kernel(DenseArgs a, float* dx
                     float s = 0.f;
 #pragma unroll
                     for (int r = 0; r < M1; r++) s += w[r] * g[j][r];
-                    if (j < npos && c < a.K1) dx[(size_t)pos[j] * a.K1 + c] = s;
+                    if (j < npos && c < a.K1) {
+                        dx[(size_t)pos[j] * a.K1 + c] = s;
+                        largest = max(largest, magnitude(s));
+                    }
                 }
             }
         }
         __syncthreads();
     }
+    raise_magnitude(a.gmax, largest);
 }
 
 // Weight and bias gradient of one dense layer: gW[c][k][r] += sum_b [k_b == k] dY[b][r] * X[b][c],

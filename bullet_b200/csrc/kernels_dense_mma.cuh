@@ -615,6 +615,7 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_dx_mma_kernel(De
                 }
     };
     fetch(warp);
+    unsigned largest = 0;
     for (int grp = warp; grp < groups; grp += 8) {
         uint32_t b[S][2][3][NB];
 #pragma unroll
@@ -636,10 +637,13 @@ __global__ void __launch_bounds__(256, (M1 > 16 ? 1 : 2)) dense_dx_mma_kernel(De
                 for (int j = 0; j < 2; j++) mma_split(c[j], dz[m][s], b[s][j]);
 #pragma unroll
             for (int h = 0; h < 2; h++)
-                if (in && 16 * m + 8 * h + g < t.y)
+                if (in && 16 * m + 8 * h + g < t.y) {
                     *reinterpret_cast<float4*>(row[2 * m + h] + grp * kMmaCols) = make_float4(c[0][2 * h], c[0][2 * h + 1], c[1][2 * h], c[1][2 * h + 1]);
+                    largest = max(max(largest, max(magnitude(c[0][2 * h]), magnitude(c[0][2 * h + 1]))), max(magnitude(c[1][2 * h]), magnitude(c[1][2 * h + 1])));
+                }
         }
     }
+    raise_magnitude(a.gmax, largest);
 }
 
 // Weight gradient of the first layer: gW[c][k][r] += sum_b [k_b == k] dz1[b][r] * x[b][c].  Positions contract, sixteen

@@ -48,6 +48,7 @@ struct OneArgs {
     float* gB;
     int want_grad, units_per_run;
     int* gave_up;          // pinned word, raised if a wait runs out
+    unsigned* gmax;        // see FtArgs
     unsigned long long* stamp;
 };
 
@@ -106,6 +107,7 @@ __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __grid_con
     const int width = min(kOneThreads, cols4), groups = kOneThreads / width, col = tid % width, group = tid / width;
     float4 acc[4];
     float g_bias = 0.f, my_loss = 0.f;
+    unsigned largest_dout = 0, largest_w = 0;
 #pragma unroll
     for (int i = 0; i < 4; i++) acc[i] = make_float4(0, 0, 0, 0);
     int cur = -1;
@@ -148,7 +150,11 @@ __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __grid_con
                 flush();
                 cur = k;
                 if (tid == 0) s_bias = __ldg(a.B + k);
-                for (int c = tid; c < cols4; c += kOneThreads) reinterpret_cast<float4*>(s_w)[c] = __ldg(reinterpret_cast<const float4*>(a.W + (size_t)k * a.K1) + c);
+                for (int c = tid; c < cols4; c += kOneThreads) {
+                    const float4 w = __ldg(reinterpret_cast<const float4*>(a.W + (size_t)k * a.K1) + c);
+                    reinterpret_cast<float4*>(s_w)[c] = w;
+                    largest_w = max(max(largest_w, max(magnitude(w.x), magnitude(w.y))), max(magnitude(w.z), magnitude(w.w)));
+                }
                 __syncthreads();
             }
             const float target = a.want_grad && in_row == 0 && row < rows ? __ldg(a.targets + s_pos[stage][row]) : 0.f;  // (arrives under the sums)
@@ -190,6 +196,7 @@ __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __grid_con
                         dout = (diff + diff) * (s * (1.f - s));
                         a.dout[b] = dout;
                         a.kept_bucket[b] = k;
+                        largest_dout = max(largest_dout, magnitude(dout));
                     }
                 }
                 s_dout[row] = dout;
@@ -222,6 +229,8 @@ __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __grid_con
     }
     flush();
     if (a.want_grad) {
+        raise_magnitude(a.gmax, largest_dout);
+        raise_magnitude(a.gmax ? a.gmax + 1 : nullptr, largest_w);
         if (tid < 32) s_loss[tid] = tid < P ? my_loss : 0.f;
         __syncthreads();
         if (warp == 0) {

@@ -63,11 +63,15 @@ struct FtArgs {
     unsigned long long* stamp_end;  // forward: the step's last stamp, cleared
     float4* zero;     // forward: the gradient buffer, where this kernel clears it (zero4 float4s), or null
     long long zero4;
+    unsigned* gmax;   // the largest |dx| (or |dout|, and |w1| behind it) of the step, as bits: the forward clears them, the dense
+                      // kernels raise them, ft_backward_mma_kernel scales by them
+    int* gave_up;     // pinned word, raised if a wait inside a kernel runs out
 };
 
 __device__ __forceinline__ void ft_step_begin(const FtArgs& a) {
     step_begin(a.stamp);
     if (a.stamp_end && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) *a.stamp_end = 0;
+    if (a.gmax && threadIdx.x < 2 && blockIdx.x == 0 && blockIdx.y == 0) a.gmax[threadIdx.x] = 0u;
     if (a.zero) {  // nothing adds to it before the kernels that follow
         const long long per = (long long)gridDim.x * gridDim.y * blockDim.x;
         for (long long i = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; i < a.zero4; i += per) a.zero[i] = make_float4(0, 0, 0, 0);

@@ -26,6 +26,15 @@ __device__ __forceinline__ void step_begin(unsigned long long* stamp) {
     if (stamp && threadIdx.x == 0 && blockIdx.x == 0 && blockIdx.y == 0) *stamp = clock_ns();
 }
 
+// The largest magnitude of a pass, kept as the bits of |v| in one word: these order as the magnitudes do, infinity above every
+// number and NaN above infinity.  A warp adds its own to the word, if there is one and it holds less.
+__device__ __forceinline__ unsigned magnitude(float v) { return __float_as_uint(v) & 0x7fffffffu; }
+__device__ __forceinline__ void raise_magnitude(unsigned* word, unsigned own) {
+    if (!word) return;
+    own = __reduce_max_sync(0xffffffffu, own);
+    if ((threadIdx.x & 31) == 0 && own > __ldcg(word)) atomicMax(word, own);
+}
+
 template <class... Params, class... Args>
 cudaError_t launch_step(bool chained, void (*kernel)(Params...), dim3 grid, int block, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t config{};

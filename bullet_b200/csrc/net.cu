@@ -31,6 +31,7 @@
 #include "kernels_dense_mma.cuh"
 #include "kernels_dense_one.cuh"
 #include "kernels_ft.cuh"
+#include "kernels_ft_mma.cuh"
 #include "kernels_opt.cuh"
 #include "kernels_prep.cuh"
 #include "host_map.h"
@@ -76,6 +77,7 @@ struct Slot {
     int n = 0;
     int n_dtiles = 0;  // CTA tiles of the dense kernels: as many as there can be, the rest are empty
     bool wide = true;                 // shape of the tiled backward that its chunks were cut for
+    bool mma = false;                 // ... or for ft_backward_mma_kernel
     int n_chunks = 0, chunk_len = 0;  // the same for the chunks of the tiled FT backward held in off_chunks, and their size
     int expect_grid = 0;              // grid size the per-block CTA counts in off_bexpect were made for
     // derived from the indices alone, so built once per upload on the copy stream (or on first use):
@@ -132,6 +134,7 @@ struct b200_net {
     Slot slots[B200_NUM_SLOTS];
     int ft_fwd_mode = B200_FT_AUTO, ft_bwd_mode = B200_FT_AUTO;
     bool bwd_wide = true;  // shape of the tiled backward (see kChunkMost)
+    bool bwd_products = true;  // small tables: the product of bytes instead of the walk over row lists
     int exchange_bulk = 0;  // the peer exchange moves gradients and weights with bulk asynchronous copies (measured no faster)
     int bwd_grab = 0;  // eighths of a unit's pieces that the tiled backward deals out in advance (0: the default)
     int wide_chunk = 0;    // the largest chunk of the 1024-thread backward that fits into shared memory
@@ -248,6 +251,12 @@ struct b200_net {
     bool keep_root() const { return dense_one() && d.ft_act == B200_ACT_SCRELU; }
     // first dense layers of four and more rows per bucket run on the tensor pipe
     bool dense_mma() const { return d.dense_out[0] >= 4; }
+    // Which batches ft_backward_mma_kernel takes: all of a table whose rows fit into one tile, unless the backward has to announce
+    // finished row blocks or was asked for by another shape.  Measured, walk / products in us, 147 rows: 512 x 256 14.5 / 8.8,
+    // 2048 x 256 14.9 / 12.7, 32768 x 64 35 / 30, 32768 x 256 105 / 40, 32768 x 1024 398 / 115 (positions x columns); 384 rows of
+    // which 27 are active, 32768 x 1024: 398 / 150.  Larger blocks in parts (768 rows, 17 active) lose: 16384 x 2048 282 / 420.
+    bool bwd_mma() const { return tiled_ok && bwd_wide && bwd_products && !overlap_mode && block_rows < b200::kMmaTileRows; }
+    unsigned* gmax = nullptr;  // see FtArgs
 };
 
 namespace {
@@ -409,9 +418,22 @@ void launch_ft_backward_tiled(const b200::FtArgs& a, const b200::TileArgs& t, bo
         b200::launch_step(chained, b200::ft_backward_tiled_kernel<PW, 512, false, ONE>, grid, 512, smem, stream, a, t);
 }
 
+template <bool PW, bool ONE>
+void launch_ft_backward_mma(b200_net* net, const b200::FtArgs& a, const b200::TileArgs& t, int grid) {
+    const auto launch = [&](auto* kernel) {
+        b200::launch_step(net->chained, kernel, grid, b200::kMmaThreads, b200::ft_mma_smem(b200::ft_mma_rows(t.block_rows)), net->stream, a, t);
+    };
+    if constexpr (!PW)
+        if (a.act != B200_ACT_CRELU) return launch(b200::ft_backward_mma_kernel<PW, ONE, true>);
+    launch(b200::ft_backward_mma_kernel<PW, ONE, false>);
+}
+
 template <bool PW>
-int launch_ft_backward(b200_net* net, const b200::FtArgs& a, const b200::TileArgs& t, bool tiled, int grid) {
-    if (tiled) {
+int launch_ft_backward(b200_net* net, const Slot& s, const b200::FtArgs& a, const b200::TileArgs& t, bool tiled, int grid) {
+    if (tiled && s.mma) {
+        if (net->dense_one()) launch_ft_backward_mma<PW, true>(net, a, t, grid);
+        else launch_ft_backward_mma<PW, false>(net, a, t, grid);
+    } else if (tiled) {
         const size_t smem = b200::ft_bwd_smem(t.block_rows, a.nnz, t.chunk_len);
         const bool wide = t.wide;
         if (net->dense_one()) launch_ft_backward_tiled<PW, true>(a, t, wide, grid, smem, net->chained, net->stream);
@@ -503,7 +525,7 @@ int ft_forward_grid(const b200_net* net, const Slot& s) {
     return (int)std::max<long long>(1, std::min<long long>(net->sm_count, line / kMinItemPairs));
 }
 int ft_backward_grid(const b200_net* net, const Slot& s, bool beside_exchange) {
-    const long long units = (long long)net->nslabs * s.n_chunks;
+    const long long units = (long long)net->nslabs * s.n_chunks * (s.mma ? 2 : 1);
     const int per_sm = s.wide ? 1 : 2;
     const int sms = net->sm_count - (beside_exchange ? std::min(net->overlap_ctas, net->sm_count - 1) : 0);
     return (int)std::max<long long>(1, std::min<long long>((long long)sms * per_sm, units));
@@ -534,6 +556,8 @@ b200::FtArgs ft_args(b200_net* net, const Slot& s) {
     a.dout = net->dz[0];
     a.out_bucket = net->kept_bucket;
     a.stamp = nullptr;
+    a.gmax = net->gmax;
+    a.gave_up = net->h_gave_up;
     a.g_table = net->G + net->find("l0w")->off;
     a.g_bias = net->G + net->find("l0b")->off;
     return a;
@@ -558,8 +582,8 @@ b200::TileArgs tile_args(b200_net* net, const Slot& s, bool backward) {
     t.chunk_len = s.chunk_len;
     t.wide = s.wide;
     t.grab = net->bwd_grab > 0 ? std::min(8, net->bwd_grab) : 6;
-    t.ent_cap = b200::ft_bwd_ent_cap(net->block_rows, net->d.nnz, s.chunk_len);
-    t.start_cap = b200::ft_bwd_start_cap(net->block_rows, net->d.nnz, s.chunk_len);
+    t.ent_cap = s.mma ? b200::ft_mma_ent_cap(net->block_rows) : b200::ft_bwd_ent_cap(net->block_rows, net->d.nnz, s.chunk_len);
+    t.start_cap = s.mma ? b200::kStepHead : b200::ft_bwd_start_cap(net->block_rows, net->d.nnz, s.chunk_len);
     if (backward && net->sig_on) {
         t.sig.done_count = net->done_count;
         t.sig.done_expect = s.dev<int>(s.off_bexpect);
@@ -598,6 +622,7 @@ b200::DenseArgs dense_args(b200_net* net, const Slot& s, bool want_grad) {
     a.partial = net->dense_partial;
     a.dz_frag = net->dz_frag;
     a.gave_up = net->h_gave_up;
+    a.gmax = net->gmax;
     a.a1 = net->a1;
     a.a2 = net->a2;
     a.out = net->out;
@@ -709,9 +734,10 @@ void cut_dense(b200_net* net, Slot& s) {
 void cut_ft(b200_net* net, Slot& s) {
     if (!net->tiled_ok) return;
     s.wide = net->bwd_wide;
-    s.chunk_len = net->bwd_chunk(s.n);
+    s.mma = net->bwd_mma();
+    s.chunk_len = s.mma ? b200::kStepPairs : net->bwd_chunk(s.n);
     s.n_chunks = most_chunks(net, s.n, s.chunk_len);
-    s.expect_grid = ft_backward_grid(net, s, net->overlap_mode);
+    s.expect_grid = s.mma ? 0 : ft_backward_grid(net, s, net->overlap_mode);
 }
 
 // Groups the slot's batch on `stream` (kernels_group.cuh); `counted`: the first pass has run with the featuriser.
@@ -746,8 +772,11 @@ int group_slot(b200_net* net, Slot& s, const b200::GroupArgs& g, bool counted, c
 }
 
 int build_csr(b200_net* net, Slot& s, cudaStream_t stream) {
-    b200::ft_csr_kernel<<<s.n_chunks, b200::kCsrThreads, b200::ft_csr_smem(net->block_rows, net->d.nnz, s.chunk_len), stream>>>(
-        ft_args(net, s), tile_args(net, s, true));
+    if (s.mma)
+        b200::ft_onehot_kernel<<<s.n_chunks, b200::kOnehotThreads, 0, stream>>>(tile_args(net, s, true));
+    else
+        b200::ft_csr_kernel<<<s.n_chunks, b200::kCsrThreads, b200::ft_csr_smem(net->block_rows, net->d.nnz, s.chunk_len), stream>>>(
+            ft_args(net, s), tile_args(net, s, true));
     LAUNCHED(net);
     s.csr_built = true;
     return 0;
@@ -800,6 +829,7 @@ int forward_dense(b200_net* net, Slot& s, bool want_grad) {
         a.want_grad = da.want_grad;
         a.stamp = da.stamp;
         a.gave_up = net->h_gave_up;
+        a.gmax = net->gmax;
         if (want_grad) net->w1_used = da.W1g, net->grad_n = s.n, net->dx_formed = false;
         const size_t smem = b200::one_smem(a.K1);
         const int units = a.ntiles * (b200::kDenseTile / b200::one_rows(a.K1)), slots = net->sm_count * std::max(1, std::min(4, (int)(220 * 1024 / smem)));
@@ -918,7 +948,9 @@ int preload_kernels(b200_net* net) {
     ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 512, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 512, true, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, true, false>);
     ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, false, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, false, false>);
     ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 512, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 512, false, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, false, false>);
-    ok = ok && load_kernel(b200::ft_csr_kernel);
+    ok = ok && load_kernel(b200::ft_csr_kernel) && load_kernel(b200::ft_onehot_kernel);
+    ok = ok && load_kernel(b200::ft_backward_mma_kernel<true, true, false>) && load_kernel(b200::ft_backward_mma_kernel<true, false, false>) && load_kernel(b200::ft_backward_mma_kernel<false, true, false>);
+    ok = ok && load_kernel(b200::ft_backward_mma_kernel<false, false, false>) && load_kernel(b200::ft_backward_mma_kernel<false, true, true>) && load_kernel(b200::ft_backward_mma_kernel<false, false, true>);
     ok = ok && load_kernel(b200::factoriser_merge_kernel) && load_kernel(b200::factoriser_grad_kernel);
     ok = ok && load_kernel(b200::adamw_flat_kernel) && load_kernel(b200::step_update_kernel) && load_kernel(b200::lookahead_kernel);
     ok = ok && load_kernel(b200::adamw_exchange_kernel<0>) && load_kernel(b200::adamw_exchange_kernel<2>);
@@ -1047,6 +1079,7 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     plan.add(&net->out, B);
     plan.add(&net->d_stamps, b200_net::kTimingRing * b200_net::kTimingEvents);
     plan.add(&net->d_status, b200_net::kLossRing);
+    if (net->tiled_ok && net->block_rows < b200::kMmaTileRows) plan.add(&net->gmax, 2);
     if (net->dense_mma()) {
         const size_t table = b200::mma_table_words(net->D1(), d.n_out_buckets, d.dense_out[0]);
         plan.add(&net->w1f, table);
@@ -1080,6 +1113,11 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
         room_for(b200::ft_bwd_chunk_narrow(d.nnz));
         for (int cp = net->wide_chunk; cp >= b200::kChunkLeast; cp -= 8) room_for(cp);
         room_for(net->wide_chunk);
+        if (R < b200::kMmaTileRows) {
+            const size_t steps = most_chunks(net, (int)B, b200::kStepPairs);
+            start_total = std::max(start_total, steps * b200::kStepHead);
+            ent_total = std::max(ent_total, steps * b200::ft_mma_ent_cap(R));
+        }
         for (auto& s : net->slots) {
             plan.add(&s.lists, 2 * B * ((d.nnz + 7) & ~7));
             plan.add(&s.csr_ent, ent_total);
@@ -1147,6 +1185,12 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
         e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, false, true>);
         e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, false, false>);
         e = e ? e : b200::allow_smem(b200::ft_csr_kernel);
+        e = e ? e : b200::allow_smem(b200::ft_backward_mma_kernel<true, true, false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_mma_kernel<true, false, false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_mma_kernel<false, true, false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_mma_kernel<false, false, false>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_mma_kernel<false, true, true>);
+        e = e ? e : b200::allow_smem(b200::ft_backward_mma_kernel<false, false, true>);
         if (e != cudaSuccess) return bail(b200::fail(B200_ERR_CUDA, "net_create: shared memory of the tiled kernels: %s", cudaGetErrorString(e)));
     }
     cudaFuncSetAttribute(b200::adamw_exchange_overlap_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b200::kOverlapSmem);
@@ -1253,6 +1297,10 @@ int b200_net_set_option(b200_net* net, const char* key, int64_t value) {
     }
     if (!strcmp(key, "ft_once")) {
         return 0;  // (no load of the tiled kernels gains from an L1 line any more: one form)
+    }
+    if (!strcmp(key, "ft_bwd_products")) {  // the same: 0 lets small tables walk row lists, too
+        net->bwd_products = value != 0;
+        return 0;
     }
     if (!strcmp(key, "ft_bwd_wide")) {  // takes effect for batches uploaded afterwards
         net->bwd_wide = value != 0;
@@ -1709,10 +1757,10 @@ int b200_backward_ft(b200_net* net, int slot, int part, int n_parts) {
             ta.first_block = part * per;
             ta.last_block = n_parts > 1 ? (part + 1) * per : net->nblocks;
             grid = ft_backward_grid(net, s, net->sig_on);
-            if (net->sig_on && grid != s.expect_grid)
+            if (net->sig_on && (s.mma || grid != s.expect_grid))
                 return b200::fail(B200_ERR_STATE, "backward_ft: the batch was uploaded before the exchange under the backward was switched on");
         }
-        int rc = d.pairwise ? launch_ft_backward<true>(net, fa, ta, tiled, grid) : launch_ft_backward<false>(net, fa, ta, tiled, grid);
+        int rc = d.pairwise ? launch_ft_backward<true>(net, s, fa, ta, tiled, grid) : launch_ft_backward<false>(net, s, fa, ta, tiled, grid);
         if (rc) return rc;
     }
     if (part == n_parts - 1) CK(cudaEventRecord(ev[4], net->stream));
@@ -2179,7 +2227,7 @@ static int step_chained(b200_net* net, Slot& s, int slot, float lr, float grad_f
         b200::TileArgs ta = tile_args(net, s, true);
         fa.stamp = net->stamp(3);
         const int grid = bwd_tiled ? ft_backward_grid(net, s, false) : 0;
-        int rc = d.pairwise ? launch_ft_backward<true>(net, fa, ta, bwd_tiled, grid) : launch_ft_backward<false>(net, fa, ta, bwd_tiled, grid);
+        int rc = d.pairwise ? launch_ft_backward<true>(net, s, fa, ta, bwd_tiled, grid) : launch_ft_backward<false>(net, s, fa, ta, bwd_tiled, grid);
         if (rc) return rc;
     }
     const bool lookahead = lookahead_due(net);

@@ -411,3 +411,80 @@ def test_nan_passes_through_the_first_dense_layer(dense):
         out = net.forward(0, n)
         assert np.array_equal(np.isnan(out), batch[2] == k)
         net.close()
+
+
+# rows, blocks, slots, width, pairwise, activation, dense layers, output buckets, positions, a row twice in a list
+PRODUCTS = {
+    "one-row": (1, 1, 1, 32, False, ACT_CRELU, (1,), 1, 3, False),
+    "rows-31": (31, 3, 20, 64, False, ACT_SCRELU, (1,), 4, 700, False),
+    "rows-32": (32, 1, 32, 40, False, ACT_CRELU, (8, 1), 2, 65, False),
+    "rows-147-ragged-width": (147, 1, 49, 72, False, ACT_CRELU, (1,), 1, 1000, False),
+    "rows-255": (255, 2, 64, 96, False, ACT_SCRELU, (4, 1), 1, 129, False),
+    "rows-256": (256, 1, 9, 64, False, ACT_CRELU, (1,), 3, 4000, False),
+    "rows-383": (383, 2, 32, 136, True, ACT_CRELU, (16, 32, 1), 8, 900, False),
+    "rows-383-one": (383, 1, 32, 64, True, ACT_CRELU, (1,), 1, 64, False),
+    "counts": (150, 2, 40, 96, False, ACT_CRELU, (1,), 2, 300, True),
+    "counts-pairwise": (300, 1, 64, 128, True, ACT_CRELU, (8, 1), 1, 150, True),
+    "sums-taken-out-on-the-way": (2, 1, 1, 8, False, ACT_CRELU, (1,), 1, 2600000, False),
+}
+
+
+@pytest.mark.parametrize("case", PRODUCTS)
+def test_products_of_bytes_are_no_further_from_64_bits_than_the_walk(case):
+    """The backward of small tables: the gradient of the table and the bias against the sums in 64 bits of the gradients at
+    the pre-activations, which follow from what the step kept.  Per sum one rounding of 2^-24 and per addend one to 2^-31 of the
+    largest gradient; the walk over lists rounds at every addition, so it is the bound, and 2^-24 where it happens to be exact."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    rows, blocks, nnz, ft_out, pairwise, act, dense, buckets, n, twice = PRODUCTS[case]
+    desc = dataclasses.replace(net_of(blocks, rows, ft_out, nnz, buckets, dense, act, pairwise), max_batch=n)
+    desc = dataclasses.replace(desc, ft_block_rows=rows if ft_out % 64 == 0 or blocks > 1 else 0)
+    if n > 100000:  # (the drawing of draw_batch sorts every list)
+        rng = np.random.default_rng(n)
+        stm, nstm = (rng.integers(0, rows, (n, 1)).astype(np.int32) for _ in range(2))
+        batch = (stm, nstm, np.zeros(n, np.int32), rng.random(n).astype(np.float32))
+    else:
+        batch = draw_batch(desc, n, seed=rows + n)
+    if twice:
+        for lists in batch[:2]:
+            lists[::3, 1] = lists[::3, 0]
+            lists[::3, -1] = lists[::3, 0]
+    w = rich_weights(desc)
+    error = {}
+    for products in (0, 1):
+        net = make_net(desc, 0, w)
+        net.set_option("ft_bwd_products", products)
+        net.upload(0, *batch)
+        net.step(0, 0.0, 1.0 / n)
+        net.loss()
+        g = net.tensors(kind=3)
+        x, dx = (net.activation(k, n * desc.dense_in0).reshape(n, 2, -1) for k in (0, 2))
+        if pairwise:
+            u = net.activation(1, n * 2 * ft_out).reshape(n, 2, 2, ft_out // 2)
+            pre = np.stack([dx * u[:, :, 1], dx * u[:, :, 0]], axis=2).astype(np.float64) * ((u > 0) & (u < 1))
+            pre = pre.reshape(n, 2, ft_out)
+        else:
+            slope = ((x > 0) & (x < 1)) * (2 * np.sqrt(x) if act == ACT_SCRELU else np.float32(1))
+            pre = dx.astype(np.float64) * slope
+        table = np.zeros((desc.n_inputs, ft_out))
+        for side in range(2):
+            index = batch[side]
+            for slot in range(nnz):
+                on = index[:, slot] >= 0
+                if n > 100000:
+                    for c in range(ft_out):
+                        table[:, c] += np.bincount(index[on, slot], pre[on, side, c], desc.n_inputs)
+                else:
+                    np.add.at(table, index[on, slot], pre[on, side])
+        bias = pre.sum((0, 1))
+        error[products] = [np.linalg.norm(g[k].astype(np.float64).reshape(ref.shape) - ref) / max(np.linalg.norm(ref), 1e-300)
+                           for k, ref in (("l0w", table), ("l0b", bias))]
+        print(case, "products" if products else "walk", error[products])
+        net.close()
+    # (both round the product at every pre-activation, 2^-24, which the reference has in common; which of several reductions into one
+    # sum comes first differs from run to run and moves the walk's error by a per cent)
+    assert error[1][0] <= max(1.05 * error[0][0], 2.0 ** -24)
+    # the bias: 40 to 136 sums of a few dozen fp32 parts that come in any order, either way; two such errors differ by less than twice
+    assert error[1][1] <= max(2 * error[0][1], 2.0 ** -24)
