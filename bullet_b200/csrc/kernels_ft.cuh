@@ -66,6 +66,7 @@ struct FtArgs {
     unsigned* gmax;   // the largest |dx| (or |dout|, and |w1| behind it) of the step, as bits: the forward clears them, the dense
                       // kernels raise them, ft_backward_mma_kernel scales by them
     int* gave_up;     // pinned word, raised if a wait inside a kernel runs out
+    int* status;      // gather forward only: where a feature outside its pair's block is reported, or null
 };
 
 __device__ __forceinline__ void ft_step_begin(const FtArgs& a) {
@@ -146,10 +147,18 @@ __device__ __forceinline__ void load_slots(const uint16_t* list, int nnz, int la
 // Takes index sets without block structure, and the small batches of networks that have it: staging the table's tiles
 // costs the tiled kernel the whole table whatever the batch holds, here only the rows of the batch are read.
 // Bound by L2 for large batches and by load latency (one pair per warp, four rows in flight) for small ones.  With a
-// factoriser the two rows of a feature are added as they arrive, so a small batch does not merge the table first.
-template <bool PAIRWISE>
+// factoriser the two rows of a feature are added as they arrive, so a small batch does not merge the table first; an instantiation
+// without one keeps more warps on an SM (operator, 2048 positions x 1024 columns, whole call: 63 us with the factoriser's registers, 54
+// without; eight rows in flight and fewer warps: 64).
+// pairs per CTA: one per warp while there are few, up to eight once that leaves two waves of eight CTAs per SM
+inline int gather_pairs(int n, int unit, int sms) {
+    const long long pieces = (long long)2 * n * ((unit + 127) / 128) / (8LL * 16 * sms);
+    return 8 * (int)(pieces < 1 ? 1 : pieces < 8 ? pieces : 8);
+}
+template <bool PAIRWISE, bool FACTOR>
 __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pairs_per_block) {
     ft_step_begin(a);
+    constexpr int U = 4;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int unit = PAIRWISE ? a.H / 2 : a.H;
     const int col = blockIdx.y * 128 + lane * 4;
@@ -171,26 +180,28 @@ __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pa
         if (a.block_rows > 0 && (mask[0] | mask[1])) {
             const uint32_t first = __shfl_sync(0xffffffffu, mask[0] ? slot[0] : slot[1], __ffs(mask[0] ? mask[0] : mask[1]) - 1);
             const uint32_t base = first / a.block_rows * a.block_rows;
+            const unsigned all0 = mask[0], all1 = mask[1];
             mask[0] &= __ballot_sync(0xffffffffu, slot[0] - base < (uint32_t)a.block_rows);
             mask[1] &= __ballot_sync(0xffffffffu, slot[1] - base < (uint32_t)a.block_rows);
+            if (a.status && lane == 0 && (mask[0] != all0 || mask[1] != all1)) *a.status = kStatusOutsideBlock;
         }
-        const uint32_t frow[2] = {a.factor ? slot[0] % a.factor_rows : 0u, a.factor ? slot[1] % a.factor_rows : 0u};
+        const uint32_t frow[2] = {FACTOR ? slot[0] % a.factor_rows : 0u, FACTOR ? slot[1] % a.factor_rows : 0u};
         float4 lo = make_float4(0, 0, 0, 0), hi = lo;
 #pragma unroll
         for (int half = 0; half < 2; half++) {
             unsigned m = mask[half];
-            while (m) {  // up to four independent row loads in flight, added in slot order
-                int s[4];
+            while (m) {  // up to U independent row loads in flight, added in slot order
+                int s[U];
                 int cnt = 0;
 #pragma unroll
-                for (int k = 0; k < 4; k++) {
+                for (int k = 0; k < U; k++) {
                     s[k] = m ? __ffs(m) - 1 : 0;
                     if (m) cnt++;
                     m &= m - 1;
                 }
-                float4 vlo[4], vhi[4], flo[4], fhi[4];
+                float4 vlo[U], vhi[U], flo[U], fhi[U];
 #pragma unroll
-                for (int k = 0; k < 4; k++) {
+                for (int k = 0; k < U; k++) {
                     const uint32_t f = __shfl_sync(0xffffffffu, slot[half], s[k]);
                     if (k < cnt && active) {
                         const float* row = a.table + (size_t)f * a.H;
@@ -198,9 +209,9 @@ __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pa
                         if (PAIRWISE) vhi[k] = __ldg(reinterpret_cast<const float4*>(row + unit + col));
                     }
                 }
-                if (a.factor) {
+                if constexpr (FACTOR) {
 #pragma unroll
-                    for (int k = 0; k < 4; k++) {
+                    for (int k = 0; k < U; k++) {
                         const uint32_t f = __shfl_sync(0xffffffffu, frow[half], s[k]);
                         if (k < cnt && active) {
                             const float* row = a.factor + (size_t)f * a.H;
@@ -209,14 +220,14 @@ __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pa
                         }
                     }
 #pragma unroll
-                    for (int k = 0; k < 4; k++)
+                    for (int k = 0; k < U; k++)
                         if (k < cnt && active) {
                             vlo[k] = add4(vlo[k], flo[k]);
                             if (PAIRWISE) vhi[k] = add4(vhi[k], fhi[k]);
                         }
                 }
 #pragma unroll
-                for (int k = 0; k < 4; k++)
+                for (int k = 0; k < U; k++)
                     if (k < cnt && active) {
                         lo = add4(lo, vlo[k]);
                         if (PAIRWISE) hi = add4(hi, vhi[k]);

@@ -394,11 +394,9 @@ int launch_ft_forward(b200_net* net, const b200::FtArgs& a, const b200::TileArgs
         CK(b200::launch_step(false, b200::ft_forward_tiled_kernel<PW>, grid, b200::kFwdThreads, b200::ft_fwd_smem(t.block_rows, t.list_len), net->stream, a, t));
     } else {
         const int unit = PW ? a.H / 2 : a.H;
-        // one pair per warp while there are few, up to eight once that leaves two waves of eight CTAs per SM
-        const long long pieces = (long long)2 * a.n * ((unit + 127) / 128);
-        const int pairs = 8 * (int)std::max<long long>(1, std::min<long long>(8, pieces / (8LL * 16 * net->sm_count)));
+        const int pairs = b200::gather_pairs(a.n, unit, net->sm_count);
         dim3 grid((2 * a.n + pairs - 1) / pairs, (unit + 127) / 128);
-        b200::ft_forward_gather_kernel<PW><<<grid, 256, 0, net->stream>>>(a, pairs);
+        (a.factor ? b200::ft_forward_gather_kernel<PW, true> : b200::ft_forward_gather_kernel<PW, false>)<<<grid, 256, 0, net->stream>>>(a, pairs);
     }
     LAUNCHED(net);
     return 0;
@@ -941,7 +939,7 @@ int preload_kernels(b200_net* net) {
     bool ok = true;
     DISPATCH_M(net->d.dense_out[0], ok = load_dense_kernels<MM>());
     ok = ok && load_kernel(b200::dense_regroup_kernel) && load_kernel(b200::dense_one_kernel<true>) && load_kernel(b200::dense_one_kernel<false>) && load_kernel(b200::dense_one_dx_kernel) && load_kernel(b200::copy_outputs_kernel) && load_kernel(b200::dense_fragments_kernel) && load_kernel(b200::dense_small_grads_kernel);
-    ok = ok && load_kernel(b200::ft_forward_gather_kernel<true>) && load_kernel(b200::ft_forward_gather_kernel<false>);
+    ok = ok && load_kernel(b200::ft_forward_gather_kernel<true, true>) && load_kernel(b200::ft_forward_gather_kernel<true, false>) && load_kernel(b200::ft_forward_gather_kernel<false, true>) && load_kernel(b200::ft_forward_gather_kernel<false, false>);
     ok = ok && load_kernel(b200::ft_backward_gather_kernel<true, true>) && load_kernel(b200::ft_backward_gather_kernel<true, false>) && load_kernel(b200::ft_backward_gather_kernel<false, true>) && load_kernel(b200::ft_backward_gather_kernel<false, false>);
     ok = ok && load_kernel(b200::ft_forward_tiled_kernel<true>) && load_kernel(b200::ft_forward_tiled_kernel<false>);
     ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, true, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, true, false>);

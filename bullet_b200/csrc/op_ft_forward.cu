@@ -131,12 +131,60 @@ int check_op(const b200_ft_op* op, const char* who) {
     return 0;
 }
 
-// Groups the pairs into `scratch` and runs the tiled forward; synchronises the stream and
+// Few positions are not worth grouping, nor the table's way through shared memory: the gather forward (one kernel, rows from L2)
+// takes them as they are.  Its time goes with the bytes of the rows, which the slots bound (about half of them are active).  Whole
+// call on a B200, gathered / grouped, us: 64 positions 20 to 24 / 36 to 230; king buckets x 1024 columns 1024 positions 38 / 58, 2048
+// (537 MB) 54 / 60, 4096 84 / 72; x 128 columns 8192 35 / 45, 16384 (537 MB) 50.5 / 52, pairwise x 2048 columns 1024 (537 MB) 71 / 81, 2048 106 / 89;
+// 768 rows x 128 columns 16384 (537 MB) 48 / 50, x 2048 columns 2048 77 / 60; 147 rows x 256 columns 8192 (822 MB) 54 / 69, x 2048 columns 512 40 / 59,
+// 2048 (1644 MB) 89 / 82.  Outputs that start on any float are for the tiled kernel.
+constexpr long long kGatherMost = 576LL << 20;
+bool few_positions(const b200_ft_op* op) {
+    if (((uintptr_t)op->bias | (uintptr_t)op->x | (op->pairwise ? (uintptr_t)op->u : 0)) & 15) return false;
+    return 8LL * op->n * op->nnz * op->ft_out <= kGatherMost;
+}
+
+int finish_op(cudaStream_t stream, const b200_ft_op* op, StatusWord& word, const int* status) {
+    int reported = 0;
+    if (!word.status) CK(cudaMemcpyAsync(&reported, status, sizeof reported, cudaMemcpyDeviceToHost, stream));
+    CK(cudaStreamSynchronize(stream));
+    word.finished = true;
+    if (word.status) reported = *reinterpret_cast<const volatile int*>(status);
+    if (reported & b200::kStatusOutsideBlock)
+        return b200::fail(B200_ERR_DATA, "a feature index fell outside the row block of its position (ft_block_rows=%d)", op->ft_block_rows);
+    return 0;
+}
+
+// Groups the pairs into `scratch` and runs the tiled forward, or the gather forward as it is; synchronises the stream and
 // reports a feature outside its block.  Allocates nothing.
 int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) {
     const int n = op->n, R = op->ft_block_rows, nblocks = op->n_inputs / R;
     StatusWord word(device, stream);
     int* status = word.status ? word.status : scratch + kStatusAt;
+    b200::FtArgs a{};
+    a.table = op->table;
+    a.bias = op->bias;
+    a.idx_stm = op->idx_stm;
+    a.idx_nstm = op->idx_nstm;
+    a.n = n;
+    a.nnz = op->nnz;
+    a.H = op->ft_out;
+    a.n_inputs = op->n_inputs;
+    a.act = op->ft_act;
+    a.x = op->x;
+    a.u = op->u;
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    if (few_positions(op)) {
+        a.block_rows = R;
+        a.status = status;
+        if (!word.status) CK(cudaMemsetAsync(status, 0, sizeof *status, stream));
+        const int unit = op->pairwise ? a.H / 2 : a.H, pairs = b200::gather_pairs(n, unit, sms);
+        const dim3 grid((2 * n + pairs - 1) / pairs, (unit + 127) / 128);
+        if (op->pairwise) b200::ft_forward_gather_kernel<true, false><<<grid, 256, 0, stream>>>(a, pairs);
+        else b200::ft_forward_gather_kernel<false, false><<<grid, 256, 0, stream>>>(a, pairs);
+        CK(cudaGetLastError());
+        return finish_op(stream, op, word, status);
+    }
     int* begin = scratch;
     int* info = scratch + kScratchHeader;
     int* pairs = info + align_ints((size_t)2 * n);
@@ -175,18 +223,6 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
     }
     CK(cudaGetLastError());
 
-    b200::FtArgs a{};
-    a.table = op->table;
-    a.bias = op->bias;
-    a.idx_stm = op->idx_stm;
-    a.idx_nstm = op->idx_nstm;
-    a.n = n;
-    a.nnz = op->nnz;
-    a.H = op->ft_out;
-    a.n_inputs = op->n_inputs;
-    a.act = op->ft_act;
-    a.x = op->x;
-    a.u = op->u;
     b200::TileArgs t{};
     t.block_rows = R;
     t.nslabs = op->ft_out / b200::kTileCols;
@@ -200,8 +236,6 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
     t.walk_warps = b200::ft_fwd_warps(R, t.list_len);
     const size_t smem = b200::ft_fwd_smem(R, t.list_len);
     // one CTA per SM, each taking an equal piece of the (block, slab, pair) work line
-    int sms = 0;
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
     const int ctas = (int)std::max<long long>(1, std::min<long long>(sms, (long long)2 * n * t.nslabs / 128));
     // the caller's arrays may start on any float: pieces of 8 and 16 bytes where they do so, else single floats
     const bool any = (((uintptr_t)op->bias | (uintptr_t)op->x | (op->pairwise ? (uintptr_t)op->u : 0)) & (op->pairwise ? 7 : 15)) != 0;
@@ -211,14 +245,7 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
     CK(b200::allow_smem(kernel));
     kernel<<<ctas, b200::kFwdThreads, smem, stream>>>(a, t);
     CK(cudaGetLastError());
-    int reported = 0;
-    if (!word.status) CK(cudaMemcpyAsync(&reported, status, sizeof reported, cudaMemcpyDeviceToHost, stream));
-    CK(cudaStreamSynchronize(stream));
-    word.finished = true;
-    if (word.status) reported = *reinterpret_cast<volatile int*>(status);
-    if (reported & b200::kStatusOutsideBlock)
-        return b200::fail(B200_ERR_DATA, "a feature index fell outside the row block of its position (ft_block_rows=%d)", R);
-    return 0;
+    return finish_op(stream, op, word, status);
 }
 
 }  // namespace

@@ -124,3 +124,18 @@ def test_op_ft_forward_on_arrays_that_start_on_any_float(oracle32, entry, name, 
         assert np.array_equal((half[:, :, 0] * half[:, :, 1]).reshape(n, -1), x_ref)
     for h in (x, u) if u else (x,):
         assert (h[0][:h[1]] == 7.0).all() and (h[0][h[1] + h[2]:] == 7.0).all()
+
+
+@pytest.mark.parametrize("past", [0, 1])
+@pytest.mark.parametrize("name,desc,game", CASES, ids=[c[0] for c in CASES])
+def test_op_ft_forward_on_either_side_of_the_gather(oracle32, name, desc, game, past):
+    """The most positions that are gathered without grouping, and one more: bit-exact, and a feature outside its block is reported."""
+    n = (576 << 20) // (8 * desc.nnz * desc.ft_out) + past
+    stm, nstm, w, table, x_ref = op_inputs(oracle32, desc, game, n, seed=65)
+    rc, x, _ = run_op("b200_op_ft_forward", desc, table, w["l0b"], stm, nstm, n)
+    assert rc == 0
+    assert np.array_equal(x, x_ref)
+    if desc.n_inputs > desc.ft_block_rows:
+        stm[n - 1, 1] = (stm[n - 1, 0] + desc.ft_block_rows) % desc.n_inputs
+        rc, _, _ = run_op("b200_op_ft_forward", desc, table, w["l0b"], stm, nstm, n)
+        assert rc == -4

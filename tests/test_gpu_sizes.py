@@ -425,7 +425,7 @@ PRODUCTS = {
     "rows-383-one": (383, 1, 32, 64, True, ACT_CRELU, (1,), 1, 64, False),
     "counts": (150, 2, 40, 96, False, ACT_CRELU, (1,), 2, 300, True),
     "counts-pairwise": (300, 1, 64, 128, True, ACT_CRELU, (8, 1), 1, 150, True),
-    "sums-taken-out-on-the-way": (2, 1, 1, 8, False, ACT_CRELU, (1,), 1, 2600000, False),
+    "sums-taken-out-on-the-way": (2, 1, 1, 32, False, ACT_CRELU, (1,), 1, 2600000, False),
 }
 
 
@@ -483,8 +483,8 @@ def test_products_of_bytes_are_no_further_from_64_bits_than_the_walk(case):
                            for k, ref in (("l0w", table), ("l0b", bias))]
         print(case, "products" if products else "walk", error[products])
         net.close()
-    # (both round the product at every pre-activation, 2^-24, which the reference has in common; which of several reductions into one
-    # sum comes first differs from run to run and moves the walk's error by a per cent)
-    assert error[1][0] <= max(1.05 * error[0][0], 2.0 ** -24)
-    # the bias: 40 to 136 sums of a few dozen fp32 parts that come in any order, either way; two such errors differ by less than twice
-    assert error[1][1] <= max(2 * error[0][1], 2.0 ** -24)
+    # Both round the product at every pre-activation, which the reference has in common, and both add fp32 parts in any order, a few of
+    # a sum here, dozens of the bias or of a batch that all CTAs share: of a few sums two such errors differ by less than twice, of
+    # thousands by a few per cent.
+    for mine, walk, sums in zip(error[1], error[0], (table.size, bias.size)):
+        assert mine <= max((1.05 if sums > 1000 else 2) * walk, 2.0 ** -24)
