@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __grid_con
                 for (int c = tid; c < cols4; c += kOneThreads) {
                     const float4 w = __ldg(reinterpret_cast<const float4*>(a.W + (size_t)k * a.K1) + c);
                     reinterpret_cast<float4*>(s_w)[c] = w;
-                    largest_w = max(max(largest_w, max(magnitude(w.x), magnitude(w.y))), max(magnitude(w.z), magnitude(w.w)));
+                    if (a.gmax) largest_w = max(max(largest_w, max(magnitude(w.x), magnitude(w.y))), max(magnitude(w.z), magnitude(w.w)));
                 }
                 __syncthreads();
             }
@@ -229,8 +229,10 @@ __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __grid_con
     }
     flush();
     if (a.want_grad) {
-        raise_magnitude(a.gmax, largest_dout);
-        raise_magnitude(a.gmax ? a.gmax + 1 : nullptr, largest_w);
+        if (a.gmax) {
+            raise_magnitude(a.gmax, largest_dout);
+            raise_magnitude(a.gmax + 1, largest_w);
+        }
         if (tid < 32) s_loss[tid] = tid < P ? my_loss : 0.f;
         __syncthreads();
         if (warp == 0) {

@@ -10,7 +10,7 @@
 // (sparse.rs:151-187).  Both forward kernels add rows in slot order, so their
 // pre-activations are bit-identical to the interpreter's fp32 result.
 //
-// Two families:
+// Two families (the backward of tables of few rows has a third form, kernels_ft_mma.cuh):
 //   *_gather : one warp per (position, perspective, 128-column chunk); rows come
 //              straight from the table (L2/HBM), gradients go out as 128-bit
 //              global reductions.  Works for any index set.
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pa
             mask[1] &= __ballot_sync(0xffffffffu, slot[1] - base < (uint32_t)a.block_rows);
             if (a.status && lane == 0 && (mask[0] != all0 || mask[1] != all1)) *a.status = kStatusOutsideBlock;
         }
-        const uint32_t frow[2] = {FACTOR ? slot[0] % a.factor_rows : 0u, FACTOR ? slot[1] % a.factor_rows : 0u};
+        const uint32_t frow[2] = {FACTOR && a.factor ? slot[0] % a.factor_rows : 0u, FACTOR && a.factor ? slot[1] % a.factor_rows : 0u};
         float4 lo = make_float4(0, 0, 0, 0), hi = lo;
 #pragma unroll
         for (int half = 0; half < 2; half++) {
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pa
                         if (PAIRWISE) vhi[k] = __ldg(reinterpret_cast<const float4*>(row + unit + col));
                     }
                 }
-                if constexpr (FACTOR) {
+                if (FACTOR && a.factor) {
 #pragma unroll
                     for (int k = 0; k < U; k++) {
                         const uint32_t f = __shfl_sync(0xffffffffu, frow[half], s[k]);

@@ -4,7 +4,7 @@
 // (ft_backward_tiled_kernel) adds 32 floats per clock and SM out of shared memory; the tensor pipe does 8192 multiply-adds of
 // bytes, zeros included.  With 27 of 147 rows active in every pair (ataxx) the dense product needs 22 times the walk's
 // operations in four digits at 256 times its rate, and no row lists.  Time of the backward with 147 rows and 32768 positions,
-// walk / product: 256 columns 105 / 40 us, 1024 columns 398 / 116 (b200_net::bwd_mma has the line between the two).
+// walk / product: 256 columns 105 / 40 us, 1024 columns 398 / 116 (b200_net::bwd_mma draws the line between the two).
 //
 // Numbers.  A gradient is rounded to a whole multiple q of the batch's unit, a power of two chosen so that |q| < 2^31 for the
 // largest gradient there can be (`gmax`), and q is split into signed bytes, q = d0 + 2^8 d1 + 2^16 d2 + 2^24 d3: four rows of the
@@ -43,25 +43,30 @@ __host__ __device__ inline size_t ft_mma_smem(int rows) { return 1024 + (size_t)
 // Byte of (row, k) in a tile of 128-byte rows with the 128-byte swizzle.
 __device__ __forceinline__ uint32_t swizzled(uint32_t row, uint32_t k) { return row * 128 + (((k >> 4) ^ (row & 7)) << 4) + (k & 15); }
 
-// Latency bound; beside the step before unless the batch is a network's first.
-constexpr int kOnehotThreads = 256;
+// Latency bound, one load deep; beside the step before unless the batch is a network's first.
+constexpr int kOnehotThreads = 1024;
 static __global__ void __launch_bounds__(kOnehotThreads) ft_onehot_kernel(TileArgs t) {
     __shared__ uint32_t seen[kMmaTileRows * 4];  // a bit per (row, pair)
     __shared__ int twice;
     const int4 chunk = t.chunks[blockIdx.x];
     if (chunk.z == 0) return;  // (the launch is sized from the batch size alone)
     const int c0 = chunk.y, cn = chunk.z, Q = t.list_len / 8;
+    static_assert(kOnehotThreads >= kStepPairs * 8, "a thread per eight slots: one load's latency");
+    const int pair = threadIdx.x / Q, q = threadIdx.x - pair * Q;
+    int len = 0, id = -1;
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (pair < cn) {
+        len = __ldg(&t.pairs[c0 + pair].y) - 8 * q;
+        v = __ldg(reinterpret_cast<const uint4*>(t.lists + (size_t)(c0 + pair) * t.list_len) + q);
+    }
+    if ((int)threadIdx.x < cn) id = __ldg(&t.pairs[c0 + threadIdx.x].x);
     for (int k = threadIdx.x; k < kMmaTileRows * 4; k += kOnehotThreads) seen[k] = 0;
     if (threadIdx.x == 0) twice = 0;
     __syncthreads();
-    for (int e = threadIdx.x; e < cn * Q; e += kOnehotThreads) {
-        const int pair = e / Q, q = e - pair * Q, len = __ldg(&t.pairs[c0 + pair].y) - 8 * q;
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(t.lists + (size_t)(c0 + pair) * t.list_len) + q);
-        const uint32_t w[4] = {v.x, v.y, v.z, v.w}, bit = 1u << (pair & 31);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w}, bit = 1u << (pair & 31);
 #pragma unroll
-        for (int h = 0; h < 8; h++)
-            if (h < len && (atomicOr(&seen[(h & 1 ? w[h >> 1] >> 16 : w[h >> 1] & 0xffffu) * 4 + (pair >> 5)], bit) & bit)) twice = 1;
-    }
+    for (int h = 0; h < 8; h++)
+        if (h < len && (atomicOr(&seen[(h & 1 ? w[h >> 1] >> 16 : w[h >> 1] & 0xffffu) * 4 + (pair >> 5)], bit) & bit)) twice = 1;
     if (threadIdx.x < 4) {
         const int held = min(32, max(0, cn - 32 * (int)threadIdx.x));
         seen[t.block_rows * 4 + threadIdx.x] = held == 32 ? ~0u : (1u << held) - 1u;
@@ -69,7 +74,7 @@ static __global__ void __launch_bounds__(kOnehotThreads) ft_onehot_kernel(TileAr
     __syncthreads();
     int* head = t.csr_start + (size_t)blockIdx.x * t.start_cap;
     if (threadIdx.x == 0) *reinterpret_cast<int4*>(head) = make_int4(twice, 0, 0, 0);
-    if (threadIdx.x < kStepPairs) head[4 + threadIdx.x] = (int)threadIdx.x < cn ? __ldg(&t.pairs[c0 + threadIdx.x].x) : -1;
+    if (threadIdx.x < kStepPairs) head[4 + threadIdx.x] = id;
     uint32_t* out = reinterpret_cast<uint32_t*>(t.csr_ent + (size_t)blockIdx.x * t.ent_cap);
     for (int k = threadIdx.x; k < t.ent_cap / 2; k += kOnehotThreads) {  // sixteen pairs of two rows a word
         const int owner = k / 4 % kMmaGroupThreads, row = owner / 8 + 16 * (k / (4 * kMmaGroupThreads) * 8 + k % 4 * 2), c = owner % 8;

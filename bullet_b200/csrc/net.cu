@@ -134,7 +134,7 @@ struct b200_net {
     Slot slots[B200_NUM_SLOTS];
     int ft_fwd_mode = B200_FT_AUTO, ft_bwd_mode = B200_FT_AUTO;
     bool bwd_wide = true;  // shape of the tiled backward (see kChunkMost)
-    bool bwd_products = true;  // small tables: the product of bytes instead of the walk over row lists
+    int bwd_products = -1;  // small tables: the product of bytes instead of the walk over row lists, always (1), never (0) or where it pays
     int exchange_bulk = 0;  // the peer exchange moves gradients and weights with bulk asynchronous copies (measured no faster)
     int bwd_grab = 0;  // eighths of a unit's pieces that the tiled backward deals out in advance (0: the default)
     int wide_chunk = 0;    // the largest chunk of the 1024-thread backward that fits into shared memory
@@ -251,11 +251,16 @@ struct b200_net {
     bool keep_root() const { return dense_one() && d.ft_act == B200_ACT_SCRELU; }
     // first dense layers of four and more rows per bucket run on the tensor pipe
     bool dense_mma() const { return d.dense_out[0] >= 4; }
-    // Which batches ft_backward_mma_kernel takes: all of a table whose rows fit into one tile, unless the backward has to announce
-    // finished row blocks or was asked for by another shape.  Measured, walk / products in us, 147 rows: 512 x 256 14.5 / 8.8,
-    // 2048 x 256 14.9 / 12.7, 32768 x 64 35 / 30, 32768 x 256 105 / 40, 32768 x 1024 398 / 115 (positions x columns); 384 rows of
-    // which 27 are active, 32768 x 1024: 398 / 150.  Larger blocks in parts (768 rows, 17 active) lose: 16384 x 2048 282 / 420.
-    bool bwd_mma() const { return tiled_ok && bwd_wide && bwd_products && !overlap_mode && block_rows < b200::kMmaTileRows; }
+    // Which batches of n positions ft_backward_mma_kernel takes: those with enough sums (positions x columns) of a table whose rows fit
+    // into one tile, unless the backward has to announce finished row blocks or was asked for by another shape.  Whole training
+    // pass with 147 rows, walk / products in us: 30000 x 64 191 to 199 / 188 to 195 and 2000 x 256 63 to 65 / 63 to 75 (no gain: the upload is
+    // as long), 9000 x 256 108 / 96, 65000 x 64 197 / 168, 2000 x 1984 133 / 104, 30000 x 960 640 / 414; the backward alone gains from 512
+    // positions on.  Larger blocks in parts (768 rows, 17 active) lose: backward of 16384 x 2048 282 / 420.
+    static constexpr long long kProductSums = 2LL << 20;
+    bool small_table() const { return tiled_ok && block_rows < b200::kMmaTileRows; }
+    bool bwd_mma(int n) const {
+        return small_table() && bwd_wide && !overlap_mode && (bwd_products > 0 || (bwd_products < 0 && (long long)n * d.ft_out >= kProductSums));
+    }
     unsigned* gmax = nullptr;  // see FtArgs
 };
 
@@ -416,21 +421,18 @@ void launch_ft_backward_tiled(const b200::FtArgs& a, const b200::TileArgs& t, bo
         b200::launch_step(chained, b200::ft_backward_tiled_kernel<PW, 512, false, ONE>, grid, 512, smem, stream, a, t);
 }
 
-template <bool PW, bool ONE>
-void launch_ft_backward_mma(b200_net* net, const b200::FtArgs& a, const b200::TileArgs& t, int grid) {
-    const auto launch = [&](auto* kernel) {
-        b200::launch_step(net->chained, kernel, grid, b200::kMmaThreads, b200::ft_mma_smem(b200::ft_mma_rows(t.block_rows)), net->stream, a, t);
-    };
-    if constexpr (!PW)
-        if (a.act != B200_ACT_CRELU) return launch(b200::ft_backward_mma_kernel<PW, ONE, true>);
-    launch(b200::ft_backward_mma_kernel<PW, ONE, false>);
+// the one of its forms that a network takes
+void (*ft_backward_mma(const b200_net* net))(b200::FtArgs, b200::TileArgs) {
+    const bool one = net->dense_one();
+    if (net->d.pairwise) return one ? b200::ft_backward_mma_kernel<true, true, false> : b200::ft_backward_mma_kernel<true, false, false>;
+    if (net->d.ft_act == B200_ACT_CRELU) return one ? b200::ft_backward_mma_kernel<false, true, false> : b200::ft_backward_mma_kernel<false, false, false>;
+    return one ? b200::ft_backward_mma_kernel<false, true, true> : b200::ft_backward_mma_kernel<false, false, true>;
 }
 
 template <bool PW>
 int launch_ft_backward(b200_net* net, const Slot& s, const b200::FtArgs& a, const b200::TileArgs& t, bool tiled, int grid) {
     if (tiled && s.mma) {
-        if (net->dense_one()) launch_ft_backward_mma<PW, true>(net, a, t, grid);
-        else launch_ft_backward_mma<PW, false>(net, a, t, grid);
+        b200::launch_step(net->chained, ft_backward_mma(net), grid, b200::kMmaThreads, b200::ft_mma_smem(b200::ft_mma_rows(t.block_rows)), net->stream, a, t);
     } else if (tiled) {
         const size_t smem = b200::ft_bwd_smem(t.block_rows, a.nnz, t.chunk_len);
         const bool wide = t.wide;
@@ -732,7 +734,7 @@ void cut_dense(b200_net* net, Slot& s) {
 void cut_ft(b200_net* net, Slot& s) {
     if (!net->tiled_ok) return;
     s.wide = net->bwd_wide;
-    s.mma = net->bwd_mma();
+    s.mma = net->bwd_mma(s.n);
     s.chunk_len = s.mma ? b200::kStepPairs : net->bwd_chunk(s.n);
     s.n_chunks = most_chunks(net, s.n, s.chunk_len);
     s.expect_grid = s.mma ? 0 : ft_backward_grid(net, s, net->overlap_mode);
@@ -946,9 +948,8 @@ int preload_kernels(b200_net* net) {
     ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 512, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 512, true, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, true, false>);
     ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, false, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, false, false>);
     ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 512, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 512, false, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, false, false>);
-    ok = ok && load_kernel(b200::ft_csr_kernel) && load_kernel(b200::ft_onehot_kernel);
-    ok = ok && load_kernel(b200::ft_backward_mma_kernel<true, true, false>) && load_kernel(b200::ft_backward_mma_kernel<true, false, false>) && load_kernel(b200::ft_backward_mma_kernel<false, true, false>);
-    ok = ok && load_kernel(b200::ft_backward_mma_kernel<false, false, false>) && load_kernel(b200::ft_backward_mma_kernel<false, true, true>) && load_kernel(b200::ft_backward_mma_kernel<false, false, true>);
+    ok = ok && load_kernel(b200::ft_csr_kernel);
+    if (net->small_table()) ok = ok && load_kernel(b200::ft_onehot_kernel) && load_kernel(ft_backward_mma(net));
     ok = ok && load_kernel(b200::factoriser_merge_kernel) && load_kernel(b200::factoriser_grad_kernel);
     ok = ok && load_kernel(b200::adamw_flat_kernel) && load_kernel(b200::step_update_kernel) && load_kernel(b200::lookahead_kernel);
     ok = ok && load_kernel(b200::adamw_exchange_kernel<0>) && load_kernel(b200::adamw_exchange_kernel<2>);
@@ -1077,7 +1078,7 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
     plan.add(&net->out, B);
     plan.add(&net->d_stamps, b200_net::kTimingRing * b200_net::kTimingEvents);
     plan.add(&net->d_status, b200_net::kLossRing);
-    if (net->tiled_ok && net->block_rows < b200::kMmaTileRows) plan.add(&net->gmax, 2);
+    if (net->small_table()) plan.add(&net->gmax, 2);
     if (net->dense_mma()) {
         const size_t table = b200::mma_table_words(net->D1(), d.n_out_buckets, d.dense_out[0]);
         plan.add(&net->w1f, table);
@@ -1183,12 +1184,7 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
         e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, false, true>);
         e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, false, false>);
         e = e ? e : b200::allow_smem(b200::ft_csr_kernel);
-        e = e ? e : b200::allow_smem(b200::ft_backward_mma_kernel<true, true, false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_mma_kernel<true, false, false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_mma_kernel<false, true, false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_mma_kernel<false, false, false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_mma_kernel<false, true, true>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_mma_kernel<false, false, true>);
+        if (net->small_table()) e = e ? e : b200::allow_smem(ft_backward_mma(net));
         if (e != cudaSuccess) return bail(b200::fail(B200_ERR_CUDA, "net_create: shared memory of the tiled kernels: %s", cudaGetErrorString(e)));
     }
     cudaFuncSetAttribute(b200::adamw_exchange_overlap_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, b200::kOverlapSmem);
@@ -1296,8 +1292,9 @@ int b200_net_set_option(b200_net* net, const char* key, int64_t value) {
     if (!strcmp(key, "ft_once")) {
         return 0;  // (no load of the tiled kernels gains from an L1 line any more: one form)
     }
-    if (!strcmp(key, "ft_bwd_products")) {  // the same: 0 lets small tables walk row lists, too
-        net->bwd_products = value != 0;
+    if (!strcmp(key, "ft_bwd_products")) {  // the same
+        if (value < -1 || value > 1) return b200::fail(B200_ERR_ARG, "ft_bwd_products must be -1, 0 or 1");
+        net->bwd_products = (int)value;
         return 0;
     }
     if (!strcmp(key, "ft_bwd_wide")) {  // takes effect for batches uploaded afterwards
