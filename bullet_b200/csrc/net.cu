@@ -254,8 +254,10 @@ struct b200_net {
     // Which batches of n positions ft_backward_mma_kernel takes: those with enough sums (positions x columns) of a table whose rows fit
     // into one tile, unless the backward has to announce finished row blocks or was asked for by another shape.  Whole training
     // pass with 147 rows, walk / products in us: 30000 x 64 191 to 199 / 188 to 195 and 2000 x 256 63 to 65 / 63 to 75 (no gain: the upload is
-    // as long), 9000 x 256 108 / 96, 65000 x 64 197 / 168, 2000 x 1984 133 / 104, 30000 x 960 640 / 414; the backward alone gains from 512
-    // positions on.  Larger blocks in parts (768 rows, 17 active) lose: backward of 16384 x 2048 282 / 420.
+    // as long), 9000 x 256 108 / 96, 65000 x 64 197 / 168, 2000 x 1984 133 / 104, 30000 x 960 640 / 414.  The line is on the
+    // safe side: 2000 x 960, 91 / 78, lies just below it, and the backward alone gains from 300 positions on (13 / 9), which whole passes that
+    // small do not show beyond their spread (300 x 256 53 to 54 / 53 to 73, 300 x 1984 54 / 56).
+    // Larger blocks in parts (768 rows) lose: backward of 16384 x 2048 282 / 420.
     static constexpr long long kProductSums = 2LL << 20;
     bool small_table() const { return tiled_ok && block_rows < b200::kMmaTileRows; }
     bool bwd_mma(int n) const {
