@@ -323,8 +323,6 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ft_backward_mma_kernel(FtArgs 
             float* to = a.g_table + ((size_t)walk.block * t.block_rows + d) * a.H + col;
             const int own_rows = x_col < width ? t.block_rows - d : -1;
             float* bias = a.g_bias + col;
-            // a unit that this CTA alone has summed is stored (nobody else writes there), parts of one are added
-            const bool whole = n == walk.steps;
             wait(&done, unit_no & 1);
             __syncwarp();
             sums_fence_after();
@@ -345,15 +343,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ft_backward_mma_kernel(FtArgs 
 #pragma unroll
                 for (int g = 0; g < 8; g++)
                     if (n0 + 4 * g == own_rows && sum[g] != 0.f) atomicAdd(bias, sum[g]);
-                if (whole) {
+                // (added also where nobody else adds: a caller that clears the gradients itself may have several passes summed)
 #pragma unroll
-                    for (int g = 0; g < 8; g++, to += four)
-                        if (n0 + 4 * g < own_rows && sum[g] != 0.f) *to = sum[g];
-                } else {
-#pragma unroll
-                    for (int g = 0; g < 8; g++, to += four)
-                        if (n0 + 4 * g < own_rows && sum[g] != 0.f) atomicAdd(to, sum[g]);
-                }
+                for (int g = 0; g < 8; g++, to += four)
+                    if (n0 + 4 * g < own_rows && sum[g] != 0.f) atomicAdd(to, sum[g]);
             }
             sums_fence_before();
             mbar_arrive(&taken);

@@ -488,3 +488,29 @@ def test_products_of_bytes_are_no_further_from_64_bits_than_the_walk(case):
     # thousands by a few per cent.
     for mine, walk, sums in zip(error[1], error[0], (table.size, bias.size)):
         assert mine <= max((1.05 if sums > 1000 else 2) * walk, 2.0 ** -24)
+
+
+@pytest.mark.parametrize("products", [0, 1])
+@pytest.mark.parametrize("dense,pairwise", [((1,), False), ((8, 1), False), ((16, 32, 1), True)])
+def test_gradients_of_two_passes_add_up_where_the_caller_clears_them(products, dense, pairwise):
+    """Row blocks and columns enough that a CTA of the product backward has whole units to itself.  Two passes over one batch give twice
+    the gradient of one; the sums differ by the order of their fp32 parts (bound above)."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    n = 700
+    desc = dataclasses.replace(net_of(8, 31, 1024, 20, 2, dense, ACT_CRELU, pairwise), max_batch=n)
+    net = make_net(desc, 0, rich_weights(desc))
+    net.set_option("ft_bwd_products", products)
+    net.set_option("manual_grad_zero", 1)
+    net.upload(0, *draw_batch(desc, n, seed=5))
+    net.grad_zero_range(0, net.stat("flat_floats"))
+    net.backward(0)
+    once = net.tensors(kind=3)
+    net.backward(0)
+    twice = net.tensors(kind=3)
+    for k, g in once.items():
+        assert np.abs(g).max() > 0, k
+        assert np.abs(twice[k] - 2 * g).max() <= 2e-5 * np.abs(2 * g).max(), k
+    net.close()
