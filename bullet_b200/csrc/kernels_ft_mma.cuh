@@ -2,18 +2,21 @@
 //
 // The table gradient of a row block is  one_hot^T [rows x pairs]  times  gradients [pairs x columns].  The walk over row lists
 // (ft_backward_tiled_kernel) adds 32 floats per clock and SM out of shared memory; the tensor pipe does 8192 multiply-adds of
-// bytes, zeros included.  With 27 of 147 rows active in every pair (ataxx) the dense product needs 22 times the walk's
-// operations in four digits at 256 times its rate, and no row lists.  Time of the backward with 147 rows and 32768 positions,
-// walk / product: 256 columns 105 / 40 us, 1024 columns 398 / 116 (b200_net::bwd_mma draws the line between the two).
+// bytes, zeros included.  With 27 of 147 rows active in every pair (ataxx) the dense product needs 44 times the walk's
+// operations in eight digits at 256 times its rate, and no row lists.  Time of the backward with 147 rows and 32768 positions,
+// walk / product: 256 columns 87 / 41 us, 1024 columns 336 / 134 (b200_net::bwd_mma draws the line between the two).
 //
-// Numbers.  A gradient is rounded to a whole multiple q of the batch's unit, a power of two chosen so that |q| < 2^31 for the
-// largest gradient there can be (`gmax`), and q is split into signed bytes, q = d0 + 2^8 d1 + 2^16 d2 + 2^24 d3: four rows of the
-// product's first factor.  Sums of bytes are exact in the 32-bit accumulators (for kUnitStepsMost steps of 128 pairs), so all the
-// error comes from the rounding to the unit, at most 2^-31 of gmax a pair, and one rounding of each sum to fp32.  A gmax that is
-// not finite takes a slow path of fp32 atomics: infinities and NaN reach the rows they belong to and no others.
+// Numbers.  A gradient times a power of two, chosen so that the largest there can be (`gmax`) stays below 2^22, is a sum of eight
+// signed bytes down to units of 2^-37 (take_piece): eight rows of the product's first factor.  All 24 bits of a gradient down to
+// 2^-36 of the largest there can be are in these; what smaller ones have below the last digit is added to their rows by fp32
+// atomics.  Sums of bytes are exact in the 32-bit accumulators (for kUnitStepsMost steps of 128 pairs), so that a sum is rounded to
+// fp32 only when its eight digits are put together (four times) and when its parts of several CTAs are added.  (Four digits in
+// units of 2^-31 of the largest, 33 us at 256 columns, left columns of small output weights and positions of small errors fewer
+// bits than fp32 does: over seven decades of weights and six of errors single sums were off by up to 2e-2 of their magnitudes.)  A gmax that is not finite takes a slow path of fp32 atomics:
+// infinities and NaN reach the rows they belong to and no others.
 //
 // ft_onehot_kernel (a CTA per chunk of at most 128 pairs, once per batch) writes the one-hot factor as bits.  In
-// ft_backward_mma_kernel a CTA holds the sums of all rows x 32 columns x four digits in tensor memory.  Three groups of four
+// ft_backward_mma_kernel a CTA holds the sums of all rows x 32 columns x eight digits in tensor memory.  Three groups of four
 // warps, each with a stage of shared memory of its own, write the digits and the one-hot bytes of every third step; one thread
 // issues the products; its warpgroup takes finished sums out, puts the digits together and adds them to the gradient.
 #pragma once
@@ -25,10 +28,10 @@ namespace b200 {
 constexpr int kStepPairs = 128;  // pairs per step (and chunk): a row of 128 bytes in both factors
 constexpr int kMmaStages = 3, kMmaGroupThreads = 128;
 constexpr int kMmaThreads = (1 + kMmaStages) * kMmaGroupThreads;
-constexpr int kUnitCols = 32;  // gradient columns of a unit: with four digits the 128 lanes of tensor memory
-constexpr int kDigitBytes = 128 * kStepPairs;
+constexpr int kUnitCols = 32;  // gradient columns of a unit: with four digits the 128 lanes of tensor memory, so that eight take two tiles
+constexpr int kDigitBytes = 128 * kStepPairs;  // of a tile
 constexpr int kUnitStepsMost = 256;  // sums of digits stay below 2^22, where a pair holds a row 64 times below 2^28
-constexpr int kMmaTileRows = 384;    // most rows of the one-hot tile: three stages fit into shared memory, the sums into tensor memory
+constexpr int kMmaTileRows = 256;    // most rows of the one-hot tile: three stages fit into shared memory, both tiles' sums into tensor memory
 constexpr int kUnitFixed = 4;        // what taking out a unit's sums costs, in steps
 
 // Rows of the one-hot tile: the table's, one that all pairs hold (its sums are the bias gradient), and up to whole loads of sums.
@@ -38,7 +41,7 @@ __host__ __device__ inline int ft_mma_rows(int R) { return (R + 1 + 31) & ~31; }
 __host__ __device__ inline int ft_mma_words(int rows) { return (rows + 127) / 128; }  // 16-byte pieces per thread
 __host__ __device__ inline int ft_mma_ent_cap(int R) { return ft_mma_words(ft_mma_rows(R)) * kMmaGroupThreads * 8; }
 constexpr int kStepHead = 4 + kStepPairs;  // ints per chunk: whether a pair holds a row twice, three unused, the pair ids (-1: none)
-__host__ __device__ inline size_t ft_mma_smem(int rows) { return 1024 + (size_t)kMmaStages * (kDigitBytes + rows * kStepPairs); }
+__host__ __device__ inline size_t ft_mma_smem(int rows) { return 1024 + (size_t)kMmaStages * (2 * kDigitBytes + rows * kStepPairs); }
 
 // Byte of (row, k) in a tile of 128-byte rows with the 128-byte swizzle.
 __device__ __forceinline__ uint32_t swizzled(uint32_t row, uint32_t k) { return row * 128 + (((k >> 4) ^ (row & 7)) << 4) + (k & 15); }
@@ -103,15 +106,19 @@ __device__ __forceinline__ void products_done(uint64_t* bar) {  // arrives when 
 }
 __device__ __forceinline__ void sums_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void sums_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void load_sums32(uint32_t at, int (&v)[32]) {
+__device__ __forceinline__ void load_sums16(uint32_t at, int (&v)[16]) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, "
-        "%22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\ntcgen05.wait::ld.sync.aligned;"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
         : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]),
-          "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]),
-          "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+          "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
         : "r"(at)
         : "memory");
+}
+// what has been loaded is there (the words pass through, so that nothing reads them before)
+__device__ __forceinline__ void loaded_sums(int (&v)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]),
+                   "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])::"memory");
 }
 __device__ __forceinline__ bool mbar_try_wait_long(uint64_t* bar, uint32_t parity) {  // asleep for some us
     uint32_t ok;
@@ -215,12 +222,36 @@ __device__ __forceinline__ float ft_gradient_at(const FtArgs& a, int pair, int c
 // v where 0 < y < 1, else 0: for outputs of the clamp (bits of positive floats order as the floats do)
 __device__ __forceinline__ float inside_only(float y, float v) { return __float_as_uint(y) - 1u < 0x3f7fffffu ? v : 0.f; }
 
+// Its value times a power of two, of the products' operands: d is dx (or w1 x dout) times that power, y the activation output of the
+// column, for pairwise networks y and other those of the two sides.
+template <bool PAIRWISE, bool ONE, bool SQUARE>
+__device__ __forceinline__ float ft_scaled_gradient(float d, float y, float other, int side) {
+    if (PAIRWISE) return side ? inside_only(other, __fmul_rn(d, y)) : inside_only(y, __fmul_rn(d, other));
+    return SQUARE ? __fmul_rn(d, ft_act_bwd(ONE ? 3 : 2, y)) : inside_only(y, d);
+}
+
+// The digits of a scaled gradient, |v| < 2^22 - 2^15, from whole multiples of 1, 2^-22 and 2^-37: the sum with 1.5 x 2^23 of these is
+// rounded to one, which its low bits hold.  Returned: three, three and two low bytes of a digit each, with 0x80 added to the first
+// two (by 0x8080 more of the multiples) and 0x40 to the third; v becomes the rest.
+__device__ __forceinline__ uint32_t take_piece(float& v, int piece) {
+    const float shift = (12582912.f + 32896.f) / (piece == 0 ? 1.f : piece == 1 ? 4194304.f : 137438953472.f);
+    const float sum = __fadd_rn(v, shift);  // (never one operation with the product that v is)
+    v = __fsub_rn(v, __fsub_rn(sum, shift));
+    return __float_as_uint(sum);
+}
+// What the i-th digit counts.
+__device__ __forceinline__ float digit_weight(int i) {
+    const int bits = i < 3 ? 8 * i : i < 6 ? 8 * (i - 3) - 22 : 8 * (i - 6) - 37;
+    return __uint_as_float((uint32_t)(127 + bits) << 23);
+}
+
 // grid = one CTA per SM.  All waits are for the CTA's own warps and products, and bounded.
-// Bound by the latency of the groups' instructions: a step (128 pairs x 32 columns, 160 rows) takes 990 clocks, its products 320
-// of them; every warp of a group has some 800 instructions for it, 365 for the digits and 130 for the one-hot bytes.  (Lists of the set
-// bytes in shared memory, to set and to clear them, instead of writing the whole tile from bits: 52 instead of 40 us.  In more
-// parts than one, for blocks of 768 rows, the digits are made once for each, and it loses to the walk: 420 against 282 us at 16384 x
-// 2048, where the 64-byte pieces of a pairwise row cost as much again.)
+// Bound by the groups' instructions and the latency between them: a step (128 pairs x 32 columns, 160 rows) takes 2150 clocks, its
+// products 640 of them; half of the issue slots are taken.  The operands of a group's next step are loaded as soon as those of this
+// one have become digits: 41 us at 256 columns instead of 46 with the loads behind the step.  (Lists of the set bytes in shared
+// memory, to set and to clear them, instead of writing the whole tile from bits, in the form of four digits: 52 instead of 40 us.  In
+// more parts than one, for blocks of 768 rows, the digits are made once for each, and it loses to the walk: 420 against 282 us at
+// 16384 x 2048, where the 64-byte pieces of a pairwise row cost as much again.)
 template <bool PAIRWISE, bool ONE, bool SQUARE>
 __global__ void __launch_bounds__(kMmaThreads, 1) ft_backward_mma_kernel(FtArgs a, TileArgs t) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -233,7 +264,7 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ft_backward_mma_kernel(FtArgs 
     constexpr int kCols = PAIRWISE ? kUnitCols / 2 : kUnitCols;  // columns of x of a unit
     const int units = (width + kCols - 1) / kCols;
     unsigned char* base = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
-    const int stage_bytes = kDigitBytes + rows * kStepPairs;
+    const int stage_bytes = 2 * kDigitBytes + rows * kStepPairs;
     volatile int* dead = &dead_s;
     if (tid == 0) {
         for (int s = 0; s < kMmaStages; s++) mbar_init(&full[s], kMmaGroupThreads), mbar_init(&empty[s], 1);
@@ -255,11 +286,11 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ft_backward_mma_kernel(FtArgs 
     __syncthreads();
     sums_fence_after();
     const uint32_t sums = sums_at;
-    // The unit: gradients are multiples of 2^-k.
+    // Scaled by 2^k, no gradient is above 2^22 - 2^15.
     const unsigned m0 = __ldcg(a.gmax), m1 = ONE ? __ldcg(a.gmax + 1) : 0u;
     const float bound = __uint_as_float(m0) * (ONE ? __uint_as_float(m1) : 1.f) * (SQUARE ? 2.f : 1.f) * 1.015625f;
     const bool finite = m0 < 0x7f800000u && m1 < 0x7f800000u && bound < __uint_as_float(0x7f800000u);
-    const int k = min(120, 157 - (int)(__float_as_uint(bound) >> 23));
+    const int k = min(120, 148 - (int)(__float_as_uint(bound) >> 23));
     const float scale = __uint_as_float((uint32_t)(127 + k) << 23), unit = __uint_as_float((uint32_t)(127 - k) << 23);
 
     MmaWalk walk{piece[0].block, piece[0].unit, piece[0].step, finite && bound > 0.f ? piece[1].before - piece[0].before : 0, 0, 0};
@@ -290,11 +321,9 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ft_backward_mma_kernel(FtArgs 
         asm volatile("setmaxnreg.dec.sync.aligned.u32 104;");
         const int d = lane >> 3, at = ((lane & 7) - 2 * warp) & 7;
         const int c = 8 * warp + 4 * (at & 1) + (at >> 1);  // this lane's gradient column in the unit
-        const float mult_keep = d & 1 ? 256.f : 1.f, mult_got = d & 1 ? 1.f : 256.f;
-        const float by_keep = d & 2 ? unit * 65536.f : unit, by_got = d & 2 ? unit : unit * 65536.f;
-        const int n1 = min(256, rows), n2 = rows - n1;
-        const uint32_t form1 = byte_product(n1), form2 = byte_product(n2), step16 = stage_bytes >> 4;
-        const uint32_t digits0 = tile_low(smem_u32(base)), hot0 = tile_low(smem_u32(base + kDigitBytes));
+        const float by_high = digit_weight(d), by_low = digit_weight(4 + d);
+        const uint32_t form = byte_product(rows), step16 = stage_bytes >> 4;
+        const uint32_t digits0 = tile_low(smem_u32(base)), hot0 = tile_low(smem_u32(base + 2 * kDigitBytes));
         int stage = 0, unit_no = 0;
         uint32_t phase = 0;
         for (int n; walk.left > 0; walk.advance(t, units, n), unit_no++) {
@@ -309,8 +338,8 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ft_backward_mma_kernel(FtArgs 
                         sums_fence_after();
 #pragma unroll
                         for (int q = 0; q < 4; q++) {
-                            multiply_bytes(sums, digits + 2 * q, hot + 2 * q, form1, s > 0 || q > 0);
-                            if (n2) multiply_bytes(sums + 256, digits + 2 * q, hot + 256 * 128 / 16 + 2 * q, form2, s > 0 || q > 0);
+                            multiply_bytes(sums, digits + 2 * q, hot + 2 * q, form, s > 0 || q > 0);
+                            multiply_bytes(sums + kMmaTileRows, digits + kDigitBytes / 16 + 2 * q, hot + 2 * q, form, s > 0 || q > 0);
                         }
                         products_done(&empty[stage]);
                         if (++stage == kMmaStages) stage = 0, phase ^= 1;
@@ -327,25 +356,29 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ft_backward_mma_kernel(FtArgs 
             __syncwarp();
             sums_fence_after();
             const size_t four = (size_t)4 * a.H;
-            for (int n0 = 0; n0 < rows; n0 += 32) {
-                int v[32];
-                load_sums32(sums + n0 + ((uint32_t)warp << 21), v);
-                float sum[8];
+            for (int n0 = 0; n0 < rows; n0 += 16) {
+                int high[16], low[16];
+                load_sums16(sums + n0 + ((uint32_t)warp << 21), high);
+                load_sums16(sums + kMmaTileRows + n0 + ((uint32_t)warp << 21), low);
+                loaded_sums(high);
+                loaded_sums(low);
+                float sum[4];
 #pragma unroll
-                for (int g = 0; g < 8; g++) {
-                    // four rows of the table, one for each digit: a lane ends up with row d's
-                    const float f0 = (float)v[4 * g], f1 = (float)v[4 * g + 1], f2 = (float)v[4 * g + 2], f3 = (float)v[4 * g + 3];
-                    const float a2 = fmaf(d & 1 ? f1 : f0, mult_keep, __shfl_xor_sync(0xffffffffu, d & 1 ? f0 : f1, 8) * mult_got);
-                    const float b2 = fmaf(d & 1 ? f3 : f2, mult_keep, __shfl_xor_sync(0xffffffffu, d & 1 ? f2 : f3, 8) * mult_got);
-                    const float got = __shfl_xor_sync(0xffffffffu, d & 2 ? a2 : b2, 16);
-                    sum[g] = fmaf(d & 2 ? b2 : a2, by_keep, got * by_got);
+                for (int g = 0; g < 4; g++) {
+                    // four rows of the table, two digits of eight: a lane ends up with all of row d's
+                    float f[4];
+#pragma unroll
+                    for (int r = 0; r < 4; r++) f[r] = fmaf((float)low[4 * g + r], by_low, (float)high[4 * g + r] * by_high);
+                    const float a2 = (d & 1 ? f[1] : f[0]) + __shfl_xor_sync(0xffffffffu, d & 1 ? f[0] : f[1], 8);
+                    const float b2 = (d & 1 ? f[3] : f[2]) + __shfl_xor_sync(0xffffffffu, d & 1 ? f[2] : f[3], 8);
+                    sum[g] = ((d & 2 ? b2 : a2) + __shfl_xor_sync(0xffffffffu, d & 2 ? a2 : b2, 16)) * unit;
                 }
 #pragma unroll
-                for (int g = 0; g < 8; g++)
+                for (int g = 0; g < 4; g++)
                     if (n0 + 4 * g == own_rows && sum[g] != 0.f) atomicAdd(bias, sum[g]);
                 // (added also where nobody else adds: a caller that clears the gradients itself may have several passes summed)
 #pragma unroll
-                for (int g = 0; g < 8; g++, to += four)
+                for (int g = 0; g < 4; g++, to += four)
                     if (n0 + 4 * g < own_rows && sum[g] != 0.f) atomicAdd(to, sum[g]);
             }
             sums_fence_before();
@@ -360,111 +393,113 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ft_backward_mma_kernel(FtArgs 
         asm volatile("setmaxnreg.inc.sync.aligned.u32 136;");
         const int group = (warp >> 2) - 1, w4 = warp & 3, tg = w4 * 32 + lane;  // of steps group, group + 3, ...
         unsigned char* digits = base + group * stage_bytes;
-        unsigned char* hot = digits + kDigitBytes;
+        unsigned char* hot = digits + 2 * kDigitBytes;
         // this lane's four columns (m) and its pairs: T sets of four
-        constexpr int T = PAIRWISE ? 1 : 2, kSides = PAIRWISE ? 2 : 1;
+        constexpr int T = PAIRWISE ? 1 : 2;
         const int m = PAIRWISE ? lane & 3 : lane & 7;
         const int quad = PAIRWISE ? lane >> 2 & 3 : lane >> 3;  // which four of sixteen pairs
         auto sixteen = [&](int e) { return PAIRWISE ? w4 + 4 * (lane >> 4) : w4 + 4 * e; };
         float4 y0[T][4], y1[PAIRWISE ? T : 1][4], dd[ONE ? 1 : T][4];
         float dout[ONE ? T : 1][4];
-        int bucket[ONE ? T : 1][4];
+        int w1_row[ONE ? T : 1][4];
         int4 ids[T];
-        int cu = -1;                    // unit of columns of the operands
-        uint32_t second = 0;            // ONE: which of the pairs are second perspectives
         constexpr int kWords = kMmaTileRows / 128;
         const int words16 = ft_mma_words(rows);
         uint4 bits[kWords];
-        int twice = 0, chunk = 0;
+        int cu = 0, chunk = 0;  // unit of columns and chunk of the step in the making
         auto fetch_ids = [&]() {  // of the step that `walk` stands on
             if (walk.left > 0)
 #pragma unroll
                 for (int e = 0; e < T; e++) ids[e] = __ldg(reinterpret_cast<const int4*>(t.csr_start + (size_t)walk.chunk() * t.start_cap + 4) + 4 * sixteen(e) + quad);
         };
-        auto fetch = [&]() {  // and, these being there, its operands
-            cu = walk.unit;
-            chunk = walk.chunk();
-            twice = __ldg(t.csr_start + (size_t)chunk * t.start_cap);
-            const uint4* src = reinterpret_cast<const uint4*>(t.csr_ent + (size_t)chunk * t.ent_cap) + tg;
+        // and, these being there, the operands of a part, when those of the step before have been used
+        auto fetch = [&](int part) {
+            if (walk.left <= 0 || (PAIRWISE && part == 0)) return;
+            const int e = PAIRWISE ? 0 : part, col = min(walk.unit * kCols + 4 * m, width - 4);
 #pragma unroll
-            for (int q = 0; q < kWords; q++)
-                if (q < words16) bits[q] = __ldg(src + q * kMmaGroupThreads);
-            const int col = min(cu * kCols + 4 * m, width - 4);
-            second = 0;
-#pragma unroll
-            for (int e = 0; e < T; e++)
-#pragma unroll
-                for (int p = 0; p < 4; p++) {
-                    const int id = p == 0 ? ids[e].x : p == 1 ? ids[e].y : p == 2 ? ids[e].z : ids[e].w, pair = max(id, 0);  // (of a pair that is none, no byte is set)
-                    const float* y = (PAIRWISE ? a.u : a.x) + (size_t)pair * a.H + col;
-                    y0[e][p] = ld_once4(reinterpret_cast<const float4*>(y));
-                    if (PAIRWISE) y1[e][p] = ld_once4(reinterpret_cast<const float4*>(y + width));
-                    if (ONE) {
-                        dout[e][p] = __ldg(a.dout + (pair >> 1));
-                        bucket[e][p] = __ldg(a.out_bucket + (pair >> 1));
-                        second |= (uint32_t)(pair & 1) << (4 * e + p);
-                    } else {
-                        dd[e][p] = ld_once4(reinterpret_cast<const float4*>(a.dx + (size_t)pair * width + col));
-                    }
-                }
-        };
-        uint32_t words[2][4][4];  // [set or side][column][digit] of four pairs each: made while the stage is still in use
-        auto make = [&]() {
-#pragma unroll
-            for (int e = 0; e < T; e++) {
-                if (ONE) {  // (the unit's weights are a few KB, in L1)
-                    const int col = min(cu * kCols + 4 * m, width - 4);
-#pragma unroll
-                    for (int p = 0; p < 4; p++)
-                        dd[0][p] = scale4(__ldg(reinterpret_cast<const float4*>(a.w1 + (size_t)(2 * bucket[e][p] + (int)(second >> (4 * e + p) & 1u)) * width + col)), dout[e][p]);
-                }
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    uint32_t q[kSides][4];
-#pragma unroll
-                    for (int p = 0; p < 4; p++) {
-                        auto comp = [&](const float4& v) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; };
-                        const float grad = comp(dd[ONE ? 0 : e][p]) * scale;
-                        float g[kSides];
-                        if constexpr (PAIRWISE) {
-                            const float lo = comp(y0[e][p]), hi = comp(y1[e][p]);
-                            g[0] = inside_only(lo, grad * hi);
-                            g[1] = inside_only(hi, grad * lo);
-                        } else {
-                            const float y = comp(y0[e][p]);
-                            g[0] = SQUARE ? grad * ft_act_bwd(ONE ? 3 : 2, y) : inside_only(y, grad);
-                        }
-#pragma unroll
-                        for (int side = 0; side < kSides; side++) q[side][p] = ((uint32_t)__float2int_rn(g[side]) + 0x00808080u) ^ 0x00808080u;
-                    }
-#pragma unroll
-                    for (int side = 0; side < kSides; side++) {
-                        // four pairs' digit of this column: one word
-                        const uint32_t a01 = __byte_perm(q[side][0], q[side][1], 0x5140), a23 = __byte_perm(q[side][2], q[side][3], 0x5140);
-                        const uint32_t b01 = __byte_perm(q[side][0], q[side][1], 0x7362), b23 = __byte_perm(q[side][2], q[side][3], 0x7362);
-                        uint32_t* to = words[e * kSides + side][j];
-                        to[0] = __byte_perm(a01, a23, 0x5410);
-                        to[1] = __byte_perm(a01, a23, 0x7632);
-                        to[2] = __byte_perm(b01, b23, 0x5410);
-                        to[3] = __byte_perm(b01, b23, 0x7632);
-                    }
+            for (int p = 0; p < 4; p++) {
+                const int id = p == 0 ? ids[e].x : p == 1 ? ids[e].y : p == 2 ? ids[e].z : ids[e].w, pair = max(id, 0);  // (of a pair that is none, no byte is set)
+                const float* y = (PAIRWISE ? a.u : a.x) + (size_t)pair * a.H + col;
+                y0[e][p] = ld_once4(reinterpret_cast<const float4*>(y));
+                if (PAIRWISE) y1[e][p] = ld_once4(reinterpret_cast<const float4*>(y + width));
+                if (ONE) {
+                    dout[e][p] = __ldg(a.dout + (pair >> 1));
+                    w1_row[e][p] = 2 * __ldg(a.out_bucket + (pair >> 1)) + (pair & 1);
+                } else {
+                    dd[e][p] = ld_once4(reinterpret_cast<const float4*>(a.dx + (size_t)pair * width + col));
                 }
             }
         };
-        // Digit d of column 4 m + j of the unit (m + 4 for the second side) is row 32 (m / 2) + 8 d + (m + 2 j) % 8 of the tile: the words
-        // that a warp stores at a time lie in 32 different banks, and a warp of the sums finds 32 bytes of neighbouring columns.
-        auto store_words = [&]() {
+        int twice = 0;
+        auto fetch_bits = [&]() {
+            if (walk.left <= 0) return;
+            twice = __ldg(t.csr_start + (size_t)walk.chunk() * t.start_cap);
+            const uint4* src = reinterpret_cast<const uint4*>(t.csr_ent + (size_t)walk.chunk() * t.ent_cap) + tg;
 #pragma unroll
-            for (int e = 0; e < T; e++)
+            for (int q = 0; q < kWords; q++)
+                if (q < words16) bits[q] = __ldg(src + q * kMmaGroupThreads);
+        };
+        // The digits are made and stored in two parts (sets of pairs, PAIRWISE: sides), the first while the stage is still in use.
+        uint32_t words[4][8];  // [column][digit] of four pairs each
+        uint32_t below = 0;    // whether any gradient of a part has bits below the last digit
+        auto make = [&](int part) {
+            const int e = PAIRWISE ? 0 : part;
+            below = 0;
+            if (ONE && (!PAIRWISE || part == 0)) {  // (the unit's weights are a few KB, in L1)
+                const int col = min(cu * kCols + 4 * m, width - 4);
 #pragma unroll
-                for (int side = 0; side < kSides; side++)
+                for (int p = 0; p < 4; p++) dd[0][p] = scale4(__ldg(reinterpret_cast<const float4*>(a.w1 + (size_t)w1_row[e][p] * width + col)), dout[e][p]);
+            }
 #pragma unroll
-                    for (int j = 0; j < 4; j++) {
-                        const uint32_t mm = m + 4 * side, s8 = (mm + 2 * j) & 7;
-                        uint32_t* to = reinterpret_cast<uint32_t*>(digits + ((mm >> 1) * 32 + s8) * 128 + ((sixteen(e) ^ s8) << 4) + 4 * quad);
+            for (int j = 0; j < 4; j++) {
+                uint32_t q[3][4];
 #pragma unroll
-                        for (int d = 0; d < 4; d++) to[256 * d] = words[e * kSides + side][j][d];
-                    }
+                for (int p = 0; p < 4; p++) {
+                    auto comp = [&](const float4& v) { return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w; };
+                    float rest = ft_scaled_gradient<PAIRWISE, ONE, SQUARE>(__fmul_rn(comp(dd[ONE ? 0 : e][p]), scale), comp(y0[e][p]), PAIRWISE ? comp(y1[e][p]) : 0.f, part);
+#pragma unroll
+                    for (int piece = 0; piece < 3; piece++) q[piece][p] = take_piece(rest, piece);
+                    below |= __float_as_uint(rest) & 0x7fffffffu;
+                }
+                // four pairs' digit of this column: one word
+                uint32_t* to = words[j];
+#pragma unroll
+                for (int piece = 0; piece < 3; piece++) {
+                    const uint32_t a01 = __byte_perm(q[piece][0], q[piece][1], 0x5140), a23 = __byte_perm(q[piece][2], q[piece][3], 0x5140);
+                    to[3 * piece] = __byte_perm(a01, a23, 0x5410) ^ 0x80808080u;
+                    to[3 * piece + 1] = __byte_perm(a01, a23, 0x7632) ^ 0x80808080u;
+                    if (piece < 2)
+                        to[3 * piece + 2] = (__byte_perm(__byte_perm(q[piece][0], q[piece][1], 0x0062), __byte_perm(q[piece][2], q[piece][3], 0x0062), 0x5410) + 0x40404040u) ^ 0x80808080u;
+                }
+            }
+        };
+        // What the digits leave of a part's gradients, by atomics: of gradients below 2^-36 of the largest there can be.
+        auto add_rest = [&](int part) {
+            const int4 c = __ldg(t.chunks + chunk);
+            for (int i = 0; i < 16; i++) {
+                const int in_chunk = 16 * sixteen(PAIRWISE ? 0 : part) + 4 * quad + (i & 3), x_col = cu * kCols + 4 * m + (i >> 2);
+                if (in_chunk >= c.z || x_col >= width) continue;
+                const int2 pair = __ldg(t.pairs + c.y + in_chunk);
+                const float* y = (PAIRWISE ? a.u : a.x) + (size_t)pair.x * a.H + x_col;
+                const float dx = ONE ? __fmul_rn(a.w1[((size_t)2 * a.out_bucket[pair.x >> 1] + (pair.x & 1)) * width + x_col], a.dout[pair.x >> 1]) : a.dx[(size_t)pair.x * width + x_col];
+                float rest = ft_scaled_gradient<PAIRWISE, ONE, SQUARE>(__fmul_rn(dx, scale), y[0], PAIRWISE ? y[width] : 0.f, part);
+                for (int piece = 0; piece < 3; piece++) take_piece(rest, piece);
+                if (rest == 0.f) continue;
+                const int col = PAIRWISE && part ? width + x_col : x_col;
+                atomicAdd(a.g_bias + col, rest * unit);
+                const uint16_t* list = t.lists + (size_t)(c.y + in_chunk) * t.list_len;
+                for (int k = 0; k < pair.y; k++) atomicAdd(a.g_table + ((size_t)c.x * t.block_rows + __ldg(list + k)) * a.H + col, rest * unit);
+            }
+        };
+        auto store_words = [&](int part) {
+            const int e = PAIRWISE ? 0 : part, side = PAIRWISE ? part : 0;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const uint32_t mm = m + 4 * side, s8 = (mm + 2 * j) & 7;
+                uint32_t* to = reinterpret_cast<uint32_t*>(digits + ((mm >> 1) * 32 + s8) * 128 + ((sixteen(e) ^ s8) << 4) + 4 * quad);
+#pragma unroll
+                for (int d = 0; d < 8; d++) to[(d >> 2) * (kDigitBytes / 4) + 256 * (d & 3)] = words[j][d];
+            }
         };
         unsigned char* own_hot = hot + (tg >> 3) * 128 + (((tg & 7) ^ (tg >> 3 & 7)) << 4);  // 16 pairs of rows tg / 8 + 16 q
         auto store_bits = [&]() {
@@ -495,22 +530,30 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ft_backward_mma_kernel(FtArgs 
             }
         };
         walk.advance(t, units, group);
-        if (walk.left > 0) {
-            fetch_ids();
-            fetch();
-        }
+        fetch_ids();
+        fetch(0);
+        fetch(1);
+        fetch_bits();
         for (uint32_t phase = 1; walk.left > 0; phase ^= 1) {
+            cu = walk.unit;
+            chunk = walk.chunk();
             walk.advance(t, units, kMmaStages);
             fetch_ids();
-            make();
+            make(0);
             wait(&empty[group], phase);  // (the first round finds the stage free)
             __syncwarp();
-            store_words();
+            store_words(0);
+            fetch(0);
+            if (below) add_rest(0);
+            make(1);
+            store_words(1);
+            fetch(1);
+            if (below) add_rest(1);
             if (twice) store_counts();
             else store_bits();
             fence_proxy_async();
             mbar_arrive(&full[group]);
-            if (walk.left > 0) fetch();
+            fetch_bits();
         }
     }
     __syncthreads();

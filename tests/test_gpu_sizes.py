@@ -420,13 +420,41 @@ PRODUCTS = {
     "rows-32": (32, 1, 32, 40, False, ACT_CRELU, (8, 1), 2, 65, False),
     "rows-147-ragged-width": (147, 1, 49, 72, False, ACT_CRELU, (1,), 1, 1000, False),
     "rows-255": (255, 2, 64, 96, False, ACT_SCRELU, (4, 1), 1, 129, False),
-    "rows-256": (256, 1, 9, 64, False, ACT_CRELU, (1,), 3, 4000, False),
-    "rows-383": (383, 2, 32, 136, True, ACT_CRELU, (16, 32, 1), 8, 900, False),
-    "rows-383-one": (383, 1, 32, 64, True, ACT_CRELU, (1,), 1, 64, False),
+    "rows-223": (223, 1, 9, 64, False, ACT_CRELU, (1,), 3, 4000, False),
+    "rows-255-pairwise": (255, 2, 32, 136, True, ACT_CRELU, (16, 32, 1), 8, 900, False),
+    "rows-255-pairwise-one": (255, 1, 32, 64, True, ACT_CRELU, (1,), 1, 64, False),
     "counts": (150, 2, 40, 96, False, ACT_CRELU, (1,), 2, 300, True),
-    "counts-pairwise": (300, 1, 64, 128, True, ACT_CRELU, (8, 1), 1, 150, True),
+    "counts-pairwise": (200, 1, 64, 128, True, ACT_CRELU, (8, 1), 1, 150, True),
     "sums-taken-out-on-the-way": (2, 1, 1, 32, False, ACT_CRELU, (1,), 1, 2600000, False),
 }
+
+
+def sums_in_64_bits(net, desc, batch):
+    """(sum, sum of magnitudes) in 64 bits of the last pass's gradients at the pre-activations, which follow from what the pass kept: of
+    the table and of the bias."""
+    n = len(batch[0])
+    x, dx = (net.activation(k, n * desc.dense_in0).reshape(n, 2, -1) for k in (0, 2))
+    if desc.pairwise:
+        u = net.activation(1, n * 2 * desc.ft_out).reshape(n, 2, 2, desc.ft_out // 2)
+        pre = np.stack([dx * u[:, :, 1], dx * u[:, :, 0]], axis=2).astype(np.float64) * ((u > 0) & (u < 1))
+        pre = pre.reshape(n, 2, desc.ft_out)
+    else:
+        slope = ((x > 0) & (x < 1)) * (2 * np.sqrt(x) if desc.ft_act == ACT_SCRELU else np.float32(1))
+        pre = dx.astype(np.float64) * slope
+    out = []
+    for values in (pre, np.abs(pre)):
+        table = np.zeros((desc.n_inputs, desc.ft_out))
+        for side in range(2):
+            index = batch[side]
+            for slot in range(desc.nnz):
+                on = index[:, slot] >= 0
+                if n > 100000:
+                    for c in range(desc.ft_out):
+                        table[:, c] += np.bincount(index[on, slot], values[on, side, c], desc.n_inputs)
+                else:
+                    np.add.at(table, index[on, slot], values[on, side])
+        out += [(table, values.sum((0, 1)))]
+    return out
 
 
 @pytest.mark.parametrize("case", PRODUCTS)
@@ -460,25 +488,7 @@ def test_products_of_bytes_are_no_further_from_64_bits_than_the_walk(case):
         net.step(0, 0.0, 1.0 / n)
         net.loss()
         g = net.tensors(kind=3)
-        x, dx = (net.activation(k, n * desc.dense_in0).reshape(n, 2, -1) for k in (0, 2))
-        if pairwise:
-            u = net.activation(1, n * 2 * ft_out).reshape(n, 2, 2, ft_out // 2)
-            pre = np.stack([dx * u[:, :, 1], dx * u[:, :, 0]], axis=2).astype(np.float64) * ((u > 0) & (u < 1))
-            pre = pre.reshape(n, 2, ft_out)
-        else:
-            slope = ((x > 0) & (x < 1)) * (2 * np.sqrt(x) if act == ACT_SCRELU else np.float32(1))
-            pre = dx.astype(np.float64) * slope
-        table = np.zeros((desc.n_inputs, ft_out))
-        for side in range(2):
-            index = batch[side]
-            for slot in range(nnz):
-                on = index[:, slot] >= 0
-                if n > 100000:
-                    for c in range(ft_out):
-                        table[:, c] += np.bincount(index[on, slot], pre[on, side, c], desc.n_inputs)
-                else:
-                    np.add.at(table, index[on, slot], pre[on, side])
-        bias = pre.sum((0, 1))
+        (table, bias), _ = sums_in_64_bits(net, desc, batch)
         error[products] = [np.linalg.norm(g[k].astype(np.float64).reshape(ref.shape) - ref) / max(np.linalg.norm(ref), 1e-300)
                            for k, ref in (("l0w", table), ("l0b", bias))]
         print(case, "products" if products else "walk", error[products])
@@ -488,6 +498,48 @@ def test_products_of_bytes_are_no_further_from_64_bits_than_the_walk(case):
     # thousands by a few per cent.
     for mine, walk, sums in zip(error[1], error[0], (table.size, bias.size)):
         assert mine <= max((1.05 if sums > 1000 else 2) * walk, 2.0 ** -24)
+
+
+@pytest.mark.parametrize("products", [0, 1])
+@pytest.mark.parametrize("dense,pairwise,act", [((1,), False, ACT_CRELU), ((1,), False, ACT_SCRELU), ((1,), True, ACT_CRELU), ((8, 1), False, ACT_SCRELU),
+                                                ((16, 32, 1), True, ACT_CRELU)])
+def test_small_gradients_beside_large_ones_keep_32_bits(products, dense, pairwise, act):
+    """Columns of the first dense layer over seven decades and positions whose gradients span six: every single sum is as close
+    to 64 bits as fp32 makes it, whatever else the batch holds.
+
+    In units of 2^-24 of a sum's magnitudes: an addend is rounded at most twice, the digits' sums (at most three times the magnitudes) four
+    times when they are put together, and the at most 48 parts that CTAs hold of a sum are added in fp32: 62, taken as 64.  The walk
+    over lists rounds in each of its up to 900 additions, a random walk of 30."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    n, rows, nnz, ft_out = 3000, 147, 40, 128
+    desc = dataclasses.replace(net_of(1, rows, ft_out, nnz, 1, dense, act, pairwise), max_batch=n)
+    w = rich_weights(desc)
+    shape = desc.tensor_shapes()["l1w"]
+    decades = 10.0 ** -np.linspace(0, 7, desc.dense_in0).astype(np.float32)
+    rng = np.random.default_rng(3)
+    rng.shuffle(decades)
+    first = w["l1w"].reshape(shape)
+    w["l1w"] = (first * (decades if shape[1] == desc.dense_in0 else decades[:, None])).astype(np.float32).ravel()
+    stm, nstm, bucket, target = draw_batch(desc, n, seed=8)
+    net = make_net(desc, 0, w)
+    net.set_option("ft_bwd_products", products)
+    net.upload(0, stm, nstm, bucket, target)
+    out = net.forward(0, n).astype(np.float64)
+    target = 1 / (1 + np.exp(-out)) + rng.choice([-1, 1], n) * 10.0 ** -rng.uniform(0.4, 6.4, n)
+    batch = (stm, nstm, bucket, target.astype(np.float32))
+    net.upload(0, *batch)
+    net.step(0, 0.0, 1.0 / n)
+    g = net.tensors(kind=3)
+    sums, magnitudes = sums_in_64_bits(net, desc, batch)
+    for k, ref, all_of_it in zip(("l0w", "l0b"), sums, magnitudes):
+        assert all_of_it.max() > 0
+        off = np.abs(g[k].reshape(ref.shape) - ref) / np.maximum(all_of_it, 2.0 ** -120)
+        print(k, off.max() * 2 ** 24)
+        assert off.max() <= 64 * 2.0 ** -24, k
+    net.close()
 
 
 @pytest.mark.parametrize("products", [0, 1])
