@@ -229,12 +229,15 @@ __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __grid_con
     }
     flush();
     if (a.want_grad) {
+        __shared__ unsigned s_largest[2][kOneThreads / 32];
         if (a.gmax) {
-            raise_magnitude(a.gmax, largest_dout);
-            raise_magnitude(a.gmax + 1, largest_w);
+            largest_dout = __reduce_max_sync(0xffffffffu, largest_dout);
+            largest_w = __reduce_max_sync(0xffffffffu, largest_w);
+            if (lane == 0) s_largest[0][warp] = largest_dout, s_largest[1][warp] = largest_w;
         }
         if (tid < 32) s_loss[tid] = tid < P ? my_loss : 0.f;
         __syncthreads();
+        if (a.gmax && (warp == 1 || warp == 2)) raise_magnitude(a.gmax + warp - 1, s_largest[warp - 1][lane % (kOneThreads / 32)]);
         if (warp == 0) {
             const float sum = warp_sum(s_loss[lane]);
             if (lane == 0 && sum != 0.f) atomicAdd(a.loss, sum);

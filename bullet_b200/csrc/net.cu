@@ -263,7 +263,8 @@ struct b200_net {
     bool bwd_mma(int n) const {
         return small_table() && bwd_wide && !overlap_mode && (bwd_products > 0 || (bwd_products < 0 && (long long)n * d.ft_out >= kProductSums));
     }
-    unsigned* gmax = nullptr;  // see FtArgs
+    unsigned* gmax = nullptr;    // see FtArgs
+    bool products_last = false;  // the last backward was ft_backward_mma_kernel
 };
 
 namespace {
@@ -433,6 +434,7 @@ void (*ft_backward_mma(const b200_net* net))(b200::FtArgs, b200::TileArgs) {
 
 template <bool PW>
 int launch_ft_backward(b200_net* net, const Slot& s, const b200::FtArgs& a, const b200::TileArgs& t, bool tiled, int grid) {
+    net->products_last = tiled && s.mma;
     if (tiled && s.mma) {
         b200::launch_step(net->chained, ft_backward_mma(net), grid, b200::kMmaThreads, b200::ft_mma_smem(b200::ft_mma_rows(t.block_rows)), net->stream, a, t);
     } else if (tiled) {
@@ -558,7 +560,7 @@ b200::FtArgs ft_args(b200_net* net, const Slot& s) {
     a.dout = net->dz[0];
     a.out_bucket = net->kept_bucket;
     a.stamp = nullptr;
-    a.gmax = net->gmax;
+    a.gmax = s.mma ? net->gmax : nullptr;
     a.gave_up = net->h_gave_up;
     a.g_table = net->G + net->find("l0w")->off;
     a.g_bias = net->G + net->find("l0b")->off;
@@ -624,7 +626,7 @@ b200::DenseArgs dense_args(b200_net* net, const Slot& s, bool want_grad) {
     a.partial = net->dense_partial;
     a.dz_frag = net->dz_frag;
     a.gave_up = net->h_gave_up;
-    a.gmax = net->gmax;
+    a.gmax = want_grad && s.mma ? net->gmax : nullptr;  // (the walk needs no scale: up to 4 us of the dense kernels)
     a.a1 = net->a1;
     a.a2 = net->a2;
     a.out = net->out;
@@ -831,7 +833,7 @@ int forward_dense(b200_net* net, Slot& s, bool want_grad) {
         a.want_grad = da.want_grad;
         a.stamp = da.stamp;
         a.gave_up = net->h_gave_up;
-        a.gmax = net->gmax;
+        a.gmax = da.gmax;
         if (want_grad) net->w1_used = da.W1g, net->grad_n = s.n, net->dx_formed = false;
         const size_t smem = b200::one_smem(a.K1);
         const int units = a.ntiles * (b200::kDenseTile / b200::one_rows(a.K1)), slots = net->sm_count * std::max(1, std::min(4, (int)(220 * 1024 / smem)));
@@ -1294,7 +1296,7 @@ int b200_net_set_option(b200_net* net, const char* key, int64_t value) {
     if (!strcmp(key, "ft_once")) {
         return 0;  // (no load of the tiled kernels gains from an L1 line any more: one form)
     }
-    if (!strcmp(key, "ft_bwd_products")) {  // the same
+    if (!strcmp(key, "ft_bwd_products")) {  // takes effect for batches uploaded afterwards
         if (value < -1 || value > 1) return b200::fail(B200_ERR_ARG, "ft_bwd_products must be -1, 0 or 1");
         net->bwd_products = (int)value;
         return 0;
@@ -2445,6 +2447,7 @@ int b200_net_get_stat(b200_net* net, const char* key, int64_t* value) {
     else if (!strcmp(key, "h2d_bytes")) *value = net->h2d_bytes;
     else if (!strcmp(key, "flat_floats")) *value = net->n_flat;
     else if (!strcmp(key, "ft_tiled")) *value = (net->fwd_tiled() ? 1 : 0) + (net->bwd_tiled() ? 2 : 0);
+    else if (!strcmp(key, "ft_products")) *value = net->products_last ? 1 : 0;
     else if (!strcmp(key, "slow_weights")) *value = net->S ? 1 : 0;
     else if (!strcmp(key, "optimiser_steps")) *value = net->opt_step;
     else return b200::fail(B200_ERR_ARG, "get_stat: unknown key '%s'", key);
