@@ -251,17 +251,24 @@ struct b200_net {
     bool keep_root() const { return dense_one() && d.ft_act == B200_ACT_SCRELU; }
     // first dense layers of four and more rows per bucket run on the tensor pipe
     bool dense_mma() const { return d.dense_out[0] >= 4; }
-    // Which batches of n positions ft_backward_mma_kernel takes: those with enough sums (positions x columns) of a table whose rows fit
-    // into one tile, unless the backward has to announce finished row blocks or was asked for by another shape.  Whole training
-    // pass with 147 rows, walk / products in us: 30000 x 64 191 to 199 / 188 to 195 and 2000 x 256 63 to 65 / 63 to 75 (no gain: the upload is
-    // as long), 9000 x 256 108 / 96, 65000 x 64 197 / 168, 2000 x 1984 133 / 104, 30000 x 960 640 / 414.  The line is on the
-    // safe side: 2000 x 960, 91 / 78, lies just below it, and the backward alone gains from 300 positions on (13 / 9), which whole passes that
-    // small do not show beyond their spread (300 x 256 53 to 54 / 53 to 73, 300 x 1984 54 / 56).
-    // Larger blocks in parts (768 rows) lose: backward of 16384 x 2048 282 / 420.
-    static constexpr long long kProductSums = 2LL << 20;
+    // Which batches of n positions ft_backward_mma_kernel takes: those it is the faster form for, of a table whose rows fit into one
+    // tile, unless the backward has to announce finished row blocks or was asked for by another shape.
     bool small_table() const { return tiled_ok && block_rows < b200::kMmaTileRows; }
-    bool bwd_mma(int n) const {
-        return small_table() && bwd_wide && !overlap_mode && (bwd_products > 0 || (bwd_products < 0 && (long long)n * d.ft_out >= kProductSums));
+    bool bwd_mma(int n) const { return small_table() && bwd_wide && !overlap_mode && (bwd_products > 0 || (bwd_products < 0 && products_pay(n))); }
+    // Both forms' ns for 128 pairs x 32 columns on one SM, fitted to the sweep below.  Products write out the whole tile whatever the
+    // lists hold, cut every block's pairs into steps of its own (one more on average is not full) and take out its sums; the walk's time goes
+    // with the active rows, of which the host knows the slots: half of them, as of the games' lists.  The line is drawn 1.4 times to the
+    // walk's side, which also leaves it small batches, where a step's latency counts.  Backward on a B200, walk / products in us (rows x blocks, active of slots):
+    //   147 x 1, 27 of 49: 32768 positions x 256 columns 87 / 41, 4096 x 1024 49 / 24, 512 x 64 12 / 9.4, 300 x 64 11.6 / 10 (walks), pairwise 16384 x 512 91 / 61
+    //   255 x 1, 17 of 32: 32768 x 256 64 / 48, 4096 x 1024 36 / 28, 3000 x 128 11.3 / 12.7 (walks), pairwise 16384 x 512 69 / 66 (walks)
+    //   255 x 1, 4 of 8: 32768 x 256 35 / 47 (walks);  64 x 1, 8 of 16: 32768 x 256 43 / 37, pairwise 16384 x 512 48 / 63 (walks)
+    //   200 x 8, 17 of 32: 16384 x 256 33 / 28, 1024 x 2048 24 / 34 (walks), pairwise 32768 x 1024 246 / 254 (walks)
+    //   147 x 64, 17 of 32: 16384 x 256 43 / 38 (given up), 1024 x 2048 52 / 131 (walks);  31 x 1000, 4 of 8: 1024 x 2048 293 / 762 (walks)
+    // Lists that are emptier than half may get the slower form: 255 rows, 4 of 32 slots, loses 12 us of 96 at 32768 x 256.
+    bool products_pay(int n) const {
+        const long long steps = ((long long)2 * n + b200::kStepPairs - 1) / b200::kStepPairs, blocks = std::min<long long>(nblocks, 2LL * n);
+        const long long product = (d.pairwise ? 1700 : 900) + b200::ft_mma_rows(block_rows) * 22 / 10, walk = 900 + 85 * d.nnz / 2;
+        return 14 * (steps + (1 + b200::kUnitFixed) * blocks) * product < 10 * steps * walk;
     }
     unsigned* gmax = nullptr;    // see FtArgs
     bool products_last = false;  // the last backward was ft_backward_mma_kernel

@@ -99,7 +99,7 @@ int b200_net_destroy(b200_net* net);
 /* Tuning switches (no counterpart in the reference; every one has a measured default):
  *   "ft_mode" / "ft_fwd_mode" / "ft_bwd_mode"  B200_FT_*; "ft_bwd_wide" 0 = two 512-thread backward CTAs per SM;
  *   "ft_bwd_products" 0 / 1 = the backward of tables of fewer than 256 rows per block never / always multiplies bytes instead of
- *   walking row lists (-1, the default: from 2 million sums on);
+ *   walking row lists (-1, the default: where that is faster);
  *   "ft_once" accepted, without effect (one form of loads is left);
  *   "ft_bwd_grab" eighths of a unit's row pieces that the tiled backward deals to its warps in advance (0 = default, more than 8 counts as 8);
  *   "exchange_bulk" 1 = the peer exchange moves gradients and weights with bulk asynchronous copies;

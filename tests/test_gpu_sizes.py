@@ -566,3 +566,36 @@ def test_gradients_of_two_passes_add_up_where_the_caller_clears_them(products, d
         assert np.abs(g).max() > 0, k
         assert np.abs(twice[k] - 2 * g).max() <= 2e-5 * np.abs(2 * g).max(), k
     net.close()
+
+
+# rows, blocks, slots, width, pairwise, dense layers, positions: which of the two is the faster backward, by its measured side of the line
+FASTER = {
+    "ataxx": (147, 1, 49, 256, False, (1,), 32768, 1),
+    "ataxx-few": (147, 1, 49, 64, False, (1,), 512, 1),
+    "ataxx-fewer": (147, 1, 49, 64, False, (1,), 100, 0),
+    "ataxx-pairwise": (147, 1, 49, 512, True, (16, 32, 1), 16384, 1),
+    "rows-255": (255, 1, 32, 256, False, (1,), 32768, 1),
+    "rows-255-short-lists": (255, 1, 8, 256, False, (1,), 32768, 0),
+    "rows-255-pairwise": (255, 1, 32, 512, True, (16, 32, 1), 16384, 0),
+    "rows-256": (256, 1, 49, 256, False, (1,), 32768, 0),
+    "eight-blocks": (200, 8, 32, 256, False, (1,), 16384, 1),
+    "eight-blocks-few-pairs": (200, 8, 32, 2048, False, (1,), 1024, 0),
+    "many-blocks": (147, 64, 32, 2048, False, (1,), 1024, 0),
+    "a-thousand-blocks": (31, 1000, 8, 2048, False, (1,), 1024, 0),
+}
+
+
+@pytest.mark.parametrize("case", FASTER)
+def test_small_tables_take_the_faster_backward(case):
+    rows, blocks, nnz, ft_out, pairwise, dense, n, products = FASTER[case]
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net
+
+    desc = dataclasses.replace(net_of(blocks, rows, ft_out, nnz, 1, dense, ACT_CRELU, pairwise), max_batch=n)
+    net = make_net(desc)
+    net.upload(0, *draw_batch(desc, n, seed=n))
+    net.step(0, 0.0, 1.0 / n)
+    net.loss()
+    assert net.stat("ft_products") == products
+    net.close()
