@@ -52,8 +52,9 @@ struct OneArgs {
     unsigned long long* stamp;
 };
 
-// SQUARE: x holds the roots of its values (activation 3 of kernels_ft.cuh).
-template <bool SQUARE>
+// SQUARE: x holds the roots of its values (activation 3 of kernels_ft.cuh).  SCALE: the largest |dout| and |W| are wanted (an
+// instantiation of its own: asking at run time costs 1 of 35 us, 16384 positions x 1024 columns, where nobody wants them).
+template <bool SQUARE, bool SCALE>
 __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __grid_constant__ OneArgs a) {
     step_begin(a.stamp);
     extern __shared__ __align__(128) float one_smem_raw[];
@@ -153,7 +154,7 @@ __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __grid_con
                 for (int c = tid; c < cols4; c += kOneThreads) {
                     const float4 w = __ldg(reinterpret_cast<const float4*>(a.W + (size_t)k * a.K1) + c);
                     reinterpret_cast<float4*>(s_w)[c] = w;
-                    if (a.gmax) largest_w = max(max(largest_w, max(magnitude(w.x), magnitude(w.y))), max(magnitude(w.z), magnitude(w.w)));
+                    if (SCALE) largest_w = max(max(largest_w, max(magnitude(w.x), magnitude(w.y))), max(magnitude(w.z), magnitude(w.w)));
                 }
                 __syncthreads();
             }
@@ -196,7 +197,7 @@ __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __grid_con
                         dout = (diff + diff) * (s * (1.f - s));
                         a.dout[b] = dout;
                         a.kept_bucket[b] = k;
-                        largest_dout = max(largest_dout, magnitude(dout));
+                        if (SCALE) largest_dout = max(largest_dout, magnitude(dout));
                     }
                 }
                 s_dout[row] = dout;
@@ -230,14 +231,14 @@ __global__ void __launch_bounds__(kOneThreads) dense_one_kernel(const __grid_con
     flush();
     if (a.want_grad) {
         __shared__ unsigned s_largest[2][kOneThreads / 32];
-        if (a.gmax) {
+        if (SCALE) {
             largest_dout = __reduce_max_sync(0xffffffffu, largest_dout);
             largest_w = __reduce_max_sync(0xffffffffu, largest_w);
             if (lane == 0) s_largest[0][warp] = largest_dout, s_largest[1][warp] = largest_w;
         }
         if (tid < 32) s_loss[tid] = tid < P ? my_loss : 0.f;
         __syncthreads();
-        if (a.gmax && (warp == 1 || warp == 2)) raise_magnitude(a.gmax + warp - 1, s_largest[warp - 1][lane % (kOneThreads / 32)]);
+        if (SCALE && (warp == 1 || warp == 2)) raise_magnitude(a.gmax + warp - 1, s_largest[warp - 1][lane % (kOneThreads / 32)]);
         if (warp == 0) {
             const float sum = warp_sum(s_loss[lane]);
             if (lane == 0 && sum != 0.f) atomicAdd(a.loss, sum);

@@ -822,6 +822,11 @@ int forward_ft_blocks(b200_net* net, Slot& s, int first_block, int last_block) {
     return net->d.pairwise ? launch_ft_forward<true>(net, fa, ta, tiled, grid) : launch_ft_forward<false>(net, fa, ta, tiled, grid);
 }
 
+void (*dense_one_form(const b200_net* net, bool scale))(b200::OneArgs) {
+    if (net->keep_root()) return scale ? b200::dense_one_kernel<true, true> : b200::dense_one_kernel<true, false>;
+    return scale ? b200::dense_one_kernel<false, true> : b200::dense_one_kernel<false, false>;
+}
+
 int forward_dense(b200_net* net, Slot& s, bool want_grad) {
     if (want_grad && !net->chained) CK(cudaEventRecord(net->tev[net->steps_begun % b200_net::kTimingRing][1], net->stream));
     if (net->zero_pending) {  // the loss and every gradient from here on land in the cleared buffer
@@ -845,7 +850,7 @@ int forward_dense(b200_net* net, Slot& s, bool want_grad) {
         const size_t smem = b200::one_smem(a.K1);
         const int units = a.ntiles * (b200::kDenseTile / b200::one_rows(a.K1)), slots = net->sm_count * std::max(1, std::min(4, (int)(220 * 1024 / smem)));
         a.units_per_run = (units + slots - 1) / slots;
-        b200::launch_step(net->chained, net->keep_root() ? b200::dense_one_kernel<true> : b200::dense_one_kernel<false>, (units + a.units_per_run - 1) / a.units_per_run, b200::kOneThreads, smem, net->stream, a);
+        b200::launch_step(net->chained, dense_one_form(net, a.gmax != nullptr), (units + a.units_per_run - 1) / a.units_per_run, b200::kOneThreads, smem, net->stream, a);
         LAUNCHED(net);
         return 0;
     }
@@ -951,7 +956,7 @@ bool load_dense_kernels() {
 int preload_kernels(b200_net* net) {
     bool ok = true;
     DISPATCH_M(net->d.dense_out[0], ok = load_dense_kernels<MM>());
-    ok = ok && load_kernel(b200::dense_regroup_kernel) && load_kernel(b200::dense_one_kernel<true>) && load_kernel(b200::dense_one_kernel<false>) && load_kernel(b200::dense_one_dx_kernel) && load_kernel(b200::copy_outputs_kernel) && load_kernel(b200::dense_fragments_kernel) && load_kernel(b200::dense_small_grads_kernel);
+    ok = ok && load_kernel(b200::dense_regroup_kernel) && load_kernel(dense_one_form(net, false)) && (!net->small_table() || load_kernel(dense_one_form(net, true))) && load_kernel(b200::dense_one_dx_kernel) && load_kernel(b200::copy_outputs_kernel) && load_kernel(b200::dense_fragments_kernel) && load_kernel(b200::dense_small_grads_kernel);
     ok = ok && load_kernel(b200::ft_forward_gather_kernel<true, true>) && load_kernel(b200::ft_forward_gather_kernel<true, false>) && load_kernel(b200::ft_forward_gather_kernel<false, true>) && load_kernel(b200::ft_forward_gather_kernel<false, false>);
     ok = ok && load_kernel(b200::ft_backward_gather_kernel<true, true>) && load_kernel(b200::ft_backward_gather_kernel<true, false>) && load_kernel(b200::ft_backward_gather_kernel<false, true>) && load_kernel(b200::ft_backward_gather_kernel<false, false>);
     ok = ok && load_kernel(b200::ft_forward_tiled_kernel<true>) && load_kernel(b200::ft_forward_tiled_kernel<false>);
@@ -1173,7 +1178,7 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
             return 0;
         };
         if (int rc2 = set_dense(d.dense_out[0])) return bail(rc2);
-        if (b200::allow_smem(b200::dense_one_kernel<true>) != cudaSuccess || b200::allow_smem(b200::dense_one_kernel<false>) != cudaSuccess) return bail(b200::fail(B200_ERR_CUDA, "net_create: shared memory of the dense kernel"));
+        if (b200::allow_smem(dense_one_form(net, false)) != cudaSuccess || (net->small_table() && b200::allow_smem(dense_one_form(net, true)) != cudaSuccess)) return bail(b200::fail(B200_ERR_CUDA, "net_create: shared memory of the dense kernel"));
     }
     if (net->tiled_ok) {
         cudaError_t e = b200::allow_smem(b200::ft_forward_tiled_kernel<true>);
