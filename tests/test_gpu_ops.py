@@ -26,8 +26,9 @@ def op_inputs(oracle32, desc, game, n, seed):
     return stm, nstm, w, table, oracle_ft_output(oracle32, desc, w, stm, nstm)
 
 
-def run_op(entry, desc, table, bias, stm, nstm, n):
-    """Calls `entry` (a b200_op_ft_forward-style symbol) on torch-owned device buffers; returns (rc, x, u)."""
+def run_op(entry, desc, table, bias, stm, nstm, n, x_at=0):
+    """Calls `entry` (a b200_op_ft_forward-style symbol) on torch-owned device buffers; returns (rc, x, u).  With x starting `x_at` floats
+    into a buffer, where that is no multiple of four, the positions are grouped however few they are."""
     import torch
 
     from bullet_b200 import _lib
@@ -39,7 +40,7 @@ def run_op(entry, desc, table, bias, stm, nstm, n):
     t_stm = torch.from_numpy(pack_indices(stm).view(np.int16)).to(dev)
     t_nstm = torch.from_numpy(pack_indices(nstm).view(np.int16)).to(dev)
     d1 = desc.ft_out if desc.pairwise else 2 * desc.ft_out
-    t_x = torch.full((n, d1), float("nan"), device=dev)
+    t_x = torch.full((n * d1 + x_at,), float("nan"), device=dev)[x_at:].view(n, d1)
     t_u = torch.full((n, 2, desc.ft_out), float("nan"), device=dev) if desc.pairwise else None
     op = _lib.CFtOp(desc.n_inputs, desc.nnz, desc.ft_out, desc.ft_act, int(desc.pairwise), desc.ft_block_rows, n,
                     t_table.data_ptr(), t_bias.data_ptr(), t_stm.data_ptr(), t_nstm.data_ptr(), t_x.data_ptr(),

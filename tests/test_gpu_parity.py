@@ -655,7 +655,7 @@ def test_kernel_forms_chosen_by_size_give_the_same_numbers(option, value):
     the forward outputs bit-identical and the step within the noise of the reduction order."""
     from bullet_b200.net import featurise
 
-    c = config(3)
+    c = config(2 if option == "ft_bwd_products" else 3)  # (products are for small tables)
     n = 4096
     desc = dataclasses.replace(c.desc, max_batch=n)
     batch = featurise(c.game, synth.records(c.game, n, seed=17), desc)
@@ -669,6 +669,8 @@ def test_kernel_forms_chosen_by_size_give_the_same_numbers(option, value):
         out = net.forward(0, n)
         net.step(0, 1e-3, 1.0 / n)
         results.append((out, net.loss(), net.tensors(0)))
+        if option == "ft_bwd_products":
+            assert net.stat("ft_products") == (value if forced else 1)
         net.close()
     (out_a, loss_a, w_a), (out_b, loss_b, w_b) = results
     assert np.array_equal(out_a, out_b)

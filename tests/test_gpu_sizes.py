@@ -74,6 +74,8 @@ def test_kernel_forms_at_the_edges_of_their_ranges(oracle32, case):
     x_ref = oracle_ft_output(oracle32, desc, w, *batch[:2])
     loss_ref, g_ref, out_ref = oracle32.net_grad(desc, w, *batch)
     net = make_net(desc, 0, w)
+    if case == "chunks-in-between-wide":
+        net.set_option("ft_bwd_products", 0)  # (what it is here for are the walk's lists)
     net.upload(0, *batch)
     out = net.forward(0, n)
     assert np.array_equal(net.activation(0, n * desc.dense_in0).reshape(n, -1), x_ref)
@@ -125,6 +127,80 @@ def test_a_loss_gradient_that_is_not_finite_stays_in_its_rows(oracle32, ft_out, 
     net.close()
 
 
+@pytest.mark.parametrize("dense,pairwise", [((1,), False), ((8, 1), False), ((16, 32, 1), True)])
+def test_products_in_parts_and_in_slots_that_change_hands(oracle32, dense, pairwise):
+    """The product backward a run of row blocks at a time, in a slot that holds batches of other sizes cut for the walk and for products
+    in turn.  Bounds as above."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    most, n = 2900, 150
+    desc = dataclasses.replace(net_of(8, 96, 128, 20, 2, dense, ACT_CRELU, pairwise), max_batch=most)
+    w = rich_weights(desc)
+    net = make_net(desc, 0, w)
+    for count, products, seed in ((most, 1, 5), (n, 0, 6), (most, 0, 7), (n, 1, 8), (most, 1, 9)):
+        net.set_option("ft_bwd_products", products)
+        batch = draw_batch(desc, count, seed)
+        net.upload(0, *batch)
+        _, g_ref, _ = oracle32.net_grad(desc, w, *batch)
+        for parts in (1, 4, 8):
+            net.backward_begin(0)
+            for part in range(parts):
+                net.backward_ft(0, part, parts)
+            net.backward_end(0)
+            assert net.stat("ft_products") == products
+            g = net.tensors(kind=3)
+            for k in g_ref:
+                assert np.abs(g[k] - g_ref[k]).max() <= 2e-5 * np.abs(g_ref[k]).max(), (k, count, parts)
+    net.close()
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+@pytest.mark.parametrize("products", [0, 1])
+@pytest.mark.parametrize("ft_out,pairwise,act,dense", [(72, False, ACT_SCRELU, (1,)), (96, False, ACT_CRELU, (1,)), (64, False, ACT_SCRELU, (8, 1)),
+                                                       (136, True, ACT_CRELU, (1,)), (128, True, ACT_CRELU, (16, 32, 1))])
+def test_products_of_gradients_that_are_not_finite(oracle32, ft_out, pairwise, act, dense, products, value):
+    """The same with both backward passes of small tables, in one row block and in three; next comes a batch that is finite.  Bounds as above."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    n, bad = 300, 117
+    blocks = 3 if ft_out % 64 == 0 else 1  # (other widths are one block)
+    desc = dataclasses.replace(net_of(blocks, 100, ft_out, 31, 1, dense, act, pairwise), max_batch=n)
+    stm, nstm, bucket, target = draw_batch(desc, n, seed=ft_out)
+    w = rich_weights(desc)
+    rest = np.arange(n) != bad
+    _, g_ref, _ = oracle32.net_grad(desc, w, stm[rest], nstm[rest], bucket[rest], target[rest])
+    _, g_all, _ = oracle32.net_grad(desc, w, stm, nstm, bucket, target)
+    broken = target.copy()
+    broken[bad] = value
+    net = make_net(desc, 0, w)
+    net.set_option("ft_bwd_products", products)
+    net.upload(0, stm, nstm, bucket, broken)
+    net.upload(1, stm, nstm, bucket, target)
+    lost = np.zeros(desc.n_inputs, dtype=bool)
+    for row in np.concatenate([stm[bad], nstm[bad]]):
+        lost[max(row, 0)] |= row >= 0
+    ref = g_ref["l0w"].reshape(desc.n_inputs, ft_out)
+    for _ in range(2):
+        net.backward(0)
+        assert net.stat("ft_products") == products
+        g = net.tensors(kind=3)
+        got = g["l0w"].reshape(desc.n_inputs, ft_out)
+        assert not np.isfinite(got[lost]).any()
+        assert not np.isfinite(g["l0b"]).any()
+        assert np.abs(got[~lost] - ref[~lost]).max() <= 2e-5 * np.abs(ref).max()
+        first = net.tensor_range("l0w")[0]
+        assert np.isfinite(net_flat(net, 3)[first + got.size:]).all()
+        net.backward(1)
+        g = net.tensors(kind=3)
+        for k in g_all:
+            assert np.abs(g[k] - g_all[k]).max() <= 2e-5 * np.abs(g_all[k]).max(), k
+    net.close()
+
+
 @pytest.mark.parametrize("nnz", [8, 32, 64])
 @pytest.mark.parametrize("rows_less", [0, 3, 16])
 def test_the_largest_tables_of_the_tiled_kernels(oracle32, nnz, rows_less):
@@ -150,8 +226,9 @@ def test_the_largest_tables_of_the_tiled_kernels(oracle32, nnz, rows_less):
         assert np.abs(g[k] - g_ref[k]).max() <= 2e-5 * np.abs(g_ref[k]).max(), k
     net.close()
     for entry in ("b200_op_ft_forward", "b200_op_ft_forward_noalloc"):
-        rc, x, _ = run_op(entry, desc, w["l0w"], w["l0b"], stm, nstm, n)
-        assert rc == 0 and np.array_equal(x, x_ref)
+        for x_at in (0, 1):  # (outputs on any float: grouped, however few positions there are)
+            rc, x, _ = run_op(entry, desc, w["l0w"], w["l0b"], stm, nstm, n, x_at)
+            assert rc == 0 and np.array_equal(x, x_ref)
 
 
 @pytest.mark.parametrize("rows", [855, 860, 861, 863, 865, 866])
@@ -200,8 +277,9 @@ def test_grouping_of_long_batches(oracle32, n):
         # (the oracle adds n terms one after the other: sqrt(n) 2^-24 of the sum in a random walk, and as much again for a drift)
         assert np.abs(g[k] - g_ref[k]).max() <= 6e-5 * np.abs(g_ref[k]).max(), k
     net.close()
-    rc, x, _ = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], *batch[:2], n)
-    assert rc == 0 and np.array_equal(x, x_ref)
+    for x_at in (0, 1):
+        rc, x, _ = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], *batch[:2], n, x_at)
+        assert rc == 0 and np.array_equal(x, x_ref)
 
 
 @pytest.mark.parametrize("case", ["blocks-32", "blocks-33", "blocks-256", "blocks-257", "rows-32-last-layer", "list-of-64", "width-8"])
@@ -419,11 +497,11 @@ PRODUCTS = {
     "rows-31": (31, 3, 20, 64, False, ACT_SCRELU, (1,), 4, 700, False),
     "rows-32": (32, 1, 32, 40, False, ACT_CRELU, (8, 1), 2, 65, False),
     "rows-147-ragged-width": (147, 1, 49, 72, False, ACT_CRELU, (1,), 1, 1000, False),
-    "rows-255": (255, 2, 64, 96, False, ACT_SCRELU, (4, 1), 1, 129, False),
+    "rows-255": (255, 2, 64, 128, False, ACT_SCRELU, (4, 1), 1, 129, False),
     "rows-223": (223, 1, 9, 64, False, ACT_CRELU, (1,), 3, 4000, False),
-    "rows-255-pairwise": (255, 2, 32, 136, True, ACT_CRELU, (16, 32, 1), 8, 900, False),
+    "rows-255-pairwise": (255, 1, 32, 136, True, ACT_CRELU, (16, 32, 1), 8, 900, False),
     "rows-255-pairwise-one": (255, 1, 32, 64, True, ACT_CRELU, (1,), 1, 64, False),
-    "counts": (150, 2, 40, 96, False, ACT_CRELU, (1,), 2, 300, True),
+    "counts": (150, 2, 40, 64, False, ACT_CRELU, (1,), 2, 300, True),
     "counts-pairwise": (200, 1, 64, 128, True, ACT_CRELU, (8, 1), 1, 150, True),
     "sums-taken-out-on-the-way": (2, 1, 1, 32, False, ACT_CRELU, (1,), 1, 2600000, False),
 }
@@ -488,7 +566,13 @@ def test_products_of_bytes_are_no_further_from_64_bits_than_the_walk(case):
         net.step(0, 0.0, 1.0 / n)
         net.loss()
         g = net.tensors(kind=3)
-        (table, bias), _ = sums_in_64_bits(net, desc, batch)
+        (table, bias), magnitudes = sums_in_64_bits(net, desc, batch)
+        assert net.stat("ft_products") == products
+        if products:
+            # every single sum, in units of 2^-24 of its magnitudes: two for an addend, twelve for the eight digits' sums put together,
+            # 148 parts at most (see test_small_gradients_beside_large_ones_keep_32_bits)
+            for k, ref, all_of_it in zip(("l0w", "l0b"), (table, bias), magnitudes):
+                assert (np.abs(g[k].reshape(ref.shape) - ref) <= 162 * 2.0 ** -24 * all_of_it).all(), k
         error[products] = [np.linalg.norm(g[k].astype(np.float64).reshape(ref.shape) - ref) / max(np.linalg.norm(ref), 1e-300)
                            for k, ref in (("l0w", table), ("l0b", bias))]
         print(case, "products" if products else "walk", error[products])
@@ -532,6 +616,7 @@ def test_small_gradients_beside_large_ones_keep_32_bits(products, dense, pairwis
     batch = (stm, nstm, bucket, target.astype(np.float32))
     net.upload(0, *batch)
     net.step(0, 0.0, 1.0 / n)
+    assert net.stat("ft_products") == products
     g = net.tensors(kind=3)
     sums, magnitudes = sums_in_64_bits(net, desc, batch)
     for k, ref, all_of_it in zip(("l0w", "l0b"), sums, magnitudes):
