@@ -135,8 +135,10 @@ int check_op(const b200_ft_op* op, const char* who) {
 // takes them as they are.  Its time goes with the bytes of the rows, which the slots bound (about half of them are active).  Whole
 // call on a B200, gathered / grouped, us: 64 positions 20 to 24 / 36 to 230; king buckets x 1024 columns 1024 positions 38 / 58, 2048
 // (537 MB) 54 / 60, 4096 84 / 72; x 128 columns 8192 35 / 45, 16384 (537 MB) 50.5 / 52, pairwise x 2048 columns 1024 (537 MB) 71 / 81, 2048 106 / 89;
-// 768 rows x 128 columns 16384 (537 MB) 48 / 50, x 2048 columns 2048 77 / 60; 147 rows x 256 columns 8192 (822 MB) 54 / 69, x 2048 columns 512 40 / 59,
-// 2048 (1644 MB) 89 / 82.  Outputs that start on any float are for the tiled kernel.
+// 768 rows x 128 columns 16384 (537 MB) 48 / 50, x 2048 columns 2048 77 / 60; 147 rows x 256 columns 8192 (822 MB) 54 / 69 (given up: one
+// line for all tables), x 2048 columns 512 40 / 59, 2048 (1644 MB) 89 / 82.  Lists that are full instead of half full lose near the line where one
+// large block is all there is: 768 rows x 128 columns 16384 55 / 49, x 2048 columns 1024 57 / 51; 16 blocks x 1024 columns 2048 60 / 59.  Outputs that
+// start on any float are for the tiled kernel.
 constexpr long long kGatherMost = 576LL << 20;
 bool few_positions(const b200_ft_op* op) {
     if (((uintptr_t)op->bias | (uintptr_t)op->x | (op->pairwise ? (uintptr_t)op->u : 0)) & 15) return false;
