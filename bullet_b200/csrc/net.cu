@@ -264,7 +264,7 @@ struct b200_net {
     //   255 x 1, 4 of 8: 32768 x 256 35 / 47 (walks);  64 x 1, 8 of 16: 32768 x 256 43 / 37, pairwise 16384 x 512 48 / 63 (walks)
     //   200 x 8, 17 of 32: 16384 x 256 33 / 28, 1024 x 2048 24 / 34 (walks), pairwise 32768 x 1024 246 / 254 (walks)
     //   147 x 64, 17 of 32: 16384 x 256 43 / 38 (given up), 1024 x 2048 52 / 131 (walks);  31 x 1000, 4 of 8: 1024 x 2048 293 / 762 (walks)
-    // Lists that are emptier than half may get the slower form: 255 rows, 4 of 32 slots, loses 12 us of 96 at 32768 x 256.
+    // Lists that are emptier than half may get the slower form: 255 rows, 4 of 32 slots, 32768 x 256 loses 13 of 98 us.
     bool products_pay(int n) const {
         const long long steps = ((long long)2 * n + b200::kStepPairs - 1) / b200::kStepPairs, blocks = std::min<long long>(nblocks, 2LL * n);
         const long long product = (d.pairwise ? 1700 : 900) + b200::ft_mma_rows(block_rows) * 22 / 10, walk = 900 + 85 * d.nnz / 2;
