@@ -26,6 +26,7 @@
 
 #include "launch.cuh"
 #include "peer_flags.cuh"
+#include "tmem.cuh"
 
 namespace b200 {
 
@@ -98,6 +99,7 @@ struct TileArgs {
     const uint16_t* lists;  // [2n][list_len]
     int list_len;     // nnz rounded up to a multiple of 8 (16-byte groups)
     int walk_warps;   // forward: see ft_fwd_warps
+    int fill_steps;   // forward: rounds of 128 rows of a tile
     // backward only: the visiting order cut into chunks of at most kChunkMost pairs that never
     // straddle a block, and per chunk the row-major lists built by ft_csr_kernel
     const int4* chunks;            // [nchunks] (block, first index into `pairs`, pairs, 0)
@@ -413,6 +415,10 @@ __device__ __forceinline__ void store_piece(float* p, float4 v) {
 // the lanes load them as 32-bit words into registers while the pairs before are still being walked, and store them into the
 // warp's buffer afterwards, so the walk itself reads no global memory.  Every lane adds its four columns with one 16-byte
 // shared-memory load and two packed adds per row, in slot order — the same order and arithmetic as the interpreter.
+// AHEAD: while a tile is walked the next one is fetched into tensor memory (64 columns of 32 lanes for each warp, which no other
+// warp touches), and copied from there when all warps have left the tile.  Fetched only then it kept the pipe idle for 26 k of 105 k clocks
+// per tile at 16384 positions (c3: 262 against 231 us).  Each warp fetches its share in one go, with the registers of the walk free, the warps
+// one after the other; a piece of it in every round instead, held in registers through the walk, cost the walk more than it saved at 131072.
 // Bound by the shared-memory pipe: 256 bytes per (row, pair, slab) at 128 bytes a clock.  (One pair per warp, 8 bytes per
 // lane, spent twice the instructions per row and was bound by their issue: 1.69 against 1.55 ms at 131072 positions and
 // width 2048, 0.273 against 0.260 ms at 16384.)
@@ -430,9 +436,18 @@ __host__ __device__ inline size_t ft_fwd_smem(int R, int list_len) {
     return (size_t)R * kTileRowBytes + (size_t)ft_fwd_warps(R, list_len) * list_len * 4 + 16;
 }
 
+// Whether the CTAs of a launch fetch a next tile while they walk (AHEAD): where many of them have one, and rounds enough to fetch it in.
+// Forward on a B200, without / with, us: 768 x 16 rows, 16384 positions, 2048 columns pairwise 252 / 231, 131072 positions 1547 / 1549,
+// 1024 columns 136 / 132, 256 columns 39 / 39; 625 pairs a tile (5003 x 512) 40.3 / 39.2, but no gain in the whole pass; 375 (3000 x 64)
+// 16.5 / 18.5, 188 (1500 x 2048) 46 / 48; two tiles in all (768 rows x 128 columns) 20.8 / 21.2.
+inline bool ft_fwd_ahead(const FtArgs& a, const TileArgs& t, int grid) {
+    const long long pairs_per_tile = 2LL * a.n / (a.n_inputs / t.block_rows);
+    return 2LL * t.nslabs * (t.last_block - t.first_block) > grid && pairs_per_tile >= 1024;
+}
+
 // ANY: bias, x and u start on any float (the operator's caller owns them); else on 8 bytes with the pairwise product, on 16
 // without, and move in pieces of that size.
-template <bool PAIRWISE, bool ANY = false>
+template <bool PAIRWISE, bool AHEAD, bool ANY = false>
 __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs a, TileArgs t) {
     ft_step_begin(a);
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -441,41 +456,50 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
     const int R = t.block_rows, half = lane >> 4, l16 = lane & 15;
     const uint32_t lane16 = 16 * l16;
     float* tile = reinterpret_cast<float*>(smem_raw);
-    // this CTA's piece [v, v_end) of the line of nslabs x (pairs of the launch's blocks) positions
-    const int pair0 = t.block_begin[t.first_block];
-    const long long line = (long long)t.nslabs * (t.block_begin[t.last_block] - pair0);
-    long long v = line * blockIdx.x / gridDim.x;
-    const long long v_end = line * (blockIdx.x + 1) / gridDim.x;
-    int block = t.first_block;
     // outputs of pair p start at p * (row length): x is [n][2 persp][H or H/2], u is [n][2][H]
     const int x_row = PAIRWISE ? a.H / 2 : a.H;
     const int words = t.list_len;  // 32-bit words of two lists
     uint32_t* ring = reinterpret_cast<uint32_t*>(smem_raw + (size_t)R * kTileRowBytes) + warp * words;
     const uint2* list = reinterpret_cast<const uint2*>(ring + half * (words / 2));
     const uint32_t* lists_w = reinterpret_cast<const uint32_t*>(t.lists);
-    while (v < v_end) {
-        // the segment v lies in: block, slab, first pair
-        long long base = (long long)t.nslabs * (t.block_begin[block] - pair0);
-        int in_block = t.block_begin[block + 1] - t.block_begin[block];
-        while (v >= base + (long long)t.nslabs * in_block) {
-            base += (long long)t.nslabs * in_block;
+    // This CTA's piece of the line of nslabs x (pairs of the launch's blocks) positions is walked in segments, runs of pairs of
+    // one tile.  `rest`: pairs from the segment's first one on; the segments after the first start at their tile's first pair.
+    int block = t.first_block, slab = 0, first, rest;
+    {
+        const int pair0 = t.block_begin[block];
+        const long long line = (long long)t.nslabs * (t.block_begin[t.last_block] - pair0), v = line * blockIdx.x / gridDim.x;
+        rest = (int)(line * (blockIdx.x + 1) / gridDim.x - v);
+        if (rest <= 0) return;
+        long long at = v;
+        int in_block = t.block_begin[block + 1] - pair0;
+        while (at >= (long long)t.nslabs * in_block) {
+            at -= (long long)t.nslabs * in_block;
             block++;
             in_block = t.block_begin[block + 1] - t.block_begin[block];
         }
-        const int slab = (int)((v - base) / in_block), first = (int)((v - base) % in_block);
-        const int last = (int)min((long long)in_block, first + (v_end - v));
-        v += last - first;
-        __syncthreads();  // every warp has left the previous tile
-        {   // fill the tile: eight threads per row, each two 16-byte pieces that its neighbours continue
-            // with a factoriser the table row is l0w[row] + l0f[row mod factor_rows], one fp32 add per
-            // element exactly as the reference forms `l0w + l0f.repeat(n)` (model/builder.rs:421-424)
-            const float* src = a.table + (size_t)block * R * a.H;
-            const int q = threadIdx.x & 7, c0 = PAIRWISE ? slab * 32 + q * 4 : slab * 64 + q * 4, c1 = PAIRWISE ? a.H / 2 + c0 : c0 + 32;
-            const bool in0 = c0 < x_row, in1 = PAIRWISE ? in0 : c1 < x_row;  // the last slab of a width that 64 does not divide
+        slab = (int)(at / in_block);
+        first = t.block_begin[block] + (int)(at - (long long)slab * in_block);
+    }
+    auto next_tile = [&](int& block, int& slab) {
+        if (++slab < t.nslabs) return;
+        slab = 0;
+        do block++;
+        while (t.block_begin[block + 1] == t.block_begin[block]);
+    };
+    // A tile's rows are filled in by eight threads each, two 16-byte pieces of a thread that its neighbours continue.
+    // With a factoriser the table row is l0w[row] + l0f[row mod factor_rows], one fp32 add per element exactly as the
+    // reference forms `l0w + l0f.repeat(n)` (model/builder.rs:421-424).
+    const int q = threadIdx.x & 7, row0 = threadIdx.x >> 3;
+    constexpr int kFillRows = kFwdThreads / 8;
+    auto fill = [&](int block, int slab, auto put) {
+        const float* src = a.table + (size_t)block * R * a.H;
+        const int c0 = PAIRWISE ? slab * 32 + q * 4 : slab * 64 + q * 4, c1 = PAIRWISE ? a.H / 2 + c0 : c0 + 32;
+        const bool in0 = c0 < x_row, in1 = PAIRWISE ? in0 : c1 < x_row;  // the last slab of a width that 64 does not divide
 #pragma unroll 3
-            for (int row = threadIdx.x >> 3; row < R; row += kFwdThreads / 8) {
-                float4* dst = reinterpret_cast<float4*>(tile + row * kTileCols);
-                float4 v0 = make_float4(0, 0, 0, 0), v1 = v0;
+        for (int step = 0; step < t.fill_steps; step++) {
+            const int row = row0 + step * kFillRows;
+            float4 v0 = make_float4(0, 0, 0, 0), v1 = v0;
+            if (row < R) {
                 if (in0) v0 = ld_once4(reinterpret_cast<const float4*>(src + (size_t)row * a.H + c0));
                 if (in1) v1 = ld_once4(reinterpret_cast<const float4*>(src + (size_t)row * a.H + c1));
                 if (a.factor) {
@@ -483,20 +507,56 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
                     if (in0) v0 = add4(v0, __ldg(reinterpret_cast<const float4*>(frow + c0)));
                     if (in1) v1 = add4(v1, __ldg(reinterpret_cast<const float4*>(frow + c1)));
                 }
-                if (PAIRWISE) {
-                    // the tile row holds (low-half column, its high-half partner) side by side, both factors of one product.
-                    // (A thread's pieces lie next to each other, 32 bytes from its neighbour's: the upper four threads of a
-                    // row store their second piece first, so that the eight stores of a quarter warp fall into eight
-                    // different bank groups)
-                    const int h = q >> 2;
-                    const float4 first4 = make_float4(v0.x, v1.x, v0.y, v1.y), second4 = make_float4(v0.z, v1.z, v0.w, v1.w);
-                    dst[2 * q + h] = h ? second4 : first4;
-                    dst[2 * q + (h ^ 1)] = h ? first4 : second4;
-                } else {
-                    dst[q] = v0;
-                    dst[q + 8] = v1;
-                }
             }
+            put(step, row, v0, v1);
+        }
+    };
+    auto put_row = [&](int row, const float4& v0, const float4& v1) {
+        float4* dst = reinterpret_cast<float4*>(tile + row * kTileCols);
+        if (PAIRWISE) {
+            // the tile row holds (low-half column, its high-half partner) side by side, both factors of one product.
+            // (A thread's pieces lie next to each other, 32 bytes from its neighbour's: the upper four threads of a
+            // row store their second piece first, so that the eight stores of a quarter warp fall into eight
+            // different bank groups)
+            const int h = q >> 2;
+            const float4 first4 = make_float4(v0.x, v1.x, v0.y, v1.y), second4 = make_float4(v0.z, v1.z, v0.w, v1.w);
+            dst[2 * q + h] = h ? second4 : first4;
+            dst[2 * q + (h ^ 1)] = h ? first4 : second4;
+        } else {
+            dst[q] = v0;
+            dst[q + 8] = v1;
+        }
+    };
+    const uint32_t spare = tmem_own(warp, 64);
+    bool filled = false;
+    for (;;) {
+        const int seg_end = min(t.block_begin[block + 1], first + rest);
+        rest -= seg_end - first;
+        int i = warp < NW ? first + 2 * warp : seg_end;
+        int2 next = make_int2(0, 0);  // this half's next pair and its length
+        uint32_t w0 = 0, w1 = 0;      // this lane's words of the next two lists
+        auto fetch = [&](int at) {
+            if (at + half < seg_end) next = __ldg(t.pairs + at + half);
+            // (a single last pair: the second list of the two may lie past the end of the lists)
+            const int have = at + 1 < seg_end ? words : words / 2;
+            const uint32_t* src = lists_w + (size_t)at * (words / 2);
+            if (at < seg_end && lane < have) w0 = __ldg(src + lane);
+            if (at < seg_end && lane + 32 < have) w1 = __ldg(src + lane + 32);
+        };
+        fetch(i);
+        if (AHEAD && !filled && rest > 0 && warp == 0) tmem_alloc_all(ring);  // (the word is not needed, the lists come later)
+        __syncthreads();  // every warp has left the previous tile
+        if (AHEAD && filled) {
+            tmem_stored();
+            for (int row = row0, at = 0; at < t.fill_steps; row += kFillRows, at++) {
+                float4 v0, v1;
+                tmem_get8(spare + 8 * at, v0, v1);
+                if (row < R) put_row(row, v0, v1);
+            }
+        } else {
+            fill(block, slab, [&](int step, int row, const float4& v0, const float4& v1) {
+                if (row < R) put_row(row, v0, v1);
+            });
         }
         // this lane's columns: two products, or four neighbours
         const int col = PAIRWISE ? slab * 32 + 2 * l16 : slab * 64 + 4 * l16;
@@ -515,20 +575,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
         }
         float* x_out = a.x + col;
         __syncthreads();
-        const int seg_end = t.block_begin[block] + last;
-        int i = warp < NW ? t.block_begin[block] + first + 2 * warp : seg_end;
-        int2 next = make_int2(0, 0);  // this half's next pair and its length
-        uint32_t w0 = 0, w1 = 0;      // this lane's words of the next two lists
-        auto fetch = [&](int at) {
-            if (at + half < seg_end) next = __ldg(t.pairs + at + half);
-            // (a single last pair: the second list of the two may lie past the end of the lists)
-            const int have = at + 1 < seg_end ? words : words / 2;
-            const uint32_t* src = lists_w + (size_t)at * (words / 2);
-            if (at < seg_end && lane < have) w0 = __ldg(src + lane);
-            if (at < seg_end && lane + 32 < have) w1 = __ldg(src + lane + 32);
-        };
-        fetch(i);
-        for (; i < seg_end; i += 2 * NW) {
+        auto round = [&]() {
             const int pair = next.x, cnt = i + half < seg_end ? next.y : 0;
             __syncwarp();  // every lane has finished with the lists of the pairs before
             if (lane < words) ring[lane] = w0;
@@ -549,8 +596,23 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
                         make_float4(ft_act_fwd(a.act, lo2(acc.a)), ft_act_fwd(a.act, hi2(acc.a)), ft_act_fwd(a.act, lo2(acc.b)), ft_act_fwd(a.act, hi2(acc.b))));
                 }
             }
+            i += 2 * NW;
+        };
+        if (AHEAD && rest > 0) {
+            const int turn = i + (seg_end - first) / (2 * NW) * warp / 32 * 2 * NW;
+            while (i < min(turn, seg_end)) round();
+            __syncwarp();
+            int next_block = block, next_slab = slab;
+            next_tile(next_block, next_slab);
+            fill(next_block, next_slab, [&](int step, int row, const float4& v0, const float4& v1) { tmem_put8(spare + 8 * step, v0, v1); });
+            filled = true;
         }
+        while (i < seg_end) round();
+        if (rest == 0) break;
+        next_tile(block, slab);
+        first = t.block_begin[block];
     }
+    if (AHEAD && filled && warp == 0) tmem_free_all();  // (every access lies before the last tile's barrier)
 }
 
 // Backward.  Positions are visited in chunks of at most CP pairs of one row block.

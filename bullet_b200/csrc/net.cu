@@ -406,7 +406,7 @@ void slot_layout(const b200_net* net, Slot& s, int n) {
 template <bool PW>
 int launch_ft_forward(b200_net* net, const b200::FtArgs& a, const b200::TileArgs& t, bool tiled, int grid) {
     if (tiled) {
-        CK(b200::launch_step(false, b200::ft_forward_tiled_kernel<PW>, grid, b200::kFwdThreads, b200::ft_fwd_smem(t.block_rows, t.list_len), net->stream, a, t));
+        CK(b200::launch_step(false, b200::ft_fwd_ahead(a, t, grid) ? b200::ft_forward_tiled_kernel<PW, true> : b200::ft_forward_tiled_kernel<PW, false>, grid, b200::kFwdThreads, b200::ft_fwd_smem(t.block_rows, t.list_len), net->stream, a, t));
     } else {
         const int unit = PW ? a.H / 2 : a.H;
         const int pairs = b200::gather_pairs(a.n, unit, net->sm_count);
@@ -587,6 +587,7 @@ b200::TileArgs tile_args(b200_net* net, const Slot& s, bool backward) {
     t.lists = s.lists;
     t.list_len = (net->d.nnz + 7) & ~7;
     t.walk_warps = b200::ft_fwd_warps(net->block_rows, t.list_len);
+    t.fill_steps = (t.block_rows + b200::kFwdThreads / 8 - 1) / (b200::kFwdThreads / 8);
     t.chunks = s.dev<int4>(s.off_chunks);
     t.csr_ent = s.csr_ent;
     t.csr_start = s.csr_start;
@@ -959,7 +960,7 @@ int preload_kernels(b200_net* net) {
     ok = ok && load_kernel(b200::dense_regroup_kernel) && load_kernel(dense_one_form(net, false)) && (!net->small_table() || load_kernel(dense_one_form(net, true))) && load_kernel(b200::dense_one_dx_kernel) && load_kernel(b200::copy_outputs_kernel) && load_kernel(b200::dense_fragments_kernel) && load_kernel(b200::dense_small_grads_kernel);
     ok = ok && load_kernel(b200::ft_forward_gather_kernel<true, true>) && load_kernel(b200::ft_forward_gather_kernel<true, false>) && load_kernel(b200::ft_forward_gather_kernel<false, true>) && load_kernel(b200::ft_forward_gather_kernel<false, false>);
     ok = ok && load_kernel(b200::ft_backward_gather_kernel<true, true>) && load_kernel(b200::ft_backward_gather_kernel<true, false>) && load_kernel(b200::ft_backward_gather_kernel<false, true>) && load_kernel(b200::ft_backward_gather_kernel<false, false>);
-    ok = ok && load_kernel(b200::ft_forward_tiled_kernel<true>) && load_kernel(b200::ft_forward_tiled_kernel<false>);
+    ok = ok && load_kernel(b200::ft_forward_tiled_kernel<true, true>) && load_kernel(b200::ft_forward_tiled_kernel<true, false>) && load_kernel(b200::ft_forward_tiled_kernel<false, true>) && load_kernel(b200::ft_forward_tiled_kernel<false, false>);
     ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, true, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, true, false>);
     ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 512, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 512, true, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, true, false>);
     ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, false, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, false, false>);
@@ -1181,8 +1182,10 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
         if (b200::allow_smem(dense_one_form(net, false)) != cudaSuccess || (net->small_table() && b200::allow_smem(dense_one_form(net, true)) != cudaSuccess)) return bail(b200::fail(B200_ERR_CUDA, "net_create: shared memory of the dense kernel"));
     }
     if (net->tiled_ok) {
-        cudaError_t e = b200::allow_smem(b200::ft_forward_tiled_kernel<true>);
-        e = e ? e : b200::allow_smem(b200::ft_forward_tiled_kernel<false>);
+        cudaError_t e = b200::allow_smem(b200::ft_forward_tiled_kernel<true, true>);
+        e = e ? e : b200::allow_smem(b200::ft_forward_tiled_kernel<true, false>);
+        e = e ? e : b200::allow_smem(b200::ft_forward_tiled_kernel<false, true>);
+        e = e ? e : b200::allow_smem(b200::ft_forward_tiled_kernel<false, false>);
         e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 1024, true, true>);
         e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 1024, true, false>);
         e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 1024, true, true>);

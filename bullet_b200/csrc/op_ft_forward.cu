@@ -236,14 +236,18 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
     t.lists = g.lists;
     t.list_len = g.list_len;
     t.walk_warps = b200::ft_fwd_warps(R, t.list_len);
+    t.fill_steps = (t.block_rows + b200::kFwdThreads / 8 - 1) / (b200::kFwdThreads / 8);
     const size_t smem = b200::ft_fwd_smem(R, t.list_len);
     // one CTA per SM, each taking an equal piece of the (block, slab, pair) work line
     const int ctas = (int)std::max<long long>(1, std::min<long long>(sms, (long long)2 * n * t.nslabs / 128));
     // the caller's arrays may start on any float: pieces of 8 and 16 bytes where they do so, else single floats
     const bool any = (((uintptr_t)op->bias | (uintptr_t)op->x | (op->pairwise ? (uintptr_t)op->u : 0)) & (op->pairwise ? 7 : 15)) != 0;
+    const bool ahead = b200::ft_fwd_ahead(a, t, ctas);
     void (*const kernel)(b200::FtArgs, b200::TileArgs) =
-        op->pairwise ? (any ? b200::ft_forward_tiled_kernel<true, true> : b200::ft_forward_tiled_kernel<true>)
-                     : (any ? b200::ft_forward_tiled_kernel<false, true> : b200::ft_forward_tiled_kernel<false>);
+        ahead ? (op->pairwise ? (any ? b200::ft_forward_tiled_kernel<true, true, true> : b200::ft_forward_tiled_kernel<true, true, false>)
+                              : (any ? b200::ft_forward_tiled_kernel<false, true, true> : b200::ft_forward_tiled_kernel<false, true, false>))
+              : (op->pairwise ? (any ? b200::ft_forward_tiled_kernel<true, false, true> : b200::ft_forward_tiled_kernel<true, false, false>)
+                              : (any ? b200::ft_forward_tiled_kernel<false, false, true> : b200::ft_forward_tiled_kernel<false, false, false>));
     CK(b200::allow_smem(kernel));
     kernel<<<ctas, b200::kFwdThreads, smem, stream>>>(a, t);
     CK(cudaGetLastError());

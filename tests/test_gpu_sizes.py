@@ -684,3 +684,48 @@ def test_small_tables_take_the_faster_backward(case):
     net.loss()
     assert net.stat("ft_products") == products
     net.close()
+
+
+@pytest.mark.parametrize("blocks,rows,ft_out,nnz,pairwise,factoriser,used", [
+    (3, 128, 1664, 16, False, 0, (0, 1, 2)),       # a whole round of rows
+    (3, 129, 1664, 16, True, 129, (0, 1, 2)),      # one row more, in the second round
+    (2, 31, 2432, 31, True, 0, (0, 1)),            # less than a round
+    (5, 200, 2048, 20, False, 200, (1, 3)),        # blocks without pairs between the tiles
+    (2, 768, 2560, 32, True, 768, (0, 1)),
+    (2, 860, 2432, 64, False, 0, (0, 1)),          # the last rounds of rows, warps that walk no lists
+    (1, 300, 4808, 12, False, 0, (0,)),            # a last slab that is not full
+    (1, 300, 4816 * 2, 12, True, 0, (0,)),
+])
+def test_tiles_fetched_while_the_one_before_is_walked(oracle32, blocks, rows, ft_out, nnz, pairwise, factoriser, used):
+    """More tiles than CTAs, with enough pairs each for the forward to fetch a CTA's next tile during the walk: rows at the edges of the
+    rounds it is fetched in, over several tiles a CTA.  Bit-exact, network (a whole batch and in parts) and operator."""
+    import dataclasses
+
+    from tests.test_gpu_ops import run_op
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    n = 515 * blocks + 7
+    desc = dataclasses.replace(net_of(blocks, rows, ft_out, nnz, 1, (1,), pairwise=pairwise), max_batch=n, factoriser_rows=factoriser)
+    if blocks == 1:
+        desc = dataclasses.replace(desc, ft_block_rows=0)
+    stm, nstm, bucket, target = draw_batch(desc, n, seed=rows + ft_out)
+    for index in (stm, nstm):  # into the blocks that are used
+        at = np.array(used)[index // rows % len(used)]
+        np.copyto(index, np.where(index >= 0, at * rows + index % rows, -1))
+    w = rich_weights(desc)
+    x_ref = oracle_x(oracle32, desc, w, stm, nstm)
+    net = make_net(desc, 0, w)
+    net.upload(0, stm, nstm, bucket, target)
+    net.forward(0, n)
+    assert np.array_equal(net.activation(0, n * desc.dense_in0).reshape(n, -1), x_ref)
+    if blocks > 1:
+        net.forward_begin(0)
+        for part in range(blocks):
+            net.forward_ft(0, part, blocks)
+        net.backward_begin(0)
+        assert np.array_equal(net.activation(0, n * desc.dense_in0).reshape(n, -1), x_ref)
+        if not factoriser:
+            for x_at in (0, 1):
+                rc, x, _ = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], stm, nstm, n, x_at)
+                assert rc == 0 and np.array_equal(x, x_ref)
+    net.close()
