@@ -106,7 +106,6 @@ struct TileArgs {
     uint16_t* csr_ent;             // [nchunks][ent_cap] pairs of the chunk grouped by row, every list starting on 16 bytes
     int* csr_start;                // [nchunks][start_cap] per row (start / 8) << 16 | length; [R] = entries in all
     int ent_cap, start_cap;
-    int grab;                      // eighths of the list pieces that the backward deals out in advance
     int chunk_len;  // CP: most pairs per chunk
     int wide;       // 1024 threads per CTA, one per SM; else 512 and two
     // backward only, data-parallel runs: the last CTA of every row block tells all ranks that the block's
@@ -397,6 +396,36 @@ __device__ __forceinline__ f32x4 sum_lines(const unsigned char* lines, const uin
     return acc;
 }
 
+// The same for lists of an even length, whose last entry may be a line of zeros: the backward's pieces are short (11 entries at 512 pairs
+// of a 768-row block), and up to three single lines at their ends cost more instructions than the added half line costs passes through
+// the pipe (c3 282 -> 270 us, c4 1974 -> 1900).  The forward's longer lists lose by it (c3 231 -> 240, 147 rows 70.6 -> 73.3).
+// TWO: the loop unrolled by two groups of four, which helps the backward without the pairwise product (1024 columns 142 -> 137 us), whose
+// warps have the registers, and hurts it with the product (c3 267 -> 270, c4 1847 -> 1871; not unrolled at all 274, 1905).
+template <bool TWO>
+__device__ __forceinline__ f32x4 sum_lines_even(const unsigned char* lines, const uint2* list, int len, uint32_t lane16) {
+    f32x4 acc = {0, 0};
+    uint2 g = *list;
+    auto four = [&]() {
+        const uint2 ahead = *++list;
+        const f32x4 v0 = quad_at(lines, entry_lo(g.x, lane16)), v1 = quad_at(lines, entry_hi(g.x, lane16));
+        const f32x4 v2 = quad_at(lines, entry_lo(g.y, lane16)), v3 = quad_at(lines, entry_hi(g.y, lane16));
+        acc = add2(add2(add2(add2(acc, v0), v1), v2), v3);
+        g = ahead;
+    };
+    len -= 4;
+    if (TWO) {
+#pragma unroll 2
+        for (; len >= 0; len -= 4) four();
+    } else {
+        for (; len >= 0; len -= 4) four();
+    }
+    if (len == -2) {
+        const f32x4 v0 = quad_at(lines, entry_lo(g.x, lane16)), v1 = quad_at(lines, entry_hi(g.x, lane16));
+        acc = add2(add2(acc, v0), v1);
+    }
+    return acc;
+}
+
 template <bool ANY>
 __device__ __forceinline__ void store_piece(float* p, float2 v) {
     if (ANY) p[0] = v.x, p[1] = v.y;
@@ -643,7 +672,7 @@ __host__ __device__ inline int ft_bwd_ent_cap(int R, int nnz, int cp) { return (
 // per chunk: entries, pieces, two unused words, then the pieces: first entry / 4 << 17 | length << 10 | row
 __host__ __device__ inline int ft_bwd_start_cap(int R, int nnz, int cp) { return (4 + R + cp * nnz / kPiece + 3) & ~3; }
 __host__ __device__ inline size_t ft_bwd_smem(int R, int nnz, int cp) {
-    return (size_t)cp * kTileRowBytes + (size_t)ft_bwd_ent_cap(R, nnz, cp) * 2 + (size_t)ft_bwd_start_cap(R, nnz, cp) * 4 + (size_t)cp * 12 +
+    return (size_t)(cp + 1) * kTileRowBytes + (size_t)ft_bwd_ent_cap(R, nnz, cp) * 2 + (size_t)ft_bwd_start_cap(R, nnz, cp) * 4 + (size_t)cp * 12 +
            32 * kTileRowBytes;  // staged lines, row lists, their pieces, what a pair needs, bias-gradient sums per warp
 }
 __host__ __device__ inline size_t ft_csr_smem(int R, int nnz, int cp) {
@@ -709,6 +738,7 @@ static __global__ void __launch_bounds__(kCsrThreads) ft_csr_kernel(FtArgs a, Ti
     const int before = __reduce_add_sync(0xffffffffu, lane < warp ? warp_tot[lane] : 0), total = __reduce_add_sync(0xffffffffu, warp_tot[lane]);
     const int first = before + incl - room;
     if (r < R) start[r] = first;
+    if (mine & 1) ent[first + mine] = (uint16_t)t.chunk_len;
     if (warp == 0) {  // places of the pieces, longest first
         int run = 0;
         for (int base = kPiece; base > 0; base -= 32) {
@@ -739,7 +769,7 @@ static __global__ void __launch_bounds__(kCsrThreads) ft_csr_kernel(FtArgs a, Ti
     if (threadIdx.x == 0) *reinterpret_cast<int4*>(out) = make_int4(total, bin[0], 0, 0);
     for (int k = 0; k < mine; k += kPiece) {
         const int n = min(kPiece, mine - k);
-        out[4 + atomicAdd(&bin[n], 1)] = ((first + k) >> 2) << 17 | n << 10 | r;
+        out[4 + atomicAdd(&bin[n], 1)] = ((first + k) >> 2) << 17 | ((n + 1) & ~1) << 10 | r;
     }
     __syncthreads();
     uint4* ent_out = reinterpret_cast<uint4*>(t.csr_ent + (size_t)blockIdx.x * t.ent_cap);
@@ -807,8 +837,8 @@ __device__ __forceinline__ int2 ft_bwd_units(const TileArgs& t, int k, int parts
 // that must precede the announcement then finds little to wait for).
 //
 // Staging: a pair's line takes 8 lanes (pairwise: 32 columns of each half of the accumulator) or 16 lanes, 16 bytes per
-// load.  Walk: a half warp per list piece (see sum_lines).  Most of the pieces are dealt to the half warps in advance,
-// longest first, the rest handed out by a shared-memory counter.  Bound by the shared-memory pipe in the walk (256 bytes
+// load, the operands of the next pairs but one under way while a pair's are used (two pairs' operands a lane: more of them make the
+// compiler spill).  Walk: a half warp per list piece (see sum_lines_even).  Bound by the shared-memory pipe in the walk (256 bytes
 // per (row, pair, slab)) and by load latency in the staging.  (One row per warp with 8 bytes per lane, rows in table order: 2.29 against 1.97 ms at 131072
 // positions and width 2048, 0.332 against 0.281 ms at 16384.)
 template <bool PAIRWISE, int THREADS, bool SIGNAL, bool ONE>
@@ -820,12 +850,12 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
     constexpr int NW = kBwdThreads / 32;
     const int R = t.block_rows, CP = t.chunk_len;
     float* g_s = reinterpret_cast<float*>(smem_raw);                                       // [CP][64] staged lines
-    uint16_t* ent = reinterpret_cast<uint16_t*>(smem_raw + (size_t)CP * kTileRowBytes);    // lists of the chunk
+    uint16_t* ent = reinterpret_cast<uint16_t*>(smem_raw + (size_t)(CP + 1) * kTileRowBytes);    // lists of the chunk
     int* start = reinterpret_cast<int*>(ent + t.ent_cap);                                  // entries, pieces, -, -, then the pieces
     int* pairs_s = start + t.start_cap;                                                    // [CP] pair ids of the chunk
     float* bias_s = reinterpret_cast<float*>(pairs_s + CP);                                // [warps][64] bias-gradient sums of a unit
     int2* one_s = reinterpret_cast<int2*>(bias_s + NW * kTileCols);                        // ONE: [CP] (loss gradient, first weight) of the pair
-    __shared__ int next_piece;  // the walk's counter
+    if (threadIdx.x < kTileCols) g_s[CP * kTileCols + threadIdx.x] = 0.f;
     const int first_chunk = t.chunk_begin[t.first_block];
     const int2 mine = SIGNAL ? make_int2(blockIdx.x, t.nslabs * (t.chunk_begin[t.last_block] - first_chunk)) : ft_bwd_units(t, blockIdx.x, gridDim.x, lane);
 
@@ -839,27 +869,27 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
     // Bias gradient: a warp leaves the sums of the pairs it staged in its line of bias_s; during the walk two warps add the
     // lines up, a thread per column, and reduce the result to global memory.  (Shared-memory float atomics in their place
     // took an eighth of all passes through the shared-memory pipe.)
-    // staging: this lane's operands of the next U pairs on their way
-    constexpr int U = PAIRWISE ? 2 : 4;
+    // staging: this lane's operands of U pairs on their way
+    constexpr int U = 2, kStep = NW * kPairsPerWarp;
     float4 y0[U], y1[U], d[U];
     const int x_row = PAIRWISE ? a.H / 2 : a.H;  // columns of x per perspective
-    auto fetch = [&](int pl0, int cn, int sl) {
+    auto fetch_one = [&](int k, int pl, int sl) {
         const int col = PAIRWISE ? sl * 32 + 4 * q : sl * 64 + 4 * q;
-#pragma unroll
-        for (int k = 0; k < U; k++) {
-            const int pl = pl0 + k * NW * kPairsPerWarp;
-            if (pl >= cn) break;
-            if (col >= x_row) {  // the last slab of a width that 64 does not divide
-                y0[k] = y1[k] = d[k] = make_float4(0, 0, 0, 0);
-                continue;
-            }
-            const int pair = pairs_s[pl];
-            const float* y = (PAIRWISE ? a.u : a.x) + (size_t)pair * a.H + col;
-            y0[k] = ld_once4(reinterpret_cast<const float4*>(y));
-            if (PAIRWISE) y1[k] = ld_once4(reinterpret_cast<const float4*>(y + a.H / 2));
-            d[k] = ONE ? __ldg(reinterpret_cast<const float4*>(a.w1 + one_s[pl].y + col))
-                       : ld_once4(reinterpret_cast<const float4*>(a.dx + (size_t)pair * x_row + col));
+        if (col >= x_row) {  // the last slab of a width that 64 does not divide
+            y0[k] = y1[k] = d[k] = make_float4(0, 0, 0, 0);
+            return;
         }
+        const int pair = pairs_s[pl];
+        const float* y = (PAIRWISE ? a.u : a.x) + (size_t)pair * a.H + col;
+        y0[k] = ld_once4(reinterpret_cast<const float4*>(y));
+        if (PAIRWISE) y1[k] = ld_once4(reinterpret_cast<const float4*>(y + a.H / 2));
+        d[k] = ONE ? __ldg(reinterpret_cast<const float4*>(a.w1 + one_s[pl].y + col))
+                   : ld_once4(reinterpret_cast<const float4*>(a.dx + (size_t)pair * x_row + col));
+    };
+    auto fetch = [&](int pl0, int cn, int sl) {
+#pragma unroll
+        for (int k = 0; k < U; k++)
+            if (pl0 + k * kStep < cn) fetch_one(k, pl0 + k * kStep, sl);
     };
     bool fetched = false;  // the unit before has fetched this one's first pairs
     int block = -1, ch_loaded = -1, cn = 0;
@@ -918,10 +948,9 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
                     *reinterpret_cast<float4*>(out) = ga;
                     sum_a = add4(sum_a, ga);
                 }
+                if (pl + U * kStep < cn) fetch_one(k, pl + U * kStep, slab);
             }
-            fetch(pl0 + U * NW * kPairsPerWarp, cn, slab);
         }
-        if (threadIdx.x == 0) next_piece = 0;
 #pragma unroll
         for (int o = kLanes; o < 32; o <<= 1) {
             sum_a = add4(sum_a, make_float4(__shfl_xor_sync(0xffffffffu, sum_a.x, o), __shfl_xor_sync(0xffffffffu, sum_a.y, o),
@@ -977,15 +1006,16 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
         }
         const int pieces = start[1];
         auto walk = [&](unsigned piece) {
-            const f32x4 acc = sum_lines(smem_raw, reinterpret_cast<const uint2*>(ent) + (piece >> 17), (int)(piece >> 10) & 0x7f, lane16);
+            const f32x4 acc = sum_lines_even<!PAIRWISE>(smem_raw, reinterpret_cast<const uint2*>(ent) + (piece >> 17), (int)(piece >> 10) & 0x7f, lane16);
             const float4 g = make_float4(lo2(acc.a), hi2(acc.a), lo2(acc.b), hi2(acc.b));
             if (col_on && (g.x != 0.f || g.y != 0.f || g.z != 0.f || g.w != 0.f))
                 atomicAdd(reinterpret_cast<float4*>(g_block + (size_t)(piece & 0x3ffu) * a.H), g);
         };
-        // most pieces are dealt to the half warps, to and fro, so that each gets the same mixture of lengths; the shortest are
-        // handed out by a counter to whoever is done first
+        // The pieces are dealt to the half warps to and fro, longest first, so that each gets the same mixture of lengths: whole rounds, which all
+        // lanes of a warp walk together, then the shortest.  (A counter for the last quarter balanced no better, and its second copy of
+        // the walk and the registers around it cost c4 1900 against 1844 us.)
         constexpr int HW = 2 * NW;
-        const int h = 2 * warp + half, dealt = pieces / HW * t.grab / 8;
+        const int h = 2 * warp + half, dealt = pieces / HW;
         unsigned piece = dealt > 0 ? (unsigned)start[4 + h] : 0u;
         for (int r = 0; r < dealt; r++) {
             const unsigned now = piece;
@@ -993,13 +1023,8 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
             walk(now);
         }
         __syncwarp();
-        for (;;) {
-            int first = 0;
-            if (lane == 0) first = atomicAdd(&next_piece, 2);
-            first = __shfl_sync(0xffffffffu, first, 0) + dealt * HW + half;
-            if (first < pieces) walk((unsigned)start[4 + first]);
-            if (first - half + 2 >= pieces) break;
-        }
+        const int last = dealt * HW + h;
+        if (last < pieces) walk((unsigned)start[4 + last]);
         fetched = next_slab;
         if (next_slab) fetch(warp * kPairsPerWarp + sub, cn, slab + 1);  // (arrives while the slowest warps finish)
         if (SIGNAL) {

@@ -136,7 +136,6 @@ struct b200_net {
     bool bwd_wide = true;  // shape of the tiled backward (see kChunkMost)
     int bwd_products = -1;  // small tables: the product of bytes instead of the walk over row lists, always (1), never (0) or where it pays
     int exchange_bulk = 0;  // the peer exchange moves gradients and weights with bulk asynchronous copies (measured no faster)
-    int bwd_grab = 0;  // eighths of a unit's pieces that the tiled backward deals out in advance (0: the default)
     int wide_chunk = 0;    // the largest chunk of the 1024-thread backward that fits into shared memory
     // Pairs per chunk for a batch of n positions: large chunks save reductions and list copies per pair, small ones fill the
     // SMs evenly when there are few units.  Measured, a unit takes a part that grows with the table's rows and the chunk's
@@ -593,7 +592,6 @@ b200::TileArgs tile_args(b200_net* net, const Slot& s, bool backward) {
     t.csr_start = s.csr_start;
     t.chunk_len = s.chunk_len;
     t.wide = s.wide;
-    t.grab = net->bwd_grab > 0 ? std::min(8, net->bwd_grab) : 6;
     t.ent_cap = s.mma ? b200::ft_mma_ent_cap(net->block_rows) : b200::ft_bwd_ent_cap(net->block_rows, net->d.nnz, s.chunk_len);
     t.start_cap = s.mma ? b200::kStepHead : b200::ft_bwd_start_cap(net->block_rows, net->d.nnz, s.chunk_len);
     if (backward && net->sig_on) {
@@ -1305,8 +1303,7 @@ int b200_net_set_option(b200_net* net, const char* key, int64_t value) {
     }
     if (!strcmp(key, "ft_bwd_grab")) {
         if (value < 0 || value > 64) return b200::fail(B200_ERR_ARG, "ft_bwd_grab must be in [0, 64]");
-        net->bwd_grab = (int)value;  // (more than eight eighths: all of them, see tile_args)
-        return 0;
+        return 0;  // (all pieces are dealt out in advance)
     }
     if (!strcmp(key, "ft_once")) {
         return 0;  // (no load of the tiled kernels gains from an L1 line any more: one form)

@@ -101,7 +101,7 @@ int b200_net_destroy(b200_net* net);
  *   "ft_bwd_products" 0 / 1 = the backward of tables of fewer than 256 rows per block never / always multiplies bytes instead of
  *   walking row lists (-1, the default: where that is faster);
  *   "ft_once" accepted, without effect (one form of loads is left);
- *   "ft_bwd_grab" eighths of a unit's row pieces that the tiled backward deals to its warps in advance (0 = default, more than 8 counts as 8);
+ *   "ft_bwd_grab" 0 to 64, without effect: the tiled backward deals all row pieces of a unit to its warps in advance;
  *   "exchange_bulk" 1 = the peer exchange moves gradients and weights with bulk asynchronous copies;
  *   "overlap_ctas", "overlap_mode", "exchange_ctas", "exchange_wait_ms", "exchange_step", "manual_grad_zero": see the
  *   data-parallel entry points below. */
