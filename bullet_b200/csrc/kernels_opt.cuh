@@ -106,9 +106,7 @@ __global__ void __launch_bounds__(256) adamw_flat_kernel(const __grid_constant__
 
 // The whole update of a single-GPU step in one launch: the factoriser's gradient (g_l0f = sum of the gradients of its copies
 // in l0w, first copy first, reduce.rs:96-120), the update of every tensor, the tables that the next forward reads instead of
-// l1w, and the step's loss and status word straight into pinned memory.  A thread that owns four columns of a factoriser row
-// owns them in all its copies: it sums their gradients while it updates them, so the table gradient is read once (the sum
-// used to be a kernel of its own that read it again).  HBM: 28 bytes per parameter.
+// l1w, and the step's loss and status word straight into pinned memory.  HBM: 28 bytes per parameter.
 struct StepUpdateArgs {
     AdamArgs adam;             // first4, total4 unused
     float4* g;                 // gradients, writable (l0f's is formed here)
@@ -148,50 +146,97 @@ __device__ __forceinline__ void store_w1(const StepUpdateArgs& u, long long e, f
     }
 }
 
-__global__ void __launch_bounds__(256, 3) step_update_kernel(const __grid_constant__ StepUpdateArgs u) {
-    step_begin(u.stamps ? u.stamps + 4 : nullptr);
+// What both kernels do with the float4 at index `i`: load and update.
+// (The moments are not needed before the next update: they leave L2 to the weights.)
+struct Held {
+    float4 p, m, v;
+};
+__device__ __forceinline__ Held load4(const AdamArgs& a, long long i) { return {a.p[i], __ldcs(a.m + i), __ldcs(a.v + i)}; }
+__device__ __forceinline__ void update4(const AdamArgs& a, const AdamSegment& s, long long i, const float4& g, Held& h) {
+    adam_op(s, a.rate, a.adj * g.x, h.p.x, h.m.x, h.v.x);
+    adam_op(s, a.rate, a.adj * g.y, h.p.y, h.m.y, h.v.y);
+    adam_op(s, a.rate, a.adj * g.z, h.p.z, h.m.z, h.v.z);
+    adam_op(s, a.rate, a.adj * g.w, h.p.w, h.m.w, h.v.w);
+    a.p[i] = h.p;
+    __stcs(a.m + i, h.m);
+    __stcs(a.v + i, h.v);
+}
+// ... and with those of the tensors before l0w but for the factoriser, by the threads `me`, `me` + `stride`, ...
+__device__ __forceinline__ void update_small(const StepUpdateArgs& u, long long me, long long stride) {
     const AdamArgs& a = u.adam;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *(volatile float*)u.h_loss = *u.loss;
-        *(volatile int*)u.h_status = u.status ? *u.status : 0;
-    }
-    const long long stride = (long long)gridDim.x * blockDim.x, me = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    auto update = [&](const AdamSegment& s, long long i, float4 g) {
-        // (the moments are not needed before the next update: they leave L2 to the weights)
-        float4 p = a.p[i], m = __ldcs(a.m + i), v = __ldcs(a.v + i);
-        adam_op(s, a.rate, a.adj * g.x, p.x, m.x, v.x);
-        adam_op(s, a.rate, a.adj * g.y, p.y, m.y, v.y);
-        adam_op(s, a.rate, a.adj * g.z, p.z, m.z, v.z);
-        adam_op(s, a.rate, a.adj * g.w, p.w, m.w, v.w);
-        a.p[i] = p;
-        __stcs(a.m + i, m);
-        __stcs(a.v + i, v);
-        return p;
-    };
-    if (u.l0f_seg >= 0) {
-        const AdamSegment &sw = a.seg[u.l0w_seg], &sf = a.seg[u.l0f_seg];
-        for (long long j = me; j < u.block4; j += stride) {
-            float4 sum = make_float4(0, 0, 0, 0);
-#pragma unroll 4
-            for (int c = 0; c < u.copies; c++) {
-                const long long i = u.l0w4 + c * u.block4 + j;
-                const float4 g = u.g[i];
-                if (c == 0) sum = g;
-                else sum.x += g.x, sum.y += g.y, sum.z += g.z, sum.w += g.w;
-                update(sw, i, g);
-            }
-            u.g[u.l0f4 + j] = sum;
-            update(sf, u.l0f4 + j, sum);
-        }
-    }
-    for (long long i = me; i < u.rest4; i += stride) {
+    const long long skipped = u.l0f_seg >= 0 ? u.block4 : 0;
+    for (long long j = me; j < u.rest4 - skipped; j += stride) {
+        const long long i = j >= u.l0f4 ? j + skipped : j;
         int si = -1;
 #pragma unroll 1
         for (int k = 0; k < a.nseg; k++)
             if (i >= a.seg[k].begin4 && i < a.seg[k].end4) si = k;
-        if (si < 0 || si == u.l0f_seg) continue;  // alignment padding between tensors
-        const float4 p = update(a.seg[si], i, u.g[i]);
-        if (i >= u.l1w4_begin && i < u.l1w4_end) store_w1(u, 4 * (i - u.l1w4_begin), p);
+        if (si < 0) continue;  // alignment padding between tensors
+        Held h = load4(a, i);
+        update4(a, a.seg[si], i, u.g[i], h);
+        if (i >= u.l1w4_begin && i < u.l1w4_end) store_w1(u, 4 * (i - u.l1w4_begin), h.p);
+    }
+}
+__device__ __forceinline__ void update_begin(const StepUpdateArgs& u) {
+    step_begin(u.stamps ? u.stamps + 4 : nullptr);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *(volatile float*)u.h_loss = *u.loss;
+        *(volatile int*)u.h_status = u.status ? *u.status : 0;
+    }
+}
+
+// Networks without a factoriser: all tensors.
+__global__ void __launch_bounds__(256, 3) step_update_kernel(const __grid_constant__ StepUpdateArgs u) {
+    update_begin(u);
+    update_small(u, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
+    if (u.stamps && threadIdx.x == 0) atomicMax(u.stamps + 7, clock_ns());
+}
+
+// Networks with a factoriser.  The first `rest` CTAs take the small tensors (the scattered stores of the dense layer's tables want the
+// time of the others), each of the others 32 float4s of every copy: a warp per copy, sixteen copies at a time, whose gradients meet in shared memory,
+// where a thread per float adds them up in order and updates the factoriser's own.  HBM, with what the backward has left in L2 to be
+// written back besides: 1536-row copies x 2048 columns x 16 (0.70 GB) 156 us, where a plain pass over clean arrays takes 111 (6.3 TB/s).
+// A thread per float4 of a copy that updated the sixteen copies one after the other took 159 there, and as long as 28 us however small the table:
+// 64 columns 28 -> 4.5, 256 32 -> 14.7, 512 39.5 -> 35.5, 1024 71.7 -> 67.4.  (A ring of bulk copies in one CTA per SM: 196; 64 or 128 float4s of a
+// copy per CTA: 160, 189; the gradients loaded to stay in L2: 160.)
+constexpr int kUpdThreads = 512, kUpdWarps = kUpdThreads / 32;
+__global__ void __launch_bounds__(kUpdThreads, 3) step_update_copies_kernel(const __grid_constant__ StepUpdateArgs u, int rest) {
+    __shared__ __align__(16) float grads[kUpdWarps][128];
+    update_begin(u);
+    if ((int)blockIdx.x < rest) {
+        update_small(u, blockIdx.x * (long long)kUpdThreads + threadIdx.x, (long long)rest * kUpdThreads);
+    } else {
+        const AdamArgs& a = u.adam;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+        const long long j0 = 32LL * (blockIdx.x - rest), j = j0 + lane, f = 4 * (u.l0f4 + j0) + threadIdx.x;
+        const bool own = threadIdx.x < 128 && j0 + threadIdx.x / 4 < u.block4;  // a float of the factoriser
+        float p = 0.f, m = 0.f, v = 0.f, sum = 0.f;
+        if (own) p = reinterpret_cast<float*>(a.p)[f], m = reinterpret_cast<float*>(a.m)[f], v = reinterpret_cast<float*>(a.v)[f];
+        for (int c0 = 0; c0 < u.copies; c0 += kUpdWarps) {
+            const int c = c0 + warp;
+            if (c < u.copies && j < u.block4) {
+                const long long i = u.l0w4 + c * u.block4 + j;
+                const float4 g = __ldcs(u.g + i);
+                Held h = load4(a, i);
+                reinterpret_cast<float4*>(grads[warp])[lane] = g;
+                update4(a, a.seg[u.l0w_seg], i, g, h);
+            }
+            __syncthreads();
+            if (threadIdx.x < 128) {
+                const int n = min(kUpdWarps, u.copies - c0);
+                if (n == kUpdWarps) {
+#pragma unroll
+                    for (int k = 0; k < kUpdWarps; k++) sum = c0 == 0 && k == 0 ? grads[0][threadIdx.x] : sum + grads[k][threadIdx.x];
+                } else
+                    for (int k = 0; k < n; k++) sum = c0 == 0 && k == 0 ? grads[0][threadIdx.x] : sum + grads[k][threadIdx.x];
+            }
+            if (c0 + kUpdWarps < u.copies) __syncthreads();
+        }
+        if (own) {
+            reinterpret_cast<float*>(u.g)[f] = sum;
+            adam_op(a.seg[u.l0f_seg], a.rate, a.adj * sum, p, m, v);
+            reinterpret_cast<float*>(a.p)[f] = p, reinterpret_cast<float*>(a.m)[f] = m, reinterpret_cast<float*>(a.v)[f] = v;
+        }
     }
     if (u.stamps && threadIdx.x == 0) atomicMax(u.stamps + 7, clock_ns());
 }

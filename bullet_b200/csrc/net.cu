@@ -966,7 +966,7 @@ int preload_kernels(b200_net* net) {
     ok = ok && load_kernel(b200::ft_csr_kernel);
     if (net->small_table()) ok = ok && load_kernel(b200::ft_onehot_kernel) && load_kernel(ft_backward_mma(net));
     ok = ok && load_kernel(b200::factoriser_merge_kernel) && load_kernel(b200::factoriser_grad_kernel);
-    ok = ok && load_kernel(b200::adamw_flat_kernel) && load_kernel(b200::step_update_kernel) && load_kernel(b200::lookahead_kernel);
+    ok = ok && load_kernel(b200::adamw_flat_kernel) && load_kernel(b200::step_update_kernel) && load_kernel(b200::step_update_copies_kernel) && load_kernel(b200::lookahead_kernel);
     ok = ok && load_kernel(b200::adamw_exchange_kernel<0>) && load_kernel(b200::adamw_exchange_kernel<2>);
     ok = ok && load_kernel(b200::adamw_exchange_kernel<4>) && load_kernel(b200::adamw_exchange_kernel<8>);
     ok = ok && load_kernel(b200::adamw_exchange_bulk_kernel<2, 256, 6>) && load_kernel(b200::adamw_exchange_bulk_kernel<2, 512, 3>);
@@ -2278,8 +2278,12 @@ static int step_chained(b200_net* net, Slot& s, int slot, float lr, float grad_f
         u.h_loss = net->h_loss + ring;
         u.h_status = net->h_status + ring;
         u.stamps = net->stamp(0);
-        const long long items = std::max(u.rest4, u.block4), blocks = std::min<long long>((items + 255) / 256, net->sm_count * 32);
-        CK(b200::launch_step(true, b200::step_update_kernel, (unsigned)blocks, 256, 0, net->stream, u));
+        if (l0f) {
+            const int rest = (int)((u.rest4 - u.block4 + b200::kUpdThreads - 1) / b200::kUpdThreads), tiles = (int)((u.block4 + 31) / 32);
+            CK(b200::launch_step(true, b200::step_update_copies_kernel, rest + tiles, b200::kUpdThreads, 0, net->stream, u, rest));
+        } else {
+            CK(b200::launch_step(true, b200::step_update_kernel, (unsigned)std::min<long long>((u.rest4 + 255) / 256, 1 << 20), 256, 0, net->stream, u));
+        }
         LAUNCHED(net);
         net->weights_moved();
         net->w1_dirty = lookahead;

@@ -729,3 +729,39 @@ def test_tiles_fetched_while_the_one_before_is_walked(oracle32, blocks, rows, ft
                 rc, x, _ = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], stm, nstm, n, x_at)
                 assert rc == 0 and np.array_equal(x, x_ref)
     net.close()
+
+
+@pytest.mark.parametrize("copies,rows,ft_out,dense,buckets", [
+    (1, 40, 64, (1,), 1), (2, 129, 64, (8, 1), 2), (15, 33, 128, (1,), 3), (16, 64, 64, (16, 32, 1), 2), (17, 31, 64, (1,), 1), (33, 24, 192, (4, 1), 2)])
+def test_update_of_networks_with_a_factoriser(copies, rows, ft_out, dense, buckets):
+    """A whole step's update: copies on either side of the sixteen that are taken at a time, copies that are no whole number of a CTA's
+    columns.  The factoriser's gradient is the sum of its copies' in order, to the last bit; the update is AdamW's from zero moments in
+    32 bits, of a few operations whose order and contraction the compiler chooses: four roundings of the weight and of the step."""
+    import dataclasses
+
+    from bullet_b200.configs import AdamWParams
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    n, lr = 700, 1e-3
+    desc = dataclasses.replace(net_of(copies, rows, ft_out, 12, buckets, dense), max_batch=n, factoriser_rows=rows)
+    w = rich_weights(desc)
+    net = make_net(desc, 0, w)
+    net.upload(0, *draw_batch(desc, n, seed=copies))
+    net.step(0, lr, 1.0 / n)
+    net.sync()
+    g, p = net.tensors(kind=3), net.tensors()
+    each = g["l0w"].reshape(copies, rows * ft_out)
+    total = each[0].copy()
+    for c in range(1, copies):
+        total += each[c]
+    assert np.array_equal(g["l0f"], total) and np.abs(total).max() > 0
+    hp = AdamWParams()
+    for k in w:
+        grad = g[k].astype(np.float64) / n
+        m, v = (1 - hp.beta1) * grad, (1 - hp.beta2) * grad * grad
+        step = lr * m / (np.sqrt(v) + 1e-8)
+        ref = np.clip(w[k].astype(np.float64).ravel() * (1 - hp.decay * lr) - step, hp.min_weight, hp.max_weight)
+        # (1 - beta is a difference of fp32 numbers: beta2's is off by up to 2^-25 / 1e-3 of itself, the root of it by half of that)
+        bound = 4 * 2.0**-24 * np.abs(ref) + (2.0**-16 + 8 * 2.0**-24) * np.abs(step) + 1e-12
+        assert (np.abs(p[k] - ref) <= bound).all(), k
+    net.close()
