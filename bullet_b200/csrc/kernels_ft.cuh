@@ -144,32 +144,46 @@ __device__ __forceinline__ void load_slots(const uint16_t* list, int nnz, int la
 }
 
 // ---------------------------------------------------------------- gather forward
-// grid = (ceil(2n / pairs_per_block), chunks); block = 256 threads (8 warps).
+// grid = (ceil(2n / pairs), column chunks); block = 256 threads (8 warps), a warp per pair and chunk.
 // Takes index sets without block structure, and the small batches of networks that have it: staging the table's tiles
 // costs the tiled kernel the whole table whatever the batch holds, here only the rows of the batch are read.
-// Bound by L2 for large batches and by load latency (one pair per warp, four rows in flight) for small ones.  With a
-// factoriser the two rows of a feature are added as they arrive, so a small batch does not merge the table first; an instantiation
-// without one keeps more warps on an SM (operator, 2048 positions x 1024 columns, whole call: 63 us with the factoriser's registers, 54
-// without; eight rows in flight and fewer warps: 64).
-// pairs per CTA: one per warp while there are few, up to eight once that leaves two waves of eight CTAs per SM
-inline int gather_pairs(int n, int unit, int sms) {
-    const long long pieces = (long long)2 * n * ((unit + 127) / 128) / (8LL * 16 * sms);
-    return 8 * (int)(pieces < 1 ? 1 : pieces < 8 ? pieces : 8);
+// Bound by load latency for few warps, then by the instructions around a row's loads: a warp takes up to 512 columns, and one row at a time
+// leaves the registers to more warps.  Operator, 2048 positions x 1024 columns (285 MB of rows from L2, whole call, us): 128 columns a warp
+// and four rows at a time 53, 256 and four 52, 256 and two 45, 256 and one 41, 512 and two 47, 512 and one 39 (rows copied ahead into a ring in
+// shared memory, 512 columns: 43); 1000 x 2048 pairwise, 256 columns: four rows 69, two 44, one 50; 8192 x 128: four 34, two 31; with a factoriser
+// (whole evaluation of 300 x 2048 pairwise): four rows 75, one 66.  Of few warps each needs the rows in flight: 300 x 1024 22 with four, 24 with one.
+// With a factoriser the two rows of a feature are added as they arrive, so a small batch does not merge the table first.
+struct GatherShape {
+    int pieces, rows;  // of 128 columns that a warp takes (with the pairwise product half of them of each half), rows at a time
+    int pairs;         // per CTA: one per warp while there are few, up to eight once that leaves two waves of eight CTAs per SM
+    dim3 grid;
+};
+inline GatherShape gather_shape(int n, int unit, bool pairwise, bool factor, int sms) {
+    const long long all = 2LL * n * ((unit + 127) / 128);
+    GatherShape g{};
+    if (all < (factor ? 16LL : 48LL) * sms) g.pieces = pairwise ? 2 : 1, g.rows = 4;
+    else if (pairwise) g.pieces = 2, g.rows = factor ? 1 : 2;
+    else if (unit > 128) g.pieces = unit >= 512 ? 4 : 2, g.rows = 1;
+    else g.pieces = 1, g.rows = factor ? 1 : 2;
+    const int wide = 128 * (pairwise ? g.pieces / 2 : g.pieces), chunks = (unit + wide - 1) / wide;
+    const long long per = 2LL * n * chunks / (8LL * 16 * sms);
+    g.pairs = 8 * (int)(per < 1 ? 1 : per < 8 ? per : 8);
+    g.grid = dim3((2 * n + g.pairs - 1) / g.pairs, chunks);
+    return g;
 }
-template <bool PAIRWISE, bool FACTOR>
+// C: pieces of 128 columns that a warp takes (with the pairwise product half of them of each half), U rows of them at a time.
+template <bool PAIRWISE, bool FACTOR, int C, int U>
 __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pairs_per_block) {
     ft_step_begin(a);
-    constexpr int U = 4;
+    constexpr int H2 = PAIRWISE ? 2 : 1;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int unit = PAIRWISE ? a.H / 2 : a.H;
-    const int col = blockIdx.y * 128 + lane * 4;
-    const bool active = col < unit;
+    const int col = blockIdx.y * (128 * C / H2) + lane * 4;
     const int pair_end = min(2 * a.n, (int)(blockIdx.x + 1) * pairs_per_block);
-    float4 bias_lo = make_float4(0, 0, 0, 0), bias_hi = bias_lo;
-    if (active) {
-        bias_lo = *reinterpret_cast<const float4*>(a.bias + col);
-        if (PAIRWISE) bias_hi = *reinterpret_cast<const float4*>(a.bias + unit + col);
-    }
+    auto at = [&](int c) { return 128 * (c / H2) + (c % H2 ? unit : 0); };  // piece c: of each half in turn; from this lane's column on
+    bool on[C];
+#pragma unroll
+    for (int c = 0; c < C; c++) on[c] = col + 128 * (c / H2) < unit;
     for (int pair = blockIdx.x * pairs_per_block + warp; pair < pair_end; pair += 8) {
         const int b = pair >> 1, p = pair & 1;
         const uint16_t* list = (p ? a.idx_nstm : a.idx_stm) + (size_t)b * a.nnz;
@@ -186,71 +200,66 @@ __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pa
             mask[1] &= __ballot_sync(0xffffffffu, slot[1] - base < (uint32_t)a.block_rows);
             if (a.status && lane == 0 && (mask[0] != all0 || mask[1] != all1)) *a.status = kStatusOutsideBlock;
         }
-        const uint32_t frow[2] = {FACTOR && a.factor ? slot[0] % a.factor_rows : 0u, FACTOR && a.factor ? slot[1] % a.factor_rows : 0u};
-        float4 lo = make_float4(0, 0, 0, 0), hi = lo;
+        const uint32_t frow[2] = {FACTOR ? slot[0] % a.factor_rows : 0u, FACTOR ? slot[1] % a.factor_rows : 0u};
+        float4 sum[C];
+#pragma unroll
+        for (int c = 0; c < C; c++) sum[c] = make_float4(0, 0, 0, 0);
 #pragma unroll
         for (int half = 0; half < 2; half++) {
             unsigned m = mask[half];
-            while (m) {  // up to U independent row loads in flight, added in slot order
-                int s[U];
+            while (m) {  // up to U rows' independent loads in flight, added in slot order
+                float4 v[U][C], w[U][C];
                 int cnt = 0;
 #pragma unroll
                 for (int k = 0; k < U; k++) {
-                    s[k] = m ? __ffs(m) - 1 : 0;
+                    const int s = m ? __ffs(m) - 1 : 0;
                     if (m) cnt++;
                     m &= m - 1;
-                }
-                float4 vlo[U], vhi[U], flo[U], fhi[U];
+                    const float* row = a.table + (size_t)__shfl_sync(0xffffffffu, slot[half], s) * a.H + col;
+                    const float* f = FACTOR ? a.factor + (size_t)__shfl_sync(0xffffffffu, frow[half], s) * a.H + col : nullptr;
 #pragma unroll
-                for (int k = 0; k < U; k++) {
-                    const uint32_t f = __shfl_sync(0xffffffffu, slot[half], s[k]);
-                    if (k < cnt && active) {
-                        const float* row = a.table + (size_t)f * a.H;
-                        vlo[k] = __ldg(reinterpret_cast<const float4*>(row + col));
-                        if (PAIRWISE) vhi[k] = __ldg(reinterpret_cast<const float4*>(row + unit + col));
-                    }
-                }
-                if (FACTOR && a.factor) {
-#pragma unroll
-                    for (int k = 0; k < U; k++) {
-                        const uint32_t f = __shfl_sync(0xffffffffu, frow[half], s[k]);
-                        if (k < cnt && active) {
-                            const float* row = a.factor + (size_t)f * a.H;
-                            flo[k] = __ldg(reinterpret_cast<const float4*>(row + col));
-                            if (PAIRWISE) fhi[k] = __ldg(reinterpret_cast<const float4*>(row + unit + col));
-                        }
-                    }
-#pragma unroll
-                    for (int k = 0; k < U; k++)
-                        if (k < cnt && active) {
-                            vlo[k] = add4(vlo[k], flo[k]);
-                            if (PAIRWISE) vhi[k] = add4(vhi[k], fhi[k]);
+                    for (int c = 0; c < C; c++)
+                        if (k < cnt && on[c]) {
+                            v[k][c] = __ldg(reinterpret_cast<const float4*>(row + at(c)));
+                            if (FACTOR) w[k][c] = __ldg(reinterpret_cast<const float4*>(f + at(c)));
                         }
                 }
 #pragma unroll
                 for (int k = 0; k < U; k++)
-                    if (k < cnt && active) {
-                        lo = add4(lo, vlo[k]);
-                        if (PAIRWISE) hi = add4(hi, vhi[k]);
-                    }
+#pragma unroll
+                    for (int c = 0; c < C; c++)
+                        if (k < cnt && on[c]) sum[c] = add4(sum[c], FACTOR ? add4(v[k][c], w[k][c]) : v[k][c]);
             }
         }
-        if (!active) continue;
-        lo = add4(lo, bias_lo);
-        if (PAIRWISE) {
-            hi = add4(hi, bias_hi);
-            const float4 ul = make_float4(crelu_f(lo.x), crelu_f(lo.y), crelu_f(lo.z), crelu_f(lo.w));
-            const float4 uh = make_float4(crelu_f(hi.x), crelu_f(hi.y), crelu_f(hi.z), crelu_f(hi.w));
-            float* up = a.u + (size_t)pair * a.H;
-            *reinterpret_cast<float4*>(up + col) = ul;
-            *reinterpret_cast<float4*>(up + unit + col) = uh;
-            *reinterpret_cast<float4*>(a.x + (size_t)b * a.H + (size_t)p * unit + col) =
-                make_float4(ul.x * uh.x, ul.y * uh.y, ul.z * uh.z, ul.w * uh.w);
-        } else {
-            *reinterpret_cast<float4*>(a.x + (size_t)b * 2 * a.H + (size_t)p * a.H + col) = make_float4(
-                ft_act_fwd(a.act, lo.x), ft_act_fwd(a.act, lo.y), ft_act_fwd(a.act, lo.z), ft_act_fwd(a.act, lo.w));
+#pragma unroll
+        for (int c = 0; c < C; c += H2) {
+            if (!on[c]) break;
+            const float* bias = a.bias + col;
+            const float4 lo = add4(sum[c], *reinterpret_cast<const float4*>(bias + at(c)));
+            if (PAIRWISE) {
+                const float4 hi = add4(sum[c + H2 - 1], *reinterpret_cast<const float4*>(bias + at(c + H2 - 1)));
+                const float4 ul = make_float4(crelu_f(lo.x), crelu_f(lo.y), crelu_f(lo.z), crelu_f(lo.w));
+                const float4 uh = make_float4(crelu_f(hi.x), crelu_f(hi.y), crelu_f(hi.z), crelu_f(hi.w));
+                float* up = a.u + (size_t)pair * a.H + col;
+                *reinterpret_cast<float4*>(up + at(c)) = ul;
+                *reinterpret_cast<float4*>(up + at(c + H2 - 1)) = uh;
+                *reinterpret_cast<float4*>(a.x + (size_t)pair * unit + col + at(c)) = make_float4(ul.x * uh.x, ul.y * uh.y, ul.z * uh.z, ul.w * uh.w);
+            } else {
+                *reinterpret_cast<float4*>(a.x + (size_t)pair * a.H + col + at(c)) = make_float4(
+                    ft_act_fwd(a.act, lo.x), ft_act_fwd(a.act, lo.y), ft_act_fwd(a.act, lo.z), ft_act_fwd(a.act, lo.w));
+            }
         }
     }
+}
+
+typedef void (*GatherKernel)(FtArgs, int);
+template <bool PAIRWISE, bool FACTOR>
+GatherKernel gather_form(const GatherShape& g) {
+    if (g.rows == 4) return ft_forward_gather_kernel<PAIRWISE, FACTOR, PAIRWISE ? 2 : 1, 4>;
+    if (PAIRWISE) return ft_forward_gather_kernel<true, FACTOR, 2, FACTOR ? 1 : 2>;
+    if (g.pieces == 4) return ft_forward_gather_kernel<false, FACTOR, 4, 1>;
+    if (g.pieces == 2) return ft_forward_gather_kernel<false, FACTOR, 2, 1>;
+    return ft_forward_gather_kernel<false, FACTOR, 1, FACTOR ? 1 : 2>;
 }
 
 // --------------------------------------------------------------- gather backward

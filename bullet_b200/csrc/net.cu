@@ -56,6 +56,7 @@ namespace {
 
 constexpr int64_t kAlignFloats = 64;       // 256-byte tensor alignment in the flat buffers
 constexpr int kGatherRowsPerPosition = 34;  // active features of both perspectives of a middling chess position
+constexpr long long kGatherMostBytes = 256 << 20;  // of all slots' rows
 constexpr int64_t kClearInForward = 2 << 20;  // floats of a gradient buffer that the forward kernel clears itself
 constexpr int kDirectOutputs = 256;        // up to as many outputs of an evaluation the kernel stores to pinned memory itself
 constexpr int kMinItemPairs = 128;         // a forward work item serves at least this many pairs per tile load
@@ -228,12 +229,19 @@ struct b200_net {
     // at 16384 positions, H = 2048: backward 0.50 ms against 0.61 ms for global vector reductions)
     bool fwd_tiled() const { return ft_fwd_mode == B200_FT_TILED || (ft_fwd_mode == B200_FT_AUTO && tiled_ok); }
     // ... for a whole batch of n positions.  The tiled forward stages every table row once whatever the batch holds, in few
-    // CTAs when there are few pairs; the gather forward reads the rows of the batch only (two per feature with a
-    // factoriser).  Measured (king buckets, 2048 wide, forward of n positions in us): n = 1 52 against 458, n = 512 86
-    // against 97, n = 1024 122 against 100: the lines cross where the gather reads about four times the table's rows.
+    // CTAs when there are few pairs; the gather forward reads the rows of the batch only, from L2 (two per feature with a
+    // factoriser).  Whole evaluation, and forward kernel of a training step, gather / tiled in us on a B200 (half of the slots active):
+    //   768 x 16 rows with a factoriser, 2048 columns pairwise: 300 79 / 129; 700 100 / 134; 1000 113 / 141, 56 / 78; 1500 132 / 145
+    //   1024 columns 700 71 / 104; 1500 93 / 108, 37 / 37; 128 columns 500 -, 10 / 33; 1500 69 / 81
+    //   768 rows x 128 columns 300 47 / 64, 7 / 12; 1500 53 / 69; 2000 -, 7 / 10.5; 6000 -, 14 / 12; x 1024 columns 300 49 / 66, 8 / 13; 1500 66 / 82;
+    //   2000 -, 20 / 22; 4000 97 / 105, 34 / 30; 147 rows x 256 columns 300 54 / 74, 7 / 11; 2000 -, 9 / 11; 6000 -, 18 / 20
+    // With a factoriser the line lies where the kernels meet at half as many columns, below where the table would be merged for the gather; else
+    // at half the bytes of where they meet with half of the slots active, as all of them may be.
     bool fwd_tiled(int n) const {
-        if (ft_fwd_mode == B200_FT_AUTO && tiled_ok && (long long)n * kGatherRowsPerPosition * (d.factoriser_rows ? 2 : 1) <= 4LL * d.n_inputs) return false;
-        return fwd_tiled();
+        const bool gather = d.factoriser_rows ? (long long)n * d.nnz < 4LL * d.n_inputs
+                                              : (long long)n * kGatherRowsPerPosition <= 4LL * d.n_inputs ||
+                                                    (n <= 2048 && 8LL * n * d.nnz * d.ft_out <= kGatherMostBytes);
+        return fwd_tiled() && !(ft_fwd_mode == B200_FT_AUTO && gather);
     }
     // The gather forward of n positions reads the merged table (one row per feature, after a pass over the whole table)
     // when the batch gathers several times the table's rows; below that it adds the factoriser row by row.
@@ -407,10 +415,8 @@ int launch_ft_forward(b200_net* net, const b200::FtArgs& a, const b200::TileArgs
     if (tiled) {
         CK(b200::launch_step(false, b200::ft_fwd_ahead(a, t, grid) ? b200::ft_forward_tiled_kernel<PW, true> : b200::ft_forward_tiled_kernel<PW, false>, grid, b200::kFwdThreads, b200::ft_fwd_smem(t.block_rows, t.list_len), net->stream, a, t));
     } else {
-        const int unit = PW ? a.H / 2 : a.H;
-        const int pairs = b200::gather_pairs(a.n, unit, net->sm_count);
-        dim3 grid((2 * a.n + pairs - 1) / pairs, (unit + 127) / 128);
-        (a.factor ? b200::ft_forward_gather_kernel<PW, true> : b200::ft_forward_gather_kernel<PW, false>)<<<grid, 256, 0, net->stream>>>(a, pairs);
+        const b200::GatherShape g = b200::gather_shape(a.n, PW ? a.H / 2 : a.H, PW, a.factor != nullptr, net->sm_count);
+        (a.factor ? b200::gather_form<PW, true>(g) : b200::gather_form<PW, false>(g))<<<g.grid, 256, 0, net->stream>>>(a, g.pairs);
     }
     LAUNCHED(net);
     return 0;
@@ -956,8 +962,11 @@ int preload_kernels(b200_net* net) {
     bool ok = true;
     DISPATCH_M(net->d.dense_out[0], ok = load_dense_kernels<MM>());
     ok = ok && load_kernel(b200::dense_regroup_kernel) && load_kernel(dense_one_form(net, false)) && (!net->small_table() || load_kernel(dense_one_form(net, true))) && load_kernel(b200::dense_one_dx_kernel) && load_kernel(b200::copy_outputs_kernel) && load_kernel(b200::dense_fragments_kernel) && load_kernel(b200::dense_small_grads_kernel);
-    ok = ok && load_kernel(b200::ft_forward_gather_kernel<true, true>) && load_kernel(b200::ft_forward_gather_kernel<true, false>) && load_kernel(b200::ft_forward_gather_kernel<false, true>) && load_kernel(b200::ft_forward_gather_kernel<false, false>);
     ok = ok && load_kernel(b200::ft_backward_gather_kernel<true, true>) && load_kernel(b200::ft_backward_gather_kernel<true, false>) && load_kernel(b200::ft_backward_gather_kernel<false, true>) && load_kernel(b200::ft_backward_gather_kernel<false, false>);
+    for (const b200::GatherShape& g : {b200::GatherShape{1, 4, 0, 0}, b200::GatherShape{1, 2, 0, 0}, b200::GatherShape{2, 1, 0, 0}, b200::GatherShape{4, 1, 0, 0}}) {
+        ok = ok && load_kernel(net->d.pairwise ? b200::gather_form<true, false>(g) : b200::gather_form<false, false>(g));
+        if (net->d.factoriser_rows) ok = ok && load_kernel(net->d.pairwise ? b200::gather_form<true, true>(g) : b200::gather_form<false, true>(g));
+    }
     ok = ok && load_kernel(b200::ft_forward_tiled_kernel<true, true>) && load_kernel(b200::ft_forward_tiled_kernel<true, false>) && load_kernel(b200::ft_forward_tiled_kernel<false, true>) && load_kernel(b200::ft_forward_tiled_kernel<false, false>);
     ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, true, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, true, false>);
     ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 512, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 512, true, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, true, false>);

@@ -132,17 +132,19 @@ int check_op(const b200_ft_op* op, const char* who) {
 }
 
 // Few positions are not worth grouping, nor the table's way through shared memory: the gather forward (one kernel, rows from L2)
-// takes them as they are.  Its time goes with the bytes of the rows, which the slots bound (about half of them are active).  Whole
-// call on a B200, gathered / grouped, us: 64 positions 20 to 24 / 36 to 230; king buckets x 1024 columns 1024 positions 38 / 58, 2048
-// (537 MB) 54 / 60, 4096 84 / 72; x 128 columns 8192 35 / 45, 16384 (537 MB) 50.5 / 52, pairwise x 2048 columns 1024 (537 MB) 71 / 81, 2048 106 / 89;
-// 768 rows x 128 columns 16384 (537 MB) 48 / 50, x 2048 columns 2048 77 / 60; 147 rows x 256 columns 8192 (822 MB) 54 / 69 (given up: one
-// line for all tables), x 2048 columns 512 40 / 59, 2048 (1644 MB) 89 / 82.  Lists that are full instead of half full lose near the line where one
-// large block is all there is: 768 rows x 128 columns 16384 55 / 49, x 2048 columns 1024 57 / 51; 16 blocks x 1024 columns 2048 60 / 59.  Outputs that
-// start on any float are for the tiled kernel.
-constexpr long long kGatherMost = 576LL << 20;
+// takes them as they are.  Its time goes with the bytes of the rows, which the slots bound (about half of them are active), the tiled form's
+// with the tiles besides, of which a CTA has at least one.  Whole call on a B200, gathered / grouped, us, by MB of slots (half of them active; all):
+//   16 blocks of 768 rows x 1024 columns: 537 38 / 60; 750 46 / 63; 1250 58 / 75; 89 / 90; 1500 63 / 77; 100 / 97; 3000 111 / 117
+//   x 2048 columns 1500 71 / 92; x 256 750 45 / 56; pairwise x 2048 1250 69 / 93; 40 blocks x 2048 1500 84 / 133; 121 / 154
+//   one block of 768 rows x 1024 columns: 750 41 / 53; 52 / 60; 1250 50 / 59; 76 / 77; four x 512 1250 84 / 77 (full)
+//   147 rows x 1024 columns (16 tiles): 765 38 / 66; 1339 68 / 90 (full); x 256 (four tiles) 765 37 / 66; 44 / 70
+//   768 rows x 128 columns (two tiles): 500 41 / 48; 512 48.5 / 48.6 (full); 937 64 / 59
+// The line lies at 1024 MB, for few tiles, which most SMs then share, at 576.  Outputs that start on any float are for the tiled kernel.
+constexpr long long kGatherMost = 1024LL << 20, kGatherMostFewTiles = 576LL << 20;
 bool few_positions(const b200_ft_op* op) {
     if (((uintptr_t)op->bias | (uintptr_t)op->x | (op->pairwise ? (uintptr_t)op->u : 0)) & 15) return false;
-    return 8LL * op->n * op->nnz * op->ft_out <= kGatherMost;
+    const long long tiles = (long long)(op->n_inputs / op->ft_block_rows) * (op->ft_out / b200::kTileCols);
+    return 8LL * op->n * op->nnz * op->ft_out <= (tiles >= 16 ? kGatherMost : kGatherMostFewTiles);
 }
 
 int finish_op(cudaStream_t stream, const b200_ft_op* op, StatusWord& word, const int* status) {
@@ -180,10 +182,8 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
         a.block_rows = R;
         a.status = status;
         if (!word.status) CK(cudaMemsetAsync(status, 0, sizeof *status, stream));
-        const int unit = op->pairwise ? a.H / 2 : a.H, pairs = b200::gather_pairs(n, unit, sms);
-        const dim3 grid((2 * n + pairs - 1) / pairs, (unit + 127) / 128);
-        if (op->pairwise) b200::ft_forward_gather_kernel<true, false><<<grid, 256, 0, stream>>>(a, pairs);
-        else b200::ft_forward_gather_kernel<false, false><<<grid, 256, 0, stream>>>(a, pairs);
+        const b200::GatherShape g = b200::gather_shape(n, op->pairwise ? a.H / 2 : a.H, op->pairwise, false, sms);
+        (op->pairwise ? b200::gather_form<true, false>(g) : b200::gather_form<false, false>(g))<<<g.grid, 256, 0, stream>>>(a, g.pairs);
         CK(cudaGetLastError());
         return finish_op(stream, op, word, status);
     }
