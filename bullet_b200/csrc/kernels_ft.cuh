@@ -184,6 +184,14 @@ __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pa
     bool on[C];
 #pragma unroll
     for (int c = 0; c < C; c++) on[c] = col + 128 * (c / H2) < unit;
+    // few warps: nothing else covers the bias's latency at the end
+    constexpr bool EARLY = U == 4;
+    auto bias_at = [&](int c) { return *reinterpret_cast<const float4*>(a.bias + col + at(c)); };
+    float4 bias[EARLY ? C : 1];
+    if (EARLY)
+#pragma unroll
+        for (int c = 0; c < C; c++)
+            if (on[c]) bias[c] = bias_at(c);
     for (int pair = blockIdx.x * pairs_per_block + warp; pair < pair_end; pair += 8) {
         const int b = pair >> 1, p = pair & 1;
         const uint16_t* list = (p ? a.idx_nstm : a.idx_stm) + (size_t)b * a.nnz;
@@ -209,21 +217,31 @@ __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pa
             unsigned m = mask[half];
             while (m) {  // up to U rows' independent loads in flight, added in slot order
                 float4 v[U][C], w[U][C];
+                uint32_t f[U], ff[U];
                 int cnt = 0;
 #pragma unroll
                 for (int k = 0; k < U; k++) {
                     const int s = m ? __ffs(m) - 1 : 0;
                     if (m) cnt++;
                     m &= m - 1;
-                    const float* row = a.table + (size_t)__shfl_sync(0xffffffffu, slot[half], s) * a.H + col;
-                    const float* f = FACTOR ? a.factor + (size_t)__shfl_sync(0xffffffffu, frow[half], s) * a.H + col : nullptr;
+                    f[k] = __shfl_sync(0xffffffffu, slot[half], s);
+                    if (FACTOR) ff[k] = __shfl_sync(0xffffffffu, frow[half], s);
+                }
+#pragma unroll
+                for (int k = 0; k < U; k++) {
+                    const float* row = a.table + (size_t)f[k] * a.H + col;
 #pragma unroll
                     for (int c = 0; c < C; c++)
-                        if (k < cnt && on[c]) {
-                            v[k][c] = __ldg(reinterpret_cast<const float4*>(row + at(c)));
-                            if (FACTOR) w[k][c] = __ldg(reinterpret_cast<const float4*>(f + at(c)));
-                        }
+                        if (k < cnt && on[c]) v[k][c] = __ldg(reinterpret_cast<const float4*>(row + at(c)));
                 }
+                if (FACTOR)
+#pragma unroll
+                    for (int k = 0; k < U; k++) {
+                        const float* row = a.factor + (size_t)ff[k] * a.H + col;
+#pragma unroll
+                        for (int c = 0; c < C; c++)
+                            if (k < cnt && on[c]) w[k][c] = __ldg(reinterpret_cast<const float4*>(row + at(c)));
+                    }
 #pragma unroll
                 for (int k = 0; k < U; k++)
 #pragma unroll
@@ -234,10 +252,9 @@ __global__ void __launch_bounds__(256) ft_forward_gather_kernel(FtArgs a, int pa
 #pragma unroll
         for (int c = 0; c < C; c += H2) {
             if (!on[c]) break;
-            const float* bias = a.bias + col;
-            const float4 lo = add4(sum[c], *reinterpret_cast<const float4*>(bias + at(c)));
+            const float4 lo = add4(sum[c], EARLY ? bias[EARLY ? c : 0] : bias_at(c));
             if (PAIRWISE) {
-                const float4 hi = add4(sum[c + H2 - 1], *reinterpret_cast<const float4*>(bias + at(c + H2 - 1)));
+                const float4 hi = add4(sum[c + H2 - 1], EARLY ? bias[EARLY ? c + H2 - 1 : 0] : bias_at(c + H2 - 1));
                 const float4 ul = make_float4(crelu_f(lo.x), crelu_f(lo.y), crelu_f(lo.z), crelu_f(lo.w));
                 const float4 uh = make_float4(crelu_f(hi.x), crelu_f(hi.y), crelu_f(hi.z), crelu_f(hi.w));
                 float* up = a.u + (size_t)pair * a.H + col;

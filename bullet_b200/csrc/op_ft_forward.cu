@@ -139,12 +139,12 @@ int check_op(const b200_ft_op* op, const char* who) {
 //   one block of 768 rows x 1024 columns: 750 41 / 53; 52 / 60; 1250 50 / 59; 76 / 77; four x 512 1250 84 / 77 (full)
 //   147 rows x 1024 columns (16 tiles): 765 38 / 66; 1339 68 / 90 (full); x 256 (four tiles) 765 37 / 66; 44 / 70
 //   768 rows x 128 columns (two tiles): 500 41 / 48; 512 48.5 / 48.6 (full); 937 64 / 59
-// The line lies at 1024 MB, for few tiles, which most SMs then share, at 576.  Outputs that start on any float are for the tiled kernel.
-constexpr long long kGatherMost = 1024LL << 20, kGatherMostFewTiles = 576LL << 20;
+// The line lies at 1536 MB for tables of a tile for every SM, for fewer tiles at 1024, for very few, which most SMs then share, at 576.  Outputs that start on any float are for the tiled kernel.
+constexpr long long kGatherMost = 1536LL << 20, kGatherMostFewTiles = 1024LL << 20, kGatherMostFewestTiles = 576LL << 20;
 bool few_positions(const b200_ft_op* op) {
     if (((uintptr_t)op->bias | (uintptr_t)op->x | (op->pairwise ? (uintptr_t)op->u : 0)) & 15) return false;
     const long long tiles = (long long)(op->n_inputs / op->ft_block_rows) * (op->ft_out / b200::kTileCols);
-    return 8LL * op->n * op->nnz * op->ft_out <= (tiles >= 16 ? kGatherMost : kGatherMostFewTiles);
+    return 8LL * op->n * op->nnz * op->ft_out <= (tiles >= 128 ? kGatherMost : tiles >= 16 ? kGatherMostFewTiles : kGatherMostFewestTiles);
 }
 
 int finish_op(cudaStream_t stream, const b200_ft_op* op, StatusWord& word, const int* status) {
