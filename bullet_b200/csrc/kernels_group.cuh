@@ -61,6 +61,7 @@ inline bool group_scans(int n) { return group_ctas(n) > 1024; }
 
 // hist[c][bin] -> sum of the rows before c, and the total in one more row.  grid = bins, block = 1024.
 static __global__ void __launch_bounds__(1024) group_scan_kernel(int* hist, int ctas, int nbins) {
+    step_begin(nullptr);
     __shared__ int warp_tot[32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int* column = hist + blockIdx.x;
@@ -101,6 +102,7 @@ __device__ __forceinline__ int valid_slots(uint4 w, int n_inputs) {
 // flight; either way one round of loads per thread for lists of up to 32 slots.  grid = group_ctas(n), block = kGroupThreads.
 constexpr int kGroupThreads = 1024;
 static __global__ void __launch_bounds__(kGroupThreads) group_lists_kernel(GroupArgs g, int vec) {
+    step_begin(nullptr);
     __shared__ int hist[kGroupMaxBlocks + kGroupMaxBuckets];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int nbins = g.nblocks + g.n_out_buckets;
@@ -256,6 +258,7 @@ constexpr int kCountedBlocks = 32;  // up to as many row blocks a window orders 
 // Latency bound (one CTA per SM at most for ordinary batches): one sweep over the histograms, a counting sort (a bitonic one
 // for many blocks: its 45 barriers took a third of the kernel's 13 us), one gather of the lists.
 static __global__ void __launch_bounds__(kPlaceThreads) group_place_kernel(GroupArgs g, int vec, int scanned) {
+    step_begin(nullptr);
     __shared__ int before[kGroupMaxBlocks + kGroupMaxBuckets], block_at[kGroupMaxBlocks + 1], bucket_at[kGroupMaxBuckets + 1];
     __shared__ int scan_s[kGroupMaxBlocks + 1], run_start[kGroupMaxBlocks];
     __shared__ unsigned key_s[kPlaceThreads];

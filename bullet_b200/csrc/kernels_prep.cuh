@@ -39,6 +39,7 @@ struct PrepArgs {
 // The records may lie in pinned host memory: they are read once, coalesced.  grid = group_ctas(n), block = kPrepThreads.
 constexpr int kPrepThreads = 512;
 static __global__ void __launch_bounds__(kPrepThreads) prep_featurise_kernel(PrepArgs p, GroupArgs g) {
+    step_begin(nullptr);
     __shared__ uint4 record_s[kGroupPositions][2];
     __shared__ int hist[kGroupMaxBlocks + kGroupMaxBuckets];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nnz = g.nnz;

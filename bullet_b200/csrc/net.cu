@@ -770,6 +770,8 @@ int group_slot(b200_net* net, Slot& s, const b200::GroupArgs& g, bool counted, c
         LAUNCHED(net);
     } else {
         const bool vec = b200::group_vec(g);
+        // beside a training step a kernel that waits for the one before would hold its SMs meanwhile
+        const bool chained = !net->trains;
         if (!counted) {
             b200::group_lists_kernel<<<b200::group_ctas(g.n), b200::kGroupThreads, 0, stream>>>(g, vec);
             LAUNCHED(net);
@@ -777,10 +779,10 @@ int group_slot(b200_net* net, Slot& s, const b200::GroupArgs& g, bool counted, c
         const bool scans = b200::group_scans(g.n);
         if (scans) {
             const int bins = g.nblocks + g.n_out_buckets;
-            b200::group_scan_kernel<<<bins, 1024, 0, stream>>>(g.hist, b200::group_ctas(g.n), bins);
+            CK(b200::launch_step(chained, b200::group_scan_kernel, bins, 1024, 0, stream, g.hist, b200::group_ctas(g.n), bins));
             LAUNCHED(net);
         }
-        b200::group_place_kernel<<<b200::group_windows(g.n), b200::kPlaceThreads, 0, stream>>>(g, vec, scans);
+        CK(b200::launch_step(chained, b200::group_place_kernel, b200::group_windows(g.n), b200::kPlaceThreads, 0, stream, g, (int)vec, (int)scans));
         LAUNCHED(net);
     }
     if (g.want_lists) s.prepared = true;

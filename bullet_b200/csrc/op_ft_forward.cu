@@ -220,8 +220,8 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
         const bool vec = b200::group_vec(g);
         b200::group_lists_kernel<<<b200::group_ctas(n), b200::kGroupThreads, 0, stream>>>(g, vec);
         const bool scans = b200::group_scans(n);
-        if (scans) b200::group_scan_kernel<<<nblocks + 1, 1024, 0, stream>>>(hist, b200::group_ctas(n), nblocks + 1);
-        b200::group_place_kernel<<<b200::group_windows(n), b200::kPlaceThreads, 0, stream>>>(g, vec, scans);
+        if (scans) CK(b200::launch_step(true, b200::group_scan_kernel, nblocks + 1, 1024, 0, stream, hist, b200::group_ctas(n), nblocks + 1));
+        CK(b200::launch_step(true, b200::group_place_kernel, b200::group_windows(n), b200::kPlaceThreads, 0, stream, g, (int)vec, (int)scans));
     }
     CK(cudaGetLastError());
 
@@ -249,8 +249,7 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
               : (op->pairwise ? (any ? b200::ft_forward_tiled_kernel<true, false, true> : b200::ft_forward_tiled_kernel<true, false, false>)
                               : (any ? b200::ft_forward_tiled_kernel<false, false, true> : b200::ft_forward_tiled_kernel<false, false, false>));
     CK(b200::allow_smem(kernel));
-    kernel<<<ctas, b200::kFwdThreads, smem, stream>>>(a, t);
-    CK(cudaGetLastError());
+    CK(b200::launch_step(true, kernel, ctas, b200::kFwdThreads, smem, stream, a, t));
     return finish_op(stream, op, word, status);
 }
 
