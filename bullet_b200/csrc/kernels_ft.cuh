@@ -11,15 +11,14 @@
 // pre-activations are bit-identical to the interpreter's fp32 result.
 //
 // Two families (the backward of tables of few rows has a third form, kernels_ft_mma.cuh):
-//   *_gather : one warp per (position, perspective, 128-column chunk); rows come
+//   *_gather : one warp per (position, perspective, chunk of columns); rows come
 //              straight from the table (L2/HBM), gradients go out as 128-bit
 //              global reductions.  Works for any index set.
 //   *_tiled  : for inputs whose active features of one perspective all lie in one
 //              aligned block of R table rows (king buckets).  A forward CTA stages one
 //              R x 64-column tile of the table in shared memory and serves every
-//              (position, perspective) of that block from it; a backward CTA keeps the
-//              matching tile of the table gradient in registers and feeds it from
-//              per-row position lists built in shared memory.
+//              (position, perspective) of that block from it; a backward CTA
+//              stages the gradients of a run of them and sums these row by row from lists.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -424,9 +423,10 @@ __device__ __forceinline__ f32x4 sum_lines(const unsigned char* lines, const uin
 
 // The same for lists of an even length, whose last entry may be a line of zeros: the backward's pieces are short (11 entries at 512 pairs
 // of a 768-row block), and up to three single lines at their ends cost more instructions than the added half line costs passes through
-// the pipe (c3 282 -> 270 us, c4 1974 -> 1900).  The forward's longer lists lose by it (c3 231 -> 240, 147 rows 70.6 -> 73.3).
+// the pipe (2048 columns pairwise, 16384 positions 282 -> 270 us, 131072 1974 -> 1900).  The forward's longer lists lose by it (231 -> 240 at 16384,
+// 147 rows 70.6 -> 73.3).
 // TWO: the loop unrolled by two groups of four, which helps the backward without the pairwise product (1024 columns 142 -> 137 us), whose
-// warps have the registers, and hurts it with the product (c3 267 -> 270, c4 1847 -> 1871; not unrolled at all 274, 1905).
+// warps have the registers, and hurts it with the product (the same sizes 267 -> 270, 1847 -> 1871; not unrolled at all 274, 1905).
 template <bool TWO>
 __device__ __forceinline__ f32x4 sum_lines_even(const unsigned char* lines, const uint2* list, int len, uint32_t lane16) {
     f32x4 acc = {0, 0};
@@ -472,7 +472,7 @@ __device__ __forceinline__ void store_piece(float* p, float4 v) {
 // shared-memory load and two packed adds per row, in slot order — the same order and arithmetic as the interpreter.
 // AHEAD: while a tile is walked the next one is fetched into tensor memory (64 columns of 32 lanes for each warp, which no other
 // warp touches), and copied from there when all warps have left the tile.  Fetched only then it kept the pipe idle for 26 k of 105 k clocks
-// per tile at 16384 positions (c3: 262 against 231 us).  Each warp fetches its share in one go, with the registers of the walk free, the warps
+// per tile at 16384 positions (2048 columns pairwise: 262 against 231 us).  Each warp fetches its share in one go, with the registers of the walk free, the warps
 // one after the other; a piece of it in every round instead, held in registers through the walk, cost the walk more than it saved at 131072.
 // Bound by the shared-memory pipe: 256 bytes per (row, pair, slab) at 128 bytes a clock.  (One pair per warp, 8 bytes per
 // lane, spent twice the instructions per row and was bound by their issue: 1.69 against 1.55 ms at 131072 positions and
@@ -695,7 +695,7 @@ constexpr int kPiece = 64;
 // entries per chunk: every slot of every pair plus up to three unused ones per row (lists start on 8 bytes), and 16 bytes
 // that a read-ahead may touch
 __host__ __device__ inline int ft_bwd_ent_cap(int R, int nnz, int cp) { return (cp * nnz + 4 * R + 8 + 7) & ~7; }
-// per chunk: entries, pieces, two unused words, then the pieces: first entry / 4 << 17 | length << 10 | row
+// per chunk: entries, pieces, two unused words, then the pieces: first entry / 4 << 17 | length, rounded up to even << 10 | row
 __host__ __device__ inline int ft_bwd_start_cap(int R, int nnz, int cp) { return (4 + R + cp * nnz / kPiece + 3) & ~3; }
 __host__ __device__ inline size_t ft_bwd_smem(int R, int nnz, int cp) {
     return (size_t)(cp + 1) * kTileRowBytes + (size_t)ft_bwd_ent_cap(R, nnz, cp) * 2 + (size_t)ft_bwd_start_cap(R, nnz, cp) * 4 + (size_t)cp * 12 +
@@ -764,7 +764,7 @@ static __global__ void __launch_bounds__(kCsrThreads) ft_csr_kernel(FtArgs a, Ti
     const int before = __reduce_add_sync(0xffffffffu, lane < warp ? warp_tot[lane] : 0), total = __reduce_add_sync(0xffffffffu, warp_tot[lane]);
     const int first = before + incl - room;
     if (r < R) start[r] = first;
-    if (mine & 1) ent[first + mine] = (uint16_t)t.chunk_len;
+    if (mine & 1) ent[first + mine] = (uint16_t)t.chunk_len;  // (there is room: lists are walked in pairs, the line past the chunk's is zero)
     if (warp == 0) {  // places of the pieces, longest first
         int run = 0;
         for (int base = kPiece; base > 0; base -= 32) {
@@ -1039,7 +1039,7 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
         };
         // The pieces are dealt to the half warps to and fro, longest first, so that each gets the same mixture of lengths: whole rounds, which all
         // lanes of a warp walk together, then the shortest.  (A counter for the last quarter balanced no better, and its second copy of
-        // the walk and the registers around it cost c4 1900 against 1844 us.)
+        // the walk and the registers around it cost 1900 against 1844 us at 131072 positions x 2048 columns.)
         constexpr int HW = 2 * NW;
         const int h = 2 * warp + half, dealt = pieces / HW;
         unsigned piece = dealt > 0 ? (unsigned)start[4 + h] : 0u;

@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(256, 3) step_update_kernel(const __grid_consta
 // Networks with a factoriser.  The first `rest` CTAs take the small tensors (the scattered stores of the dense layer's tables want the
 // time of the others), each of the others 32 float4s of every copy: a warp per copy, sixteen copies at a time, whose gradients meet in shared memory,
 // where a thread per float adds them up in order and updates the factoriser's own.  HBM, with what the backward has left in L2 to be
-// written back besides: 1536-row copies x 2048 columns x 16 (0.70 GB) 156 us, where a plain pass over clean arrays takes 111 (6.3 TB/s).
+// written back besides: 16 copies of 768 rows x 2048 columns (0.75 GB) 156 to 160 us, where a plain pass over clean arrays takes 111 (6.3 TB/s).
 // A thread per float4 of a copy that updated the sixteen copies one after the other took 159 there, and as long as 28 us however small the table:
 // 64 columns 28 -> 4.5, 256 32 -> 14.7, 512 39.5 -> 35.5, 1024 71.7 -> 67.4.  (A ring of bulk copies in one CTA per SM: 196; 64 or 128 float4s of a
 // copy per CTA: 160, 189; the gradients loaded to stay in L2: 160.)
