@@ -4,7 +4,7 @@
 // (ft_backward_tiled_kernel) adds 32 floats per clock and SM out of shared memory; the tensor pipe does 8192 multiply-adds of
 // bytes, zeros included.  With 27 of 147 rows active in every pair (ataxx) the dense product needs 44 times the walk's
 // operations in eight digits at 256 times its rate, and no row lists.  Time of the backward with 147 rows and 32768 positions,
-// walk / product: 256 columns 87 / 41 us, 1024 columns 336 / 134 (b200_net::bwd_mma draws the line between the two).
+// walk / product: 256 columns 83 / 41 us, 1024 columns 323 / 134 (b200_net::bwd_mma draws the line between the two).
 //
 // Numbers.  A gradient times a power of two, chosen so that the largest there can be (`gmax`) stays below 2^22, is a sum of eight
 // signed bytes down to units of 2^-37 (take_piece): eight rows of the product's first factor.  All 24 bits of a gradient down to

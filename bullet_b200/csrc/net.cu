@@ -266,11 +266,11 @@ struct b200_net {
     // lists hold, cut every block's pairs into steps of its own (one more on average is not full) and take out its sums; the walk's time goes
     // with the active rows, of which the host knows the slots: half of them, as of the games' lists.  The line is drawn 1.4 times to the
     // walk's side, which also leaves it small batches, where a step's latency counts.  Backward on a B200, walk / products in us (rows x blocks, active of slots):
-    //   147 x 1, 27 of 49: 32768 positions x 256 columns 87 / 41, 4096 x 1024 49 / 24, 512 x 64 12 / 9.4, 300 x 64 11.6 / 10 (walks), pairwise 16384 x 512 91 / 61
-    //   255 x 1, 17 of 32: 32768 x 256 64 / 48, 4096 x 1024 36 / 28, 3000 x 128 11.3 / 12.7 (walks), pairwise 16384 x 512 69 / 66 (walks)
-    //   255 x 1, 4 of 8: 32768 x 256 35 / 47 (walks);  64 x 1, 8 of 16: 32768 x 256 43 / 37, pairwise 16384 x 512 48 / 63 (walks)
-    //   200 x 8, 17 of 32: 16384 x 256 33 / 28, 1024 x 2048 24 / 34 (walks), pairwise 32768 x 1024 246 / 254 (walks)
-    //   147 x 64, 17 of 32: 16384 x 256 43 / 38 (given up), 1024 x 2048 52 / 131 (walks);  31 x 1000, 4 of 8: 1024 x 2048 293 / 762 (walks)
+    //   147 x 1, 27 of 49: 32768 positions x 256 columns 83 / 41, 4096 x 1024 46 / 24, 512 x 64 11.0 / 9.6, 300 x 64 10.5 / 9.7 (walks), pairwise 16384 x 512 88 / 62
+    //   255 x 1, 17 of 32: 32768 x 256 60 / 47, 4096 x 1024 34 / 28, 3000 x 128 9.7 / 12.5 (walks), pairwise 16384 x 512 66 / 75 (walks)
+    //   255 x 1, 4 of 8: 32768 x 256 31 / 47 (walks);  64 x 1, 8 of 16: 32768 x 256 39 / 36.5, pairwise 16384 x 512 45 / 58 (walks)
+    //   200 x 8, 17 of 32: 16384 x 256 32 / 28, 1024 x 2048 22 / 34 (walks), pairwise 32768 x 1024 235 / 252 (walks)
+    //   147 x 64, 17 of 32: 16384 x 256 39.5 / 38 (given up), 1024 x 2048 41 / 131 (walks);  31 x 1000, 4 of 8: 1024 x 2048 293 / 762 (walks; with the walk of before)
     // Lists that are emptier than half may get the slower form: 255 rows, 4 of 32 slots, 32768 x 256 loses 13 of 98 us.
     bool products_pay(int n) const {
         const long long steps = ((long long)2 * n + b200::kStepPairs - 1) / b200::kStepPairs, blocks = std::min<long long>(nblocks, 2LL * n);
