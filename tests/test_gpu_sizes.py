@@ -765,3 +765,57 @@ def test_update_of_networks_with_a_factoriser(copies, rows, ft_out, dense, bucke
         bound = 4 * 2.0**-24 * np.abs(ref) + (2.0**-16 + 8 * 2.0**-24) * np.abs(step) + 1e-12
         assert (np.abs(p[k] - ref) <= bound).all(), k
     net.close()
+
+
+@pytest.mark.parametrize("n,ft_out,nnz,pairwise", [
+    (901, 576, 12, False),     # 512 columns a warp, a second chunk that is not full
+    (1301, 320, 40, False),    # 256 columns a warp, lists of more than 32 slots
+    (3601, 64, 33, False),     # less than 128 columns
+    (1303, 768, 20, True),     # 128 columns of each half, two rows at a time
+    (20011, 128, 5, False),    # several pairs a warp, the last one's alone
+    (97, 576, 12, False),      # few warps: four rows at a time
+    (97, 768, 35, True),
+])
+def test_shapes_of_the_gather_forward(oracle32, n, ft_out, nnz, pairwise):
+    """The operator's gather forward in its shapes, bit-exact, and a feature outside its block reported."""
+    import dataclasses
+
+    from tests.test_gpu_ops import run_op
+    from tests.test_gpu_parity import rich_weights
+
+    desc = dataclasses.replace(net_of(3, 96, ft_out, nnz, 1, (1,), pairwise=pairwise), max_batch=n)
+    stm, nstm, _, _ = draw_batch(desc, n, seed=n)
+    w = rich_weights(desc)
+    x_ref = oracle_x(oracle32, desc, w, stm, nstm)
+    rc, x, _ = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], stm, nstm, n)
+    assert rc == 0 and np.array_equal(x, x_ref)
+    stm[n // 2, :2] = [3, 100]  # rows of two blocks
+    rc, _, _ = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], stm, nstm, n)
+    assert rc != 0
+
+
+@pytest.mark.parametrize("n,ft_out,pairwise,dense", [(203, 1024, False, (1,)), (701, 192, False, (8, 1)), (1301, 64, False, (1,)), (703, 512, True, (16, 32, 1)),
+                                                     (61, 512, True, (16, 32, 1)), (61, 192, False, (1,))])
+def test_shapes_of_the_gather_forward_with_a_factoriser(oracle32, n, ft_out, pairwise, dense):
+    """... with the factoriser's row added on the way: batches on either side of the line to four rows at a time, all of them below that to
+    the tiled forward.  Bit-exact; gradients with the bounds above (the backward walks lists)."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    desc = dataclasses.replace(net_of(64, 96, ft_out, 12, 2, dense, pairwise=pairwise), max_batch=n, factoriser_rows=96)
+    assert n * desc.nnz < 4 * desc.n_inputs
+    batch = draw_batch(desc, n, seed=n + ft_out)
+    w = rich_weights(desc)
+    x_ref = oracle_x(oracle32, desc, w, *batch[:2])
+    _, g_ref, out_ref = oracle32.net_grad(desc, w, *batch)
+    net = make_net(desc, 0, w)
+    net.upload(0, *batch)
+    out = net.forward(0, n)
+    assert np.array_equal(net.activation(0, n * desc.dense_in0).reshape(n, -1), x_ref)
+    assert np.abs(out - out_ref).max() <= 2e-5 * np.abs(out_ref).max()
+    net.step(0, 0.0, 1.0 / n)
+    g = net.tensors(kind=3)
+    for k in g_ref:
+        assert np.abs(g[k] - g_ref[k]).max() <= 2e-5 * np.abs(g_ref[k]).max(), k
+    net.close()
