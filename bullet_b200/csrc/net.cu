@@ -2293,7 +2293,7 @@ static int step_chained(b200_net* net, Slot& s, int slot, float lr, float grad_f
             const int rest = (int)((u.rest4 - u.block4 + b200::kUpdThreads - 1) / b200::kUpdThreads), tiles = (int)((u.block4 + 31) / 32);
             CK(b200::launch_step(true, b200::step_update_copies_kernel, rest + tiles, b200::kUpdThreads, 0, net->stream, u, rest));
         } else {
-            CK(b200::launch_step(true, b200::step_update_kernel, (unsigned)std::min<long long>((u.rest4 + 255) / 256, 1 << 20), 256, 0, net->stream, u));
+            CK(b200::launch_step(true, b200::step_update_kernel, (unsigned)std::min<long long>((u.rest4 + 255) / 256, net->sm_count * 32), 256, 0, net->stream, u));
         }
         LAUNCHED(net);
         net->weights_moved();
