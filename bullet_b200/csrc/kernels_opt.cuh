@@ -146,7 +146,7 @@ __device__ __forceinline__ void store_w1(const StepUpdateArgs& u, long long e, f
     }
 }
 
-// What both kernels do with the float4 at index `i`: load and update.
+// What both kernels below do with the float4 at index `i`: load and update.
 // (The moments are not needed before the next update: they leave L2 to the weights.)
 struct Held {
     float4 p, m, v;
@@ -161,17 +161,17 @@ __device__ __forceinline__ void update4(const AdamArgs& a, const AdamSegment& s,
     __stcs(a.m + i, h.m);
     __stcs(a.v + i, h.v);
 }
-// ... and with those of the tensors before l0w but for the factoriser, by the threads `me`, `me` + `stride`, ...
-__device__ __forceinline__ void update_small(const StepUpdateArgs& u, long long me, long long stride) {
+// ... and with those of the tensors before l0w but for the factoriser, by the threads `me`, `me` + `stride`, ...  `skipped`: the factoriser's
+// float4s, where its range is not to be dealt out among the threads; else (0) they step over it one by one, which costs many threads less.
+__device__ __forceinline__ void update_small(const StepUpdateArgs& u, long long me, long long stride, long long skipped) {
     const AdamArgs& a = u.adam;
-    const long long skipped = u.l0f_seg >= 0 ? u.block4 : 0;
     for (long long j = me; j < u.rest4 - skipped; j += stride) {
         const long long i = j >= u.l0f4 ? j + skipped : j;
         int si = -1;
 #pragma unroll 1
         for (int k = 0; k < a.nseg; k++)
             if (i >= a.seg[k].begin4 && i < a.seg[k].end4) si = k;
-        if (si < 0) continue;  // alignment padding between tensors
+        if (si < 0 || si == u.l0f_seg) continue;  // alignment padding between tensors
         const float4 g = u.g[i];
         Held h = load4(a, i);
         update4(a, a.seg[si], i, g, h);
@@ -186,36 +186,77 @@ __device__ __forceinline__ void update_begin(const StepUpdateArgs& u) {
     }
 }
 
-// Networks without a factoriser: all tensors.  HBM: 16 blocks of 768 rows x 2048 columns 147 us (4.8 TB/s with the gradient's dirty lines, which go out
+// A thread per float4, with a factoriser per float4 of it and of all its copies in turn (see update_by_thread).
+// HBM: 16 blocks of 768 rows x 2048 columns 147 us (4.8 TB/s with the gradient's dirty lines, which go out
 // besides), x 1024 73.  (A float4 a thread, however many CTAs that takes, and the gradient loaded behind the other three: 181 and 89.)
-__global__ void __launch_bounds__(256, 3) step_update_kernel(const __grid_constant__ StepUpdateArgs u) {
+constexpr int kUpdCtas = 3;  // resident on an SM
+__global__ void __launch_bounds__(256, kUpdCtas) step_update_kernel(const __grid_constant__ StepUpdateArgs u) {
     update_begin(u);
-    update_small(u, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)gridDim.x * blockDim.x);
+    const long long stride = (long long)gridDim.x * blockDim.x, me = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    if (u.l0f_seg >= 0) {
+        const AdamArgs& a = u.adam;
+        for (long long j = me; j < u.block4; j += stride) {
+            float4 sum = make_float4(0, 0, 0, 0);
+#pragma unroll 4
+            for (int c = 0; c < u.copies; c++) {
+                const long long i = u.l0w4 + c * u.block4 + j;
+                const float4 g = u.g[i];
+                if (c == 0) sum = g;
+                else sum.x += g.x, sum.y += g.y, sum.z += g.z, sum.w += g.w;
+                Held h = load4(a, i);
+                update4(a, a.seg[u.l0w_seg], i, g, h);
+            }
+            u.g[u.l0f4 + j] = sum;
+            Held h = load4(a, u.l0f4 + j);
+            update4(a, a.seg[u.l0f_seg], u.l0f4 + j, sum, h);
+        }
+    }
+    update_small(u, me, stride, 0);
     if (u.stamps && threadIdx.x == 0) atomicMax(u.stamps + 7, clock_ns());
 }
 
-// Networks with a factoriser.  The first `rest` CTAs take the small tensors (the scattered stores of the dense layer's tables want the
-// time of the others), each of the others 32 float4s of every copy: a warp per copy, sixteen copies at a time, whose gradients meet in shared memory,
+// A warp per copy.  The first `rest` CTAs take the small tensors (the scattered stores of the dense layer's tables want the
+// time of the others), each of the others `sets` times 32 float4s of every copy, as many copies at a time as sixteen warps take in equal rounds:
+// ten copies have CTAs of ten warps, four four sets in sixteen.  The gradients of a set meet in shared memory,
 // where a thread per float adds them up in order and updates the factoriser's own.  HBM, with what the backward has left in L2 to be
-// written back besides: 16 copies of 768 rows x 2048 columns (0.75 GB) 156 to 160 us, where a plain pass over clean arrays takes 111 (6.3 TB/s).
-// A thread per float4 of a copy that updated the sixteen copies one after the other took 159 there, and as long as 28 us however small the table:
-// 64 columns 28 -> 4.5, 256 32 -> 14.7, 512 39.5 -> 35.5, 1024 71.7 -> 67.4.  (A ring of bulk copies in one CTA per SM: 196; 64 or 128 float4s of a
-// copy per CTA: 160, 189; the gradients loaded to stay in L2: 160.)
+// written back besides: 16 copies of 768 rows x 2048 columns (0.75 GB) 154 to 159 us, where a plain pass over clean arrays of them takes 111.
+// (A ring of bulk copies in one CTA per SM: 196; 64 or 128 float4s of a copy per CTA: 160, 189; the gradients loaded to stay in L2: 160.)
 constexpr int kUpdThreads = 512, kUpdWarps = kUpdThreads / 32;
-__global__ void __launch_bounds__(kUpdThreads, 3) step_update_copies_kernel(const __grid_constant__ StepUpdateArgs u, int rest) {
+struct CopiesShape {
+    int copies, sets;  // copies at a time, sets of 32 float4s of each
+    int threads() const { return 32 * copies * sets; }
+};
+inline CopiesShape copies_shape(int copies) {
+    const int rounds = (copies + kUpdWarps - 1) / kUpdWarps, at_a_time = (copies + rounds - 1) / rounds;
+    return {at_a_time, kUpdWarps / at_a_time};
+}
+// Which of the two forms.  A thread that takes all copies needs the latency of every copy's loads in turn, which many threads hide and few do not:
+// it is as fast where its CTAs fill their waves.  Update on a B200, us, by thread / by warps, 768 rows:
+//   128 columns, 4 copies 5.3 / 4.4, 16 15.6 / 7.5; 320 (a wave not much more than half full) 4 6.3 / 6.2, 10 14.5 / 12, 16 27.7 / 20.7; 384 4 6.5 / 7.3, 10 15.5 / 13.4
+//   448 (a full wave from here) 4 6.8 / 7.7, 8 12.4 / 12.9, 12 20.5 / 18.8, 16 30 / 27.5; 512 4 7.0 / 9.1, 10 18.5 / 20, 16 32.7 / 34.2, 24 52 / 48.5
+//   768 (a second wave of few) 10 34.7 / 32.5, 16 58 / 51; 1024 4 16.6 / 18, 10 41 / 43, 16 71 / 69, 17 78 / 74; 2048 4 40 / 40, 10 95 / 94, 16 153 / 154, 24 230 / 222
+//   (a warp per copy in CTAs of sixteen whatever the copies: 1024 columns, 1 copy 28, where a thread takes 7; 4 34; 10 50; 17 92)
+// Few copies leave a set too few threads for the factoriser's floats.
+inline bool update_by_thread(int copies, long long block4, int sms) {
+    const long long ctas = (block4 + 255) / 256, wave = (long long)kUpdCtas * sms, waves = (ctas + wave - 1) / wave;
+    return copies < 4 || (copies < kUpdWarps && 4 * ctas >= 3 * waves * wave);
+}
+__global__ void __launch_bounds__(kUpdThreads, 3) step_update_copies_kernel(const __grid_constant__ StepUpdateArgs u, int rest, CopiesShape shape) {
     __shared__ __align__(16) float grads[kUpdWarps][128];
     update_begin(u);
     if ((int)blockIdx.x < rest) {
-        update_small(u, blockIdx.x * (long long)kUpdThreads + threadIdx.x, (long long)rest * kUpdThreads);
+        update_small(u, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)rest * blockDim.x, u.block4);
     } else {
         const AdamArgs& a = u.adam;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        const long long j0 = 32LL * (blockIdx.x - rest), j = j0 + lane, f = 4 * (u.l0f4 + j0) + threadIdx.x;
-        const bool own = threadIdx.x < 128 && j0 + threadIdx.x / 4 < u.block4;  // a float of the factoriser
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, set = warp / shape.copies, k0 = warp - set * shape.copies;
+        const int t = 32 * k0 + lane;  // (a set has 128 threads and more)
+        const long long j0 = 32 * ((long long)(blockIdx.x - rest) * shape.sets + set), j = j0 + lane, f = 4 * (u.l0f4 + j0) + t;
+        const bool own = t < 128 && j0 + t / 4 < u.block4;  // a float of the factoriser
+        const float(*const mine)[128] = grads + set * shape.copies;
         float p = 0.f, m = 0.f, v = 0.f, sum = 0.f;
         if (own) p = reinterpret_cast<float*>(a.p)[f], m = reinterpret_cast<float*>(a.m)[f], v = reinterpret_cast<float*>(a.v)[f];
-        for (int c0 = 0; c0 < u.copies; c0 += kUpdWarps) {
-            const int c = c0 + warp;
+        for (int c0 = 0; c0 < u.copies; c0 += shape.copies) {
+            const int c = c0 + k0;
             if (c < u.copies && j < u.block4) {
                 const long long i = u.l0w4 + c * u.block4 + j;
                 const float4 g = __ldcs(u.g + i);
@@ -224,15 +265,13 @@ __global__ void __launch_bounds__(kUpdThreads, 3) step_update_copies_kernel(cons
                 update4(a, a.seg[u.l0w_seg], i, g, h);
             }
             __syncthreads();
-            if (threadIdx.x < 128) {
-                const int n = min(kUpdWarps, u.copies - c0);
-                if (n == kUpdWarps) {
+            if (t < 128) {
+                const int n = min(shape.copies, u.copies - c0);
 #pragma unroll
-                    for (int k = 0; k < kUpdWarps; k++) sum = c0 == 0 && k == 0 ? grads[0][threadIdx.x] : sum + grads[k][threadIdx.x];
-                } else
-                    for (int k = 0; k < n; k++) sum = c0 == 0 && k == 0 ? grads[0][threadIdx.x] : sum + grads[k][threadIdx.x];
+                for (int k = 0; k < kUpdWarps; k++)
+                    if (k < n) sum = c0 == 0 && k == 0 ? mine[0][t] : sum + mine[k][t];
             }
-            if (c0 + kUpdWarps < u.copies) __syncthreads();
+            if (c0 + shape.copies < u.copies) __syncthreads();
         }
         if (own) {
             reinterpret_cast<float*>(u.g)[f] = sum;

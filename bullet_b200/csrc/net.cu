@@ -279,6 +279,7 @@ struct b200_net {
     }
     unsigned* gmax = nullptr;    // see FtArgs
     bool products_last = false;  // the last backward was ft_backward_mma_kernel
+    bool update_copies = false;  // the last whole step's update took a warp per copy of the factoriser
 };
 
 namespace {
@@ -2289,11 +2290,15 @@ static int step_chained(b200_net* net, Slot& s, int slot, float lr, float grad_f
         u.h_loss = net->h_loss + ring;
         u.h_status = net->h_status + ring;
         u.stamps = net->stamp(0);
-        if (l0f) {
-            const int rest = (int)((u.rest4 - u.block4 + b200::kUpdThreads - 1) / b200::kUpdThreads), tiles = (int)((u.block4 + 31) / 32);
-            CK(b200::launch_step(true, b200::step_update_copies_kernel, rest + tiles, b200::kUpdThreads, 0, net->stream, u, rest));
+        net->update_copies = l0f && !b200::update_by_thread(u.copies, u.block4, net->sm_count);
+        if (net->update_copies) {
+            const b200::CopiesShape shape = b200::copies_shape(u.copies);
+            const int threads = shape.threads(), wide = 32 * shape.sets;
+            const int rest = (int)((u.rest4 - u.block4 + threads - 1) / threads), tiles = (int)((u.block4 + wide - 1) / wide);
+            CK(b200::launch_step(true, b200::step_update_copies_kernel, rest + tiles, threads, 0, net->stream, u, rest, shape));
         } else {
-            CK(b200::launch_step(true, b200::step_update_kernel, (unsigned)std::min<long long>((u.rest4 + 255) / 256, net->sm_count * 32), 256, 0, net->stream, u));
+            const long long items = std::max(u.rest4, u.block4);
+            CK(b200::launch_step(true, b200::step_update_kernel, (unsigned)std::min<long long>((items + 255) / 256, net->sm_count * 32), 256, 0, net->stream, u));
         }
         LAUNCHED(net);
         net->weights_moved();
@@ -2475,6 +2480,7 @@ int b200_net_get_stat(b200_net* net, const char* key, int64_t* value) {
     else if (!strcmp(key, "flat_floats")) *value = net->n_flat;
     else if (!strcmp(key, "ft_tiled")) *value = (net->fwd_tiled() ? 1 : 0) + (net->bwd_tiled() ? 2 : 0);
     else if (!strcmp(key, "ft_products")) *value = net->products_last ? 1 : 0;
+    else if (!strcmp(key, "update_copies")) *value = net->update_copies ? 1 : 0;
     else if (!strcmp(key, "slow_weights")) *value = net->S ? 1 : 0;
     else if (!strcmp(key, "optimiser_steps")) *value = net->opt_step;
     else return b200::fail(B200_ERR_ARG, "get_stat: unknown key '%s'", key);

@@ -731,11 +731,15 @@ def test_tiles_fetched_while_the_one_before_is_walked(oracle32, blocks, rows, ft
     net.close()
 
 
-@pytest.mark.parametrize("copies,rows,ft_out,dense,buckets", [
-    (1, 40, 64, (1,), 1), (2, 129, 64, (8, 1), 2), (15, 33, 128, (1,), 3), (16, 64, 64, (16, 32, 1), 2), (17, 31, 64, (1,), 1), (33, 24, 192, (4, 1), 2)])
-def test_update_of_networks_with_a_factoriser(copies, rows, ft_out, dense, buckets):
-    """A whole step's update: copies on either side of the sixteen that are taken at a time, copies that are no whole number of a CTA's
-    columns.  The factoriser's gradient is the sum of its copies' in order, to the last bit; the update is AdamW's from zero moments in
+@pytest.mark.parametrize("copies,rows,ft_out,dense,buckets,by_warps", [
+    (1, 40, 64, (1,), 1, 0), (2, 129, 64, (8, 1), 2, 0), (3, 31, 64, (1,), 1, 0),   # a thread takes all copies
+    (5, 700, 512, (1,), 2, 0),                                                     # ... of a wide table
+    (4, 31, 64, (8, 1), 1, 1), (5, 129, 64, (1,), 2, 1), (8, 33, 64, (1,), 1, 1),  # sets of warps: four, three and a warp less, two
+    (15, 33, 128, (1,), 3, 1), (16, 64, 64, (16, 32, 1), 2, 1), (16, 700, 512, (1,), 1, 1),
+    (17, 31, 64, (1,), 1, 1), (33, 24, 192, (4, 1), 2, 1), (40, 24, 64, (1,), 1, 1)])  # rounds: two of nine, three of eleven and fourteen
+def test_update_of_networks_with_a_factoriser(copies, rows, ft_out, dense, buckets, by_warps):
+    """A whole step's update in both its forms: copies on either side of the sixteen that are taken at a time, copies that are no whole number
+    of a CTA's columns.  The factoriser's gradient is the sum of its copies' in order, to the last bit; the update is AdamW's from zero moments in
     32 bits, of a few operations whose order and contraction the compiler chooses: four roundings of the weight and of the step."""
     import dataclasses
 
@@ -749,6 +753,7 @@ def test_update_of_networks_with_a_factoriser(copies, rows, ft_out, dense, bucke
     net.upload(0, *draw_batch(desc, n, seed=copies))
     net.step(0, lr, 1.0 / n)
     net.sync()
+    assert net.stat("update_copies") == by_warps
     g, p = net.tensors(kind=3), net.tensors()
     each = g["l0w"].reshape(copies, rows * ft_out)
     total = each[0].copy()
@@ -765,6 +770,28 @@ def test_update_of_networks_with_a_factoriser(copies, rows, ft_out, dense, bucke
         bound = 4 * 2.0**-24 * np.abs(ref) + (2.0**-16 + 8 * 2.0**-24) * np.abs(step) + 1e-12
         assert (np.abs(p[k] - ref) <= bound).all(), k
     net.close()
+
+
+def test_update_goes_with_the_parameters_not_with_the_copies():
+    """The update's time per parameter with few copies of the factoriser against sixteen, which keep every warp of a CTA busy.  Few copies take
+    0.85 of it (their tables fit into L2); CTAs of sixteen warps whatever the copies are took 3.4 and 1.6 of it with one copy and four."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    n, per_float = 1024, {}
+    for copies in (16, 1, 4):
+        desc = dataclasses.replace(net_of(copies, 768, 1024, 12, 1, (1,)), max_batch=n, factoriser_rows=768)
+        net = make_net(desc, 0, rich_weights(desc))
+        net.upload(0, *draw_batch(desc, n, seed=copies))
+        times = []
+        for _ in range(6):
+            for _ in range(10):
+                net.step(0, 1e-3, 1.0 / n)
+            times.append(net.timings()["optimiser"])
+        per_float[copies] = min(times) / (copies + 1)
+        net.close()
+    assert per_float[1] <= 1.4 * per_float[16] and per_float[4] <= 1.4 * per_float[16], per_float
 
 
 @pytest.mark.parametrize("n,ft_out,nnz,pairwise", [
