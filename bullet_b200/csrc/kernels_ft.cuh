@@ -157,12 +157,20 @@ struct GatherShape {
     int pairs;         // per CTA: one per warp while there are few, up to eight once that leaves two waves of eight CTAs per SM
     dim3 grid;
 };
+// Four rows at a time up to `few` warps per SM of that form.  Forward alone, us, 768 x 16 rows, four / one row at a time, half of the slots active,
+// at 24, 40, 48, 56, 64, 72, 96 warps:
+//   with a factoriser  x 512 columns 10 / 16, 14.2 / 16.8, 16.1 / 17.1; x 1024 16 / 24, 19.2 / 23.8, 20.4 / 24.5; x 64 7.5 / 11.8
+//   without  x 512 -, 8.7 / 14.5, 12.2 / 14.5, 12.4 / 14.3, 12.5 / 14.5, 12.7 / 14.6, 15.4 / 14.8; x 1024 -, 14.2 / 21.9, 16.1 / 21.7, 17.4 / 21.8, 17.4 / 21.8,
+//   17.8 / 21.5, 21.5 / 21.7; 147 rows, where the rows come sooner, x 256 54 warps 11.1 / 9.0, x 512 11.5 / 11.8, x 1024 12.4 / 13.4
+// 512 columns a warp where that halves the chunks of 256: a chunk's warps take a row's latency each, however few columns they have.  Two / four pieces,
+// 2048 positions, 768 rows: 320 columns 14.6 / 10.6, 448 15.6 / 11.5, 576 (three chunks or two) 17.6 / 18.2, 768 18.4 / 19.2, 896 23.2 / 20.1.
 inline GatherShape gather_shape(int n, int unit, bool pairwise, bool factor, int sms) {
     const long long all = 2LL * n * ((unit + 127) / 128);
+    const int few = pairwise ? factor ? 16 : 48 : factor ? 40 : unit >= 1024 ? 64 : 48;
     GatherShape g{};
-    if (all < (factor ? 16LL : 48LL) * sms) g.pieces = pairwise ? 2 : 1, g.rows = 4;
+    if (all < (long long)few * sms) g.pieces = pairwise ? 2 : 1, g.rows = 4;
     else if (pairwise) g.pieces = 2, g.rows = factor ? 1 : 2;
-    else if (unit > 128) g.pieces = unit >= 512 ? 4 : 2, g.rows = 1;
+    else if (unit > 128) g.pieces = (unit + 255) / 256 == 2 * ((unit + 511) / 512) ? 4 : 2, g.rows = 1;
     else g.pieces = 1, g.rows = factor ? 1 : 2;
     const int wide = 128 * (pairwise ? g.pieces / 2 : g.pieces), chunks = (unit + wide - 1) / wide;
     const long long per = 2LL * n * chunks / (8LL * 16 * sms);

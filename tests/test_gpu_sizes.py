@@ -421,6 +421,13 @@ def oracle_x(oracle32, desc, w, stm, nstm):
     return oracle_ft_output(oracle32, desc, w, stm, nstm)
 
 
+def oracle_u(oracle32, desc, w, stm, nstm):
+    """The pairwise halves before their product, of a network without a factoriser: [n][2][ft_out]."""
+    n, h = len(stm), desc.ft_out
+    sums = [oracle32.sparse_matmul(w["l0w"], idx, n, h, desc.n_inputs, h, 0, desc.nnz).reshape(n, h) + w["l0b"][None, :] for idx in (stm, nstm)]
+    return np.stack([oracle32.act_forward(ACT_CRELU, a.ravel()).reshape(n, h) for a in sums], axis=1)
+
+
 @pytest.mark.parametrize("dense,buckets", [((4, 1), 1), ((8, 1), 3), ((16, 32, 1), 2), ((32, 32, 1), 2)])
 def test_products_of_the_first_dense_layer_keep_32_bits(dense, buckets):
     """One position: the weight gradient is x times the gradient at the layer's output, one product an entry, and that gradient is
@@ -795,8 +802,12 @@ def test_update_goes_with_the_parameters_not_with_the_copies():
 
 
 @pytest.mark.parametrize("n,ft_out,nnz,pairwise", [
-    (901, 576, 12, False),     # 512 columns a warp, a second chunk that is not full
-    (1301, 320, 40, False),    # 256 columns a warp, lists of more than 32 slots
+    (901, 576, 12, False),     # 256 columns a warp, a third chunk that is not full
+    (901, 960, 12, False),     # 512 columns a warp, a second chunk that is not full
+    (1301, 320, 40, False),    # ... a chunk that is not full, lists of more than 32 slots
+    (1901, 192, 40, False),    # 256 columns a warp, a chunk that is not full
+    (590, 1024, 9, False),     # on either side of where wide tables go on to one row at a time
+    (593, 1024, 9, False),
     (3601, 64, 33, False),     # less than 128 columns
     (1303, 768, 20, True),     # 128 columns of each half, two rows at a time
     (20011, 128, 5, False),    # several pairs a warp, the last one's alone
@@ -814,15 +825,43 @@ def test_shapes_of_the_gather_forward(oracle32, n, ft_out, nnz, pairwise):
     stm, nstm, _, _ = draw_batch(desc, n, seed=n)
     w = rich_weights(desc)
     x_ref = oracle_x(oracle32, desc, w, stm, nstm)
-    rc, x, _ = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], stm, nstm, n)
+    rc, x, u = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], stm, nstm, n)
     assert rc == 0 and np.array_equal(x, x_ref)
+    if pairwise:
+        assert np.array_equal(u, oracle_u(oracle32, desc, w, stm, nstm))
     stm[n // 2, :2] = [3, 100]  # rows of two blocks
     rc, _, _ = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], stm, nstm, n)
     assert rc != 0
 
 
+@pytest.mark.parametrize("factoriser,more,less,most", [
+    (0, (2048, 320), (2048, 256), 1.3),       # 64 columns more: 1.1, and 1.6 as a chunk of their own
+    (768, (157, 1024), (129, 1024), 1.45),    # 17 warps per SM against 14: 1.1, and 1.8 with one row at a time
+])
+def test_gather_forward_has_no_cliffs(factoriser, more, less, most):
+    """Time of the forward of (positions, columns) `more` against that of `less`, by any index set: rules on sizes may not cost more than they give."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    took = []
+    for n, ft_out in (more, less):
+        desc = dataclasses.replace(net_of(16 if factoriser else 1, 768, ft_out, 32, 1, (1,)), max_batch=n, factoriser_rows=factoriser)
+        batch = draw_batch(desc, n, seed=3)
+        net = make_net(dataclasses.replace(desc, ft_block_rows=0), 0, rich_weights(desc))
+        net.upload(0, *batch)
+        times = []
+        for _ in range(6):
+            for _ in range(10):
+                net.step(0, 1e-3, 1.0 / n)
+            times.append(net.timings()["ft_forward"])
+        took.append(min(times))
+        net.close()
+    assert took[0] <= most * took[1], took
+
+
 @pytest.mark.parametrize("n,ft_out,pairwise,dense", [(203, 1024, False, (1,)), (701, 192, False, (8, 1)), (1301, 64, False, (1,)), (703, 512, True, (16, 32, 1)),
-                                                     (61, 512, True, (16, 32, 1)), (61, 192, False, (1,))])
+                                                     (61, 512, True, (16, 32, 1)), (61, 192, False, (1,)), (985, 320, False, (1,)), (369, 1024, False, (1,)), (371, 1024, False, (1,))])
 def test_shapes_of_the_gather_forward_with_a_factoriser(oracle32, n, ft_out, pairwise, dense):
     """... with the factoriser's row added on the way: batches on either side of the line to four rows at a time, all of them below that to
     the tiled forward.  Bit-exact; gradients with the bounds above (the backward walks lists)."""
