@@ -56,7 +56,8 @@ namespace {
 
 constexpr int64_t kAlignFloats = 64;       // 256-byte tensor alignment in the flat buffers
 constexpr int kGatherRowsPerPosition = 34;  // active features of both perspectives of a middling chess position
-constexpr long long kGatherMostBytes = 256 << 20;  // of all slots' rows
+constexpr long long kGatherMostBytes = 100 << 20, kGatherMostPerRow = 200 << 10;  // see b200_net::fwd_tiled
+constexpr long long kGatherMore = 8 << 20;
 constexpr int64_t kClearInForward = 2 << 20;  // floats of a gradient buffer that the forward kernel clears itself
 constexpr int kDirectOutputs = 256;        // up to as many outputs of an evaluation the kernel stores to pinned memory itself
 constexpr int kMinItemPairs = 128;         // a forward work item serves at least this many pairs per tile load
@@ -230,17 +231,22 @@ struct b200_net {
     bool fwd_tiled() const { return ft_fwd_mode == B200_FT_TILED || (ft_fwd_mode == B200_FT_AUTO && tiled_ok); }
     // ... for a whole batch of n positions.  The tiled forward stages every table row once whatever the batch holds, in few
     // CTAs when there are few pairs; the gather forward reads the rows of the batch only, from L2 (two per feature with a
-    // factoriser).  Whole evaluation, and forward kernel of a training step, gather / tiled in us on a B200 (half of the slots active):
-    //   768 x 16 rows with a factoriser, 2048 columns pairwise: 300 79 / 129; 700 100 / 134; 1000 113 / 141, 56 / 78; 1500 132 / 145
-    //   1024 columns 700 71 / 104; 1500 93 / 108, 37 / 37; 128 columns 500 -, 10 / 33; 1500 69 / 81
-    //   768 rows x 128 columns 300 47 / 64, 7 / 12; 1500 53 / 69; 2000 -, 7 / 10.5; 6000 -, 14 / 12; x 1024 columns 300 49 / 66, 8 / 13; 1500 66 / 82;
-    //   2000 -, 20 / 22; 4000 97 / 105, 34 / 30; 147 rows x 256 columns 300 54 / 74, 7 / 11; 2000 -, 9 / 11; 6000 -, 18 / 20
-    // With a factoriser the line lies where the kernels meet at half as many columns, below where the table would be merged for the gather; else
-    // at half the bytes of where they meet with half of the slots active, as all of them may be.
+    // factoriser).  Drawn for lists that are full, whose rows cost the gather twice as much and the tiled walk little more.
+    // Forward kernel of a training step on a B200, us, gather / tiled, half of the slots active; all:
+    //   with a factoriser, by rows of the batch over the table's: 768 x 16 rows, 2048 columns pairwise 2.1 57 / 79; 69 / 88, 2.9 62 / 76; 80 / 92, 3.4 66 / 78; 89 / 86
+    //   1024 columns 2.1 25 / 41; 29 / 45, 2.9 33 / 37; 44 / 47, 3.4 34 / 37; 46 / 40; 128 columns 3.9 12 / 19; 13 / 21; 768 x 32 x 1024 3.0 55 / 69; 75 / 81, 3.9 62 / 75; 94 / 86
+    //   768 x 10 x 1024 2.9 20 / 28; 26 / 30, 4.0 27 / 28; 40 / 32; 768 x 4 x 1024 4.0 16 / 18; 18 / 20, x 2048 pairwise 2.9 22 / 28; 25 / 30, 4.0 30 / 26; 37 / 29
+    //   96 x 64 rows x 1024 3.9 19 / 35; 26 / 35, x 256 7 / 19; 8 / 19: the wider the table the sooner, as the tiles take a time of their own besides: below three times the
+    //   rows by the more of a wide table, up to four times of a narrow one (the merged table begins at five)
+    //   without, by MB of slots: 768 rows x 1024 columns 160 11.0 / 12.6; 12.5 / 15.0, 256 12.5 / 15.6; 16.5 / 17.8, 320 18.8 / 16.7; 26 / 20; 768 x 512 256 12.0 / 14.0; 15.3 / 17.5
+    //   147 rows x 512 128 9.0 / 11.2; 11.4 / 13.2, 160 11 / 11.3; 13 / 12.2, 256 12.4 / 12.0; 14.7 / 14.6; x 2048 128 9.5 / 11.9; 11.5 / 13.6, 256 14.2 / 12.6; 16.3 / 14.7
+    //   31 x 4 rows x 512 96 8.1 / 8.0; 9.7 / 10.1, 128 9.0 / 8.8; 11.3 / 10.2, 192 9.9 / 9.7; 12.0 / 12.1: the more rows a tile has the later
     bool fwd_tiled(int n) const {
-        const bool gather = d.factoriser_rows ? (long long)n * d.nnz < 4LL * d.n_inputs
+        const long long rows = (long long)n * d.nnz;
+        const int columns = d.ft_out > 512 ? (d.ft_out + 255) & ~255 : d.ft_out;  // as gather_shape's warps take them
+        const bool gather = d.factoriser_rows ? rows < 4LL * d.n_inputs && (4 * rows - 11LL * d.n_inputs) * d.ft_out < kGatherMore
                                               : (long long)n * kGatherRowsPerPosition <= 4LL * d.n_inputs ||
-                                                    (n <= 2048 && 8LL * n * d.nnz * d.ft_out <= kGatherMostBytes);
+                                                    (n <= 2048 && 8 * rows * columns <= kGatherMostBytes + kGatherMostPerRow * block_rows);
         return fwd_tiled() && !(ft_fwd_mode == B200_FT_AUTO && gather);
     }
     // The gather forward of n positions reads the merged table (one row per feature, after a pass over the whole table)
@@ -278,6 +284,7 @@ struct b200_net {
         return 14 * (steps + (1 + b200::kUnitFixed) * blocks) * product < 10 * steps * walk;
     }
     unsigned* gmax = nullptr;    // see FtArgs
+    int fwd_last = 0;            // the last forward's kernel: 0 gather, 1 tiled, 2 tiled with the next tile fetched ahead
     bool products_last = false;  // the last backward was ft_backward_mma_kernel
     bool update_copies = false;  // the last whole step's update took a warp per copy of the factoriser
 };
@@ -413,8 +420,10 @@ void slot_layout(const b200_net* net, Slot& s, int n) {
 
 template <bool PW>
 int launch_ft_forward(b200_net* net, const b200::FtArgs& a, const b200::TileArgs& t, bool tiled, int grid) {
+    const bool ahead = tiled && b200::ft_fwd_ahead(a, t, grid);
+    net->fwd_last = tiled ? ahead ? 2 : 1 : 0;
     if (tiled) {
-        CK(b200::launch_step(false, b200::ft_fwd_ahead(a, t, grid) ? b200::ft_forward_tiled_kernel<PW, true> : b200::ft_forward_tiled_kernel<PW, false>, grid, b200::kFwdThreads, b200::ft_fwd_smem(t.block_rows, t.list_len), net->stream, a, t));
+        CK(b200::launch_step(false, ahead ? b200::ft_forward_tiled_kernel<PW, true> : b200::ft_forward_tiled_kernel<PW, false>, grid, b200::kFwdThreads, b200::ft_fwd_smem(t.block_rows, t.list_len), net->stream, a, t));
     } else {
         const b200::GatherShape g = b200::gather_shape(a.n, PW ? a.H / 2 : a.H, PW, a.factor != nullptr, net->sm_count);
         (a.factor ? b200::gather_form<PW, true>(g) : b200::gather_form<PW, false>(g))<<<g.grid, 256, 0, net->stream>>>(a, g.pairs);
@@ -2479,6 +2488,7 @@ int b200_net_get_stat(b200_net* net, const char* key, int64_t* value) {
     else if (!strcmp(key, "h2d_bytes")) *value = net->h2d_bytes;
     else if (!strcmp(key, "flat_floats")) *value = net->n_flat;
     else if (!strcmp(key, "ft_tiled")) *value = (net->fwd_tiled() ? 1 : 0) + (net->bwd_tiled() ? 2 : 0);
+    else if (!strcmp(key, "ft_forward")) *value = net->fwd_last;
     else if (!strcmp(key, "ft_products")) *value = net->products_last ? 1 : 0;
     else if (!strcmp(key, "update_copies")) *value = net->update_copies ? 1 : 0;
     else if (!strcmp(key, "slow_weights")) *value = net->S ? 1 : 0;

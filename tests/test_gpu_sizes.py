@@ -834,6 +834,35 @@ def test_shapes_of_the_gather_forward(oracle32, n, ft_out, nnz, pairwise):
     assert rc != 0
 
 
+@pytest.mark.parametrize("blocks,rows,ft_out,nnz,factoriser,n", [
+    (64, 96, 512, 12, 96, 1749),   # 2.75 times the table's rows and 2 M floats more
+    (16, 96, 64, 12, 96, 511),     # four times
+    (8, 100, 64, 50, 100, 63),
+    (1, 147, 512, 49, 0, 672),     # 100 MB of slots, and 200 KB for each of a block's rows
+    (1, 147, 640, 49, 0, 448),     # ... of columns rounded up to 256
+    (4, 31, 1024, 31, 0, 437),
+    (1, 768, 64, 20, 0, 2048),     # positions
+])
+def test_lines_between_the_gather_and_the_tiled_forward(oracle32, blocks, rows, ft_out, nnz, factoriser, n):
+    """The last batch that the gather forward takes, and one position more, by evaluations and steps.  Bit-exact."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    desc = dataclasses.replace(net_of(blocks, rows, ft_out, nnz, 1, (1,)), max_batch=n + 1, factoriser_rows=factoriser)
+    w = rich_weights(desc)
+    net = make_net(desc, 0, w)
+    batch = draw_batch(desc, n + 1, seed=n)
+    x_ref = oracle_x(oracle32, desc, w, *batch[:2])
+    for count in (n, n + 1):
+        net.upload(0, *[a[:count] for a in batch])
+        for run in (lambda: net.forward(0, count), lambda: net.step(0, 0.0, 1.0 / count)):
+            run()
+            assert (net.stat("ft_forward") > 0) == (count > n)
+            assert np.array_equal(net.activation(0, count * desc.dense_in0).reshape(count, -1), x_ref[:count])
+    net.close()
+
+
 @pytest.mark.parametrize("factoriser,more,less,most", [
     (0, (2048, 320), (2048, 256), 1.3),       # 64 columns more: 1.1, and 1.6 as a chunk of their own
     (768, (157, 1024), (129, 1024), 1.45),    # 17 warps per SM against 14: 1.1, and 1.8 with one row at a time
