@@ -132,19 +132,19 @@ int check_op(const b200_ft_op* op, const char* who) {
 }
 
 // Few positions are not worth grouping, nor the table's way through shared memory: the gather forward (one kernel, rows from L2)
-// takes them as they are.  Its time goes with the bytes of the rows, which the slots bound (about half of them are active), the tiled form's
-// with the tiles besides, of which a CTA has at least one.  Whole call on a B200, gathered / grouped, us, by MB of slots (half of them active; all):
-//   16 blocks of 768 rows x 1024 columns: 537 38 / 60; 750 46 / 63; 1250 58 / 75; 89 / 90; 1500 63 / 77; 100 / 97; 3000 111 / 117
-//   x 2048 columns 1500 71 / 92; x 256 750 45 / 56; pairwise x 2048 1250 69 / 93; 40 blocks x 2048 1500 84 / 133; 121 / 154
-//   one block of 768 rows x 1024 columns: 750 41 / 53; 52 / 60; 1250 50 / 59; 76 / 77; four x 512 1250 84 / 77 (full)
-//   147 rows x 1024 columns (16 tiles): 765 38 / 66; 1339 68 / 90 (full); x 256 (four tiles) 765 37 / 66; 44 / 70
-//   768 rows x 128 columns (two tiles): 500 41 / 48; 512 48.5 / 48.6 (full); 937 64 / 59
-// The line lies at 1536 MB for tables of a tile for every SM, for fewer tiles at 1024, for very few, which most SMs then share, at 576.  Outputs that start on any float are for the tiled kernel.
-constexpr long long kGatherMost = 1536LL << 20, kGatherMostFewTiles = 1024LL << 20, kGatherMostFewestTiles = 576LL << 20;
-bool few_positions(const b200_ft_op* op) {
+// takes them as they are.  Its time goes with the bytes of the rows, which the slots bound, the tiled form's
+// with the tiles besides, of which a CTA has at least one.  Whole call on a B200, us, gathered / grouped, by MB of slots (half of them active; all):
+//   512 tiles and more: 16 blocks of 768 rows x 2048 columns pairwise 1500 77 / 93; 107 / 111; 40 blocks x 2048 1500 91 / 133; 121 / 154; 96 rows x 64 blocks x 512 1500 71 / 115; 101 / 130
+//   a tile for every SM: 16 blocks of 768 rows x 1024 890 45 / 57; 66 / 67, 1150 54 / 64; 77 / 78, 1500 65 / 72; 99 / 93; pairwise 1500 73 / 80; 105 / 100
+//   16 tiles and more: eight blocks of 768 rows x 1024 700 40 / 46; 56 / 55, 1000 49 / 52; 71 / 65; four x 512 890 44 / 49; 63 / 61, 1000 48 / 51; 69 / 64
+//   147 rows x 1024 890 37 / 60; 49 / 70, 1000 42 / 64; 60 / 75
+//   fewer, which most SMs then share: 147 rows x 256 570 29 / 38; 36 / 50; 768 rows x 128 570 39 / 45; 49 / 54, 700 -, 46; -, 52
+// The lines lie where full lists meet.  Outputs that start on any float are for the tiled kernel.
+constexpr long long kGatherMostManyTiles = 1536LL << 20, kGatherMost = 1152LL << 20, kGatherMostFewTiles = 896LL << 20, kGatherMostFewestTiles = 576LL << 20;
+bool few_positions(const b200_ft_op* op, int sms) {
     if (((uintptr_t)op->bias | (uintptr_t)op->x | (op->pairwise ? (uintptr_t)op->u : 0)) & 15) return false;
     const long long tiles = (long long)(op->n_inputs / op->ft_block_rows) * (op->ft_out / b200::kTileCols);
-    return 8LL * op->n * op->nnz * op->ft_out <= (tiles >= 128 ? kGatherMost : tiles >= 16 ? kGatherMostFewTiles : kGatherMostFewestTiles);
+    return 8LL * op->n * op->nnz * op->ft_out <= (tiles >= 512 ? kGatherMostManyTiles : tiles >= sms ? kGatherMost : tiles >= 16 ? kGatherMostFewTiles : kGatherMostFewestTiles);
 }
 
 int finish_op(cudaStream_t stream, const b200_ft_op* op, StatusWord& word, const int* status) {
@@ -178,7 +178,7 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
     a.u = op->u;
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    if (few_positions(op)) {
+    if (few_positions(op, sms)) {
         a.block_rows = R;
         a.status = status;
         if (!word.status) CK(cudaMemsetAsync(status, 0, sizeof *status, stream));

@@ -140,3 +140,48 @@ def test_op_ft_forward_on_either_side_of_the_gather(oracle32, name, desc, game, 
         stm[n - 1, 1] = (stm[n - 1, 0] + desc.ft_block_rows) % desc.n_inputs
         rc, _, _ = run_op("b200_op_ft_forward", desc, table, w["l0b"], stm, nstm, n)
         assert rc == -4
+
+
+TRACE = """
+import ctypes, sys
+import torch
+from bullet_b200 import _lib
+lib = _lib.load()
+torch.zeros(1, device="cuda")
+for blocks, ft_out, nnz, n in eval(sys.argv[1]):
+    rows = 64
+    table, bias = torch.zeros((blocks * rows, ft_out), device="cuda"), torch.zeros(ft_out, device="cuda")
+    index = torch.zeros((2, n, nnz), device="cuda", dtype=torch.int16)
+    x = torch.zeros(n * 2 * ft_out, device="cuda")
+    op = _lib.CFtOp(blocks * rows, nnz, ft_out, 1, 0, rows, n, table.data_ptr(), bias.data_ptr(), index[0].data_ptr(), index[1].data_ptr(), x.data_ptr(), None)
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU, torch.profiler.ProfilerActivity.CUDA]) as trace:
+        rc = lib.b200_op_ft_forward(0, None, ctypes.byref(op))
+        torch.cuda.synchronize()
+    assert rc == 0
+    names = [e.name for e in trace.events()]
+    print(" ".join(sorted({k for k in ("ft_forward_gather", "ft_forward_tiled", "Malloc", "cudaFree") if any(k in name for name in names)})))
+"""
+
+
+def traced(calls):
+    """What each call of b200_op_ft_forward, (row blocks, columns, slots, positions), launches and asks of the allocator."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", TRACE, repr(calls)], cwd=root, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr
+    seen = [set(line.split()) for line in done.stdout.splitlines()]
+    if not any(seen):
+        pytest.skip("this machine lets no process trace its runtime calls")
+    return seen
+
+
+def test_lines_between_gathered_and_grouped_calls():
+    """The last call that is gathered and one position more, for tables of a few tiles, of one for a part of the SMs, of one for each, and of many."""
+    lines = [(1, 512, 64, 576 * 4), (1, 1024, 64, 896 * 2), (4, 2048, 64, 896), (5, 2048, 64, 1152), (16, 2048, 64, 1536)]
+    seen = traced([(b, h, nnz, n + more) for b, h, nnz, n in lines for more in (0, 1)])
+    for k in range(len(lines)):
+        assert "ft_forward_gather" in seen[2 * k] and "ft_forward_tiled" in seen[2 * k + 1], lines[k]
