@@ -158,11 +158,28 @@ int finish_op(cudaStream_t stream, const b200_ft_op* op, StatusWord& word, const
     return 0;
 }
 
-// Groups the pairs into `scratch` and runs the tiled forward, or the gather forward as it is; synchronises the stream and
-// reports a feature outside its block.  Allocates nothing.
+// Scratch out of the device's pool, for one call.
+struct PoolScratch {
+    ~PoolScratch() {
+        if (at) cudaFreeAsync(at, stream);
+    }
+    cudaStream_t stream;
+    int* at = nullptr;
+};
+
+// Groups the pairs into scratch and runs the tiled forward, or the gather forward as it is; synchronises the stream and
+// reports a feature outside its block.  `scratch` null: from the pool, if the call needs any; else nothing is allocated.
 int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) {
     const int n = op->n, R = op->ft_block_rows, nblocks = op->n_inputs / R;
+    int sms = 0;
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    const bool gathered = few_positions(op, sms);
+    PoolScratch own{stream};
     StatusWord word(device, stream);
+    if (!scratch && !(gathered && word.status)) {
+        if (int rc = b200::op_pool_alloc(device, stream, scratch_ints(n, op->nnz, nblocks) * sizeof(int), &own.at)) return rc;
+        scratch = own.at;
+    }
     int* status = word.status ? word.status : scratch + kStatusAt;
     b200::FtArgs a{};
     a.table = op->table;
@@ -176,9 +193,7 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
     a.act = op->ft_act;
     a.x = op->x;
     a.u = op->u;
-    int sms = 0;
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-    if (few_positions(op, sms)) {
+    if (gathered) {
         a.block_rows = R;
         a.status = status;
         if (!word.status) CK(cudaMemsetAsync(status, 0, sizeof *status, stream));
@@ -255,7 +270,8 @@ int run_op(int device, cudaStream_t stream, const b200_ft_op* op, int* scratch) 
 
 }  // namespace
 
-// One pool per device for the scratch of b200_op_ft_forward.  It keeps at most kPoolKeep bytes between calls, for as long as the
+// One pool per device for the scratch of b200_op_ft_forward (cudaMalloc and cudaFree synchronise the device and cost 0.6 ms and more a
+// call; the pool's stream-ordered ones do not).  It keeps at most kPoolKeep bytes between calls, for as long as the
 // process lives or until a network that finds no room for its own buffers has it give those back (op_pool_trim).  Stream-ordered, so calls on several streams and
 // threads never share memory that is in use.
 namespace b200 {
@@ -301,13 +317,7 @@ extern "C" {
 int b200_op_ft_forward(int device, void* stream, const b200_ft_op* op) {
     if (int rc = check_op(op, "op_ft_forward")) return rc;
     CK(cudaSetDevice(device));
-    // cudaMalloc and cudaFree synchronise the device and cost 0.6 ms and more a call; the pool's stream-ordered ones do not
-    int* scratch = nullptr;
-    cudaStream_t on = static_cast<cudaStream_t>(stream);
-    if (int rc = b200::op_pool_alloc(device, on, scratch_ints(op->n, op->nnz, op->n_inputs / op->ft_block_rows) * sizeof(int), &scratch)) return rc;
-    const int rc = run_op(device, on, op, scratch);
-    cudaFreeAsync(scratch, on);
-    return rc;
+    return run_op(device, static_cast<cudaStream_t>(stream), op, nullptr);
 }
 
 // Same result as b200_op_ft_forward without touching the allocator.  It is meant for code

@@ -185,3 +185,10 @@ def test_lines_between_gathered_and_grouped_calls():
     seen = traced([(b, h, nnz, n + more) for b, h, nnz, n in lines for more in (0, 1)])
     for k in range(len(lines)):
         assert "ft_forward_gather" in seen[2 * k] and "ft_forward_tiled" in seen[2 * k + 1], lines[k]
+
+
+def test_gathered_calls_take_no_scratch():
+    """A call that groups nothing asks nothing of the allocator, so it runs where there is no room left; one that groups has its scratch from the pool."""
+    gathered, grouped = traced([(4, 512, 20, 300), (1, 512, 64, 3000)])
+    assert gathered == {"ft_forward_gather"}
+    assert grouped == {"ft_forward_tiled", "Malloc", "cudaFree"}
