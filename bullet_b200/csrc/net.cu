@@ -970,21 +970,32 @@ bool load_dense_kernels() {
         return load_kernel(b200::dense_forward_kernel<MM>) && load_kernel(b200::dense_dx_kernel<MM>) && load_kernel(b200::dense_wgrad_kernel<MM>);
 }
 
+// The forms of the feature transformer's kernels that a network's kind takes, whatever its batches: each(kernel, has dynamic shared memory).
+template <bool PW, bool ONE, class Each>
+void each_ft_form_of(bool tiled, Each& each) {
+    each(b200::ft_backward_gather_kernel<PW, ONE>, false);
+    if (!tiled) return;
+    each(b200::ft_forward_tiled_kernel<PW, true>, true), each(b200::ft_forward_tiled_kernel<PW, false>, true);
+    each(b200::ft_backward_tiled_kernel<PW, 1024, true, ONE>, true), each(b200::ft_backward_tiled_kernel<PW, 1024, false, ONE>, true);
+    each(b200::ft_backward_tiled_kernel<PW, 512, true, ONE>, true), each(b200::ft_backward_tiled_kernel<PW, 512, false, ONE>, true);
+    each(b200::ft_csr_kernel, true);
+}
+template <class Each>
+void each_ft_form(const b200_net* net, Each each) {
+    const bool one = net->dense_one();
+    if (net->d.pairwise) one ? each_ft_form_of<true, true>(net->tiled_ok, each) : each_ft_form_of<true, false>(net->tiled_ok, each);
+    else one ? each_ft_form_of<false, true>(net->tiled_ok, each) : each_ft_form_of<false, false>(net->tiled_ok, each);
+}
+
 int preload_kernels(b200_net* net) {
     bool ok = true;
     DISPATCH_M(net->d.dense_out[0], ok = load_dense_kernels<MM>());
     ok = ok && load_kernel(b200::dense_regroup_kernel) && load_kernel(dense_one_form(net, false)) && (!net->small_table() || load_kernel(dense_one_form(net, true))) && load_kernel(b200::dense_one_dx_kernel) && load_kernel(b200::copy_outputs_kernel) && load_kernel(b200::dense_fragments_kernel) && load_kernel(b200::dense_small_grads_kernel);
-    ok = ok && load_kernel(b200::ft_backward_gather_kernel<true, true>) && load_kernel(b200::ft_backward_gather_kernel<true, false>) && load_kernel(b200::ft_backward_gather_kernel<false, true>) && load_kernel(b200::ft_backward_gather_kernel<false, false>);
     for (const b200::GatherShape& g : {b200::GatherShape{1, 4, 0, 0}, b200::GatherShape{1, 2, 0, 0}, b200::GatherShape{2, 1, 0, 0}, b200::GatherShape{4, 1, 0, 0}}) {
         ok = ok && load_kernel(net->d.pairwise ? b200::gather_form<true, false>(g) : b200::gather_form<false, false>(g));
         if (net->d.factoriser_rows) ok = ok && load_kernel(net->d.pairwise ? b200::gather_form<true, true>(g) : b200::gather_form<false, true>(g));
     }
-    ok = ok && load_kernel(b200::ft_forward_tiled_kernel<true, true>) && load_kernel(b200::ft_forward_tiled_kernel<true, false>) && load_kernel(b200::ft_forward_tiled_kernel<false, true>) && load_kernel(b200::ft_forward_tiled_kernel<false, false>);
-    ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, true, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, true, false>);
-    ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 512, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 512, true, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, true, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, true, false>);
-    ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 1024, false, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 1024, false, false>);
-    ok = ok && load_kernel(b200::ft_backward_tiled_kernel<true, 512, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<true, 512, false, false>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, false, true>) && load_kernel(b200::ft_backward_tiled_kernel<false, 512, false, false>);
-    ok = ok && load_kernel(b200::ft_csr_kernel);
+    each_ft_form(net, [&](auto* kernel, bool) { ok = ok && load_kernel(kernel); });
     if (net->small_table()) ok = ok && load_kernel(b200::ft_onehot_kernel) && load_kernel(ft_backward_mma(net));
     ok = ok && load_kernel(b200::factoriser_merge_kernel) && load_kernel(b200::factoriser_grad_kernel);
     ok = ok && load_kernel(b200::adamw_flat_kernel) && load_kernel(b200::step_update_kernel) && load_kernel(b200::step_update_copies_kernel) && load_kernel(b200::lookahead_kernel);
@@ -1201,27 +1212,10 @@ int b200_net_create(int device, void* stream, const b200_net_desc* desc, b200_ne
         if (b200::allow_smem(dense_one_form(net, false)) != cudaSuccess || (net->small_table() && b200::allow_smem(dense_one_form(net, true)) != cudaSuccess)) return bail(b200::fail(B200_ERR_CUDA, "net_create: shared memory of the dense kernel"));
     }
     if (net->tiled_ok) {
-        cudaError_t e = b200::allow_smem(b200::ft_forward_tiled_kernel<true, true>);
-        e = e ? e : b200::allow_smem(b200::ft_forward_tiled_kernel<true, false>);
-        e = e ? e : b200::allow_smem(b200::ft_forward_tiled_kernel<false, true>);
-        e = e ? e : b200::allow_smem(b200::ft_forward_tiled_kernel<false, false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 1024, true, true>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 1024, true, false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 1024, true, true>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 1024, true, false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 512, true, true>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 512, true, false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, true, true>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, true, false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 1024, false, true>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 1024, false, false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 1024, false, true>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 1024, false, false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 512, false, true>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<true, 512, false, false>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, false, true>);
-        e = e ? e : b200::allow_smem(b200::ft_backward_tiled_kernel<false, 512, false, false>);
-        e = e ? e : b200::allow_smem(b200::ft_csr_kernel);
+        cudaError_t e = cudaSuccess;
+        each_ft_form(net, [&](auto* kernel, bool dynamic) {
+            if (dynamic && e == cudaSuccess) e = b200::allow_smem(kernel);
+        });
         if (net->small_table()) e = e ? e : b200::allow_smem(ft_backward_mma(net));
         if (e != cudaSuccess) return bail(b200::fail(B200_ERR_CUDA, "net_create: shared memory of the tiled kernels: %s", cudaGetErrorString(e)));
     }
