@@ -66,7 +66,7 @@ __device__ __forceinline__ float act_fwd(int act, float v) { return act == 0 ? v
 __device__ __forceinline__ float act_bwd(int act, float y) { return act == 0 ? 1.f : ft_act_bwd(act, y); }
 
 // Network outputs into pinned host memory, coalesced (they are computed in the order of the output buckets).
-static __global__ void __launch_bounds__(256) copy_outputs_kernel(const float* __restrict__ out, float* __restrict__ host, int n) {
+static __global__ void __launch_bounds__(256) copy_outputs_kernel(const float* out, float* host, int n) {
     step_begin(nullptr);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) host[i] = out[i];
 }

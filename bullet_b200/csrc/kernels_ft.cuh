@@ -380,9 +380,15 @@ __device__ __forceinline__ float hi2(f32x2 v) { return __uint_as_float((unsigned
 
 // Loads of data that is read once per kernel and must not claim L1 lines: with 196-228 KB of the SM's 256 KB
 // configured as shared memory only 28-60 KB of L1 are left, less than these kernels keep in flight.
+// ld_fresh4: what the kernel before wrote, which may still be writing when this one begins (launch.cuh).
 __device__ __forceinline__ float4 ld_once4(const float4* p) {
     float4 v;
     asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_fresh4(const float4* p) {
+    float4 v;
+    asm volatile("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
     return v;
 }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
@@ -600,12 +606,12 @@ __global__ void __launch_bounds__(kFwdThreads, 1) ft_forward_tiled_kernel(FtArgs
         int2 next = make_int2(0, 0);  // this half's next pair and its length
         uint32_t w0 = 0, w1 = 0;      // this lane's words of the next two lists
         auto fetch = [&](int at) {
-            if (at + half < seg_end) next = __ldg(t.pairs + at + half);
+            if (at + half < seg_end) next = t.pairs[at + half];
             // (a single last pair: the second list of the two may lie past the end of the lists)
             const int have = at + 1 < seg_end ? words : words / 2;
             const uint32_t* src = lists_w + (size_t)at * (words / 2);
-            if (at < seg_end && lane < have) w0 = __ldg(src + lane);
-            if (at < seg_end && lane + 32 < have) w1 = __ldg(src + lane + 32);
+            if (at < seg_end && lane < have) w0 = src[lane];
+            if (at < seg_end && lane + 32 < have) w1 = src[lane + 32];
         };
         fetch(i);
         if (AHEAD && !filled && rest > 0 && warp == 0) tmem_alloc_all(ring);  // (the word is not needed, the lists come later)
@@ -919,7 +925,7 @@ __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_til
         y0[k] = ld_once4(reinterpret_cast<const float4*>(y));
         if (PAIRWISE) y1[k] = ld_once4(reinterpret_cast<const float4*>(y + a.H / 2));
         d[k] = ONE ? __ldg(reinterpret_cast<const float4*>(a.w1 + one_s[pl].y + col))
-                   : ld_once4(reinterpret_cast<const float4*>(a.dx + (size_t)pair * x_row + col));
+                   : ld_fresh4(reinterpret_cast<const float4*>(a.dx + (size_t)pair * x_row + col));
     };
     auto fetch = [&](int pl0, int cn, int sl) {
 #pragma unroll

@@ -423,10 +423,10 @@ __global__ void __launch_bounds__(kMmaThreads, 1) ft_backward_mma_kernel(FtArgs 
                 y0[e][p] = ld_once4(reinterpret_cast<const float4*>(y));
                 if (PAIRWISE) y1[e][p] = ld_once4(reinterpret_cast<const float4*>(y + width));
                 if (ONE) {
-                    dout[e][p] = __ldg(a.dout + (pair >> 1));
+                    dout[e][p] = __ldcg(a.dout + (pair >> 1));
                     w1_row[e][p] = 2 * __ldg(a.out_bucket + (pair >> 1)) + (pair & 1);
                 } else {
-                    dd[e][p] = ld_once4(reinterpret_cast<const float4*>(a.dx + (size_t)pair * width + col));
+                    dd[e][p] = ld_fresh4(reinterpret_cast<const float4*>(a.dx + (size_t)pair * width + col));
                 }
             }
         };

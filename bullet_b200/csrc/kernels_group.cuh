@@ -273,8 +273,8 @@ static __global__ void __launch_bounds__(kPlaceThreads) group_place_kernel(Group
     if (scanned) {
         const int ctas = group_ctas(g.n), mine = (int)blockIdx.x * (kWindowPositions / kGroupPositions);
         if (tid < nbins) {
-            before[tid] = __ldg(g.hist + (size_t)mine * nbins + tid);
-            *(tid < nb ? &block_at[tid] : &bucket_at[tid - nb]) = __ldg(g.hist + (size_t)ctas * nbins + tid);
+            before[tid] = __ldcg(g.hist + (size_t)mine * nbins + tid);
+            *(tid < nb ? &block_at[tid] : &bucket_at[tid - nb]) = __ldcg(g.hist + (size_t)ctas * nbins + tid);
         }
     } else {  // totals, and what lies before this window, of every bin
         int width = 1;
@@ -283,7 +283,7 @@ static __global__ void __launch_bounds__(kPlaceThreads) group_place_kernel(Group
         int total = 0, prior = 0;
         if (bin < nbins) {
             for (int c = tid / width; c < ctas; c += kPlaceThreads / width) {
-                const int v = __ldg(g.hist + (size_t)c * nbins + bin);
+                const int v = __ldcg(g.hist + (size_t)c * nbins + bin);
                 total += v;
                 if (c < mine) prior += v;
             }
@@ -371,7 +371,7 @@ static __global__ void __launch_bounds__(kPlaceThreads) group_place_kernel(Group
                     w[u] = make_uint4(~0u, ~0u, ~0u, ~0u);
                     if (j < live) {
                         const int pair = base + (int)(key_s[j] & 0x3ffu);
-                        w[u] = __ldg(reinterpret_cast<const uint4*>(((pair & 1) ? g.nstm : g.stm) + (size_t)(pair >> 1) * g.nnz) + (e & (q_of - 1)));
+                        w[u] = __ldcg(reinterpret_cast<const uint4*>(((pair & 1) ? g.nstm : g.stm) + (size_t)(pair >> 1) * g.nnz) + (e & (q_of - 1)));
                     }
                 }
 #pragma unroll

@@ -282,6 +282,31 @@ def test_grouping_of_long_batches(oracle32, n):
         assert rc == 0 and np.array_equal(x, x_ref)
 
 
+@pytest.mark.parametrize("n", [3000, 140000])
+def test_groupings_that_follow_each_other_in_the_same_memory(oracle32, n):
+    """Two batches of different lists in turn through one scratch and one slot, with and without the kernel that sums the counts up: every
+    kernel of a chain reads what the one before it wrote this time.  Bit-exact."""
+    import dataclasses
+
+    from tests.test_gpu_ops import run_op
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    desc = dataclasses.replace(net_of(5, 60, 64, 8, 3, (1,)), max_batch=n)
+    w = rich_weights(desc)
+    batches = [draw_batch(desc, n, seed=k) for k in (1, 2)]
+    refs = [oracle_x(oracle32, desc, w, *b[:2]) for b in batches]
+    for turn in range(6):
+        rc, x, _ = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], *batches[turn % 2][:2], n, 1)
+        assert rc == 0 and np.array_equal(x, refs[turn % 2])
+    net = make_net(desc, 2, w)  # (that never trains: its groupings are chained)
+    for turn in range(6):
+        net.upload(0, *batches[turn % 2])
+        net.forward(0, n)
+        assert net.stat("ft_forward") > 0
+        assert np.array_equal(net.activation(0, n * desc.dense_in0).reshape(n, -1), refs[turn % 2])
+    net.close()
+
+
 @pytest.mark.parametrize("case", ["blocks-32", "blocks-33", "blocks-256", "blocks-257", "rows-32-last-layer", "list-of-64", "width-8"])
 def test_groupings_that_the_kernels_made(case):
     """The positions by output bucket and the pairs by row block that lie on the device, for every way of grouping, before and
