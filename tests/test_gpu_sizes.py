@@ -763,15 +763,11 @@ def test_tiles_fetched_while_the_one_before_is_walked(oracle32, blocks, rows, ft
     net.close()
 
 
-@pytest.mark.parametrize("copies,rows,ft_out,dense,buckets,by_warps", [
-    (1, 40, 64, (1,), 1, 0), (2, 129, 64, (8, 1), 2, 0), (3, 31, 64, (1,), 1, 0),   # a thread takes all copies
-    (5, 700, 512, (1,), 2, 0),                                                     # ... of a wide table
-    (4, 31, 64, (8, 1), 1, 1), (5, 129, 64, (1,), 2, 1), (8, 33, 64, (1,), 1, 1),  # sets of warps: four, three and a warp less, two
-    (15, 33, 128, (1,), 3, 1), (16, 64, 64, (16, 32, 1), 2, 1), (16, 700, 512, (1,), 1, 1),
-    (17, 31, 64, (1,), 1, 1), (33, 24, 192, (4, 1), 2, 1), (40, 24, 64, (1,), 1, 1)])  # rounds: two of nine, three of eleven and fourteen
-def test_update_of_networks_with_a_factoriser(copies, rows, ft_out, dense, buckets, by_warps):
-    """A whole step's update in both its forms: copies on either side of the sixteen that are taken at a time, copies that are no whole number
-    of a CTA's columns.  The factoriser's gradient is the sum of its copies' in order, to the last bit; the update is AdamW's from zero moments in
+@pytest.mark.parametrize("copies,rows,ft_out,dense,buckets", [
+    (1, 40, 64, (1,), 1), (2, 129, 64, (8, 1), 2), (15, 33, 128, (1,), 3), (16, 64, 64, (16, 32, 1), 2), (17, 31, 64, (1,), 1), (33, 24, 192, (4, 1), 2)])
+def test_update_of_networks_with_a_factoriser(copies, rows, ft_out, dense, buckets):
+    """A whole step's update: copies on either side of the sixteen that are taken at a time, copies that are no whole number of a CTA's
+    columns.  The factoriser's gradient is the sum of its copies' in order, to the last bit; the update is AdamW's from zero moments in
     32 bits, of a few operations whose order and contraction the compiler chooses: four roundings of the weight and of the step."""
     import dataclasses
 
@@ -785,7 +781,6 @@ def test_update_of_networks_with_a_factoriser(copies, rows, ft_out, dense, bucke
     net.upload(0, *draw_batch(desc, n, seed=copies))
     net.step(0, lr, 1.0 / n)
     net.sync()
-    assert net.stat("update_copies") == by_warps
     g, p = net.tensors(kind=3), net.tensors()
     each = g["l0w"].reshape(copies, rows * ft_out)
     total = each[0].copy()
@@ -801,6 +796,29 @@ def test_update_of_networks_with_a_factoriser(copies, rows, ft_out, dense, bucke
         # (1 - beta is a difference of fp32 numbers: beta2's is off by up to 2^-25 / 1e-3 of itself, the root of it by half of that)
         bound = 4 * 2.0**-24 * np.abs(ref) + (2.0**-16 + 8 * 2.0**-24) * np.abs(step) + 1e-12
         assert (np.abs(p[k] - ref) <= bound).all(), k
+    net.close()
+
+
+@pytest.mark.parametrize("copies,rows,ft_out,dense,buckets,by_warps", [
+    (1, 40, 64, (1,), 1, 0), (2, 129, 64, (8, 1), 2, 0), (3, 31, 64, (1,), 1, 0),   # a thread takes all copies
+    (5, 700, 512, (1,), 2, 0),                                                     # ... of a wide table
+    (4, 31, 64, (8, 1), 1, 1), (5, 129, 64, (1,), 2, 1), (8, 33, 64, (1,), 1, 1),  # sets of warps: four, three and a warp less, two
+    (15, 33, 128, (1,), 3, 1), (16, 64, 64, (16, 32, 1), 2, 1), (16, 700, 512, (1,), 1, 1),
+    (17, 31, 64, (1,), 1, 1), (33, 24, 192, (4, 1), 2, 1), (40, 24, 64, (1,), 1, 1)])  # rounds: two of nine, three of eleven and fourteen
+def test_forms_of_the_update_with_a_factoriser(copies, rows, ft_out, dense, buckets, by_warps):
+    """The same for the edges of both its forms, and which of them a network takes."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    test_update_of_networks_with_a_factoriser(copies, rows, ft_out, dense, buckets)
+    n = 100
+    desc = dataclasses.replace(net_of(copies, rows, ft_out, 12, buckets, dense), max_batch=n, factoriser_rows=rows)
+    net = make_net(desc, 0, rich_weights(desc))
+    net.upload(0, *draw_batch(desc, n, seed=copies))
+    net.step(0, 1e-3, 1.0 / n)
+    net.sync()
+    assert net.stat("update_copies") == by_warps
     net.close()
 
 
@@ -828,11 +846,7 @@ def test_update_goes_with_the_parameters_not_with_the_copies():
 
 @pytest.mark.parametrize("n,ft_out,nnz,pairwise", [
     (901, 576, 12, False),     # 256 columns a warp, a third chunk that is not full
-    (901, 960, 12, False),     # 512 columns a warp, a second chunk that is not full
-    (1301, 320, 40, False),    # ... a chunk that is not full, lists of more than 32 slots
-    (1901, 192, 40, False),    # 256 columns a warp, a chunk that is not full
-    (590, 1024, 9, False),     # on either side of where wide tables go on to one row at a time
-    (593, 1024, 9, False),
+    (1301, 320, 40, False),    # 512 columns a warp, a chunk that is not full, lists of more than 32 slots
     (3601, 64, 33, False),     # less than 128 columns
     (1303, 768, 20, True),     # 128 columns of each half, two rows at a time
     (20011, 128, 5, False),    # several pairs a warp, the last one's alone
@@ -850,13 +864,43 @@ def test_shapes_of_the_gather_forward(oracle32, n, ft_out, nnz, pairwise):
     stm, nstm, _, _ = draw_batch(desc, n, seed=n)
     w = rich_weights(desc)
     x_ref = oracle_x(oracle32, desc, w, stm, nstm)
-    rc, x, u = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], stm, nstm, n)
+    rc, x, _ = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], stm, nstm, n)
     assert rc == 0 and np.array_equal(x, x_ref)
-    if pairwise:
-        assert np.array_equal(u, oracle_u(oracle32, desc, w, stm, nstm))
     stm[n // 2, :2] = [3, 100]  # rows of two blocks
     rc, _, _ = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], stm, nstm, n)
     assert rc != 0
+
+
+@pytest.mark.parametrize("n,ft_out,nnz", [
+    (901, 960, 12),     # 512 columns a warp, a second chunk that is not full
+    (1901, 192, 40),    # 256 columns a warp, a chunk that is not full
+    (590, 1024, 9),     # on either side of where wide tables go on to one row at a time
+    (593, 1024, 9),
+])
+def test_more_shapes_of_the_gather_forward(oracle32, n, ft_out, nnz):
+    test_shapes_of_the_gather_forward(oracle32, n, ft_out, nnz, False)
+
+
+@pytest.mark.parametrize("n,ft_out,nnz", [
+    (1303, 768, 20),    # 128 columns of each half, two rows at a time
+    (97, 768, 35),      # few warps: four rows at a time
+    (97, 320, 35),      # a second chunk that is not full
+    (2100, 320, 64),
+])
+def test_halves_before_the_pairwise_product(oracle32, n, ft_out, nnz):
+    """Both operator outputs of the pairwise form, gathered and (outputs on any float) grouped.  Bit-exact."""
+    import dataclasses
+
+    from tests.test_gpu_ops import run_op
+    from tests.test_gpu_parity import rich_weights
+
+    desc = dataclasses.replace(net_of(3, 96, ft_out, nnz, 1, (1,), pairwise=True), max_batch=n)
+    stm, nstm, _, _ = draw_batch(desc, n, seed=n)
+    w = rich_weights(desc)
+    x_ref, u_ref = oracle_x(oracle32, desc, w, stm, nstm), oracle_u(oracle32, desc, w, stm, nstm)
+    for x_at in (0, 1):
+        rc, x, u = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], stm, nstm, n, x_at)
+        assert rc == 0 and np.array_equal(x, x_ref) and np.array_equal(u, u_ref)
 
 
 @pytest.mark.parametrize("blocks,rows,ft_out,nnz,factoriser,n", [
@@ -915,7 +959,7 @@ def test_gather_forward_has_no_cliffs(factoriser, more, less, most):
 
 
 @pytest.mark.parametrize("n,ft_out,pairwise,dense", [(203, 1024, False, (1,)), (701, 192, False, (8, 1)), (1301, 64, False, (1,)), (703, 512, True, (16, 32, 1)),
-                                                     (61, 512, True, (16, 32, 1)), (61, 192, False, (1,)), (985, 320, False, (1,)), (369, 1024, False, (1,)), (371, 1024, False, (1,))])
+                                                     (61, 512, True, (16, 32, 1)), (61, 192, False, (1,))])
 def test_shapes_of_the_gather_forward_with_a_factoriser(oracle32, n, ft_out, pairwise, dense):
     """... with the factoriser's row added on the way: batches on either side of the line to four rows at a time, all of them below that to
     the tiled forward.  Bit-exact; gradients with the bounds above (the backward walks lists)."""
@@ -939,3 +983,8 @@ def test_shapes_of_the_gather_forward_with_a_factoriser(oracle32, n, ft_out, pai
     for k in g_ref:
         assert np.abs(g[k] - g_ref[k]).max() <= 2e-5 * np.abs(g_ref[k]).max(), k
     net.close()
+
+
+@pytest.mark.parametrize("n,ft_out", [(985, 320), (369, 1024), (371, 1024)])
+def test_more_shapes_of_the_gather_forward_with_a_factoriser(oracle32, n, ft_out):
+    test_shapes_of_the_gather_forward_with_a_factoriser(oracle32, n, ft_out, False, (1,))
