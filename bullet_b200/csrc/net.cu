@@ -286,6 +286,7 @@ struct b200_net {
     unsigned* gmax = nullptr;    // see FtArgs
     int fwd_last = 0;            // the last forward's kernel: 0 gather, 1 tiled, 2 tiled with the next tile fetched ahead
     bool products_last = false;  // the last backward was ft_backward_mma_kernel
+    int chunk_last = 0;          // pairs per chunk of the last backward, 0: the gather
     bool update_copies = false;  // the last whole step's update took a warp per copy of the factoriser
 };
 
@@ -457,6 +458,7 @@ void (*ft_backward_mma(const b200_net* net))(b200::FtArgs, b200::TileArgs) {
 template <bool PW>
 int launch_ft_backward(b200_net* net, const Slot& s, const b200::FtArgs& a, const b200::TileArgs& t, bool tiled, int grid) {
     net->products_last = tiled && s.mma;
+    net->chunk_last = tiled ? t.chunk_len : 0;
     if (tiled && s.mma) {
         b200::launch_step(net->chained, ft_backward_mma(net), grid, b200::kMmaThreads, b200::ft_mma_smem(b200::ft_mma_rows(t.block_rows)), net->stream, a, t);
     } else if (tiled) {
@@ -2484,6 +2486,7 @@ int b200_net_get_stat(b200_net* net, const char* key, int64_t* value) {
     else if (!strcmp(key, "ft_tiled")) *value = (net->fwd_tiled() ? 1 : 0) + (net->bwd_tiled() ? 2 : 0);
     else if (!strcmp(key, "ft_forward")) *value = net->fwd_last;
     else if (!strcmp(key, "ft_products")) *value = net->products_last ? 1 : 0;
+    else if (!strcmp(key, "ft_chunk")) *value = net->chunk_last;
     else if (!strcmp(key, "update_copies")) *value = net->update_copies ? 1 : 0;
     else if (!strcmp(key, "slow_weights")) *value = net->S ? 1 : 0;
     else if (!strcmp(key, "optimiser_steps")) *value = net->opt_step;

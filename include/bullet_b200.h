@@ -282,7 +282,8 @@ int b200_get_timings(b200_net* net, b200_timings* out);
 /* Counters: "launches" (kernels launched so far), "h2d_bytes" (batch bytes copied so far),
  * "flat_floats" (length of the flat parameter buffer), "ft_tiled" (bit 0: the forward runs the
  * tiled kernel, bit 1: the backward does), "ft_forward" (the last forward's kernel: 0 the gather, 1 the tiled one, 2 the tiled
- * one that fetches a CTA's next tile ahead), "ft_products" (1: the last backward was the product of bytes), "update_copies" (1: the last b200_step's
+ * one that fetches a CTA's next tile ahead), "ft_products" (1: the last backward was the product of bytes), "ft_chunk" (pairs per chunk of the last
+ * tiled backward, 0 after the gather), "update_copies" (1: the last b200_step's
  * update took a warp per copy of the factoriser). */
 int b200_net_get_stat(b200_net* net, const char* key, int64_t* value);
 /* Debug/inspection: copy an internal activation buffer of the last pass to the host.

@@ -650,8 +650,8 @@ def test_full_size_properties_without_the_oracle():
 
 @pytest.mark.parametrize("option,value", [("ft_once", 0), ("ft_bwd_wide", 0), ("ft_bwd_grab", 3), ("ft_bwd_products", 0)])
 def test_kernel_forms_chosen_by_size_give_the_same_numbers(option, value):
-    """The tiled kernels come in forms the library picks for speed (loads with or without L1 allocation, one or two
-    backward CTAs per SM, how many rows a warp of the backward takes at a time): forcing another form must leave
+    """The tiled kernels come in forms the library picks for speed (one or two backward CTAs per SM, row lists or products of
+    bytes), and accept options that no longer choose any (ft_once, ft_bwd_grab): setting one must leave
     the forward outputs bit-identical and the step within the noise of the reduction order."""
     from bullet_b200.net import featurise
 

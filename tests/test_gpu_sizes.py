@@ -93,6 +93,39 @@ def test_kernel_forms_at_the_edges_of_their_ranges(oracle32, case):
     net.close()
 
 
+@pytest.mark.parametrize("case", [name for name, (desc, _) in CASES.items() if desc.ft_out % 64 == 0 or (desc.ft_out >= 32 and desc.n_inputs < 890)])
+def test_tiled_forward_at_the_edges_of_its_ranges(oracle32, case):
+    """The cases above by the tiled forward, where the library's choice for so few positions is the gather: asked for by name, or, for
+    tables that promise no blocks of whole slabs, with more positions than the gather takes (the two of 900 rows that do not promise any
+    have no tiled form).  Evaluations and steps; bounds as above."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, oracle_ft_output, rich_weights
+
+    desc, n = CASES[case]
+    promised = desc.ft_out % 64 == 0
+    n = n if promised else max(n, 2049)
+    desc = dataclasses.replace(desc, max_batch=n)
+    batch = draw_batch(desc, n, seed=len(case) + n)
+    w = rich_weights(desc)
+    x_ref = oracle_ft_output(oracle32, desc, w, *batch[:2])
+    loss_ref, g_ref, out_ref = oracle32.net_grad(desc, w, *batch)
+    net = make_net(desc, 2 if promised else 0, w)
+    net.upload(0, *batch)
+    out = net.forward(0, n)
+    assert net.stat("ft_forward") > 0
+    assert np.array_equal(net.activation(0, n * desc.dense_in0).reshape(n, -1), x_ref)
+    assert np.abs(out - out_ref).max() <= 2e-5 * np.abs(out_ref).max()
+    net.step(0, 0.0, 1.0 / n)
+    assert net.stat("ft_forward") > 0
+    assert np.array_equal(net.activation(0, n * desc.dense_in0).reshape(n, -1), x_ref)
+    assert abs(net.loss() - loss_ref) <= 2e-5 * loss_ref
+    g = net.tensors(kind=3)
+    for k in g_ref:
+        assert np.abs(g[k] - g_ref[k]).max() <= 2e-5 * np.abs(g_ref[k]).max(), k
+    net.close()
+
+
 @pytest.mark.parametrize("ft_out,pairwise,act,buckets", [(72, False, ACT_SCRELU, 1), (96, False, ACT_CRELU, 3), (136, True, ACT_CRELU, 2)])
 @pytest.mark.parametrize("mode", [0, 1])
 def test_a_loss_gradient_that_is_not_finite_stays_in_its_rows(oracle32, ft_out, pairwise, act, buckets, mode):
@@ -233,8 +266,8 @@ def test_the_largest_tables_of_the_tiled_kernels(oracle32, nnz, rows_less):
 
 @pytest.mark.parametrize("rows", [855, 860, 861, 863, 865, 866])
 def test_the_longest_chunks_of_the_backward(oracle32, rows):
-    """Row counts on either side of where chunks of 640 pairs just fit into shared memory, with a batch that is cut into 148 of
-    them (one for every SM), and with one that is not.  Bounds as above."""
+    """Row counts past where chunks of 640 pairs fit into shared memory, with a batch of 148 of those (one for every SM), which is cut into
+    others, and with a short one.  Bounds as above."""
     import dataclasses
 
     from tests.test_gpu_parity import make_net, rich_weights
@@ -251,6 +284,29 @@ def test_the_longest_chunks_of_the_backward(oracle32, rows):
         g = net.tensors(kind=3)
         for k in g_ref:
             assert np.abs(g[k] - g_ref[k]).max() <= 2e-5 * np.abs(g_ref[k]).max(), k
+    net.close()
+
+
+@pytest.mark.parametrize("rows,chunk", [(832, 640), (838, 640), (839, 640), (840, 640), (841, 632), (843, 632), (846, 632)])
+def test_the_tightest_chunks_of_the_backward(oracle32, rows, chunk):
+    """Chunks of 640 pairs, a line of zeros behind them, and their lists fill shared memory to the last byte at 840 rows; one row more has
+    632.  Batches that are cut into 148 of them (one for every SM).  Bounds as above."""
+    import dataclasses
+
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    n = 148 * chunk // 2
+    desc = dataclasses.replace(net_of(1, rows, 64, 32, 1, (1,)), max_batch=n)
+    w = rich_weights(desc)
+    net = make_net(desc, 0, w)
+    batch = draw_batch(desc, n, seed=rows)
+    net.upload(0, *batch)
+    net.backward(0)
+    assert net.stat("ft_chunk") == chunk
+    _, g_ref, _ = oracle32.net_grad(desc, w, *batch)
+    g = net.tensors(kind=3)
+    for k in g_ref:
+        assert np.abs(g[k] - g_ref[k]).max() <= 2e-5 * np.abs(g_ref[k]).max(), k
     net.close()
 
 
@@ -724,7 +780,7 @@ def test_small_tables_take_the_faster_backward(case):
     (2, 31, 2432, 31, True, 0, (0, 1)),            # less than a round
     (5, 200, 2048, 20, False, 200, (1, 3)),        # blocks without pairs between the tiles
     (2, 768, 2560, 32, True, 768, (0, 1)),
-    (2, 860, 2432, 64, False, 0, (0, 1)),          # the last rounds of rows, warps that walk no lists
+    (2, 860, 2432, 64, False, 0, (0, 1)),          # the last rounds of rows
     (1, 300, 4808, 12, False, 0, (0,)),            # a last slab that is not full
     (1, 300, 4816 * 2, 12, True, 0, (0,)),
 ])
@@ -761,6 +817,40 @@ def test_tiles_fetched_while_the_one_before_is_walked(oracle32, blocks, rows, ft
                 rc, x, _ = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], stm, nstm, n, x_at)
                 assert rc == 0 and np.array_equal(x, x_ref)
     net.close()
+
+
+@pytest.mark.parametrize("blocks,rows,ft_out,nnz,pairwise,factoriser", [
+    (3, 128, 1664, 16, False, 0), (3, 129, 1664, 16, True, 129), (2, 31, 2432, 31, True, 0), (5, 200, 2048, 20, False, 200), (2, 768, 2560, 32, True, 768),
+    (2, 876, 2432, 64, False, 0),   # a warp that walks no lists
+    (2, 890, 2432, 64, True, 0),    # ... as many of them as there can be
+    (1, 300, 4808, 20, False, 0),   # a last slab that is not full
+    (1, 300, 4816 * 2, 12, True, 0),
+])
+def test_the_forward_that_fetches_tiles_ahead_is_the_one_that_runs(oracle32, blocks, rows, ft_out, nnz, pairwise, factoriser):
+    """Evaluations and steps of the sizes above take that form, also with warps that only fetch.  Bit-exact, and so is the operator."""
+    import dataclasses
+
+    from tests.test_gpu_ops import run_op
+    from tests.test_gpu_parity import make_net, rich_weights
+
+    n = 515 * blocks + 7
+    desc = dataclasses.replace(net_of(blocks, rows, ft_out, nnz, 1, (1,), pairwise=pairwise), max_batch=n, factoriser_rows=factoriser)
+    if blocks == 1:
+        desc = dataclasses.replace(desc, ft_block_rows=0)
+    batch = draw_batch(desc, n, seed=rows + ft_out)
+    w = rich_weights(desc)
+    x_ref = oracle_x(oracle32, desc, w, *batch[:2])
+    net = make_net(desc, 0, w)
+    net.upload(0, *batch)
+    for run in (lambda: net.forward(0, n), lambda: net.step(0, 0.0, 1.0 / n)):
+        run()
+        assert net.stat("ft_forward") == 2
+        assert np.array_equal(net.activation(0, n * desc.dense_in0).reshape(n, -1), x_ref)
+    net.close()
+    if blocks > 1 and not factoriser:
+        for x_at in (0, 1):
+            rc, x, _ = run_op("b200_op_ft_forward", desc, w["l0w"], w["l0b"], *batch[:2], n, x_at)
+            assert rc == 0 and np.array_equal(x, x_ref)
 
 
 @pytest.mark.parametrize("copies,rows,ft_out,dense,buckets", [
