@@ -219,16 +219,18 @@ __global__ void __launch_bounds__(256, kUpdCtas) step_update_kernel(const __grid
 // time of the others), each of the others `sets` times 32 float4s of every copy, as many copies at a time as sixteen warps take in equal rounds:
 // ten copies have CTAs of ten warps, four four sets in sixteen.  The gradients of a set meet in shared memory,
 // where a thread per float adds them up in order and updates the factoriser's own.  HBM, with what the backward has left in L2 to be
-// written back besides: 16 copies of 768 rows x 2048 columns (0.75 GB) 154 to 159 us, where a plain pass over clean arrays of them takes 111.
+// written back besides: 16 copies of 768 rows x 2048 columns (0.75 GB, of which 0.70 pass through DRAM) 152 to 157 us, where a plain pass over clean arrays
+// takes 111 (6.3 TB/s of the 0.70).
 // (A ring of bulk copies in one CTA per SM: 196; 64 or 128 float4s of a copy per CTA: 160, 189; the gradients loaded to stay in L2: 160.)
 constexpr int kUpdThreads = 512, kUpdWarps = kUpdThreads / 32;
 struct CopiesShape {
     int copies, sets;  // copies at a time, sets of 32 float4s of each
+    int by_copies;     // 2^16 / copies, rounded up: a warp's set without a division
     int threads() const { return 32 * copies * sets; }
 };
 inline CopiesShape copies_shape(int copies) {
     const int rounds = (copies + kUpdWarps - 1) / kUpdWarps, at_a_time = (copies + rounds - 1) / rounds;
-    return {at_a_time, kUpdWarps / at_a_time};
+    return {at_a_time, kUpdWarps / at_a_time, (1 << 16) / at_a_time + 1};
 }
 // Which of the two forms.  A thread that takes all copies needs the latency of every copy's loads in turn, which many threads hide and few do not:
 // it is as fast where its CTAs fill their waves.  Update on a B200, us, by thread / by warps, 768 rows:
@@ -241,21 +243,27 @@ inline bool update_by_thread(int copies, long long block4, int sms) {
     const long long ctas = (block4 + 255) / 256, wave = (long long)kUpdCtas * sms, waves = (ctas + wave - 1) / wave;
     return copies < 4 || (copies < kUpdWarps && 4 * ctas >= 3 * waves * wave);
 }
+// SIXTEEN: sixteen copies at a time, which fill the CTA, in an instantiation of its own, where what is known of them takes none of the forty
+// registers and no time before the first loads (768 rows, us, general form / this one: 64 columns 4.67 / 4.38, 256 15.5 / 14.9, 512 33.9 / 33.3,
+// 1024 73.1 / 73.6; with a division for a warp's set and a predicate for each of sixteen sums 2048 columns 156 to 161 against 152, 1024 71 against 69 in a whole step).
+template <bool SIXTEEN>
 __global__ void __launch_bounds__(kUpdThreads, 3) step_update_copies_kernel(const __grid_constant__ StepUpdateArgs u, int rest, CopiesShape shape) {
     __shared__ __align__(16) float grads[kUpdWarps][128];
     update_begin(u);
+    const int threads = SIXTEEN ? kUpdThreads : (int)blockDim.x;
     if ((int)blockIdx.x < rest) {
-        update_small(u, blockIdx.x * (long long)blockDim.x + threadIdx.x, (long long)rest * blockDim.x, u.block4);
+        update_small(u, blockIdx.x * (long long)threads + threadIdx.x, (long long)rest * threads, u.block4);
     } else {
         const AdamArgs& a = u.adam;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, set = warp / shape.copies, k0 = warp - set * shape.copies;
-        const int t = 32 * k0 + lane;  // (a set has 128 threads and more)
-        const long long j0 = 32 * ((long long)(blockIdx.x - rest) * shape.sets + set), j = j0 + lane, f = 4 * (u.l0f4 + j0) + t;
+        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, at_a_time = SIXTEEN ? kUpdWarps : shape.copies;
+        const int set = SIXTEEN ? 0 : warp * shape.by_copies >> 16, k0 = SIXTEEN ? warp : warp - set * shape.copies;
+        const int t = SIXTEEN ? (int)threadIdx.x : 32 * k0 + lane;  // (a set has 128 threads and more)
+        const long long tile = (int)blockIdx.x - rest, j0 = 32 * (SIXTEEN ? tile : tile * shape.sets + set), j = j0 + lane, f = 4 * (u.l0f4 + j0) + t;
         const bool own = t < 128 && j0 + t / 4 < u.block4;  // a float of the factoriser
-        const float(*const mine)[128] = grads + set * shape.copies;
+        const float(*const mine)[128] = SIXTEEN ? grads : grads + set * shape.copies;
         float p = 0.f, m = 0.f, v = 0.f, sum = 0.f;
         if (own) p = reinterpret_cast<float*>(a.p)[f], m = reinterpret_cast<float*>(a.m)[f], v = reinterpret_cast<float*>(a.v)[f];
-        for (int c0 = 0; c0 < u.copies; c0 += shape.copies) {
+        for (int c0 = 0; c0 < u.copies; c0 += at_a_time) {
             const int c = c0 + k0;
             if (c < u.copies && j < u.block4) {
                 const long long i = u.l0w4 + c * u.block4 + j;
@@ -266,12 +274,14 @@ __global__ void __launch_bounds__(kUpdThreads, 3) step_update_copies_kernel(cons
             }
             __syncthreads();
             if (t < 128) {
-                const int n = min(shape.copies, u.copies - c0);
+                const int n = min(at_a_time, u.copies - c0);
+                if (SIXTEEN && n == kUpdWarps) {
 #pragma unroll
-                for (int k = 0; k < kUpdWarps; k++)
-                    if (k < n) sum = c0 == 0 && k == 0 ? mine[0][t] : sum + mine[k][t];
+                    for (int k = 0; k < kUpdWarps; k++) sum = c0 == 0 && k == 0 ? mine[0][t] : sum + mine[k][t];
+                } else
+                    for (int k = 0; k < n; k++) sum = c0 == 0 && k == 0 ? mine[0][t] : sum + mine[k][t];
             }
-            if (c0 + shape.copies < u.copies) __syncthreads();
+            if (c0 + at_a_time < u.copies) __syncthreads();
         }
         if (own) {
             reinterpret_cast<float*>(u.g)[f] = sum;

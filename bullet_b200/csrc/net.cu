@@ -1000,7 +1000,7 @@ int preload_kernels(b200_net* net) {
     each_ft_form(net, [&](auto* kernel, bool) { ok = ok && load_kernel(kernel); });
     if (net->small_table()) ok = ok && load_kernel(b200::ft_onehot_kernel) && load_kernel(ft_backward_mma(net));
     ok = ok && load_kernel(b200::factoriser_merge_kernel) && load_kernel(b200::factoriser_grad_kernel);
-    ok = ok && load_kernel(b200::adamw_flat_kernel) && load_kernel(b200::step_update_kernel) && load_kernel(b200::step_update_copies_kernel) && load_kernel(b200::lookahead_kernel);
+    ok = ok && load_kernel(b200::adamw_flat_kernel) && load_kernel(b200::step_update_kernel) && load_kernel(b200::step_update_copies_kernel<true>) && load_kernel(b200::step_update_copies_kernel<false>) && load_kernel(b200::lookahead_kernel);
     ok = ok && load_kernel(b200::adamw_exchange_kernel<0>) && load_kernel(b200::adamw_exchange_kernel<2>);
     ok = ok && load_kernel(b200::adamw_exchange_kernel<4>) && load_kernel(b200::adamw_exchange_kernel<8>);
     ok = ok && load_kernel(b200::adamw_exchange_bulk_kernel<2, 256, 6>) && load_kernel(b200::adamw_exchange_bulk_kernel<2, 512, 3>);
@@ -2300,7 +2300,7 @@ static int step_chained(b200_net* net, Slot& s, int slot, float lr, float grad_f
             const b200::CopiesShape shape = b200::copies_shape(u.copies);
             const int threads = shape.threads(), wide = 32 * shape.sets;
             const int rest = (int)((u.rest4 - u.block4 + threads - 1) / threads), tiles = (int)((u.block4 + wide - 1) / wide);
-            CK(b200::launch_step(true, b200::step_update_copies_kernel, rest + tiles, threads, 0, net->stream, u, rest, shape));
+            CK(b200::launch_step(true, shape.copies == b200::kUpdWarps ? b200::step_update_copies_kernel<true> : b200::step_update_copies_kernel<false>, rest + tiles, threads, 0, net->stream, u, rest, shape));
         } else {
             const long long items = std::max(u.rest4, u.block4);
             CK(b200::launch_step(true, b200::step_update_kernel, (unsigned)std::min<long long>((items + 255) / 256, net->sm_count * 32), 256, 0, net->stream, u));
