@@ -102,8 +102,8 @@ struct TileArgs {
     // backward only: the visiting order cut into chunks of at most kChunkMost pairs that never
     // straddle a block, and per chunk the row-major lists built by ft_csr_kernel
     const int4* chunks;            // [nchunks] (block, first index into `pairs`, pairs, 0)
-    uint16_t* csr_ent;             // [nchunks][ent_cap] pairs of the chunk grouped by row, every list starting on 16 bytes
-    int* csr_start;                // [nchunks][start_cap] per row (start / 8) << 16 | length; [R] = entries in all
+    uint16_t* csr_ent;             // [nchunks][ent_cap] pairs of the chunk grouped by row, every list starting on 8 bytes
+    int* csr_start;                // [nchunks][start_cap] entries, pieces, two unused words, then the pieces (see ft_bwd_start_cap)
     int ent_cap, start_cap;
     int chunk_len;  // CP: most pairs per chunk
     int wide;       // 1024 threads per CTA, one per SM; else 512 and two
@@ -358,10 +358,10 @@ __global__ void __launch_bounds__(256) ft_backward_gather_kernel(FtArgs a, int p
 }
 
 // ------------------------------------------------------------------ tiled kernels
-// A tile row holds 64 floats of one table row as 32 (A, B) pairs; lane l owns pair l and
-// moves it with one 64-bit shared-memory access and one packed f32x2 add.  Without pairwise
-// the pair is two neighbouring columns (64s + 2l, 64s + 2l + 1); with pairwise it is the
-// low-half column 32s + l and its partner H/2 + 32s + l, i.e. both factors of one product.
+// A tile row holds 64 floats of one table row; lane l of a half warp owns floats 4l to 4l + 3 and
+// moves them with one 16-byte shared-memory access and two packed f32x2 adds.  Without pairwise
+// they are neighbouring columns, 64s + 4l on; with pairwise the low-half columns 32s + 2l and 32s + 2l + 1,
+// each before its partner H/2 further on, i.e. both factors of two products.
 constexpr int kTileCols = 64;
 constexpr int kTileRowBytes = kTileCols * 4;
 
@@ -879,8 +879,8 @@ __device__ __forceinline__ int2 ft_bwd_units(const TileArgs& t, int k, int parts
 //
 // Staging: a pair's line takes 8 lanes (pairwise: 32 columns of each half of the accumulator) or 16 lanes, 16 bytes per
 // load, the operands of the next pairs but one under way while a pair's are used (two pairs' operands a lane: more of them make the
-// compiler spill).  Walk: a half warp per list piece (see sum_lines_even).  Bound by the shared-memory pipe in the walk (256 bytes
-// per (row, pair, slab)) and by load latency in the staging.  (One row per warp with 8 bytes per lane, rows in table order: 2.29 against 1.97 ms at 131072
+// compiler spill).  Walk: a half warp per list piece (see sum_lines_even).  Bound by the instructions around the rows and the latency of
+// shared memory in the walk (256 bytes per (row, pair, slab); the pipe is busy 70 to 75 % of it) and by load latency in the staging.  (One row per warp with 8 bytes per lane, rows in table order: 2.29 against 1.97 ms at 131072
 // positions and width 2048, 0.332 against 0.281 ms at 16384.)
 template <bool PAIRWISE, int THREADS, bool SIGNAL, bool ONE>
 __global__ void __launch_bounds__(THREADS, 2048 / (2 * THREADS)) ft_backward_tiled_kernel(FtArgs a, TileArgs t) {
