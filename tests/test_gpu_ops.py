@@ -192,3 +192,66 @@ def test_gathered_calls_take_no_scratch():
     gathered, grouped = traced([(4, 512, 20, 300), (1, 512, 64, 3000)])
     assert gathered == {"ft_forward_gather"}
     assert grouped == {"ft_forward_tiled", "Malloc", "cudaFree"}
+
+
+LOADS = """
+import dataclasses, sys
+import torch
+
+from tests.test_gpu_parity import make_net, rich_weights
+from tests.test_gpu_sizes import draw_batch, net_of
+torch.zeros(1, device="cuda")
+blocks, rows, ft_out, dense, pairwise, factoriser = eval(sys.argv[1])
+most = 4000
+desc = dataclasses.replace(net_of(blocks, rows, ft_out, 12, 2, dense, pairwise=pairwise), max_batch=most, factoriser_rows=factoriser)
+w = rich_weights(desc)
+batches = [draw_batch(desc, n, seed=n) for n in (1, 150, most)]
+
+
+def loaded(run):
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CPU, torch.profiler.ProfilerActivity.CUDA]) as trace:
+        run()
+        torch.cuda.synchronize()
+    return [e.name for e in trace.events()].count("Lazy Function Loading")
+
+
+def work():
+    for mode in (0, 1, 2):
+        net.set_option("ft_mode", mode)
+        for wide in (0, 1):
+            net.set_option("ft_bwd_wide", wide)
+            for batch in batches:
+                n = len(batch[0])
+                net.upload(0, *batch)
+                net.forward(0, n)
+                net.step(0, 1e-3, 1.0 / n)
+                net.loss()
+                net.backward(0)
+                net.update(1e-3, 1.0 / n)
+
+
+first = []
+def create():
+    first.append(make_net(desc, 0, w))
+created = loaded(create)
+net = first[0]
+print(created, loaded(work))
+"""
+
+
+@pytest.mark.parametrize("net,most", [
+    ((4, 300, 128, (16, 32, 1), True, 300), 58), ((4, 300, 128, (1,), False, 0), 58), ((1, 147, 64, (8, 1), False, 0), 58), ((2, 147, 128, (1,), True, 0), 58)])
+def test_networks_load_the_kernels_of_their_kind_when_they_are_made(net, most):
+    """All of them, as a load later may wait for kernels that run, and not those of other kinds: the first form of the two tiled kernels for every kind
+    made it 70 in a fresh process."""
+    import os
+    import subprocess
+    import sys
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", LOADS, repr(net)], cwd=root, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr
+    created, later = map(int, done.stdout.split()[-2:])
+    if not created:
+        pytest.skip("this machine lets no process trace its runtime calls")
+    assert later == 0 and created <= most, (created, later)
